@@ -1,0 +1,36 @@
+"""GPU tests of the kernel variants at the sizes where their tiling or dispatch changes: edges of tiles, remainders,
+the smallest and largest sizes of a rule.  Oracle or plain fp32 / fp64 torch as the reference."""
+import pytest
+import torch
+
+from oracle import mamba2_oracle as orc
+from util import assert_close, randn
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def pm():
+    import __graft_entry__ as ge
+    ge.build()
+    import pm_b200
+    assert torch.cuda.is_available()
+    return pm_b200
+
+
+@pytest.mark.parametrize("offset", [0, 1])        # 1: buffers off the 16-byte grid take the scalar kernels
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 1023, 4099, 1024 * 1024 + 2])
+def test_adamw_sizes_and_alignment(pm, n, offset):
+    p0, g = randn((n,), 1), randn((n,), 2)
+    p_ref, m_ref, v_ref = [p0.clone()], [torch.zeros(n)], [torch.zeros(n)]
+    buf = torch.zeros(n + 1, device="cuda")
+    buf[offset:offset + n] = p0.cuda()
+    opt = pm.AdamW(buf[offset:offset + n], lr=3e-3, weight_decay=0.1)
+    sumsq = opt.step(g.cuda(), max_norm=0.5)
+    g_ref = [g.clone()]
+    norm = orc.clip_grad_norm(g_ref, 0.5)
+    orc.adamw_step(p_ref, g_ref, m_ref, v_ref, 1, lr=3e-3, wd=0.1)
+    assert abs(float(sumsq.item()) ** 0.5 - norm) < 1e-5 * norm
+    assert_close(buf[offset:offset + n], p_ref[0], tol=1e-5, what="params")
+    assert_close(opt.m, m_ref[0], tol=1e-5, what="m")
+    assert_close(opt.v, v_ref[0], tol=1e-5, what="v")
