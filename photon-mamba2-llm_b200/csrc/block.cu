@@ -4,6 +4,7 @@
 // transient workspace that every layer reuses.
 #include "common.cuh"
 #include "kernels.h"
+#include "ssd_fused.h"
 #include "ssd_tc.h"
 
 namespace pmb {
@@ -181,14 +182,68 @@ static pmb_status block_fwd_core(cudaStream_t st, const Dims& d, const pmb_block
   return PMB_OK;
 }
 
+// Buffers of a block forward that keeps nothing for a backward and takes the one-kernel scan: a part of what
+// block_ws_layout asks for in every mode, so a workspace of that size always holds it.
+struct FwdWs { float *xzd, *act, *y, *rstd, *normed; uint16_t *bc_hi, *bc_lo, *x_hi, *x_lo, *normed_hi, *normed_lo, *win_hi, *win_lo, *wout_hi, *wout_lo; };
+static bool fwd_ws_layout(const Dims& d, void* base, size_t bytes, bool bf16, bool pairs, bool presplit, bool plain, FwdWs* w) {
+  Arena ar(base, bytes);
+  const size_t md = (size_t)d.M * d.D, mi = (size_t)d.M * d.I, bc = (size_t)d.M * 2 * d.G * d.N;
+  w->xzd = ar.take<float>((size_t)d.M * d.J);
+  w->act = ar.take<float>((size_t)d.M * d.X);
+  w->y = ar.take<float>(mi);
+  w->rstd = ar.take<float>((size_t)d.M);
+  w->normed = (bf16 || pairs) ? nullptr : ar.take<float>(mi);
+  w->bc_hi = ar.take<uint16_t>(bc);
+  w->bc_lo = plain ? nullptr : ar.take<uint16_t>(bc);
+  w->normed_hi = (bf16 || pairs) ? ar.take<uint16_t>(mi) : nullptr;
+  w->normed_lo = pairs ? ar.take<uint16_t>(mi) : nullptr;
+  if (pairs) { w->x_hi = ar.take<uint16_t>(md); w->x_lo = ar.take<uint16_t>(md); }
+  if (pairs && !presplit) {
+    const size_t dj = (size_t)d.D * d.J, id = (size_t)d.I * d.D;
+    w->win_hi = ar.take<uint16_t>(dj); w->win_lo = ar.take<uint16_t>(dj); w->wout_hi = ar.take<uint16_t>(id); w->wout_lo = ar.take<uint16_t>(id);
+  }
+  return base && ar.ok;
+}
+
 pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, const void* x, const void* residual,
                      void* out, void* ws, size_t ws_bytes, const Weights16* wx, bool x_pair_ready, bool emit_out_pair) {
   const Weights16* w16 = storage_is_bf16(wx) ? wx : nullptr;
   const bool pr = !w16 && block_uses_pairs(d);
-  BlockWs w;
-  if (block_ws_layout(d, ws, ws_bytes, &w, w16 != nullptr, 1, 0, wx && wx->pairs) == 0 || !ws)
-    return fail(PMB_ERR_WORKSPACE, "block workspace too small (%zu < %zu)", ws_bytes, block_ws_bytes(d, w16 != nullptr));
-  PMB_TRY(block_fwd_core(st, d, p, x, w, wx, x_pair_ready && pr));
+  BlockWs w{};
+  if (ssd_chain_enabled() && ssd_chain_shape(d.P, d.N)) {
+    // nothing is kept for a backward: the scan is one kernel that takes dt_raw, x and the B | C pair as the conv left them
+    const bool plain = w16 && ssd_plain16_shape(d.P, d.N, d.Q);
+    FwdWs f{};
+    if (!fwd_ws_layout(d, ws, ws_bytes, w16 != nullptr, pr, wx && wx->pairs, plain, &f))
+      return fail(PMB_ERR_WORKSPACE, "block workspace too small (%zu < %zu)", ws_bytes, block_ws_bytes(d, w16 != nullptr));
+    if (w16) PMB_TRY(gemm_bf16(st, 0, 0, d.M, d.J, d.D, x, d.D, w16->in_proj, d.J, f.xzd, d.J, nullptr, 0));
+    else if (pr) {
+      Pair16 win;
+      if (!x_pair_ready) PMB_TRY(split_pair16(st, static_cast<const float*>(x), d.M, d.D, d.D, f.x_hi, f.x_lo, d.D));
+      PMB_TRY(weight_pair(st, wx, true, p.in_proj_weight, d.D, d.J, f.win_hi, f.win_lo, &win));
+      PMB_TRY(gemm_pairs(st, 0, 0, d.M, d.J, d.D, Pair16{f.x_hi, f.x_lo, d.D}, win, f.xzd, d.J, nullptr));
+    }
+    else PMB_TRY(gemm(st, 0, 0, d.M, d.J, d.D, static_cast<const float*>(x), d.D, p.in_proj_weight, d.J, f.xzd, d.J, nullptr, 0));
+    ConvPairOut bc{f.bc_hi, f.bc_lo, d.I, 2 * d.G * d.N};
+    PMB_TRY(conv_silu_dt_fwd(st, d, f.xzd, p.conv1d_weight, p.conv1d_bias, p.dt_bias, f.act, nullptr, &bc));
+    if (!bc.hi) PMB_TRY(split_pair16_strided(st, f.act + d.I, d.M, 2 * d.G * d.N, d.X, f.bc_hi, f.bc_lo, 2 * d.G * d.N));
+    ChainArgs a{};
+    a.B = d.B; a.T = d.T; a.H = d.H; a.P = d.P; a.N = d.N; a.G = d.G; a.blocks = plain ? d.Q / SCAN_STEP : 1;
+    const int gn = d.G * d.N;
+    a.b = Op16{f.bc_hi, f.bc_lo, 2 * gn};
+    a.c = Op16{f.bc_hi + gn, f.bc_lo ? f.bc_lo + gn : nullptr, 2 * gn};
+    a.x = f.act; a.ldx = d.X; a.D = p.d_skip;
+    a.dt_raw = f.xzd + d.I + d.X; a.ld_raw = d.J; a.dt_bias = p.dt_bias; a.a_log = p.a_log;
+    a.y = f.y; a.ldy = d.I;
+    PMB_TRY(ssd_chain_fwd(st, a));
+    PMB_TRY(gated_rmsnorm_fwd(st, d.M, d.I, d.eps, f.y, f.xzd, d.J, p.norm_weight, f.normed, f.rstd, f.normed_hi, f.normed_lo));
+    w.normed16 = f.normed_hi; w.normed_hi = f.normed_hi; w.normed_lo = f.normed_lo; w.normed = f.normed; w.x_hi = f.x_hi; w.x_lo = f.x_lo;
+    w.wout_hi = f.wout_hi; w.wout_lo = f.wout_lo;
+  } else {
+    if (block_ws_layout(d, ws, ws_bytes, &w, w16 != nullptr, 1, 0, wx && wx->pairs) == 0 || !ws)
+      return fail(PMB_ERR_WORKSPACE, "block workspace too small (%zu < %zu)", ws_bytes, block_ws_bytes(d, w16 != nullptr));
+    PMB_TRY(block_fwd_core(st, d, p, x, w, wx, x_pair_ready && pr));
+  }
   if (w16) PMB_TRY(gemm_bf16(st, 0, 0, d.M, d.D, d.I, w.normed16, d.I, w16->out_proj, d.D, out, d.D, residual, 1));
   else if (pr) {
     Pair16 wout;

@@ -1103,6 +1103,12 @@ static bool fused_enabled() {
   return on != 0;
 }
 
+bool ssd_chain_enabled() {
+  static const bool simt = [] { const char* e = getenv("PMB_SSD_ENGINE"); return e && strcmp(e, "simt") == 0; }();
+  return fused_enabled() && !simt;
+}
+bool ssd_plain16_shape(int P, int N, int Q) { return P == 64 && N == 64 && (Q == 128 || Q == 256); }
+
 // x~[b,t,h,:] = x[b,t,h,:] * dt[b,t,h] as a bf16 pair (only when the fused cumsum kernel did not already write it)
 __global__ void __launch_bounds__(256) xt_pair_kernel(const float* __restrict__ x, int64_t ldx, const float* __restrict__ dt,
                                                       uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, int64_t rows, int H, int P,

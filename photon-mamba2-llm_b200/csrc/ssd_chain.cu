@@ -1,0 +1,693 @@
+// Forward of the chunked SSD scan as one kernel (mamba2/ssd_ops.rs:167-284 computes the same chain op by op): one CTA
+// owns one (batch, head) and walks its sequence in steps of 128 tokens with the state in registers, so that neither
+// C B^T, nor the decay mask, nor the chunk states pass through HBM and a call is one launch.
+//
+// Per step (t, s = tokens of the step, S = inclusive cumulative sum of a inside it, h = state entering it):
+//   x~[s,:] = x[s,:] dt[s],  xs[s,:] = x~[s,:] exp(S_end - S_s)             transform warps -> shared memory (bf16 operands)
+//   G = C B^T   (128 x 128)                                                 tensor core, TMEM
+//   M[t,s] = G[t,s] exp(S_t - S_s) [s <= t]                                 mask warps, TMEM -> registers -> TMEM over G
+//   y[t,:] = M x~ + exp(S_t) C_t h + D x[t,:]                               tensor core, mask warps' epilogue
+//   h <- exp(S_end) h + B^T xs                                              tensor core, state warps' registers
+// S, xs and h can also be kept per chunk of two steps (plain bf16 operands): the second step's rows then see the first
+// one's columns through a masked tile of their own and h as it entered the chunk.
+// Operands are plain bf16 (NS = 1) or (hi, lo) bf16 pairs of fp32 values (NS = 2, three MMAs per product).  Sequences of
+// any length: rows past the end arrive as zeros (TMA fills them per batch) and carry a = 0.  d_state up to 128 and d_head
+// up to 64, in multiples of 8: the 64-wide tiles are zero-filled beyond them.
+//
+// warp 0 = TMA producer (B and C tiles), 1 = MMA issuer, 4..11 = two mask groups of four warps (columns 0-63 / 64-127 of
+// the masked tile; then one half of the output columns each), 12..19 = transform, 20..23 = state.  The MMA issuer runs
+// G one step ahead, the mask warps mask step i + 1 before they drain step i, and the only chain from step to step is
+// h -> h (a few hundred clocks), so the roles overlap.
+// What bounds it: the instructions of the mask warps (mask 2500-2900 clocks, drain and store 3500 of a step of about 6600 with
+// plain operands, 8200 with pairs; two warps of the role per scheduler, so the chains inside a warp count).  The code
+// is kept small (rolled loops): at 130 KB of straight-line code every role waited for instruction fetches and a step took twice
+// as long.  Measured at 24 heads of 64 x 64: 23 us for 4 x 512 tokens on pairs, 147 us for 8 x 2048 on plain operands in chunks of
+// 256, 53 us for 1 x 1337 on pairs; the four kernels it replaces there (prepare, states, state pass, masked product) took 52 and
+// 290 us, the FMA contractions that served the odd length 590 us.  Every mbarrier wait is bounded; on expiry the CTA raises the status
+// word, every role stops issuing work, copies in flight are waited for (bounded) and TMEM is freed on the way out.
+#include <cuda_bf16.h>
+#include <mutex>
+#include <unordered_map>
+#include "tc_common.cuh"
+#include "kernels.h"
+#include "ssd_fused.h"
+
+namespace pmb {
+
+static __device__ unsigned int g_chain_status = 0;
+
+pmb_status read_clear_device_status_chain(unsigned int* word) {
+  unsigned int zero = 0;
+  PMB_CUDA(cudaMemcpyFromSymbol(word, g_chain_status, sizeof(unsigned int)));
+  if (*word) PMB_CUDA(cudaMemcpyToSymbol(g_chain_status, &zero, sizeof(unsigned int)));
+  return PMB_OK;
+}
+
+namespace sc {
+
+using namespace tcx;
+
+constexpr int L = SCAN_STEP;            // tokens per step (= the MMA's M)
+constexpr int PW = 64;                  // width of the head tile
+constexpr int T128 = L * 128;           // bytes of a 128-row x 64-element bf16 tile (128-byte rows)
+constexpr int T64 = 64 * 128;
+// Six warpgroups; setmaxnreg shares the block's 80 x 768 registers out by what a role keeps live (40 + 2 x 88 + 2 x 72 + 120 per
+// thread of the six groups).
+constexpr int W_MASK = 4, W_XF = 12, W_ST = 20, NWARPS = 24, NTHREADS = 32 * NWARPS, XF_THREADS = 256;
+template <int R> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
+template <int R> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
+
+// NB = 128-token blocks per chunk: S, the decay of xs and the state are relative to chunks of NB blocks.
+template <int NS, int NK, int NB>
+struct Geo {
+  static constexpr int BT = NS * NK * T128;              // B (or C) of a step
+  static constexpr int STAGE = 2 * BT;                   // [B | C]
+  static constexpr int XT = NS * T128;                   // x~ (or xs)
+  static constexpr int XBUF = 2 * XT;                    // [x~ | xs]
+  static constexpr int HB = NS * NK * T64;               // state operand, rows n of 128 bytes
+  static constexpr bool BIG = NS * NK == 4;              // pairs at d_state 128: one stage of B | C is all that fits
+  static constexpr int STG = BIG ? 1 : 2;
+  static constexpr int XB = NS == 1 ? 2 : 1;
+  static constexpr int NSB = NB == 1 ? XB + 1 : 2;       // copies of S: a chunk's S is read until its last tile has been masked
+  static_assert(NB == 1 || (STG == 2 && XB == 2), "both blocks of a chunk are resident");
+  static constexpr int TILES = STG * STAGE + XB * XBUF + HB;
+  static constexpr int AHEAD = BIG ? 0 : (NS * NK == 2 ? 3 : 4);              // 16-byte pieces of x that every transform thread has in flight
+  static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 256 /*barriers*/ + NSB * NB * L * 4 + (BIG ? 4 : 8) * NB * L /*row factors*/ + AHEAD * XF_THREADS * 16;
+};
+
+struct Maps { CUtensorMap b[2], c[2]; };                 // [0] = hi (or the plain bf16 tensor), [1] = lo
+
+struct Params {
+  int T, H, hpg, N, P, nsteps;
+  const float* x; const uint16_t* x16; int64_t ldx;
+  const float* dt_raw; int64_t ld_raw; const float* dt_bias; const float* a_log;   // raw mode: dt and A are formed here
+  const float* dt; const float* A; const float* a;                                 // (dt, A) or a alone
+  const float* D;
+  const float* init;                                     // (B,H,N,P) or NULL
+  float* y; uint16_t* y16; int64_t ldy;
+  float* dt_out; float* A_out; float* S_out;             // optional from here on: what a backward reads
+  uint16_t* x_keep;                                      // (B,T,H,P) copy of x16
+  uint16_t *hp_hi, *hp_lo;                               // (B,nsteps,H,N,P)
+  float* last;                                           // (B,H,N,P)
+  unsigned int* status;
+};
+
+__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo, bool want_lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  if (want_lo) {
+    const float2 hf = __bfloat1622float2(h);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(a - hf.x, b - hf.y);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+  }
+}
+__device__ __forceinline__ void st_shared_v2(uint32_t a, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+      : "memory");
+}
+
+template <int NS, int NK, int NB, bool XIN16>
+__global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid_constant__ Maps maps, const Params p) {
+  using GE = Geo<NS, NK, NB>;
+  constexpr int STG = GE::STG, XB = GE::XB, NSB = GE::NSB;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  uint8_t* base_ptr = smem_raw + (base - raw);
+  const uint32_t ring_s = base, xbuf_s = ring_s + STG * GE::STAGE, h_s = xbuf_s + XB * GE::XBUF, bars = h_s + GE::HB;
+  enum { FULL = 0, EMPTY = 2, XRDY = 4, XFREE = 6, SRDY = 8 /*4*/, GFULL = 12, MRDY = 14, UFULL = 16, UFREE, HRDY, HFREE, ACCFULL, ACCFREE, NBAR };
+  static_assert(8 * NBAR + 16 + 48 <= 256, "barrier block");
+  auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
+  uint8_t* bar_ptr = base_ptr + (bars - base);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 8 * NBAR);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+  float* wsum = reinterpret_cast<float*>(bar_ptr + 8 * NBAR + 16);
+  float* sEnd = wsum + 8;                                   // S_end of the last four chunks
+  float* sS = reinterpret_cast<float*>(bar_ptr + 256);
+  float2* sfac = reinterpret_cast<float2*>(sS + NSB * NB * L);   // (dt, exp(S_end - S)) of the step's rows
+  float* sdt = sS + NSB * NB * L;                                // BIG: dt alone, the last kilobyte is not there
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int h = (int)blockIdx.x % p.H, bb = (int)blockIdx.x / p.H, g = h / p.hpg;
+  const int n = p.nsteps;
+  const int64_t tokb = (int64_t)bb * p.T;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(FULL + i), 1); mbar_init(bar(EMPTY + i), 1);
+      mbar_init(bar(XRDY + i), 8); mbar_init(bar(XFREE + i), 1);
+      mbar_init(bar(GFULL + i), 1); mbar_init(bar(MRDY + i), 8);
+    }
+    for (int i = 0; i < 4; ++i) mbar_init(bar(SRDY + i), 8);
+    mbar_init(bar(UFULL), 1); mbar_init(bar(UFREE), 4); mbar_init(bar(HRDY), 4); mbar_init(bar(HFREE), 1);
+    mbar_init(bar(ACCFULL), 1); mbar_init(bar(ACCFREE), 8);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "n"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t tG = tmem, tA1 = tmem + 256, tA2 = tmem + 320, tU = tmem + 384;
+
+  auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
+  // bounded waits that also end as soon as another role of the CTA has given up
+  auto wait = [&](int b, uint32_t parity, unsigned int code) -> bool {
+    if (*abort_flag) return false;
+    if (mbar_wait(bar(b), parity & 1u)) return true;
+    give_up(code);
+    return false;
+  };
+
+  if (warp < W_MASK) {
+  regs_dec<40>();
+  if (warp == 0) {
+    // ---------------- TMA producer: B and C tiles of each step ----------------
+    if (lane == 0) {
+      int issued = 0;
+      for (int i = 0; i < n; ++i) {
+        const int s = i % STG;
+        if (!wait(EMPTY + s, (uint32_t)(i / STG) ^ 1u, 1u)) break;
+        mbar_expect_tx(bar(FULL + s), GE::STAGE);
+        const uint32_t dst = ring_s + s * GE::STAGE;
+#pragma unroll
+        for (int sp = 0; sp < NS; ++sp)
+#pragma unroll
+          for (int kt = 0; kt < NK; ++kt) {
+            tma_load_4d(dst + (sp * NK + kt) * T128, &maps.b[sp], 64 * kt, i * L, g, bb, bar(FULL + s));
+            tma_load_4d(dst + GE::BT + (sp * NK + kt) * T128, &maps.c[sp], 64 * kt, i * L, g, bb, bar(FULL + s));
+          }
+        issued = i + 1;
+      }
+      if (*abort_flag)
+        for (int i = (issued > STG ? issued - STG : 0); i < issued; ++i) mbar_wait(bar(FULL + i % STG), (uint32_t)((i / STG) & 1));
+    }
+  } else if (warp == 1) {
+    // ---------------- MMA issuer (the whole warp waits; one elected lane issues) ----------------
+    const uint32_t dh = desc_hi(1024, 2);
+    const uint32_t id_g = idesc_bf16(0, 0, L, L);            // G: both operands K-major
+    const uint32_t id_v = idesc_bf16(0, 1, L, PW);           // x x~, x h: B operand MN-major
+    const uint32_t id_u = idesc_bf16(1, 1, L, PW);           // B^T xs: both operands MN-major
+    auto kstep = [&](uint32_t d, uint32_t alo, uint32_t as, uint32_t blo, uint32_t bs, uint32_t idesc, uint32_t acc) {
+      if (NS == 2) {
+        mma_f16_h(d, alo + as, dh, blo, dh, idesc, acc);          // lo x hi
+        mma_f16_h(d, alo, dh, blo + bs, dh, idesc, 1u);           // hi x lo
+        mma_f16_h(d, alo, dh, blo, dh, idesc, 1u);                // hi x hi
+      } else {
+        mma_f16_h(d, alo, dh, blo, dh, idesc, acc);
+      }
+    };
+    auto all = [&](bool v) -> bool { return __all_sync(0xffffffffu, v); };
+    // G of the item (block k, earlier or same block kb of its chunk) into buffer m & 1
+    auto mma_g = [&](int m, int k, int kb) -> bool {
+      if (!all(wait(FULL + k % STG, (uint32_t)(k / STG), 2u))) return false;      // (block kb <= k has landed before)
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t b0 = desc_lo(ring_s + (kb % STG) * GE::STAGE, 16), c0 = desc_lo(ring_s + (k % STG) * GE::STAGE + GE::BT, 16);
+      // (the buffer's previous content, the masked tile of item m - 2, is read by products issued before this one)
+      if (elect_one()) {
+#pragma unroll
+        for (int kt = 0; kt < NK; ++kt)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t o = (uint32_t)(kt * T128 + q * 32) >> 4;
+            kstep(tG + (uint32_t)((m & 1) * L), c0 + o, (NK * T128) >> 4, b0 + o, (NK * T128) >> 4, id_g, (kt | q) ? 1u : 0u);
+          }
+        umma_commit(bar(GFULL + (m & 1)));
+      }
+      __syncwarp();
+      return true;
+    };
+    bool ok = mma_g(0, 0, 0);
+    int m = 0;                                               // item: (block, column block), the diagonal one last
+#pragma unroll 1
+    for (int k = 0; k < n && ok; ++k) {
+      const int s = k % STG, xb = k % XB, rb = k % NB, c = k / NB;
+      if (STG == 1 && k > 0 && !(ok = mma_g(m, k, k))) break;
+#pragma unroll 1
+      for (int cb = 0; cb <= rb; ++cb, ++m) {
+        if (STG == 2) {                                      // one item ahead
+          if (cb < rb) ok = mma_g(m + 1, k, k - rb + cb + 1);
+          else if (k + 1 < n) ok = mma_g(m + 1, k + 1, k + 1 - (k + 1) % NB);
+          if (!ok) break;
+        }
+        if (cb == 0) {
+          // acc2 = C h
+          if (!(ok = all(wait(HRDY, (uint32_t)c, 8u) && (k == 0 || wait(ACCFREE, (uint32_t)(k - 1), 8u))))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (elect_one()) {
+            const uint32_t c0 = desc_lo(ring_s + s * GE::STAGE + GE::BT, 16), h0 = desc_lo(h_s, T64);
+#pragma unroll
+            for (int kt = 0; kt < NK; ++kt)
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+                kstep(tA2, c0 + ((uint32_t)(kt * T128 + q * 32) >> 4), (NK * T128) >> 4, h0 + ((uint32_t)(kt * T64 + q * 2048) >> 4), (NK * T64) >> 4, id_v,
+                      (kt | q) ? 1u : 0u);
+            if (rb == NB - 1 || k + 1 == n) umma_commit(bar(HFREE));
+          }
+          __syncwarp();
+        }
+        // acc1 += M x~, the masked tile read from TMEM: per 32 columns [hi: 16 | lo: 16], 8 columns per k-step of 16
+        if (!(ok = all((cb < rb || wait(XRDY + xb, (uint32_t)(k / XB), 4u)) && wait(MRDY + (m & 1), (uint32_t)(m >> 1), 16u)))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t xt0 = desc_lo(xbuf_s + ((k - rb + cb) % XB) * GE::XBUF, T128);
+        if (elect_one()) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint32_t ta = tG + (uint32_t)((m & 1) * L + (q >> 1) * 32 + (q & 1) * 8), vb = xt0 + ((uint32_t)(q * 2048) >> 4);
+            const uint32_t acc = (q | cb) ? 1u : 0u;
+            if (NS == 2) {
+              mma_f16_ts_h(tA1, ta + 16u, vb, dh, id_v, acc);
+              mma_f16_ts_h(tA1, ta, vb + (T128 >> 4), dh, id_v, 1u);
+              mma_f16_ts_h(tA1, ta, vb, dh, id_v, 1u);
+            } else {
+              mma_f16_ts_h(tA1, ta, vb, dh, id_v, acc);
+            }
+          }
+          if (cb == rb) umma_commit(bar(ACCFULL));
+          else umma_commit(bar(XFREE + (k - rb + cb) % XB));      // (the earlier block of the chunk is done with)
+        }
+        __syncwarp();
+      }
+      if (!ok) break;
+      // U (+)= B^T xs: the chunk's contribution to the state
+      if (!(ok = all(rb > 0 || c == 0 || wait(UFREE, (uint32_t)(c - 1), 4u)))) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (elect_one()) {
+        // (M = 128 over one or two 64-wide blocks of d_state; with one block the second reads the tile behind it and
+        // its rows of U are never looked at)
+        const uint32_t b0 = desc_lo(ring_s + s * GE::STAGE, T128), xs0 = desc_lo(xbuf_s + xb * GE::XBUF + GE::XT, T128);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const uint32_t o = (uint32_t)(q * 2048) >> 4;
+          kstep(tU, b0 + o, (NK * T128) >> 4, xs0 + o, T128 >> 4, id_u, (q | rb) ? 1u : 0u);
+        }
+        if (rb == NB - 1 || k + 1 == n) umma_commit(bar(UFULL));
+        if (rb == NB - 1) umma_commit(bar(XFREE + xb));
+        umma_commit(bar(EMPTY + s));
+      }
+      __syncwarp();
+    }
+  }
+  } else if (warp < W_XF) {
+    // ---------------- mask groups, then epilogue of the step before ----------------
+    regs_inc<88>();
+    const int quarter = warp & 3, grp = (warp - W_MASK) >> 2, r_local = quarter * 32 + lane;
+    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+    bool ok = true;
+    const float dv = p.D ? p.D[h] : 0.0f;
+    // the accumulators are drained in fragments of 16 rows x 8 columns (a quad of lanes holds 8 columns of a row: whole
+    // 32-byte sectors per store), so a thread's output rows are er + {0, 8, 16, 24} and not the row that it masks
+    const int er = quarter * 32 + (lane >> 2), ec = (lane & 3) * 2;
+    float fac[4] = {0.0f, 0.0f, 0.0f, 0.0f};                // exp(S) of those rows in the step whose epilogue is due
+    int k = 0, rb = 0, cb = 0;                              // this item: block k = block rb of its chunk, column block cb
+    // item after item; after the first tile of a block has been masked, the block before it is drained
+    for (int m = 0; k <= n; ++m) {
+      float fnext[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      const bool first = cb == 0;
+      if (ok && k < n) {
+        const int c = k / NB;
+        const float* S = sS + (c % NSB) * NB * L;
+        const bool got = wait(SRDY + (c % NSB), (uint32_t)(c / NSB), 32u) && wait(GFULL + (m & 1), (uint32_t)(m >> 1), 32u);
+        ok = __all_sync(0xffffffffu, got);
+        if (ok) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const float* Sc = S + cb * L;                      // S of the tile's columns
+          const float S_row = S[rb * L + r_local];
+          if (first) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) fnext[e] = __expf(S[rb * L + er + 8 * e]);
+          }
+          const int c0 = grp * 64;
+          const uint32_t tg = tG + lane_addr + (uint32_t)((m & 1) * L + c0);
+          const bool above = cb == rb && grp == 1 && quarter < 2;       // every column of this half is past every row of this warp
+          const bool below = cb < rb || (grp == 0 && quarter >= 2);      // no column of this half is past any row of this warp
+#pragma unroll 1
+          for (int half = 0; half < 2; ++half) {
+            uint32_t mh[16], ml[16];
+            if (above) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) { mh[e] = 0u; ml[e] = 0u; }
+            } else {
+              uint32_t r[32];
+              tmem_ld32(tg + (uint32_t)(half * 32), r);
+#pragma unroll
+              for (int e2 = 0; e2 < 16; ++e2) {
+                const int col = c0 + half * 32 + 2 * e2;
+                const float2 sv = *reinterpret_cast<const float2*>(Sc + col);
+                float m0 = __uint_as_float(r[2 * e2]) * __expf(S_row - sv.x), m1 = __uint_as_float(r[2 * e2 + 1]) * __expf(S_row - sv.y);
+                if (!below) { m0 = col <= r_local ? m0 : 0.0f; m1 = col + 1 <= r_local ? m1 : 0.0f; }
+                ml[e2] = 0u;
+                split2(m0, m1, mh[e2], ml[e2], NS == 2);
+              }
+            }
+            tmem_st16(tg + (uint32_t)(half * 32), mh);
+            if (NS == 2) tmem_st16(tg + (uint32_t)(half * 32 + 16), ml);
+          }
+          tmem_wait_st();
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(MRDY + (m & 1)));
+        }
+      }
+      if (ok && first && k > 0) {
+        const int i = k;
+        const int col = h * p.P + 32 * grp + ec;
+        float2 x[4][2];                                     // the skip term's x of one 16-row half
+        auto fetch_x = [&](int rh) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int t = (i - 1) * L + er + 16 * rh + 8 * e;
+            const float* xr = p.x + (tokb + t) * p.ldx + col;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              x[q][e] = p.D && t < p.T && 32 * grp + 8 * q < p.P ? *reinterpret_cast<const float2*>(xr + 8 * q) : make_float2(0.0f, 0.0f);
+          }
+        };
+        fetch_x(0);                                         // (requested ahead of the accumulators)
+        ok = __all_sync(0xffffffffu, wait(ACCFULL, (uint32_t)(i - 1), 64u));
+        if (ok) {
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          // both accumulators into registers, combined, and handed back before anything waits for memory
+          float2 o[2][4][2];                                // [16-row half][8-column group][row, row + 8]
+#pragma unroll
+          for (int rh = 0; rh < 2; ++rh)
+#pragma unroll
+            for (int c16 = 0; c16 < 2; ++c16) {
+              uint32_t a1[8], a2[8];
+              const uint32_t ta = lane_addr + ((uint32_t)(16 * rh) << 16) + (uint32_t)(32 * grp + 16 * c16);
+              tmem_ld16x256_x2(tA1 + ta, a1);
+              tmem_ld16x256_x2(tA2 + ta, a2);
+              tmem_wait_ld();
+#pragma unroll
+              for (int q = 0; q < 2; ++q)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                  const float f = fac[2 * rh + e];
+                  o[rh][2 * c16 + q][e] = make_float2(fmaf(f, __uint_as_float(a2[4 * q + 2 * e]), __uint_as_float(a1[4 * q + 2 * e])),
+                                                      fmaf(f, __uint_as_float(a2[4 * q + 2 * e + 1]), __uint_as_float(a1[4 * q + 2 * e + 1])));
+                }
+            }
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(ACCFREE));
+#pragma unroll
+          for (int rh = 0; rh < 2; ++rh) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) { o[rh][q][e].x = fmaf(dv, x[q][e].x, o[rh][q][e].x); o[rh][q][e].y = fmaf(dv, x[q][e].y, o[rh][q][e].y); }
+            if (rh == 0) fetch_x(1);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int t = (i - 1) * L + er + 16 * rh + 8 * e;
+              if (!p.y16 && t < p.T) {
+                float* yr = p.y + (tokb + t) * p.ldy + col;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) if (32 * grp + 8 * q < p.P) *reinterpret_cast<float2*>(yr + 8 * q) = o[rh][q][e];
+              }
+              if (p.y16) {
+                // neighbouring lanes swap halves, so that a lane writes four columns and a quad one whole sector
+#pragma unroll
+                for (int q = 0; q < 4; q += 2) {
+                  uint32_t v0, v1, z;
+                  split2(o[rh][q][e].x, o[rh][q][e].y, v0, z, false); split2(o[rh][q + 1][e].x, o[rh][q + 1][e].y, v1, z, false);
+                  const bool odd = lane & 1;
+                  const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
+                  const uint2 w = odd ? make_uint2(got, v1) : make_uint2(v0, got);
+                  // even lanes: columns ec .. ec + 3 of the first eight; odd lanes: ec - 2 .. ec + 1 of the second
+                  if (t < p.T && 32 * grp + 8 * (q + (odd ? 1 : 0)) < p.P)
+                    *reinterpret_cast<uint2*>(p.y16 + (tokb + t) * p.ldy + col + 8 * q + (odd ? 6 : 0)) = w;
+                }
+              }
+            }
+          }
+        }
+      }
+      if (first) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) fac[e] = fnext[e];
+      }
+      if (cb == rb) { ++k; rb = rb + 1 == NB ? 0 : rb + 1; cb = 0; } else ++cb;
+    }
+  } else if (warp < W_ST) {
+    // ---------------- transform: S of the step, x -> x~ and xs ----------------
+    regs_dec<72>();
+    const int wx = warp - W_XF, tid = threadIdx.x - 32 * W_XF;
+    const float Ah = p.dt_raw ? -expf(p.a_log[h]) : (p.dt ? p.A[h] : 1.0f);
+    const float bias = p.dt_raw ? p.dt_bias[h] : 0.0f;
+    if (p.dt_raw && p.A_out && bb == 0 && tid == 0) p.A_out[h] = Ah;
+    constexpr int LPR = XIN16 ? 8 : 16;                     // lanes per row, 16 bytes each
+    constexpr int RPI = 8 * (32 / LPR), NIT = L / RPI;      // rows per pass of the eight warps, passes
+    constexpr int EPL = XIN16 ? 8 : 4;                      // elements per lane
+    const int j = lane % LPR, r0 = wx * (32 / LPR) + lane / LPR;
+    const bool jcol = EPL * j < p.P;
+    // this lane's place in a row of an operand tile (rows of 128 bytes, 16-byte pieces xor-swizzled by the row)
+    const uint32_t place = (uint32_t)(r0 * 128) + (XIN16 ? (uint32_t)((j ^ (r0 & 7)) << 4) : (uint32_t)((((j >> 1) ^ (r0 & 7)) << 4) + (j & 1) * 8));
+    // x: every thread copies the pieces that it will read itself, AHEAD passes before it reads them, into a ring of its own
+    // (cp.async; no barrier; rows past the end arrive as zeros)
+    constexpr int RING = GE::AHEAD > 0 ? GE::AHEAD : 1;
+    const uint32_t xring = smem_u32(sfac + NB * L) + (uint32_t)tid * 16u;
+    const char* src = XIN16 ? reinterpret_cast<const char*>(p.x16 + (tokb + r0) * p.ldx + h * p.P + (jcol ? EPL * j : 0))
+                            : reinterpret_cast<const char*>(p.x + (tokb + r0) * p.ldx + h * p.P + (jcol ? EPL * j : 0));
+    const int64_t sstep = (int64_t)RPI * p.ldx * (XIN16 ? 2 : 4);
+    int frow = r0;                                          // row of the next piece to request
+    auto request = [&](uint32_t slot) {
+      const bool in = frow < p.T && jcol;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(xring + slot), "l"(src), "r"(in ? 16 : 0) : "memory");
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      frow += RPI;
+      if (frow < p.T) src += sstep;                         // (the address stays inside the tensor)
+    };
+    auto fetch_a = [&](int c) -> float {                    // of this thread's token of chunk c
+      const int t = c * NB * L + tid;
+      if (tid >= NB * L || t >= p.T) return 0.0f;
+      const int64_t tk = tokb + t;
+      if (p.dt_raw) return p.dt_raw[tk * p.ld_raw + h];
+      return p.dt ? p.dt[tk * p.H + h] : p.a[tk * p.H + h];
+    };
+    if (GE::AHEAD > 0) {
+      if (r0 >= p.T) { src = XIN16 ? reinterpret_cast<const char*>(p.x16) : reinterpret_cast<const char*>(p.x); }
+#pragma unroll 1
+      for (int q = 0; q < RING; ++q) request((uint32_t)q * (XF_THREADS * 16));
+    }
+    float av = fetch_a(0);
+    uint32_t slot = 0;
+    bool ok = true;
+    for (int i = 0; i < n; ++i) {
+      const int c = i / NB, rb = i % NB;
+      float* S = sS + (c % NSB) * NB * L;
+      if (rb == 0) {
+        // S of the chunk.  A warp that gave up keeps reaching the named barriers: it skips the work, not the barrier.
+        const int t = c * NB * L + tid;
+        const bool in = tid < NB * L && t < p.T;
+        float dtv = 1.0f, v = av;
+        if (p.dt_raw) { dtv = in ? softplus_acc(av + bias) : 0.0f; v = Ah * dtv; }
+        else if (p.dt) { dtv = av; v = Ah * av; }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const float u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
+        if (lane == 31 && tid < NB * L) wsum[wx] = v;
+        asm volatile("bar.sync 4, 256;" ::: "memory");
+        if (tid < NB * L) {
+          float off = 0.0f, send = 0.0f;                    // fixed order
+#pragma unroll
+          for (int q = 0; q < 4 * NB; ++q) { if (q == wx) off = send; send += wsum[q]; }
+          v += off;
+          if (tid == NB * L - 1) v = send;
+          // (nobody reads the buffer's old content any more: this thread has waited for the last products of the step, with
+          // two operand buffers of the second last, before the block before this one; those products read tiles masked with it)
+          S[tid] = v;
+          if (GE::BIG) sdt[tid] = dtv; else sfac[tid] = make_float2(dtv, __expf(send - v));
+          if (tid == NB * L - 1) sEnd[c & 3] = send;
+          if (in) {
+            if (p.S_out) p.S_out[((int64_t)bb * p.H + h) * p.T + t] = v;
+            if (p.dt_out) p.dt_out[(tokb + t) * p.H + h] = dtv;
+          }
+        }
+        asm volatile("bar.sync 4, 256;" ::: "memory");
+        if (lane == 0) mbar_arrive(bar(SRDY + (c % NSB)));
+        if (i + NB < n) av = fetch_a(c + 1);
+      }
+      if (ok && i >= XB) ok = __all_sync(0xffffffffu, wait(XFREE + (i % XB), (uint32_t)(i / XB - 1), 128u));
+      if (ok) {
+        uint32_t dst = xbuf_s + (i % XB) * GE::XBUF + place;
+#pragma unroll 2
+        for (int it = 0; it < NIT; ++it, dst += RPI * 128) {
+          uint4 xq = make_uint4(0u, 0u, 0u, 0u);
+          if (GE::AHEAD > 0) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(RING - 1) : "memory");
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(xq.x), "=r"(xq.y), "=r"(xq.z), "=r"(xq.w) : "r"(xring + slot) : "memory");
+          } else {
+            if (frow < p.T && jcol) xq = *reinterpret_cast<const uint4*>(src);
+            frow += RPI; src += sstep;
+          }
+          const int rc = rb * L + it * RPI + r0;            // row of the chunk
+          const float2 f = GE::BIG ? make_float2(sdt[rc], __expf(sEnd[c & 3] - S[rc])) : sfac[rc];
+          if (XIN16) {
+            const uint32_t in4[4] = {xq.x, xq.y, xq.z, xq.w};
+            uint32_t s4[4], z;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) split2(__uint_as_float(in4[e] << 16) * f.y, __uint_as_float(in4[e] & 0xffff0000u) * f.y, s4[e], z, false);
+            st_shared_v4(dst, in4[0], in4[1], in4[2], in4[3]);
+            st_shared_v4(dst + GE::XT, s4[0], s4[1], s4[2], s4[3]);
+            // (the backward of the bf16 scan is not handed x again)
+            const int row = i * L + it * RPI + r0;
+            if (p.x_keep && jcol && row < p.T) *reinterpret_cast<uint4*>(p.x_keep + (tokb + row) * p.ldx + h * p.P + EPL * j) = xq;
+          } else {
+            const float f0 = __uint_as_float(xq.x) * f.x, f1 = __uint_as_float(xq.y) * f.x, f2 = __uint_as_float(xq.z) * f.x, f3 = __uint_as_float(xq.w) * f.x;
+            uint32_t h0, h1, l0 = 0u, l1 = 0u, g0, g1, k0 = 0u, k1 = 0u;
+            split2(f0, f1, h0, l0, NS == 2); split2(f2, f3, h1, l1, NS == 2);
+            split2(f0 * f.y, f1 * f.y, g0, k0, NS == 2); split2(f2 * f.y, f3 * f.y, g1, k1, NS == 2);
+            st_shared_v2(dst, h0, h1);
+            st_shared_v2(dst + GE::XT, g0, g1);
+            if (NS == 2) { st_shared_v2(dst + T128, l0, l1); st_shared_v2(dst + GE::XT + T128, k0, k1); }
+          }
+          if (GE::AHEAD > 0) {
+            request(slot);                                  // (this pass has consumed the slot)
+            slot = slot + XF_THREADS * 16 == RING * XF_THREADS * 16 ? 0u : slot + XF_THREADS * 16;
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(XRDY + (i % XB)));
+      }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+  } else {
+    // ---------------- state: h in registers (thread = row n of the state) ----------------
+    regs_inc<120>();
+    const int quarter = warp & 3, nr = quarter * 32 + lane;
+    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+    const bool active = nr < p.N;                           // rows past d_state hold zeros
+    const bool tile = quarter * 32 < 64 * NK;               // this warp's rows exist in the operand tile
+    const int64_t NP = (int64_t)p.N * p.P;
+    float hv[PW];
+#pragma unroll
+    for (int q = 0; q < PW / 4; ++q) {
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (p.init && active && 4 * q < p.P) v = *reinterpret_cast<const float4*>(p.init + ((int64_t)bb * p.H + h) * NP + (int64_t)nr * p.P + 4 * q);
+      hv[4 * q] = v.x; hv[4 * q + 1] = v.y; hv[4 * q + 2] = v.z; hv[4 * q + 3] = v.w;
+    }
+    bool ok = true;
+    const int nch = (n + NB - 1) / NB;
+    for (int i = 0; i < nch && ok; ++i) {                   // chunk after chunk
+      if (i > 0) ok = __all_sync(0xffffffffu, wait(HFREE, (uint32_t)(i - 1), 256u));
+      if (!ok) break;
+      const int64_t so = (((int64_t)bb * nch + i) * p.H + h) * NP + (int64_t)nr * p.P;
+      if (tile) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {                       // eight 16-byte chunks of the row
+          uint32_t hi[4], lo[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) split2(hv[8 * c + 2 * e], hv[8 * c + 2 * e + 1], hi[e], lo[e], NS == 2);
+          const uint32_t a = h_s + (uint32_t)(nr * 128 + ((c ^ (nr & 7)) << 4));
+          st_shared_v4(a, hi[0], hi[1], hi[2], hi[3]);
+          if (NS == 2) st_shared_v4(a + NK * T64, lo[0], lo[1], lo[2], lo[3]);
+          if (p.hp_hi && active && 8 * c < p.P) {
+            *reinterpret_cast<uint4*>(p.hp_hi + so + 8 * c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            if (NS == 2) *reinterpret_cast<uint4*>(p.hp_lo + so + 8 * c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          }
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(HRDY));
+      ok = __all_sync(0xffffffffu, wait(SRDY + (i % NSB), (uint32_t)(i / NSB), 512u) && wait(UFULL, (uint32_t)i, 512u));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const float dec = __expf(sEnd[i & 3]);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t u[16];
+        tmem_ld16(tU + lane_addr + (uint32_t)(16 * q), u);
+        tmem_wait_ld();
+        if (active) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) hv[16 * q + e] = fmaf(dec, hv[16 * q + e], __uint_as_float(u[e]));
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(UFREE));
+    }
+    if (ok && p.last && active) {
+      float* dst = p.last + ((int64_t)bb * p.H + h) * NP + (int64_t)nr * p.P;
+#pragma unroll
+      for (int q = 0; q < PW / 4; ++q)
+        if (4 * q < p.P) *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
+  }
+}
+
+// ---- host side -------------------------------------------------------------------------------------------
+static unsigned int* status_ptr() {
+  static unsigned int* ptr[PMB_MAX_DEVICES] = {nullptr};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= PMB_MAX_DEVICES) dev = 0;
+  if (!ptr[dev]) cudaGetSymbolAddress((void**)&ptr[dev], g_chain_status);
+  return ptr[dev];
+}
+
+template <int NS, int NK, int NB, bool XIN16>
+static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
+  using GE = Geo<NS, NK, NB>;
+  static_assert(GE::SMEM <= 227 * 1024, "shared-memory plan");
+  Maps ms{};
+  for (int sp = 0; sp < 2; ++sp) {
+    const bool lo = sp && NS == 2;
+    PMB_TRY(sf::bf16_map4(&ms.b[sp], lo ? a.b.lo : a.b.hi, a.N, a.T, a.G, a.B, a.b.pitch, a.N, (int64_t)a.T * a.b.pitch, 64, L));
+    PMB_TRY(sf::bf16_map4(&ms.c[sp], lo ? a.c.lo : a.c.hi, a.N, a.T, a.G, a.B, a.c.pitch, a.N, (int64_t)a.T * a.c.pitch, 64, L));
+  }
+  Params p{};
+  p.T = a.T; p.H = a.H; p.hpg = a.H / a.G; p.N = a.N; p.P = a.P; p.nsteps = (int)cdiv(a.T, L);
+  p.x = a.x; p.x16 = a.x16; p.ldx = a.ldx;
+  p.dt_raw = a.dt_raw; p.ld_raw = a.ld_raw; p.dt_bias = a.dt_bias; p.a_log = a.a_log; p.dt = a.dt; p.A = a.A; p.a = a.a; p.D = a.D;
+  p.init = a.init; p.y = a.y; p.y16 = a.y16; p.ldy = a.ldy; p.dt_out = a.dt_out; p.A_out = a.A_out; p.S_out = a.S_out;
+  p.x_keep = a.x_keep; p.hp_hi = a.hp_hi; p.hp_lo = a.hp_lo; p.last = a.last; p.status = status_ptr();
+  PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_fwd_kernel<NS, NK, NB, XIN16>);
+  ssd_chain_fwd_kernel<NS, NK, NB, XIN16><<<(unsigned)(a.B * a.H), NTHREADS, GE::SMEM, st>>>(ms, p);
+  PMB_LAUNCHED();
+  return PMB_OK;
+}
+
+}  // namespace sc
+
+pmb_status ssd_chain_fwd(cudaStream_t st, const ChainArgs& a) {
+  const bool pairs = a.b.lo != nullptr;
+  if (!ssd_chain_shape(a.P, a.N) || a.H % a.G != 0 || (int64_t)a.B * a.H > 0x7fffffff) return fail(PMB_ERR_UNSUPPORTED, "ssd_chain: unsupported shape (P=%d N=%d)", a.P, a.N);
+  if ((a.c.lo != nullptr) != pairs || (a.x16 && pairs) || (!a.x && !a.x16)) return fail(PMB_ERR_ARG, "ssd_chain: operands must be all pairs or all plain bf16");
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  if (!al16(a.x) || !al16(a.x16) || !al16(a.y) || !al16(a.y16) || !al16(a.init) || (a.ldx & (a.x16 ? 7 : 3)) || (a.ldy & 3))
+    return fail(PMB_ERR_SHAPE, "ssd_chain: x, y and state rows must be 16-byte aligned");
+  const double tok = (double)a.B * a.T;
+  // G and the masked product over the causal half of a step, the state update and the carried-state product
+  ProfScope prof(st, "ssd_chain_fwd", tok * a.H * ((double)SCAN_STEP * (a.N + a.P) + 4.0 * a.N * a.P), 0.0);
+  const bool wide = a.N > 64;
+  if (a.blocks == 2) {
+    if (pairs || wide || a.x16 || a.T % (2 * SCAN_STEP)) return fail(PMB_ERR_UNSUPPORTED, "ssd_chain: chunks of two steps need plain bf16 operands, d_state <= 64 and whole chunks");
+    return sc::launch<1, 1, 2, false>(st, a);
+  }
+  if (a.x16) return wide ? sc::launch<1, 2, 1, true>(st, a) : sc::launch<1, 1, 1, true>(st, a);
+  if (!pairs) return wide ? sc::launch<1, 2, 1, false>(st, a) : sc::launch<1, 1, 1, false>(st, a);
+  return wide ? sc::launch<2, 2, 1, false>(st, a) : sc::launch<2, 1, 1, false>(st, a);
+}
+
+}  // namespace pmb

@@ -542,47 +542,55 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
 
 // ---- host side -------------------------------------------------------------------------------------------
 struct MapKey {
-  const void* base; int64_t d0, d1, d2, s0, s1; int b0, b1;
+  const void* base; int rank; int64_t d[4], s[3]; int b0, b1;
   bool operator==(const MapKey& o) const {
-    return base == o.base && d0 == o.d0 && d1 == o.d1 && d2 == o.d2 && s0 == o.s0 && s1 == o.s1 && b0 == o.b0 && b1 == o.b1;
+    return base == o.base && rank == o.rank && d[0] == o.d[0] && d[1] == o.d[1] && d[2] == o.d[2] && d[3] == o.d[3] && s[0] == o.s[0] && s[1] == o.s[1] &&
+           s[2] == o.s[2] && b0 == o.b0 && b1 == o.b1;
   }
 };
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
     size_t h = std::hash<const void*>()(k.base);
     auto mix = [&](int64_t v) { h ^= std::hash<int64_t>()(v) + 0x9e3779b97f4a7c15ULL + (h << 6) + (h >> 2); };
-    mix(k.d0); mix(k.d1); mix(k.d2); mix(k.s0); mix(k.s1); mix(k.b0); mix(k.b1);
+    for (int64_t v : k.d) mix(v);
+    for (int64_t v : k.s) mix(v);
+    mix(k.b0); mix(k.b1); mix(k.rank);
     return h;
   }
 };
 static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;   // shared by all devices and host threads
 static std::mutex g_maps_mu;
 
-// rank-3 bf16 map: dims (d0 contiguous, d1 rows with pitch s0 elements, d2 with pitch s1 elements), box (b0, b1, 1),
-// 128-byte swizzle
-pmb_status bf16_map3(CUtensorMap* out, const uint16_t* base, int64_t d0, int64_t d1, int64_t d2, int64_t s0, int64_t s1, int b0, int b1) {
-  MapKey key{base, d0, d1, d2, s0, s1, b0, b1};
+static pmb_status bf16_map(CUtensorMap* out, const uint16_t* base, int rank, int64_t d0, int64_t d1, int64_t d2, int64_t d3, int64_t s0, int64_t s1, int64_t s2, int b0, int b1) {
+  MapKey key{base, rank, {d0, d1, d2, d3}, {s0, s1, s2}, b0, b1};
   std::lock_guard<std::mutex> lock(g_maps_mu);
   auto it = g_maps.find(key);
   if (it == g_maps.end()) {
     if (g_maps.size() > 8192) g_maps.clear();
     EncodeTiledFn enc = get_encode();
     if (!enc) return fail(PMB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    cuuint64_t dims[3] = {(cuuint64_t)d0, (cuuint64_t)d1, (cuuint64_t)d2};
-    cuuint64_t strides[2] = {(cuuint64_t)s0 * 2, (cuuint64_t)s1 * 2};
-    cuuint32_t box[3] = {(cuuint32_t)b0, (cuuint32_t)b1, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
+    cuuint64_t dims[4] = {(cuuint64_t)d0, (cuuint64_t)d1, (cuuint64_t)d2, (cuuint64_t)d3};
+    cuuint64_t strides[3] = {(cuuint64_t)s0 * 2, (cuuint64_t)s1 * 2, (cuuint64_t)s2 * 2};
+    cuuint32_t box[4] = {(cuuint32_t)b0, (cuuint32_t)b1, 1, 1};
+    cuuint32_t estr[4] = {1, 1, 1, 1};
     CUtensorMap m;
-    CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<uint16_t*>(base), dims, strides, box, estr,
+    CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<uint16_t*>(base), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
-      return fail(PMB_ERR_CUDA, "cuTensorMapEncodeTiled (bf16, rank 3) failed with code %d (dims %lld %lld %lld, pitches %lld %lld)", (int)r,
-                  (long long)d0, (long long)d1, (long long)d2, (long long)s0, (long long)s1);
+      return fail(PMB_ERR_CUDA, "cuTensorMapEncodeTiled (bf16, rank %d) failed with code %d (dims %lld %lld %lld %lld, pitches %lld %lld %lld)", rank, (int)r,
+                  (long long)d0, (long long)d1, (long long)d2, (long long)d3, (long long)s0, (long long)s1, (long long)s2);
     it = g_maps.emplace(key, m).first;
   }
   *out = it->second;
   return PMB_OK;
+}
+// (a map's rank has to be the rank of the copies that use it)
+pmb_status bf16_map3(CUtensorMap* out, const uint16_t* base, int64_t d0, int64_t d1, int64_t d2, int64_t s0, int64_t s1, int b0, int b1) {
+  return bf16_map(out, base, 3, d0, d1, d2, 1, s0, s1, 0, b0, b1);
+}
+pmb_status bf16_map4(CUtensorMap* out, const uint16_t* base, int64_t d0, int64_t d1, int64_t d2, int64_t d3, int64_t s0, int64_t s1, int64_t s2, int b0, int b1) {
+  return bf16_map(out, base, 4, d0, d1, d2, d3, s0, s1, s2, b0, b1);
 }
 
 static unsigned int* status_ptr() {

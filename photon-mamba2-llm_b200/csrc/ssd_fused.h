@@ -27,6 +27,32 @@ struct FusedArgs {
   float* rpart;            // (B*nc*H, Q/128, Q)  r_t = sum_{s<t} W[t,s], one partial per row block of s (valid for t >= 128*block)
 };
 
+// ---- forward of the whole scan as one kernel (ssd_chain.cu), in steps of SCAN_STEP tokens
+constexpr int SCAN_STEP = 128;
+struct ChainArgs {
+  int B, T, H, P, N, G;
+  int blocks = 1;                              // steps per chunk (what S, xs and the states are relative to): 1 or 2
+  Op16 b, c;                                   // (B,T,G,N), pitch = elements between tokens, group stride N
+  const float* x; const uint16_t* x16; int64_t ldx;      // one of the two: fp32 (scaled by dt here) or bf16 (taken as x~)
+  const float* dt_raw; int64_t ld_raw; const float* dt_bias; const float* a_log;   // either these four (dt and A formed here),
+  const float* dt; const float* A;             // or dt and A,
+  const float* a;                              // or a (x~ = x)
+  const float* D;                              // skip weights or NULL (fp32 x only)
+  const float* init;                           // (B,H,N,P) or NULL
+  float* y; uint16_t* y16; int64_t ldy;        // one of the two
+  float *dt_out, *A_out, *S_out;               // optional: what the backward reads
+  uint16_t* x_keep;                            // copy of x16, (B,T,H,P)
+  uint16_t *hp_hi, *hp_lo;                     // state entering each step, (B,steps,H,N,P)
+  float* last;                                 // (B,H,N,P)
+};
+inline bool ssd_chain_shape(int P, int N) { return P > 0 && P <= 64 && P % 8 == 0 && N > 0 && N <= 128 && N % 8 == 0; }
+bool ssd_chain_enabled();      // false when PMB_SSD_FUSED=0 or PMB_SSD_ENGINE=simt
+// bf16-storage blocks: shapes whose scan reads its operands rounded to bf16 (whole chunks of 128 or 256 tokens at d_state =
+// d_head = 64); every other shape keeps (hi, lo) pairs of the fp32 values there
+bool ssd_plain16_shape(int P, int N, int Q);
+pmb_status ssd_chain_fwd(cudaStream_t st, const ChainArgs& a);
+pmb_status read_clear_device_status_chain(unsigned int* word);
+
 // Shapes the fused kernels take: block_len a multiple of 128 (at most 1024); d_state and d_head in {64, 128} with
 // plain bf16 operands, d_state = d_head = 64 with (hi, lo) pairs (what fits the shared-memory plan of both modes).
 // The other contractions below take d_head = 64 only.
@@ -52,6 +78,10 @@ pmb_status ssd_pairs_dbc(cudaStream_t st, const SsdIn& in, const SsdWs& ws, int 
 namespace sf {
 // cached rank-3 bf16 tensor map: dims (d0 contiguous, d1 rows with pitch s0 elements, d2 with pitch s1), box (b0, b1, 1)
 pmb_status bf16_map3(CUtensorMap* out, const uint16_t* base, int64_t d0, int64_t d1, int64_t d2, int64_t s0, int64_t s1, int b0, int b1);
+// cached rank-4 bf16 tensor map of a token-major operand: dims (d0 contiguous, T tokens with pitch s0, d2 heads / groups
+// with pitch s1, B sequences with pitch s2), box (b0, b1, 1, 1).  A box that reaches past the end of a sequence (or past
+// d0) is filled with zeros there, never with the next sequence's rows.
+pmb_status bf16_map4(CUtensorMap* out, const uint16_t* base, int64_t d0, int64_t T, int64_t d2, int64_t B, int64_t s0, int64_t s1, int64_t s2, int b0, int b1);
 }
 
 }  // namespace pmb

@@ -22,6 +22,7 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 }
 // Bounded wait: false when the phase did not complete within `limit` polls (SPIN_LIMIT by default).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t limit = SPIN_LIMIT) {
+#pragma unroll 1
   for (uint32_t i = 0; i < limit; ++i) {
     uint32_t ok;
     asm volatile(
@@ -40,6 +41,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
 // tensor core): sleeps between polls, so that the polling warps do not take issue slots from the single thread that
 // issues the MMAs on the same scheduler.  False when the phase did not complete within `limit` polls.
 __device__ __forceinline__ bool mbar_wait_idle(uint32_t bar, uint32_t parity, uint32_t limit = SPIN_LIMIT >> 2) {
+#pragma unroll 1
   for (uint32_t i = 0; i < limit; ++i) {
     uint32_t ok;
     asm volatile(
@@ -53,6 +55,15 @@ __device__ __forceinline__ bool mbar_wait_idle(uint32_t bar, uint32_t parity, ui
     __nanosleep(96);
   }
   return false;
+}
+
+// One lane of a converged warp.  Code that issues MMAs runs with the whole warp and guards only the issue with this: the
+// descriptors are then warp-uniform values in uniform registers, where tcgen05.mma wants them; inside `if (lane == 0)`
+// every one of them is moved there first (75 instead of about 35 clocks per 128 x 64 x 16 MMA).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
+  return ok != 0;
 }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
@@ -195,6 +206,26 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+
+// 32 lanes x 16 consecutive fp32 columns, without the wait: several loads may be in flight before tmem_wait_ld()
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// 16 lanes x 16 columns as two 16 x 8 fragments: lane l holds rows l/4 (r[0], r[1]) and l/4 + 8 (r[2], r[3]), columns
+// 2(l%4) and 2(l%4) + 1; r[4..7] the same for columns 8..15.  The lane part of the address is a multiple of 16.
+__device__ __forceinline__ void tmem_ld16x256_x2(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
