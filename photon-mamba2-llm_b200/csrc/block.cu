@@ -66,11 +66,22 @@ struct BlockWs {
   float *dnormed, *dxzd, *dact, *ddt, *dA, *scratch, *scratch2;   // scratch: conv partials; scratch2: norm partials
   size_t scratch_bytes, scratch2_bytes;
   uint16_t *normed16, *dxzd16;   // bf16 copies of the two GEMM operands (bf16-storage mode only)
+  float* slabs;                  // split-K slabs of the two weight gradients (bf16-storage mode only)
   // fp32 mode with pair GEMMs: (hi, lo) bf16 pairs of every GEMM operand
   uint16_t *x_hi, *x_lo, *dout_hi, *dout_lo, *normed_hi, *normed_lo, *dxzd_hi, *dxzd_lo, *win_hi, *win_lo, *wout_hi, *wout_lo;
 };
 
 bool block_uses_pairs(const Dims& d) { return gemm_pairs_enabled() && !(d.D % 8) && !(d.J % 8) && !(d.I % 8); }
+
+// bf16 storage: the two weight gradients share a launch with the data gradient of their projection and split K by this rule
+static int64_t tiles256(int64_t M, int64_t N) { return cdiv(M, 256) * cdiv(N, 256); }
+static int dwout_ksplit(const Dims& d) { return gemm_bf16_ksplit(d.I, d.D, d.M, tiles256(d.M, d.I), cdiv(d.D, 64)); }
+static int dwin_ksplit(const Dims& d) { return gemm_bf16_ksplit(d.D, d.J, d.M, tiles256(d.M, d.D), cdiv(d.J, 64)); }
+static size_t slab_floats(const Dims& d) {
+  const int so = dwout_ksplit(d), si = dwin_ksplit(d);
+  const size_t a = so > 1 ? (size_t)so * align_up((size_t)d.I, 256) * d.D : 0, b = si > 1 ? (size_t)si * align_up((size_t)d.D, 256) * d.J : 0;
+  return a > b ? a : b;
+}
 
 // The workspace has a forward part (everything the recompute produces and the gradient kernels read) and a
 // backward part.  With nslots == 2 the forward part exists twice, so that the recompute of the next block can run
@@ -115,6 +126,7 @@ static size_t block_ws_layout(const Dims& d, void* base, size_t bytes, BlockWs* 
   w.scratch2_bytes = gated_rmsnorm_bwd_ws_bytes(d.M, d.I);
   w.scratch2 = reinterpret_cast<float*>(ar.take<char>(w.scratch2_bytes));
   w.dxzd16 = ar.take<uint16_t>(bf16 ? mj : 0);
+  w.slabs = ar.take<float>(bf16 ? slab_floats(d) : 0);
   if (pairs) {
     w.dout_hi = ar.take<uint16_t>(md); w.dout_lo = ar.take<uint16_t>(md);
     w.dxzd_hi = ar.take<uint16_t>(mj); w.dxzd_lo = ar.take<uint16_t>(mj);
@@ -298,8 +310,13 @@ static pmb_status block_grads(cudaStream_t st, const Dims& d, const pmb_block_pa
   if (recompute_done) PMB_CUDA(cudaStreamWaitEvent(st, recompute_done, 0));
   // out_proj: dW_out = normed^T dout;  dnormed = dout W_out^T
   if (w16) {
-    PMB_TRY(gemm_bf16(st, 1, 0, d.I, d.D, d.M, w.normed16, d.I, dout, d.D, g.out_proj_weight, d.D, nullptr, 0));
-    PMB_TRY(gemm_bf16(st, 0, 1, d.M, d.I, d.D, dout, d.D, w16->out_proj, d.D, w.dnormed, d.I, nullptr, 0));
+    const int sp = (reinterpret_cast<uintptr_t>(g.out_proj_weight) & 15) ? 1 : dwout_ksplit(d);
+    const int64_t rows = (int64_t)align_up((size_t)d.I, 256);
+    const PlainGemm gw{1, 0, d.I, d.D, d.M, w.normed16, d.I, dout, d.D, sp > 1 ? w.slabs : g.out_proj_weight, d.D, nullptr, 0, sp, rows};
+    const PlainGemm gn{0, 1, d.M, d.I, d.D, dout, d.D, w16->out_proj, d.D, w.dnormed, d.I, nullptr, 0};
+    const PlainGemm both[2] = {d.M >= d.D ? gw : gn, d.M >= d.D ? gn : gw};
+    PMB_TRY(gemm_bf16_group(st, both, 2));
+    if (sp > 1) PMB_TRY(sum_slabs(st, w.slabs, sp, rows * d.D, (int64_t)d.I * d.D, g.out_proj_weight, 0));
   } else if (pr && gl) {
     PMB_TRY(order_after(st, gl->ev[2], gl->s));                 // the recomputed normed pair is ready
     PMB_TRY(gemm_pairs(gl->s, 1, 0, d.I, d.D, d.M, Pair16{w.normed_hi, w.normed_lo, d.I}, dop, g.out_proj_weight, d.D, nullptr));
@@ -359,8 +376,18 @@ static pmb_status block_grads(cudaStream_t st, const Dims& d, const pmb_block_pa
                         w.scratch, w.scratch_bytes, gl, ph, pl));
   // in_proj: dW_in = x^T dxzd;  dx = dxzd W_in^T (+ accumulated residual gradient)
   if (w16) {
-    PMB_TRY(gemm_bf16(st, 1, 0, d.D, d.J, d.M, x, d.D, w.dxzd16, d.J, g.in_proj_weight, d.J, nullptr, 0));
-    PMB_TRY(gemm_bf16(st, 0, 1, d.M, d.D, d.J, w.dxzd16, d.J, w16->in_proj, d.J, dx, d.D, dx_accum, 1));
+    const int sp = (reinterpret_cast<uintptr_t>(g.in_proj_weight) & 15) || (int64_t)d.D * d.J % 4 ? 1 : dwin_ksplit(d);
+    const int64_t rows = (int64_t)align_up((size_t)d.D, 256);
+    const PlainGemm gw{1, 0, d.D, d.J, d.M, x, d.D, w.dxzd16, d.J, sp > 1 ? w.slabs : g.in_proj_weight, d.J, nullptr, 0, sp, rows};
+    const PlainGemm gx{0, 1, d.M, d.D, d.J, w.dxzd16, d.J, w16->in_proj, d.J, dx, d.D, dx_accum, 1};
+    if (dx == x) {                       // (dW_in has to have read x before dx lands there)
+      PMB_TRY(gemm_bf16_group(st, &gw, 1));
+      PMB_TRY(gemm_bf16_group(st, &gx, 1));
+    } else {
+      const PlainGemm both[2] = {d.M >= d.J ? gw : gx, d.M >= d.J ? gx : gw};
+      PMB_TRY(gemm_bf16_group(st, both, 2));
+    }
+    if (sp > 1) PMB_TRY(sum_slabs(st, w.slabs, sp, rows * d.J, (int64_t)d.D * d.J, g.in_proj_weight, 0));
   } else if (pr) {
     // x and W_in were split by the recompute above
     const Pair16 win = (wx && wx->pairs) ? Pair16{wx->in_proj, wx->in_lo, d.J} : Pair16{w.win_hi, w.win_lo, d.J};

@@ -68,6 +68,9 @@ struct Params {
   void* C; int64_t ldc; const void* R; int out_bf16;
   int tma_out;     // fp32 result (and residual) meet the TMA rules: the epilogue stores through shared memory
   uint16_t* e_hi; uint16_t* e_lo; int64_t lde;   // optional second output: the result as a bf16 pair (TMA-store epilogue only)
+  // split K: tiles of split i cover k-tiles [i * kt_per, (i + 1) * kt_per) and go to rows i * slab_rows .. of C, whose
+  // slabs the caller adds up (kt_per covers all of K when there is one split)
+  int kt_per, slab_rows;
 };
 
 __device__ __forceinline__ float bf16_bits_to_float(uint16_t b) { return __uint_as_float((uint32_t)b << 16); }
@@ -137,9 +140,27 @@ __device__ __forceinline__ void store_row_piece(const Params& p, int m, int nb, 
 // pr[1].tiles on the second, and so on (unused entries have tiles == 0).
 // Two products whose tile counts each fill the 148 SMs badly (weight-gradient and data-gradient of one projection)
 // then share the machine instead of running as two ragged waves.
-struct Problem { CUtensorMap mA, mB, mAlo, mBlo, mC, mR; Params p; int tiles_n; int tiles; };
+struct Problem { CUtensorMap mA, mB, mAlo, mBlo, mC, mR; Params p; int tiles_n; int tiles_mn; int tiles; };
 constexpr int MAX_GROUP = 4;
-struct Group { Problem pr[MAX_GROUP]; };
+// Order of the tiles on the persistent CTA-pair kernel.  lead == 0: cluster c takes tiles c, c + clusters, ...  lead > 0 (fewer
+// than the clusters): the first `lead` tiles are the long ones (weight gradients: K is the token count) and take one cluster
+// each; meanwhile the other clusters take `rounds` of the short tiles each, and what is left goes round all of them.
+// (Round-robin alone would give the clusters with a long tile their full share of the short ones on top.)
+struct Group { Problem pr[MAX_GROUP]; int lead, rounds; };
+__device__ __forceinline__ int pair_tile_at(const Group& g, int c, int clusters, int j) {
+  if (g.lead == 0) return c + j * clusters;
+  const int f = clusters - g.lead;
+  if (c < g.lead) return j == 0 ? c : g.lead + f * g.rounds + (j - 1) * clusters + c;
+  return j < g.rounds ? g.lead + j * f + (c - g.lead) : g.lead + f * g.rounds + (j - g.rounds) * clusters + c;
+}
+// split of one tile of a problem and its k-tiles; `tile` becomes the tile's index inside the split's slab of C
+__device__ __forceinline__ int split_of(const Problem& q, int* tile, int* kt0, int* kt1) {
+  const int sp = *tile / q.tiles_mn, num_kt = (q.p.K + TBK - 1) / TBK;
+  *tile -= sp * q.tiles_mn;
+  *kt0 = sp * q.p.kt_per;
+  *kt1 = min(num_kt, *kt0 + q.p.kt_per);
+  return sp;
+}
 __device__ __forceinline__ int pick_problem(const Group& g, int id, int* local) {
   int which = 0, base = 0;
 #pragma unroll
@@ -162,7 +183,7 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 // staging slots (slot0) and TMA stores, the residual block TMA-loaded into the slot first (barriers rbar0 / rbar1);
 // everything else is stored row by row.  `st` carries the slot parity and the residual barriers' phases across tiles.
 struct EpiState { uint32_t pc = 0, rph0 = 0, rph1 = 0; };
-__device__ __forceinline__ void epilogue_rows(const Problem& q, const Params& p, uint32_t tmem_acc, int row0, int n0, int ncols, uint32_t slot0,
+__device__ __forceinline__ void epilogue_rows(const Problem& q, const Params& p, uint32_t tmem_acc, int row0, int rowoff, int n0, int ncols, uint32_t slot0,
                                               uint32_t rbar0, uint32_t rbar1, EpiState& st, int lane, volatile uint32_t* abort_flag) {
   if (p.tma_out) {
     if (row0 < p.M) {
@@ -228,7 +249,7 @@ __device__ __forceinline__ void epilogue_rows(const Problem& q, const Params& p,
         __syncwarp();
         ++st.pc;
         if (lane == 0) {
-          tma_store_2d(&q.mC, slot0 + slot * EPI_SLOT_BYTES, n0 + c0, row0);
+          tma_store_2d(&q.mC, slot0 + slot * EPI_SLOT_BYTES, n0 + c0, rowoff + row0);
           bulk_commit();
           bulk_wait_read<1>();               // the other slot's store has read its data: the slot is free again
           if (res && c0 + 32 < ncols && n0 + c0 + 32 < p.N) {
@@ -246,7 +267,7 @@ __device__ __forceinline__ void epilogue_rows(const Problem& q, const Params& p,
     for (int c0 = 0; c0 < ncols; c0 += 32) {
       uint32_t r[32];
       tmem_ld32(tmem_acc + (uint32_t)c0, r);
-      if (m < p.M) store_row_piece(p, m, n0 + c0, r);
+      if (m < p.M) store_row_piece(p, rowoff + m, n0 + c0, r);
     }
   }
 }
@@ -333,9 +354,10 @@ gemm_bf16_kernel(const __grid_constant__ Group g, const int total_tiles, unsigne
         int tile;
         const Problem& q = g.pr[pick_problem(g, tid, &tile)];
         const Params& p = q.p;
+        int kt0, kt1;
+        split_of(q, &tile, &kt0, &kt1);
         const int m0 = (tile / q.tiles_n) * TBM, n0 = (tile % q.tiles_n) * TBN;
-        const int num_kt = (p.K + TBK - 1) / TBK;
-        for (int kt = 0; kt < num_kt; ++kt) {
+        for (int kt = kt0; kt < kt1; ++kt) {
           if (!mbar_wait(empty_bar(s), ph ^ 1u)) { atomicOr(&g_bf16_status, 1u); *abort_flag = 1; stop = true; break; }
           if (*abort_flag) { stop = true; break; }
           const uint32_t a_dst = tiles + s * STAGE_BYTES, b_dst = a_dst + TILE_BYTES;
@@ -396,7 +418,8 @@ gemm_bf16_kernel(const __grid_constant__ Group g, const int total_tiles, unsigne
         int tile;
         const Problem& q = g.pr[pick_problem(g, tid, &tile)];
         const Params& p = q.p;
-        const int num_kt = (p.K + TBK - 1) / TBK;
+        int kt0, kt1;
+        split_of(q, &tile, &kt0, &kt1);
         // kind::f16 descriptor: fp32 accumulate (bit 4), A/B format bf16 (=1) at bits 7 and 10, majorness, N, M
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)p.a_mn_major << 15) | ((uint32_t)p.b_mn_major << 16) |
                                ((uint32_t)(TBN >> 3) << 17) | ((uint32_t)(TBM >> 4) << 24);
@@ -408,7 +431,7 @@ gemm_bf16_kernel(const __grid_constant__ Group g, const int total_tiles, unsigne
         if (!mbar_wait(acc_empty(b), (((uint32_t)it >> 1) & 1u) ^ 1u)) { atomicOr(&g_bf16_status, 4u); *abort_flag = 1; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t tmem_acc = tmem_base + (uint32_t)(b * TBN);
-        for (int kt = 0; kt < num_kt; ++kt) {
+        for (int kt = kt0; kt < kt1; ++kt) {
           if (!mbar_wait(full_bar(s), ph)) { atomicOr(&g_bf16_status, 2u); *abort_flag = 1; stop = true; break; }
           if (*abort_flag) { stop = true; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -416,7 +439,7 @@ gemm_bf16_kernel(const __grid_constant__ Group g, const int total_tiles, unsigne
           uint32_t al = desc_lo(a_s, a_lbo), bl = desc_lo(a_s + TILE_BYTES, b_lbo);
 #pragma unroll
           for (int k = 0; k < TBK / 16; ++k) {
-            const uint32_t acc = (kt > 0 || k > 0) ? 1u : 0u;
+            const uint32_t acc = (kt > kt0 || k > 0) ? 1u : 0u;
             if (SPLIT) {
               mma_f16_h(tmem_acc, al + LO_OFF, d_hi, bl, d_hi, idesc, acc);
               mma_f16_h(tmem_acc, al, d_hi, bl + LO_OFF, d_hi, idesc, 1u);
@@ -448,6 +471,8 @@ gemm_bf16_kernel(const __grid_constant__ Group g, const int total_tiles, unsigne
       int tile;
       const Problem& q = g.pr[pick_problem(g, tid, &tile)];
       const Params& p = q.p;
+      int kt0, kt1;
+      const int rowoff = split_of(q, &tile, &kt0, &kt1) * p.slab_rows;
       const int m0 = (tile / q.tiles_n) * TBM, n0 = (tile % q.tiles_n) * TBN;
       const int b = it & 1;
       const bool acc_ok = __all_sync(0xffffffffu, mbar_wait_idle(acc_full(b), ((uint32_t)it >> 1) & 1u));
@@ -456,7 +481,7 @@ gemm_bf16_kernel(const __grid_constant__ Group g, const int total_tiles, unsigne
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_acc = tmem_base + (uint32_t)(b * TBN) + ((uint32_t)(quarter * 32) << 16);
       const int row0 = m0 + quarter * 32;
-      epilogue_rows(q, p, tmem_acc, row0, n0, TBN, slot0, r_bar(ew, 0), r_bar(ew, 1), est, lane, abort_flag);
+      epilogue_rows(q, p, tmem_acc, row0, rowoff, n0, TBN, slot0, r_bar(ew, 0), r_bar(ew, 1), est, lane, abort_flag);
       // every TMEM read of this warp has completed (tcgen05.wait::ld): hand the accumulator back
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -739,14 +764,16 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
       int s = 0; uint32_t ph = 0;
       int in_flight = 0;
       bool stop = false;
-      for (int tid = cluster_id; tid < total_tiles && !stop; tid += nclusters) {
-        int tile;
+      for (int j = 0; !stop; ++j) {
+        const int tid = pair_tile_at(g, cluster_id, nclusters, j);
+        if (tid >= total_tiles) break;
+        int tile, kt0, kt1;
         const Problem& q = g.pr[pick_problem(g, tid, &tile)];
         const Params& p = q.p;
+        split_of(q, &tile, &kt0, &kt1);
         const int m0 = (tile / q.tiles_n) * 256 + (int)rank * TBM;
         const int nb0 = (tile % q.tiles_n) * BN2 + (int)rank * BNH;
-        const int num_kt = (p.K + TBK - 1) / TBK;
-        for (int kt = 0; kt < num_kt; ++kt) {
+        for (int kt = kt0; kt < kt1; ++kt) {
           if (!mbar_wait(empty_bar(s), ph ^ 1u)) { atomicOr(&g_bf16_status, 1u); *abort_flag = 1; stop = true; break; }
           if (*abort_flag) { stop = true; break; }
           const uint32_t a_dst = tiles + s * STAGE_BYTES, b_dst = a_dst + TILE_BYTES;
@@ -804,11 +831,13 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
       int s = 0; uint32_t ph = 0;
       int it = 0;
       bool stop = false;
-      for (int tid = cluster_id; tid < total_tiles && !stop; tid += nclusters, ++it) {
-        int tile;
+      for (; !stop; ++it) {
+        const int tid = pair_tile_at(g, cluster_id, nclusters, it);
+        if (tid >= total_tiles) break;
+        int tile, kt0, kt1;
         const Problem& q = g.pr[pick_problem(g, tid, &tile)];
         const Params& p = q.p;
-        const int num_kt = (p.K + TBK - 1) / TBK;
+        split_of(q, &tile, &kt0, &kt1);
         // M = 256 (two CTAs x 128 rows), N = BN2
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)p.a_mn_major << 15) | ((uint32_t)p.b_mn_major << 16) |
                                ((uint32_t)(BN2 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
@@ -818,7 +847,7 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
         if (!mbar_wait(acc_empty(b), (((uint32_t)it >> 1) & 1u) ^ 1u)) { atomicOr(&g_bf16_status, 4u); *abort_flag = 1; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t tmem_acc = tmem_base + (uint32_t)(b * BN2);
-        for (int kt = 0; kt < num_kt; ++kt) {
+        for (int kt = kt0; kt < kt1; ++kt) {
           if (!mbar_wait(full_bar(s), ph)) { atomicOr(&g_bf16_status, 2u); *abort_flag = 1; stop = true; break; }
           if (*abort_flag) { stop = true; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -826,7 +855,7 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
           uint32_t al = desc_lo(a_s, a_lbo), bl = desc_lo(a_s + TILE_BYTES, b_lbo);
 #pragma unroll
           for (int k = 0; k < TBK / 16; ++k) {
-            const uint32_t acc = (kt > 0 || k > 0) ? 1u : 0u;
+            const uint32_t acc = (kt > kt0 || k > 0) ? 1u : 0u;
             if (SPLIT) {
               mma_f16_pair_h(tmem_acc, al + LO_OFF, d_hi, bl, d_hi, idesc, acc);
               mma_f16_pair_h(tmem_acc, al, d_hi, bl + LO_OFF, d_hi, idesc, 1u);
@@ -851,10 +880,13 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
     EpiState est;
     const uint32_t ae[2] = {map_to_cta(acc_empty(0), 0), map_to_cta(acc_empty(1), 0)};      // the leader's barriers
     int it = 0;
-    for (int tid = cluster_id; tid < total_tiles; tid += nclusters, ++it) {
-      int tile;
+    for (;; ++it) {
+      const int tid = pair_tile_at(g, cluster_id, nclusters, it);
+      if (tid >= total_tiles) break;
+      int tile, kt0, kt1;
       const Problem& q = g.pr[pick_problem(g, tid, &tile)];
       const Params& p = q.p;
+      const int rowoff = split_of(q, &tile, &kt0, &kt1) * p.slab_rows;
       const int m0 = (tile / q.tiles_n) * 256 + (int)rank * TBM, n0 = (tile % q.tiles_n) * BN2;
       const int b = it & 1;
       const bool acc_ok = __all_sync(0xffffffffu, mbar_wait_idle(acc_full(b), ((uint32_t)it >> 1) & 1u));
@@ -863,7 +895,7 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_acc = tmem_base + (uint32_t)(b * BN2) + ((uint32_t)(quarter * 32) << 16);
       const int row0 = m0 + quarter * 32;
-      epilogue_rows(q, p, tmem_acc, row0, n0, BN2, slot0, r_bar(ew, 0), r_bar(ew, 1), est, lane, abort_flag);
+      epilogue_rows(q, p, tmem_acc, row0, rowoff, n0, BN2, slot0, r_bar(ew, 0), r_bar(ew, 1), est, lane, abort_flag);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(ae[b]);
@@ -914,11 +946,11 @@ static pmb_status make_map(CUtensorMap* map, const void* base, int64_t inner, in
 
 // Maps for the epilogue of the single-CTA kernel: 32 x 32 fp32 blocks of C (and of R, which shares C's pitch).
 // Leaves tma_out = 0 when the result is bf16 or breaks a TMA rule; the kernel then stores row by row.
-static pmb_status make_out_maps(Problem* q) {
+static pmb_status make_out_maps(Problem* q, int slabs = 1) {
   Params& p = q->p;
   p.tma_out = 0;
   if (p.out_bf16 || (p.ldc & 3) || (reinterpret_cast<uintptr_t>(p.C) & 15) || (p.R && (reinterpret_cast<uintptr_t>(p.R) & 15))) return PMB_OK;
-  PMB_TRY(make_map(&q->mC, p.C, p.N, p.M, p.ldc, 32, 32, true));
+  PMB_TRY(make_map(&q->mC, p.C, p.N, slabs > 1 ? (int64_t)slabs * p.slab_rows : p.M, p.ldc, 32, 32, true));
   if (p.R) PMB_TRY(make_map(&q->mR, p.R, p.N, p.M, p.ldc, 32, 32, true));
   p.tma_out = 1;
   return PMB_OK;
@@ -993,49 +1025,120 @@ static unsigned persistent_grid(int64_t tiles) {
 
 }  // namespace hb
 
-// Row pitches must be multiples of 8 elements (16 bytes) and the bases 16-byte aligned (TMA rules).
-pmb_status gemm_bf16(cudaStream_t st, int ta, int tb, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
-                     const void* B, int64_t ldb, void* C, int64_t ldc, const void* R, int out_bf16) {
+namespace hb {
+
+static int64_t ktiles(int64_t K) { return cdiv(K, TBK); }
+
+// Long tiles first on the pair kernel (Group): the leading problems whose tiles are at least twice as long as those of the last
+// one, when they have fewer tiles than there are clusters.
+static void set_lead(Group* g, int n, int clusters) {
+  g->lead = g->rounds = 0;
+  if (n < 2) return;
+  const Problem& last = g->pr[n - 1];
+  const int64_t b = last.p.kt_per;
+  int64_t lead = 0, a = 0;
+  for (int i = 0; i + 1 < n; ++i) { lead += g->pr[i].tiles; if (g->pr[i].p.kt_per > a) a = g->pr[i].p.kt_per; }
+  if (lead >= clusters || a < 2 * b) return;
+  g->lead = (int)lead; g->rounds = (int)(a / b);
+}
+
+}  // namespace hb
+
+// Splits of K for a product that shares a launch with `other_tiles` tiles of `other_kt` k-tiles: as many as bring its tiles down
+// to an even share of the launch's k-tiles per cluster (a weight gradient has few tiles as long as the token count: at 16384 tokens
+// 18 of them kept 18 of the 74 clusters busy four times as long as the rest of the launch needed), at most 8.
+int gemm_bf16_ksplit(int64_t M, int64_t N, int64_t K, int64_t other_tiles, int64_t other_kt) {
+  const int64_t tiles = cdiv(M, 256) * cdiv(N, 256), kt = hb::ktiles(K);
+  const int64_t share = cdiv(tiles * kt + other_tiles * other_kt, 74);
+  int64_t sp = cdiv(kt, share > 8 ? share : 8);
+  if (sp > 8) sp = 8;
+  return (int)cdiv(kt, cdiv(kt, sp));          // (no empty split)
+}
+
+// C = op(A) op(B) (+ R) on bf16 operands, up to MAX_GROUP independent products in one launch (the ones with the longest K first).
+// Row pitches must be multiples of 8 elements (16 bytes) and the bases 16-byte aligned (TMA rules).  ksplit > 1: C is fp32 and
+// receives ksplit slabs of slab_rows rows (a multiple of 256, at least M), which the caller adds up.
+pmb_status gemm_bf16_group(cudaStream_t st, const PlainGemm* gs, int n) {
   using namespace hb;
-  if (M <= 0 || N <= 0 || K <= 0) return fail(PMB_ERR_SHAPE, "gemm_bf16: non-positive dimension");
-  if ((reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15) || (lda & 7) || (ldb & 7))
-    return fail(PMB_ERR_SHAPE, "gemm_bf16: operands need 16-byte aligned bases and row pitches that are multiples of 8 elements");
-  if (cdiv(M, TBM) * cdiv(N, TBN) > 0x7fffffff) return fail(PMB_ERR_SHAPE, "gemm_bf16: too many tiles");
+  if (n < 1 || n > MAX_GROUP) return fail(PMB_ERR_ARG, "gemm_bf16_group: 1 to %d products per launch", MAX_GROUP);
   PMB_SMEM_OPT_IN(Cfg<false>::SMEM_BYTES, gemm_bf16_kernel<false>);
   Group g{};
-  Problem& q = g.pr[0];
-  if (!ta) PMB_TRY(make_map(&q.mA, A, K, M, lda, TBK, TBM)); else PMB_TRY(make_map(&q.mA, A, M, K, lda, 64, TBK));
-  if (tb) PMB_TRY(make_map(&q.mB, B, K, N, ldb, TBK, TBN)); else PMB_TRY(make_map(&q.mB, B, N, K, ldb, 64, TBK));
-  Params& p = q.p;
-  p.M = (int)M; p.N = (int)N; p.K = (int)K;
-  p.a_mn_major = ta ? 1 : 0; p.b_mn_major = tb ? 0 : 1;
-  p.C = C; p.ldc = ldc; p.R = R; p.out_bf16 = out_bf16;
-  q.tiles_n = (int)cdiv(N, TBN); q.tiles = (int)(cdiv(M, TBM) * cdiv(N, TBN));
-  PMB_TRY(make_out_maps(&q));
-  for (int i = 1; i < MAX_GROUP; ++i) { g.pr[i].tiles_n = 1; g.pr[i].tiles = 0; }
-  {
-    static const int env = [] { const char* e = getenv("PMB_GEMM_PAIR"); return e ? atoi(e) : -1; }();
-    static const int min_clusters = [] { const char* e = getenv("PMB_GEMM_PAIR_MIN"); return e ? atoi(e) : 18; }();
-    const int64_t clusters = cdiv(M, 256) * cdiv(N, 256);
-    const bool pair = env >= 0 ? env != 0 : (M > 128 && clusters >= min_clusters);
-    if (pair) {
-      // 256x256 tiles on the persistent CTA-pair kernel (see pick_pair_mode)
-      PMB_SMEM_OPT_IN((PairPCfg<false, 256>::SMEM_BYTES), gemm_bf16_pairp_kernel<false, 256>);
-      q.tiles_n = (int)cdiv(N, 256); q.tiles = (int)clusters;
-      ProfScope prof(st, "gemm_bf16", 2.0 * M * N * K, 2.0 * ((double)M * K + (double)K * N) + (out_bf16 ? 2.0 : 4.0) * M * N * (R ? 2 : 1));
-      const int64_t slots = persistent_grid(148) / 2;
-      const unsigned grid = 2u * (unsigned)(clusters < slots ? clusters : slots);
-      gemm_bf16_pairp_kernel<false, 256><<<grid, NTHREADS, PairPCfg<false, 256>::SMEM_BYTES, st>>>(g, (int)clusters);
-      PMB_LAUNCHED();
-      return PMB_OK;
-    }
+  double flops = 0.0, bytes = 0.0;
+  int64_t clusters = 0, tiles = 0;
+  bool tall = true;
+  for (int i = 0; i < n; ++i) {
+    const PlainGemm& e = gs[i];
+    if (e.M <= 0 || e.N <= 0 || e.K <= 0) return fail(PMB_ERR_SHAPE, "gemm_bf16: non-positive dimension");
+    if ((reinterpret_cast<uintptr_t>(e.A) & 15) || (reinterpret_cast<uintptr_t>(e.B) & 15) || (e.lda & 7) || (e.ldb & 7))
+      return fail(PMB_ERR_SHAPE, "gemm_bf16: operands need 16-byte aligned bases and row pitches that are multiples of 8 elements");
+    if (e.ksplit > 1 && (e.out_bf16 || e.R || e.slab_rows < e.M || e.slab_rows % 256)) return fail(PMB_ERR_ARG, "gemm_bf16: split products go to fp32 slabs");
+    Problem& q = g.pr[i];
+    if (!e.ta) PMB_TRY(make_map(&q.mA, e.A, e.K, e.M, e.lda, TBK, TBM)); else PMB_TRY(make_map(&q.mA, e.A, e.M, e.K, e.lda, 64, TBK));
+    if (e.tb) PMB_TRY(make_map(&q.mB, e.B, e.K, e.N, e.ldb, TBK, TBN)); else PMB_TRY(make_map(&q.mB, e.B, e.N, e.K, e.ldb, 64, TBK));
+    Params& p = q.p;
+    p.M = (int)e.M; p.N = (int)e.N; p.K = (int)e.K;
+    p.a_mn_major = e.ta ? 1 : 0; p.b_mn_major = e.tb ? 0 : 1;
+    p.C = e.C; p.ldc = e.ldc; p.R = e.R; p.out_bf16 = e.out_bf16;
+    const int sp = e.ksplit > 1 ? e.ksplit : 1;
+    p.kt_per = (int)cdiv(ktiles(e.K), sp); p.slab_rows = sp > 1 ? (int)e.slab_rows : 0;
+    const int splits = (int)cdiv(ktiles(e.K), p.kt_per);
+    if (splits < sp) return fail(PMB_ERR_ARG, "gemm_bf16: more splits than k-tiles");
+    PMB_TRY(make_out_maps(&q, sp));
+    clusters += cdiv(e.M, 256) * cdiv(e.N, 256) * sp;
+    tiles += cdiv(e.M, TBM) * cdiv(e.N, TBN) * sp;
+    tall = tall && e.M > 128;
+    flops += 2.0 * e.M * e.N * e.K;
+    bytes += 2.0 * ((double)e.M * e.K + (double)e.K * e.N) + (e.out_bf16 ? 2.0 : 4.0) * e.M * e.N * (e.R ? 2 : 1);
   }
-  ProfScope prof(st, "gemm_bf16", 2.0 * M * N * K, 2.0 * ((double)M * K + (double)K * N) + (out_bf16 ? 2.0 : 4.0) * M * N * (R ? 2 : 1));
-  {
+  if (tiles > 0x7fffffff) return fail(PMB_ERR_SHAPE, "gemm_bf16: too many tiles");
+  static const int env = [] { const char* e = getenv("PMB_GEMM_PAIR"); return e ? atoi(e) : -1; }();
+  static const int min_clusters = [] { const char* e = getenv("PMB_GEMM_PAIR_MIN"); return e ? atoi(e) : 18; }();
+  const bool pair = env >= 0 ? env != 0 : (tall && clusters >= min_clusters);      // see pick_pair_mode
+  for (int i = 0; i < n; ++i) {
+    Problem& q = g.pr[i];
+    const int64_t tm = pair ? cdiv(gs[i].M, 256) : cdiv(gs[i].M, TBM), tn = pair ? cdiv(gs[i].N, 256) : cdiv(gs[i].N, TBN);
+    q.tiles_n = (int)tn; q.tiles_mn = (int)(tm * tn); q.tiles = q.tiles_mn * (gs[i].ksplit > 1 ? gs[i].ksplit : 1);
+  }
+  for (int i = n; i < MAX_GROUP; ++i) { g.pr[i].tiles_n = g.pr[i].tiles_mn = 1; g.pr[i].tiles = 0; }
+  ProfScope prof(st, "gemm_bf16", flops, bytes);
+  if (pair) {
+    PMB_SMEM_OPT_IN((PairPCfg<false, 256>::SMEM_BYTES), gemm_bf16_pairp_kernel<false, 256>);
+    const int64_t slots = persistent_grid(148) / 2;
+    const unsigned grid = 2u * (unsigned)(clusters < slots ? clusters : slots);
+    set_lead(&g, n, (int)(grid / 2));
+    gemm_bf16_pairp_kernel<false, 256><<<grid, NTHREADS, PairPCfg<false, 256>::SMEM_BYTES, st>>>(g, (int)clusters);
+  } else {
     unsigned long long t0 = 0;
-    unsigned long long* sc = sched_counter(st, q.tiles, &t0);
-    gemm_bf16_kernel<false><<<persistent_grid(q.tiles), NTHREADS, Cfg<false>::SMEM_BYTES, st>>>(g, q.tiles, sc, t0);
+    unsigned long long* sc = sched_counter(st, tiles, &t0);
+    gemm_bf16_kernel<false><<<persistent_grid(tiles), NTHREADS, Cfg<false>::SMEM_BYTES, st>>>(g, (int)tiles, sc, t0);
   }
+  PMB_LAUNCHED();
+  return PMB_OK;
+}
+
+pmb_status gemm_bf16(cudaStream_t st, int ta, int tb, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
+                     const void* B, int64_t ldb, void* C, int64_t ldc, const void* R, int out_bf16) {
+  const PlainGemm e{ta, tb, M, N, K, A, lda, B, ldb, C, ldc, R, out_bf16};
+  return gemm_bf16_group(st, &e, 1);
+}
+
+// out = sum of n slabs, fixed order; `pitch` elements apart, `elems` each; out fp32 or bf16
+__global__ void __launch_bounds__(256) sum_slabs_kernel(const float* __restrict__ part, int n, int64_t pitch, int64_t elems, void* __restrict__ out, int out_bf16) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (i >= elems) return;
+  float4 a = *reinterpret_cast<const float4*>(part + i);
+#pragma unroll 4
+  for (int s = 1; s < n; ++s) {
+    const float4 b = *reinterpret_cast<const float4*>(part + (int64_t)s * pitch + i);
+    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+  }
+  if (out_bf16) store_pair4(static_cast<uint16_t*>(out) + i, nullptr, a.x, a.y, a.z, a.w);
+  else *reinterpret_cast<float4*>(static_cast<float*>(out) + i) = a;
+}
+pmb_status sum_slabs(cudaStream_t st, const float* part, int n, int64_t pitch, int64_t elems, void* out, int out_bf16) {
+  if (elems & 3) return fail(PMB_ERR_SHAPE, "sum_slabs: the element count must be a multiple of 4");
+  ProfScope prof(st, "splitk_sum", 0.0, (4.0 * n + (out_bf16 ? 2.0 : 4.0)) * elems);
+  sum_slabs_kernel<<<(unsigned)cdiv(elems / 4, 256), 256, 0, st>>>(part, n, pitch, elems, out, out_bf16);
   PMB_LAUNCHED();
   return PMB_OK;
 }
@@ -1120,7 +1223,7 @@ static int pick_pair_mode(const PairGemm* gs, int n, int tile_mode) {
   static const int half_wave = [] { const char* e = getenv("PMB_GEMM_PAIR_MIN"); return e ? atoi(e) : 18; }();
   for (int i = 0; i < n; ++i) {
     if (gs[i].M <= 128) return 0;        // a pair tile would be half empty
-    if (cdiv(gs[i].M, 256) * cdiv(gs[i].N, 256) < half_wave) return 0;
+    if (cdiv(gs[i].M, 256) * cdiv(gs[i].N, 256) * (gs[i].ksplit > 1 ? gs[i].ksplit : 1) < half_wave) return 0;
   }
   return 4;
 }
@@ -1134,7 +1237,7 @@ pmb_status gemm_pairs_group(cudaStream_t st, const PairGemm* gs, int n, int tile
   if (n < 1 || n > MAX_GROUP) return fail(PMB_ERR_ARG, "gemm_pairs_group: 1 to %d products per launch", MAX_GROUP);
   PMB_SMEM_OPT_IN(Cfg<true>::SMEM_BYTES, gemm_bf16_kernel<true>);
   Group g{};
-  for (int i = 1; i < MAX_GROUP; ++i) { g.pr[i].tiles_n = 1; g.pr[i].tiles = 0; }
+  for (int i = 1; i < MAX_GROUP; ++i) { g.pr[i].tiles_n = g.pr[i].tiles_mn = 1; g.pr[i].tiles = 0; }
   double flops = 0.0, bytes = 0.0;
   int64_t total = 0;
   for (int i = 0; i < n; ++i) {
@@ -1153,12 +1256,17 @@ pmb_status gemm_pairs_group(cudaStream_t st, const PairGemm* gs, int n, int tile
     p.M = (int)M; p.N = (int)N; p.K = (int)K;
     p.a_mn_major = e.ta ? 1 : 0; p.b_mn_major = e.tb ? 0 : 1;
     p.C = e.C; p.ldc = e.ldc; p.R = e.R; p.out_bf16 = 0;
-    PMB_TRY(make_out_maps(&q));
+    const int sp = e.ksplit > 1 ? e.ksplit : 1;
+    if (sp > 1 && (e.R || e.emit.hi || e.slab_rows < M || e.slab_rows % 256)) return fail(PMB_ERR_ARG, "gemm_pairs: split products go to fp32 slabs");
+    p.kt_per = (int)cdiv(ktiles(K), sp); p.slab_rows = sp > 1 ? (int)e.slab_rows : 0;
+    if (cdiv(ktiles(K), p.kt_per) < sp) return fail(PMB_ERR_ARG, "gemm_pairs: more splits than k-tiles");
+    PMB_TRY(make_out_maps(&q, sp));
     p.e_hi = const_cast<uint16_t*>(e.emit.hi); p.e_lo = const_cast<uint16_t*>(e.emit.lo); p.lde = e.emit.ld;   // (Pair16 is declared for reading; this one is written)
     if (p.e_hi && (!p.tma_out || !p.e_lo || (p.lde & 7) || ((reinterpret_cast<uintptr_t>(p.e_hi) | reinterpret_cast<uintptr_t>(p.e_lo)) & 15)))
       return fail(PMB_ERR_UNSUPPORTED, "gemm_pairs: the pair output needs the TMA-store epilogue, 16-byte aligned arrays and a pitch that is a multiple of 8");
     q.tiles_n = (int)cdiv(N, TBN);
-    const int64_t t = cdiv(M, TBM) * cdiv(N, TBN);
+    q.tiles_mn = (int)(cdiv(M, TBM) * cdiv(N, TBN));
+    const int64_t t = (int64_t)q.tiles_mn * sp;
     total += t;
     if (total > 0x7fffffff) return fail(PMB_ERR_UNSUPPORTED, "gemm_pairs: too many tiles");
     q.tiles = (int)t;
@@ -1166,7 +1274,7 @@ pmb_status gemm_pairs_group(cudaStream_t st, const PairGemm* gs, int n, int tile
     bytes += 4.0 * ((double)M * K + (double)K * N + (double)M * N * (e.R ? 2 : 1));
   }
   int pair_mode = pick_pair_mode(gs, n, tile_mode);
-  for (int i = 0; i < n; ++i) if (gs[i].emit.hi && pair_mode <= 2) pair_mode = 0;      // (the one-tile-per-cluster kernels do not write the pair output)
+  for (int i = 0; i < n; ++i) if ((gs[i].emit.hi || gs[i].ksplit > 1) && pair_mode <= 2) pair_mode = 0;      // (the one-tile-per-cluster kernels do not write the pair output)
   if (pair_mode) {
     const int bn2 = (pair_mode == 2 || pair_mode == 4) ? 256 : 128;
     PMB_SMEM_OPT_IN((PairCfg<true, 256>::SMEM_BYTES), gemm_bf16_pair_kernel<true, 256>);
@@ -1178,13 +1286,15 @@ pmb_status gemm_pairs_group(cudaStream_t st, const PairGemm* gs, int n, int tile
       // B boxes of the pair kernel are BN2/2 rows tall (K-major tiles); MN-major boxes stay 64 columns wide
       if (e.tb) { PMB_TRY(make_map(&q.mB, e.B.hi, e.K, e.N, e.B.ld, TBK, bn2 / 2)); PMB_TRY(make_map(&q.mBlo, e.B.lo, e.K, e.N, e.B.ld, TBK, bn2 / 2)); }
       q.tiles_n = (int)cdiv(e.N, bn2);
-      q.tiles = (int)(cdiv(e.M, 256) * cdiv(e.N, bn2));
+      q.tiles_mn = (int)(cdiv(e.M, 256) * cdiv(e.N, bn2));
+      q.tiles = q.tiles_mn * (e.ksplit > 1 ? e.ksplit : 1);
       clusters += q.tiles;
     }
     if (pair_mode >= 3) {
       ProfScope prof(st, "gemm_bf16x2", flops, bytes);
       const int64_t slots = persistent_grid(148) / 2;
       const unsigned grid = 2u * (unsigned)(clusters < slots ? clusters : slots);
+      set_lead(&g, n, (int)(grid / 2));
       if (pair_mode == 4) {
         PMB_SMEM_OPT_IN((PairPCfg<true, 256>::SMEM_BYTES), gemm_bf16_pairp_kernel<true, 256>);
         gemm_bf16_pairp_kernel<true, 256><<<grid, NTHREADS, PairPCfg<true, 256>::SMEM_BYTES, st>>>(g, (int)clusters);

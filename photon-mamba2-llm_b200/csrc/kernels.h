@@ -141,6 +141,13 @@ pmb_status read_clear_device_status(unsigned int* word);
 // ---- gemm_bf16.cu: bf16 operands, fp32 accumulation; C and R are fp32 or bf16 (out_bf16)
 pmb_status gemm_bf16(cudaStream_t st, int ta, int tb, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
                      const void* B, int64_t ldb, void* C, int64_t ldc, const void* R, int out_bf16);
+// One product of a launch.  ksplit > 1: K is cut into ksplit parts whose fp32 results go to slabs of slab_rows rows of C
+// (slab_rows a multiple of 256, at least M; ldc as given); sum_slabs adds them up in a fixed order.
+struct PlainGemm { int ta, tb; int64_t M, N, K; const void* A; int64_t lda; const void* B; int64_t ldb; void* C; int64_t ldc; const void* R; int out_bf16;
+                   int ksplit = 1; int64_t slab_rows = 0; };
+pmb_status gemm_bf16_group(cudaStream_t st, const PlainGemm* g, int n);      // the ones with the longest K first
+int gemm_bf16_ksplit(int64_t M, int64_t N, int64_t K, int64_t other_tiles, int64_t other_kt);
+pmb_status sum_slabs(cudaStream_t st, const float* part, int n, int64_t pitch, int64_t elems, void* out, int out_bf16);
 pmb_status read_clear_device_status_bf16(unsigned int* word);
 // fp32 matrices as (hi, lo) bf16 pairs: hi = bf16(a), lo = bf16(a - hi); ld = row pitch in elements (multiple of 8)
 struct Pair16 { const uint16_t* hi; const uint16_t* lo; int64_t ld; };
@@ -154,7 +161,8 @@ pmb_status gemm_pairs(cudaStream_t st, int ta, int tb, int64_t M, int64_t N, int
                       float* C, int64_t ldc, const float* R, int tile_mode = -1);
 // `emit` (optional): the result is also written as a bf16 pair with row pitch emit.ld, for the product that reads it
 // next as an operand (needs the TMA-store epilogue: C 16-byte aligned, ldc a multiple of 4; otherwise the call fails)
-struct PairGemm { int ta, tb; int64_t M, N, K; Pair16 A, B; float* C; int64_t ldc; const float* R; Pair16 emit = Pair16{nullptr, nullptr, 0}; };
+struct PairGemm { int ta, tb; int64_t M, N, K; Pair16 A, B; float* C; int64_t ldc; const float* R; Pair16 emit = Pair16{nullptr, nullptr, 0};
+                  int ksplit = 1; int64_t slab_rows = 0; };      // (split K as in PlainGemm)
 // up to four independent products in one launch (tiles of g[0] first: give it the longer K)
 pmb_status gemm_pairs_group(cudaStream_t st, const PairGemm* g, int n, int tile_mode = -1);
 bool gemm_pairs_enabled();   // false when PMB_GEMM_ENGINE is tf32 or simt

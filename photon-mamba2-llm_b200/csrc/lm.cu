@@ -17,7 +17,17 @@ namespace pmb {
 // Row tile of the tied head: (rows, vocab) fp32 logits exist for one tile at a time.  1024 rows (206 MB at a 50k
 // vocabulary) cost 1.7 % of the headline step against 2048 (412 MB); PMB_LM_TILE_ROWS overrides it (>= 128).
 constexpr int LM_TILE_ROWS = 1024;
-constexpr int HEAD_SPLITK = 3;
+// fp32 storage: dhidden = dlogits E has few tiles (12 clusters of 256 x 256 for a full row tile at d_model 768) and K = vocab:
+// split K so that the product the whole backward waits for fills the machine once (one launch, fp32 slabs, then a sum).
+// (bf16 storage does not split here: the sums' rounding would flip bf16 roundings of the gradient stream that 24 blocks
+// amplify to the size of the storage's own error.  There dhidden shares a launch with the table gradient: 360 + 75 us -> 230.)
+static int head_ksplit(int64_t rows, int D, int V) {
+  const int64_t tiles = cdiv(rows, 256) * cdiv(D, 256), kt = cdiv(V, 64);
+  int64_t sp = 74 / tiles;
+  if (sp > 8) sp = 8;
+  if (sp > kt / 8) sp = kt / 8;
+  return sp < 2 ? 1 : (int)cdiv(kt, cdiv(kt, sp));
+}
 
 __global__ void embedding_fwd_kernel(const float* __restrict__ table, const int64_t* __restrict__ ids, float* __restrict__ out,
                                      int64_t rows, int D, int V, unsigned int* __restrict__ bad) {
@@ -231,18 +241,6 @@ __global__ void hier_kernel(const T* __restrict__ in, const T* __restrict__ a, T
   st_act(out + i, v);
 }
 
-// out = sum of n slabs of `elems` floats (split-K partial products), float4 lanes
-__global__ void sum_slabs_kernel(const float* __restrict__ part, int n, int64_t elems, float* __restrict__ out) {
-  int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
-  if (i >= elems) return;
-  float4 a = *reinterpret_cast<const float4*>(part + i);
-  for (int s = 1; s < n; ++s) {
-    const float4 b = *reinterpret_cast<const float4*>(part + (int64_t)s * elems + i);
-    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-  }
-  *reinterpret_cast<float4*>(out + i) = a;
-}
-
 __global__ void __launch_bounds__(256) mean_kernel(const float* __restrict__ v, int64_t n, float* __restrict__ out) {
   __shared__ float red[32];
   float s = 0.0f;
@@ -281,7 +279,7 @@ struct pmb_lm {
   int pairs = 0;
   int ce_inplace = 0;         // the logits row fits in shared memory: the gradient pair overwrites the logits tile
   uint16_t *params_hi = nullptr, *params_lo = nullptr, *dlog_hi = nullptr, *dlog_lo = nullptr, *hid_hi = nullptr, *hid_lo = nullptr;
-  float* dh_part = nullptr;   // HEAD_SPLITK partial products of dhidden = dlogits E (few tiles, very long K)
+  float* dh_part = nullptr;   // split-K slabs of dhidden = dlogits E (few tiles, very long K)
   uint16_t* l1_pair = nullptr; // two-level fp32 model: (hi, lo) pairs of `pooled` and `dh1`, 4 x (M/group, D) bf16
   std::vector<Weights16> lw16;
   // hierarchical variant (L1 > 0): level 0 = layers [0,L0) at token rate, level 1 = layers [L0,L0+L1) at 1/group rate
@@ -372,8 +370,18 @@ static pmb_status lm_create_impl(const pmb_mamba2_config* cfg, int L0, int L1, i
     lm->ce_inplace = ((size_t)vocab * 4 <= (size_t)CE_MAX_SMEM) ? 1 : 0;
     if (!lm->ce_inplace) ok = ok && alloc((void**)&lm->dlog_hi, tv) && alloc((void**)&lm->dlog_lo, tv);
     ok = ok && alloc((void**)&lm->hid_hi, td) && alloc((void**)&lm->hid_lo, td);
-    ok = ok && alloc((void**)&lm->dh_part, (size_t)HEAD_SPLITK * lm->tile_rows * d.D * 4);
-    pair_bytes = (lm->ce_inplace ? 0 : 2 * tv) + 2 * td + (size_t)HEAD_SPLITK * lm->tile_rows * d.D * 4;
+    pair_bytes = (lm->ce_inplace ? 0 : 2 * tv) + 2 * td;
+  }
+  if (lm->pairs) {
+    // (the last row tile may be shorter and split further: at most eight slabs)
+    size_t need = 0;
+    for (int64_t rows : {(int64_t)lm->tile_rows, d.M % lm->tile_rows}) {
+      const int sp = rows > 0 ? head_ksplit(rows, d.D, vocab) : 1;
+      const size_t b = sp > 1 ? (size_t)sp * align_up((size_t)rows, 256) * d.D * 4 : 0;
+      if (b > need) need = b;
+    }
+    ok = ok && alloc((void**)&lm->dh_part, need ? need : 256);
+    pair_bytes += need;
   }
   if (lm->bf16) {
     ok = ok && alloc((void**)&lm->params16, (size_t)o * 2);
@@ -583,29 +591,21 @@ extern "C" pmb_status pmb_lm_step_device(pmb_lm* lm, void* stream, const int64_t
       const uint16_t* dl16 = lm->ce_inplace ? reinterpret_cast<const uint16_t*>(lm->logits) : lm->dlogits16;
       const int64_t ldl = lm->ce_inplace ? 2 * (int64_t)Vp : Vp;
       if (!lm->ce_inplace) PMB_TRY(cast_f32_bf16(st, lm->logits, lm->dlogits16, rows * Vp));
-      PMB_TRY(gemm_bf16(st, 0, 0, rows, D, V, dl16, ldl, table16, D, dhid + (size_t)r0 * D * 2, D, nullptr, 1));
-      PMB_TRY(gemm_bf16(st, 1, 0, V, D, rows, dl16, ldl, hrows, D, dtable, D, r0 == 0 ? nullptr : dtable, 0));
+      // one launch: the few long tiles of dhidden take a cluster each, the many short ones of dE the others
+      const PlainGemm both[2] = {{0, 0, rows, D, V, dl16, ldl, table16, D, dhid + (size_t)r0 * D * 2, D, nullptr, 1},
+                                 {1, 0, V, D, rows, dl16, ldl, hrows, D, dtable, D, r0 == 0 ? nullptr : dtable, 0}};
+      PMB_TRY(gemm_bf16_group(st, both, 2));
     } else if (prs && table_lane) {
       // only dhidden is needed now; the embedding-table gradient runs on its own stream (next to the first blocks of
       // the stack backward for the last row tile) and is joined before the embedding scatter.  With several row tiles
       // the next tile's logits overwrite the buffer this tile's dE still reads, so the caller's stream waits for the
       // lane before each further tile (below).
-      // dhidden has 16 x 6 tiles and K = vocab: split K three ways (one launch, three products into three slabs)
-      // so that the product the whole backward waits for uses the machine, then add the slabs
-      {
-        PairGemm parts[HEAD_SPLITK];
-        const int64_t kstep = (int64_t)align_up((size_t)cdiv(V, HEAD_SPLITK), 64);
-        int np = 0;
-        for (int64_t k0 = 0; k0 < V && np < HEAD_SPLITK; k0 += kstep, ++np) {
-          const int64_t kk = V - k0 < kstep ? V - k0 : kstep;
-          parts[np] = PairGemm{0, 0, rows, D, kk, Pair16{dlog_p.hi + k0, dlog_p.lo + k0, dlog_p.ld},
-                               Pair16{table_p.hi + k0 * D, table_p.lo + k0 * D, table_p.ld}, lm->dh_part + (size_t)np * rows * D, D, nullptr};
-        }
-        PMB_TRY(gemm_pairs_group(st, parts, np));
-        ProfScope prof(st, "head_splitk_sum", 0.0, 4.0 * (np + 1) * rows * D);
-        sum_slabs_kernel<<<(unsigned)cdiv(rows * D / 4, 256), 256, 0, st>>>(lm->dh_part, np, rows * D, lm->dhidden + r0 * D);
-        PMB_LAUNCHED();
-      }
+      const int sp = head_ksplit(rows, D, V);
+      const int64_t srows = (int64_t)align_up((size_t)rows, 256);
+      PairGemm e{0, 0, rows, D, V, dlog_p, table_p, sp > 1 ? lm->dh_part : lm->dhidden + r0 * D, D, nullptr};
+      e.ksplit = sp; e.slab_rows = srows;
+      PMB_TRY(gemm_pairs_group(st, &e, 1));
+      if (sp > 1) PMB_TRY(sum_slabs(st, lm->dh_part, sp, srows * D, rows * D, lm->dhidden + r0 * D, 0));
       PMB_TRY(order_after(st, table_lane->ev[0], table_lane->s));
       PMB_TRY(gemm_pairs(table_lane->s, 1, 0, V, D, rows, dlog_p, hid_p, dtable, D, r0 == 0 ? nullptr : dtable));
       if (r0 + rows < M) PMB_TRY(order_after(table_lane->s, table_lane->ev[2], st));   // the tile buffers are reused next

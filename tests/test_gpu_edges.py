@@ -54,3 +54,20 @@ def test_block_forward_lengths(pm, B, T, P, N, G):
     torch.cuda.synchronize()
     assert pm.device_status() == 0
     assert_close(out, orc.block_forward(p, cfg, x), what=f"B={B} T={T} P={P} N={N} G={G}")
+
+
+# token counts at which the weight gradients of the bf16-storage block split K or not, with and without whole tiles
+@pytest.mark.parametrize("B,T", [(1, 40), (1, 1100), (3, 1024)])
+def test_block_bf16_weight_gradient_splits(pm, B, T):
+    D, H, P, N = 128, 8, 32, 16
+    cfg, p, blk = _block(pm, D, H, P, N, 1, 64, torch.bfloat16)
+    x, cot = randn((B, T, D), 5).bfloat16(), randn((B, T, D), 6).bfloat16()
+    dx, grads = blk.backward(x.cuda(), cot.cuda())
+    torch.cuda.synchronize()
+    assert pm.device_status() == 0
+    leaves = {k: v.clone().requires_grad_(True) for k, v in p.items()}
+    xr = x.float().requires_grad_(True)
+    orc.block_forward(leaves, cfg, xr).backward(cot.float())
+    assert_close(dx.float(), xr.grad, tol=3e-2, what="dx")
+    for k in ("in_proj_weight", "out_proj_weight"):
+        assert_close(grads[k], leaves[k].grad, tol=2e-2, what=k)
