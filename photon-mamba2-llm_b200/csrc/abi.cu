@@ -143,6 +143,8 @@ extern "C" pmb_status pmb_device_status(int32_t* h_word_out) {
   w |= (w2 & 0x7fu) << 8;
   PMB_TRY(read_clear_device_status_chain(&w2));
   w |= ((w2 | (w2 >> 7)) & 0x7fu) << 8;
+  PMB_TRY(read_clear_device_status_decode(&w2));
+  w |= (w2 & 0xffu) << 24;
   if (h_word_out) *h_word_out = (int32_t)w;
   return PMB_OK;
 }

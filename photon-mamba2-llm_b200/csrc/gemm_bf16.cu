@@ -944,6 +944,11 @@ static pmb_status make_map(CUtensorMap* map, const void* base, int64_t inner, in
   return PMB_OK;
 }
 
+// bf16 operand map for other translation units (128-byte swizzle)
+pmb_status pair_operand_map(CUtensorMap* map, const uint16_t* base, int64_t inner, int64_t outer, int64_t ld, int box_inner, int box_outer) {
+  return make_map(map, base, inner, outer, ld, box_inner, box_outer);
+}
+
 // Maps for the epilogue of the single-CTA kernel: 32 x 32 fp32 blocks of C (and of R, which shares C's pitch).
 // Leaves tma_out = 0 when the result is bf16 or breaks a TMA rule; the kernel then stores row by row.
 static pmb_status make_out_maps(Problem* q, int slabs = 1) {

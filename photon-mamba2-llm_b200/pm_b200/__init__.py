@@ -144,7 +144,9 @@ def _check(status: int):
 
 
 def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """Raw handle of the current stream.  (The Stream object of torch.cuda.current_stream() costs more host time than the
+    launch of a small kernel.)"""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _ptr(t):
@@ -516,6 +518,9 @@ class Mamba2Block:
             raise PmbError(2, f"compute dtype {compute_dtype} is not supported")
         self.bf16 = compute_dtype == torch.bfloat16
         self._ws = None
+        self._cfg = C.byref(config.c())
+        self._params_c, self._params_key = None, None
+        self._step_ws = {}
         self.refresh_weights()
 
     def refresh_weights(self):
@@ -523,6 +528,14 @@ class Mamba2Block:
         if self.bf16:
             self.w_in16 = to_bf16(self.params["in_proj_weight"])
             self.w_out16 = to_bf16(self.params["out_proj_weight"])
+
+    def _params_struct(self):
+        """The C view of the parameters, rebuilt when one of the tensors was replaced."""
+        p = self.params
+        key = [p[k].data_ptr() for k in PARAM_ORDER]
+        if key != self._params_key:
+            self._params_c, self._params_key = _params_struct(p), key
+        return C.byref(self._params_c)
 
     def _io(self, t, name):
         want = torch.bfloat16 if self.bf16 else torch.float32
@@ -532,7 +545,7 @@ class Mamba2Block:
 
     def _workspace(self, B, T, device):
         fn = lib.pmb_mamba2_block_workspace_bytes_bf16 if self.bf16 else lib.pmb_mamba2_block_workspace_bytes
-        n = fn(C.byref(self.config.c()), B, T)
+        n = fn(self._cfg, B, T)
         if n == 0:
             raise PmbError(1, lib.pmb_last_error().decode())
         if self._ws is None or self._ws.numel() < n:
@@ -543,14 +556,14 @@ class Mamba2Block:
         B, T, D = x.shape
         ws = self._workspace(B, T, x.device)
         out = torch.empty_like(x)
-        ps = _params_struct(self.params)
+        ps = self._params_struct()
         self._io(x, "x")
         if self.bf16:
-            _check(lib.pmb_mamba2_block_fwd_bf16(_stream(), C.byref(self.config.c()), C.byref(ps), self.w_in16.data_ptr(),
+            _check(lib.pmb_mamba2_block_fwd_bf16(_stream(), self._cfg, ps, self.w_in16.data_ptr(),
                                                  self.w_out16.data_ptr(), B, T, x.data_ptr(), _ptr(residual), out.data_ptr(),
                                                  ws.data_ptr(), ws.numel()))
         else:
-            _check(lib.pmb_mamba2_block_fwd(_stream(), C.byref(self.config.c()), C.byref(ps), B, T, x.data_ptr(),
+            _check(lib.pmb_mamba2_block_fwd(_stream(), self._cfg, ps, B, T, x.data_ptr(),
                                             _ptr(residual), out.data_ptr(), ws.data_ptr(), ws.numel()))
         return out
 
@@ -560,14 +573,14 @@ class Mamba2Block:
         ws = self._workspace(B, T, x.device)
         dx = torch.empty_like(x)
         grads = {k: torch.empty_like(v) for k, v in self.params.items()}
-        ps, gs = _params_struct(self.params), _params_struct(grads)
+        ps, gs = self._params_struct(), _params_struct(grads)
         self._io(x, "x"); self._io(dout, "dout")
         if self.bf16:
-            _check(lib.pmb_mamba2_block_bwd_bf16(_stream(), C.byref(self.config.c()), C.byref(ps), self.w_in16.data_ptr(),
+            _check(lib.pmb_mamba2_block_bwd_bf16(_stream(), self._cfg, ps, self.w_in16.data_ptr(),
                                                  self.w_out16.data_ptr(), B, T, x.data_ptr(), dout.data_ptr(), _ptr(dx_accum),
                                                  dx.data_ptr(), C.byref(gs), ws.data_ptr(), ws.numel()))
         else:
-            _check(lib.pmb_mamba2_block_bwd(_stream(), C.byref(self.config.c()), C.byref(ps), B, T, x.data_ptr(),
+            _check(lib.pmb_mamba2_block_bwd(_stream(), self._cfg, ps, B, T, x.data_ptr(),
                                             dout.data_ptr(), _ptr(dx_accum), dx.data_ptr(), C.byref(gs),
                                             ws.data_ptr(), ws.numel()))
         return dx, grads
@@ -580,13 +593,17 @@ class Mamba2Block:
     def step(self, x_t, state):
         """`Mamba2Block::step`: x_t (B,1,D); the state dict is updated in place and returned."""
         B = x_t.shape[0]
-        n = lib.pmb_mamba2_step_workspace_bytes(C.byref(self.config.c()), B)
-        ws = torch.empty(n, device=x_t.device, dtype=torch.uint8)
+        stream = _stream()
+        ws = self._step_ws.get((stream, B))          # one workspace per stream: steps on several streams may overlap
+        if ws is None:
+            n = lib.pmb_mamba2_step_workspace_bytes(self._cfg, B)
+            if len(self._step_ws) >= 8:
+                self._step_ws.clear()
+            ws = self._step_ws[(stream, B)] = torch.empty(n, device=x_t.device, dtype=torch.uint8)
         y = torch.empty_like(x_t)
-        ps = _params_struct(self.params)
-        _check(lib.pmb_mamba2_step(_stream(), C.byref(self.config.c()), C.byref(ps), B, _dev(x_t, "x_t").data_ptr(),
+        _check(lib.pmb_mamba2_step(stream, self._cfg, self._params_struct(), B, _dev(x_t, "x_t").data_ptr(),
                                    state["ssm_state"].data_ptr(), state["conv_window"].data_ptr(), y.data_ptr(),
-                                   ws.data_ptr(), n))
+                                   ws.data_ptr(), ws.numel()))
         return y, state
 
 

@@ -71,3 +71,22 @@ def test_block_bf16_weight_gradient_splits(pm, B, T):
     assert_close(dx.float(), xr.grad, tol=3e-2, what="dx")
     for k in ("in_proj_weight", "out_proj_weight"):
         assert_close(grads[k], leaves[k].grad, tol=2e-2, what=k)
+
+
+# batch sizes around the switch from streamed FMA to tensor-core projections and its tile widths; widths with ragged column
+# tiles; the last two are served by the general kernels
+@pytest.mark.parametrize("B", [1, 2, 3, 5, 9, 16, 17, 33, 70, 130, 300])
+@pytest.mark.parametrize("D,H,P,N,G", [(64, 4, 32, 16, 1), (72, 6, 24, 40, 6), (200, 8, 64, 128, 1), (36, 3, 5, 7, 1)])
+def test_decode_batches(pm, B, D, H, P, N, G):
+    cfg, p, blk = _block(pm, D, H, P, N, G, 64, torch.float32)
+    st = blk.zero_state(B)
+    ref = {"ssm_state": randn((B, H, N, P), 7, 0.3), "conv_window": randn((B, cfg.xbc_dim, 3), 8, 0.5)}
+    st["ssm_state"].copy_(ref["ssm_state"]); st["conv_window"].copy_(ref["conv_window"])
+    for step in range(2):
+        x = randn((B, 1, D), 20 + step)
+        y, st = blk.step(x.cuda(), st)
+        y_ref, ref = orc.block_step(p, cfg, x, ref)
+        assert_close(y, y_ref, what=f"y step {step}")
+        assert_close(st["ssm_state"], ref["ssm_state"], what="state")
+        assert_close(st["conv_window"], ref["conv_window"], what="window")
+    assert pm.device_status() == 0
