@@ -143,6 +143,10 @@ extern "C" pmb_status pmb_device_status(int32_t* h_word_out) {
   w |= (w2 & 0x7fu) << 8;
   PMB_TRY(read_clear_device_status_chain(&w2));
   w |= ((w2 | (w2 >> 7)) & 0x7fu) << 8;
+  PMB_TRY(read_clear_device_status_chain_bwd(&w2));
+  w |= ((w2 | (w2 >> 7)) & 0x7fu) << 8;
+  PMB_TRY(read_clear_device_status_heads(&w2));
+  w |= ((w2 | (w2 >> 7)) & 0x7fu) << 8;
   PMB_TRY(read_clear_device_status_decode(&w2));
   w |= (w2 & 0xffu) << 24;
   if (h_word_out) *h_word_out = (int32_t)w;

@@ -63,6 +63,8 @@ pmb_status cast_f32_bf16(cudaStream_t st, const float* src, uint16_t* dst, int64
 struct BlockWs {
   float *xzd, *act, *dt, *y, *rstd, *normed, *Aneg;
   SsdWs ssd;
+  float *seg, *seg_bwd;          // states (and their adjoints) of the segments that few long sequences are cut into
+  int nseg;
   float *dnormed, *dxzd, *dact, *ddt, *dA, *scratch, *scratch2;   // scratch: conv partials; scratch2: norm partials
   size_t scratch_bytes, scratch2_bytes;
   uint16_t *normed16, *dxzd16;   // bf16 copies of the two GEMM operands (bf16-storage mode only)
@@ -83,6 +85,19 @@ static size_t slab_floats(const Dims& d) {
   return a > b ? a : b;
 }
 
+// The scan of a block that has a backward runs as ssd_chain.cu / ssd_chain_bwd.cu / ssd_heads.cu on (hi, lo) pairs: every
+// sequence length, d_state and d_head up to 64.  (bf16 blocks whose operands are plain bf16, and d_state 128, keep the kernels
+// that work chunk by chunk.)
+// Long chunks off the 128-token grid (a sequence that no chunk divides is one chunk) in fp32 outside of a model keep the FMA
+// contractions: those form d(a_log) and d(dt_bias) as <dY, y> - <x~, dx~>, whose rounding grows with the chunk (5e-4 of the
+// gradient's norm against fp64 at 3 x 700 tokens, where the sums of the chain kernel are off by 2e-5); from 256 tokens on (64 with
+// heads narrower than 64) the two forms are further apart than fp32 results of one call may move.
+static bool block_uses_chain_bwd(const Dims& d, bool bf16, bool in_model) {
+  const bool dims = bf16 ? !ssd_plain16_shape(d.P, d.N, d.Q) && d.D % 8 == 0 && d.J % 8 == 0 && d.I % 8 == 0 : block_uses_pairs(d);
+  const bool close = bf16 || in_model || ssd_fused_supported(d.P, d.N, d.Q, true) || d.Q <= (d.P >= 64 ? 256 : 64);
+  return dims && close && ssd_chain_enabled() && ssd_chain_bwd_shape(d.P, d.N, true) && d.I <= 2048;
+}
+
 // The workspace has a forward part (everything the recompute produces and the gradient kernels read) and a
 // backward part.  With nslots == 2 the forward part exists twice, so that the recompute of the next block can run
 // (on another stream) while the gradient kernels of the current block still read the other copy; `slot` selects
@@ -91,7 +106,8 @@ static size_t slab_floats(const Dims& d) {
 static size_t block_ws_layout(const Dims& d, void* base, size_t bytes, BlockWs* out, bool bf16 = false, int nslots = 1, int slot = 0, bool presplit = false) {
   Arena ar(base, bytes);
   BlockWs w{};
-  const bool pairs = !bf16 && block_uses_pairs(d);
+  const bool pairs = !bf16 && block_uses_pairs(d), chain = block_uses_chain_bwd(d, bf16, presplit);
+  const size_t hp = (size_t)d.M * d.I, steps_np = (size_t)d.B * cdiv(d.T, SCAN_STEP) * d.H * d.N * d.P;
   const size_t md = (size_t)d.M * d.D, mi = (size_t)d.M * d.I, mj = (size_t)d.M * d.J, dj = (size_t)d.D * d.J, id = (size_t)d.I * d.D;
   for (int sl = 0; sl < nslots; ++sl) {
     BlockWs f{};
@@ -102,7 +118,14 @@ static size_t block_ws_layout(const Dims& d, void* base, size_t bytes, BlockWs* 
     f.rstd = ar.take<float>((size_t)d.M);
     f.normed = ar.take<float>(pairs ? 0 : mi);       // with pair GEMMs the normalised output only exists as a pair
     f.Aneg = ar.take<float>((size_t)d.H);
-    ssd_ws_take(ar, d.B, d.T, d.H, d.P, d.N, d.G, d.Q, &f.ssd, 1);     // what the scan's forward leaves for its backward
+    // what the scan's forward leaves for its backward
+    if (chain) {
+      f.ssd.S = ar.take<float>((size_t)d.M * d.H);
+      f.ssd.bc_hi = ar.take<uint16_t>((size_t)d.M * 2 * d.G * d.N); f.ssd.bc_lo = ar.take<uint16_t>((size_t)d.M * 2 * d.G * d.N);
+      f.ssd.hp_hi = ar.take<uint16_t>(steps_np); f.ssd.hp_lo = ar.take<uint16_t>(steps_np);
+    }
+    else ssd_ws_take(ar, d.B, d.T, d.H, d.P, d.N, d.G, d.Q, &f.ssd, 1);
+    f.seg = ar.take<float>(ssd_chain_shape(d.P, d.N) ? ssd_chain_seg_floats(d.B, d.T, d.H, d.P, d.N) : 0);
     f.normed16 = ar.take<uint16_t>(bf16 ? mi : 0);
     if (pairs) {
       f.x_hi = ar.take<uint16_t>(md); f.x_lo = ar.take<uint16_t>(md);
@@ -113,7 +136,17 @@ static size_t block_ws_layout(const Dims& d, void* base, size_t bytes, BlockWs* 
   }
   // the gradient of the normalised gate output may overwrite it: dW_out (which reads `normed`, or its bf16 copy)
   // is enqueued before the GEMM that writes `dnormed`.  With pair GEMMs there is no fp32 `normed` to reuse.
-  ssd_ws_take(ar, d.B, d.T, d.H, d.P, d.N, d.G, d.Q, &w.ssd, 2);       // the scan's backward-only buffers: one copy
+  // the scan's backward-only buffers: one copy
+  if (chain) {
+    w.ssd.xt_hi = ar.take<uint16_t>(hp); w.ssd.xt_lo = ar.take<uint16_t>(hp); w.ssd.dy_hi = ar.take<uint16_t>(hp); w.ssd.dy_lo = ar.take<uint16_t>(hp);
+    w.ssd.dh_hi = ar.take<uint16_t>(steps_np); w.ssd.dh_lo = ar.take<uint16_t>(steps_np);
+    int per = 0;
+    w.nseg = ssd_chain_segments(d.B, d.T, d.H, &per);
+    w.ssd.part = ar.take<float>((size_t)3 * d.B * w.nseg * d.H);
+    w.seg_bwd = ar.take<float>(ssd_chain_seg_floats(d.B, d.T, d.H, d.P, d.N));
+    w.ssd.splitk = ar.take<float>(ssd_heads_part_floats(d.B, d.T, d.H, d.N, d.G));
+  }
+  else ssd_ws_take(ar, d.B, d.T, d.H, d.P, d.N, d.G, d.Q, &w.ssd, 2);
   w.dnormed = pairs ? ar.take<float>(mi) : w.normed;
   // (with pair GEMMs the three producers of dxzd write the pair directly and the fp32 copy is never formed)
   w.dxzd = pairs ? nullptr : ar.take<float>(mj);
@@ -149,6 +182,18 @@ static SsdIn ssd_inputs(const Dims& d, const pmb_block_params& p, const BlockWs&
   return in;
 }
 
+static ChainArgs chain_inputs(const Dims& d, const pmb_block_params& p, const float* xzd, const float* act, const uint16_t* bc_hi, const uint16_t* bc_lo, float* y) {
+  ChainArgs a{};
+  a.B = d.B; a.T = d.T; a.H = d.H; a.P = d.P; a.N = d.N; a.G = d.G;
+  const int gn = d.G * d.N;
+  a.b = Op16{bc_hi, bc_lo, 2 * gn};
+  a.c = Op16{bc_hi + gn, bc_lo ? bc_lo + gn : nullptr, 2 * gn};
+  a.x = act; a.ldx = d.X; a.D = p.d_skip;
+  a.dt_raw = xzd + d.I + d.X; a.ld_raw = d.J; a.dt_bias = p.dt_bias; a.a_log = p.a_log;
+  a.y = y; a.ldy = d.I;
+  return a;
+}
+
 // Steps 1-8 of Mamba2Block::forward (block.rs:143-222): everything up to the normalised gate output.
 // In bf16-storage mode (w16 != NULL) x is bf16, the two projections run as bf16 GEMMs with fp32 accumulation
 // against bf16 copies of the weights, and everything between them (the reference's "fp32 islands",
@@ -180,12 +225,20 @@ static pmb_status block_fwd_core(cudaStream_t st, const Dims& d, const pmb_block
   ConvPairOut bc{};
   // (bf16 storage: the scan reads the hi halves alone, so the lo halves are not written)
   if (w.ssd.bc_hi) bc = ConvPairOut{w.ssd.bc_hi, w16 ? nullptr : w.ssd.bc_lo, d.I, 2 * d.G * d.N};
+  const bool chain = block_uses_chain_bwd(d, w16 != nullptr, wx && wx->pairs);
+  if (chain) bc.lo = w.ssd.bc_lo;
   PMB_TRY(conv_silu_dt_fwd(st, d, w.xzd, p.conv1d_weight, p.conv1d_bias, p.dt_bias, w.act, nullptr, w.ssd.bc_hi ? &bc : nullptr));
   SsdIn sin = ssd_inputs(d, p, w);
+  if (chain) {
+    ChainArgs a = chain_inputs(d, p, w.xzd, w.act, w.ssd.bc_hi, w.ssd.bc_lo, w.y);
+    a.S_out = w.ssd.S; a.dt_out = w.dt; a.A_out = w.Aneg; a.hp_hi = w.ssd.hp_hi; a.hp_lo = w.ssd.hp_lo; a.seg = w.seg;
+    PMB_TRY(ssd_chain_fwd(st, a));
+  } else {
   sin.plain16 = w16 != nullptr;
   sin.bc_pair_ready = bc.hi != nullptr;
   sin.dt_raw = w.xzd + d.I + d.X; sin.ld_raw = d.J; sin.dt_bias = p.dt_bias; sin.a_log = p.a_log;
   PMB_TRY(ssd_fwd(st, sin, nullptr, w.y, d.I, nullptr, w.ssd));
+  }
   // with pair GEMMs the normalised output is only ever a GEMM operand: write it as a pair, skip the fp32 copy
   // (bf16 storage: the same with a plain bf16 rounding, lo == NULL)
   if (pr) PMB_TRY(gated_rmsnorm_fwd(st, d.M, d.I, d.eps, w.y, w.xzd, d.J, p.norm_weight, nullptr, w.rstd, w.normed_hi, w.normed_lo));
@@ -196,7 +249,7 @@ static pmb_status block_fwd_core(cudaStream_t st, const Dims& d, const pmb_block
 
 // Buffers of a block forward that keeps nothing for a backward and takes the one-kernel scan: a part of what
 // block_ws_layout asks for in every mode, so a workspace of that size always holds it.
-struct FwdWs { float *xzd, *act, *y, *rstd, *normed; uint16_t *bc_hi, *bc_lo, *x_hi, *x_lo, *normed_hi, *normed_lo, *win_hi, *win_lo, *wout_hi, *wout_lo; };
+struct FwdWs { float *xzd, *act, *y, *rstd, *normed, *seg; uint16_t *bc_hi, *bc_lo, *x_hi, *x_lo, *normed_hi, *normed_lo, *win_hi, *win_lo, *wout_hi, *wout_lo; };
 static bool fwd_ws_layout(const Dims& d, void* base, size_t bytes, bool bf16, bool pairs, bool presplit, bool plain, FwdWs* w) {
   Arena ar(base, bytes);
   const size_t md = (size_t)d.M * d.D, mi = (size_t)d.M * d.I, bc = (size_t)d.M * 2 * d.G * d.N;
@@ -204,6 +257,7 @@ static bool fwd_ws_layout(const Dims& d, void* base, size_t bytes, bool bf16, bo
   w->act = ar.take<float>((size_t)d.M * d.X);
   w->y = ar.take<float>(mi);
   w->rstd = ar.take<float>((size_t)d.M);
+  w->seg = ar.take<float>(ssd_chain_seg_floats(d.B, d.T, d.H, d.P, d.N));
   w->normed = (bf16 || pairs) ? nullptr : ar.take<float>(mi);
   w->bc_hi = ar.take<uint16_t>(bc);
   w->bc_lo = plain ? nullptr : ar.take<uint16_t>(bc);
@@ -222,9 +276,13 @@ pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, 
   const Weights16* w16 = storage_is_bf16(wx) ? wx : nullptr;
   const bool pr = !w16 && block_uses_pairs(d);
   BlockWs w{};
-  if (ssd_chain_enabled() && ssd_chain_shape(d.P, d.N)) {
+  const bool plain = w16 && ssd_plain16_shape(d.P, d.N, d.Q);
+  // (plain bf16 chunks keep the rounding of the kernels that work chunk by chunk, so their sequences are not cut: few long ones
+  // are faster chunk by chunk.  One step of a chain takes 3.5 us; those kernels 30 us and 0.1 us per step of a head.)
+  const int64_t steps = cdiv(d.T, SCAN_STEP);
+  const bool by_chunks = plain && 3.5 * steps > 30.0 + 0.1 * (double)((int64_t)d.B * d.H * steps);
+  if (ssd_chain_enabled() && ssd_chain_shape(d.P, d.N) && !by_chunks) {
     // nothing is kept for a backward: the scan is one kernel that takes dt_raw, x and the B | C pair as the conv left them
-    const bool plain = w16 && ssd_plain16_shape(d.P, d.N, d.Q);
     FwdWs f{};
     if (!fwd_ws_layout(d, ws, ws_bytes, w16 != nullptr, pr, wx && wx->pairs, plain, &f))
       return fail(PMB_ERR_WORKSPACE, "block workspace too small (%zu < %zu)", ws_bytes, block_ws_bytes(d, w16 != nullptr));
@@ -239,14 +297,9 @@ pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, 
     ConvPairOut bc{f.bc_hi, f.bc_lo, d.I, 2 * d.G * d.N};
     PMB_TRY(conv_silu_dt_fwd(st, d, f.xzd, p.conv1d_weight, p.conv1d_bias, p.dt_bias, f.act, nullptr, &bc));
     if (!bc.hi) PMB_TRY(split_pair16_strided(st, f.act + d.I, d.M, 2 * d.G * d.N, d.X, f.bc_hi, f.bc_lo, 2 * d.G * d.N));
-    ChainArgs a{};
-    a.B = d.B; a.T = d.T; a.H = d.H; a.P = d.P; a.N = d.N; a.G = d.G; a.blocks = plain ? d.Q / SCAN_STEP : 1;
-    const int gn = d.G * d.N;
-    a.b = Op16{f.bc_hi, f.bc_lo, 2 * gn};
-    a.c = Op16{f.bc_hi + gn, f.bc_lo ? f.bc_lo + gn : nullptr, 2 * gn};
-    a.x = f.act; a.ldx = d.X; a.D = p.d_skip;
-    a.dt_raw = f.xzd + d.I + d.X; a.ld_raw = d.J; a.dt_bias = p.dt_bias; a.a_log = p.a_log;
-    a.y = f.y; a.ldy = d.I;
+    ChainArgs a = chain_inputs(d, p, f.xzd, f.act, f.bc_hi, f.bc_lo, f.y);
+    a.blocks = plain ? d.Q / SCAN_STEP : 1;
+    if (!plain) a.seg = f.seg;
     PMB_TRY(ssd_chain_fwd(st, a));
     PMB_TRY(gated_rmsnorm_fwd(st, d.M, d.I, d.eps, f.y, f.xzd, d.J, p.norm_weight, f.normed, f.rstd, f.normed_hi, f.normed_lo));
     w.normed16 = f.normed_hi; w.normed_hi = f.normed_hi; w.normed_lo = f.normed_lo; w.normed = f.normed; w.x_hi = f.x_hi; w.x_lo = f.x_lo;
@@ -340,7 +393,8 @@ static pmb_status block_grads(cudaStream_t st, const Dims& d, const pmb_block_pa
   sin.plain16 = w16 != nullptr;
   NormBwdExtra ex{};
   ex.dz_hi = ph; ex.dz_lo = pl;
-  if ((pr || w16) && ssd_tc_supported(sin) && (d.P % 4 == 0)) {
+  const bool chain = block_uses_chain_bwd(d, w16 != nullptr, wx && wx->pairs);
+  if (!chain && (pr || w16) && ssd_tc_supported(sin) && (d.P % 4 == 0)) {
     ex.S = w.ssd.S; ex.H = d.H; ex.P = d.P; ex.T = d.T; sin.dys_ready = true;
     if (w.ssd.dy_hi) {   // the scan backward runs on bf16 pairs: dY and dY exp(S) leave the norm backward as pairs
       ex.dy_hi = w.ssd.dy_hi; ex.dy_lo = w16 ? nullptr : w.ssd.dy_lo; sin.dy_pair_ready = true;
@@ -352,14 +406,36 @@ static pmb_status block_grads(cudaStream_t st, const Dims& d, const pmb_block_pa
   PMB_TRY(gated_rmsnorm_bwd(st, d.M, d.I, w.dnormed, w.y, w.xzd, d.J, p.norm_weight, w.rstd, w.dnormed, w.dxzd, d.J,
                             g.norm_weight, w.scratch2, w.scratch2_bytes, gl, &ex));
   // scan
+  bool scan_dt = chain;
+  if (chain) {
+    const int gn = d.G * d.N;
+    const Op16 ob{w.ssd.bc_hi, w.ssd.bc_lo, 2 * gn}, oc{w.ssd.bc_hi + gn, w.ssd.bc_lo + gn, 2 * gn};
+    ChainBwdArgs a{};
+    a.B = d.B; a.T = d.T; a.H = d.H; a.P = d.P; a.N = d.N; a.G = d.G; a.b = ob; a.c = oc;
+    a.hp_hi = w.ssd.hp_hi; a.hp_lo = w.ssd.hp_lo; a.S = w.ssd.S; a.x = w.act; a.ldx = d.X; a.dy = w.dnormed; a.lddy = d.I;
+    a.dt = w.dt; a.A = w.Aneg; a.D = p.d_skip; a.dx = w.dact; a.lddx = d.X;
+    a.xt_hi = w.ssd.xt_hi; a.xt_lo = w.ssd.xt_lo; a.dyo_hi = w.ssd.dy_hi; a.dyo_lo = w.ssd.dy_lo; a.dh_hi = w.ssd.dh_hi; a.dh_lo = w.ssd.dh_lo;
+    a.raw_hi = ph; a.raw_lo = pl; a.ld_raw = d.J; a.raw_col = d.I + d.X; a.part = w.ssd.part; a.seg = w.seg_bwd;
+    PMB_TRY(ssd_chain_bwd(st, a));
+    cudaStream_t sh = st;
+    if (gl) { PMB_TRY(order_after(st, gl->ev[5], gl->s)); sh = gl->s; }
+    PMB_TRY(ssd_head_finish(sh, w.ssd.part, d.B * w.nseg, d.H, w.Aneg, w.dA, g.d_skip, g.dt_bias, g.a_log));
+    HeadsArgs ha{};
+    ha.B = d.B; ha.T = d.T; ha.H = d.H; ha.P = d.P; ha.N = d.N; ha.G = d.G; ha.b = ob; ha.c = oc;
+    ha.dy = Op16{w.ssd.dy_hi, w.ssd.dy_lo, d.I}; ha.xt = Op16{w.ssd.xt_hi, w.ssd.xt_lo, d.I};
+    ha.hp_hi = w.ssd.hp_hi; ha.hp_lo = w.ssd.hp_lo; ha.dh_hi = w.ssd.dh_hi; ha.dh_lo = w.ssd.dh_lo; ha.S = w.ssd.S;
+    ha.db = w.dact + d.I; ha.dc = w.dact + d.I + gn; ha.ld = d.X; ha.part = w.ssd.splitk;
+    PMB_TRY(ssd_heads(st, ha));
+  } else {
   SsdGrads sg{};
   sg.dx = w.dact; sg.lddx = d.X;
   sg.db = w.dact + d.I; sg.dc = w.dact + d.I + d.G * d.N; sg.lddbc = d.X;
   sg.da = nullptr; sg.ddt = w.ddt; sg.dA = w.dA; sg.dD = g.d_skip;
   // the pair path of the scan backward writes the dt columns of the dxzd pair, d_dt_bias and d_a_log itself
-  const bool scan_dt = ph && ssd_bwd_takes_pairs(sin, w.dnormed, d.I, sg);
+  scan_dt = ph && ssd_bwd_takes_pairs(sin, w.dnormed, d.I, sg);
   if (scan_dt) { sg.raw.hi = ph; sg.raw.lo = pl; sg.raw.ld = d.J; sg.raw.col0 = d.I + d.X; sg.raw.d_dt_bias = g.dt_bias; sg.raw.d_a_log = g.a_log; }
   PMB_TRY(ssd_bwd(st, sin, w.y, d.I, w.dnormed, d.I, sg, w.ssd));
+  }
   // otherwise the dt columns (one block per head: a latency-bound loop over the tokens) run next to the conv backward
   if (!scan_dt) {
     cudaStream_t sdt = st;

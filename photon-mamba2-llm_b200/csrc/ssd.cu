@@ -953,6 +953,12 @@ __global__ void head_finish_kernel(const float* __restrict__ part, int rows, int
   if (d_a_log) d_a_log[h] = A[h] * a;
 }
 
+pmb_status ssd_head_finish(cudaStream_t st, const float* part, int rows, int H, const float* A, float* dA, float* dD, float* d_dt_bias, float* d_a_log) {
+  head_finish_kernel<<<(unsigned)cdiv(H, 128), 128, 0, st>>>(part, rows, H, A, dA, dD, d_dt_bias, d_a_log);
+  PMB_LAUNCHED();
+  return PMB_OK;
+}
+
 // Sums the split-K partial tiles in a fixed order.  mode 0: dG (lower-triangular 64x64 tiles only, the
 // others were never produced); mode 1/2: dC/dB rows go to out + token * ld + g * cols.
 __global__ void splitk_reduce_kernel(const float* __restrict__ part, int nsplit, int rows, int cols, int mode, int G, int Q,

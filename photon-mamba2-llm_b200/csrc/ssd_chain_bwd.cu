@@ -1,0 +1,809 @@
+// Backward of the chunked SSD scan along a sequence as one kernel: the adjoint of ssd_chain.cu's forward except for the three
+// sums over heads (dG, dC, dB), which ssd_pairs.cu forms next to it.  One CTA owns one (batch, head) and walks its steps of 128
+// tokens from the last to the first with the state's adjoint dh in registers.
+//
+// Per step (rows s, columns t of the masked tile; S = inclusive cumulative sum of a in the step; h = state entering it, as the forward
+// left it; dh = adjoint of the state leaving it):
+//   GT = B C^T,  dMT = x~ dY^T   (128 x 128 each)                             tensor core
+//   MT[s,t] = GT exp(S_t - S_s) [t >= s];  W[s,t] = dMT MT [t > s]            mask warps: MT back into TMEM, W summed along
+//                                                                             rows and columns in fixed orders
+//   dx~ = MT dY + exp(S_end - S_s) B dh                                       tensor core, mask warps' epilogue
+//   f_t = exp(S_t) <dY_t, C_t h>,  e_s = exp(S_end - S_s) <x~_s, B_s dh>      tensor core, epilogue
+//   dS_t = sum_s W[s,t] - sum_u W[t,u] + f_t - e_t, dS_last += sum_s e_s + exp(S_end) <dh, h>;  da = reverse cumulative sum
+//   dh <- exp(S_end) dh + C^T (exp(S) dY)                                     tensor core, state warps' registers
+// The row and column sums of W come from the same registers, so that the near-total cancellation in sum_t S_t dS_t (the gradient of
+// A) is between identically rounded numbers; <dY, y> - <x~, dx~> from separately rounded products loses it.
+//
+// warp 0 = TMA loads (B, C, h), 1 = MMA issuer, 2 = per-token gradients (da / ddt and the per-head sums), 3 = TMA stores of the bf16
+// operands x~ and dY that the sums over heads read, 4..11 = two mask groups (columns 0-63 / 64-127; then half of the output
+// columns each), 12..19 = transform (x -> x~, dY -> dY and dY exp(S), all into shared memory), 20..23 = state.
+// What bounds it: the mask warps (masked tile and sums of W, then three accumulators drained against x~ and dY), about 10 us per step;
+// GT and dMT of the next step form under the epilogue, the state chain and the loads under the masks.
+// Measured at 24 heads of 64 x 64 on pairs: 42 us for 4 x 512 tokens (the d(states) product, reverse pass, masked product and row
+// kernel it replaces: 118 us), 30 us for 2 x 384, 76 us for 2 x 1000 (1.7 ms of FMA contractions with ssd_heads.cu's share).
+// Every mbarrier wait is bounded, as in the forward.
+#include <cuda_bf16.h>
+#include "tc_common.cuh"
+#include "kernels.h"
+#include "ssd_fused.h"
+
+namespace pmb {
+
+static __device__ unsigned int g_chain_bwd_status = 0;
+
+pmb_status read_clear_device_status_chain_bwd(unsigned int* word) {
+  unsigned int zero = 0;
+  PMB_CUDA(cudaMemcpyFromSymbol(word, g_chain_bwd_status, sizeof(unsigned int)));
+  if (*word) PMB_CUDA(cudaMemcpyToSymbol(g_chain_bwd_status, &zero, sizeof(unsigned int)));
+  return PMB_OK;
+}
+
+namespace scb {
+
+using namespace tcx;
+
+constexpr int L = SCAN_STEP, PW = 64, T128 = L * 128, T64 = 64 * 128;
+constexpr int W_MASK = 4, W_XF = 12, W_ST = 20, NTHREADS = 32 * 24, XF_THREADS = 256;
+// (shares of the block's 80 x 768 registers: 72, 2 x 80, 2 x 72 and 104 per thread of the six warpgroups)
+template <int R> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
+template <int R> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
+
+template <int NS, int NK>
+struct Geo {
+  static constexpr int BT = NS * NK * T128;              // B (or C)
+  static constexpr int HT = NS * NK * T64;               // h, dh: rows n of 128 bytes
+  static constexpr int STAGE = 2 * BT + HT;              // [B | C | h]
+  static constexpr int XT = NS * T128;                   // x~, dY, dY exp(S)
+  static constexpr int XBUF = 3 * XT;
+  static constexpr int XB = NS == 1 ? 2 : 1;
+  static constexpr int NSB = XB + 2;
+  static constexpr int AHEAD = 2;                        // pieces of x and of dY that a transform thread has in flight
+  static constexpr int TILES = STAGE + XB * XBUF + HT;
+  static constexpr int ROWS = 12 * L;                    // per-row sums: [2 groups] of W, e, f, <dx~, x~>; [4 quarters] column sums of W
+  static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 512 /*barriers, small sums*/ + (2 * NSB * L + 2 * ROWS) * 4 + 2 * AHEAD * XF_THREADS * 16;
+};
+
+struct Maps { CUtensorMap b[2], c[2], h[2], xt[2], dy[2]; };      // [0] = hi (or the plain bf16 tensor), [1] = lo
+
+struct Params {
+  int T, H, hpg, N, P, nsteps;
+  const float* S;                                        // (B,H,T)
+  const float* x; const uint16_t* x16; int64_t ldx;
+  const float* dy; const uint16_t* dy16; int64_t lddy;
+  const float* dt; const float* A;                       // (B,T,H), (H); NULL: x~ = x and da is the result
+  const float* D;
+  float* dx; uint16_t* dx16; int64_t lddx;
+  int store_ops;                                         // x~ and dY go out as bf16 operands (maps xt, dy)
+  uint16_t *dh_hi, *dh_lo;                               // (B,nsteps,H,N,P)
+  float* da;                                             // (B,T,H)
+  uint16_t *raw_hi, *raw_lo; int64_t ld_raw; int raw_col;                  // dt mode: gradient before the softplus as a bf16 pair (raw_lo may be NULL)
+  float* part; int64_t part_pitch;                       // dt mode: per (b, h) sums for dA, dD and d_dt_bias, `part_pitch` apart
+  int nseg, per;                                         // segments of a sequence, steps per segment
+  int state_only;                                        // first of two passes over segments: only seg_h and seg_d are formed
+  float *seg_h, *seg_d;                                  // (B*H,nseg,N,P), (B*H,nseg): adjoint that a segment hands back when it receives none, decay over it
+  unsigned int* status;
+};
+
+__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo, bool want_lo) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  if (want_lo) {
+    const float2 hf = __bfloat1622float2(h);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(a - hf.x, b - hf.y);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+  }
+}
+__device__ __forceinline__ void st_shared_v2(uint32_t a, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void st_shared_v4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ uint32_t ld_shared(uint32_t a) { uint32_t v; asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
+__device__ __forceinline__ float2 bf2(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(src) : "memory");
+}
+
+// On entry every lane holds its row's values for 16 consecutive columns; on exit lane l holds the sum of column l & 15 over the
+// warp's 32 rows.  Fixed order.
+__device__ __forceinline__ float warp_column_sums16(float (&v)[16], int lane) {
+#pragma unroll
+  for (int w = 8; w >= 1; w >>= 1) {
+    const bool upper = (lane & w) != 0;
+#pragma unroll
+    for (int k = 0; k < w; ++k) {
+      const float keep = upper ? v[k + w] : v[k];
+      const float send = upper ? v[k] : v[k + w];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+}
+
+template <int NS, int NK, bool IN16>
+__global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
+  using GE = Geo<NS, NK>;
+  constexpr int XB = GE::XB, NSB = GE::NSB;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  uint8_t* base_ptr = smem_raw + (base - raw);
+  const uint32_t b_s = base, c_s = b_s + GE::BT, hin_s = c_s + GE::BT, xbuf_s = base + GE::STAGE, dh_s = xbuf_s + XB * GE::XBUF, bars = dh_s + GE::HT;
+  enum { FULL = 0, EMPTY, XRDY /*2*/, XFREE = XRDY + 2 /*2*/, SRDY = XFREE + 2 /*4*/, GFULL = SRDY + 4, MRDY, ACCFULL, ACCFREE, UFULL, UFREE, HRDY, HFREE,
+         RRDY /*2*/, RFREE = RRDY + 2 /*2*/, NBAR = RFREE + 2 };
+  static_assert(8 * NBAR + 16 + 64 <= 512 && NSB <= 4, "barrier block");
+  auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
+  uint8_t* bar_ptr = base_ptr + (bars - base);
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 8 * NBAR);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+  float* ddw = reinterpret_cast<float*>(bar_ptr + 8 * NBAR + 16);      // [2 steps][4 state warps] <dh, h>
+  float* dDw = ddw + 8;                                                // [8 transform warps] <dY, x>
+  float* sS = reinterpret_cast<float*>(bar_ptr + 512);                 // [NSB] S and dt of a step's tokens
+  float* sRows = sS + 2 * NSB * L;                                     // [2 steps] per-row sums
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int bh = (int)blockIdx.x / p.nseg, seg = (int)blockIdx.x % p.nseg;
+  const int h = bh % p.H, bb = bh / p.H, g = h / p.hpg;
+  const int n = min(p.per, p.nsteps - seg * p.per), last = seg * p.per + n - 1;      // steps of this CTA's segment, the last one of them
+  const int64_t tokb = (int64_t)bb * p.T;
+  if (threadIdx.x == 0) {
+    mbar_init(bar(FULL), 1); mbar_init(bar(EMPTY), p.state_only ? 1 : 5);
+    for (int i = 0; i < 2; ++i) { mbar_init(bar(XRDY + i), 8); mbar_init(bar(XFREE + i), p.state_only ? 1 : 10); mbar_init(bar(RRDY + i), 12); mbar_init(bar(RFREE + i), 1); }
+    for (int i = 0; i < 4; ++i) mbar_init(bar(SRDY + i), 8);
+    mbar_init(bar(GFULL), 1); mbar_init(bar(MRDY), 8); mbar_init(bar(ACCFULL), 1); mbar_init(bar(ACCFREE), 8);
+    mbar_init(bar(UFULL), 1); mbar_init(bar(UFREE), 4); mbar_init(bar(HRDY), 4); mbar_init(bar(HFREE), 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "n"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t tG = tmem, tM = tmem + 128, tA1 = tmem + 256, tA2 = tmem + 320, tA3 = tmem + 384, tU = tmem + 448;
+
+  auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
+  // bounded waits that also end as soon as another role of the CTA has given up
+  auto wait = [&](int b, uint32_t parity, unsigned int code) -> bool {
+    if (*abort_flag) return false;
+    if (mbar_wait(bar(b), parity & 1u)) return true;
+    give_up(code);
+    return false;
+  };
+  auto all = [&](bool v) -> bool { return __all_sync(0xffffffffu, v); };
+
+  // k = 0, 1, ... counts the steps as they are walked; step last - k of the sequence
+  if (warp < W_MASK) {
+    regs_dec<72>();
+    if (warp == 0) {
+      // ---------------- TMA producer: B, C and the entering state ----------------
+      if (lane == 0) {
+        int issued = 0;
+        for (int k = 0; k < n; ++k) {
+          const int i = last - k;
+          if (!wait(EMPTY, (uint32_t)k ^ 1u, 1u)) break;
+          mbar_expect_tx(bar(FULL), p.state_only ? GE::BT : GE::STAGE);
+#pragma unroll
+          for (int sp = 0; sp < NS; ++sp)
+#pragma unroll
+            for (int kt = 0; kt < NK; ++kt) {
+              tma_load_4d(c_s + (sp * NK + kt) * T128, &maps.c[sp], 64 * kt, i * L, g, bb, bar(FULL));
+              if (p.state_only) continue;
+              tma_load_4d(b_s + (sp * NK + kt) * T128, &maps.b[sp], 64 * kt, i * L, g, bb, bar(FULL));
+              tma_load_4d(hin_s + (sp * NK + kt) * T64, &maps.h[sp], 0, 64 * kt, h, bb * p.nsteps + i, bar(FULL));
+            }
+          issued = k + 1;
+        }
+        if (*abort_flag && issued > 0) mbar_wait(bar(FULL), (uint32_t)((issued - 1) & 1));
+      }
+    } else if (warp == 1) {
+      // ---------------- MMA issuer (the whole warp waits; one elected lane issues) ----------------
+      const uint32_t dhi = desc_hi(1024, 2);
+      const uint32_t id_g = idesc_bf16(0, 0, L, L);            // both operands K-major
+      const uint32_t id_v = idesc_bf16(0, 1, L, PW);           // B operand MN-major
+      const uint32_t id_u = idesc_bf16(1, 1, L, PW);           // both operands MN-major
+      auto kstep = [&](uint32_t d, uint32_t alo, uint32_t as, uint32_t blo, uint32_t bs, uint32_t idesc, uint32_t acc) {
+        if (NS == 2) {
+          mma_f16_h(d, alo + as, dhi, blo, dhi, idesc, acc);          // lo x hi
+          mma_f16_h(d, alo, dhi, blo + bs, dhi, idesc, 1u);           // hi x lo
+          mma_f16_h(d, alo, dhi, blo, dhi, idesc, 1u);                // hi x hi
+        } else {
+          mma_f16_h(d, alo, dhi, blo, dhi, idesc, acc);
+        }
+      };
+      const uint32_t BS = (NK * T128) >> 4, HS = (NK * T64) >> 4, XS = T128 >> 4;      // from a hi tile to its lo tile
+      bool ok = true;
+#pragma unroll 1
+      for (int k = 0; k < n && ok; ++k) {
+        const int xb = k % XB;
+        const uint32_t xt_s = xbuf_s + xb * GE::XBUF, dy_s = xt_s + GE::XT, dys_s = dy_s + GE::XT;
+        if (!(ok = all(wait(FULL, (uint32_t)k, 2u) && wait(XRDY + xb, (uint32_t)(k / XB), 2u)))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (!p.state_only) {
+        // (both accumulators were read by the mask warps before they reported the last tile; the products that read the masked
+        // tile over GT were issued before this)
+        if (elect_one()) {
+          const uint32_t b0 = desc_lo(b_s, 16), c0 = desc_lo(c_s, 16), x0 = desc_lo(xt_s, 16), y0 = desc_lo(dy_s, 16);
+#pragma unroll
+          for (int kt = 0; kt < NK; ++kt)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const uint32_t o = (uint32_t)(kt * T128 + q * 32) >> 4;
+              kstep(tG, b0 + o, BS, c0 + o, BS, id_g, (kt | q) ? 1u : 0u);
+            }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) kstep(tM, x0 + 2 * q, XS, y0 + 2 * q, XS, id_g, q ? 1u : 0u);
+          umma_commit(bar(GFULL));
+        }
+        __syncwarp();
+        }
+        // U = C^T (exp(S) dY): the step's contribution to the state's adjoint (with one 64-wide block of d_state the second half
+        // of M reads the tile behind it and its rows of U are never looked at)
+        if (!(ok = all(k == 0 || wait(UFREE, (uint32_t)(k - 1), 4u)))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (elect_one()) {
+          const uint32_t c0 = desc_lo(c_s, T128), y0 = desc_lo(dys_s, T128);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) kstep(tU, c0 + ((uint32_t)(q * 2048) >> 4), BS, y0 + ((uint32_t)(q * 2048) >> 4), XS, id_u, q ? 1u : 0u);
+          umma_commit(bar(UFULL));
+          if (p.state_only) { umma_commit(bar(EMPTY)); umma_commit(bar(XFREE + xb)); }
+        }
+        __syncwarp();
+        if (p.state_only) continue;
+        // B dh and C h
+        if (!(ok = all(wait(HRDY, (uint32_t)k, 8u) && (k == 0 || wait(ACCFREE, (uint32_t)(k - 1), 8u))))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (elect_one()) {
+          const uint32_t b0 = desc_lo(b_s, 16), c0 = desc_lo(c_s, 16), d0 = desc_lo(dh_s, T64), h0 = desc_lo(hin_s, T64);
+#pragma unroll
+          for (int kt = 0; kt < NK; ++kt)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const uint32_t oa = (uint32_t)(kt * T128 + q * 32) >> 4, ob = (uint32_t)(kt * T64 + q * 2048) >> 4;
+              kstep(tA2, b0 + oa, BS, d0 + ob, HS, id_v, (kt | q) ? 1u : 0u);
+              kstep(tA3, c0 + oa, BS, h0 + ob, HS, id_v, (kt | q) ? 1u : 0u);
+            }
+          umma_commit(bar(HFREE));
+          umma_commit(bar(EMPTY));
+        }
+        __syncwarp();
+        // MT dY, the masked tile read from TMEM: per 16 columns [hi: 8 | lo: 8]
+        if (!(ok = all(wait(MRDY, (uint32_t)k, 16u)))) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (elect_one()) {
+          const uint32_t y0 = desc_lo(dy_s, T128);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint32_t ta = tG + (uint32_t)(16 * q), vb = y0 + ((uint32_t)(q * 2048) >> 4);
+            if (NS == 2) {
+              mma_f16_ts_h(tA1, ta + 8u, vb, dhi, id_v, q ? 1u : 0u);
+              mma_f16_ts_h(tA1, ta, vb + XS, dhi, id_v, 1u);
+              mma_f16_ts_h(tA1, ta, vb, dhi, id_v, 1u);
+            } else {
+              mma_f16_ts_h(tA1, ta, vb, dhi, id_v, q ? 1u : 0u);
+            }
+          }
+          umma_commit(bar(ACCFULL));
+          umma_commit(bar(XFREE + xb));
+        }
+        __syncwarp();
+      }
+    } else if (p.state_only) {
+    } else if (warp == 2) {
+      // ---------------- per-token gradients (lane = four consecutive tokens) ----------------
+      const bool dtm = p.dt != nullptr;
+      const float Ah = dtm ? p.A[h] : 1.0f;
+      float accA = 0.0f, accB = 0.0f;
+      for (int k = 0; k < n; ++k) {
+        const int i = last - k;
+        if (!all(wait(SRDY + (k % NSB), (uint32_t)(k / NSB), 1024u) && wait(RRDY + (k & 1), (uint32_t)(k >> 1), 1024u))) break;
+        const float4* R = reinterpret_cast<const float4*>(sRows + (k & 1) * GE::ROWS) + lane;
+        const float* S = sS + (k % NSB) * 2 * L;
+        const float4 S4 = reinterpret_cast<const float4*>(S)[lane], dt4 = reinterpret_cast<const float4*>(S + L)[lane];
+        const float send = S[L - 1];
+        auto two = [&](int a) { const float4 u = R[a * 32], v = R[(a + 1) * 32]; return make_float4(u.x + v.x, u.y + v.y, u.z + v.z, u.w + v.w); };
+        const float4 r4 = two(0), e4 = two(2), f4 = two(4), q4 = two(6), ca = two(8), cb = two(10);
+        const float Sv[4] = {S4.x, S4.y, S4.z, S4.w}, dtv[4] = {dt4.x, dt4.y, dt4.z, dt4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
+        float d[4] = {ca.x + cb.x - r4.x, ca.y + cb.y - r4.y, ca.z + cb.z - r4.z, ca.w + cb.w - r4.w};
+        const float ev[4] = {e4.x, e4.y, e4.z, e4.w}, fv[4] = {f4.x, f4.y, f4.z, f4.w};
+        float es = 0.0f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float e = __expf(send - Sv[j]) * ev[j];
+          es += e;
+          d[j] += __expf(Sv[j]) * fv[j] - e;
+        }
+        es = warp_sum(es);
+        const float* dw = ddw + (k & 1) * 4;
+        if (lane == 31) d[3] += es + __expf(send) * ((dw[0] + dw[1]) + (dw[2] + dw[3]));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(RFREE + (k & 1)));
+        // reverse cumulative sum over the step
+        d[2] += d[3]; d[1] += d[2]; d[0] += d[1];
+        float tail = d[0];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const float u = __shfl_down_sync(0xffffffffu, tail, o); if (lane + o < 32) tail += u; }
+        tail -= d[0];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int t = i * L + 4 * lane + j;
+          if (t >= p.T) continue;
+          const float da = d[j] + tail;
+          if (p.da) p.da[(tokb + t) * p.H + h] = da;
+          if (dtm) {
+            // gradient w.r.t. the pre-softplus dt: (<dx~, x> + A da) (1 - exp(-dt)), with <dx~, x> = <dx~, x~> / dt
+            const float sg = -expm1f(-dtv[j]);
+            const float gr = fmaf(Ah * da, sg, qv[j] * (dtv[j] > 0.0f ? sg / dtv[j] : 1.0f));
+            uint32_t hh, ll;
+            split_bf16_pair(gr, hh, ll);
+            const int64_t o = (tokb + t) * p.ld_raw + p.raw_col + h;
+            p.raw_hi[o] = (uint16_t)hh;
+            if (p.raw_lo) p.raw_lo[o] = (uint16_t)ll;
+            accA = fmaf(da, dtv[j], accA);
+            accB += gr;
+          }
+        }
+      }
+      if (dtm) {
+        accA = warp_sum(accA); accB = warp_sum(accB);
+        // (row of `part`: segment by segment of a sequence)
+        if (lane == 0) { const int64_t o = ((int64_t)bb * p.nseg + seg) * p.H + h; p.part[o] = accA; p.part[2 * p.part_pitch + o] = accB; }
+      }
+    } else {
+      // ---------------- stores of the operands that the sums over heads read ----------------
+      if (lane == 0) {
+        for (int k = 0; k < n; ++k) {
+          const int xb = k % XB, i = last - k;
+          if (!wait(XRDY + xb, (uint32_t)(k / XB), 2048u)) break;
+          if (p.store_ops) {
+#pragma unroll
+            for (int sp = 0; sp < NS; ++sp) {
+              tma_store_4d(&maps.xt[sp], xbuf_s + xb * GE::XBUF + sp * T128, 0, i * L, h, bb);
+              tma_store_4d(&maps.dy[sp], xbuf_s + xb * GE::XBUF + GE::XT + sp * T128, 0, i * L, h, bb);
+            }
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          }
+          mbar_arrive(bar(XFREE + xb));
+        }
+        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+      }
+    }
+  } else if (warp < W_XF) {
+    // ---------------- mask groups, then the epilogue of the same step ----------------
+
+    const int quarter = warp & 3, grp = (warp - W_MASK) >> 2, r_local = quarter * 32 + lane;
+    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+    const bool dtm = p.dt != nullptr;
+    const float dv = p.D ? p.D[h] : 0.0f;
+    const int er = quarter * 32 + (lane >> 2), ec = (lane & 3) * 2;
+    bool ok = !p.state_only;
+    for (int k = 0; k < n && ok; ++k) {
+      const int xb = k % XB, i = last - k;
+      float* R = sRows + (k & 1) * GE::ROWS;
+      const float* S = sS + (k % NSB) * 2 * L;
+      ok = all((k < 2 || wait(RFREE + (k & 1), (uint32_t)((k >> 1) - 1), 32u)) && wait(SRDY + (k % NSB), (uint32_t)(k / NSB), 32u) &&
+               wait(GFULL, (uint32_t)k, 32u));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      {
+        const float S_row = S[r_local];
+        float rsum = 0.0f;
+#pragma unroll 1
+        for (int ch = 0; ch < 4; ++ch) {
+          const int c0 = grp * 64 + ch * 16;
+          uint32_t m[16];
+          float cs = 0.0f;
+          if (c0 + 15 < quarter * 32) {                     // every column is before every row of this warp
+#pragma unroll
+            for (int e = 0; e < 16; ++e) m[e] = 0u;
+          } else {
+            uint32_t gr[16], dr[16];
+            tmem_ld16(tG + lane_addr + (uint32_t)c0, gr);
+            tmem_ld16(tM + lane_addr + (uint32_t)c0, dr);
+            tmem_wait_ld();
+            float w[16];
+#pragma unroll
+            for (int e2 = 0; e2 < 8; ++e2) {
+              const int col = c0 + 2 * e2;
+              const float2 sv = *reinterpret_cast<const float2*>(S + col);
+              float m0 = __uint_as_float(gr[2 * e2]) * __expf(sv.x - S_row), m1 = __uint_as_float(gr[2 * e2 + 1]) * __expf(sv.y - S_row);
+              m0 = col >= r_local ? m0 : 0.0f;
+              m1 = col + 1 >= r_local ? m1 : 0.0f;
+              w[2 * e2] = col > r_local ? m0 * __uint_as_float(dr[2 * e2]) : 0.0f;
+              w[2 * e2 + 1] = col + 1 > r_local ? m1 * __uint_as_float(dr[2 * e2 + 1]) : 0.0f;
+              rsum += w[2 * e2];
+              rsum += w[2 * e2 + 1];
+              split2(m0, m1, m[e2], m[8 + e2], NS == 2);
+              if (NS == 1) m[8 + e2] = 0u;
+            }
+            cs = warp_column_sums16(w, lane);
+          }
+          tmem_st16(tG + lane_addr + (uint32_t)c0, m);
+          if (lane < 16) R[(8 + quarter) * L + c0 + lane] = cs;
+        }
+        R[grp * L + r_local] = rsum;
+        tmem_wait_st();
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(MRDY));
+      }
+      // epilogue: fragments of 16 rows x 8 columns (whole 32-byte sectors per store)
+      ok = all(wait(XRDY + xb, (uint32_t)(k / XB), 64u) && wait(ACCFULL, (uint32_t)k, 64u));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const float send = S[L - 1];
+      const uint32_t xt_s = xbuf_s + xb * GE::XBUF, dy_s = xt_s + GE::XT;
+      const int colb = h * p.P + 32 * grp + ec;
+#pragma unroll 1
+      for (int rh = 0; rh < 2; ++rh) {
+        float fx[2], dtr[2], es[2] = {0.0f, 0.0f}, fs[2] = {0.0f, 0.0f}, qs[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          fx[e] = __expf(send - S[er + 16 * rh + 8 * e]);
+          dtr[e] = dtm ? S[L + er + 16 * rh + 8 * e] : 1.0f;
+        }
+        float2 o[4][2];
+#pragma unroll
+        for (int c16 = 0; c16 < 2; ++c16) {
+          uint32_t a1[8], a2[8], a3[8];
+          const uint32_t ta = lane_addr + ((uint32_t)(16 * rh) << 16) + (uint32_t)(32 * grp + 16 * c16);
+          tmem_ld16x256_x2(tA1 + ta, a1);
+          tmem_ld16x256_x2(tA2 + ta, a2);
+          tmem_ld16x256_x2(tA3 + ta, a3);
+          tmem_wait_ld();
+#pragma unroll
+          for (int q = 0; q < 2; ++q)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const uint32_t at = (uint32_t)((er + 16 * rh + 8 * e) * 128) + (uint32_t)(((4 * grp + 2 * c16 + q) ^ (lane >> 2)) << 4) + (uint32_t)((lane & 3) * 4);
+              float2 xv = bf2(ld_shared(xt_s + at)), yv = bf2(ld_shared(dy_s + at));
+              if (NS == 2) {
+                const float2 xl = bf2(ld_shared(xt_s + T128 + at)), yl = bf2(ld_shared(dy_s + T128 + at));
+                xv.x += xl.x; xv.y += xl.y; yv.x += yl.x; yv.y += yl.y;
+              }
+              const int r = 4 * q + 2 * e;
+              const float u0 = __uint_as_float(a2[r]), u1 = __uint_as_float(a2[r + 1]);
+              const float d0 = fmaf(fx[e], u0, __uint_as_float(a1[r])), d1 = fmaf(fx[e], u1, __uint_as_float(a1[r + 1]));
+              es[e] = fmaf(u0, xv.x, fmaf(u1, xv.y, es[e]));
+              fs[e] = fmaf(__uint_as_float(a3[r]), yv.x, fmaf(__uint_as_float(a3[r + 1]), yv.y, fs[e]));
+              qs[e] = fmaf(d0, xv.x, fmaf(d1, xv.y, qs[e]));
+              o[2 * c16 + q][e] = make_float2(fmaf(d0, dtr[e], dv * yv.x), fmaf(d1, dtr[e], dv * yv.y));
+            }
+        }
+        if (rh == 1) {
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) { mbar_arrive(bar(ACCFREE)); mbar_arrive(bar(XFREE + xb)); }
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+#pragma unroll
+          for (int s = 1; s < 4; s <<= 1) {                 // the quad of lanes that shares a row
+            es[e] += __shfl_xor_sync(0xffffffffu, es[e], s);
+            fs[e] += __shfl_xor_sync(0xffffffffu, fs[e], s);
+            qs[e] += __shfl_xor_sync(0xffffffffu, qs[e], s);
+          }
+          const int row = er + 16 * rh + 8 * e;
+          if ((lane & 3) == 0) { R[(2 + grp) * L + row] = es[e]; R[(4 + grp) * L + row] = fs[e]; R[(6 + grp) * L + row] = qs[e]; }
+          const int t = i * L + row;
+          if (!IN16) {
+            if (t < p.T) {
+              float* dr = p.dx + (tokb + t) * p.lddx + colb;
+#pragma unroll
+              for (int q = 0; q < 4; ++q) if (32 * grp + 8 * q < p.P) *reinterpret_cast<float2*>(dr + 8 * q) = o[q][e];
+            }
+          } else {
+            // neighbouring lanes swap halves, so that a lane writes four columns and a quad one whole sector
+#pragma unroll
+            for (int q = 0; q < 4; q += 2) {
+              uint32_t v0, v1, z;
+              split2(o[q][e].x, o[q][e].y, v0, z, false); split2(o[q + 1][e].x, o[q + 1][e].y, v1, z, false);
+              const bool odd = lane & 1;
+              const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
+              const uint2 wv = odd ? make_uint2(got, v1) : make_uint2(v0, got);
+              if (t < p.T && 32 * grp + 8 * (q + (odd ? 1 : 0)) < p.P)
+                *reinterpret_cast<uint2*>(p.dx16 + (tokb + t) * p.lddx + colb + 8 * q + (odd ? 6 : 0)) = wv;
+            }
+          }
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(RRDY + (k & 1)));
+    }
+  } else if (warp < W_ST) {
+    // ---------------- transform: x -> x~, dY -> dY and dY exp(S) ----------------
+    regs_dec<72>();
+    const int wx = warp - W_XF, tid = threadIdx.x - 32 * W_XF;
+    const bool dtm = p.dt != nullptr;
+    constexpr int LPR = IN16 ? 8 : 16;                      // lanes per row, 16 bytes each
+    constexpr int RPI = 8 * (32 / LPR), NIT = L / RPI;      // rows per pass of the eight warps, passes
+    constexpr int EPL = IN16 ? 8 : 4;                       // elements per lane
+    constexpr int AHEAD = GE::AHEAD;
+    const int j = lane % LPR, r0 = wx * (32 / LPR) + lane / LPR;
+    const bool jcol = EPL * j < p.P;
+    const uint32_t place = (uint32_t)(r0 * 128) + (IN16 ? (uint32_t)((j ^ (r0 & 7)) << 4) : (uint32_t)((((j >> 1) ^ (r0 & 7)) << 4) + (j & 1) * 8));
+    // every thread copies the pieces that it will read itself, AHEAD passes before it reads them (cp.async into slots of its own; no
+    // barrier; rows past the end and columns past d_head arrive as zeros)
+    const uint32_t ring = smem_u32(sRows + 2 * GE::ROWS) + (uint32_t)tid * 16u;
+    constexpr uint32_t SLOT = 2 * XF_THREADS * 16;          // [x | dY]
+    const int esz = IN16 ? 2 : 4;
+    const char* xsrc = (IN16 ? reinterpret_cast<const char*>(p.x16) : reinterpret_cast<const char*>(p.x)) + (int64_t)(h * p.P + (jcol ? EPL * j : 0)) * esz;
+    const char* ysrc = (IN16 ? reinterpret_cast<const char*>(p.dy16) : reinterpret_cast<const char*>(p.dy)) + (int64_t)(h * p.P + (jcol ? EPL * j : 0)) * esz;
+    int rk = 0, rit = 0;                                    // the next piece to request: step and pass
+    auto request = [&](uint32_t slot) {
+      if (rk < n) {
+        const int row = (last - rk) * L + rit * RPI + r0;
+        const bool in = row < p.T && jcol;
+        const int64_t tk = tokb + (row < p.T ? row : p.T - 1);      // (the address stays inside the tensor)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + slot), "l"(xsrc + tk * p.ldx * esz), "r"(in ? 16 : 0) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + slot + XF_THREADS * 16), "l"(ysrc + tk * p.lddy * esz), "r"(in ? 16 : 0) : "memory");
+        if (++rit == NIT) { rit = 0; ++rk; }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const float* Sg = p.S + ((int64_t)bb * p.H + h) * p.T;
+    float s_next = 0.0f, d_next = 1.0f;
+    auto fetch_s = [&](int k) {                             // S and dt of this thread's token of the step
+      if (tid >= L || k >= n) return;
+      const int t = (last - k) * L + tid;
+      s_next = Sg[t < p.T ? t : p.T - 1];                   // (a = 0 past the end)
+      if (dtm) d_next = t < p.T ? p.dt[(tokb + t) * p.H + h] : 0.0f;
+    };
+#pragma unroll 1
+    for (int q = 0; q < AHEAD; ++q) request((uint32_t)q * SLOT);
+    fetch_s(0);
+    uint32_t slot = 0;
+    float dD = 0.0f;
+    bool ok = true;
+    for (int k = 0; k < n; ++k) {
+      const int xb = k % XB;
+      float* S = sS + (k % NSB) * 2 * L;
+      if (ok && k >= XB) ok = all(wait(XFREE + xb, (uint32_t)(k / XB - 1), 128u));
+      // (whoever reads the ring's old entry has finished: NSB - XB - 1 steps lie between it and the step just freed)
+      if (ok && tid < L) { S[tid] = s_next; S[L + tid] = d_next; }
+      asm volatile("bar.sync 4, 256;" ::: "memory");        // (a warp that gave up keeps reaching the named barrier)
+      if (!ok) continue;
+      if (lane == 0) mbar_arrive(bar(SRDY + (k % NSB)));
+      fetch_s(k + 1);
+      uint32_t dst = xbuf_s + xb * GE::XBUF + place;
+#pragma unroll 2
+      for (int it = 0; it < NIT; ++it, dst += RPI * 128) {
+        uint4 xq, yq;
+        asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD - 1) : "memory");
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(xq.x), "=r"(xq.y), "=r"(xq.z), "=r"(xq.w) : "r"(ring + slot) : "memory");
+        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(yq.x), "=r"(yq.y), "=r"(yq.z), "=r"(yq.w) : "r"(ring + slot + XF_THREADS * 16) : "memory");
+        const int row = it * RPI + r0;
+        const float f = __expf(S[row]);
+        if (IN16) {
+          const uint32_t y4[4] = {yq.x, yq.y, yq.z, yq.w};
+          uint32_t s4[4], z;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) { const float2 v = bf2(y4[e]); split2(v.x * f, v.y * f, s4[e], z, false); }
+          st_shared_v4(dst, xq.x, xq.y, xq.z, xq.w);
+          st_shared_v4(dst + GE::XT, yq.x, yq.y, yq.z, yq.w);
+          st_shared_v4(dst + 2 * GE::XT, s4[0], s4[1], s4[2], s4[3]);
+        } else {
+          const float dt = S[L + row];
+          const float xv[4] = {__uint_as_float(xq.x), __uint_as_float(xq.y), __uint_as_float(xq.z), __uint_as_float(xq.w)};
+          const float yv[4] = {__uint_as_float(yq.x), __uint_as_float(yq.y), __uint_as_float(yq.z), __uint_as_float(yq.w)};
+          uint32_t h0, h1, l0 = 0u, l1 = 0u;
+          split2(xv[0] * dt, xv[1] * dt, h0, l0, NS == 2); split2(xv[2] * dt, xv[3] * dt, h1, l1, NS == 2);
+          st_shared_v2(dst, h0, h1);
+          if (NS == 2) st_shared_v2(dst + T128, l0, l1);
+          split2(yv[0], yv[1], h0, l0, NS == 2); split2(yv[2], yv[3], h1, l1, NS == 2);
+          st_shared_v2(dst + GE::XT, h0, h1);
+          if (NS == 2) st_shared_v2(dst + GE::XT + T128, l0, l1);
+          split2(yv[0] * f, yv[1] * f, h0, l0, NS == 2); split2(yv[2] * f, yv[3] * f, h1, l1, NS == 2);
+          st_shared_v2(dst + 2 * GE::XT, h0, h1);
+          if (NS == 2) st_shared_v2(dst + 2 * GE::XT + T128, l0, l1);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) dD = fmaf(xv[e], yv[e], dD);
+        }
+        request(slot);                                      // (this pass has consumed the slot)
+        slot = slot + SLOT == AHEAD * SLOT ? 0u : slot + SLOT;
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(XRDY + xb));
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    dD = warp_sum(dD);
+    if (lane == 0) dDw[wx] = dD;
+  } else {
+    // ---------------- state: dh in registers (thread = row n of the state) ----------------
+    regs_inc<104>();
+    const int quarter = warp & 3, nr = quarter * 32 + lane;
+    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+    const bool active = nr < p.N;                           // rows past d_state hold zeros
+    const bool tile = quarter * 32 < 64 * NK;               // this warp's rows exist in the operand tile
+    const int64_t NP = (int64_t)p.N * p.P;
+    float hv[PW];
+#pragma unroll
+    for (int q = 0; q < PW; ++q) hv[q] = 0.0f;
+    if (!p.state_only && active)
+      for (int j = p.nseg - 1; j > seg; --j) {              // what the segments after this one hand back
+        const float* F = p.seg_h + ((int64_t)bh * p.nseg + j) * NP + (int64_t)nr * p.P;
+        const float dj = p.seg_d[bh * p.nseg + j];
+#pragma unroll
+        for (int q = 0; q < PW / 4; ++q) {
+          if (4 * q >= p.P) continue;
+          const float4 v = *reinterpret_cast<const float4*>(F + 4 * q);
+          hv[4 * q] = fmaf(dj, hv[4 * q], v.x); hv[4 * q + 1] = fmaf(dj, hv[4 * q + 1], v.y);
+          hv[4 * q + 2] = fmaf(dj, hv[4 * q + 2], v.z); hv[4 * q + 3] = fmaf(dj, hv[4 * q + 3], v.w);
+          if (q % 4 == 3) asm volatile("" ::: "memory");      // (no more than four loads in flight: registers)
+        }
+      }
+    bool ok = true;
+    float stot = 0.0f;
+    for (int k = 0; k < n && ok; ++k) {
+      const int i = last - k;
+      if (!p.state_only) {
+      if (k > 0) ok = all(wait(HFREE, (uint32_t)(k - 1), 256u));
+      if (!ok) break;
+      const int64_t so = (((int64_t)bb * p.nsteps + i) * p.H + h) * NP + (int64_t)nr * p.P;
+      if (tile) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {                       // eight 16-byte chunks of the row
+          uint32_t hi[4], lo[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) split2(hv[8 * c + 2 * e], hv[8 * c + 2 * e + 1], hi[e], lo[e], NS == 2);
+          const uint32_t a = dh_s + (uint32_t)(nr * 128 + ((c ^ (nr & 7)) << 4));
+          st_shared_v4(a, hi[0], hi[1], hi[2], hi[3]);
+          if (NS == 2) st_shared_v4(a + NK * T64, lo[0], lo[1], lo[2], lo[3]);
+          if (active && 8 * c < p.P) {
+            *reinterpret_cast<uint4*>(p.dh_hi + so + 8 * c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+            if (NS == 2) *reinterpret_cast<uint4*>(p.dh_lo + so + 8 * c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+          }
+        }
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(HRDY));
+      // <dh, h>
+      ok = all(wait(FULL, (uint32_t)k, 512u) && (k < 2 || wait(RFREE + (k & 1), (uint32_t)((k >> 1) - 1), 512u)));
+      if (!ok) break;
+      float dot = 0.0f;
+      if (active) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const uint32_t a = hin_s + (uint32_t)(nr * 128 + ((c ^ (nr & 7)) << 4));
+          uint32_t v[4];
+#pragma unroll
+          for (int sp = 0; sp < NS; ++sp) {
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a + sp * NK * T64) : "memory");
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { const float2 u = bf2(v[e]); dot = fmaf(u.x, hv[8 * c + 2 * e], fmaf(u.y, hv[8 * c + 2 * e + 1], dot)); }
+          }
+        }
+      }
+      dot = warp_sum(dot);
+      if (lane == 0) {
+        ddw[(k & 1) * 4 + quarter] = dot;
+        mbar_arrive(bar(RRDY + (k & 1)));
+        mbar_arrive(bar(EMPTY));
+      }
+      }
+      ok = all(wait(SRDY + (k % NSB), (uint32_t)(k / NSB), 512u) && wait(UFULL, (uint32_t)k, 512u));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const float send = sS[(k % NSB) * 2 * L + L - 1], dec = __expf(send);
+      stot += send;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t u[16];
+        tmem_ld16(tU + lane_addr + (uint32_t)(16 * q), u);
+        tmem_wait_ld();
+        if (active) {
+#pragma unroll
+          for (int e = 0; e < 16; ++e) hv[16 * q + e] = fmaf(dec, hv[16 * q + e], __uint_as_float(u[e]));
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(UFREE));
+    }
+    if (ok && p.state_only) {
+      if (nr == 0) p.seg_d[blockIdx.x] = __expf(stot);
+      float* dst = p.seg_h + (int64_t)blockIdx.x * NP + (int64_t)nr * p.P;
+      if (active) {
+#pragma unroll
+        for (int q = 0; q < PW / 4; ++q)
+          if (4 * q < p.P) *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (threadIdx.x == 0 && p.part && !p.state_only) {
+    float t = 0.0f;                                         // fixed order
+    for (int q = 0; q < 8; ++q) t += dDw[q];
+    p.part[p.part_pitch + ((int64_t)bb * p.nseg + seg) * p.H + h] = t;
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
+  }
+}
+
+// ---- host side -------------------------------------------------------------------------------------------
+static unsigned int* status_ptr() {
+  static unsigned int* ptr[PMB_MAX_DEVICES] = {nullptr};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= PMB_MAX_DEVICES) dev = 0;
+  if (!ptr[dev]) cudaGetSymbolAddress((void**)&ptr[dev], g_chain_bwd_status);
+  return ptr[dev];
+}
+
+template <int NS, int NK, bool IN16>
+static pmb_status launch(cudaStream_t st, const ChainBwdArgs& a) {
+  using GE = Geo<NS, NK>;
+  static_assert(GE::SMEM <= 227 * 1024, "shared-memory plan");
+  const int n = (int)cdiv(a.T, L);
+  Maps ms{};
+  for (int sp = 0; sp < 2; ++sp) {
+    const bool lo = sp && NS == 2;
+    const int64_t st_h = (int64_t)a.N * a.P, hp = (int64_t)a.H * a.P;
+    PMB_TRY(sf::bf16_map4(&ms.b[sp], lo ? a.b.lo : a.b.hi, a.N, a.T, a.G, a.B, a.b.pitch, a.N, (int64_t)a.T * a.b.pitch, 64, L));
+    PMB_TRY(sf::bf16_map4(&ms.c[sp], lo ? a.c.lo : a.c.hi, a.N, a.T, a.G, a.B, a.c.pitch, a.N, (int64_t)a.T * a.c.pitch, 64, L));
+    PMB_TRY(sf::bf16_map4(&ms.h[sp], lo ? a.hp_lo : a.hp_hi, a.P, a.N, a.H, (int64_t)a.B * n, a.P, st_h, a.H * st_h, 64, 64));
+    if (a.xt_hi) {
+      PMB_TRY(sf::bf16_map4(&ms.xt[sp], lo ? a.xt_lo : a.xt_hi, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
+      PMB_TRY(sf::bf16_map4(&ms.dy[sp], lo ? a.dyo_lo : a.dyo_hi, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
+    }
+  }
+  Params p{};
+  p.T = a.T; p.H = a.H; p.hpg = a.H / a.G; p.N = a.N; p.P = a.P; p.nsteps = n;
+  p.S = a.S; p.x = a.x; p.x16 = a.x16; p.ldx = a.ldx; p.dy = a.dy; p.dy16 = a.dy16; p.lddy = a.lddy; p.dt = a.dt; p.A = a.A; p.D = a.D;
+  p.dx = a.dx; p.dx16 = a.dx16; p.lddx = a.lddx; p.store_ops = a.xt_hi != nullptr; p.dh_hi = a.dh_hi; p.dh_lo = a.dh_lo; p.da = a.da;
+  p.raw_hi = a.raw_hi; p.raw_lo = a.raw_lo; p.ld_raw = a.ld_raw; p.raw_col = a.raw_col; p.part = a.part; p.status = status_ptr();
+  p.nseg = 1; p.per = n;
+  if (a.seg) {
+    p.nseg = ssd_chain_segments(a.B, a.T, a.H, &p.per);
+    p.seg_h = a.seg; p.seg_d = a.seg + (size_t)a.B * a.H * p.nseg * a.N * a.P;
+  }
+  p.part_pitch = (int64_t)a.B * a.H * p.nseg;
+  PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_bwd_kernel<NS, NK, IN16>);
+  const unsigned grid = (unsigned)((int64_t)a.B * a.H * p.nseg);
+  if (p.nseg > 1) {
+    p.state_only = 1;
+    ssd_chain_bwd_kernel<NS, NK, IN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
+    PMB_LAUNCHED();
+    p.state_only = 0;
+  }
+  ssd_chain_bwd_kernel<NS, NK, IN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
+  PMB_LAUNCHED();
+  return PMB_OK;
+}
+
+}  // namespace scb
+
+pmb_status ssd_chain_bwd(cudaStream_t st, const ChainBwdArgs& a) {
+  const bool pairs = a.b.lo != nullptr, in16 = a.x16 != nullptr;
+  if (!ssd_chain_bwd_shape(a.P, a.N, pairs) || a.H % a.G != 0 || (int64_t)a.B * a.H > 0x7fffffff)
+    return fail(PMB_ERR_UNSUPPORTED, "ssd_chain_bwd: unsupported shape (P=%d N=%d)", a.P, a.N);
+  if (in16 == pairs || (in16 && (!a.dy16 || !a.dx16 || a.dt)) || (!in16 && (!a.x || !a.dy || !a.dx)) || (a.dt && (!a.A || !a.raw_hi || !a.part)))
+    return fail(PMB_ERR_ARG, "ssd_chain_bwd: operands must be all pairs of fp32 values or all plain bf16");
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  if (!al16(a.x) || !al16(a.x16) || !al16(a.dy) || !al16(a.dy16) || !al16(a.dx) || !al16(a.dx16) || (a.ldx & (in16 ? 7 : 3)) || (a.lddy & (in16 ? 7 : 3)) || (a.lddx & 3))
+    return fail(PMB_ERR_SHAPE, "ssd_chain_bwd: x, dy and dx rows must be 16-byte aligned");
+  const double tok = (double)a.B * a.T;
+  ProfScope prof(st, "ssd_chain_bwd", tok * a.H * ((double)SCAN_STEP * (a.N + 2.0 * a.P) + 6.0 * a.N * a.P), 0.0);
+  if (pairs) return scb::launch<2, 1, false>(st, a);
+  return a.N > 64 ? scb::launch<1, 2, true>(st, a) : scb::launch<1, 1, true>(st, a);
+}
+
+}  // namespace pmb

@@ -44,7 +44,10 @@ struct ChainArgs {
   uint16_t* x_keep;                            // copy of x16, (B,T,H,P)
   uint16_t *hp_hi, *hp_lo;                     // state entering each step, (B,steps,H,N,P)
   float* last;                                 // (B,H,N,P)
+  float* seg = nullptr;                        // ssd_chain_seg_floats() floats: lets few long sequences be walked in segments (blocks == 1)
 };
+int ssd_chain_segments(int B, int T, int H, int* per);      // segments of a sequence; *per = steps of each (the last may have fewer)
+size_t ssd_chain_seg_floats(int B, int T, int H, int P, int N);
 inline bool ssd_chain_shape(int P, int N) { return P > 0 && P <= 64 && P % 8 == 0 && N > 0 && N <= 128 && N % 8 == 0; }
 bool ssd_chain_enabled();      // false when PMB_SSD_FUSED=0 or PMB_SSD_ENGINE=simt
 // bf16-storage blocks: shapes whose scan reads its operands rounded to bf16 (whole chunks of 128 or 256 tokens at d_state =
@@ -52,6 +55,44 @@ bool ssd_chain_enabled();      // false when PMB_SSD_FUSED=0 or PMB_SSD_ENGINE=s
 bool ssd_plain16_shape(int P, int N, int Q);
 pmb_status ssd_chain_fwd(cudaStream_t st, const ChainArgs& a);
 pmb_status read_clear_device_status_chain(unsigned int* word);
+
+// ---- its backward (ssd_chain_bwd.cu): everything but the sums over heads.  fp32 tensors with (hi, lo) pairs of B, C and the states, or
+// bf16 tensors with plain bf16 operands (x is then x~ and `da` the result).
+struct ChainBwdArgs {
+  int B, T, H, P, N, G;
+  Op16 b, c;                                   // as in ChainArgs
+  const uint16_t *hp_hi, *hp_lo;               // (B,steps,H,N,P) as the forward left it
+  const float* S;                              // (B,H,T) relative to steps
+  const float* x; const uint16_t* x16; int64_t ldx;
+  const float* dy; const uint16_t* dy16; int64_t lddy;
+  const float* dt; const float* A; const float* D;       // dt mode (fp32): (B,T,H), (H), skip weights or NULL
+  float* dx; uint16_t* dx16; int64_t lddx;
+  uint16_t *xt_hi, *xt_lo, *dyo_hi, *dyo_lo;   // optional (B,T,H,P): x~ and dY as operand pairs
+  uint16_t *dh_hi, *dh_lo;                     // (B,steps,H,N,P) adjoint of the state leaving each step
+  float* da;                                   // (B,T,H) or NULL
+  uint16_t *raw_hi, *raw_lo; int64_t ld_raw; int raw_col;   // dt mode: gradient before the softplus, at [token * ld_raw + raw_col + h]
+  float* part;                                 // dt mode: 3 x (B * segments,H): sums for dA, dD, d_dt_bias
+  float* seg;                                  // as in ChainArgs, or NULL: no segments
+};
+inline bool ssd_chain_bwd_shape(int P, int N, bool pairs) { return P > 0 && P <= 64 && P % 8 == 0 && N > 0 && N <= (pairs ? 64 : 128) && N % 8 == 0; }
+// the per-head sums over `rows` rows of each of part's three sections; d_a_log = A dA
+pmb_status ssd_head_finish(cudaStream_t st, const float* part, int rows, int H, const float* A, float* dA, float* dD, float* d_dt_bias, float* d_a_log);
+pmb_status ssd_chain_bwd(cudaStream_t st, const ChainBwdArgs& a);
+pmb_status read_clear_device_status_chain_bwd(unsigned int* word);
+
+// ---- the sums over heads next to it (ssd_heads.cu): dB and dC from the operands that the two passes leave
+struct HeadsArgs {
+  int B, T, H, P, N, G;
+  Op16 b, c, dy, xt;                           // b, c as in ChainArgs; dy and xt (B,T,H,P)
+  const uint16_t *hp_hi, *hp_lo, *dh_hi, *dh_lo;       // (B,steps,H,N,P)
+  const float* S;                              // (B,H,T)
+  float *dc, *db; uint16_t *dc16, *db16; int64_t ld;   // fp32 or bf16 token rows, group g at column g * N
+  float* part;                                 // ssd_heads_part_floats() floats
+};
+int ssd_heads_nsplit(int B, int T, int H, int G);
+size_t ssd_heads_part_floats(int B, int T, int H, int N, int G);
+pmb_status ssd_heads(cudaStream_t st, const HeadsArgs& a);
+pmb_status read_clear_device_status_heads(unsigned int* word);
 
 // Shapes the fused kernels take: block_len a multiple of 128 (at most 1024); d_state and d_head in {64, 128} with
 // plain bf16 operands, d_state = d_head = 64 with (hi, lo) pairs (what fits the shared-memory plan of both modes).

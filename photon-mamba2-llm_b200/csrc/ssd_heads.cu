@@ -1,0 +1,442 @@
+// The three sums over the heads of a group in the backward of the SSD scan, as one kernel over tiles of one step (128 tokens) of
+// one group (mamba2/ssd_ops.rs:201-234 and its autograd compute the same quantities op by op):
+//   dG[t,s] = sum_h exp(S_h,t - S_h,s) [s <= t] <dY_h,t, x~_h,s>
+//   dC[t,:] = dG B   + sum_h exp(S_h,t)            dY_h,t h_h      (h = state entering the step)
+//   dB[s,:] = dG^T C + sum_h exp(S_h,end - S_h,s)  x~_h,s dh_h     (dh = adjoint of the state leaving it)
+// Per head the tensor core forms dY x~^T, dY h^T and x~ dh^T from four tiles; the decays are applied where the products are added
+// up in registers, so no copy of dY or x~ scaled by them exists and dG never leaves the SM.  With few tiles the heads of a group
+// are split over CTAs; dC and dB are linear in dG, so every CTA finishes its own heads' share and the shares are added in a fixed
+// order (heads_sum_kernel).  d_state is taken in halves of 64: a second pass over the heads forms the second half.
+//
+// warp 0 = TMA, 1 = MMA issuer, 2 = S of the heads, 4..11 = dG (64 columns per thread), 12..15 = dC, 16..19 = dB (64 columns per
+// thread).  Two operand stages, two sets of accumulators: the products of the next head run under the sums of this one.
+// What bounds it: the exponentials and the multiply-adds of the dG warps (64 of each per thread and head).
+// Measured at 24 heads of 64 x 64 on pairs, 4 x 512 tokens: 18 us + 3 us for the sum of the shares; the three contractions and their
+// sums that it replaces took 45 us and read copies of dY and x~ scaled by the decays that are not made any more.
+#include <cuda_bf16.h>
+#include "tc_common.cuh"
+#include "kernels.h"
+#include "ssd_fused.h"
+
+namespace pmb {
+
+static __device__ unsigned int g_heads_status = 0;
+
+pmb_status read_clear_device_status_heads(unsigned int* word) {
+  unsigned int zero = 0;
+  PMB_CUDA(cudaMemcpyFromSymbol(word, g_heads_status, sizeof(unsigned int)));
+  if (*word) PMB_CUDA(cudaMemcpyToSymbol(g_heads_status, &zero, sizeof(unsigned int)));
+  return PMB_OK;
+}
+
+namespace shd {
+
+using namespace tcx;
+
+constexpr int L = SCAN_STEP, T128 = L * 128, T64 = 64 * 128;
+constexpr int W_G = 4, W_C = 12, NTHREADS = 32 * 20;
+
+template <int NS>
+struct Geo {
+  static constexpr int XT = NS * T128, HT = NS * T64;
+  static constexpr int STAGE = 2 * XT + 2 * HT;            // [dY | x~ | h | dh]; at the end of a pass [B | C]
+  static constexpr int DG = 2 * XT;                        // dG as an operand: two 64-column tiles (hi), then lo
+  static constexpr bool OWN_DG = NS == 1;                  // pairs: dG goes over the stage that the last head has left
+  static constexpr int RING = 4;                           // heads whose S is in shared memory
+  static constexpr int TILES = 2 * STAGE + (OWN_DG ? DG : 0);
+  static_assert(OWN_DG || DG <= STAGE, "dG fits a stage");
+  static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 256 /*barriers*/ + RING * L * 4;
+};
+
+struct Maps { CUtensorMap dy[2], xt[2], h[2], dh[2], b[2], c[2]; };
+
+struct Params {
+  int T, H, G, hpg, N, n, nsplit, passes;
+  const float* S;
+  float *dc, *db; int64_t ld;                              // token rows, group g at column g * N
+  uint16_t *dc16, *db16;                                   // the same as bf16 (instead)
+  float* part;                                             // nsplit > 1: [tile][split][dC | dB][128][N]
+  unsigned int* status;
+};
+
+__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t pack2(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+template <int NS>
+__global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_constant__ Maps maps, const Params p) {
+  using GE = Geo<NS>;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  uint8_t* base_ptr = smem_raw + (base - raw);
+  const uint32_t bars = base + GE::TILES;
+  enum { FULL = 0 /*2*/, EMPTY = 2 /*2*/, MFULL = 4 /*2*/, MFREE = 6 /*2*/, CFULL = 8 /*2*/, CFREE = 10 /*2*/, SRDY = 12 /*4*/, SFREE = 16 /*4*/, DGRDY = 20, NBAR };
+  static_assert(8 * NBAR + 8 <= 256, "barrier block");
+  auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
+  uint8_t* bar_ptr = base_ptr + GE::TILES;
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 8 * NBAR);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+  float* sS = reinterpret_cast<float*>(bar_ptr + 256);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  int id = (int)blockIdx.x;
+  const int split = id % p.nsplit; id /= p.nsplit;
+  const int tile = id;
+  const int g = id % p.G; id /= p.G;
+  const int i = id % p.n, bb = id / p.n;
+  const int nh = (p.hpg - split + p.nsplit - 1) / p.nsplit;
+  auto head = [&](int j) { return g * p.hpg + split + j * p.nsplit; };
+  const int per_pass = nh + 1, nitems = p.passes * per_pass;     // the heads, then the product with dG
+  if (threadIdx.x == 0) {
+    for (int q = 0; q < 2; ++q) {
+      mbar_init(bar(FULL + q), 1); mbar_init(bar(EMPTY + q), 1); mbar_init(bar(MFULL + q), 1); mbar_init(bar(MFREE + q), 8);
+      mbar_init(bar(CFULL + q), 1); mbar_init(bar(CFREE + q), 8);
+    }
+    for (int q = 0; q < 4; ++q) { mbar_init(bar(SRDY + q), 1); mbar_init(bar(SFREE + q), 16); }
+    mbar_init(bar(DGRDY), 8);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)), "n"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t tM = tmem, tC = tmem + 256, tB = tmem + 384;
+  // the stage that dG goes over: the one the last head of the first pass was in
+  const uint32_t dg_s = GE::OWN_DG ? base + 2 * GE::STAGE : base + (uint32_t)((nh - 1) & 1) * GE::STAGE;
+
+  auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
+  auto wait = [&](int b, uint32_t parity, unsigned int code) -> bool {
+    if (*abort_flag) return false;
+    if (mbar_wait(bar(b), parity & 1u)) return true;
+    give_up(code);
+    return false;
+  };
+  auto all = [&](bool v) -> bool { return __all_sync(0xffffffffu, v); };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int issued = 0;
+      for (int m = 0; m < nitems; ++m) {
+        const int s = m & 1, ps = m / per_pass, j = m - ps * per_pass;
+        if (!wait(EMPTY + s, (uint32_t)(m >> 1) ^ 1u, 1u)) break;
+        const uint32_t st = base + s * GE::STAGE;
+        if (j < nh) {
+          const int h = head(j);
+          mbar_expect_tx(bar(FULL + s), GE::STAGE);
+#pragma unroll
+          for (int sp = 0; sp < NS; ++sp) {
+            tma_load_4d(st + sp * T128, &maps.dy[sp], 0, i * L, h, bb, bar(FULL + s));
+            tma_load_4d(st + GE::XT + sp * T128, &maps.xt[sp], 0, i * L, h, bb, bar(FULL + s));
+            tma_load_4d(st + 2 * GE::XT + sp * T64, &maps.h[sp], 0, 64 * ps, h, bb * p.n + i, bar(FULL + s));
+            tma_load_4d(st + 2 * GE::XT + GE::HT + sp * T64, &maps.dh[sp], 0, 64 * ps, h, bb * p.n + i, bar(FULL + s));
+          }
+        } else {
+          mbar_expect_tx(bar(FULL + s), 2 * GE::XT);
+#pragma unroll
+          for (int sp = 0; sp < NS; ++sp) {
+            tma_load_4d(st + sp * T128, &maps.b[sp], 64 * ps, i * L, g, bb, bar(FULL + s));
+            tma_load_4d(st + GE::XT + sp * T128, &maps.c[sp], 64 * ps, i * L, g, bb, bar(FULL + s));
+          }
+        }
+        issued = m + 1;
+      }
+      if (*abort_flag)
+        for (int m = (issued > 2 ? issued - 2 : 0); m < issued; ++m) mbar_wait(bar(FULL + (m & 1)), (uint32_t)((m >> 1) & 1));
+    }
+  } else if (warp == 1) {
+    const uint32_t dhi = desc_hi(1024, 2);
+    const uint32_t id_m = idesc_bf16(0, 0, L, L), id_h = idesc_bf16(0, 0, L, 64);      // both operands K-major
+    const uint32_t id_c = idesc_bf16(0, 1, L, 64), id_b = idesc_bf16(1, 1, L, 64);     // dG B and dG^T C
+    auto kstep = [&](uint32_t d, uint32_t alo, uint32_t as, uint32_t blo, uint32_t bs, uint32_t idesc, uint32_t acc) {
+      if (NS == 2) {
+        mma_f16_h(d, alo + as, dhi, blo, dhi, idesc, acc);
+        mma_f16_h(d, alo, dhi, blo + bs, dhi, idesc, 1u);
+        mma_f16_h(d, alo, dhi, blo, dhi, idesc, 1u);
+      } else {
+        mma_f16_h(d, alo, dhi, blo, dhi, idesc, acc);
+      }
+    };
+    const uint32_t XS = T128 >> 4, HS = T64 >> 4, DS = (2 * T128) >> 4;
+    bool ok = true;
+#pragma unroll 1
+    for (int m = 0; m < nitems && ok; ++m) {
+      const int s = m & 1, ps = m / per_pass, j = m - ps * per_pass;
+      const uint32_t st = base + s * GE::STAGE;
+      ok = all(wait(FULL + s, (uint32_t)(m >> 1), 2u) && (m < 2 || wait(CFREE + s, (uint32_t)((m >> 1) - 1), 4u)) &&
+               (ps > 0 || j >= nh || j < 2 || wait(MFREE + (j & 1), (uint32_t)((j >> 1) - 1), 8u)) && (j < nh || wait(DGRDY, 0u, 16u)));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (elect_one()) {
+        const uint32_t dC = tC + (uint32_t)(64 * s), dB = tB + (uint32_t)(64 * s);
+        if (j < nh) {
+          const uint32_t y0 = desc_lo(st, 16), x0 = desc_lo(st + GE::XT, 16), h0 = desc_lo(st + 2 * GE::XT, 16), d0 = desc_lo(st + 2 * GE::XT + GE::HT, 16);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            if (ps == 0) kstep(tM + (uint32_t)(128 * (j & 1)), y0 + 2 * q, XS, x0 + 2 * q, XS, id_m, q ? 1u : 0u);
+            kstep(dC, y0 + 2 * q, XS, h0 + 2 * q, HS, id_h, q ? 1u : 0u);
+            kstep(dB, x0 + 2 * q, XS, d0 + 2 * q, HS, id_h, q ? 1u : 0u);
+          }
+          if (ps == 0) umma_commit(bar(MFULL + (j & 1)));
+        } else {
+          const uint32_t gk = desc_lo(dg_s, 16), gm = desc_lo(dg_s, T128), b0 = desc_lo(st, T128), c0 = desc_lo(st + GE::XT, T128);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint32_t o = (uint32_t)(q * 2048) >> 4;
+            kstep(dC, gk + ((uint32_t)((q >> 2) * T128 + (q & 3) * 32) >> 4), DS, b0 + o, XS, id_c, q ? 1u : 0u);
+            kstep(dB, gm + o, DS, c0 + o, XS, id_b, q ? 1u : 0u);
+          }
+        }
+        umma_commit(bar(CFULL + s));
+        umma_commit(bar(EMPTY + s));
+      }
+      __syncwarp();
+    }
+  } else if (warp == 2) {
+    // S of a head's 128 tokens (a = 0 past the end of the sequence); every head once per pass
+    for (int m = 0; m < p.passes * nh; ++m) {
+      const int r = m % GE::RING;
+      if (m >= GE::RING && !all(wait(SFREE + r, (uint32_t)(m / GE::RING - 1), 32u))) break;
+      const float* Sg = p.S + ((int64_t)bb * p.H + head(m % nh)) * p.T;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int t = i * L + lane + 32 * e;
+        sS[r * L + lane + 32 * e] = Sg[t < p.T ? t : p.T - 1];
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(SRDY + r));
+    }
+  } else if (warp >= W_G && warp < W_C) {
+    // ---------------- dG ----------------
+    const int quarter = warp & 3, grp = (warp - W_G) >> 2, row = quarter * 32 + lane;
+    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+    float acc[64];
+#pragma unroll
+    for (int e = 0; e < 64; ++e) acc[e] = 0.0f;
+    bool ok = true;
+    const bool above = grp == 1 && quarter < 2;                // every column of this half is past every row of this warp
+    for (int j = 0; j < nh && ok; ++j) {
+      const float* S = sS + (j % GE::RING) * L;
+      ok = all(wait(SRDY + (j % GE::RING), (uint32_t)(j / GE::RING), 64u) && wait(MFULL + (j & 1), (uint32_t)(j >> 1), 64u));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (!above) {
+        const float S_row = S[row];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint32_t v[16];
+          tmem_ld16(tM + lane_addr + (uint32_t)(128 * (j & 1) + grp * 64 + 16 * q), v);
+          tmem_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 16; e += 4) {
+            const int col = grp * 64 + 16 * q + e;
+            const float4 s4 = *reinterpret_cast<const float4*>(S + col);
+            const float sv[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const float w = col + u <= row ? __expf(S_row - sv[u]) : 0.0f;
+              acc[16 * q + e + u] = fmaf(__uint_as_float(v[e + u]), w, acc[16 * q + e + u]);
+            }
+          }
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) { mbar_arrive(bar(MFREE + (j & 1))); mbar_arrive(bar(SFREE + (j % GE::RING))); }
+    }
+    if (ok) {
+      // (all products of the last head are done: its stage is free for dG)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          hi[e] = pack2(acc[8 * c + 2 * e], acc[8 * c + 2 * e + 1]);
+          lo[e] = pack2(acc[8 * c + 2 * e] - __uint_as_float(hi[e] << 16), acc[8 * c + 2 * e + 1] - __uint_as_float(hi[e] & 0xffff0000u));
+        }
+        const uint32_t a = dg_s + (uint32_t)(grp * T128 + row * 128 + ((c ^ (row & 7)) << 4));
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
+        if (NS == 2) asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a + 2 * T128), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(DGRDY));
+    }
+  } else if (warp >= W_C) {
+    // ---------------- dC (first four warps) and dB ----------------
+    const int quarter = warp & 3, which = (warp - W_C) >> 2, row = quarter * 32 + lane;
+    const uint32_t src = (which ? tB : tC) + ((uint32_t)(quarter * 32) << 16);
+    bool ok = true;
+    int m = 0, hs = 0;
+    for (int ps = 0; ps < p.passes && ok; ++ps) {
+      float acc[64];
+#pragma unroll
+      for (int e = 0; e < 64; ++e) acc[e] = 0.0f;
+      for (int j = 0; j <= nh && ok; ++j, ++m) {
+        const int s = m & 1;
+        float f = 1.0f;
+        if (j < nh) {
+          ok = all(wait(SRDY + (hs % GE::RING), (uint32_t)(hs / GE::RING), 128u));
+          if (!ok) break;
+          const float* S = sS + (hs % GE::RING) * L;
+          f = __expf(which ? S[L - 1] - S[row] : S[row]);
+        }
+        ok = all(wait(CFULL + s, (uint32_t)(m >> 1), 128u));
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint32_t v[16];
+          tmem_ld16(src + (uint32_t)(64 * s + 16 * q), v);
+          tmem_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) acc[16 * q + e] = fmaf(__uint_as_float(v[e]), f, acc[16 * q + e]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(CFREE + s));
+        if (j < nh) {
+          if (lane == 0) {
+            mbar_arrive(bar(SFREE + (hs % GE::RING)));
+            if (ps > 0) mbar_arrive(bar(SFREE + (hs % GE::RING)));      // (the dG warps take part in the first pass only)
+          }
+          ++hs;
+        }
+      }
+      if (!ok) break;
+      const int t = i * L + row, w = p.N - 64 * ps;            // columns of this half (a multiple of 8)
+      if (p.nsplit > 1) {
+        float4* dst = reinterpret_cast<float4*>(p.part + ((((int64_t)tile * p.nsplit + split) * 2 + which) * L + row) * p.N + 64 * ps);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) if (4 * e < w) dst[e] = make_float4(acc[4 * e], acc[4 * e + 1], acc[4 * e + 2], acc[4 * e + 3]);
+      } else if (t < p.T) {
+        const int64_t o = ((int64_t)bb * p.T + t) * p.ld + (int64_t)g * p.N + 64 * ps;
+        uint16_t* o16 = which ? p.db16 : p.dc16;
+        if (o16) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e)
+            if (8 * e < w) *reinterpret_cast<uint4*>(o16 + o + 8 * e) = make_uint4(pack2(acc[8 * e], acc[8 * e + 1]), pack2(acc[8 * e + 2], acc[8 * e + 3]),
+                                                                                    pack2(acc[8 * e + 4], acc[8 * e + 5]), pack2(acc[8 * e + 6], acc[8 * e + 7]));
+        } else {
+          float4* dst = reinterpret_cast<float4*>((which ? p.db : p.dc) + o);
+#pragma unroll
+          for (int e = 0; e < 16; ++e) if (4 * e < w) dst[e] = make_float4(acc[4 * e], acc[4 * e + 1], acc[4 * e + 2], acc[4 * e + 3]);
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
+  }
+}
+
+// Adds the shares of the splits in a fixed order; four columns per thread.
+__global__ void __launch_bounds__(256) heads_sum_kernel(const float* __restrict__ part, Params p, int64_t total) {
+  const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= total) return;
+  const int n4 = p.N / 4, c = (int)(q % n4); int64_t r = q / n4;
+  const int row = (int)(r % L); r /= L;
+  const int which = (int)(r & 1); r >>= 1;
+  const int g = (int)(r % p.G); const int64_t bi = r / p.G;
+  const int t = (int)(bi % p.n) * L + row;
+  if (t >= p.T) return;
+  const float4* src = reinterpret_cast<const float4*>(part) + ((r * p.nsplit * 2 + which) * L + row) * n4 + c;
+  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 4
+  for (int k = 0; k < p.nsplit; ++k) {
+    const float4 v = src[(int64_t)k * 2 * L * n4];
+    s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+  }
+  const int64_t o = ((bi / p.n) * p.T + t) * p.ld + (int64_t)g * p.N + 4 * c;
+  uint16_t* o16 = which ? p.db16 : p.dc16;
+  if (o16) *reinterpret_cast<uint2*>(o16 + o) = make_uint2(pack2(s.x, s.y), pack2(s.z, s.w));
+  else *reinterpret_cast<float4*>((which ? p.db : p.dc) + o) = s;
+}
+
+static unsigned int* status_ptr() {
+  static unsigned int* ptr[PMB_MAX_DEVICES] = {nullptr};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= PMB_MAX_DEVICES) dev = 0;
+  if (!ptr[dev]) cudaGetSymbolAddress((void**)&ptr[dev], g_heads_status);
+  return ptr[dev];
+}
+
+template <int NS>
+static pmb_status launch(cudaStream_t st, const HeadsArgs& a, int nsplit) {
+  using GE = Geo<NS>;
+  static_assert(GE::SMEM <= 227 * 1024, "shared-memory plan");
+  const int n = (int)cdiv(a.T, L);
+  Maps ms{};
+  for (int sp = 0; sp < 2; ++sp) {
+    const bool lo = sp && NS == 2;
+    const int64_t st_h = (int64_t)a.N * a.P, hp = (int64_t)a.H * a.P;
+    PMB_TRY(sf::bf16_map4(&ms.dy[sp], lo ? a.dy.lo : a.dy.hi, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
+    PMB_TRY(sf::bf16_map4(&ms.xt[sp], lo ? a.xt.lo : a.xt.hi, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
+    PMB_TRY(sf::bf16_map4(&ms.h[sp], lo ? a.hp_lo : a.hp_hi, a.P, a.N, a.H, (int64_t)a.B * n, a.P, st_h, a.H * st_h, 64, 64));
+    PMB_TRY(sf::bf16_map4(&ms.dh[sp], lo ? a.dh_lo : a.dh_hi, a.P, a.N, a.H, (int64_t)a.B * n, a.P, st_h, a.H * st_h, 64, 64));
+    PMB_TRY(sf::bf16_map4(&ms.b[sp], lo ? a.b.lo : a.b.hi, a.N, a.T, a.G, a.B, a.b.pitch, a.N, (int64_t)a.T * a.b.pitch, 64, L));
+    PMB_TRY(sf::bf16_map4(&ms.c[sp], lo ? a.c.lo : a.c.hi, a.N, a.T, a.G, a.B, a.c.pitch, a.N, (int64_t)a.T * a.c.pitch, 64, L));
+  }
+  Params p{};
+  p.T = a.T; p.H = a.H; p.G = a.G; p.hpg = a.H / a.G; p.N = a.N; p.n = n; p.nsplit = nsplit; p.passes = (int)cdiv(a.N, 64);
+  p.S = a.S; p.dc = a.dc; p.db = a.db; p.ld = a.ld; p.dc16 = a.dc16; p.db16 = a.db16; p.part = a.part; p.status = status_ptr();
+  const int64_t tiles = (int64_t)a.B * n * a.G;
+  PMB_SMEM_OPT_IN(GE::SMEM, ssd_heads_kernel<NS>);
+  ssd_heads_kernel<NS><<<(unsigned)(tiles * nsplit), NTHREADS, GE::SMEM, st>>>(ms, p);
+  PMB_LAUNCHED();
+  if (nsplit > 1) {
+    const int64_t total = tiles * 2 * L * (a.N / 4);
+    heads_sum_kernel<<<(unsigned)cdiv(total, 256), 256, 0, st>>>(a.part, p, total);
+    PMB_LAUNCHED();
+  }
+  return PMB_OK;
+}
+
+}  // namespace shd
+
+// One CTA per SM: as many splits as fill the machine once, then the fewest with the same number of heads per CTA.
+int ssd_heads_nsplit(int B, int T, int H, int G) {
+  const int64_t tiles = (int64_t)B * cdiv(T, SCAN_STEP) * G;
+  const int hpg = H / G;
+  int want = tiles >= 148 ? 1 : (int)(148 / tiles);
+  if (want > hpg) want = hpg;
+  const int per = (int)cdiv(hpg, want);
+  return (int)cdiv(hpg, per);
+}
+size_t ssd_heads_part_floats(int B, int T, int H, int N, int G) {
+  const int ns = ssd_heads_nsplit(B, T, H, G);
+  return ns > 1 ? (size_t)B * cdiv(T, SCAN_STEP) * G * ns * 2 * SCAN_STEP * N : 0;
+}
+
+pmb_status ssd_heads(cudaStream_t st, const HeadsArgs& a) {
+  const bool pairs = a.b.lo != nullptr;
+  if (!ssd_chain_bwd_shape(a.P, a.N, pairs) || a.H % a.G != 0) return fail(PMB_ERR_UNSUPPORTED, "ssd_heads: unsupported shape (P=%d N=%d)", a.P, a.N);
+  if ((a.dy.lo != nullptr) != pairs || (a.xt.lo != nullptr) != pairs) return fail(PMB_ERR_ARG, "ssd_heads: operands must be all pairs or all plain bf16");
+  const int nsplit = ssd_heads_nsplit(a.B, a.T, a.H, a.G);
+  const int64_t tiles = (int64_t)a.B * cdiv(a.T, SCAN_STEP) * a.G;
+  if (tiles * nsplit > 0x7fffffff) return fail(PMB_ERR_SHAPE, "ssd_heads: too many tiles");
+  auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
+  if (!al16(a.dc) || !al16(a.db) || !al16(a.dc16) || !al16(a.db16) || !al16(a.part) || (a.ld & (a.dc16 ? 7 : 3))) return fail(PMB_ERR_SHAPE, "ssd_heads: dB and dC rows must be 16-byte aligned");
+  const double tok = (double)a.B * a.T;
+  ProfScope prof(st, "ssd_heads", tok * (a.H * ((double)SCAN_STEP * a.P + 4.0 * a.N * a.P) + 2.0 * a.G * SCAN_STEP * a.N), 0.0);
+  return pairs ? shd::launch<2>(st, a, nsplit) : shd::launch<1>(st, a, nsplit);
+}
+
+}  // namespace pmb
