@@ -93,14 +93,21 @@ size_t ssd_ws_layout(int B, int T, int H, int P, int N, int G, int Q, void* base
 // the same buffers taken from a caller's arena in two parts: bit 0 = forward-written / backward-read, bit 1 = backward only
 struct Arena;
 void ssd_ws_take(Arena& ar, int B, int T, int H, int P, int N, int G, int Q, SsdWs* w, int part);
-// The scan on bf16 inputs as they are (plain bf16 tensor-core operands, fp32 recurrence; no fp32 staging copies).
-// Shapes: d_head 64, d_state 64 or 128, block_len % 128 == 0, at most 64 chunks per sequence.
+// The scan on bf16 inputs as they are (bf16 tensor-core operands, fp32 recurrence; no fp32 staging copies): any length, d_head up to
+// 64 and d_state up to 128 in multiples of 8.
+struct Scan16Ws {
+  bool plain;                          // what is formed on the way is rounded to bf16 (whole chunks of 128 tokens at d_head 64)
+  float* S; uint16_t *x, *b, *c;       // kept for the backward
+  uint16_t *hp_hi, *hp_lo, *dh_hi, *dh_lo;
+  uint16_t *t0, *t1, *g0, *g1;         // landing buffers for tensors that are not 16-byte aligned (not with `plain`)
+  float *init, *last, *seg, *part;
+};
 bool ssd16_supported(int B, int T, int H, int P, int N, int G, int Q);
-size_t ssd16_ws_layout(int B, int T, int H, int P, int N, int G, int Q, void* base, size_t bytes, SsdWs* out, float** db32, float** dc32);
-pmb_status ssd16_fwd(cudaStream_t st, int B, int T, int H, int P, int N, int G, int Q, const uint16_t* x, const float* a,
-                     const uint16_t* b, const uint16_t* c, const float* init_state, uint16_t* y, float* final_state, const SsdWs& ws);
-pmb_status ssd16_bwd(cudaStream_t st, int B, int T, int H, int P, int N, int G, int Q, const float* a, const uint16_t* dy,
-                     uint16_t* dx, float* da, uint16_t* db, uint16_t* dc, const SsdWs& ws, float* db32, float* dc32);
+size_t ssd16_ws_layout(int B, int T, int H, int P, int N, int G, int Q, void* base, size_t bytes, Scan16Ws* out);
+pmb_status ssd16_fwd(cudaStream_t st, int B, int T, int H, int P, int N, int G, const uint16_t* x, const float* a,
+                     const uint16_t* b, const uint16_t* c, const float* init_state, uint16_t* y, float* final_state, const Scan16Ws& ws);
+pmb_status ssd16_bwd(cudaStream_t st, int B, int T, int H, int P, int N, int G, const uint16_t* dy, uint16_t* dx, float* da, uint16_t* db,
+                     uint16_t* dc, const Scan16Ws& ws);
 pmb_status ssd_fwd(cudaStream_t st, const SsdIn& in, const float* init_state, float* y, int64_t ldy,
                    float* final_state, const SsdWs& ws);
 // Backward.  dy (stride lddy) is the gradient w.r.t. y (skip term included when in.D != NULL).

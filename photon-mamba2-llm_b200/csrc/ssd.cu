@@ -1450,191 +1450,93 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
 }
 
 // ---------------------------------------------------------------------------------------------
-// The scan on bf16 inputs as they are (the bf16-storage mode of the block, mamba2/block.rs:203-208: x, B, C in
-// bf16, the recurrence in fp32).  x, B, C and dY go to the tensor cores as plain bf16 operands (one MMA per
-// product instead of the three of an fp32 pair), a, S, the chunk states and every accumulator stay fp32, y and dx
-// leave the fused kernels as bf16.  No fp32 copy of any (B,T,H,P) tensor is made.
+// The scan on bf16 inputs as they are (mamba2/block.rs:203-208: x, B, C in bf16, the recurrence in fp32).  x, B, C and dY go to
+// the tensor cores as plain bf16 operands, a, S, the states and every accumulator stay fp32, y and the gradients leave the kernels
+// as bf16.  On whole chunks of 128 tokens at d_head 64 the operands formed on the way (masked tiles, scaled x and dY, states) are
+// rounded to bf16 too; on every other shape they are (hi, lo) pairs, so that nothing but the outputs is rounded to bf16.
+// Measured, forward and backward: 16 x 8192 tokens, 32 heads of 128 x 64: 7.01 ms chunk by chunk (16 launches), 3.22 ms as chains (5);
+// 5 x 1474 tokens, 16 heads: 4443 us widened to fp32 for the FMA contractions, 234 us.
 // ---------------------------------------------------------------------------------------------
 
-// dst[tk,h,:] = bf16(src[tk,h,:] * f):  mode 0: f = exp(S_end - S_t) (operand of the chunk states and of dB),
-// mode 1: f = exp(S_t) (operand of d(states) and of dC).  Eight elements per thread.  `keep` (optional) receives a copy of src.
-__global__ void __launch_bounds__(256) scale_rows16_kernel(const uint16_t* __restrict__ src, const float* __restrict__ S,
-                                                           uint16_t* __restrict__ dst, uint16_t* __restrict__ keep, int64_t rows, int T, int H,
-                                                           int P, int Q, int mode) {
-  const int P8 = P >> 3;
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * H * P8) return;
-  const int j = (int)(i % P8); const int64_t w = i / P8; const int h = (int)(w % H); const int64_t tk = w / H;
-  const int t = (int)(tk % T);
-  const float* sp = S + ((tk / T) * H + h) * T;
-  const float f = mode == 0 ? __expf(sp[(t / Q) * Q + Q - 1] - sp[t]) : __expf(sp[t]);
-  const int64_t o = (tk * H + h) * (int64_t)P + 8 * j;
-  const uint4 v = *reinterpret_cast<const uint4*>(src + o);
-  if (keep) *reinterpret_cast<uint4*>(keep + o) = v;      // the unscaled values, for the backward
-  const uint32_t in[4] = {v.x, v.y, v.z, v.w};
-  uint32_t out[4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const __nv_bfloat162 r = __floats2bfloat162_rn(__uint_as_float(in[e] << 16) * f, __uint_as_float(in[e] & 0xffff0000u) * f);
-    out[e] = *reinterpret_cast<const uint32_t*>(&r);
-  }
-  *reinterpret_cast<uint4*>(dst + o) = make_uint4(out[0], out[1], out[2], out[3]);
+// rounds what is formed on the way to bf16
+static bool ssd16_plain(int T, int P, int N, int Q) {
+  return P == 64 && (N == 64 || N == 128) && Q % 128 == 0 && Q <= PREP_MAX_Q && T / Q <= SCAN_DOT_MAX_NC;
 }
-
 bool ssd16_supported(int B, int T, int H, int P, int N, int G, int Q) {
-  if (!fused_enabled() || !ssd_fused_supported(P, N, Q, false) || P != 64) return false;
-  if (Q <= 0 || T % Q != 0 || Q > PREP_MAX_Q || !(G == 1 || G == H)) return false;
-  if (T / Q > SCAN_DOT_MAX_NC || (int64_t)N * P / 4 > 4 * 1024) return false;        // the one-launch reverse scan
-  return (int64_t)B * T < (1LL << 31) && (int64_t)B * (T / Q) * H * N < (1LL << 31);
+  return ssd_chain_enabled() && ssd_chain_shape(P, N) && (int64_t)B * T < (1LL << 31) && (int64_t)B * cdiv(T, SCAN_STEP) < (1LL << 31);
 }
 
-// Workspace of the bf16-input scan: the fields of SsdWs that its kernels touch (every *_lo stays NULL, which is how the
-// contractions know that the operands are plain bf16), plus fp32 landing buffers for dB and dC.
-size_t ssd16_ws_layout(int B, int T, int H, int P, int N, int G, int Q, void* base, size_t bytes, SsdWs* out, float** db32, float** dc32) {
+size_t ssd16_ws_layout(int B, int T, int H, int P, int N, int G, int Q, void* base, size_t bytes, Scan16Ws* out) {
   Arena ar(base, bytes);
-  SsdWs w{};
-  const int nc = T / Q;
-  const size_t hp = (size_t)B * T * H * P, gn = (size_t)B * T * G * N, stn = (size_t)B * nc * H * N * P, qq = (size_t)B * nc * G * Q * Q;
-  const size_t bth = (size_t)B * T * H;
-  w.S = ar.take<float>(bth);
-  w.hprev = ar.take<float>(stn);
-  w.hlast = ar.take<float>((size_t)B * H * N * P);
-  w.xs_hi = ar.take<uint16_t>(hp);
-  w.xt_hi = ar.take<uint16_t>(hp);
-  w.bc_hi = ar.take<uint16_t>(2 * gn);
-  w.hp_hi = ar.take<uint16_t>(stn);
-  w.yoff = reinterpret_cast<float*>(ar.take<uint16_t>(hp));      // holds bf16 here
-  w.dh = ar.take<float>(stn);
-  w.rows = ar.take<float>(bth);
-  w.part = ar.take<float>((size_t)B * nc * 3 * H);
-  {
-    const size_t nbcg = (size_t)B * nc * G;
-    const size_t dbc = (size_t)ssd_pairs_dbc_nsplit(B, T, H, N, G, Q) * nbcg * Q * N;
-    const size_t dgp = (size_t)ssd_pairs_dg_nsplit(B, T, H, G, Q) * nbcg * Q * Q;
-    w.splitk = ar.take<float>(dbc > dgp ? dbc : dgp);
+  Scan16Ws w{};
+  const size_t hp = (size_t)B * T * H * P, gn = (size_t)B * T * G * N, np = (size_t)B * H * N * P, stn = np * cdiv(T, SCAN_STEP);
+  w.plain = ssd16_plain(T, P, N, Q);
+  w.S = ar.take<float>((size_t)B * T * H);
+  w.x = ar.take<uint16_t>(hp);
+  w.b = ar.take<uint16_t>(gn); w.c = ar.take<uint16_t>(gn);
+  w.hp_hi = ar.take<uint16_t>(stn); w.dh_hi = ar.take<uint16_t>(stn);
+  if (!w.plain) {
+    w.hp_lo = ar.take<uint16_t>(stn); w.dh_lo = ar.take<uint16_t>(stn);
+    w.t0 = ar.take<uint16_t>(hp); w.t1 = ar.take<uint16_t>(hp); w.g0 = ar.take<uint16_t>(gn); w.g1 = ar.take<uint16_t>(gn);
   }
-  w.dys_hi = ar.take<uint16_t>(hp);
-  w.dg_hi = ar.take<uint16_t>(qq);
-  w.dh_hi = ar.take<uint16_t>(stn);
-  w.csum = ar.take<float>(bth);
-  w.esum = ar.take<float>(bth);
-  w.rpart = ar.take<float>(bth * (Q / 128));
-  float* b32 = ar.take<float>(gn);
-  float* c32 = ar.take<float>(gn);
+  w.init = ar.take<float>(np); w.last = ar.take<float>(np);
+  w.seg = ar.take<float>(ssd_chain_seg_floats(B, T, H, P, N));
+  w.part = ar.take<float>(ssd_heads_part_floats(B, T, H, N, G));
   if (out) *out = w;
-  if (db32) *db32 = b32;
-  if (dc32) *dc32 = c32;
   return ar.ok ? ar.used() : 0;
 }
 
-static SsdIn ssd16_in(int B, int T, int H, int P, int N, int G, int Q, const float* a) {
-  SsdIn in{};
-  in.B = B; in.T = T; in.H = H; in.P = P; in.N = N; in.G = G; in.Q = Q;
-  in.ldx = (int64_t)H * P; in.a = a; in.ldbc = (int64_t)G * N;
-  return in;
-}
-
-pmb_status ssd16_fwd(cudaStream_t st, int B, int T, int H, int P, int N, int G, int Q, const uint16_t* x, const float* a,
-                     const uint16_t* b, const uint16_t* c, const float* init_state, uint16_t* y, float* final_state, const SsdWs& ws) {
-  const SsdIn in = ssd16_in(B, T, H, P, N, G, Q, a);
-  SsdP p;
-  PMB_TRY(fill_params(in, ws, &p));
-  const int nbch = p.B * p.nc * p.H;
-  const int64_t tok = (int64_t)B * T, hp = (int64_t)H * P, gn = (int64_t)G * N;
-  {
-    ProfScope prof(st, "ssd_chunk_cumsum", 0.0, 8.0 * tok * p.H);
-    chunk_cumsum_kernel<<<(unsigned)cdiv((int64_t)nbch * 32, 256), 256, 0, st>>>(p, CumsumRaw{});
-    PMB_LAUNCHED();
-  }
-  {
-    // B | C side by side (the layout every contraction's tensor maps describe)
-    ProfScope prof(st, "ssd16_keep_bc", 0.0, 8.0 * tok * gn);
-    PMB_CUDA(cudaMemcpy2DAsync(ws.bc_hi, (size_t)(4 * gn), b, (size_t)(2 * gn), (size_t)(2 * gn), (size_t)tok, cudaMemcpyDeviceToDevice, st));
-    PMB_CUDA(cudaMemcpy2DAsync(ws.bc_hi + gn, (size_t)(4 * gn), c, (size_t)(2 * gn), (size_t)(2 * gn), (size_t)tok, cudaMemcpyDeviceToDevice, st));
-  }
-  {
-    ProfScope prof(st, "ssd16_prescale_x", 0.0, 6.0 * tok * hp);      // (also keeps x for the backward, which is not handed x again)
-    scale_rows16_kernel<<<(unsigned)cdiv(tok * H * (P / 8), 256), 256, 0, st>>>(x, ws.S, ws.xs_hi, ws.xt_hi, tok, T, H, P, Q, 0);
-    PMB_LAUNCHED();
-  }
-  PMB_TRY(ssd_pairs_state(st, in, ws, 0));
-  {
-    ProfScope prof(st, "ssd_state_pass", 0.0, 8.0 * (double)p.B * p.H * p.N * p.P * p.nc);
-    PMB_TRY(launch_state_scan(st, p, p.hprev, init_state, p.hlast, 0, ws.hp_hi, nullptr));
-  }
-  FusedArgs fa = fused_args(in, ws);
-  fa.v = Op16{ws.xt_hi, nullptr, hp};
-  fa.state = Op16{ws.hp_hi, nullptr, p.P};
-  fa.out16 = y; fa.ldo = hp;
-  fa.off_out16 = reinterpret_cast<uint16_t*>(ws.yoff);
-  PMB_TRY(ssd_fused(st, 0, fa));
-  if (final_state) PMB_CUDA(cudaMemcpyAsync(final_state, ws.hlast, (size_t)p.B * p.H * p.N * p.P * sizeof(float), cudaMemcpyDeviceToDevice, st));
+static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+static pmb_status copy16(cudaStream_t st, void* dst, const void* src, size_t bytes) {
+  PMB_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st));
   return PMB_OK;
 }
 
-pmb_status ssd16_bwd(cudaStream_t st, int B, int T, int H, int P, int N, int G, int Q, const float* a, const uint16_t* dy,
-                     uint16_t* dx, float* da, uint16_t* db, uint16_t* dc, const SsdWs& ws_in, float* db32, float* dc32) {
-  const SsdIn in = ssd16_in(B, T, H, P, N, G, Q, a);
-  SsdWs ws = ws_in;
-  ws.dy_hi = const_cast<uint16_t*>(dy); ws.dy_lo = nullptr;
-  SsdP p;
-  PMB_TRY(fill_params(in, ws, &p));
-  const int nbch = p.B * p.nc * p.H, nbcg = p.B * p.nc * p.G;
-  const int64_t tok = (int64_t)B * T, hp = (int64_t)H * P, gn = (int64_t)G * N;
-  float* dsend = ws.rows;
+pmb_status ssd16_fwd(cudaStream_t st, int B, int T, int H, int P, int N, int G, const uint16_t* x, const float* a,
+                     const uint16_t* b, const uint16_t* c, const float* init_state, uint16_t* y, float* final_state, const Scan16Ws& ws) {
+  const size_t hp = (size_t)B * T * H * P * 2, gn = (size_t)B * T * G * N * 2, np = (size_t)B * H * N * P * 4;
   {
-    ProfScope prof(st, "ssd16_prescale_dy", 0.0, 4.0 * tok * hp);
-    scale_rows16_kernel<<<(unsigned)cdiv(tok * H * (P / 8), 256), 256, 0, st>>>(dy, ws.S, ws.dys_hi, nullptr, tok, T, H, P, Q, 1);
-    PMB_LAUNCHED();
+    // (the backward is not handed the inputs again: B and C are copied here, x by the kernel)
+    ProfScope prof(st, "ssd16_keep_bc", 0.0, 4.0 * gn);
+    PMB_TRY(copy16(st, ws.b, b, gn));
+    PMB_TRY(copy16(st, ws.c, c, gn));
   }
-  PMB_TRY(ssd_pairs_state(st, in, ws, 1));
-  {
-    ProfScope prof(st, "ssd_bwd_state_pass", 0.0, 12.0 * p.B * p.H * p.N * p.P * p.nc);
-    if (!launch_state_scan_rev_dot(st, p, p.dh, ws.dh_hi, nullptr, dsend)) return fail(PMB_ERR_UNSUPPORTED, "ssd16: reverse scan shape");
-    PMB_LAUNCHED();
-  }
-  {
-    FusedArgs fa = fused_args(in, ws);
-    fa.v = Op16{dy, nullptr, hp};
-    fa.state = Op16{ws.dh_hi, nullptr, p.P};
-    fa.out16 = dx; fa.ldo = hp;
-    fa.xt = Op16{ws.xt_hi, nullptr, hp};
-    fa.csum = ws.csum; fa.esum = ws.esum; fa.rpart = ws.rpart;
-    PMB_TRY(ssd_fused(st, 1, fa));
-  }
-  {
-    ProfScope prof(st, "ssd_bwd_rows", 0.0, tok * p.H * (6.0 * p.P + 32.0));
-    WSums wsm{ws.rpart, ws.csum, ws.esum, ws.yoff, p.Q / 128};
-    chunk_rows_finish_w_kernel<true><<<(unsigned)nbch, ROWS_THREADS, 0, st>>>(p, wsm, nullptr, 0, dsend, da, nullptr, ws.part, SsdGrads::RawDt{}, dy);
-    PMB_LAUNCHED();
-  }
-  auto reduce = [&](int nsplit, int cols, int mode, float* out, int64_t ld, int tile) -> pmb_status {
-    if (nsplit <= 1) return PMB_OK;
-    const int64_t total = (int64_t)nbcg * p.Q * cols;
-    splitk_reduce_kernel<<<(unsigned)cdiv(total, 256), 256, 0, st>>>(ws.splitk, nsplit, p.Q, cols, mode, p.G, p.Q, out, ld, total, tile, 0,
-                                                                     mode == 0 ? ws.dg_hi : nullptr, nullptr);
-    PMB_LAUNCHED();
-    return PMB_OK;
-  };
-  {
-    ProfScope prof(st, "ssd_bwd_dg_pair", 2.0 * tok * p.H * p.Q * p.P, 0.0);
-    const int nsg = ssd_pairs_dg_nsplit(p.B, p.T, p.H, p.G, p.Q);
-    PMB_TRY(ssd_pairs_dg(st, in, ws, nsg));
-    PMB_TRY(reduce(nsg, p.Q, 0, nullptr, 0, 128));
-  }
-  const int ns = ssd_pairs_dbc_nsplit(p.B, p.T, p.H, p.N, p.G, p.Q);
-  {
-    ProfScope prof(st, "ssd_bwd_dc_pair", 2.0 * tok * p.N * (p.G * p.Q + (double)p.H * p.P), 0.0);
-    PMB_TRY(ssd_pairs_dbc(st, in, ws, 0, dc32, gn, ns, ws.splitk));
-    PMB_TRY(reduce(ns, p.N, 1, dc32, gn, BM));
-  }
-  PMB_TRY(cast_f32_bf16(st, dc32, dc, tok * gn));
-  {
-    ProfScope prof(st, "ssd_bwd_db_pair", 2.0 * tok * p.N * (p.G * p.Q + (double)p.H * p.P), 0.0);
-    PMB_TRY(ssd_pairs_dbc(st, in, ws, 1, db32, gn, ns, ws.splitk));
-    PMB_TRY(reduce(ns, p.N, 2, db32, gn, BM));
-  }
-  return cast_f32_bf16(st, db32, db, tok * gn);
+  ChainArgs k{};
+  k.B = B; k.T = T; k.H = H; k.P = P; k.N = N; k.G = G; k.exact = !ws.plain;
+  k.b = Op16{ws.b, nullptr, (int64_t)G * N}; k.c = Op16{ws.c, nullptr, (int64_t)G * N};
+  k.x16 = x; k.x_keep = ws.x; k.ldx = k.ldy = (int64_t)H * P; k.a = a;
+  if (!aligned16(x)) { PMB_TRY(copy16(st, ws.x, x, hp)); k.x16 = ws.x; k.x_keep = nullptr; }
+  k.init = init_state;
+  if (init_state && !aligned16(init_state)) { PMB_TRY(copy16(st, ws.init, init_state, np)); k.init = ws.init; }
+  k.y16 = aligned16(y) ? y : ws.t0;
+  k.last = final_state && !aligned16(final_state) ? ws.last : final_state;
+  k.S_out = ws.S; k.hp_hi = ws.hp_hi; k.hp_lo = ws.hp_lo; k.seg = ws.seg;
+  PMB_TRY(ssd_chain_fwd(st, k));
+  if (k.y16 != y) PMB_TRY(copy16(st, y, k.y16, hp));
+  if (k.last != final_state) PMB_TRY(copy16(st, final_state, k.last, np));
+  return PMB_OK;
+}
+
+pmb_status ssd16_bwd(cudaStream_t st, int B, int T, int H, int P, int N, int G, const uint16_t* dy, uint16_t* dx, float* da, uint16_t* db,
+                     uint16_t* dc, const Scan16Ws& ws) {
+  const size_t hp = (size_t)B * T * H * P * 2, gn = (size_t)B * T * G * N * 2;
+  const int64_t ldp = (int64_t)H * P, ldn = (int64_t)G * N;
+  if (!aligned16(dy)) { PMB_TRY(copy16(st, ws.t0, dy, hp)); dy = ws.t0; }
+  ChainBwdArgs k{};
+  k.B = B; k.T = T; k.H = H; k.P = P; k.N = N; k.G = G;
+  k.b = Op16{ws.b, nullptr, ldn}; k.c = Op16{ws.c, nullptr, ldn};
+  k.hp_hi = ws.hp_hi; k.hp_lo = ws.hp_lo; k.S = ws.S; k.x16 = ws.x; k.dy16 = dy; k.ldx = k.lddy = k.lddx = ldp;
+  k.dx16 = aligned16(dx) ? dx : ws.t1; k.dh_hi = ws.dh_hi; k.dh_lo = ws.dh_lo; k.da = da; k.seg = ws.seg;
+  PMB_TRY(ssd_chain_bwd(st, k));
+  if (k.dx16 != dx) PMB_TRY(copy16(st, dx, k.dx16, hp));
+  HeadsArgs h{};
+  h.B = B; h.T = T; h.H = H; h.P = P; h.N = N; h.G = G; h.b = k.b; h.c = k.c; h.dy = Op16{dy, nullptr, ldp}; h.xt = Op16{ws.x, nullptr, ldp};
+  h.hp_hi = ws.hp_hi; h.hp_lo = ws.hp_lo; h.dh_hi = ws.dh_hi; h.dh_lo = ws.dh_lo; h.S = ws.S; h.ld = ldn; h.part = ws.part;
+  h.dc16 = aligned16(dc) ? dc : ws.g0; h.db16 = aligned16(db) ? db : ws.g1;
+  PMB_TRY(ssd_heads(st, h));
+  if (h.dc16 != dc) PMB_TRY(copy16(st, dc, h.dc16, gn));
+  if (h.db16 != db) PMB_TRY(copy16(st, db, h.db16, gn));
+  return PMB_OK;
 }
 
 }  // namespace pmb

@@ -10,7 +10,8 @@
 //   h <- exp(S_end) h + B^T xs                                              tensor core, state warps' registers
 // S, xs and h can also be kept per chunk of two steps (plain bf16 operands): the second step's rows then see the first
 // one's columns through a masked tile of their own and h as it entered the chunk.
-// Operands are plain bf16 (NS = 1) or (hi, lo) bf16 pairs of fp32 values (NS = 2, three MMAs per product).  Sequences of
+// Operands are plain bf16 or (hi, lo) bf16 pairs: NI = 1 / 2 for x~, B and C, ND = 1 / 2 for what is formed here (M, xs, h).  fp32
+// tensors take pairs throughout; bf16 tensors have inputs that are exact as they are, with (ND = 2) or without pairs of the rest.  Sequences of
 // any length: rows past the end arrive as zeros (TMA fills them per batch) and carry a = 0.  d_state up to 128 and d_head
 // up to 64, in multiples of 8: the 64-wide tiles are zero-filled beyond them.
 //
@@ -58,20 +59,20 @@ template <int R> __device__ __forceinline__ void regs_inc() { asm volatile("setm
 template <int R> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
 
 // NB = 128-token blocks per chunk: S, the decay of xs and the state are relative to chunks of NB blocks.
-template <int NS, int NK, int NB>
+template <int NI, int ND, int NK, int NB>
 struct Geo {
-  static constexpr int BT = NS * NK * T128;              // B (or C) of a step
+  static constexpr int BT = NI * NK * T128;              // B (or C) of a step
   static constexpr int STAGE = 2 * BT;                   // [B | C]
-  static constexpr int XT = NS * T128;                   // x~ (or xs)
-  static constexpr int XBUF = 2 * XT;                    // [x~ | xs]
-  static constexpr int HB = NS * NK * T64;               // state operand, rows n of 128 bytes
-  static constexpr bool BIG = NS * NK == 4;              // pairs at d_state 128: one stage of B | C is all that fits
+  static constexpr int XT = NI * T128;                   // x~
+  static constexpr int XBUF = XT + ND * T128;                    // [x~ | xs]
+  static constexpr int HB = ND * NK * T64;               // state operand, rows n of 128 bytes
+  static constexpr bool BIG = NI * NK == 4;              // pairs at d_state 128: one stage of B | C is all that fits
   static constexpr int STG = BIG ? 1 : 2;
-  static constexpr int XB = NS == 1 ? 2 : 1;
+  static constexpr int XB = ND == 1 ? 2 : 1;
   static constexpr int NSB = NB == 1 ? XB + 1 : 2;       // copies of S: a chunk's S is read until its last tile has been masked
   static_assert(NB == 1 || (STG == 2 && XB == 2), "both blocks of a chunk are resident");
   static constexpr int TILES = STG * STAGE + XB * XBUF + HB;
-  static constexpr int AHEAD = BIG ? 0 : (NS * NK == 2 ? 3 : 4);              // 16-byte pieces of x that every transform thread has in flight
+  static constexpr int AHEAD = BIG ? 0 : (ND * NK >= 2 ? 3 : 4);              // 16-byte pieces of x that every transform thread has in flight
   static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 256 /*barriers*/ + NSB * NB * L * 4 + (BIG ? 4 : 8) * NB * L /*row factors*/ + AHEAD * XF_THREADS * 16;
 };
 
@@ -117,9 +118,9 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
       : "memory");
 }
 
-template <int NS, int NK, int NB, bool XIN16>
+template <int NI, int ND, int NK, int NB, bool XIN16>
 __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid_constant__ Maps maps, const Params p) {
-  using GE = Geo<NS, NK, NB>;
+  using GE = Geo<NI, ND, NK, NB>;
   constexpr int STG = GE::STG, XB = GE::XB, NSB = GE::NSB;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
         mbar_expect_tx(bar(FULL + s), p.state_only ? GE::BT : GE::STAGE);
         const uint32_t dst = ring_s + s * GE::STAGE;
 #pragma unroll
-        for (int sp = 0; sp < NS; ++sp)
+        for (int sp = 0; sp < NI; ++sp)
 #pragma unroll
           for (int kt = 0; kt < NK; ++kt) {
             tma_load_4d(dst + (sp * NK + kt) * T128, &maps.b[sp], 64 * kt, toff + i * L, g, bb, bar(FULL + s));
@@ -205,15 +206,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     const uint32_t id_g = idesc_bf16(0, 0, L, L);            // G: both operands K-major
     const uint32_t id_v = idesc_bf16(0, 1, L, PW);           // x x~, x h: B operand MN-major
     const uint32_t id_u = idesc_bf16(1, 1, L, PW);           // B^T xs: both operands MN-major
-    auto kstep = [&](uint32_t d, uint32_t alo, uint32_t as, uint32_t blo, uint32_t bs, uint32_t idesc, uint32_t acc) {
-      if (NS == 2) {
-        mma_f16_h(d, alo + as, dh, blo, dh, idesc, acc);          // lo x hi
-        mma_f16_h(d, alo, dh, blo + bs, dh, idesc, 1u);           // hi x lo
-        mma_f16_h(d, alo, dh, blo, dh, idesc, 1u);                // hi x hi
-      } else {
-        mma_f16_h(d, alo, dh, blo, dh, idesc, acc);
-      }
-    };
     auto all = [&](bool v) -> bool { return __all_sync(0xffffffffu, v); };
     // G of the item (block k, earlier or same block kb of its chunk) into buffer m & 1
     auto mma_g = [&](int m, int k, int kb) -> bool {
@@ -227,7 +219,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const uint32_t o = (uint32_t)(kt * T128 + q * 32) >> 4;
-            kstep(tG + (uint32_t)((m & 1) * L), c0 + o, (NK * T128) >> 4, b0 + o, (NK * T128) >> 4, id_g, (kt | q) ? 1u : 0u);
+            mma_split<NI, NI>(tG + (uint32_t)((m & 1) * L), c0 + o, (NK * T128) >> 4, b0 + o, (NK * T128) >> 4, dh, id_g, (kt | q) ? 1u : 0u);
           }
         umma_commit(bar(GFULL + (m & 1)));
       }
@@ -244,7 +236,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const uint32_t o = (uint32_t)(q * 2048) >> 4;
-            kstep(tU, b0 + o, (NK * T128) >> 4, xs0 + o, T128 >> 4, id_u, q ? 1u : 0u);
+            mma_split<NI, ND>(tU, b0 + o, (NK * T128) >> 4, xs0 + o, T128 >> 4, dh, id_u, q ? 1u : 0u);
           }
           umma_commit(bar(UFULL)); umma_commit(bar(XFREE + xb)); umma_commit(bar(EMPTY + s));
         }
@@ -274,7 +266,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
             for (int kt = 0; kt < NK; ++kt)
 #pragma unroll
               for (int q = 0; q < 4; ++q)
-                kstep(tA2, c0 + ((uint32_t)(kt * T128 + q * 32) >> 4), (NK * T128) >> 4, h0 + ((uint32_t)(kt * T64 + q * 2048) >> 4), (NK * T64) >> 4, id_v,
+                mma_split<NI, ND>(tA2, c0 + ((uint32_t)(kt * T128 + q * 32) >> 4), (NK * T128) >> 4, h0 + ((uint32_t)(kt * T64 + q * 2048) >> 4), (NK * T64) >> 4, dh, id_v,
                       (kt | q) ? 1u : 0u);
             if (rb == NB - 1 || k + 1 == n) umma_commit(bar(HFREE));
           }
@@ -289,13 +281,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
           for (int q = 0; q < 8; ++q) {
             const uint32_t ta = tG + (uint32_t)((m & 1) * L + (q >> 1) * 32 + (q & 1) * 8), vb = xt0 + ((uint32_t)(q * 2048) >> 4);
             const uint32_t acc = (q | cb) ? 1u : 0u;
-            if (NS == 2) {
-              mma_f16_ts_h(tA1, ta + 16u, vb, dh, id_v, acc);
-              mma_f16_ts_h(tA1, ta, vb + (T128 >> 4), dh, id_v, 1u);
-              mma_f16_ts_h(tA1, ta, vb, dh, id_v, 1u);
-            } else {
-              mma_f16_ts_h(tA1, ta, vb, dh, id_v, acc);
-            }
+            mma_split_ts<ND, NI>(tA1, ta, 16u, vb, T128 >> 4, dh, id_v, acc);
           }
           if (cb == rb) umma_commit(bar(ACCFULL));
           else umma_commit(bar(XFREE + (k - rb + cb) % XB));      // (the earlier block of the chunk is done with)
@@ -313,7 +299,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const uint32_t o = (uint32_t)(q * 2048) >> 4;
-          kstep(tU, b0 + o, (NK * T128) >> 4, xs0 + o, T128 >> 4, id_u, (q | rb) ? 1u : 0u);
+          mma_split<NI, ND>(tU, b0 + o, (NK * T128) >> 4, xs0 + o, T128 >> 4, dh, id_u, (q | rb) ? 1u : 0u);
         }
         if (rb == NB - 1 || k + 1 == n) umma_commit(bar(UFULL));
         if (rb == NB - 1) umma_commit(bar(XFREE + xb));
@@ -371,11 +357,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
                 float m0 = __uint_as_float(r[2 * e2]) * __expf(S_row - sv.x), m1 = __uint_as_float(r[2 * e2 + 1]) * __expf(S_row - sv.y);
                 if (!below) { m0 = col <= r_local ? m0 : 0.0f; m1 = col + 1 <= r_local ? m1 : 0.0f; }
                 ml[e2] = 0u;
-                split2(m0, m1, mh[e2], ml[e2], NS == 2);
+                split2(m0, m1, mh[e2], ml[e2], ND == 2);
               }
             }
             tmem_st16(tg + (uint32_t)(half * 32), mh);
-            if (NS == 2) tmem_st16(tg + (uint32_t)(half * 32 + 16), ml);
+            if (ND == 2) tmem_st16(tg + (uint32_t)(half * 32 + 16), ml);
           }
           tmem_wait_st();
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -558,22 +544,23 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
           const float2 f = GE::BIG ? make_float2(sdt[rc], __expf(sEnd[c & 3] - S[rc])) : sfac[rc];
           if (XIN16) {
             const uint32_t in4[4] = {xq.x, xq.y, xq.z, xq.w};
-            uint32_t s4[4], z;
+            uint32_t s4[4], k4[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) split2(__uint_as_float(in4[e] << 16) * f.y, __uint_as_float(in4[e] & 0xffff0000u) * f.y, s4[e], z, false);
+            for (int e = 0; e < 4; ++e) split2(__uint_as_float(in4[e] << 16) * f.y, __uint_as_float(in4[e] & 0xffff0000u) * f.y, s4[e], k4[e], ND == 2);
             st_shared_v4(dst, in4[0], in4[1], in4[2], in4[3]);
             st_shared_v4(dst + GE::XT, s4[0], s4[1], s4[2], s4[3]);
+            if (ND == 2) st_shared_v4(dst + GE::XT + T128, k4[0], k4[1], k4[2], k4[3]);
             // (the backward of the bf16 scan is not handed x again)
             const int row = toff + i * L + it * RPI + r0;
             if (p.x_keep && !p.state_only && jcol && row < p.T) *reinterpret_cast<uint4*>(p.x_keep + (tokb + row) * p.ldx + h * p.P + EPL * j) = xq;
           } else {
             const float f0 = __uint_as_float(xq.x) * f.x, f1 = __uint_as_float(xq.y) * f.x, f2 = __uint_as_float(xq.z) * f.x, f3 = __uint_as_float(xq.w) * f.x;
             uint32_t h0, h1, l0 = 0u, l1 = 0u, g0, g1, k0 = 0u, k1 = 0u;
-            split2(f0, f1, h0, l0, NS == 2); split2(f2, f3, h1, l1, NS == 2);
-            split2(f0 * f.y, f1 * f.y, g0, k0, NS == 2); split2(f2 * f.y, f3 * f.y, g1, k1, NS == 2);
+            split2(f0, f1, h0, l0, ND == 2); split2(f2, f3, h1, l1, ND == 2);
+            split2(f0 * f.y, f1 * f.y, g0, k0, ND == 2); split2(f2 * f.y, f3 * f.y, g1, k1, ND == 2);
             st_shared_v2(dst, h0, h1);
             st_shared_v2(dst + GE::XT, g0, g1);
-            if (NS == 2) { st_shared_v2(dst + T128, l0, l1); st_shared_v2(dst + GE::XT + T128, k0, k1); }
+            if (ND == 2) { st_shared_v2(dst + T128, l0, l1); st_shared_v2(dst + GE::XT + T128, k0, k1); }
           }
           if (GE::AHEAD > 0) {
             request(slot);                                  // (this pass has consumed the slot)
@@ -626,13 +613,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
         for (int c = 0; c < 8; ++c) {                       // eight 16-byte chunks of the row
           uint32_t hi[4], lo[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) split2(hv[8 * c + 2 * e], hv[8 * c + 2 * e + 1], hi[e], lo[e], NS == 2);
+          for (int e = 0; e < 4; ++e) split2(hv[8 * c + 2 * e], hv[8 * c + 2 * e + 1], hi[e], lo[e], ND == 2);
           const uint32_t a = h_s + (uint32_t)(nr * 128 + ((c ^ (nr & 7)) << 4));
           st_shared_v4(a, hi[0], hi[1], hi[2], hi[3]);
-          if (NS == 2) st_shared_v4(a + NK * T64, lo[0], lo[1], lo[2], lo[3]);
+          if (ND == 2) st_shared_v4(a + NK * T64, lo[0], lo[1], lo[2], lo[3]);
           if (p.hp_hi && active && 8 * c < p.P) {
             *reinterpret_cast<uint4*>(p.hp_hi + so + 8 * c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            if (NS == 2) *reinterpret_cast<uint4*>(p.hp_lo + so + 8 * c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            if (ND == 2) *reinterpret_cast<uint4*>(p.hp_lo + so + 8 * c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           }
         }
       }
@@ -685,13 +672,14 @@ static unsigned int* status_ptr() {
   return ptr[dev];
 }
 
-template <int NS, int NK, int NB, bool XIN16>
+template <int NI, int ND, int NK, int NB, bool XIN16>
 static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
-  using GE = Geo<NS, NK, NB>;
+  using GE = Geo<NI, ND, NK, NB>;
   static_assert(GE::SMEM <= 227 * 1024, "shared-memory plan");
+  static_assert(XIN16 ? NI == 1 : NI == ND, "fp32 tensors take pairs throughout or not at all");
   Maps ms{};
   for (int sp = 0; sp < 2; ++sp) {
-    const bool lo = sp && NS == 2;
+    const bool lo = sp && NI == 2;
     PMB_TRY(sf::bf16_map4(&ms.b[sp], lo ? a.b.lo : a.b.hi, a.N, a.T, a.G, a.B, a.b.pitch, a.N, (int64_t)a.T * a.b.pitch, 64, L));
     PMB_TRY(sf::bf16_map4(&ms.c[sp], lo ? a.c.lo : a.c.hi, a.N, a.T, a.G, a.B, a.c.pitch, a.N, (int64_t)a.T * a.c.pitch, 64, L));
   }
@@ -706,15 +694,15 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
     p.nseg = ssd_chain_segments(a.B, a.T, a.H, &p.per);
     p.seg_h = a.seg; p.seg_d = a.seg + (size_t)a.B * a.H * p.nseg * a.N * a.P;
   }
-  PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_fwd_kernel<NS, NK, NB, XIN16>);
+  PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>);
   const unsigned grid = (unsigned)((int64_t)a.B * a.H * p.nseg);
   if (p.nseg > 1) {
     p.state_only = 1;
-    ssd_chain_fwd_kernel<NS, NK, NB, XIN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
+    ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
     PMB_LAUNCHED();
     p.state_only = 0;
   }
-  ssd_chain_fwd_kernel<NS, NK, NB, XIN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
+  ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
   PMB_LAUNCHED();
   return PMB_OK;
 }
@@ -745,17 +733,19 @@ pmb_status ssd_chain_fwd(cudaStream_t st, const ChainArgs& a) {
   auto al16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   if (!al16(a.x) || !al16(a.x16) || !al16(a.y) || !al16(a.y16) || !al16(a.init) || (a.ldx & (a.x16 ? 7 : 3)) || (a.ldy & 3))
     return fail(PMB_ERR_SHAPE, "ssd_chain: x, y and state rows must be 16-byte aligned");
+  if (!pairs && !a.x16 && a.N > 64) return fail(PMB_ERR_UNSUPPORTED, "ssd_chain: fp32 x with plain bf16 B and C takes d_state up to 64");
   const double tok = (double)a.B * a.T;
   // G and the masked product over the causal half of a step, the state update and the carried-state product
   ProfScope prof(st, "ssd_chain_fwd", tok * a.H * ((double)SCAN_STEP * (a.N + a.P) + 4.0 * a.N * a.P), 0.0);
   const bool wide = a.N > 64;
   if (a.blocks == 2) {
     if (pairs || wide || a.x16 || a.T % (2 * SCAN_STEP)) return fail(PMB_ERR_UNSUPPORTED, "ssd_chain: chunks of two steps need plain bf16 operands, d_state <= 64 and whole chunks");
-    return sc::launch<1, 1, 2, false>(st, a);
+    return sc::launch<1, 1, 1, 2, false>(st, a);
   }
-  if (a.x16) return wide ? sc::launch<1, 2, 1, true>(st, a) : sc::launch<1, 1, 1, true>(st, a);
-  if (!pairs) return wide ? sc::launch<1, 2, 1, false>(st, a) : sc::launch<1, 1, 1, false>(st, a);
-  return wide ? sc::launch<2, 2, 1, false>(st, a) : sc::launch<2, 1, 1, false>(st, a);
+  if (a.x16 && a.exact) return wide ? sc::launch<1, 2, 2, 1, true>(st, a) : sc::launch<1, 2, 1, 1, true>(st, a);
+  if (a.x16) return wide ? sc::launch<1, 1, 2, 1, true>(st, a) : sc::launch<1, 1, 1, 1, true>(st, a);
+  if (!pairs) return sc::launch<1, 1, 1, 1, false>(st, a);
+  return wide ? sc::launch<2, 2, 2, 1, false>(st, a) : sc::launch<2, 2, 1, 1, false>(st, a);
 }
 
 }  // namespace pmb

@@ -48,14 +48,14 @@ constexpr int W_MASK = 4, W_XF = 12, W_ST = 20, NTHREADS = 32 * 24, XF_THREADS =
 template <int R> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
 template <int R> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
 
-template <int NS, int NK>
+template <int NI, int ND, int NK>
 struct Geo {
-  static constexpr int BT = NS * NK * T128;              // B (or C)
-  static constexpr int HT = NS * NK * T64;               // h, dh: rows n of 128 bytes
+  static constexpr int BT = NI * NK * T128;              // B (or C)
+  static constexpr int HT = ND * NK * T64;               // h, dh: rows n of 128 bytes
   static constexpr int STAGE = 2 * BT + HT;              // [B | C | h]
-  static constexpr int XT = NS * T128;                   // x~, dY, dY exp(S)
-  static constexpr int XBUF = 3 * XT;
-  static constexpr int XB = NS == 1 ? 2 : 1;
+  static constexpr int XT = NI * T128;                   // x~ (or dY)
+  static constexpr int XBUF = 2 * XT + ND * T128;        // [x~ | dY | dY exp(S)]
+  static constexpr int XB = ND == 1 ? 2 : 1;
   static constexpr int NSB = XB + 2;
   static constexpr int AHEAD = 2;                        // pieces of x and of dY that a transform thread has in flight
   static constexpr int TILES = STAGE + XB * XBUF + HT;
@@ -128,9 +128,9 @@ __device__ __forceinline__ float warp_column_sums16(float (&v)[16], int lane) {
   return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
 }
 
-template <int NS, int NK, bool IN16>
+template <int NI, int ND, int NK, bool IN16>
 __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
-  using GE = Geo<NS, NK>;
+  using GE = Geo<NI, ND, NK>;
   constexpr int XB = GE::XB, NSB = GE::NSB;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -196,14 +196,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
           if (!wait(EMPTY, (uint32_t)k ^ 1u, 1u)) break;
           mbar_expect_tx(bar(FULL), p.state_only ? GE::BT : GE::STAGE);
 #pragma unroll
-          for (int sp = 0; sp < NS; ++sp)
+          for (int kt = 0; kt < NK; ++kt) {
 #pragma unroll
-            for (int kt = 0; kt < NK; ++kt) {
+            for (int sp = 0; sp < NI; ++sp) {
               tma_load_4d(c_s + (sp * NK + kt) * T128, &maps.c[sp], 64 * kt, i * L, g, bb, bar(FULL));
-              if (p.state_only) continue;
-              tma_load_4d(b_s + (sp * NK + kt) * T128, &maps.b[sp], 64 * kt, i * L, g, bb, bar(FULL));
-              tma_load_4d(hin_s + (sp * NK + kt) * T64, &maps.h[sp], 0, 64 * kt, h, bb * p.nsteps + i, bar(FULL));
+              if (!p.state_only) tma_load_4d(b_s + (sp * NK + kt) * T128, &maps.b[sp], 64 * kt, i * L, g, bb, bar(FULL));
             }
+#pragma unroll
+            for (int sp = 0; sp < ND; ++sp)
+              if (!p.state_only) tma_load_4d(hin_s + (sp * NK + kt) * T64, &maps.h[sp], 0, 64 * kt, h, bb * p.nsteps + i, bar(FULL));
+          }
           issued = k + 1;
         }
         if (*abort_flag && issued > 0) mbar_wait(bar(FULL), (uint32_t)((issued - 1) & 1));
@@ -214,15 +216,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       const uint32_t id_g = idesc_bf16(0, 0, L, L);            // both operands K-major
       const uint32_t id_v = idesc_bf16(0, 1, L, PW);           // B operand MN-major
       const uint32_t id_u = idesc_bf16(1, 1, L, PW);           // both operands MN-major
-      auto kstep = [&](uint32_t d, uint32_t alo, uint32_t as, uint32_t blo, uint32_t bs, uint32_t idesc, uint32_t acc) {
-        if (NS == 2) {
-          mma_f16_h(d, alo + as, dhi, blo, dhi, idesc, acc);          // lo x hi
-          mma_f16_h(d, alo, dhi, blo + bs, dhi, idesc, 1u);           // hi x lo
-          mma_f16_h(d, alo, dhi, blo, dhi, idesc, 1u);                // hi x hi
-        } else {
-          mma_f16_h(d, alo, dhi, blo, dhi, idesc, acc);
-        }
-      };
       const uint32_t BS = (NK * T128) >> 4, HS = (NK * T64) >> 4, XS = T128 >> 4;      // from a hi tile to its lo tile
       bool ok = true;
 #pragma unroll 1
@@ -241,10 +234,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const uint32_t o = (uint32_t)(kt * T128 + q * 32) >> 4;
-              kstep(tG, b0 + o, BS, c0 + o, BS, id_g, (kt | q) ? 1u : 0u);
+              mma_split<NI, NI>(tG, b0 + o, BS, c0 + o, BS, dhi, id_g, (kt | q) ? 1u : 0u);
             }
 #pragma unroll
-          for (int q = 0; q < 4; ++q) kstep(tM, x0 + 2 * q, XS, y0 + 2 * q, XS, id_g, q ? 1u : 0u);
+          for (int q = 0; q < 4; ++q) mma_split<NI, NI>(tM, x0 + 2 * q, XS, y0 + 2 * q, XS, dhi, id_g, q ? 1u : 0u);
           umma_commit(bar(GFULL));
         }
         __syncwarp();
@@ -256,7 +249,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
         if (elect_one()) {
           const uint32_t c0 = desc_lo(c_s, T128), y0 = desc_lo(dys_s, T128);
 #pragma unroll
-          for (int q = 0; q < 8; ++q) kstep(tU, c0 + ((uint32_t)(q * 2048) >> 4), BS, y0 + ((uint32_t)(q * 2048) >> 4), XS, id_u, q ? 1u : 0u);
+          for (int q = 0; q < 8; ++q) mma_split<NI, ND>(tU, c0 + ((uint32_t)(q * 2048) >> 4), BS, y0 + ((uint32_t)(q * 2048) >> 4), XS, dhi, id_u, q ? 1u : 0u);
           umma_commit(bar(UFULL));
           if (p.state_only) { umma_commit(bar(EMPTY)); umma_commit(bar(XFREE + xb)); }
         }
@@ -272,8 +265,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const uint32_t oa = (uint32_t)(kt * T128 + q * 32) >> 4, ob = (uint32_t)(kt * T64 + q * 2048) >> 4;
-              kstep(tA2, b0 + oa, BS, d0 + ob, HS, id_v, (kt | q) ? 1u : 0u);
-              kstep(tA3, c0 + oa, BS, h0 + ob, HS, id_v, (kt | q) ? 1u : 0u);
+              mma_split<NI, ND>(tA2, b0 + oa, BS, d0 + ob, HS, dhi, id_v, (kt | q) ? 1u : 0u);
+              mma_split<NI, ND>(tA3, c0 + oa, BS, h0 + ob, HS, dhi, id_v, (kt | q) ? 1u : 0u);
             }
           umma_commit(bar(HFREE));
           umma_commit(bar(EMPTY));
@@ -287,13 +280,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const uint32_t ta = tG + (uint32_t)(16 * q), vb = y0 + ((uint32_t)(q * 2048) >> 4);
-            if (NS == 2) {
-              mma_f16_ts_h(tA1, ta + 8u, vb, dhi, id_v, q ? 1u : 0u);
-              mma_f16_ts_h(tA1, ta, vb + XS, dhi, id_v, 1u);
-              mma_f16_ts_h(tA1, ta, vb, dhi, id_v, 1u);
-            } else {
-              mma_f16_ts_h(tA1, ta, vb, dhi, id_v, q ? 1u : 0u);
-            }
+            mma_split_ts<ND, NI>(tA1, ta, 8u, vb, XS, dhi, id_v, q ? 1u : 0u);
           }
           umma_commit(bar(ACCFULL));
           umma_commit(bar(XFREE + xb));
@@ -369,7 +356,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
           if (!wait(XRDY + xb, (uint32_t)(k / XB), 2048u)) break;
           if (p.store_ops) {
 #pragma unroll
-            for (int sp = 0; sp < NS; ++sp) {
+            for (int sp = 0; sp < NI; ++sp) {
               tma_store_4d(&maps.xt[sp], xbuf_s + xb * GE::XBUF + sp * T128, 0, i * L, h, bb);
               tma_store_4d(&maps.dy[sp], xbuf_s + xb * GE::XBUF + GE::XT + sp * T128, 0, i * L, h, bb);
             }
@@ -426,8 +413,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
               w[2 * e2 + 1] = col + 1 > r_local ? m1 * __uint_as_float(dr[2 * e2 + 1]) : 0.0f;
               rsum += w[2 * e2];
               rsum += w[2 * e2 + 1];
-              split2(m0, m1, m[e2], m[8 + e2], NS == 2);
-              if (NS == 1) m[8 + e2] = 0u;
+              split2(m0, m1, m[e2], m[8 + e2], ND == 2);
+              if (ND == 1) m[8 + e2] = 0u;
             }
             cs = warp_column_sums16(w, lane);
           }
@@ -470,7 +457,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
             for (int e = 0; e < 2; ++e) {
               const uint32_t at = (uint32_t)((er + 16 * rh + 8 * e) * 128) + (uint32_t)(((4 * grp + 2 * c16 + q) ^ (lane >> 2)) << 4) + (uint32_t)((lane & 3) * 4);
               float2 xv = bf2(ld_shared(xt_s + at)), yv = bf2(ld_shared(dy_s + at));
-              if (NS == 2) {
+              if (NI == 2) {
                 const float2 xl = bf2(ld_shared(xt_s + T128 + at)), yl = bf2(ld_shared(dy_s + T128 + at));
                 xv.x += xl.x; xv.y += xl.y; yv.x += yl.x; yv.y += yl.y;
               }
@@ -589,26 +576,27 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
         const float f = __expf(S[row]);
         if (IN16) {
           const uint32_t y4[4] = {yq.x, yq.y, yq.z, yq.w};
-          uint32_t s4[4], z;
+          uint32_t s4[4], k4[4];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) { const float2 v = bf2(y4[e]); split2(v.x * f, v.y * f, s4[e], z, false); }
+          for (int e = 0; e < 4; ++e) { const float2 v = bf2(y4[e]); split2(v.x * f, v.y * f, s4[e], k4[e], ND == 2); }
           st_shared_v4(dst, xq.x, xq.y, xq.z, xq.w);
           st_shared_v4(dst + GE::XT, yq.x, yq.y, yq.z, yq.w);
           st_shared_v4(dst + 2 * GE::XT, s4[0], s4[1], s4[2], s4[3]);
+          if (ND == 2) st_shared_v4(dst + 2 * GE::XT + T128, k4[0], k4[1], k4[2], k4[3]);
         } else {
           const float dt = S[L + row];
           const float xv[4] = {__uint_as_float(xq.x), __uint_as_float(xq.y), __uint_as_float(xq.z), __uint_as_float(xq.w)};
           const float yv[4] = {__uint_as_float(yq.x), __uint_as_float(yq.y), __uint_as_float(yq.z), __uint_as_float(yq.w)};
           uint32_t h0, h1, l0 = 0u, l1 = 0u;
-          split2(xv[0] * dt, xv[1] * dt, h0, l0, NS == 2); split2(xv[2] * dt, xv[3] * dt, h1, l1, NS == 2);
+          split2(xv[0] * dt, xv[1] * dt, h0, l0, ND == 2); split2(xv[2] * dt, xv[3] * dt, h1, l1, ND == 2);
           st_shared_v2(dst, h0, h1);
-          if (NS == 2) st_shared_v2(dst + T128, l0, l1);
-          split2(yv[0], yv[1], h0, l0, NS == 2); split2(yv[2], yv[3], h1, l1, NS == 2);
+          if (ND == 2) st_shared_v2(dst + T128, l0, l1);
+          split2(yv[0], yv[1], h0, l0, ND == 2); split2(yv[2], yv[3], h1, l1, ND == 2);
           st_shared_v2(dst + GE::XT, h0, h1);
-          if (NS == 2) st_shared_v2(dst + GE::XT + T128, l0, l1);
-          split2(yv[0] * f, yv[1] * f, h0, l0, NS == 2); split2(yv[2] * f, yv[3] * f, h1, l1, NS == 2);
+          if (ND == 2) st_shared_v2(dst + GE::XT + T128, l0, l1);
+          split2(yv[0] * f, yv[1] * f, h0, l0, ND == 2); split2(yv[2] * f, yv[3] * f, h1, l1, ND == 2);
           st_shared_v2(dst + 2 * GE::XT, h0, h1);
-          if (NS == 2) st_shared_v2(dst + 2 * GE::XT + T128, l0, l1);
+          if (ND == 2) st_shared_v2(dst + 2 * GE::XT + T128, l0, l1);
 #pragma unroll
           for (int e = 0; e < 4; ++e) dD = fmaf(xv[e], yv[e], dD);
         }
@@ -659,13 +647,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
         for (int c = 0; c < 8; ++c) {                       // eight 16-byte chunks of the row
           uint32_t hi[4], lo[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) split2(hv[8 * c + 2 * e], hv[8 * c + 2 * e + 1], hi[e], lo[e], NS == 2);
+          for (int e = 0; e < 4; ++e) split2(hv[8 * c + 2 * e], hv[8 * c + 2 * e + 1], hi[e], lo[e], ND == 2);
           const uint32_t a = dh_s + (uint32_t)(nr * 128 + ((c ^ (nr & 7)) << 4));
           st_shared_v4(a, hi[0], hi[1], hi[2], hi[3]);
-          if (NS == 2) st_shared_v4(a + NK * T64, lo[0], lo[1], lo[2], lo[3]);
+          if (ND == 2) st_shared_v4(a + NK * T64, lo[0], lo[1], lo[2], lo[3]);
           if (active && 8 * c < p.P) {
             *reinterpret_cast<uint4*>(p.dh_hi + so + 8 * c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            if (NS == 2) *reinterpret_cast<uint4*>(p.dh_lo + so + 8 * c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            if (ND == 2) *reinterpret_cast<uint4*>(p.dh_lo + so + 8 * c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
           }
         }
       }
@@ -682,7 +670,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
           const uint32_t a = hin_s + (uint32_t)(nr * 128 + ((c ^ (nr & 7)) << 4));
           uint32_t v[4];
 #pragma unroll
-          for (int sp = 0; sp < NS; ++sp) {
+          for (int sp = 0; sp < ND; ++sp) {
             asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a + sp * NK * T64) : "memory");
 #pragma unroll
             for (int e = 0; e < 4; ++e) { const float2 u = bf2(v[e]); dot = fmaf(u.x, hv[8 * c + 2 * e], fmaf(u.y, hv[8 * c + 2 * e + 1], dot)); }
@@ -748,18 +736,19 @@ static unsigned int* status_ptr() {
   return ptr[dev];
 }
 
-template <int NS, int NK, bool IN16>
+template <int NI, int ND, int NK, bool IN16>
 static pmb_status launch(cudaStream_t st, const ChainBwdArgs& a) {
-  using GE = Geo<NS, NK>;
+  using GE = Geo<NI, ND, NK>;
   static_assert(GE::SMEM <= 227 * 1024, "shared-memory plan");
+  static_assert(IN16 ? NI == 1 : NI == ND, "fp32 tensors take pairs throughout");
   const int n = (int)cdiv(a.T, L);
   Maps ms{};
   for (int sp = 0; sp < 2; ++sp) {
-    const bool lo = sp && NS == 2;
+    const bool lo = sp && NI == 2, lod = sp && ND == 2;
     const int64_t st_h = (int64_t)a.N * a.P, hp = (int64_t)a.H * a.P;
     PMB_TRY(sf::bf16_map4(&ms.b[sp], lo ? a.b.lo : a.b.hi, a.N, a.T, a.G, a.B, a.b.pitch, a.N, (int64_t)a.T * a.b.pitch, 64, L));
     PMB_TRY(sf::bf16_map4(&ms.c[sp], lo ? a.c.lo : a.c.hi, a.N, a.T, a.G, a.B, a.c.pitch, a.N, (int64_t)a.T * a.c.pitch, 64, L));
-    PMB_TRY(sf::bf16_map4(&ms.h[sp], lo ? a.hp_lo : a.hp_hi, a.P, a.N, a.H, (int64_t)a.B * n, a.P, st_h, a.H * st_h, 64, 64));
+    PMB_TRY(sf::bf16_map4(&ms.h[sp], lod ? a.hp_lo : a.hp_hi, a.P, a.N, a.H, (int64_t)a.B * n, a.P, st_h, a.H * st_h, 64, 64));
     if (a.xt_hi) {
       PMB_TRY(sf::bf16_map4(&ms.xt[sp], lo ? a.xt_lo : a.xt_hi, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
       PMB_TRY(sf::bf16_map4(&ms.dy[sp], lo ? a.dyo_lo : a.dyo_hi, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
@@ -776,15 +765,15 @@ static pmb_status launch(cudaStream_t st, const ChainBwdArgs& a) {
     p.seg_h = a.seg; p.seg_d = a.seg + (size_t)a.B * a.H * p.nseg * a.N * a.P;
   }
   p.part_pitch = (int64_t)a.B * a.H * p.nseg;
-  PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_bwd_kernel<NS, NK, IN16>);
+  PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_bwd_kernel<NI, ND, NK, IN16>);
   const unsigned grid = (unsigned)((int64_t)a.B * a.H * p.nseg);
   if (p.nseg > 1) {
     p.state_only = 1;
-    ssd_chain_bwd_kernel<NS, NK, IN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
+    ssd_chain_bwd_kernel<NI, ND, NK, IN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
     PMB_LAUNCHED();
     p.state_only = 0;
   }
-  ssd_chain_bwd_kernel<NS, NK, IN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
+  ssd_chain_bwd_kernel<NI, ND, NK, IN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
   PMB_LAUNCHED();
   return PMB_OK;
 }
@@ -802,8 +791,9 @@ pmb_status ssd_chain_bwd(cudaStream_t st, const ChainBwdArgs& a) {
     return fail(PMB_ERR_SHAPE, "ssd_chain_bwd: x, dy and dx rows must be 16-byte aligned");
   const double tok = (double)a.B * a.T;
   ProfScope prof(st, "ssd_chain_bwd", tok * a.H * ((double)SCAN_STEP * (a.N + 2.0 * a.P) + 6.0 * a.N * a.P), 0.0);
-  if (pairs) return scb::launch<2, 1, false>(st, a);
-  return a.N > 64 ? scb::launch<1, 2, true>(st, a) : scb::launch<1, 1, true>(st, a);
+  if (pairs) return scb::launch<2, 2, 1, false>(st, a);
+  if (a.hp_lo) return a.N > 64 ? scb::launch<1, 2, 2, true>(st, a) : scb::launch<1, 2, 1, true>(st, a);
+  return a.N > 64 ? scb::launch<1, 1, 2, true>(st, a) : scb::launch<1, 1, 1, true>(st, a);
 }
 
 }  // namespace pmb

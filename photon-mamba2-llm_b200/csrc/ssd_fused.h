@@ -31,6 +31,7 @@ struct FusedArgs {
 constexpr int SCAN_STEP = 128;
 struct ChainArgs {
   int B, T, H, P, N, G;
+  bool exact = false;                          // x16: what is formed from the inputs (M, xs, the states) is kept as pairs, so that nothing is rounded to bf16 but y
   int blocks = 1;                              // steps per chunk (what S, xs and the states are relative to): 1 or 2
   Op16 b, c;                                   // (B,T,G,N), pitch = elements between tokens, group stride N
   const float* x; const uint16_t* x16; int64_t ldx;      // one of the two: fp32 (scaled by dt here) or bf16 (taken as x~)

@@ -9,10 +9,11 @@
 // order (heads_sum_kernel).  d_state is taken in halves of 64: a second pass over the heads forms the second half.
 //
 // warp 0 = TMA, 1 = MMA issuer, 2 = S of the heads, 4..11 = dG (64 columns per thread), 12..15 = dC, 16..19 = dB (64 columns per
-// thread).  Two operand stages, two sets of accumulators: the products of the next head run under the sums of this one.
+// thread).  Two or three operand stages, two sets of accumulators: the products of the next head run under the sums of this one.
 // What bounds it: the exponentials and the multiply-adds of the dG warps (64 of each per thread and head).
 // Measured at 24 heads of 64 x 64 on pairs, 4 x 512 tokens: 18 us + 3 us for the sum of the shares; the three contractions and their
-// sums that it replaces took 45 us and read copies of dY and x~ scaled by the decays that are not made any more.
+// sums that it replaces took 45 us and read copies of dY and x~ scaled by the decays that are not made any more.  bf16, 32 heads of 128 x 64, 16 x 8192 tokens: 836 us with two
+// stages, 820 with three (3.2 GB of operands; the contractions it replaces: 1070 us).
 #include <cuda_bf16.h>
 #include "tc_common.cuh"
 #include "kernels.h"
@@ -36,15 +37,16 @@ using namespace tcx;
 constexpr int L = SCAN_STEP, T128 = L * 128, T64 = 64 * 128;
 constexpr int W_G = 4, W_C = 12, NTHREADS = 32 * 20;
 
-template <int NS>
+template <int NI, int ND>
 struct Geo {
-  static constexpr int XT = NS * T128, HT = NS * T64;
+  static constexpr int XT = NI * T128, HT = ND * T64;
   static constexpr int STAGE = 2 * XT + 2 * HT;            // [dY | x~ | h | dh]; at the end of a pass [B | C]
-  static constexpr int DG = 2 * XT;                        // dG as an operand: two 64-column tiles (hi), then lo
-  static constexpr bool OWN_DG = NS == 1;                  // pairs: dG goes over the stage that the last head has left
+  static constexpr int DG = ND * 2 * T128;                        // dG as an operand: two 64-column tiles (hi), then lo
+  static constexpr bool OWN_DG = NI == 1;                  // pairs: dG goes over the stage that the last head has left
   static constexpr int RING = 4;                           // heads whose S is in shared memory
-  static constexpr int TILES = 2 * STAGE + (OWN_DG ? DG : 0);
-  static_assert(OWN_DG || DG <= STAGE, "dG fits a stage");
+  static constexpr int STG = NI == 1 && ND == 1 ? 3 : 2;   // (what fits)
+  static constexpr int TILES = STG * STAGE + (OWN_DG ? DG : 0);
+  static_assert(OWN_DG || (DG <= STAGE && STG == 2), "dG fits a stage");
   static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 256 /*barriers*/ + RING * L * 4;
 };
 
@@ -70,15 +72,15 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-template <int NS>
+template <int NI, int ND>
 __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_constant__ Maps maps, const Params p) {
-  using GE = Geo<NS>;
+  using GE = Geo<NI, ND>;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - raw);
   const uint32_t bars = base + GE::TILES;
-  enum { FULL = 0 /*2*/, EMPTY = 2 /*2*/, MFULL = 4 /*2*/, MFREE = 6 /*2*/, CFULL = 8 /*2*/, CFREE = 10 /*2*/, SRDY = 12 /*4*/, SFREE = 16 /*4*/, DGRDY = 20, NBAR };
+  enum { FULL = 0 /*3*/, EMPTY = 3 /*3*/, MFULL = 6 /*2*/, MFREE = 8 /*2*/, CFULL = 10 /*2*/, CFREE = 12 /*2*/, SRDY = 14 /*4*/, SFREE = 18 /*4*/, DGRDY = 22, NBAR };
   static_assert(8 * NBAR + 8 <= 256, "barrier block");
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
   uint8_t* bar_ptr = base_ptr + GE::TILES;
@@ -97,9 +99,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
   const int per_pass = nh + 1, nitems = p.passes * per_pass;     // the heads, then the product with dG
   if (threadIdx.x == 0) {
     for (int q = 0; q < 2; ++q) {
-      mbar_init(bar(FULL + q), 1); mbar_init(bar(EMPTY + q), 1); mbar_init(bar(MFULL + q), 1); mbar_init(bar(MFREE + q), 8);
+      mbar_init(bar(MFULL + q), 1); mbar_init(bar(MFREE + q), 8);
       mbar_init(bar(CFULL + q), 1); mbar_init(bar(CFREE + q), 8);
     }
+    for (int q = 0; q < GE::STG; ++q) { mbar_init(bar(FULL + q), 1); mbar_init(bar(EMPTY + q), 1); }
     for (int q = 0; q < 4; ++q) { mbar_init(bar(SRDY + q), 1); mbar_init(bar(SFREE + q), 16); }
     mbar_init(bar(DGRDY), 8);
     *abort_flag = 0;
@@ -116,7 +119,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
   const uint32_t tmem = *tmem_slot;
   const uint32_t tM = tmem, tC = tmem + 256, tB = tmem + 384;
   // the stage that dG goes over: the one the last head of the first pass was in
-  const uint32_t dg_s = GE::OWN_DG ? base + 2 * GE::STAGE : base + (uint32_t)((nh - 1) & 1) * GE::STAGE;
+  const uint32_t dg_s = GE::OWN_DG ? base + GE::STG * GE::STAGE : base + (uint32_t)((nh - 1) & 1) * GE::STAGE;
 
   auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
   auto wait = [&](int b, uint32_t parity, unsigned int code) -> bool {
@@ -131,23 +134,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
     if (lane == 0) {
       int issued = 0;
       for (int m = 0; m < nitems; ++m) {
-        const int s = m & 1, ps = m / per_pass, j = m - ps * per_pass;
-        if (!wait(EMPTY + s, (uint32_t)(m >> 1) ^ 1u, 1u)) break;
+        const int s = m % GE::STG, ps = m / per_pass, j = m - ps * per_pass;
+        if (!wait(EMPTY + s, (uint32_t)(m / GE::STG) ^ 1u, 1u)) break;
         const uint32_t st = base + s * GE::STAGE;
         if (j < nh) {
           const int h = head(j);
           mbar_expect_tx(bar(FULL + s), GE::STAGE);
 #pragma unroll
-          for (int sp = 0; sp < NS; ++sp) {
+          for (int sp = 0; sp < NI; ++sp) {
             tma_load_4d(st + sp * T128, &maps.dy[sp], 0, i * L, h, bb, bar(FULL + s));
             tma_load_4d(st + GE::XT + sp * T128, &maps.xt[sp], 0, i * L, h, bb, bar(FULL + s));
+          }
+#pragma unroll
+          for (int sp = 0; sp < ND; ++sp) {
             tma_load_4d(st + 2 * GE::XT + sp * T64, &maps.h[sp], 0, 64 * ps, h, bb * p.n + i, bar(FULL + s));
             tma_load_4d(st + 2 * GE::XT + GE::HT + sp * T64, &maps.dh[sp], 0, 64 * ps, h, bb * p.n + i, bar(FULL + s));
           }
         } else {
           mbar_expect_tx(bar(FULL + s), 2 * GE::XT);
 #pragma unroll
-          for (int sp = 0; sp < NS; ++sp) {
+          for (int sp = 0; sp < NI; ++sp) {
             tma_load_4d(st + sp * T128, &maps.b[sp], 64 * ps, i * L, g, bb, bar(FULL + s));
             tma_load_4d(st + GE::XT + sp * T128, &maps.c[sp], 64 * ps, i * L, g, bb, bar(FULL + s));
           }
@@ -155,28 +161,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
         issued = m + 1;
       }
       if (*abort_flag)
-        for (int m = (issued > 2 ? issued - 2 : 0); m < issued; ++m) mbar_wait(bar(FULL + (m & 1)), (uint32_t)((m >> 1) & 1));
+        for (int m = (issued > GE::STG ? issued - GE::STG : 0); m < issued; ++m) mbar_wait(bar(FULL + m % GE::STG), (uint32_t)((m / GE::STG) & 1));
     }
   } else if (warp == 1) {
     const uint32_t dhi = desc_hi(1024, 2);
     const uint32_t id_m = idesc_bf16(0, 0, L, L), id_h = idesc_bf16(0, 0, L, 64);      // both operands K-major
     const uint32_t id_c = idesc_bf16(0, 1, L, 64), id_b = idesc_bf16(1, 1, L, 64);     // dG B and dG^T C
-    auto kstep = [&](uint32_t d, uint32_t alo, uint32_t as, uint32_t blo, uint32_t bs, uint32_t idesc, uint32_t acc) {
-      if (NS == 2) {
-        mma_f16_h(d, alo + as, dhi, blo, dhi, idesc, acc);
-        mma_f16_h(d, alo, dhi, blo + bs, dhi, idesc, 1u);
-        mma_f16_h(d, alo, dhi, blo, dhi, idesc, 1u);
-      } else {
-        mma_f16_h(d, alo, dhi, blo, dhi, idesc, acc);
-      }
-    };
     const uint32_t XS = T128 >> 4, HS = T64 >> 4, DS = (2 * T128) >> 4;
     bool ok = true;
 #pragma unroll 1
     for (int m = 0; m < nitems && ok; ++m) {
-      const int s = m & 1, ps = m / per_pass, j = m - ps * per_pass;
-      const uint32_t st = base + s * GE::STAGE;
-      ok = all(wait(FULL + s, (uint32_t)(m >> 1), 2u) && (m < 2 || wait(CFREE + s, (uint32_t)((m >> 1) - 1), 4u)) &&
+      const int s = m & 1, sg = m % GE::STG, ps = m / per_pass, j = m - ps * per_pass;
+      const uint32_t st = base + sg * GE::STAGE;
+      ok = all(wait(FULL + sg, (uint32_t)(m / GE::STG), 2u) && (m < 2 || wait(CFREE + s, (uint32_t)((m >> 1) - 1), 4u)) &&
                (ps > 0 || j >= nh || j < 2 || wait(MFREE + (j & 1), (uint32_t)((j >> 1) - 1), 8u)) && (j < nh || wait(DGRDY, 0u, 16u)));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -186,9 +183,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
           const uint32_t y0 = desc_lo(st, 16), x0 = desc_lo(st + GE::XT, 16), h0 = desc_lo(st + 2 * GE::XT, 16), d0 = desc_lo(st + 2 * GE::XT + GE::HT, 16);
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            if (ps == 0) kstep(tM + (uint32_t)(128 * (j & 1)), y0 + 2 * q, XS, x0 + 2 * q, XS, id_m, q ? 1u : 0u);
-            kstep(dC, y0 + 2 * q, XS, h0 + 2 * q, HS, id_h, q ? 1u : 0u);
-            kstep(dB, x0 + 2 * q, XS, d0 + 2 * q, HS, id_h, q ? 1u : 0u);
+            if (ps == 0) mma_split<NI, NI>(tM + (uint32_t)(128 * (j & 1)), y0 + 2 * q, XS, x0 + 2 * q, XS, dhi, id_m, q ? 1u : 0u);
+            mma_split<NI, ND>(dC, y0 + 2 * q, XS, h0 + 2 * q, HS, dhi, id_h, q ? 1u : 0u);
+            mma_split<NI, ND>(dB, x0 + 2 * q, XS, d0 + 2 * q, HS, dhi, id_h, q ? 1u : 0u);
           }
           if (ps == 0) umma_commit(bar(MFULL + (j & 1)));
         } else {
@@ -196,12 +193,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const uint32_t o = (uint32_t)(q * 2048) >> 4;
-            kstep(dC, gk + ((uint32_t)((q >> 2) * T128 + (q & 3) * 32) >> 4), DS, b0 + o, XS, id_c, q ? 1u : 0u);
-            kstep(dB, gm + o, DS, c0 + o, XS, id_b, q ? 1u : 0u);
+            mma_split<ND, NI>(dC, gk + ((uint32_t)((q >> 2) * T128 + (q & 3) * 32) >> 4), DS, b0 + o, XS, dhi, id_c, q ? 1u : 0u);
+            mma_split<ND, NI>(dB, gm + o, DS, c0 + o, XS, dhi, id_b, q ? 1u : 0u);
           }
         }
         umma_commit(bar(CFULL + s));
-        umma_commit(bar(EMPTY + s));
+        umma_commit(bar(EMPTY + sg));
       }
       __syncwarp();
     }
@@ -269,7 +266,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
         }
         const uint32_t a = dg_s + (uint32_t)(grp * T128 + row * 128 + ((c ^ (row & 7)) << 4));
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
-        if (NS == 2) asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a + 2 * T128), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
+        if (ND == 2) asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a + 2 * T128), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
@@ -378,19 +375,19 @@ static unsigned int* status_ptr() {
   return ptr[dev];
 }
 
-template <int NS>
+template <int NI, int ND>
 static pmb_status launch(cudaStream_t st, const HeadsArgs& a, int nsplit) {
-  using GE = Geo<NS>;
+  using GE = Geo<NI, ND>;
   static_assert(GE::SMEM <= 227 * 1024, "shared-memory plan");
   const int n = (int)cdiv(a.T, L);
   Maps ms{};
   for (int sp = 0; sp < 2; ++sp) {
-    const bool lo = sp && NS == 2;
+    const bool lo = sp && NI == 2, lod = sp && ND == 2;
     const int64_t st_h = (int64_t)a.N * a.P, hp = (int64_t)a.H * a.P;
     PMB_TRY(sf::bf16_map4(&ms.dy[sp], lo ? a.dy.lo : a.dy.hi, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
     PMB_TRY(sf::bf16_map4(&ms.xt[sp], lo ? a.xt.lo : a.xt.hi, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
-    PMB_TRY(sf::bf16_map4(&ms.h[sp], lo ? a.hp_lo : a.hp_hi, a.P, a.N, a.H, (int64_t)a.B * n, a.P, st_h, a.H * st_h, 64, 64));
-    PMB_TRY(sf::bf16_map4(&ms.dh[sp], lo ? a.dh_lo : a.dh_hi, a.P, a.N, a.H, (int64_t)a.B * n, a.P, st_h, a.H * st_h, 64, 64));
+    PMB_TRY(sf::bf16_map4(&ms.h[sp], lod ? a.hp_lo : a.hp_hi, a.P, a.N, a.H, (int64_t)a.B * n, a.P, st_h, a.H * st_h, 64, 64));
+    PMB_TRY(sf::bf16_map4(&ms.dh[sp], lod ? a.dh_lo : a.dh_hi, a.P, a.N, a.H, (int64_t)a.B * n, a.P, st_h, a.H * st_h, 64, 64));
     PMB_TRY(sf::bf16_map4(&ms.b[sp], lo ? a.b.lo : a.b.hi, a.N, a.T, a.G, a.B, a.b.pitch, a.N, (int64_t)a.T * a.b.pitch, 64, L));
     PMB_TRY(sf::bf16_map4(&ms.c[sp], lo ? a.c.lo : a.c.hi, a.N, a.T, a.G, a.B, a.c.pitch, a.N, (int64_t)a.T * a.c.pitch, 64, L));
   }
@@ -398,8 +395,8 @@ static pmb_status launch(cudaStream_t st, const HeadsArgs& a, int nsplit) {
   p.T = a.T; p.H = a.H; p.G = a.G; p.hpg = a.H / a.G; p.N = a.N; p.n = n; p.nsplit = nsplit; p.passes = (int)cdiv(a.N, 64);
   p.S = a.S; p.dc = a.dc; p.db = a.db; p.ld = a.ld; p.dc16 = a.dc16; p.db16 = a.db16; p.part = a.part; p.status = status_ptr();
   const int64_t tiles = (int64_t)a.B * n * a.G;
-  PMB_SMEM_OPT_IN(GE::SMEM, ssd_heads_kernel<NS>);
-  ssd_heads_kernel<NS><<<(unsigned)(tiles * nsplit), NTHREADS, GE::SMEM, st>>>(ms, p);
+  PMB_SMEM_OPT_IN(GE::SMEM, ssd_heads_kernel<NI, ND>);
+  ssd_heads_kernel<NI, ND><<<(unsigned)(tiles * nsplit), NTHREADS, GE::SMEM, st>>>(ms, p);
   PMB_LAUNCHED();
   if (nsplit > 1) {
     const int64_t total = tiles * 2 * L * (a.N / 4);
@@ -436,7 +433,8 @@ pmb_status ssd_heads(cudaStream_t st, const HeadsArgs& a) {
   if (!al16(a.dc) || !al16(a.db) || !al16(a.dc16) || !al16(a.db16) || !al16(a.part) || (a.ld & (a.dc16 ? 7 : 3))) return fail(PMB_ERR_SHAPE, "ssd_heads: dB and dC rows must be 16-byte aligned");
   const double tok = (double)a.B * a.T;
   ProfScope prof(st, "ssd_heads", tok * (a.H * ((double)SCAN_STEP * a.P + 4.0 * a.N * a.P) + 2.0 * a.G * SCAN_STEP * a.N), 0.0);
-  return pairs ? shd::launch<2>(st, a, nsplit) : shd::launch<1>(st, a, nsplit);
+  if (pairs) return shd::launch<2, 2>(st, a, nsplit);
+  return a.hp_lo ? shd::launch<1, 2>(st, a, nsplit) : shd::launch<1, 1>(st, a, nsplit);
 }
 
 }  // namespace pmb

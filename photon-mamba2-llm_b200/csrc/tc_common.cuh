@@ -178,6 +178,22 @@ __device__ __forceinline__ void mma_f16_ts_h(uint32_t tmem_d, uint32_t tmem_a, u
       ::"r"(tmem_d), "r"(tmem_a), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate));
 }
 
+// One k-step of a product whose operands are stored as bf16 (1) or as a (hi, lo) pair of bf16 (2): every term but lo x lo.  `as` / `bs`
+// lead from the hi tile to the lo tile.
+template <int NA, int NB>
+__device__ __forceinline__ void mma_split(uint32_t d, uint32_t a, uint32_t as, uint32_t b, uint32_t bs, uint32_t dhi, uint32_t idesc, uint32_t acc) {
+  if (NA == 2) { mma_f16_h(d, a + as, dhi, b, dhi, idesc, acc); acc = 1u; }
+  if (NB == 2) { mma_f16_h(d, a, dhi, b + bs, dhi, idesc, acc); acc = 1u; }
+  mma_f16_h(d, a, dhi, b, dhi, idesc, acc);
+}
+// the same with the A operand in TMEM
+template <int NA, int NB>
+__device__ __forceinline__ void mma_split_ts(uint32_t d, uint32_t ta, uint32_t as, uint32_t b, uint32_t bs, uint32_t dhi, uint32_t idesc, uint32_t acc) {
+  if (NA == 2) { mma_f16_ts_h(d, ta + as, b, dhi, idesc, acc); acc = 1u; }
+  if (NB == 2) { mma_f16_ts_h(d, ta, b + bs, dhi, idesc, acc); acc = 1u; }
+  mma_f16_ts_h(d, ta, b, dhi, idesc, acc);
+}
+
 // 16 registers per thread -> 32 lanes x 16 consecutive 32-bit columns of TMEM (thread = lane/row)
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
   asm volatile(

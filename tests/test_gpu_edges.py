@@ -109,3 +109,34 @@ def test_decode_batches(pm, B, D, H, P, N, G):
         assert_close(st["ssm_state"], ref["ssm_state"], what="state")
         assert_close(st["conv_window"], ref["conv_window"], what="window")
     assert pm.device_status() == 0
+
+
+# the bf16-input scan off the 128-token grid keeps everything but its outputs at fp32 precision: lengths around a step, segments,
+# narrow heads and states, one and two halves of d_state, tensors that start off a 16-byte boundary
+@pytest.mark.parametrize("B,T", [(1, 1), (2, 127), (1, 129), (3, 200), (1, 700)])
+@pytest.mark.parametrize("P,N,G,off", [(64, 64, 1, 0), (64, 128, 1, 0), (64, 128, 4, 0), (32, 16, 1, 0), (64, 72, 1, 3)])
+def test_scan_bf16_lengths(pm, B, T, P, N, G, off):
+    H = 4
+
+    def put(t):
+        return torch.cat([torch.zeros(off, dtype=t.dtype), t.flatten()]).cuda()[off:].view(t.shape)
+    x, b, c, dy = randn((B, T, H, P), 1).bfloat16(), randn((B, T, G, N), 2).bfloat16(), randn((B, T, G, N), 3).bfloat16(), randn((B, T, H, P), 4).bfloat16()
+    a = -torch.nn.functional.softplus(randn((B, T, H), 5) - 2.0)
+    init = randn((B, H, N, P), 6)
+    scan = pm.SsdScanBf16(put(x), a.cuda(), put(b), put(c), 128)
+    y, last = scan.forward(init_state=put(init), want_final_state=True)
+    y0 = scan.forward()
+    dx, da, db, dc = scan.backward(put(dy))
+    torch.cuda.synchronize()
+    assert pm.device_status() == 0
+    leaves = [t.float().requires_grad_(True) for t in (x, a, b, c)]
+    be, ce = (t.expand(B, T, H, N) for t in leaves[2:])
+    ref, _ = orc.ssd_scan_chunked(leaves[0], leaves[1], be, ce, T, return_final_state=True)
+    ref.backward(dy.float())
+    with torch.no_grad():
+        ref_i, last_i = orc.ssd_scan_chunked(leaves[0], leaves[1], be, ce, T, initial_state=init, return_final_state=True)
+    for got, want, tol, what in ((y0.float(), ref, 5e-3, "y"), (y.float(), ref_i, 5e-3, "y from a state"), (last, last_i, 1e-4, "final state"),
+                                 (dx.float(), leaves[0].grad, 5e-3, "dx"), (da, leaves[1].grad, 1e-4, "da"),
+                                 (db.float(), leaves[2].grad, 5e-3, "db"), (dc.float(), leaves[3].grad, 5e-3, "dc")):
+        if T > 1 or what != "da":      # (one token: da is exactly zero)
+            assert_close(got, want, tol=tol, what=what)
