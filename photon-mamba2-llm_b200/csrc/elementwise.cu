@@ -5,25 +5,39 @@
 
 namespace pmb {
 
+constexpr int COLSUM_LANES = 32;
 __global__ void column_sum_kernel(const float* __restrict__ partial, int64_t rows, int cols, float* __restrict__ out);
 
 // ---------------------------------------------------------------------------------------------
-// conv1d (causal, depthwise) + bias + SiLU, forward.   u[t,c] = b[c] + sum_k w[c,k] * xbc[t-(K-1)+k, c]
-// Layout stays (B,T,channels): a thread owns VEC adjacent channels and walks TT consecutive time steps
-// with the K-1 previous inputs in registers, so every global access is a coalesced vector access and
-// each input row is read (TT+K-1)/TT times.
+// conv1d (causal, depthwise) + bias + SiLU.   u[t,c] = b[c] + sum_k w[c,k] * xbc[t-(K-1)+k, c]
+// Layout stays (B,T,channels): a thread owns VEC adjacent channels and walks a run of time steps with the K-1 previous inputs in
+// registers and the next CONV_AHEAD rows on their way, so that every global access is a coalesced vector access and each input
+// row is read (run+K-1)/run times.  Bound by HBM.  A CTA of the vector kernels is 16 runs of 8 channel quads (128-byte strips of
+// its rows): no thread is idle for any channel count that is a multiple of 32.
+// Measured at 8 x 2048 tokens of 1664 channels: forward 68 us with runs of 8 all requested up front, @CF; backward 131 us, @CB.
 // ---------------------------------------------------------------------------------------------
-template <int K, int VEC, int TT>
-// (eight CTAs per SM: the 1024 CTAs of a 2048-token launch are then resident at once instead of 1.15 waves)
-__global__ void __launch_bounds__(128, 8) conv_silu_fwd_kernel(const float* __restrict__ xzd, int64_t ldx, int col0,
-                                                            const float* __restrict__ w, const float* __restrict__ bias,
-                                                            float* __restrict__ act, int X, int T, ConvPairOut po) {
-  int c = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
-  if (c >= X) return;
-  int tblocks = (T + TT - 1) / TT;
-  int b = blockIdx.y / tblocks;
-  int t0 = (blockIdx.y % tblocks) * TT;
-  int t1 = min(t0 + TT, T);
+constexpr int CONV_AHEAD = 4;
+constexpr int CONV_SLICES = 16;
+constexpr int CONV_STRIP_THREADS = CONV_SLICES * 8;
+
+// Steps per run: 32 where that still gives eight CTAs per SM (the halo of K - 1 rows is then a tenth), else 16 or 8.
+static int conv_run(const Dims& d) {
+  for (int run = 32; run > 8; run >>= 1)
+    if (cdiv(d.X, 32) * d.B * cdiv(d.T, CONV_SLICES * run) >= 148 * 8) return run;
+  return 8;
+}
+
+template <int VEC>
+__device__ __forceinline__ void conv_load(const float* p, float (&o)[VEC]) {
+  if (VEC == 4) { const float4 q = *reinterpret_cast<const float4*>(p); o[0] = q.x; o[1 % VEC] = q.y; o[2 % VEC] = q.z; o[3 % VEC] = q.w; }
+  else o[0] = *p;
+}
+
+// channels [c, c + VEC) of batch b, time steps [t0, t1)
+template <int K, int VEC>
+__device__ __forceinline__ void conv_fwd_thread(const float* __restrict__ xzd, int64_t ldx, int col0, const float* __restrict__ w,
+                                                const float* __restrict__ bias, float* __restrict__ act, int X, int T,
+                                                const ConvPairOut& po, int c, int b, int t0, int t1) {
   float wr[VEC][K], br[VEC], win[VEC][K];
 #pragma unroll
   for (int v = 0; v < VEC; ++v) {
@@ -34,53 +48,68 @@ __global__ void __launch_bounds__(128, 8) conv_silu_fwd_kernel(const float* __re
   const float* src = xzd + (int64_t)b * T * ldx + col0 + c;
 #pragma unroll
   for (int k = 0; k < K - 1; ++k) {
-    int t = t0 - (K - 1) + k;
-    if (VEC == 4) {
-      float4 q = t >= 0 ? *reinterpret_cast<const float4*>(src + (int64_t)t * ldx) : make_float4(0, 0, 0, 0);
-      win[0][k] = q.x; win[1 % VEC][k] = q.y; win[2 % VEC][k] = q.z; win[3 % VEC][k] = q.w;
-    } else {
-      win[0][k] = t >= 0 ? src[(int64_t)t * ldx] : 0.0f;
-    }
-  }
-  float* dst = act + (int64_t)b * T * X + c;
-  // TT is a compile-time constant: all TT rows are requested before the first one is used
-  float cur[TT][VEC];
-#pragma unroll
-  for (int i = 0; i < TT; ++i) {
-    const int t = t0 + i;
-    if (VEC == 4) {
-      float4 q = t < t1 ? *reinterpret_cast<const float4*>(src + (int64_t)t * ldx) : make_float4(0, 0, 0, 0);
-      cur[i][0] = q.x; cur[i][1 % VEC] = q.y; cur[i][2 % VEC] = q.z; cur[i][3 % VEC] = q.w;
-    } else {
-      cur[i][0] = t < t1 ? src[(int64_t)t * ldx] : 0.0f;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < TT; ++i) {
-    const int t = t0 + i;
+    const int t = t0 - (K - 1) + k;
     float o[VEC];
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) {
-      win[v][K - 1] = cur[i][v];
-      float u = br[v];
+    for (int v = 0; v < VEC; ++v) o[v] = 0.0f;
+    if (t >= 0) conv_load<VEC>(src + (int64_t)t * ldx, o);
 #pragma unroll
-      for (int k = 0; k < K; ++k) u = fmaf(wr[v][k], win[v][k], u);
-      o[v] = u * sigmoid_acc(u);
+    for (int v = 0; v < VEC; ++v) win[v][k] = o[v];
+  }
+  float ring[CONV_AHEAD][VEC];
+  const float* nx = src + (int64_t)t0 * ldx;                  // the next row to request
+  auto request = [&](int t, float (&o)[VEC]) {
+    if (t < t1) conv_load<VEC>(nx, o);
+    nx += ldx;
+  };
 #pragma unroll
-      for (int k = 0; k < K - 1; ++k) win[v][k] = win[v][k + 1];
-    }
-    if (t < t1) {
-      if (VEC == 4) {
-        *reinterpret_cast<float4*>(dst + (int64_t)t * X) = make_float4(o[0], o[1 % VEC], o[2 % VEC], o[3 % VEC]);
-        // the B | C columns also go out as a bf16 pair (operands of the fused scan kernels)
-        if (po.hi && c >= po.col0) {
-          const int64_t o16 = ((int64_t)b * T + t) * po.width + (c - po.col0);
-          store_pair4(po.hi + o16, po.lo ? po.lo + o16 : nullptr, o[0], o[1 % VEC], o[2 % VEC], o[3 % VEC]);
-        }
+  for (int q = 0; q < CONV_AHEAD; ++q) request(t0 + q, ring[q]);
+  float* dst = act + ((int64_t)b * T + t0) * X + c;
+  int64_t o16 = ((int64_t)b * T + t0) * po.width + (c - po.col0);
+  const bool pair = VEC == 4 && po.hi && c >= po.col0;        // the B | C columns also go out as a bf16 pair (operands of the scan)
+  for (int tb = t0; tb < t1; tb += CONV_AHEAD) {
+#pragma unroll
+    for (int q = 0; q < CONV_AHEAD; ++q) {
+      const int t = tb + q;
+      if (t >= t1) break;
+      float o[VEC];
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) win[v][K - 1] = ring[q][v];
+      request(t + CONV_AHEAD, ring[q]);
+#pragma unroll
+      for (int v = 0; v < VEC; ++v) {
+        float u = br[v];
+#pragma unroll
+        for (int k = 0; k < K; ++k) u = fmaf(wr[v][k], win[v][k], u);
+        o[v] = u * sigmoid_acc(u);
+#pragma unroll
+        for (int k = 0; k < K - 1; ++k) win[v][k] = win[v][k + 1];
       }
-      else dst[(int64_t)t * X] = o[0];
+      if (VEC == 4) *reinterpret_cast<float4*>(dst) = make_float4(o[0], o[1 % VEC], o[2 % VEC], o[3 % VEC]);
+      else *dst = o[0];
+      if (pair) store_pair4(po.hi + o16, po.lo ? po.lo + o16 : nullptr, o[0], o[1 % VEC], o[2 % VEC], o[3 % VEC]);
+      dst += X; o16 += po.width;
     }
   }
+}
+
+template <int K>
+__global__ void __launch_bounds__(CONV_STRIP_THREADS) conv_silu_fwd_strip_kernel(const float* __restrict__ xzd, int64_t ldx, int col0,
+                                                                                 const float* __restrict__ w, const float* __restrict__ bias,
+                                                                                 float* __restrict__ act, int X, int T, int run, ConvPairOut po) {
+  const int c = (blockIdx.x * 8 + (threadIdx.x & 7)) * 4;
+  const int tblocks = (T + CONV_SLICES * run - 1) / (CONV_SLICES * run);
+  const int b = blockIdx.y / tblocks, t0 = (blockIdx.y % tblocks) * (CONV_SLICES * run) + (threadIdx.x >> 3) * run;
+  if (c < X && t0 < T) conv_fwd_thread<K, 4>(xzd, ldx, col0, w, bias, act, X, T, po, c, b, t0, min(t0 + run, T));
+}
+// any channel count and alignment
+template <int K>
+__global__ void __launch_bounds__(128) conv_silu_fwd_kernel(const float* __restrict__ xzd, int64_t ldx, int col0, const float* __restrict__ w,
+                                                            const float* __restrict__ bias, float* __restrict__ act, int X, int T, int run) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int tblocks = (T + run - 1) / run;
+  const int b = blockIdx.y / tblocks, t0 = (blockIdx.y % tblocks) * run;
+  if (c < X) conv_fwd_thread<K, 1>(xzd, ldx, col0, w, bias, act, X, T, ConvPairOut{}, c, b, t0, min(t0 + run, T));
 }
 
 __global__ void dt_softplus_kernel(const float* __restrict__ xzd, int64_t ldx, int col0, const float* __restrict__ dt_bias,
@@ -95,24 +124,19 @@ __global__ void dt_softplus_kernel(const float* __restrict__ xzd, int64_t ldx, i
 template <int K>
 static pmb_status launch_conv_fwd_k(cudaStream_t st, const Dims& d, const float* xzd, const float* w, const float* b, float* act,
                                     ConvPairOut* pair) {
-  // time steps per thread: short runs keep enough threads in flight for small token counts
-  const bool long_runs = d.M >= 32768;
-  const int TT = long_runs ? 16 : 8;
+  const int run = conv_run(d);
   bool vec = (d.X % 4 == 0) && (d.J % 4 == 0) && (d.I % 4 == 0) && ((reinterpret_cast<uintptr_t>(xzd) | reinterpret_cast<uintptr_t>(act)) % 16 == 0);
-  int tblocks = (d.T + TT - 1) / TT;
   ConvPairOut po{};
   if (pair) {
     if (vec && pair->hi && ((reinterpret_cast<uintptr_t>(pair->hi) | reinterpret_cast<uintptr_t>(pair->lo)) % 8 == 0) && pair->width % 4 == 0) po = *pair;
     else pair->hi = nullptr;       // tells the caller that the pair was not written
   }
   if (vec) {
-    dim3 grid((unsigned)cdiv(d.X / 4, 128), (unsigned)(d.B * tblocks));
-    if (long_runs) conv_silu_fwd_kernel<K, 4, 16><<<grid, 128, 0, st>>>(xzd, d.J, d.I, w, b, act, d.X, d.T, po);
-    else conv_silu_fwd_kernel<K, 4, 8><<<grid, 128, 0, st>>>(xzd, d.J, d.I, w, b, act, d.X, d.T, po);
+    dim3 grid((unsigned)cdiv(d.X, 32), (unsigned)(d.B * cdiv(d.T, CONV_SLICES * run)));
+    conv_silu_fwd_strip_kernel<K><<<grid, CONV_STRIP_THREADS, 0, st>>>(xzd, d.J, d.I, w, b, act, d.X, d.T, run, po);
   } else {
-    dim3 grid((unsigned)cdiv(d.X, 128), (unsigned)(d.B * tblocks));
-    if (long_runs) conv_silu_fwd_kernel<K, 1, 16><<<grid, 128, 0, st>>>(xzd, d.J, d.I, w, b, act, d.X, d.T, po);
-    else conv_silu_fwd_kernel<K, 1, 8><<<grid, 128, 0, st>>>(xzd, d.J, d.I, w, b, act, d.X, d.T, po);
+    dim3 grid((unsigned)cdiv(d.X, 128), (unsigned)(d.B * cdiv(d.T, run)));
+    conv_silu_fwd_kernel<K><<<grid, 128, 0, st>>>(xzd, d.J, d.I, w, b, act, d.X, d.T, run);
   }
   PMB_LAUNCHED();
   return PMB_OK;
@@ -142,12 +166,11 @@ pmb_status conv_silu_dt_fwd(cudaStream_t st, const Dims& d, const float* xzd, co
 // ---------------------------------------------------------------------------------------------
 // conv backward.  du = dact * silu'(u) with u recomputed from the pre-conv window;
 // dxbc[t',c] = sum_k w[c,k] du[t'+(K-1)-k, c];  dw[c,k] = sum_{b,t} du[t,c] xbc[t-(K-1)+k,c];  db = sum du.
-// A thread owns one channel and TT time steps; per-(block-row) partial dw/db go to `partial`
-// (rows = gridDim.y, K+1 values per channel) and are summed by column_sum_kernel (fixed order).
+// Partial dw/db go to `partial` (rows = gridDim.y, K+1 values per channel) and are summed by column_sum_kernel (fixed order).
 // ---------------------------------------------------------------------------------------------
 // The work of one thread: channels [c, c + VEC) of batch b, time steps [t0, t1); writes its rows of the data gradient
 // and leaves its share of the parameter gradients in dwacc / dbacc.
-template <int K, int VEC, int TT>
+template <int K, int VEC>
 __device__ __forceinline__ void conv_bwd_thread(const float* __restrict__ xzd, int64_t ldx, int col0, const float* __restrict__ w,
                                                 const float* __restrict__ bias, const float* __restrict__ dact,
                                                 float* __restrict__ dxzd, int X, int T, uint16_t* __restrict__ pair_hi,
@@ -161,8 +184,6 @@ __device__ __forceinline__ void conv_bwd_thread(const float* __restrict__ xzd, i
     for (int k = 0; k < K; ++k) wr[v][k] = w[(c + v) * K + k];
   }
   const float* src = xzd + (int64_t)b * T * ldx + col0 + c;
-  const float* dsrc = dact + (int64_t)b * T * X + c;
-  float* ddst = dxzd + (int64_t)b * T * ldx + col0 + c;
   // xin holds xbc[t-(K-1) .. t]; dus holds du[t-(K-1) .. t] for the current t.
   float xin[VEC][K], dus[VEC][K];
 #pragma unroll
@@ -171,90 +192,89 @@ __device__ __forceinline__ void conv_bwd_thread(const float* __restrict__ xzd, i
 #pragma unroll
     for (int k = 0; k < K; ++k) { dwacc[v][k] = 0.0f; dus[v][k] = 0.0f; xin[v][k] = 0.0f; }
   }
-  auto load = [&](const float* p, float (&o)[VEC]) {
-    if (VEC == 4) { float4 q = *reinterpret_cast<const float4*>(p); o[0] = q.x; o[1 % VEC] = q.y; o[2 % VEC] = q.z; o[3 % VEC] = q.w; }
-    else o[0] = *p;
-  };
 #pragma unroll
   for (int k = 0; k < K - 1; ++k) {
     int t = t0 - (K - 1) + k;
     float o[VEC];
 #pragma unroll
     for (int v = 0; v < VEC; ++v) o[v] = 0.0f;
-    if (t >= 0) load(src + (int64_t)t * ldx, o);
+    if (t >= 0) conv_load<VEC>(src + (int64_t)t * ldx, o);
 #pragma unroll
     for (int v = 0; v < VEC; ++v) xin[v][k + 1] = o[v];
   }
   // Walk t from t0 to t1-1+(K-1): du[t] is needed by dxbc[t-(K-1) .. t]; du beyond the sequence end is 0.
-  int tend = min(t1 + K - 1, T + K - 1);
-  // all rows of the run are requested before the first one is used (TT is a compile-time constant)
-  float xall[TT + K - 1][VEC], dall[TT + K - 1][VEC];
+  const int tend = t1 + K - 1;
+  const int tl = min(tend, T);                                 // rows that exist
+  float xr[CONV_AHEAD][VEC], dr[CONV_AHEAD][VEC];
+  const float* nx = src + (int64_t)t0 * ldx;
+  const float* nd = dact + ((int64_t)b * T + t0) * X + c;
+  auto request = [&](int t, int q) {
+    if (t < tl) { conv_load<VEC>(nx, xr[q]); conv_load<VEC>(nd, dr[q]); }
+    nx += ldx; nd += X;
+  };
 #pragma unroll
-  for (int i = 0; i < TT + K - 1; ++i) {
-    const int t = t0 + i;
+  for (int q = 0; q < CONV_AHEAD; ++q) request(t0 + q, q);
+  int64_t off = ((int64_t)b * T + t0 - (K - 1)) * ldx + col0 + c;      // of row t - (K - 1)
+  for (int tb = t0; tb < tend; tb += CONV_AHEAD) {
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) { xall[i][v] = 0.0f; dall[i][v] = 0.0f; }
-    if (t < tend && t < T) { load(src + (int64_t)t * ldx, xall[i]); load(dsrc + (int64_t)t * X, dall[i]); }
-  }
+    for (int q = 0; q < CONV_AHEAD; ++q) {
+      const int t = tb + q;
+      if (t >= tend) break;
+      float xn[VEC], dn[VEC], g[VEC];
 #pragma unroll
-  for (int i = 0; i < TT + K - 1; ++i) {
-    const int t = t0 + i;
-    float xn[VEC], dn[VEC];
+      for (int v = 0; v < VEC; ++v) { xn[v] = xr[q][v]; dn[v] = dr[q][v]; }
+      request(t + CONV_AHEAD, q);
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) { xn[v] = xall[i][v]; dn[v] = dall[i][v]; }
-    float g[VEC];
+      for (int v = 0; v < VEC; ++v) {
 #pragma unroll
-    for (int v = 0; v < VEC; ++v) {
+        for (int k = 0; k < K - 1; ++k) { xin[v][k] = xin[v][k + 1]; dus[v][k] = dus[v][k + 1]; }
+        float du = 0.0f;
+        if (t < T) {
+          xin[v][K - 1] = xn[v];
+          float u = br[v];
 #pragma unroll
-      for (int k = 0; k < K - 1; ++k) { xin[v][k] = xin[v][k + 1]; dus[v][k] = dus[v][k + 1]; }
-      float du = 0.0f;
-      if (t < T) {
-        xin[v][K - 1] = xn[v];
-        float u = br[v];
+          for (int k = 0; k < K; ++k) u = fmaf(wr[v][k], xin[v][k], u);
+          float s = sigmoid_acc(u);
+          du = dn[v] * (s + u * s * (1.0f - s));
+          if (t < t1) {  // this run owns the parameter-gradient contribution of t in [t0,t1)
+            dbacc[v] += du;
 #pragma unroll
-        for (int k = 0; k < K; ++k) u = fmaf(wr[v][k], xin[v][k], u);
-        float s = sigmoid_acc(u);
-        du = dn[v] * (s + u * s * (1.0f - s));
-        if (t < t1) {  // this block owns the parameter-gradient contribution of t in [t0,t1)
-          dbacc[v] += du;
-#pragma unroll
-          for (int k = 0; k < K; ++k) dwacc[v][k] = fmaf(du, xin[v][k], dwacc[v][k]);
+            for (int k = 0; k < K; ++k) dwacc[v][k] = fmaf(du, xin[v][k], dwacc[v][k]);
+          }
         }
-      }
-      dus[v][K - 1] = du;
-      float acc = 0.0f;   // dxbc[tp] = sum_k w[k] * du[tp + (K-1) - k] = sum_k w[k] * dus[K-1-k]
+        dus[v][K - 1] = du;
+        float acc = 0.0f;   // dxbc[tp] = sum_k w[k] * du[tp + (K-1) - k] = sum_k w[k] * dus[K-1-k]
 #pragma unroll
-      for (int k = 0; k < K; ++k) acc = fmaf(wr[v][k], dus[v][K - 1 - k], acc);
-      g[v] = acc;
-    }
-    int tp = t - (K - 1);
-    if (t < tend && tp >= t0 && tp < t1) {
-      const int64_t off = ((int64_t)b * T + tp) * ldx + col0 + c;
-      if (pair_hi) {       // the gradient is only a GEMM operand: write it as a (hi, lo) bf16 pair with the same pitch
-        if (VEC == 4) store_pair4(pair_hi + off, pair_lo ? pair_lo + off : nullptr, g[0], g[1 % VEC], g[2 % VEC], g[3 % VEC]);
-        else { uint32_t h, l; split_bf16_pair(g[0], h, l); pair_hi[off] = (uint16_t)h; if (pair_lo) pair_lo[off] = (uint16_t)l; }
-      } else if (VEC == 4) *reinterpret_cast<float4*>(ddst + (int64_t)tp * ldx) = make_float4(g[0], g[1 % VEC], g[2 % VEC], g[3 % VEC]);
-      else ddst[(int64_t)tp * ldx] = g[0];
+        for (int k = 0; k < K; ++k) acc = fmaf(wr[v][k], dus[v][K - 1 - k], acc);
+        g[v] = acc;
+      }
+      if (t - (K - 1) >= t0) {
+        if (pair_hi) {       // the gradient is only a GEMM operand: write it as a (hi, lo) bf16 pair with the same pitch
+          if (VEC == 4) store_pair4(pair_hi + off, pair_lo ? pair_lo + off : nullptr, g[0], g[1 % VEC], g[2 % VEC], g[3 % VEC]);
+          else { uint32_t h, l; split_bf16_pair(g[0], h, l); pair_hi[off] = (uint16_t)h; if (pair_lo) pair_lo[off] = (uint16_t)l; }
+        } else if (VEC == 4) *reinterpret_cast<float4*>(dxzd + off) = make_float4(g[0], g[1 % VEC], g[2 % VEC], g[3 % VEC]);
+        else dxzd[off] = g[0];
+      }
+      off += ldx;
     }
   }
 }
 
 // partial = [gridDim.y rows of X*K weight partials][gridDim.y rows of X bias partials]
-// One thread = one channel group and TT time steps, its own partial row (any shape, any alignment).
-template <int K, int VEC, int TT>
+// One thread = VEC channels and a run of time steps, its own partial row (any shape, any alignment).
+template <int K, int VEC>
 __global__ void __launch_bounds__(128) conv_silu_bwd_kernel(const float* __restrict__ xzd, int64_t ldx, int col0,
                                                             const float* __restrict__ w, const float* __restrict__ bias,
                                                             const float* __restrict__ dact, float* __restrict__ dxzd,
-                                                            float* __restrict__ partial, int X, int T,
+                                                            float* __restrict__ partial, int X, int T, int run,
                                                             uint16_t* __restrict__ pair_hi, uint16_t* __restrict__ pair_lo) {
   int c = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (c >= X) return;
-  int tblocks = (T + TT - 1) / TT;
+  int tblocks = (T + run - 1) / run;
   int b = blockIdx.y / tblocks;
-  int t0 = (blockIdx.y % tblocks) * TT;
-  int t1 = min(t0 + TT, T);
+  int t0 = (blockIdx.y % tblocks) * run;
   float dwacc[VEC][K], dbacc[VEC];
-  conv_bwd_thread<K, VEC, TT>(xzd, ldx, col0, w, bias, dact, dxzd, X, T, pair_hi, pair_lo, c, b, t0, t1, dwacc, dbacc);
+  conv_bwd_thread<K, VEC>(xzd, ldx, col0, w, bias, dact, dxzd, X, T, pair_hi, pair_lo, c, b, t0, min(t0 + run, T), dwacc, dbacc);
   float* prow = partial + (int64_t)blockIdx.y * X * K;
   float* pbias = partial + (int64_t)gridDim.y * X * K + (int64_t)blockIdx.y * X;
 #pragma unroll
@@ -265,27 +285,22 @@ __global__ void __launch_bounds__(128) conv_silu_bwd_kernel(const float* __restr
   }
 }
 
-// The same work with the parameter-gradient partials summed inside the CTA: 128 threads = 16 time slices x 8 channel
-// quads (a 128-byte strip of every row), so a CTA covers 16 TT time steps of 32 channels and writes ONE partial row
-// entry per channel instead of one per thread: 16 times fewer partial bytes than the kernel above, which at a few
-// thousand tokens moved more partial sums than data.  Sums run in a fixed order (shuffles, then the warps in order).
-// (The thread keeps TT + K - 1 rows of two tensors in registers, about 170 of them: small CTAs let three share an SM.)
-constexpr int CONV_SLICES = 16;
-constexpr int CONV_STRIP_THREADS = CONV_SLICES * 8;
-template <int K, int TT>
-__global__ void __launch_bounds__(CONV_STRIP_THREADS) conv_silu_bwd_strip_kernel(const float* __restrict__ xzd, int64_t ldx, int col0,
+// The same work with the parameter-gradient partials summed inside the CTA: one partial row entry per channel and CTA instead of
+// one per thread, which at a few thousand tokens moved more partial sums than data.  Sums run in a fixed order (shuffles, then the
+// warps in order).
+template <int K>
+__global__ void __launch_bounds__(CONV_STRIP_THREADS, 3) conv_silu_bwd_strip_kernel(const float* __restrict__ xzd, int64_t ldx, int col0,
                                                                   const float* __restrict__ w, const float* __restrict__ bias,
                                                                   const float* __restrict__ dact, float* __restrict__ dxzd,
-                                                                  float* __restrict__ partial, int X, int T,
+                                                                  float* __restrict__ partial, int X, int T, int run,
                                                                   uint16_t* __restrict__ pair_hi, uint16_t* __restrict__ pair_lo) {
   constexpr int NV = 4 * K + 4, NW = CONV_STRIP_THREADS / 32;
   __shared__ float red[NW][8][NV];
   const int tx = threadIdx.x & 7, slice = threadIdx.x >> 3, warp = threadIdx.x >> 5;
   const int c = (blockIdx.x * 8 + tx) * 4;
-  const int tblocks = (T + CONV_SLICES * TT - 1) / (CONV_SLICES * TT);
+  const int tblocks = (T + CONV_SLICES * run - 1) / (CONV_SLICES * run);
   const int b = blockIdx.y / tblocks;
-  const int t0 = (blockIdx.y % tblocks) * (CONV_SLICES * TT) + slice * TT;
-  const int t1 = min(t0 + TT, T);
+  const int t0 = (blockIdx.y % tblocks) * (CONV_SLICES * run) + slice * run;
   float dwacc[4][K], dbacc[4];
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
@@ -293,7 +308,7 @@ __global__ void __launch_bounds__(CONV_STRIP_THREADS) conv_silu_bwd_strip_kernel
 #pragma unroll
     for (int k = 0; k < K; ++k) dwacc[v][k] = 0.0f;
   }
-  if (c < X && t0 < T) conv_bwd_thread<K, 4, TT>(xzd, ldx, col0, w, bias, dact, dxzd, X, T, pair_hi, pair_lo, c, b, t0, t1, dwacc, dbacc);
+  if (c < X && t0 < T) conv_bwd_thread<K, 4>(xzd, ldx, col0, w, bias, dact, dxzd, X, T, pair_hi, pair_lo, c, b, t0, min(t0 + run, T), dwacc, dbacc);
   float vals[NV];
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
@@ -324,24 +339,13 @@ __global__ void __launch_bounds__(CONV_STRIP_THREADS) conv_silu_bwd_strip_kernel
   }
 }
 
-// time steps per thread: long runs recompute fewer halo rows (K - 1 per run) and write fewer partial sums; measured at
-// 2048 tokens with the strip kernel: 4 steps 49 us, 8 steps 42 us, 16 steps 55 us per launch (PMB_CONV_TT overrides)
-static int conv_bwd_tt(const Dims& d) {
-  static const int forced = [] { const char* e = getenv("PMB_CONV_TT"); return e ? atoi(e) : 0; }();
-  if (forced == 4 || forced == 8 || forced == 16) return forced;
-  return d.M >= 32768 ? 16 : 8;
-}
-
 size_t conv_bwd_ws_bytes(const Dims& d) {
-  const int CONV_BWD_TT = conv_bwd_tt(d);
-  int tblocks = (d.T + CONV_BWD_TT - 1) / CONV_BWD_TT;
-  return align_up((size_t)d.B * tblocks * d.X * (d.K + 1) * sizeof(float), 256);
+  return align_up((size_t)d.B * cdiv(d.T, conv_run(d)) * d.X * (d.K + 1) * sizeof(float), 256);
 }
 
 // Rows of `partial` the launch below writes (what column_sum has to add up).
 static int64_t conv_bwd_partial_rows(const Dims& d, bool strip) {
-  const int tt = conv_bwd_tt(d);
-  return (int64_t)d.B * (strip ? cdiv(d.T, CONV_SLICES * tt) : cdiv(d.T, tt));
+  return (int64_t)d.B * cdiv(d.T, (strip ? CONV_SLICES : 1) * conv_run(d));
 }
 static bool conv_bwd_strip_ok(const Dims& d, const float* xzd, const float* dact, const float* dxzd) {
   return (d.X % 4 == 0) && (d.J % 4 == 0) && (d.I % 4 == 0) && d.K <= 4 &&
@@ -351,27 +355,18 @@ static bool conv_bwd_strip_ok(const Dims& d, const float* xzd, const float* dact
 template <int K>
 static pmb_status launch_conv_bwd_k(cudaStream_t st, const Dims& d, const float* xzd, const float* w, const float* b,
                                     const float* dact, float* dxzd, float* partial, uint16_t* pair_hi, uint16_t* pair_lo) {
-  const int tt = conv_bwd_tt(d);
-  int tblocks = (d.T + tt - 1) / tt;
+  const int run = conv_run(d);
+  const bool strip = conv_bwd_strip_ok(d, xzd, dact, dxzd);
   bool vec = (d.X % 4 == 0) && (d.J % 4 == 0) && (d.I % 4 == 0) &&
              ((reinterpret_cast<uintptr_t>(xzd) | reinterpret_cast<uintptr_t>(dact) | reinterpret_cast<uintptr_t>(dxzd)) % 16 == 0);
-  if (conv_bwd_strip_ok(d, xzd, dact, dxzd)) {
-    if constexpr (K <= 4) {
-      dim3 grid((unsigned)cdiv(d.X, 32), (unsigned)conv_bwd_partial_rows(d, true));
-      if (tt == 16) conv_silu_bwd_strip_kernel<K, 16><<<grid, CONV_STRIP_THREADS, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, pair_hi, pair_lo);
-      else if (tt == 8) conv_silu_bwd_strip_kernel<K, 8><<<grid, CONV_STRIP_THREADS, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, pair_hi, pair_lo);
-      else conv_silu_bwd_strip_kernel<K, 4><<<grid, CONV_STRIP_THREADS, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, pair_hi, pair_lo);
-    }
+  const unsigned rows = (unsigned)conv_bwd_partial_rows(d, strip);
+  if (strip) {
+    if constexpr (K <= 4)
+      conv_silu_bwd_strip_kernel<K><<<dim3((unsigned)cdiv(d.X, 32), rows), CONV_STRIP_THREADS, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, run, pair_hi, pair_lo);
   } else if (vec) {
-    dim3 grid((unsigned)cdiv(d.X / 4, 128), (unsigned)(d.B * tblocks));
-    if (tt == 16) conv_silu_bwd_kernel<K, 4, 16><<<grid, 128, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, pair_hi, pair_lo);
-    else if (tt == 8) conv_silu_bwd_kernel<K, 4, 8><<<grid, 128, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, pair_hi, pair_lo);
-    else conv_silu_bwd_kernel<K, 4, 4><<<grid, 128, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, pair_hi, pair_lo);
+    conv_silu_bwd_kernel<K, 4><<<dim3((unsigned)cdiv(d.X / 4, 128), rows), 128, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, run, pair_hi, pair_lo);
   } else {
-    dim3 grid((unsigned)cdiv(d.X, 128), (unsigned)(d.B * tblocks));
-    if (tt == 16) conv_silu_bwd_kernel<K, 1, 16><<<grid, 128, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, pair_hi, pair_lo);
-    else if (tt == 8) conv_silu_bwd_kernel<K, 1, 8><<<grid, 128, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, pair_hi, pair_lo);
-    else conv_silu_bwd_kernel<K, 1, 4><<<grid, 128, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, pair_hi, pair_lo);
+    conv_silu_bwd_kernel<K, 1><<<dim3((unsigned)cdiv(d.X, 128), rows), 128, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, run, pair_hi, pair_lo);
   }
   PMB_LAUNCHED();
   return PMB_OK;
@@ -396,9 +391,9 @@ pmb_status conv_silu_bwd(cudaStream_t st, const Dims& d, const float* xzd, const
   const int64_t rows = conv_bwd_partial_rows(d, conv_bwd_strip_ok(d, xzd, dact, dxzd));
   cudaStream_t rs = st;
   if (red) { PMB_TRY(order_after(st, red->ev[4], red->s)); rs = red->s; }
-  column_sum_kernel<<<(unsigned)cdiv(d.X * d.K, 32), 256, 0, rs>>>(partial, rows, d.X * d.K, dw);
+  column_sum_kernel<<<(unsigned)cdiv(d.X * d.K, 32), 32 * COLSUM_LANES, 0, rs>>>(partial, rows, d.X * d.K, dw);
   PMB_LAUNCHED();
-  column_sum_kernel<<<(unsigned)cdiv(d.X, 32), 256, 0, rs>>>(partial + rows * d.X * d.K, rows, d.X, db);
+  column_sum_kernel<<<(unsigned)cdiv(d.X, 32), 32 * COLSUM_LANES, 0, rs>>>(partial + rows * d.X * d.K, rows, d.X, db);
   PMB_LAUNCHED();
   return PMB_OK;
 }
@@ -452,40 +447,59 @@ __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_fwd_kernel(const f
   }
 }
 
-// float4 variant: width % 4 == 0, 16-byte aligned rows.  PER float4 per thread, blockDim.x * PER >= width / 4.
+// Sum over the block with one barrier: every warp adds up the warps' sums itself (the same tree in each, the one of block_sum).
+// `red` alternates between two buffers from call to call, so that no second barrier keeps a fast warp out.
+__device__ __forceinline__ float block_sum_once(float v, float* red) {
+  const int lane = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+  v = warp_sum(v);
+  if (lane == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return warp_sum(lane < nw ? red[lane] : 0.0f);
+}
+
+// float4 variant: width % 4 == 0, 16-byte aligned rows.  PER float4 per thread, blockDim.x * PER >= width / 4.  Bound by HBM; a block
+// walks `nrows` rows and requests the next one before it reduces the current one.  Measured at 16384 rows of 1536 with a bf16 output
+// (250 MB): 51 us with a block per row, @F.
 template <int PER>
 __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_fwd_vec_kernel(const float* __restrict__ y, const float* __restrict__ z,
                                                                              int64_t ldz, const float* __restrict__ w,
                                                                              float* __restrict__ out, float* __restrict__ rstd,
                                                                              int width, float eps, uint16_t* __restrict__ out_hi,
-                                                                             uint16_t* __restrict__ out_lo) {
-  __shared__ float red[32];
-  const int64_t row = blockIdx.x;
+                                                                             uint16_t* __restrict__ out_lo, int64_t rows, int nrows) {
+  __shared__ float red[2][32];
   const int nvec = width >> 2;
-  const float4* y4 = reinterpret_cast<const float4*>(y + row * width);
-  const float4* z4 = reinterpret_cast<const float4*>(z + row * ldz);
-  float4 g[PER];
-  float ss = 0.0f;
+  const int64_t r0 = (int64_t)blockIdx.x * nrows;
+  const int64_t r1 = r0 + nrows < rows ? r0 + nrows : rows;
+  float4 yn[PER], zn[PER];
+  auto request = [&](int64_t row) {
 #pragma unroll
-  for (int n = 0; n < PER; ++n) {
-    const int i = threadIdx.x + n * blockDim.x;
-    g[n] = make_float4(0, 0, 0, 0);
-    if (i < nvec) {
-      const float4 yv = y4[i], zv = z4[i];
-      g[n] = make_float4(yv.x * zv.x * sigmoid_acc(zv.x), yv.y * zv.y * sigmoid_acc(zv.y), yv.z * zv.z * sigmoid_acc(zv.z),
-                         yv.w * zv.w * sigmoid_acc(zv.w));
-      ss = fmaf(g[n].x, g[n].x, fmaf(g[n].y, g[n].y, fmaf(g[n].z, g[n].z, fmaf(g[n].w, g[n].w, ss))));
+    for (int n = 0; n < PER; ++n) {
+      const int i = threadIdx.x + n * blockDim.x;
+      yn[n] = zn[n] = make_float4(0, 0, 0, 0);
+      if (i < nvec) { yn[n] = reinterpret_cast<const float4*>(y + row * width)[i]; zn[n] = reinterpret_cast<const float4*>(z + row * ldz)[i]; }
     }
-  }
-  const float tot = block_sum(ss, red);
-  const float r = 1.0f / sqrtf(tot / (float)width + eps);
-  if (threadIdx.x == 0 && rstd) rstd[row] = r;
+  };
   auto split = [](float v, uint32_t& h, uint32_t& l) {   // (hi, lo) bf16 pair, round to nearest even
     const uint32_t u = __float_as_uint(v);
     h = (u + 0x7fffu + ((u >> 16) & 1u)) >> 16;
     const uint32_t ul = __float_as_uint(v - __uint_as_float(h << 16));
     l = (ul + 0x7fffu + ((ul >> 16) & 1u)) >> 16;
   };
+  if (r0 < r1) request(r0);
+  for (int64_t row = r0; row < r1; ++row) {
+  float4 g[PER];
+  float ss = 0.0f;
+#pragma unroll
+  for (int n = 0; n < PER; ++n) {
+    const float4 yv = yn[n], zv = zn[n];
+    g[n] = make_float4(yv.x * zv.x * sigmoid_acc(zv.x), yv.y * zv.y * sigmoid_acc(zv.y), yv.z * zv.z * sigmoid_acc(zv.z),
+                       yv.w * zv.w * sigmoid_acc(zv.w));
+    ss = fmaf(g[n].x, g[n].x, fmaf(g[n].y, g[n].y, fmaf(g[n].z, g[n].z, fmaf(g[n].w, g[n].w, ss))));
+  }
+  if (row + 1 < r1) request(row + 1);
+  const float tot = block_sum_once(ss, red[row & 1]);
+  const float r = 1.0f / sqrtf(tot / (float)width + eps);
+  if (threadIdx.x == 0 && rstd) rstd[row] = r;
 #pragma unroll
   for (int n = 0; n < PER; ++n) {
     const int i = threadIdx.x + n * blockDim.x;
@@ -500,6 +514,7 @@ __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_fwd_vec_kernel(con
         if (out_lo) reinterpret_cast<uint2*>(out_lo + row * width)[i] = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
       }
     }
+  }
   }
 }
 
@@ -522,8 +537,11 @@ pmb_status gated_rmsnorm_fwd(cudaStream_t st, int64_t rows, int width, float eps
   if (norm_vec_ok(width, ldz, y, z, w, out, out_hi) && (!out_lo || (reinterpret_cast<uintptr_t>(out_lo) & 15) == 0)) {
     int per = 1;
     const int threads = norm_vec_threads(width, &per);
-    if (per == 1) gated_rmsnorm_fwd_vec_kernel<1><<<(unsigned)rows, threads, 0, st>>>(y, z, ldz, w, out, rstd, width, eps, out_hi, out_lo);
-    else gated_rmsnorm_fwd_vec_kernel<2><<<(unsigned)rows, threads, 0, st>>>(y, z, ldz, w, out, rstd, width, eps, out_hi, out_lo);
+    // four to eight blocks share an SM; with fewer rows than fill it that way every row has a block
+    const int nr = (int)cdiv(rows, 148 * 6);
+    const unsigned nblk = (unsigned)cdiv(rows, nr);
+    if (per == 1) gated_rmsnorm_fwd_vec_kernel<1><<<nblk, threads, 0, st>>>(y, z, ldz, w, out, rstd, width, eps, out_hi, out_lo, rows, nr);
+    else gated_rmsnorm_fwd_vec_kernel<2><<<nblk, threads, 0, st>>>(y, z, ldz, w, out, rstd, width, eps, out_hi, out_lo, rows, nr);
     PMB_LAUNCHED();
     return PMB_OK;
   }
@@ -585,16 +603,19 @@ __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_bwd_kernel(const f
   }
 }
 
-// float4 variant of the backward (same row blocking and partial layout).  Optional extras (see NormBwdExtra):
-// dz as a (hi, lo) bf16 pair instead of fp32, and dY exp(S) for the scan backward.
+// float4 variant of the backward.  Optional extras (see NormBwdExtra): dz as a (hi, lo) bf16 pair instead of fp32, and dY exp(S) for
+// the scan backward.  Bound by HBM (reads of dout, y, z, writes of dy and the bf16 copies).  A block walks `nrows` rows and requests
+// the next one before it reduces the current one; few long blocks also leave few partial sums of dw (one row of them per block).
+// Measured at 16384 rows of 1536 with plain bf16 copies (550 MB): 136 us + 60 us of partial sums with four rows per block and no
+// request ahead, @N.
 template <int PER>
-__global__ void __launch_bounds__(NORM_THREADS, 3) gated_rmsnorm_bwd_vec_kernel(const float* __restrict__ dout, const float* __restrict__ y,
+__global__ void __launch_bounds__(NORM_THREADS, 2) gated_rmsnorm_bwd_vec_kernel(const float* __restrict__ dout, const float* __restrict__ y,
                                                                              const float* __restrict__ z, int64_t ldz,
                                                                              const float* __restrict__ w, const float* __restrict__ rstd,
                                                                              float* __restrict__ dy, float* __restrict__ dz, int64_t lddz,
-                                                                             float* __restrict__ dw_partial, int64_t rows, int width,
+                                                                             float* __restrict__ dw_partial, int64_t rows, int width, int nrows,
                                                                              NormBwdExtra ex) {
-  __shared__ float red[32];
+  __shared__ float red[2][32];
   const int nvec = width >> 2;
   float4 dwacc[PER], wv[PER];
 #pragma unroll
@@ -603,30 +624,36 @@ __global__ void __launch_bounds__(NORM_THREADS, 3) gated_rmsnorm_bwd_vec_kernel(
     dwacc[n] = make_float4(0, 0, 0, 0);
     wv[n] = i < nvec ? reinterpret_cast<const float4*>(w)[i] : make_float4(0, 0, 0, 0);
   }
-  const int64_t r0 = (int64_t)blockIdx.x * NORM_ROWS;
-  for (int rr = 0; rr < NORM_ROWS; ++rr) {
-    const int64_t row = r0 + rr;
-    if (row >= rows) break;  // uniform across the block
+  const int64_t r0 = (int64_t)blockIdx.x * nrows;
+  const int64_t r1 = r0 + nrows < rows ? r0 + nrows : rows;
+  float4 zn[PER], yn[PER], dnn[PER];
+  auto request = [&](int64_t row) {
+#pragma unroll
+    for (int n = 0; n < PER; ++n) {
+      const int i = threadIdx.x + n * blockDim.x;
+      zn[n] = yn[n] = dnn[n] = make_float4(0, 0, 0, 0);
+      if (i < nvec) {
+        zn[n] = reinterpret_cast<const float4*>(z + row * ldz)[i];
+        yn[n] = reinterpret_cast<const float4*>(y + row * width)[i];
+        dnn[n] = reinterpret_cast<const float4*>(dout + row * width)[i];
+      }
+    }
+  };
+  if (r0 < r1) request(r0);
+  for (int64_t row = r0; row < r1; ++row) {
     const float r = rstd[row];
     float4 zv[PER], yv[PER], dn[PER], gv[PER], sv[PER];
     float dot = 0.0f;
 #pragma unroll
-    for (int n = 0; n < PER; ++n) {
-      const int i = threadIdx.x + n * blockDim.x;
-      zv[n] = yv[n] = dn[n] = gv[n] = sv[n] = make_float4(0, 0, 0, 0);
-      if (i < nvec) {
-        zv[n] = reinterpret_cast<const float4*>(z + row * ldz)[i];
-        yv[n] = reinterpret_cast<const float4*>(y + row * width)[i];
-        dn[n] = reinterpret_cast<const float4*>(dout + row * width)[i];
-      }
-    }
+    for (int n = 0; n < PER; ++n) { zv[n] = zn[n]; yv[n] = yn[n]; dn[n] = dnn[n]; }
+    if (row + 1 < r1) request(row + 1);
 #pragma unroll
     for (int n = 0; n < PER; ++n) {
       sv[n] = make_float4(sigmoid_acc(zv[n].x), sigmoid_acc(zv[n].y), sigmoid_acc(zv[n].z), sigmoid_acc(zv[n].w));
       gv[n] = make_float4(yv[n].x * zv[n].x * sv[n].x, yv[n].y * zv[n].y * sv[n].y, yv[n].z * zv[n].z * sv[n].z, yv[n].w * zv[n].w * sv[n].w);
       dot = fmaf(dn[n].x * gv[n].x, wv[n].x, fmaf(dn[n].y * gv[n].y, wv[n].y, fmaf(dn[n].z * gv[n].z, wv[n].z, fmaf(dn[n].w * gv[n].w, wv[n].w, dot))));
     }
-    const float tot = block_sum(dot, red);
+    const float tot = block_sum_once(dot, red[row & 1]);
     const float coef = r * r * r * tot / (float)width;
 #pragma unroll
     for (int n = 0; n < PER; ++n) {
@@ -666,21 +693,24 @@ __global__ void __launch_bounds__(NORM_THREADS, 3) gated_rmsnorm_bwd_vec_kernel(
   }
 }
 
-// out[j] = sum_r partial[r*cols + j].  Block = 32 columns x 8 row lanes; each lane sums rows ty, ty+8, ...
-// and the 8 lane sums are added in a fixed order (deterministic).
-__global__ void __launch_bounds__(256) column_sum_kernel(const float* __restrict__ partial, int64_t rows, int cols, float* __restrict__ out) {
-  __shared__ float sh[8][33];
+// out[j] = sum_r partial[r*cols + j].  Block = 32 columns x COLSUM_LANES row lanes; each lane sums rows ty, ty + COLSUM_LANES, ...
+// (four loads in flight) and the lanes' sums are added in a fixed order (deterministic).  The columns alone give few blocks, so
+// what counts is the length of a lane's chain of loads: 23 us for 4096 rows of 1536 columns with 8 lanes.
+__global__ void __launch_bounds__(32 * COLSUM_LANES) column_sum_kernel(const float* __restrict__ partial, int64_t rows, int cols, float* __restrict__ out) {
+  __shared__ float sh[COLSUM_LANES][33];
   int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   int j = blockIdx.x * 32 + tx;
   float s = 0.0f;
-  if (j < cols)
-    for (int64_t r = ty; r < rows; r += 8) s += partial[r * cols + j];
+  if (j < cols) {
+#pragma unroll 4
+    for (int64_t r = ty; r < rows; r += COLSUM_LANES) s += partial[r * cols + j];
+  }
   sh[ty][tx] = s;
   __syncthreads();
   if (ty == 0 && j < cols) {
     float t = 0.0f;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) t += sh[k][tx];
+    for (int k = 0; k < COLSUM_LANES; ++k) t += sh[k][tx];
     out[j] = t;
   }
 }
@@ -697,23 +727,27 @@ pmb_status gated_rmsnorm_bwd(cudaStream_t st, int64_t rows, int width, const flo
   if (width > NORM_THREADS * NORM_MAX_PER_THREAD) return fail(PMB_ERR_SHAPE, "rmsnorm width %d too large", width);
   if (ws_bytes < gated_rmsnorm_bwd_ws_bytes(rows, width)) return fail(PMB_ERR_WORKSPACE, "rmsnorm bwd workspace too small");
   float* partial = static_cast<float*>(ws);
-  int64_t nblk = cdiv(rows, NORM_ROWS);
   ProfScope prof(st, "gated_rmsnorm_bwd", 0.0, 4.0 * rows * 5.0 * width);
+  int64_t nblk = cdiv(rows, NORM_ROWS);
   const bool vec_ok = norm_vec_ok(width, ldz, dout, y, z, w, dy) && (lddz % 4 == 0) &&
                       ((reinterpret_cast<uintptr_t>(dz) | reinterpret_cast<uintptr_t>(partial)) & 15) == 0;
   if ((ex.dz_hi || ex.dys || ex.dy_hi || ex.dys_hi) && !vec_ok) return fail(PMB_ERR_UNSUPPORTED, "gated_rmsnorm_bwd: pair / scaled outputs need the vector kernel's alignment");
   if (vec_ok) {
     int per = 1;
     const int threads = norm_vec_threads(width, &per);
-    if (per == 1) gated_rmsnorm_bwd_vec_kernel<1><<<(unsigned)nblk, threads, 0, st>>>(dout, y, z, ldz, w, rstd, dy, dz, lddz, partial, rows, width, ex);
-    else gated_rmsnorm_bwd_vec_kernel<2><<<(unsigned)nblk, threads, 0, st>>>(dout, y, z, ldz, w, rstd, dy, dz, lddz, partial, rows, width, ex);
+    // two blocks per SM walk the rows; below four rows each the partial sums would outgrow the workspace's rows
+    int64_t nr = cdiv(rows, 2 * 148);
+    if (nr < NORM_ROWS) nr = NORM_ROWS;
+    nblk = cdiv(rows, nr);
+    if (per == 1) gated_rmsnorm_bwd_vec_kernel<1><<<(unsigned)nblk, threads, 0, st>>>(dout, y, z, ldz, w, rstd, dy, dz, lddz, partial, rows, width, (int)nr, ex);
+    else gated_rmsnorm_bwd_vec_kernel<2><<<(unsigned)nblk, threads, 0, st>>>(dout, y, z, ldz, w, rstd, dy, dz, lddz, partial, rows, width, (int)nr, ex);
   } else {
     gated_rmsnorm_bwd_kernel<<<(unsigned)nblk, NORM_THREADS, 0, st>>>(dout, y, z, ldz, w, rstd, dy, dz, lddz, partial, rows, width);
   }
   PMB_LAUNCHED();
   cudaStream_t rs = st;
   if (red) { PMB_TRY(order_after(st, red->ev[4], red->s)); rs = red->s; }
-  column_sum_kernel<<<(unsigned)cdiv(width, 32), 256, 0, rs>>>(partial, nblk, width, dw);
+  column_sum_kernel<<<(unsigned)cdiv(width, 32), 32 * COLSUM_LANES, 0, rs>>>(partial, nblk, width, dw);
   PMB_LAUNCHED();
   return PMB_OK;
 }
@@ -765,7 +799,7 @@ pmb_status gated_rmsnorm_bwd_static(cudaStream_t st, int64_t rows, int width, co
 }
 
 pmb_status column_sum(cudaStream_t st, const float* partial, int64_t rows, int cols, float* out) {
-  column_sum_kernel<<<(unsigned)cdiv(cols, 32), 256, 0, st>>>(partial, rows, cols, out);
+  column_sum_kernel<<<(unsigned)cdiv(cols, 32), 32 * COLSUM_LANES, 0, st>>>(partial, rows, cols, out);
   PMB_LAUNCHED();
   return PMB_OK;
 }
