@@ -14,7 +14,8 @@ __global__ void column_sum_kernel(const float* __restrict__ partial, int64_t row
 // registers and the next CONV_AHEAD rows on their way, so that every global access is a coalesced vector access and each input
 // row is read (run+K-1)/run times.  Bound by HBM.  A CTA of the vector kernels is 16 runs of 8 channel quads (128-byte strips of
 // its rows): no thread is idle for any channel count that is a multiple of 32.
-// Measured at 8 x 2048 tokens of 1664 channels: forward 68 us with runs of 8 all requested up front, @CF; backward 131 us, @CB.
+// Measured at 8 x 2048 tokens of 1664 channels: forward 68 us with runs of 8 all requested up front, 49 now;
+// backward 131 us, 110 now.
 // ---------------------------------------------------------------------------------------------
 constexpr int CONV_AHEAD = 4;
 constexpr int CONV_SLICES = 16;
@@ -459,7 +460,7 @@ __device__ __forceinline__ float block_sum_once(float v, float* red) {
 
 // float4 variant: width % 4 == 0, 16-byte aligned rows.  PER float4 per thread, blockDim.x * PER >= width / 4.  Bound by HBM; a block
 // walks `nrows` rows and requests the next one before it reduces the current one.  Measured at 16384 rows of 1536 with a bf16 output
-// (250 MB): 51 us with a block per row, @F.
+// (250 MB): 51 us with a block per row, 44 now.
 template <int PER>
 __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_fwd_vec_kernel(const float* __restrict__ y, const float* __restrict__ z,
                                                                              int64_t ldz, const float* __restrict__ w,
@@ -607,7 +608,7 @@ __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_bwd_kernel(const f
 // the scan backward.  Bound by HBM (reads of dout, y, z, writes of dy and the bf16 copies).  A block walks `nrows` rows and requests
 // the next one before it reduces the current one; few long blocks also leave few partial sums of dw (one row of them per block).
 // Measured at 16384 rows of 1536 with plain bf16 copies (550 MB): 136 us + 60 us of partial sums with four rows per block and no
-// request ahead, @N.
+// request ahead, 145 us + 3 now.
 template <int PER>
 __global__ void __launch_bounds__(NORM_THREADS, 2) gated_rmsnorm_bwd_vec_kernel(const float* __restrict__ dout, const float* __restrict__ y,
                                                                              const float* __restrict__ z, int64_t ldz,
