@@ -66,7 +66,10 @@ struct Params {
   int M, N, K;
   int a_mn_major, b_mn_major;
   void* C; int64_t ldc; const void* R; int out_bf16;
-  int tma_out;     // fp32 result (and residual) meet the TMA rules: the epilogue stores through shared memory
+  int tma_out;     // result (and residual) meet the TMA rules: the epilogue stores through shared memory
+  int red;         // fp32 result added onto C: the TMA store adds in L2 and no residual block is loaded
+  int bn;          // width of the persistent CTA-pair kernel's tiles (256 or 128)
+  int pairs;       // operands are (hi, lo) pairs
   uint16_t* e_hi; uint16_t* e_lo; int64_t lde;   // optional second output: the result as a bf16 pair (TMA-store epilogue only)
   // split K: tiles of split i cover k-tiles [i * kt_per, (i + 1) * kt_per) and go to rows i * slab_rows .. of C, whose
   // slabs the caller adds up (kt_per covers all of K when there is one split)
@@ -147,7 +150,7 @@ constexpr int MAX_GROUP = 4;
 // each; meanwhile the other clusters take `rounds` of the short tiles each, and what is left goes round all of them.
 // (Round-robin alone would give the clusters with a long tile their full share of the short ones on top.)
 struct Group { Problem pr[MAX_GROUP]; int lead, rounds; };
-__device__ __forceinline__ int pair_tile_at(const Group& g, int c, int clusters, int j) {
+__host__ __device__ __forceinline__ int pair_tile_at(const Group& g, int c, int clusters, int j) {
   if (g.lead == 0) return c + j * clusters;
   const int f = clusters - g.lead;
   if (c < g.lead) return j == 0 ? c : g.lead + f * g.rounds + (j - 1) * clusters + c;
@@ -179,42 +182,121 @@ template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // Epilogue of one tile for one epilogue warp: its 32 rows (row0 ..) x `ncols` columns (n0 ..) of the accumulator at
-// `tmem_acc` (lane offset included).  fp32 results that meet the TMA rules leave through the warp's two swizzled
-// staging slots (slot0) and TMA stores, the residual block TMA-loaded into the slot first (barriers rbar0 / rbar1);
-// everything else is stored row by row.  `st` carries the slot parity and the residual barriers' phases across tiles.
-struct EpiState { uint32_t pc = 0, rph0 = 0, rph1 = 0; };
-__device__ __forceinline__ void epilogue_rows(const Problem& q, const Params& p, uint32_t tmem_acc, int row0, int rowoff, int n0, int ncols, uint32_t slot0,
-                                              uint32_t rbar0, uint32_t rbar1, EpiState& st, int lane, volatile uint32_t* abort_flag) {
-  if (p.tma_out) {
-    if (row0 < p.M) {
-      const bool res = p.R != nullptr;
-      if (res && lane == 0) {
-        const uint32_t slot = st.pc & 1u;
-        mbar_expect_tx((slot ? rbar1 : rbar0), EPI_SLOT_BYTES);
-        tma_load_2d(slot0 + slot * EPI_SLOT_BYTES, &q.mR, n0, row0, (slot ? rbar1 : rbar0));
-      }
+// `tmem_acc` (lane offset included).  Results that meet the TMA rules leave through the warp's NSLOT swizzled staging slots of 32
+// rows of 128 bytes (32 fp32 or 64 bf16 columns) and TMA stores.  The residual blocks are TMA-loaded into the slots: the first NSLOT
+// of a tile by prefetch(), while its products still run (four slots hold all of a 256-wide bf16 tile), further ones as soon as
+// a slot's store has read it.  Everything else is stored row by row.  `pc` and `rph` carry the slot in turn and the residual
+// barriers' phases across tiles.
+__device__ __forceinline__ void tma_add_2d(const CUtensorMap* map, uint32_t src, int c0, int c1) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(src) : "memory");
+}
+template <int NSLOT>
+struct Epilogue {
+  uint32_t slot0, rbar0;                     // the warp's slots and their residual barriers (8 bytes apart)
+  uint32_t pc = 0, rph = 0, loading = 0;     // (loading: lane 0's record of the slots with a load in flight)
+  __device__ __forceinline__ bool loads(const Params& p) const { return p.tma_out && p.R && !p.red; }
+  __device__ __forceinline__ void load(const Problem& q, uint32_t slot, int c, int row0) {
+    mbar_expect_tx(rbar0 + 8u * slot, EPI_SLOT_BYTES);
+    tma_load_2d(slot0 + slot * EPI_SLOT_BYTES, &q.mR, c, row0, rbar0 + 8u * slot);
+    loading |= 1u << slot;
+  }
+  __device__ __forceinline__ void prefetch(const Problem& q, const Params& p, int row0, int n0, int ncols, int lane) {
+    if (!loads(p) || row0 >= p.M || n0 >= p.N || lane != 0) return;
+    const int bw = p.out_bf16 ? 64 : 32, end = min(ncols, p.N - n0);
+    bulk_wait_read<0>();
+    for (int i = 0; i < NSLOT && i * bw < end; ++i) load(q, (pc + i) % NSLOT, n0 + i * bw, row0);
+  }
+  // before the CTA leaves: stores have been written, loads (of a tile that was given up) have landed or are given up on
+  __device__ __forceinline__ void drain(int lane) {
+    if (lane != 0) return;
+    for (int i = 0; i < NSLOT; ++i) if ((loading >> i) & 1u) mbar_wait(rbar0 + 8u * i, (rph >> i) & 1u);
+    bulk_wait_all();
+  }
+  __device__ __forceinline__ void run(const Problem& q, const Params& p, uint32_t tmem_acc, int row0, int rowoff, int n0, int ncols, int lane, volatile uint32_t* abort_flag) {
+    if (!p.tma_out) {
+      const int m = row0 + lane;
 #pragma unroll 1
-      for (int c0 = 0; c0 < ncols && n0 + c0 < p.N; c0 += 32) {
-        const uint32_t slot = st.pc & 1u;
-        const uint32_t sbase = slot0 + slot * EPI_SLOT_BYTES + (uint32_t)lane * 128u;
+      for (int c0 = 0; c0 < ncols; c0 += 32) {
         uint32_t r[32];
         tmem_ld32(tmem_acc + (uint32_t)c0, r);
-        if (res) {
-          const uint32_t rp = slot ? st.rph1 : st.rph0;
-          const bool landed = __all_sync(0xffffffffu, mbar_wait((slot ? rbar1 : rbar0), rp));
-          if (slot) st.rph1 ^= 1u; else st.rph0 ^= 1u;
-          if (!landed) { if (lane == 0) { atomicOr(&g_bf16_status, 16u); *abort_flag = 1; } }
-          else {
+        if (m < p.M) store_row_piece(p, rowoff + m, n0 + c0, r);
+      }
+      return;
+    }
+    if (row0 >= p.M) return;
+    const bool res = loads(p);
+    if (!res && !p.red && !p.e_hi && !p.out_bf16) {
+      // nothing to add and fp32: 16 x 8 fragments go out as they are, a quad of lanes one whole 32-byte sector, and nobody waits
+      const int r = row0 + (lane >> 2), c = n0 + (lane & 3) * 2;
+      float* base = static_cast<float*>(p.C) + (int64_t)(rowoff + r) * p.ldc + c;
+#pragma unroll 1
+      for (int c0 = 0; c0 < ncols && n0 + c0 < p.N; c0 += 32) {
+        uint32_t v[4][8];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              float4 v;
-              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                           : "r"(sbase + (uint32_t)((j ^ (lane & 7)) * 16)));
-              r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + v.x);
-              r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + v.y);
-              r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + v.z);
-              r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + v.w);
+        for (int i = 0; i < 4; ++i) tmem_ld16x256_x2(tmem_acc + ((uint32_t)(16 * (i >> 1)) << 16) + (uint32_t)(c0 + 16 * (i & 1)), v[i]);
+        tmem_wait_ld();
+        auto put = [&](bool inside) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {                   // e & 1: row + 8, e >> 1: columns + 8
+              const int dr = 16 * (i >> 1) + 8 * (e & 1), dc = c0 + 16 * (i & 1) + 8 * (e >> 1);
+              const uint2 o = make_uint2(v[i][4 * (e >> 1) + 2 * (e & 1)], v[i][4 * (e >> 1) + 2 * (e & 1) + 1]);
+              float* at = base + (int64_t)dr * p.ldc + dc;
+              if (inside || (r + dr < p.M && c + dc + 1 < p.N)) *reinterpret_cast<uint2*>(at) = o;
+              else if (r + dr < p.M && c + dc < p.N) *at = __uint_as_float(o.x);
             }
+        };
+        if (row0 + 32 <= p.M && n0 + c0 + 32 <= p.N) put(true); else put(false);
+      }
+      return;
+    }
+    const int bw = p.out_bf16 ? 64 : 32, end = min(ncols, p.N - n0);
+#pragma unroll 1
+    for (int c0 = 0; c0 < end; c0 += bw) {
+      const uint32_t slot = pc % NSLOT, sbase = slot0 + slot * EPI_SLOT_BYTES + (uint32_t)lane * 128u;
+      bool landed = res;
+      if (res) {
+        landed = __all_sync(0xffffffffu, mbar_wait(rbar0 + 8u * slot, (rph >> slot) & 1u));
+        rph ^= 1u << slot;
+        loading &= ~(1u << slot);
+        if (!landed && lane == 0) { atomicOr(&g_bf16_status, 16u); *abort_flag = 1; }
+      }
+#pragma unroll 1
+      for (int half = 0; 32 * half < bw; ++half) {
+        uint32_t r[32];
+        tmem_ld32(tmem_acc + (uint32_t)(c0 + 32 * half), r);
+        if (p.out_bf16) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const uint32_t at = sbase + (uint32_t)(((4 * half + j) ^ (lane & 7)) * 16);
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(r[8 * j + e]);
+            if (landed) {
+              uint32_t w[4];
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(at));
+#pragma unroll
+              for (int e = 0; e < 4; ++e) { v[2 * e] += __uint_as_float(w[e] << 16); v[2 * e + 1] += __uint_as_float(w[e] & 0xffff0000u); }
+            }
+            uint32_t o[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[e] = (uint32_t)float_to_bf16_bits(v[2 * e]) | ((uint32_t)float_to_bf16_bits(v[2 * e + 1]) << 16);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+          }
+          continue;
+        }
+        if (landed) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            float4 v;
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                         : "r"(sbase + (uint32_t)((j ^ (lane & 7)) * 16)));
+            r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + v.x);
+            r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + v.y);
+            r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + v.z);
+            r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + v.w);
           }
         }
         if (p.e_hi) {
@@ -245,32 +327,25 @@ __device__ __forceinline__ void epilogue_rows(const Problem& q, const Params& p,
         for (int j = 0; j < 8; ++j)
           asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sbase + (uint32_t)((j ^ (lane & 7)) * 16)),
                        "r"(r[4 * j]), "r"(r[4 * j + 1]), "r"(r[4 * j + 2]), "r"(r[4 * j + 3]) : "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        ++st.pc;
-        if (lane == 0) {
-          tma_store_2d(&q.mC, slot0 + slot * EPI_SLOT_BYTES, n0 + c0, rowoff + row0);
-          bulk_commit();
-          bulk_wait_read<1>();               // the other slot's store has read its data: the slot is free again
-          if (res && c0 + 32 < ncols && n0 + c0 + 32 < p.N) {
-            const uint32_t nslot = st.pc & 1u;
-            mbar_expect_tx((nslot ? rbar1 : rbar0), EPI_SLOT_BYTES);
-            tma_load_2d(slot0 + nslot * EPI_SLOT_BYTES, &q.mR, n0 + c0 + 32, row0, (nslot ? rbar1 : rbar0));
-          }
-        }
-        __syncwarp();
       }
-    }
-  } else {
-    const int m = row0 + lane;
-#pragma unroll 1
-    for (int c0 = 0; c0 < ncols; c0 += 32) {
-      uint32_t r[32];
-      tmem_ld32(tmem_acc + (uint32_t)c0, r);
-      if (m < p.M) store_row_piece(p, rowoff + m, n0 + c0, r);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      ++pc;
+      if (lane == 0) {
+        if (p.red) tma_add_2d(&q.mC, slot0 + slot * EPI_SLOT_BYTES, n0 + c0, rowoff + row0);
+        else tma_store_2d(&q.mC, slot0 + slot * EPI_SLOT_BYTES, n0 + c0, rowoff + row0);
+        bulk_commit();
+        if (res && c0 + NSLOT * bw < end) {
+          bulk_wait_read<0>();
+          load(q, slot, n0 + c0 + NSLOT * bw, row0);
+        } else {
+          bulk_wait_read<NSLOT - 1>();       // the next slot's last store has read its data
+        }
+      }
+      __syncwarp();
     }
   }
-}
+};
 
 // Persistent: CTA b works on tiles b, b + gridDim.x, ... of the group.  The operand ring and its phases run on
 // across tiles, so the producer is already loading the next tile while the last k-tiles of this one are
@@ -458,8 +533,7 @@ gemm_bf16_kernel(const __grid_constant__ Group g, const int total_tiles, unsigne
   } else {
     const int ew = warp - 2;                       // staging slots and residual barriers of this warp
     const int quarter = warp & 3;                  // the TMEM lanes this warp may read
-    const uint32_t slot0 = epi + (uint32_t)ew * (2 * EPI_SLOT_BYTES);
-    EpiState est;                                  // slot parity and residual-barrier phases, carried across tiles
+    Epilogue<2> est{epi + (uint32_t)ew * (2 * EPI_SLOT_BYTES), r_bar(ew, 0)};
     for (int it = 0;; ++it) {
       const int qs = it % NQ;
       const bool have = __all_sync(0xffffffffu, mbar_wait_idle(tq_full(qs), ((uint32_t)(it / NQ)) & 1u));
@@ -475,19 +549,20 @@ gemm_bf16_kernel(const __grid_constant__ Group g, const int total_tiles, unsigne
       const int rowoff = split_of(q, &tile, &kt0, &kt1) * p.slab_rows;
       const int m0 = (tile / q.tiles_n) * TBM, n0 = (tile % q.tiles_n) * TBN;
       const int b = it & 1;
+      est.prefetch(q, p, m0 + quarter * 32, n0, TBN, lane);
       const bool acc_ok = __all_sync(0xffffffffu, mbar_wait_idle(acc_full(b), ((uint32_t)it >> 1) & 1u));
       if (!acc_ok && lane == 0) { atomicOr(&g_bf16_status, 8u); *abort_flag = 1; }
       if (!acc_ok || __any_sync(0xffffffffu, *abort_flag != 0)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t tmem_acc = tmem_base + (uint32_t)(b * TBN) + ((uint32_t)(quarter * 32) << 16);
       const int row0 = m0 + quarter * 32;
-      epilogue_rows(q, p, tmem_acc, row0, rowoff, n0, TBN, slot0, r_bar(ew, 0), r_bar(ew, 1), est, lane, abort_flag);
+      est.run(q, p, tmem_acc, row0, rowoff, n0, TBN, lane, abort_flag);
       // every TMEM read of this warp has completed (tcgen05.wait::ld): hand the accumulator back
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_empty(b));
     }
-    if (lane == 0) bulk_wait_all();
+    est.drain(lane);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -538,6 +613,11 @@ __device__ __forceinline__ void mma_bf16_pair(uint32_t tmem_d, uint64_t adesc, u
 }
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster_addr) {
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
+}
+
+// the same to the barrier at this offset in both CTAs of the pair
+__device__ __forceinline__ void umma_commit_both(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
 
 // BN2 = width of the pair's tile (256 or 128); each CTA loads BN2/2 columns of B.
@@ -702,22 +782,31 @@ gemm_bf16_pair_kernel(const __grid_constant__ Group g) {
 }
 
 // ---- persistent CTA-pair variant ----------------------------------------------------------------------------
+// (BN2 = the widest tile; a problem may ask for 128-wide ones, see choose_widths.)
+// What bounds it: at long K the tensor cores under the power limit (8192^3 plain: 946 us when single lanes issued loads and MMAs from
+// inside `if (lane == 0)`, 791 us = 1390 TFLOP/s with one elected lane of a converged warp and one commit for both CTAs); at K = 768 the
+// 256 KB of fp32 that a tile writes.  Four epilogue warps were the limit there: products with a bf16 residual 67 -> 40 us, the two
+// gradients of in_proj at 16384 tokens 165 -> 129, of the tied head per 1024 rows 339 -> 254.
 // The CTA-pair kernel above as a tile loop: cluster c works on tiles c, c + clusters, ...; the operand ring keeps
 // running across tiles; the accumulator alternates between two TMEM buffers of BN2 columns, so each CTA drains its
 // 128 rows of tile i (through the same TMA-store epilogue as the single-CTA kernel) while the leader issues tile
-// i + 1.  The epilogue warps of BOTH CTAs hand a buffer back by arriving on the leader's acc_empty barrier (count 8).
+// i + 1.  The epilogue warps of BOTH CTAs hand a buffer back by arriving on the leader's acc_empty barrier.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
 template <bool SPLIT, int BN2> struct PairPCfg {
   static constexpr int STAGE_BYTES = PairCfg<SPLIT, BN2>::STAGE_BYTES;
-  static constexpr int STAGES = (192 * 1024) / STAGE_BYTES > 8 ? 8 : (192 * 1024) / STAGE_BYTES;
-  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 + 512;
+  // eight epilogue warps (two per TMEM quarter, half of the columns each) with a staging slot each
+  static constexpr int EPI_WARPS = 8, THREADS = 32 * (2 + EPI_WARPS);
+  static constexpr int NSLOT = 1, RING = 192 * 1024;
+  static constexpr int STAGES = RING / STAGE_BYTES > 8 ? 8 : RING / STAGE_BYTES;
+  static constexpr int EPI = EPI_WARPS * NSLOT * EPI_SLOT_BYTES;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI + 1024 + 512;
   static constexpr int TMEM = 2 * BN2;
 };
 
 template <bool SPLIT, int BN2>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairPCfg<SPLIT, BN2>::THREADS, 1)
 gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
   const uint32_t rank = cluster_rank();
   const int cluster_id = (int)(blockIdx.x >> 1), nclusters = (int)(gridDim.x >> 1);
@@ -725,26 +814,26 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
   constexpr int TILE_B = BNH * TBK * 2;
   constexpr int HALF_BYTES = TILE_BYTES + TILE_B;
   constexpr int STAGE_BYTES = PairPCfg<SPLIT, BN2>::STAGE_BYTES;
-  constexpr int STAGES = PairPCfg<SPLIT, BN2>::STAGES;
+  constexpr int STAGES = PairPCfg<SPLIT, BN2>::STAGES, NSLOT = PairPCfg<SPLIT, BN2>::NSLOT, EPI = PairPCfg<SPLIT, BN2>::EPI;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t tiles = (raw + 1023u) & ~1023u;
   uint8_t* tiles_ptr = smem_raw + (tiles - raw);
   const uint32_t epi = tiles + STAGES * STAGE_BYTES;
-  const uint32_t bars = epi + EPI_BYTES;
+  const uint32_t bars = epi + EPI;
   auto full_bar = [&](int s) { return bars + 8u * s; };
   auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
   auto acc_full = [&](int b) { return bars + 8u * (2 * STAGES + b); };
   auto acc_empty = [&](int b) { return bars + 8u * (2 * STAGES + 2 + b); };
-  auto r_bar = [&](int w, int slot) { return bars + 8u * (2 * STAGES + 4 + 2 * w + slot); };
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(tiles_ptr + STAGES * STAGE_BYTES + EPI_BYTES + 8 * (2 * STAGES + 12));
+  auto r_bar = [&](int w, int slot) { return bars + 8u * (2 * STAGES + 4 + NSLOT * w + slot); };
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(tiles_ptr + STAGES * STAGE_BYTES + EPI + 8 * (2 * STAGES + 4 + PairPCfg<SPLIT, BN2>::EPI_WARPS * NSLOT));
   volatile uint32_t* abort_flag = tmem_slot + 1;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 8); }
-    for (int w = 0; w < 4; ++w) { mbar_init(r_bar(w, 0), 1); mbar_init(r_bar(w, 1), 1); }
+    for (int b = 0; b < 2; ++b) { mbar_init(acc_full(b), 1); mbar_init(acc_empty(b), 2 * PairPCfg<SPLIT, BN2>::EPI_WARPS); }
+    for (int w = 0; w < PairPCfg<SPLIT, BN2>::EPI_WARPS * NSLOT; ++w) mbar_init(r_bar(0, w), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -760,124 +849,113 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int s = 0; uint32_t ph = 0;
-      int in_flight = 0;
-      bool stop = false;
-      for (int j = 0; !stop; ++j) {
-        const int tid = pair_tile_at(g, cluster_id, nclusters, j);
-        if (tid >= total_tiles) break;
-        int tile, kt0, kt1;
-        const Problem& q = g.pr[pick_problem(g, tid, &tile)];
-        const Params& p = q.p;
-        split_of(q, &tile, &kt0, &kt1);
-        const int m0 = (tile / q.tiles_n) * 256 + (int)rank * TBM;
-        const int nb0 = (tile % q.tiles_n) * BN2 + (int)rank * BNH;
-        for (int kt = kt0; kt < kt1; ++kt) {
-          if (!mbar_wait(empty_bar(s), ph ^ 1u)) { atomicOr(&g_bf16_status, 1u); *abort_flag = 1; stop = true; break; }
-          if (*abort_flag) { stop = true; break; }
-          const uint32_t a_dst = tiles + s * STAGE_BYTES, b_dst = a_dst + TILE_BYTES;
-          const uint32_t fb = map_to_cta(full_bar(s), 0);            // the leader's barrier collects both CTAs' bytes
-          if (rank == 0) mbar_expect_tx(full_bar(s), 2 * STAGE_BYTES);
-          const int k0 = kt * TBK;
-          if (!p.a_mn_major) {
-            tma_load_2d_pair(a_dst, &q.mA, k0, m0, fb);
-          } else {
-#pragma unroll
-            for (int j = 0; j < TBM / 64; ++j) tma_load_2d_pair(a_dst + j * (TBK * 128), &q.mA, m0 + 64 * j, k0, fb);
-          }
-          if (!p.b_mn_major) {
-            tma_load_2d_pair(b_dst, &q.mB, k0, nb0, fb);
-          } else {
-#pragma unroll
-            for (int j = 0; j < BNH / 64; ++j) tma_load_2d_pair(b_dst + j * (TBK * 128), &q.mB, nb0 + 64 * j, k0, fb);
-          }
+    // (the whole warp waits, one elected lane issues)
+    int s = 0; uint32_t ph = 0;
+    int in_flight = 0;
+    bool stop = false;
+    const uint32_t fb0 = map_to_cta(full_bar(0), 0);               // the leader's barriers collect both CTAs' bytes
+    for (int j = 0; !stop; ++j) {
+      const int tid = pair_tile_at(g, cluster_id, nclusters, j);
+      if (tid >= total_tiles) break;
+      int tile, kt0, kt1;
+      const Problem& q = g.pr[pick_problem(g, tid, &tile)];
+      const Params& p = q.p;
+      split_of(q, &tile, &kt0, &kt1);
+      const int m0 = (tile / q.tiles_n) * 256 + (int)rank * TBM, bnh = p.bn >> 1;      // (tiles of bn <= BN2 columns)
+      const int nb0 = (tile % q.tiles_n) * p.bn + (int)rank * bnh;
+      const uint32_t tx = 2u * (uint32_t)(STAGE_BYTES - (SPLIT ? 2 : 1) * (BNH - bnh) * TBK * 2);
+      const bool amn = p.a_mn_major, bmn = p.b_mn_major, wide = BNH > 64 && bnh > 64;
+      for (int kt = kt0; kt < kt1; ++kt) {
+        const bool got = __all_sync(0xffffffffu, mbar_wait(empty_bar(s), ph ^ 1u));
+        if (!got && lane == 0) { atomicOr(&g_bf16_status, 1u); *abort_flag = 1; }
+        if (!got || __any_sync(0xffffffffu, *abort_flag != 0)) { stop = true; break; }
+        const uint32_t a_dst = tiles + s * STAGE_BYTES, b_dst = a_dst + TILE_BYTES, fb = fb0 + 8u * s;
+        const int k0 = kt * TBK;
+        if (elect_one()) {
+          if (rank == 0) mbar_expect_tx(full_bar(s), tx);
+          auto load = [&](uint32_t dst, const CUtensorMap* map, bool mn, int row0, bool two) {
+            if (!mn) { tma_load_2d_pair(dst, map, k0, row0, fb); return; }
+            tma_load_2d_pair(dst, map, row0, k0, fb);
+            if (two) tma_load_2d_pair(dst + TBK * 128, map, row0 + 64, k0, fb);
+          };
+          load(a_dst, &q.mA, amn, m0, true);
+          load(b_dst, &q.mB, bmn, nb0, wide);
           if (SPLIT) {
-            const uint32_t al_dst = a_dst + HALF_BYTES, bl_dst = al_dst + TILE_BYTES;
-            if (!p.a_mn_major) {
-              tma_load_2d_pair(al_dst, &q.mAlo, k0, m0, fb);
-            } else {
-#pragma unroll
-              for (int j = 0; j < TBM / 64; ++j) tma_load_2d_pair(al_dst + j * (TBK * 128), &q.mAlo, m0 + 64 * j, k0, fb);
-            }
-            if (!p.b_mn_major) {
-              tma_load_2d_pair(bl_dst, &q.mBlo, k0, nb0, fb);
-            } else {
-#pragma unroll
-              for (int j = 0; j < BNH / 64; ++j) tma_load_2d_pair(bl_dst + j * (TBK * 128), &q.mBlo, nb0 + 64 * j, k0, fb);
-            }
+            load(a_dst + HALF_BYTES, &q.mAlo, amn, m0, true);
+            load(b_dst + HALF_BYTES, &q.mBlo, bmn, nb0, wide);
           }
-          if (in_flight < STAGES) ++in_flight;
-          if (++s == STAGES) { s = 0; ph ^= 1u; }
         }
+        __syncwarp();
+        if (in_flight < STAGES) ++in_flight;
+        if (++s == STAGES) { s = 0; ph ^= 1u; }
       }
-      // after giving up, the leader still waits (bounded) for the loads both CTAs have in flight
-      if (*abort_flag && rank == 0) {
-        for (int i = 0; i < in_flight; ++i) {
-          if (--s < 0) { s = STAGES - 1; ph ^= 1u; }
-          mbar_wait(full_bar(s), ph);
-        }
+    }
+    // after giving up, the leader still waits (bounded) for the loads both CTAs have in flight
+    if (*abort_flag && rank == 0 && lane == 0) {
+      for (int i = 0; i < in_flight; ++i) {
+        if (--s < 0) { s = STAGES - 1; ph ^= 1u; }
+        mbar_wait(full_bar(s), ph);
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    // The whole warp of the leader waits and one elected lane issues: descriptors then stay in uniform registers, and a k-tile's
+    // commit reaches both CTAs as one instruction (see the comment above the kernel for what that gave).
+    if (rank == 0) {
       const uint32_t d_hi = desc_hi(1024, 2);
       constexpr uint32_t LO_OFF = HALF_BYTES >> 4;
-      uint32_t eb0[STAGES], eb1[STAGES];
-#pragma unroll
-      for (int i = 0; i < STAGES; ++i) { eb0[i] = map_to_cta(empty_bar(i), 0); eb1[i] = map_to_cta(empty_bar(i), 1); }
-      const uint32_t af0[2] = {map_to_cta(acc_full(0), 0), map_to_cta(acc_full(1), 0)};
-      const uint32_t af1[2] = {map_to_cta(acc_full(0), 1), map_to_cta(acc_full(1), 1)};
       int s = 0; uint32_t ph = 0;
-      int it = 0;
       bool stop = false;
-      for (; !stop; ++it) {
+      for (int it = 0; !stop; ++it) {
         const int tid = pair_tile_at(g, cluster_id, nclusters, it);
         if (tid >= total_tiles) break;
         int tile, kt0, kt1;
         const Problem& q = g.pr[pick_problem(g, tid, &tile)];
         const Params& p = q.p;
         split_of(q, &tile, &kt0, &kt1);
-        // M = 256 (two CTAs x 128 rows), N = BN2
+        // M = 256 (two CTAs x 128 rows), N = bn
         const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)p.a_mn_major << 15) | ((uint32_t)p.b_mn_major << 16) |
-                               ((uint32_t)(BN2 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
+                               ((uint32_t)(p.bn >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
         const uint32_t a_lbo = p.a_mn_major ? TBK * 128 : 16, b_lbo = p.b_mn_major ? TBK * 128 : 16;
         const uint32_t a_step = (p.a_mn_major ? 2048u : 32u) >> 4, b_step = (p.b_mn_major ? 2048u : 32u) >> 4;
         const int b = it & 1;
-        if (!mbar_wait(acc_empty(b), (((uint32_t)it >> 1) & 1u) ^ 1u)) { atomicOr(&g_bf16_status, 4u); *abort_flag = 1; break; }
+        if (!__all_sync(0xffffffffu, mbar_wait(acc_empty(b), (((uint32_t)it >> 1) & 1u) ^ 1u))) {
+          if (lane == 0) { atomicOr(&g_bf16_status, 4u); *abort_flag = 1; }
+          break;
+        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t tmem_acc = tmem_base + (uint32_t)(b * BN2);
         for (int kt = kt0; kt < kt1; ++kt) {
-          if (!mbar_wait(full_bar(s), ph)) { atomicOr(&g_bf16_status, 2u); *abort_flag = 1; stop = true; break; }
-          if (*abort_flag) { stop = true; break; }
+          const bool got = __all_sync(0xffffffffu, mbar_wait(full_bar(s), ph));
+          if (!got && lane == 0) { atomicOr(&g_bf16_status, 2u); *abort_flag = 1; }
+          if (!got || __any_sync(0xffffffffu, *abort_flag != 0)) { stop = true; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a_s = tiles + s * STAGE_BYTES;
-          uint32_t al = desc_lo(a_s, a_lbo), bl = desc_lo(a_s + TILE_BYTES, b_lbo);
+          const uint32_t al0 = desc_lo(a_s, a_lbo), bl0 = desc_lo(a_s + TILE_BYTES, b_lbo);
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < TBK / 16; ++k) {
-            const uint32_t acc = (kt > kt0 || k > 0) ? 1u : 0u;
-            if (SPLIT) {
-              mma_f16_pair_h(tmem_acc, al + LO_OFF, d_hi, bl, d_hi, idesc, acc);
-              mma_f16_pair_h(tmem_acc, al, d_hi, bl + LO_OFF, d_hi, idesc, 1u);
-              mma_f16_pair_h(tmem_acc, al, d_hi, bl, d_hi, idesc, 1u);
-            } else {
-              mma_f16_pair_h(tmem_acc, al, d_hi, bl, d_hi, idesc, acc);
+            for (int k = 0; k < TBK / 16; ++k) {
+              const uint32_t acc = (kt > kt0 || k > 0) ? 1u : 0u, al = al0 + k * a_step, bl = bl0 + k * b_step;
+              if (SPLIT) {
+                mma_f16_pair_h(tmem_acc, al + LO_OFF, d_hi, bl, d_hi, idesc, acc);
+                mma_f16_pair_h(tmem_acc, al, d_hi, bl + LO_OFF, d_hi, idesc, 1u);
+                mma_f16_pair_h(tmem_acc, al, d_hi, bl, d_hi, idesc, 1u);
+              } else {
+                mma_f16_pair_h(tmem_acc, al, d_hi, bl, d_hi, idesc, acc);
+              }
             }
-            al += a_step; bl += b_step;
+            umma_commit_both(empty_bar(s));
           }
-#pragma unroll
-          for (int i = 0; i < STAGES; ++i)
-            if (i == s) { umma_commit_pair(eb0[i]); umma_commit_pair(eb1[i]); }
+          __syncwarp();
           if (++s == STAGES) { s = 0; ph ^= 1u; }
         }
-        if (!stop) { umma_commit_pair(af0[b]); umma_commit_pair(af1[b]); }
+        if (!stop && elect_one()) umma_commit_both(acc_full(b));
+        __syncwarp();
       }
     }
   } else {
     const int ew = warp - 2;
-    const int quarter = warp & 3;
-    const uint32_t slot0 = epi + (uint32_t)ew * (2 * EPI_SLOT_BYTES);
-    EpiState est;
+    const int quarter = warp & 3, chalf = ew >> 2;             // this warp's TMEM lanes and half of the columns
+    Epilogue<NSLOT> est{epi + (uint32_t)ew * (NSLOT * EPI_SLOT_BYTES), r_bar(ew, 0)};
     const uint32_t ae[2] = {map_to_cta(acc_empty(0), 0), map_to_cta(acc_empty(1), 0)};      // the leader's barriers
     int it = 0;
     for (;; ++it) {
@@ -887,20 +965,21 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
       const Problem& q = g.pr[pick_problem(g, tid, &tile)];
       const Params& p = q.p;
       const int rowoff = split_of(q, &tile, &kt0, &kt1) * p.slab_rows;
-      const int m0 = (tile / q.tiles_n) * 256 + (int)rank * TBM, n0 = (tile % q.tiles_n) * BN2;
+      const int m0 = (tile / q.tiles_n) * 256 + (int)rank * TBM, cw = p.bn >> 1, n0 = (tile % q.tiles_n) * p.bn + chalf * cw;
       const int b = it & 1;
+      est.prefetch(q, p, m0 + quarter * 32, n0, cw, lane);
       const bool acc_ok = __all_sync(0xffffffffu, mbar_wait_idle(acc_full(b), ((uint32_t)it >> 1) & 1u));
       if (!acc_ok && lane == 0) { atomicOr(&g_bf16_status, 8u); *abort_flag = 1; }
       if (!acc_ok || __any_sync(0xffffffffu, *abort_flag != 0)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t tmem_acc = tmem_base + (uint32_t)(b * BN2) + ((uint32_t)(quarter * 32) << 16);
+      const uint32_t tmem_acc = tmem_base + (uint32_t)(b * BN2 + chalf * cw) + ((uint32_t)(quarter * 32) << 16);
       const int row0 = m0 + quarter * 32;
-      epilogue_rows(q, p, tmem_acc, row0, rowoff, n0, BN2, slot0, r_bar(ew, 0), r_bar(ew, 1), est, lane, abort_flag);
+      est.run(q, p, tmem_acc, row0, rowoff, n0, cw, lane, abort_flag);
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(ae[b]);
     }
-    if (lane == 0) bulk_wait_all();
+    est.drain(lane);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -950,13 +1029,25 @@ pmb_status pair_operand_map(CUtensorMap* map, const uint16_t* base, int64_t inne
 }
 
 // Maps for the epilogue of the single-CTA kernel: 32 x 32 fp32 blocks of C (and of R, which shares C's pitch).
-// Leaves tma_out = 0 when the result is bf16 or breaks a TMA rule; the kernel then stores row by row.
+// (32 x 64 of a bf16 result: row by row, a thread's 64 bytes apart from its neighbour's, the bf16 results with a residual took longer
+// than their products: out_proj at 16384 tokens 67 us, 48 this way, 40 with
+// eight epilogue warps.)  Leaves tma_out = 0 when a TMA rule is broken (a store
+// clips a row at whole 16 bytes, so a width that ends inside them would reach into the pitch); the kernel then stores row by row.
 static pmb_status make_out_maps(Problem* q, int slabs = 1) {
   Params& p = q->p;
-  p.tma_out = 0;
-  if (p.out_bf16 || (p.ldc & 3) || (reinterpret_cast<uintptr_t>(p.C) & 15) || (p.R && (reinterpret_cast<uintptr_t>(p.R) & 15))) return PMB_OK;
+  p.tma_out = p.red = 0;
+  if (p.out_bf16) {
+    if (slabs > 1 || (p.N & 7) || (p.ldc & 7) || (reinterpret_cast<uintptr_t>(p.C) & 15) || (p.R && (reinterpret_cast<uintptr_t>(p.R) & 15))) return PMB_OK;
+    PMB_TRY(make_map(&q->mC, p.C, p.N, p.M, p.ldc, 64, 32));
+    if (p.R) PMB_TRY(make_map(&q->mR, p.R, p.N, p.M, p.ldc, 64, 32));
+    p.tma_out = 1;
+    return PMB_OK;
+  }
+  if ((p.ldc & 3) || (p.R && (p.N & 3)) || (reinterpret_cast<uintptr_t>(p.C) & 15) || (p.R && (reinterpret_cast<uintptr_t>(p.R) & 15))) return PMB_OK;
   PMB_TRY(make_map(&q->mC, p.C, p.N, slabs > 1 ? (int64_t)slabs * p.slab_rows : p.M, p.ldc, 32, 32, true));
-  if (p.R) PMB_TRY(make_map(&q->mR, p.R, p.N, p.M, p.ldc, 32, 32, true));
+  // (one addend per element and launch, so the order of the additions is as it was: C, then the product)
+  p.red = p.R == p.C && slabs == 1 && !p.e_hi;
+  if (p.R && !p.red) PMB_TRY(make_map(&q->mR, p.R, p.N, p.M, p.ldc, 32, 32, true));
   p.tma_out = 1;
   return PMB_OK;
 }
@@ -1034,17 +1125,70 @@ namespace hb {
 
 static int64_t ktiles(int64_t K) { return cdiv(K, TBK); }
 
-// Long tiles first on the pair kernel (Group): the leading problems whose tiles are at least twice as long as those of the last
-// one, when they have fewer tiles than there are clusters.
+// What a tile of the CTA-pair kernel costs, in k-tiles of 256 columns: a 128-wide one has half the columns, but with one MMA per product
+// hardly less than the time (311 ns against 299 per k-tile; the loads and barriers of a k-tile set the pace), with three 0.6 of it.
+static double tile_cost(const Problem& q) { return (double)q.p.kt_per * (q.p.bn == 256 ? 1.0 : q.p.pairs ? 0.6 : 0.9) + 1.0; }
+
+// Long tiles first on the pair kernel (Group): the leading problems whose tiles cost at least twice those of the last one, when they
+// have fewer tiles than there are clusters.
 static void set_lead(Group* g, int n, int clusters) {
   g->lead = g->rounds = 0;
   if (n < 2) return;
   const Problem& last = g->pr[n - 1];
-  const int64_t b = last.p.kt_per;
-  int64_t lead = 0, a = 0;
-  for (int i = 0; i + 1 < n; ++i) { lead += g->pr[i].tiles; if (g->pr[i].p.kt_per > a) a = g->pr[i].p.kt_per; }
-  if (lead >= clusters || a < 2 * b) return;
+  const double b = tile_cost(last);
+  int64_t lead = 0;
+  double a = 0.0;
+  for (int i = 0; i + 1 < n; ++i) { lead += g->pr[i].tiles; const double c = tile_cost(g->pr[i]); if (c > a) a = c; }
+  if (lead >= clusters || a < 2.0 * b) return;
   g->lead = (int)lead; g->rounds = (int)(a / b);
+}
+
+static void set_tiles(Problem* q, int bn) {
+  const int splits = (int)cdiv(ktiles(q->p.K), q->p.kt_per);
+  q->p.bn = bn;
+  q->tiles_n = (int)cdiv(q->p.N, bn);
+  q->tiles_mn = (int)(cdiv(q->p.M, 256) * q->tiles_n);
+  q->tiles = q->tiles_mn * splits;
+}
+
+// The longest cluster's work for the widths that are set.
+static double makespan(Group* g, int n, int slots) {
+  int64_t tiles = 0;
+  double total = 0.0, most = 0.0;
+  for (int i = 0; i < n; ++i) {
+    const double c = tile_cost(g->pr[i]);
+    tiles += g->pr[i].tiles; total += c * g->pr[i].tiles;
+    if (c > most) most = c;
+  }
+  const int clusters = (int)(tiles < slots ? tiles : slots);
+  set_lead(g, n, clusters);
+  if (tiles > 8 * slots) return total / clusters > most ? total / clusters : most;
+  double worst = 0.0;
+  for (int c = 0; c < clusters; ++c) {
+    double t = 0.0;
+    for (int j = 0;; ++j) {
+      const int id = pair_tile_at(*g, c, clusters, j);
+      if (id >= tiles) break;
+      int base = 0, i = 0;
+      while (id >= base + g->pr[i].tiles) base += g->pr[i++].tiles;
+      t += tile_cost(g->pr[i]);
+    }
+    if (t > worst) worst = t;
+  }
+  return worst;
+}
+
+// Tile widths of the products of a launch: 256 columns, or 128 where the shorter tiles bring the longest cluster down by a tenth (few
+// tiles: 2048 x 768 outputs are 24 tiles of 256 columns; on pairs with K = 1536 they took 44 us, 48 tiles of 128 columns 28).  Every sum runs over K in the same order at either width.
+static void choose_widths(Group* g, int n, int slots) {
+  double best = 0.0;
+  int pick = 0;
+  for (int mask = 0; mask < (1 << n); ++mask) {
+    for (int i = 0; i < n; ++i) set_tiles(&g->pr[i], (mask >> i) & 1 ? 128 : 256);
+    const double t = makespan(g, n, slots);
+    if (mask == 0 || t < 0.9 * best) { best = t; pick = mask; }
+  }
+  for (int i = 0; i < n; ++i) set_tiles(&g->pr[i], (pick >> i) & 1 ? 128 : 256);
 }
 
 }  // namespace hb
@@ -1097,7 +1241,7 @@ pmb_status gemm_bf16_group(cudaStream_t st, const PlainGemm* gs, int n) {
   }
   if (tiles > 0x7fffffff) return fail(PMB_ERR_SHAPE, "gemm_bf16: too many tiles");
   static const int env = [] { const char* e = getenv("PMB_GEMM_PAIR"); return e ? atoi(e) : -1; }();
-  static const int min_clusters = [] { const char* e = getenv("PMB_GEMM_PAIR_MIN"); return e ? atoi(e) : 18; }();
+  static const int min_clusters = [] { const char* e = getenv("PMB_GEMM_PAIR_MIN"); return e ? atoi(e) : 4; }();
   const bool pair = env >= 0 ? env != 0 : (tall && clusters >= min_clusters);      // see pick_pair_mode
   for (int i = 0; i < n; ++i) {
     Problem& q = g.pr[i];
@@ -1109,9 +1253,15 @@ pmb_status gemm_bf16_group(cudaStream_t st, const PlainGemm* gs, int n) {
   if (pair) {
     PMB_SMEM_OPT_IN((PairPCfg<false, 256>::SMEM_BYTES), gemm_bf16_pairp_kernel<false, 256>);
     const int64_t slots = persistent_grid(148) / 2;
+    choose_widths(&g, n, (int)slots);
+    clusters = 0;
+    for (int i = 0; i < n; ++i) {
+      clusters += g.pr[i].tiles;
+      if (gs[i].tb) PMB_TRY(make_map(&g.pr[i].mB, gs[i].B, gs[i].K, gs[i].N, gs[i].ldb, TBK, g.pr[i].p.bn / 2));
+    }
     const unsigned grid = 2u * (unsigned)(clusters < slots ? clusters : slots);
     set_lead(&g, n, (int)(grid / 2));
-    gemm_bf16_pairp_kernel<false, 256><<<grid, NTHREADS, PairPCfg<false, 256>::SMEM_BYTES, st>>>(g, (int)clusters);
+    gemm_bf16_pairp_kernel<false, 256><<<grid, (PairPCfg<false, 256>::THREADS), PairPCfg<false, 256>::SMEM_BYTES, st>>>(g, (int)clusters);
   } else {
     unsigned long long t0 = 0;
     unsigned long long* sc = sched_counter(st, tiles, &t0);
@@ -1218,14 +1368,11 @@ static int pick_pair_mode(const PairGemm* gs, int n, int tile_mode) {
   static const int env = [] { const char* e = getenv("PMB_GEMM_PAIR"); return e ? atoi(e) : -1; }();
   const int forced = tile_mode >= 0 ? tile_mode : env;
   if (forced >= 0 && forced <= 4) return forced;          // 3 / 4: the persistent CTA-pair kernel with 256x128 / 256x256 tiles
-  // 256x256 CTA-pair tiles on the persistent pair kernel fetch half the operand bytes per flop and read half as
-  // much shared memory per MMA.  Alone, at 2048 tokens, they win where there is at least half a wave of the 74
-  // cluster slots (in_proj forward 36.8 against 39.6 us, dnormed 23.1 against 28.2, dW_in 41.4 against 55.7) and lose
-  // below (out_proj forward 33.3 against 27.0 us at 24 clusters); inside the training step, where other streams'
-  // kernels fill the SMs a short launch leaves idle, the threshold that measured best is 18 clusters per product
-  // (step 13.35 ms with the single-CTA kernel everywhere, 13.05 at 37, 12.86 at 18, 12.95 at 12).
-  // 256x128 pair tiles measured no faster than single-CTA tiles.  PMB_GEMM_PAIR_MIN overrides the threshold.
-  static const int half_wave = [] { const char* e = getenv("PMB_GEMM_PAIR_MIN"); return e ? atoi(e) : 18; }();
+  // CTA-pair tiles fetch half the operand bytes per flop, read half as much shared memory per MMA, and come 256 or 128 columns
+  // wide (choose_widths); below four clusters per product too few SMs take part.  Residual stack of four layers at 2 x 384 tokens of
+  // d_model 768: 1226 us with the line at 18 clusters, 1150 at 9 and at 4; training step at 2 x 512: 1240, 1154, 1153; prefill of
+  // 160 tokens at d_model 1024: 99, 97, 89; the smallest block is 5 % slower without a line.  PMB_GEMM_PAIR_MIN overrides it.
+  static const int half_wave = [] { const char* e = getenv("PMB_GEMM_PAIR_MIN"); return e ? atoi(e) : 4; }();
   for (int i = 0; i < n; ++i) {
     if (gs[i].M <= 128) return 0;        // a pair tile would be half empty
     if (cdiv(gs[i].M, 256) * cdiv(gs[i].N, 256) * (gs[i].ksplit > 1 ? gs[i].ksplit : 1) < half_wave) return 0;
@@ -1260,13 +1407,13 @@ pmb_status gemm_pairs_group(cudaStream_t st, const PairGemm* gs, int n, int tile
     Params& p = q.p;
     p.M = (int)M; p.N = (int)N; p.K = (int)K;
     p.a_mn_major = e.ta ? 1 : 0; p.b_mn_major = e.tb ? 0 : 1;
-    p.C = e.C; p.ldc = e.ldc; p.R = e.R; p.out_bf16 = 0;
+    p.C = e.C; p.ldc = e.ldc; p.R = e.R; p.out_bf16 = 0; p.pairs = 1;
     const int sp = e.ksplit > 1 ? e.ksplit : 1;
     if (sp > 1 && (e.R || e.emit.hi || e.slab_rows < M || e.slab_rows % 256)) return fail(PMB_ERR_ARG, "gemm_pairs: split products go to fp32 slabs");
     p.kt_per = (int)cdiv(ktiles(K), sp); p.slab_rows = sp > 1 ? (int)e.slab_rows : 0;
     if (cdiv(ktiles(K), p.kt_per) < sp) return fail(PMB_ERR_ARG, "gemm_pairs: more splits than k-tiles");
-    PMB_TRY(make_out_maps(&q, sp));
     p.e_hi = const_cast<uint16_t*>(e.emit.hi); p.e_lo = const_cast<uint16_t*>(e.emit.lo); p.lde = e.emit.ld;   // (Pair16 is declared for reading; this one is written)
+    PMB_TRY(make_out_maps(&q, sp));
     if (p.e_hi && (!p.tma_out || !p.e_lo || (p.lde & 7) || ((reinterpret_cast<uintptr_t>(p.e_hi) | reinterpret_cast<uintptr_t>(p.e_lo)) & 15)))
       return fail(PMB_ERR_UNSUPPORTED, "gemm_pairs: the pair output needs the TMA-store epilogue, 16-byte aligned arrays and a pitch that is a multiple of 8");
     q.tiles_n = (int)cdiv(N, TBN);
@@ -1281,31 +1428,30 @@ pmb_status gemm_pairs_group(cudaStream_t st, const PairGemm* gs, int n, int tile
   int pair_mode = pick_pair_mode(gs, n, tile_mode);
   for (int i = 0; i < n; ++i) if ((gs[i].emit.hi || gs[i].ksplit > 1) && pair_mode <= 2) pair_mode = 0;      // (the one-tile-per-cluster kernels do not write the pair output)
   if (pair_mode) {
-    const int bn2 = (pair_mode == 2 || pair_mode == 4) ? 256 : 128;
+    const int64_t slots = persistent_grid(148) / 2;
+    if (pair_mode == 4) choose_widths(&g, n, (int)slots);
+    else for (int i = 0; i < n; ++i) set_tiles(&g.pr[i], pair_mode == 2 ? 256 : 128);
     PMB_SMEM_OPT_IN((PairCfg<true, 256>::SMEM_BYTES), gemm_bf16_pair_kernel<true, 256>);
     PMB_SMEM_OPT_IN((PairCfg<true, 128>::SMEM_BYTES), gemm_bf16_pair_kernel<true, 128>);
     int64_t clusters = 0;
     for (int i = 0; i < n; ++i) {
       const PairGemm& e = gs[i];
       Problem& q = g.pr[i];
-      // B boxes of the pair kernel are BN2/2 rows tall (K-major tiles); MN-major boxes stay 64 columns wide
-      if (e.tb) { PMB_TRY(make_map(&q.mB, e.B.hi, e.K, e.N, e.B.ld, TBK, bn2 / 2)); PMB_TRY(make_map(&q.mBlo, e.B.lo, e.K, e.N, e.B.ld, TBK, bn2 / 2)); }
-      q.tiles_n = (int)cdiv(e.N, bn2);
-      q.tiles_mn = (int)(cdiv(e.M, 256) * cdiv(e.N, bn2));
-      q.tiles = q.tiles_mn * (e.ksplit > 1 ? e.ksplit : 1);
+      // B boxes of the pair kernels are half a tile tall (K-major tiles); MN-major boxes stay 64 columns wide
+      const int half = q.p.bn / 2;
+      if (e.tb) { PMB_TRY(make_map(&q.mB, e.B.hi, e.K, e.N, e.B.ld, TBK, half)); PMB_TRY(make_map(&q.mBlo, e.B.lo, e.K, e.N, e.B.ld, TBK, half)); }
       clusters += q.tiles;
     }
     if (pair_mode >= 3) {
       ProfScope prof(st, "gemm_bf16x2", flops, bytes);
-      const int64_t slots = persistent_grid(148) / 2;
       const unsigned grid = 2u * (unsigned)(clusters < slots ? clusters : slots);
       set_lead(&g, n, (int)(grid / 2));
       if (pair_mode == 4) {
         PMB_SMEM_OPT_IN((PairPCfg<true, 256>::SMEM_BYTES), gemm_bf16_pairp_kernel<true, 256>);
-        gemm_bf16_pairp_kernel<true, 256><<<grid, NTHREADS, PairPCfg<true, 256>::SMEM_BYTES, st>>>(g, (int)clusters);
+        gemm_bf16_pairp_kernel<true, 256><<<grid, (PairPCfg<true, 256>::THREADS), PairPCfg<true, 256>::SMEM_BYTES, st>>>(g, (int)clusters);
       } else {
         PMB_SMEM_OPT_IN((PairPCfg<true, 128>::SMEM_BYTES), gemm_bf16_pairp_kernel<true, 128>);
-        gemm_bf16_pairp_kernel<true, 128><<<grid, NTHREADS, PairPCfg<true, 128>::SMEM_BYTES, st>>>(g, (int)clusters);
+        gemm_bf16_pairp_kernel<true, 128><<<grid, (PairPCfg<true, 128>::THREADS), PairPCfg<true, 128>::SMEM_BYTES, st>>>(g, (int)clusters);
       }
       PMB_LAUNCHED();
       return PMB_OK;

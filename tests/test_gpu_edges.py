@@ -140,3 +140,30 @@ def test_scan_bf16_lengths(pm, B, T, P, N, G, off):
                                  (db.float(), leaves[2].grad, 5e-3, "db"), (dc.float(), leaves[3].grad, 5e-3, "dc")):
         if T > 1 or what != "da":      # (one token: da is exactly zero)
             assert_close(got, want, tol=tol, what=what)
+
+
+# the CTA-pair GEMM's ways of storing a result: ragged edges (odd widths, rows past the last whole tile), fp32 and bf16, a residual
+# loaded ahead, a result added onto C, and the two tile widths (few tiles with a long K take the narrow one on pairs)
+@pytest.mark.parametrize("M,N,K", [(2048, 768, 1536), (1100, 1411, 200), (300, 4616, 72)])
+@pytest.mark.parametrize("out16,res", [(0, 0), (1, 0), (1, 1), (0, 1), (0, 2)])
+def test_gemm_pair_tiles_store(pm, M, N, K, out16, res):
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    a, b = (torch.randn(*s, device="cuda", generator=g, dtype=torch.bfloat16) for s in ((M, K), (K, (N + 7) // 8 * 8)))
+    ld = (N + 7) // 8 * 8
+    dt = torch.bfloat16 if out16 else torch.float32
+    c = torch.randn(M, ld, device="cuda", generator=g).to(dt)
+    r = c if res == 2 else torch.randn(M, ld, device="cuda", generator=g).to(dt)
+    want = a.float() @ b[:, :N].float() + (r[:, :N].float() if res else 0.0)
+    past = c[:, N:].clone()
+    st = pm.lib.pmb_gemm_bf16(pm._stream(), 0, 0, M, N, K, a.data_ptr(), K, b.data_ptr(), ld, c.data_ptr(), ld, r.data_ptr() if res else None, out16)
+    assert st == 0 and pm.device_status() == 0
+    assert_close(c[:, :N].float(), want, tol=5e-3 if out16 else 1e-5, what=f"{M}x{N}x{K}")
+    assert torch.equal(c[:, N:], past)                  # nothing beyond the result's columns
+
+
+@pytest.mark.parametrize("M,N,K", [(2048, 768, 1536), (1000, 1224, 136)])
+def test_gemm_pair_tiles_on_pairs(pm, M, N, K):
+    a, b = randn((M, K), 1).cuda(), randn((K, N), 2).cuda()
+    out = pm.matmul(a, b)
+    assert pm.device_status() == 0
+    assert_close(out, a.double() @ b.double(), tol=3e-5, what=f"{M}x{N}x{K}")
