@@ -272,7 +272,7 @@ static bool fwd_ws_layout(const Dims& d, void* base, size_t bytes, bool bf16, bo
 }
 
 pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, const void* x, const void* residual,
-                     void* out, void* ws, size_t ws_bytes, const Weights16* wx, bool x_pair_ready, bool emit_out_pair) {
+                     void* out, void* ws, size_t ws_bytes, const Weights16* wx, bool x_pair_ready, bool emit_out_pair, bool backward_follows) {
   const Weights16* w16 = storage_is_bf16(wx) ? wx : nullptr;
   const bool pr = !w16 && block_uses_pairs(d);
   BlockWs w{};
@@ -281,7 +281,9 @@ pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, 
   // are faster chunk by chunk.  One step of a chain takes 3.5 us; those kernels 30 us and 0.1 us per step of a head.)
   const int64_t steps = cdiv(d.T, SCAN_STEP);
   const bool by_chunks = plain && 3.5 * steps > 30.0 + 0.1 * (double)((int64_t)d.B * d.H * steps);
-  if (ssd_chain_enabled() && ssd_chain_shape(d.P, d.N) && !by_chunks) {
+  // (the backward of a stack whose blocks keep the FMA contractions amplifies any difference between the forward's scan and its own)
+  const bool as_backward = backward_follows && !w16 && !block_uses_chain_bwd(d, false, wx && wx->pairs);
+  if (ssd_chain_enabled() && ssd_chain_shape(d.P, d.N) && !by_chunks && !as_backward) {
     // nothing is kept for a backward: the scan is one kernel that takes dt_raw, x and the B | C pair as the conv left them
     FwdWs f{};
     if (!fwd_ws_layout(d, ws, ws_bytes, w16 != nullptr, pr, wx && wx->pairs, plain, &f))
@@ -536,7 +538,7 @@ pmb_status stack_fwd(cudaStream_t st, const Dims& d, int n_layers, const pmb_blo
   char* base = static_cast<char*>(saved);
   for (int l = 0; l < n_layers; ++l) {
     const void* h = base + (size_t)l * slot;
-    PMB_TRY(block_fwd(st, d, layers[l], h, h, base + (size_t)(l + 1) * slot, ws, ws_bytes, w16 ? &w16[l] : nullptr, l > 0, l + 1 < n_layers));
+    PMB_TRY(block_fwd(st, d, layers[l], h, h, base + (size_t)(l + 1) * slot, ws, ws_bytes, w16 ? &w16[l] : nullptr, l > 0, l + 1 < n_layers, true));
   }
   return PMB_OK;
 }

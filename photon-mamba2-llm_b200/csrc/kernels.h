@@ -193,7 +193,8 @@ size_t block_ws_bytes(const Dims& d, bool bf16 = false);
 size_t stack_ws_bytes(const Dims& d, bool bf16 = false, bool presplit = false);   // two forward slots: lets stack_bwd recompute one block ahead
 pmb_status cast_f32_bf16(cudaStream_t st, const float* src, uint16_t* dst, int64_t n);
 pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, const void* x, const void* residual,
-                     void* out, void* ws, size_t ws_bytes, const Weights16* w16, bool x_pair_ready = false, bool emit_out_pair = false);
+                     void* out, void* ws, size_t ws_bytes, const Weights16* w16, bool x_pair_ready = false, bool emit_out_pair = false,
+                     bool backward_follows = false);
 pmb_status block_bwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, const void* x, const void* dout,
                      const void* dx_accum, void* dx, const pmb_block_grads& g, void* ws, size_t ws_bytes, const Weights16* w16,
                      bool dout_pair_ready = false, bool emit_dx_pair = false);
