@@ -605,12 +605,12 @@ __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_bwd_kernel(const f
 }
 
 // float4 variant of the backward.  Optional extras (see NormBwdExtra): dz as a (hi, lo) bf16 pair instead of fp32, and dY exp(S) for
-// the scan backward.  Bound by HBM (reads of dout, y, z, writes of dy and the bf16 copies).  A block walks `nrows` rows and requests
-// the next one before it reduces the current one; few long blocks also leave few partial sums of dw (one row of them per block).
-// Measured at 16384 rows of 1536 with plain bf16 copies (550 MB): 136 us + 60 us of partial sums with four rows per block and no
-// request ahead, 145 us + 3 now.
+// the scan backward.  Bound by HBM (reads of dout, y, z, writes of dy and the bf16 copies).  A block walks `nrows` rows
+// with its share of dw in registers: few long blocks leave few partial sums (one row of them per block), and the three to five blocks
+// that share an SM cover each other's loads (two blocks per SM with the next row requested ahead: 145 us, three: 181).
+// Measured at 16384 rows of 1536 with plain bf16 copies (550 MB): 136 us + 60 us of partial sums with four rows per block, 117 us + 3 now.
 template <int PER>
-__global__ void __launch_bounds__(NORM_THREADS, 2) gated_rmsnorm_bwd_vec_kernel(const float* __restrict__ dout, const float* __restrict__ y,
+__global__ void __launch_bounds__(NORM_THREADS, 3) gated_rmsnorm_bwd_vec_kernel(const float* __restrict__ dout, const float* __restrict__ y,
                                                                              const float* __restrict__ z, int64_t ldz,
                                                                              const float* __restrict__ w, const float* __restrict__ rstd,
                                                                              float* __restrict__ dy, float* __restrict__ dz, int64_t lddz,
@@ -627,27 +627,20 @@ __global__ void __launch_bounds__(NORM_THREADS, 2) gated_rmsnorm_bwd_vec_kernel(
   }
   const int64_t r0 = (int64_t)blockIdx.x * nrows;
   const int64_t r1 = r0 + nrows < rows ? r0 + nrows : rows;
-  float4 zn[PER], yn[PER], dnn[PER];
-  auto request = [&](int64_t row) {
-#pragma unroll
-    for (int n = 0; n < PER; ++n) {
-      const int i = threadIdx.x + n * blockDim.x;
-      zn[n] = yn[n] = dnn[n] = make_float4(0, 0, 0, 0);
-      if (i < nvec) {
-        zn[n] = reinterpret_cast<const float4*>(z + row * ldz)[i];
-        yn[n] = reinterpret_cast<const float4*>(y + row * width)[i];
-        dnn[n] = reinterpret_cast<const float4*>(dout + row * width)[i];
-      }
-    }
-  };
-  if (r0 < r1) request(r0);
   for (int64_t row = r0; row < r1; ++row) {
     const float r = rstd[row];
     float4 zv[PER], yv[PER], dn[PER], gv[PER], sv[PER];
     float dot = 0.0f;
 #pragma unroll
-    for (int n = 0; n < PER; ++n) { zv[n] = zn[n]; yv[n] = yn[n]; dn[n] = dnn[n]; }
-    if (row + 1 < r1) request(row + 1);
+    for (int n = 0; n < PER; ++n) {
+      const int i = threadIdx.x + n * blockDim.x;
+      zv[n] = yv[n] = dn[n] = make_float4(0, 0, 0, 0);
+      if (i < nvec) {
+        zv[n] = reinterpret_cast<const float4*>(z + row * ldz)[i];
+        yv[n] = reinterpret_cast<const float4*>(y + row * width)[i];
+        dn[n] = reinterpret_cast<const float4*>(dout + row * width)[i];
+      }
+    }
 #pragma unroll
     for (int n = 0; n < PER; ++n) {
       sv[n] = make_float4(sigmoid_acc(zv[n].x), sigmoid_acc(zv[n].y), sigmoid_acc(zv[n].z), sigmoid_acc(zv[n].w));
@@ -736,8 +729,8 @@ pmb_status gated_rmsnorm_bwd(cudaStream_t st, int64_t rows, int width, const flo
   if (vec_ok) {
     int per = 1;
     const int threads = norm_vec_threads(width, &per);
-    // two blocks per SM walk the rows; below four rows each the partial sums would outgrow the workspace's rows
-    int64_t nr = cdiv(rows, 2 * 148);
+    // two waves of the blocks that fit; below four rows each the partial sums would outgrow the workspace's rows
+    int64_t nr = cdiv(rows, 8 * 148);
     if (nr < NORM_ROWS) nr = NORM_ROWS;
     nblk = cdiv(rows, nr);
     if (per == 1) gated_rmsnorm_bwd_vec_kernel<1><<<(unsigned)nblk, threads, 0, st>>>(dout, y, z, ldz, w, rstd, dy, dz, lddz, partial, rows, width, (int)nr, ex);
