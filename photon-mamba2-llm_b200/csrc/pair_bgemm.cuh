@@ -141,8 +141,13 @@ pair_bgemm_kernel(const __grid_constant__ MapSet maps, Op op, unsigned int* __re
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    // ---------------- MMA issuer (the whole warp waits, one elected lane issues) ----------------
+    auto wait_all = [&](uint32_t bar, uint32_t parity, unsigned int code) -> bool {
+      const bool got = __all_sync(0xffffffffu, mbar_wait(bar, parity));
+      if (!got && lane == 0) { atomicOr(status, code); *abort_flag = 1; }
+      return got && !__any_sync(0xffffffffu, *abort_flag != 0);
+    };
+    {
       int it = 0;
       bool stop = false;
       const uint32_t d_hi = desc_hi(1024, 2);
@@ -158,19 +163,20 @@ pair_bgemm_kernel(const __grid_constant__ MapSet maps, Op op, unsigned int* __re
         uint32_t tmem_d = tmem_acc;
         if (Op::SEG_EPI) {
           tmem_d = tmem_acc + (uint32_t)((sg & 1) * BN);
-          if (sg >= 2 && !mbar_wait(free_bar(sg & 1), (uint32_t)(((sg >> 1) - 1) & 1))) { atomicOr(status, 32u); *abort_flag = 1; stop = true; break; }
+          if (sg >= 2 && !wait_all(free_bar(sg & 1), (uint32_t)(((sg >> 1) - 1) & 1), 32u)) { stop = true; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
         for (int kt = kt0; kt < kt1; ++kt, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait(full_bar(s), ph)) { atomicOr(status, 2u); *abort_flag = 1; stop = true; break; }
-          if (*abort_flag) { stop = true; break; }
+          if (!wait_all(full_bar(s), ph, 2u)) { stop = true; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a_s = tiles + s * G::STAGE_BYTES;
-          uint32_t al = desc_lo(a_s, a_lbo), bl = desc_lo(a_s + G::A_BYTES, b_lbo);
+          const uint32_t al0 = desc_lo(a_s, a_lbo), bl0 = desc_lo(a_s + G::A_BYTES, b_lbo);
+          if (elect_one()) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
+            const uint32_t al = al0 + k * a_step, bl = bl0 + k * b_step;
             const bool first = Op::SEG_EPI ? (kt == kt0 && k == 0) : (it == 0 && k == 0);
             if (NS == 2) {
               mma_f16_h(tmem_d, al + LO, d_hi, bl, d_hi, idesc, first ? 0u : 1u);
@@ -179,13 +185,16 @@ pair_bgemm_kernel(const __grid_constant__ MapSet maps, Op op, unsigned int* __re
             } else {
               mma_f16_h(tmem_d, al, d_hi, bl, d_hi, idesc, first ? 0u : 1u);
             }
-            al += a_step; bl += b_step;
           }
           umma_commit(empty_bar(s));
+          }
+          __syncwarp();
         }
-        if (Op::SEG_EPI && !stop) umma_commit(seg_bar(sg & 1));
+        if (Op::SEG_EPI && !stop && elect_one()) umma_commit(seg_bar(sg & 1));
+        __syncwarp();
       }
-      umma_commit(accum_bar);
+      if (elect_one()) umma_commit(accum_bar);
+      __syncwarp();
     }
   } else {
     // ---------------- epilogue warps ----------------

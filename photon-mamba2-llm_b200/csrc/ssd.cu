@@ -759,17 +759,13 @@ __global__ void __launch_bounds__(PREP_THREADS) chunk_rows_finish_kernel(SsdP p,
 // goes through y - D x or through two separately rounded matrix products.  da = reverse cumsum(dS);
 // ddt = <dx~, x> + A da;  dx = dx~ dt + D dY;  per-chunk partials of dA and dD.
 struct WSums { const float* rpart; const float* csum; const float* esum; const float* yoff; int nb; };
-// Each half-warp has two rows in flight per pass (all loads of both rows are issued before the first use), and two
-// CTAs fit on an SM, so that the 192 CTAs of a 2048-token launch at 24 heads are resident at once (one CTA per SM
-// meant a second wave of 44 CTAs).
+// Each half-warp has two rows in flight per pass (all loads of both rows are issued before the first use), and three CTAs share an
+// SM: while one sums over its chunk another streams.  16384 tokens, 24 heads: 159 us with two CTAs, 127 with three (500 MB).
 constexpr int ROWS_THREADS = 256;
-// LEAN16 (the bf16-input scan: no dt, no skip term, dx = dx~ already written by the fused kernel): only <dY, y_off>
-// is formed per row, dY (dy16) and y_off (ws.yoff, reinterpreted) both read as bf16 rows of H*P.
-template <bool LEAN16>
-__global__ void __launch_bounds__(ROWS_THREADS, LEAN16 ? 3 : 2) chunk_rows_finish_w_kernel(SsdP p, WSums ws, float* __restrict__ dx, int64_t lddx,
+__global__ void __launch_bounds__(ROWS_THREADS, 3) chunk_rows_finish_w_kernel(SsdP p, WSums ws, float* __restrict__ dx, int64_t lddx,
                                                                            const float* __restrict__ dd, float* __restrict__ da_out,
                                                                            float* __restrict__ ddt_out, float* __restrict__ part,
-                                                                           SsdGrads::RawDt raw, const uint16_t* __restrict__ dy16) {
+                                                                           SsdGrads::RawDt raw) {
   __shared__ float s_ddtx[PREP_MAX_Q], s_dS[PREP_MAX_Q], s_dD[PREP_MAX_Q], s_dt[PREP_MAX_Q], s_e[PREP_MAX_Q], wsum[ROWS_THREADS / 32], red[32];
   constexpr int NHW = ROWS_THREADS / 16;
   const int w = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
@@ -779,54 +775,7 @@ __global__ void __launch_bounds__(ROWS_THREADS, LEAN16 ? 3 : 2) chunk_rows_finis
   const int P4 = p.P >> 2;
   const int hw = tid >> 4, l16 = lane & 15;
   const int64_t hp = (int64_t)p.H * p.P;
-  if (LEAN16) {
-    // eight lanes per row (16 bytes of dY and of y_off each per pass), four rows per warp and four such groups in
-    // flight per thread; y_off was written as bf16 by the fused forward kernel
-    const uint16_t* yoff16 = reinterpret_cast<const uint16_t*>(ws.yoff);
-    const int P8 = p.P >> 3, l8 = lane & 7, sub = lane >> 3;
-    constexpr int NW = ROWS_THREADS / 32, U = 4;
-    for (int tb = 0; tb < p.Q; tb += NW * 4 * U) {
-      int t[U]; float s2[U], rr[U], cs[U], es[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        t[u] = tb + (u * NW + wid) * 4 + sub; s2[u] = 0.0f; rr[u] = 0.0f; cs[u] = 0.0f; es[u] = 0.0f;
-        if (t[u] < p.Q && l8 == 0) {
-          const int64_t idx = (tok0 + t[u]) * p.H + h;
-          for (int rb = 0; rb <= t[u] / 128; ++rb) rr[u] += ws.rpart[((int64_t)w * ws.nb + rb) * p.Q + t[u]];
-          cs[u] = ws.csum[idx]; es[u] = ws.esum[idx];
-        }
-      }
-      for (int j = l8; j < P8; j += 8) {
-        uint4 d[U], y[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (t[u] < p.Q) {
-            const int64_t o = (tok0 + t[u]) * hp + h * p.P + 8 * j;
-            d[u] = *reinterpret_cast<const uint4*>(dy16 + o);
-            y[u] = *reinterpret_cast<const uint4*>(yoff16 + o);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (t[u] < p.Q) {
-            const uint32_t dw[4] = {d[u].x, d[u].y, d[u].z, d[u].w}, yw[4] = {y[u].x, y[u].y, y[u].z, y[u].w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              s2[u] = fmaf(__uint_as_float(dw[e] << 16), __uint_as_float(yw[e] << 16), s2[u]);
-              s2[u] = fmaf(__uint_as_float(dw[e] & 0xffff0000u), __uint_as_float(yw[e] & 0xffff0000u), s2[u]);
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-#pragma unroll
-        for (int o = 4; o > 0; o >>= 1) s2[u] += __shfl_xor_sync(0xffffffffu, s2[u], o);
-        if (t[u] < p.Q && l8 == 0) { s_e[t[u]] = es[u]; s_dS[t[u]] = ((rr[u] - cs[u]) + s2[u]) - es[u]; }
-      }
-    }
-  }
-  for (int tb = 0; !LEAN16 && tb < p.Q; tb += 2 * NHW) {
+  for (int tb = 0; tb < p.Q; tb += 2 * NHW) {
     const int t[2] = {tb + hw, tb + NHW + hw};
     float s1[2] = {0.0f, 0.0f}, s2[2] = {0.0f, 0.0f}, s3[2] = {0.0f, 0.0f}, dtv[2] = {1.0f, 1.0f};
     float rr[2] = {0.0f, 0.0f}, cs[2] = {0.0f, 0.0f}, es[2] = {0.0f, 0.0f};
@@ -1326,7 +1275,7 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
                           reinterpret_cast<uintptr_t>(g.dx) | reinterpret_cast<uintptr_t>(p.dxt)) % 16 == 0);
     if (fz) {
       WSums wsm{ws.rpart, ws.csum, ws.esum, ws.yoff, p.Q / 128};
-      chunk_rows_finish_w_kernel<false><<<(unsigned)nbch, ROWS_THREADS, 0, st>>>(p, wsm, g.dx, g.lddx, dsend, g.da, g.ddt, ws.part, in.dt ? g.raw : SsdGrads::RawDt{}, nullptr);
+      chunk_rows_finish_w_kernel<<<(unsigned)nbch, ROWS_THREADS, 0, st>>>(p, wsm, g.dx, g.lddx, dsend, g.da, g.ddt, ws.part, in.dt ? g.raw : SsdGrads::RawDt{});
       PMB_LAUNCHED();
     } else if (vec_ok && nbch <= 4 * 148 && p.Q <= PREP_MAX_Q) {
       chunk_rows_finish_kernel<<<(unsigned)nbch, PREP_THREADS, 0, st>>>(p, g.dx, g.lddx, dsend, g.da, g.ddt, ws.part);

@@ -254,8 +254,9 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    // ---------------- MMA issuer (the whole warp waits, one elected lane issues) ----------------
+    auto wait_all = [&](int b, uint32_t parity, unsigned int code) -> bool { return __all_sync(0xffffffffu, wait(b, parity, code)); };
+    {
       const uint32_t id_g = idesc_bf16(0, 0, RB, CW);       // G: both operands K-major
       const uint32_t id_v = idesc_bf16(0, 1, RB, P);        // x V and x state: B operand MN-major
       // Operand descriptors as (lo, hi) halves: hi never changes, lo = address field | leading offset.  A product
@@ -273,27 +274,31 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
           mma_f16_h(d, alo, dh, blo, dh, idesc, acc);
         }
       };
-      bool ok = wait(R_FULL, 0u, 2u) && wait(LD_FULL + 0, 0u, 2u);
+      bool ok = wait_all(R_FULL, 0u, 2u) && wait_all(LD_FULL + 0, 0u, 2u);
       if (ok) {
         // carried-state term: acc2 = R x state  (K = d_state)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t r0 = lo_k(rop_s), s0 = lo_mn(ring_s);
+        if (elect_one()) {
 #pragma unroll
         for (int kt = 0; kt < NK; ++kt)
 #pragma unroll
           for (int k = 0; k < 4; ++k)
             kstep(tA2, r0 + ((kt * T128 + k * 32) >> 4), (NK * T128) >> 4, s0 + ((kt * PB * T64 + k * 2048) >> 4), (NK * PB * T64) >> 4, id_v, (kt | k) ? 1u : 0u);
         umma_commit(bar(LD_EMPTY + 0));
+        }
+        __syncwarp();
       }
       // G of column block jj into TMEM buffer jj & 1
       auto mma_g = [&](int jj) -> bool {
         const int it = jj + 1, s = it % STAGES;
-        if (!wait(LD_FULL + s, (uint32_t)((it / STAGES) & 1), 2u)) return false;
+        if (!wait_all(LD_FULL + s, (uint32_t)((it / STAGES) & 1), 2u)) return false;
         // (TM: the buffer's previous content, masked tile jj - 2, was read by a product issued before this one)
-        if (!GE::TM && jj >= 2 && !wait(G_FREE + (jj & 1), (uint32_t)(((jj >> 1) - 1) & 1), 4u)) return false;
+        if (!GE::TM && jj >= 2 && !wait_all(G_FREE + (jj & 1), (uint32_t)(((jj >> 1) - 1) & 1), 4u)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t cop = ring_s + s * GE::STAGE;
         const uint32_t r0 = lo_k(rop_s), c0d = lo_k(cop);
+        if (elect_one()) {
 #pragma unroll
         for (int kt = 0; kt < NK; ++kt)
 #pragma unroll
@@ -310,6 +315,8 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
                     c0d + ((GE::COP + pb * T64 + k * 32) >> 4), (PB * T64) >> 4, id_g, (pb | k) ? 1u : 0u);
         }
         umma_commit(bar(G_FULL + (jj & 1)));
+        }
+        __syncwarp();
         return true;
       };
       // G runs two blocks ahead of the masked product: one block for each mask group
@@ -317,9 +324,10 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
       if (ok && ncb > 1) ok = mma_g(1);
       for (int jj = 0; jj < ncb && ok; ++jj) {
         const int mb = jj % MB, s = (jj + 1) % STAGES;
-        if (!wait(M_READY + mb, (uint32_t)((jj / MB) & 1), 8u)) { ok = false; break; }
+        if (!wait_all(M_READY + mb, (uint32_t)((jj / MB) & 1), 8u)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t m0d = lo_k(mop_s + mb * GE::MOP1), v0d = lo_mn(ring_s + s * GE::STAGE + GE::COP);
+        if (elect_one()) {
         if (GE::TM) {
           // masked tile in TMEM, in place of G: per 32 k of the block [hi: 16 columns | lo: 16 columns], 8 columns per k-step
           const uint32_t bs = (PB * T64) >> 4;
@@ -343,9 +351,12 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
         }
         umma_commit(bar(LD_EMPTY + s));
         umma_commit(bar(M_FREE + mb));
+        }
+        __syncwarp();
         if (jj + 2 < ncb && !mma_g(jj + 2)) { ok = false; break; }
       }
-      umma_commit(bar(ACC_FULL));
+      if (elect_one()) umma_commit(bar(ACC_FULL));
+      __syncwarp();
     }
   } else {
     // ---------------- mask (TMEM -> registers -> shared-memory operand), then epilogue ----------------
