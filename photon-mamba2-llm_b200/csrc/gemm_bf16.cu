@@ -1207,7 +1207,7 @@ int gemm_bf16_ksplit(int64_t M, int64_t N, int64_t K, int64_t other_tiles, int64
 // C = op(A) op(B) (+ R) on bf16 operands, up to MAX_GROUP independent products in one launch (the ones with the longest K first).
 // Row pitches must be multiples of 8 elements (16 bytes) and the bases 16-byte aligned (TMA rules).  ksplit > 1: C is fp32 and
 // receives ksplit slabs of slab_rows rows (a multiple of 256, at least M), which the caller adds up.
-pmb_status gemm_bf16_group(cudaStream_t st, const PlainGemm* gs, int n) {
+pmb_status gemm_bf16_group(cudaStream_t st, const PlainGemm* gs, int n, int max_clusters) {
   using namespace hb;
   if (n < 1 || n > MAX_GROUP) return fail(PMB_ERR_ARG, "gemm_bf16_group: 1 to %d products per launch", MAX_GROUP);
   PMB_SMEM_OPT_IN(Cfg<false>::SMEM_BYTES, gemm_bf16_kernel<false>);
@@ -1252,7 +1252,8 @@ pmb_status gemm_bf16_group(cudaStream_t st, const PlainGemm* gs, int n) {
   ProfScope prof(st, "gemm_bf16", flops, bytes);
   if (pair) {
     PMB_SMEM_OPT_IN((PairPCfg<false, 256>::SMEM_BYTES), gemm_bf16_pairp_kernel<false, 256>);
-    const int64_t slots = persistent_grid(148) / 2;
+    int64_t slots = persistent_grid(148) / 2;
+    if (max_clusters > 0 && slots > max_clusters) slots = max_clusters;
     choose_widths(&g, n, (int)slots);
     clusters = 0;
     for (int i = 0; i < n; ++i) {

@@ -7,7 +7,7 @@ namespace pmb {
 // ---- abi.cu: side streams for kernels that do not depend on each other.  One stream and six events per (device,
 // lane index), created on first use (so the first call should come before any stream capture).  lane 0: scan
 // backward chains; 1: gradient GEMMs of a block that are off the critical path; 2: scan forward; 3: recompute-ahead;
-// 4: embedding-table gradient of the LM head; 5: unused; 6: the gradient kernels of the stack backward (high priority,
+// 4: embedding-table gradient (fp32) or gradient of the hidden rows (bf16) of the LM head; 5: unused; 6: the gradient kernels of the stack backward (high priority,
 // like lane 0).  *out stays NULL past device 63.
 struct SideLane { cudaStream_t s = nullptr; cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr}; };
 pmb_status get_side_lane(int idx, SideLane** out);
@@ -153,7 +153,8 @@ pmb_status gemm_bf16(cudaStream_t st, int ta, int tb, int64_t M, int64_t N, int6
 // (slab_rows a multiple of 256, at least M; ldc as given); sum_slabs adds them up in a fixed order.
 struct PlainGemm { int ta, tb; int64_t M, N, K; const void* A; int64_t lda; const void* B; int64_t ldb; void* C; int64_t ldc; const void* R; int out_bf16;
                    int ksplit = 1; int64_t slab_rows = 0; };
-pmb_status gemm_bf16_group(cudaStream_t st, const PlainGemm* g, int n);      // the ones with the longest K first
+// the ones with the longest K first; max_clusters > 0: leaves the other CTA pairs' SMs to launches of other streams
+pmb_status gemm_bf16_group(cudaStream_t st, const PlainGemm* g, int n, int max_clusters = 0);
 int gemm_bf16_ksplit(int64_t M, int64_t N, int64_t K, int64_t other_tiles, int64_t other_kt);
 pmb_status sum_slabs(cudaStream_t st, const float* part, int n, int64_t pitch, int64_t elems, void* out, int out_bf16);
 pmb_status read_clear_device_status_bf16(unsigned int* word);

@@ -280,6 +280,7 @@ struct pmb_lm {
   float* saved = nullptr;     // (L+1) x (M, D)
   float* dhidden = nullptr;   // (M, D)
   float* logits = nullptr;    // (tile_rows, Vp)
+  float* logits2 = nullptr;   // bf16 storage, long products: a second tile, so that dhidden of one runs under the next one's kernels
   float* row_loss = nullptr;  // (M)
   float* loss = nullptr;      // scalar
   unsigned int* bad = nullptr;
@@ -317,6 +318,15 @@ struct pmb_lm {
   char* gather = nullptr;         // world_size x [(M, D) rows | (M) ids]
   size_t gather_bytes = 0;
 };
+
+// bf16 storage: dhidden = dlogits E of a row tile is a handful of tiles with K = vocab (12 CTA pairs for 236 us at d_model 768 and a
+// 50k vocabulary).  When its pairs are a small part of the machine and its K is long, it runs on a lane of its own under the table
+// gradient of its tile and the logits and cross entropy of the next one, which leave it its SMs.  Per 1024 rows: 424 us with the two
+// gradients in one launch, 363 overlapped.
+static int head_lane_clusters(int64_t rows, int D, int V) {
+  const int64_t t = cdiv(rows, 256) * cdiv(D, 256);
+  return t <= 18 && V >= 8192 ? (int)t : 0;
+}
 
 static int64_t tensor_elems(const Dims& d, int which) {
   switch (which) {
@@ -403,6 +413,10 @@ static pmb_status lm_create_impl(const pmb_mamba2_config* cfg, int L0, int L1, i
     ok = ok && alloc((void**)&lm->params16, (size_t)o * 2);
     lm->ce_inplace = ((size_t)vocab * 4 <= (size_t)CE_MAX_SMEM) ? 1 : 0;
     if (!lm->ce_inplace) ok = ok && alloc((void**)&lm->dlogits16, (size_t)lm->tile_rows * lm->Vp * 2);
+    else if (d.M > lm->tile_rows && head_lane_clusters(lm->tile_rows, d.D, vocab)) {
+      ok = ok && alloc((void**)&lm->logits2, (size_t)lm->tile_rows * lm->Vp * 4);
+      pair_bytes += (size_t)lm->tile_rows * lm->Vp * 4;
+    }
   }
   if (L1 > 0) {
     ok = ok && alloc(&lm->saved1, slot1 * (L1 + 1));
@@ -456,7 +470,7 @@ extern "C" void pmb_lm_destroy(pmb_lm* lm) {
   if (!lm) return;
   cudaFree(lm->params); cudaFree(lm->grads); cudaFree(lm->saved); cudaFree(lm->dhidden); cudaFree(lm->logits);
   cudaFree(lm->row_loss); cudaFree(lm->loss); cudaFree(lm->bad); cudaFree(lm->ids); cudaFree(lm->targets); cudaFree(lm->ws); cudaFree(lm->params16); cudaFree(lm->dlogits16);
-  cudaFree(lm->params_hi); cudaFree(lm->params_lo); cudaFree(lm->dlog_hi); cudaFree(lm->dlog_lo); cudaFree(lm->hid_hi); cudaFree(lm->hid_lo); cudaFree(lm->dh_part);
+  cudaFree(lm->params_hi); cudaFree(lm->params_lo); cudaFree(lm->dlog_hi); cudaFree(lm->dlog_lo); cudaFree(lm->hid_hi); cudaFree(lm->hid_lo); cudaFree(lm->dh_part); cudaFree(lm->logits2);
   cudaFree(lm->gather); cudaFree(lm->l1_pair); cudaFree(lm->saved1); cudaFree(lm->pooled); cudaFree(lm->dpool); cudaFree(lm->dh1); cudaFree(lm->hsum);
   delete lm;
 }
@@ -478,6 +492,7 @@ extern "C" void pmb_lm_activation_detail(const pmb_lm* lm, int64_t* h_out3) {
   h_out3[0] = (int64_t)((size_t)lm->d.M * lm->d.D * esz * (lm->L0 + 1) + (lm->L1 > 0 ? (size_t)lm->d1.M * lm->d.D * esz * (lm->L1 + 1) : 0));                          // stored for backward: block inputs
   h_out3[1] = (int64_t)lm->ws_bytes;                                                              // transient: one block's workspace
   h_out3[2] = (int64_t)((size_t)lm->tile_rows * lm->Vp * (lm->ce_inplace ? 4 : (lm->bf16 ? 6 : (lm->pairs ? 8 : 4))) + (size_t)lm->d.M * lm->d.D * esz +
+                        (lm->logits2 ? (size_t)lm->tile_rows * lm->Vp * 4 : 0) +
                         (lm->pairs ? (size_t)lm->tile_rows * lm->d.D * 4 : 0));  // transient: logits tile (+ its gradient's pair), d(hidden)
 }
 extern "C" const float* pmb_lm_loss_device(const pmb_lm* lm) { return lm ? lm->loss : nullptr; }
@@ -580,14 +595,22 @@ extern "C" pmb_status pmb_lm_step_device(pmb_lm* lm, void* stream, const int64_t
     static const int on = [] { const char* e = getenv("PMB_HEAD_CONCURRENT"); return (e && e[0] == '0') ? 0 : 1; }();
     if (on) PMB_TRY(get_side_lane(4, &table_lane));
   }
-  for (int64_t r0 = 0; r0 < M; r0 += lm->tile_rows) {
+  SideLane* dh_lane = nullptr;
+  if (lm->logits2) PMB_TRY(get_side_lane(4, &dh_lane));
+  const int lane_clusters = dh_lane ? head_lane_clusters(lm->tile_rows, D, V) : 0;
+  float* const tile0 = lm->logits;
+  for (int64_t r0 = 0, tile = 0; r0 < M; r0 += lm->tile_rows, ++tile) {
+    float* const logits = dh_lane && (tile & 1) ? lm->logits2 : tile0;
+    const bool on_lane = dh_lane && r0 + lm->tile_rows < M;                 // (the last tile has nothing to run under)
+    const int others = dh_lane && tile > 0 ? 74 - lane_clusters : 0;        // what the previous tile's dhidden leaves
+    if (dh_lane && tile > 1) PMB_CUDA(cudaStreamWaitEvent(st, dh_lane->ev[1 + (tile & 1)], 0));      // the buffer's last reader
     int64_t rows = M - r0 < lm->tile_rows ? M - r0 : lm->tile_rows;
     const void* hrows = hidden + (size_t)r0 * D * esz;
     // logits = hidden E^T   (photon/embedding.rs:54-60), kept in fp32 for the softmax
     const Pair16 hid_p{lm->hid_hi, lm->hid_lo, D};
     const Pair16 dlog_p = lm->ce_inplace ? Pair16{reinterpret_cast<uint16_t*>(lm->logits), reinterpret_cast<uint16_t*>(lm->logits) + Vp, 2 * (int64_t)Vp}
                                          : Pair16{lm->dlog_hi, lm->dlog_lo, Vp};
-    if (h16) PMB_TRY(gemm_bf16(st, 0, 1, rows, V, D, hrows, D, table16, D, lm->logits, Vp, nullptr, 0));
+    if (h16) { const PlainGemm e{0, 1, rows, V, D, hrows, D, table16, D, logits, Vp, nullptr, 0}; PMB_TRY(gemm_bf16_group(st, &e, 1, others)); }
     else if (prs) {
       PMB_TRY(split_pair16(st, static_cast<const float*>(hrows), rows, D, D, lm->hid_hi, lm->hid_lo, D));
       PMB_TRY(gemm_pairs(st, 0, 1, rows, V, D, hid_p, table_p, lm->logits, Vp, nullptr));
@@ -597,8 +620,8 @@ extern "C" pmb_status pmb_lm_step_device(pmb_lm* lm, void* stream, const int64_t
     if ((prs || h16) && lm->ce_inplace) {
       PMB_SMEM_OPT_IN(CE_MAX_SMEM, cross_entropy_pair_inplace_kernel);
       // (one CTA per SM; more where a short row lets several share one)
-      const int64_t ctas = 148 * (V * 4 > 100 * 1024 ? 1 : 2);
-      cross_entropy_pair_inplace_kernel<<<(unsigned)(rows < ctas ? rows : ctas), CE_THREADS, (size_t)V * 4, st>>>(lm->logits, Vp, V, d_targets + r0, lm->row_loss + r0,
+      const int64_t ctas = (others ? 2 * others : 148) * (V * 4 > 100 * 1024 ? 1 : 2);
+      cross_entropy_pair_inplace_kernel<<<(unsigned)(rows < ctas ? rows : ctas), CE_THREADS, (size_t)V * 4, st>>>(logits, Vp, V, d_targets + r0, lm->row_loss + r0,
                                                                                                                   1.0f / (float)M, prs ? 1 : 0, lm->bad, rows);
     } else
       cross_entropy_kernel<<<(unsigned)rows, 256, 0, st>>>(lm->logits, Vp, V, d_targets + r0, lm->row_loss + r0, 1.0f / (float)M,
@@ -607,13 +630,21 @@ extern "C" pmb_status pmb_lm_step_device(pmb_lm* lm, void* stream, const int64_t
     // dhidden = dlogits E ;  dE (+)= dlogits^T hidden
     if (h16) {
       // in place: the bf16 gradient sits at the start of each logits row (pitch 2*Vp bf16 elements)
-      const uint16_t* dl16 = lm->ce_inplace ? reinterpret_cast<const uint16_t*>(lm->logits) : lm->dlogits16;
+      const uint16_t* dl16 = lm->ce_inplace ? reinterpret_cast<const uint16_t*>(logits) : lm->dlogits16;
       const int64_t ldl = lm->ce_inplace ? 2 * (int64_t)Vp : Vp;
       if (!lm->ce_inplace) PMB_TRY(cast_f32_bf16(st, lm->logits, lm->dlogits16, rows * Vp));
       // one launch: the few long tiles of dhidden take a cluster each, the many short ones of dE the others
       const PlainGemm both[2] = {{0, 0, rows, D, V, dl16, ldl, table16, D, dhid + (size_t)r0 * D * 2, D, nullptr, 1},
                                  {1, 0, V, D, rows, dl16, ldl, hrows, D, dtable, D, r0 == 0 ? nullptr : dtable, 0}};
-      PMB_TRY(gemm_bf16_group(st, both, 2));
+      if (on_lane) {
+        PMB_TRY(order_after(st, dh_lane->ev[0], dh_lane->s));
+        PMB_TRY(gemm_bf16_group(dh_lane->s, &both[0], 1));
+        PMB_CUDA(cudaEventRecord(dh_lane->ev[1 + (tile & 1)], dh_lane->s));
+        PMB_TRY(gemm_bf16_group(st, &both[1], 1, 74 - lane_clusters));
+      } else {
+        if (dh_lane) PMB_CUDA(cudaStreamWaitEvent(st, dh_lane->ev[1 + ((tile + 1) & 1)], 0));       // the previous tile's: all of dhidden is there
+        PMB_TRY(gemm_bf16_group(st, both, 2));
+      }
     } else if (prs && table_lane) {
       // only dhidden is needed now; the embedding-table gradient runs on its own stream (next to the first blocks of
       // the stack backward for the last row tile) and is joined before the embedding scatter.  With several row tiles
