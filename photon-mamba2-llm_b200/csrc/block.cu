@@ -194,6 +194,18 @@ static ChainArgs chain_inputs(const Dims& d, const pmb_block_params& p, const fl
   return a;
 }
 
+// bf16-storage blocks on whole chunks: plain bf16 operands, and few long sequences scanned chunk by chunk instead of as chains.  (Plain
+// bf16 chunks keep the rounding of the kernels that work chunk by chunk, so their sequences are not cut into segments.  One step of a
+// chain takes 3.5 us; those kernels 30 us and 0.1 us per step of a head.  Where a backward follows the chain also writes what that reads:
+// 7.7 us per step against 30 us and 0.07.  Long-context step 49.09 -> 47.14 ms; with the first line, blocks of 48 chains of twelve steps
+// lost 4 %.)
+static bool block_plain16(const Dims& d, bool bf16) { return bf16 && ssd_plain16_shape(d.P, d.N, d.Q); }
+static bool scan_by_chunks(const Dims& d, bool bf16, bool keep) {
+  const double steps = (double)cdiv(d.T, SCAN_STEP), chains = (double)d.B * d.H;
+  if (!block_plain16(d, bf16)) return false;
+  return keep ? 7.7 * steps * (chains > 148.0 ? chains / 148.0 : 1.0) > 30.0 + 0.07 * chains * steps : 3.5 * steps > 30.0 + 0.1 * chains * steps;
+}
+
 // Steps 1-8 of Mamba2Block::forward (block.rs:143-222): everything up to the normalised gate output.
 // In bf16-storage mode (w16 != NULL) x is bf16, the two projections run as bf16 GEMMs with fp32 accumulation
 // against bf16 copies of the weights, and everything between them (the reference's "fp32 islands",
@@ -232,6 +244,12 @@ static pmb_status block_fwd_core(cudaStream_t st, const Dims& d, const pmb_block
   if (chain) {
     ChainArgs a = chain_inputs(d, p, w.xzd, w.act, w.ssd.bc_hi, w.ssd.bc_lo, w.y);
     a.S_out = w.ssd.S; a.dt_out = w.dt; a.A_out = w.Aneg; a.hp_hi = w.ssd.hp_hi; a.hp_lo = w.ssd.hp_lo; a.seg = w.seg;
+    PMB_TRY(ssd_chain_fwd(st, a));
+  } else if (block_plain16(d, w16 != nullptr) && bc.hi && ssd_chain_enabled() && !scan_by_chunks(d, true, true)) {
+    // the backward reads S, the states, x~, xs and the carried part of y: the chain leaves them on its way
+    ChainArgs a = chain_inputs(d, p, w.xzd, w.act, w.ssd.bc_hi, nullptr, w.y);
+    a.blocks = d.Q / SCAN_STEP;
+    a.S_out = w.ssd.S; a.dt_out = w.dt; a.A_out = w.Aneg; a.hp_hi = w.ssd.hp_hi; a.hprev = w.ssd.hprev; a.yoff = w.ssd.yoff; a.xt = w.ssd.xt_hi; a.xs = w.ssd.xs_hi;
     PMB_TRY(ssd_chain_fwd(st, a));
   } else {
   sin.plain16 = w16 != nullptr;
@@ -276,11 +294,7 @@ pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, 
   const Weights16* w16 = storage_is_bf16(wx) ? wx : nullptr;
   const bool pr = !w16 && block_uses_pairs(d);
   BlockWs w{};
-  const bool plain = w16 && ssd_plain16_shape(d.P, d.N, d.Q);
-  // (plain bf16 chunks keep the rounding of the kernels that work chunk by chunk, so their sequences are not cut: few long ones
-  // are faster chunk by chunk.  One step of a chain takes 3.5 us; those kernels 30 us and 0.1 us per step of a head.)
-  const int64_t steps = cdiv(d.T, SCAN_STEP);
-  const bool by_chunks = plain && 3.5 * steps > 30.0 + 0.1 * (double)((int64_t)d.B * d.H * steps);
+  const bool plain = block_plain16(d, w16 != nullptr), by_chunks = scan_by_chunks(d, w16 != nullptr, false);
   // (the backward of a stack whose blocks keep the FMA contractions amplifies any difference between the forward's scan and its own)
   const bool as_backward = backward_follows && !w16 && !block_uses_chain_bwd(d, false, wx && wx->pairs);
   if (ssd_chain_enabled() && ssd_chain_shape(d.P, d.N) && !by_chunks && !as_backward) {

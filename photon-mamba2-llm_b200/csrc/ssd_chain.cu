@@ -76,7 +76,7 @@ struct Geo {
   static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 256 /*barriers*/ + NSB * NB * L * 4 + (BIG ? 4 : 8) * NB * L /*row factors*/ + AHEAD * XF_THREADS * 16;
 };
 
-struct Maps { CUtensorMap b[2], c[2]; };                 // [0] = hi (or the plain bf16 tensor), [1] = lo
+struct Maps { CUtensorMap b[2], c[2], xt, xs; };         // [0] = hi (or the plain bf16 tensor), [1] = lo
 
 struct Params {
   int T, H, hpg, N, P, nsteps;
@@ -90,6 +90,10 @@ struct Params {
   uint16_t* x_keep;                                      // (B,T,H,P) copy of x16
   uint16_t *hp_hi, *hp_lo;                               // (B,nsteps,H,N,P)
   float* last;                                           // (B,H,N,P)
+  // plain operands, for a backward that works chunk by chunk: state entering each chunk in fp32, exp(S) C h of every token, and
+  // (store_ops) x~ and xs as the kernel formed them
+  float *hprev, *yoff;
+  int store_ops;
   int nseg, per;                                         // segments of a sequence, steps per segment
   int state_only;                                        // first of two passes over segments: only seg_h and seg_d are formed
   float *seg_h, *seg_d;                                  // (B*H,nseg,N,P), (B*H,nseg): state that a segment leaves when it starts from none, decay over it
@@ -116,6 +120,11 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
       "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
       : "memory");
+}
+
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(src) : "memory");
 }
 
 template <int NI, int ND, int NK, int NB, bool XIN16>
@@ -148,7 +157,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar(FULL + i), 1); mbar_init(bar(EMPTY + i), 1);
-      mbar_init(bar(XRDY + i), 8); mbar_init(bar(XFREE + i), 1);
+      mbar_init(bar(XRDY + i), 8); mbar_init(bar(XFREE + i), ND == 1 && p.store_ops ? 2 : 1);
       mbar_init(bar(GFULL + i), 1); mbar_init(bar(MRDY + i), 8);
     }
     for (int i = 0; i < 4; ++i) mbar_init(bar(SRDY + i), 8);
@@ -199,6 +208,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       }
       if (*abort_flag)
         for (int i = (issued > STG ? issued - STG : 0); i < issued; ++i) mbar_wait(bar(FULL + i % STG), (uint32_t)((i / STG) & 1));
+    }
+  } else if (ND == 1 && warp == 3 && p.store_ops) {
+    // ---------------- x~ and xs go out as they lie in shared memory ----------------
+    if (lane == 0) {
+      for (int i = 0; i < n; ++i) {
+        const int xb = i % XB;
+        if (!wait(XRDY + xb, (uint32_t)(i / XB), 1024u)) break;
+        tma_store_4d(&maps.xt, xbuf_s + xb * GE::XBUF, 0, toff + i * L, h, bb);
+        tma_store_4d(&maps.xs, xbuf_s + xb * GE::XBUF + GE::XT, 0, toff + i * L, h, bb);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        mbar_arrive(bar(XFREE + xb));
+      }
+      asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer (the whole warp waits; one elected lane issues) ----------------
@@ -403,6 +426,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                   const float f = fac[2 * rh + e];
+                  if (NI == 1 && !XIN16 && p.yoff) {
+                    const int t = toff + (i - 1) * L + er + 16 * rh + 8 * e;
+                    if (t < p.T && 32 * grp + 16 * c16 + 8 * q < p.P)
+                      *reinterpret_cast<float2*>(p.yoff + (tokb + t) * (int64_t)(p.H * p.P) + col + 16 * c16 + 8 * q) =
+                          make_float2(f * __uint_as_float(a2[4 * q + 2 * e]), f * __uint_as_float(a2[4 * q + 2 * e + 1]));
+                  }
                   o[rh][2 * c16 + q][e] = make_float2(fmaf(f, __uint_as_float(a2[4 * q + 2 * e]), __uint_as_float(a1[4 * q + 2 * e])),
                                                       fmaf(f, __uint_as_float(a2[4 * q + 2 * e + 1]), __uint_as_float(a1[4 * q + 2 * e + 1])));
                 }
@@ -557,7 +586,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
             const float f0 = __uint_as_float(xq.x) * f.x, f1 = __uint_as_float(xq.y) * f.x, f2 = __uint_as_float(xq.z) * f.x, f3 = __uint_as_float(xq.w) * f.x;
             uint32_t h0, h1, l0 = 0u, l1 = 0u, g0, g1, k0 = 0u, k1 = 0u;
             split2(f0, f1, h0, l0, ND == 2); split2(f2, f3, h1, l1, ND == 2);
-            split2(f0 * f.y, f1 * f.y, g0, k0, ND == 2); split2(f2 * f.y, f3 * f.y, g1, k1, ND == 2);
+            if (ND == 2) { split2(f0 * f.y, f1 * f.y, g0, k0, true); split2(f2 * f.y, f3 * f.y, g1, k1, true); }
+            else {                                          // (x (dt exp): rounded as the chunk-by-chunk kernels round it)
+              const float fx = f.x * f.y;
+              split2(__uint_as_float(xq.x) * fx, __uint_as_float(xq.y) * fx, g0, k0, false); split2(__uint_as_float(xq.z) * fx, __uint_as_float(xq.w) * fx, g1, k1, false);
+            }
             st_shared_v2(dst, h0, h1);
             st_shared_v2(dst + GE::XT, g0, g1);
             if (ND == 2) { st_shared_v2(dst + T128, l0, l1); st_shared_v2(dst + GE::XT + T128, k0, k1); }
@@ -608,6 +641,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       if (i > 0 && !p.state_only) ok = __all_sync(0xffffffffu, wait(HFREE, (uint32_t)(i - 1), 256u));
       if (!ok) break;
       const int64_t so = (((int64_t)bb * ncht + i0 / NB + i) * p.H + h) * NP + (int64_t)nr * p.P;
+      if (ND == 1 && p.hprev && active) {
+#pragma unroll
+        for (int q = 0; q < PW / 4; ++q)
+          if (4 * q < p.P) *reinterpret_cast<float4*>(p.hprev + so + 4 * q) = make_float4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
+      }
       if (tile && !p.state_only) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {                       // eight 16-byte chunks of the row
@@ -688,6 +726,12 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
   p.x = a.x; p.x16 = a.x16; p.ldx = a.ldx;
   p.dt_raw = a.dt_raw; p.ld_raw = a.ld_raw; p.dt_bias = a.dt_bias; p.a_log = a.a_log; p.dt = a.dt; p.A = a.A; p.a = a.a; p.D = a.D;
   p.init = a.init; p.y = a.y; p.y16 = a.y16; p.ldy = a.ldy; p.dt_out = a.dt_out; p.A_out = a.A_out; p.S_out = a.S_out;
+  p.hprev = a.hprev; p.yoff = a.yoff; p.store_ops = a.xt != nullptr;
+  if (p.store_ops) {
+    const int64_t hp = (int64_t)a.H * a.P;
+    PMB_TRY(sf::bf16_map4(&ms.xt, a.xt, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
+    PMB_TRY(sf::bf16_map4(&ms.xs, a.xs, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
+  }
   p.x_keep = a.x_keep; p.hp_hi = a.hp_hi; p.hp_lo = a.hp_lo; p.last = a.last; p.status = status_ptr();
   p.nseg = 1; p.per = p.nsteps;
   if (NB == 1 && a.seg) {
@@ -734,6 +778,7 @@ pmb_status ssd_chain_fwd(cudaStream_t st, const ChainArgs& a) {
   if (!al16(a.x) || !al16(a.x16) || !al16(a.y) || !al16(a.y16) || !al16(a.init) || (a.ldx & (a.x16 ? 7 : 3)) || (a.ldy & 3))
     return fail(PMB_ERR_SHAPE, "ssd_chain: x, y and state rows must be 16-byte aligned");
   if (!pairs && !a.x16 && a.N > 64) return fail(PMB_ERR_UNSUPPORTED, "ssd_chain: fp32 x with plain bf16 B and C takes d_state up to 64");
+  if ((a.hprev || a.yoff || a.xt) && (pairs || a.x16 || a.seg || (a.xt != nullptr) != (a.xs != nullptr))) return fail(PMB_ERR_ARG, "ssd_chain: the chunk outputs go with fp32 x on plain operands");
   const double tok = (double)a.B * a.T;
   // G and the masked product over the causal half of a step, the state update and the carried-state product
   ProfScope prof(st, "ssd_chain_fwd", tok * a.H * ((double)SCAN_STEP * (a.N + a.P) + 4.0 * a.N * a.P), 0.0);

@@ -45,6 +45,8 @@ struct ChainArgs {
   uint16_t* x_keep;                            // copy of x16, (B,T,H,P)
   uint16_t *hp_hi, *hp_lo;                     // state entering each step, (B,steps,H,N,P)
   float* last;                                 // (B,H,N,P)
+  float *hprev, *yoff;                         // plain operands with fp32 x: (B,chunks,H,N,P) state entering each chunk, (B,T,H,P) exp(S) C h
+  uint16_t *xt, *xs;                           // ... and the operands x~ and xs, (B,T,H,P)
   float* seg = nullptr;                        // ssd_chain_seg_floats() floats: lets few long sequences be walked in segments (blocks == 1)
 };
 int ssd_chain_segments(int B, int T, int H, int* per);      // segments of a sequence; *per = steps of each (the last may have fewer)
