@@ -210,13 +210,17 @@ static bool scan_by_chunks(const Dims& d, bool bf16, bool keep) {
 // In bf16-storage mode (w16 != NULL) x is bf16, the two projections run as bf16 GEMMs with fp32 accumulation
 // against bf16 copies of the weights, and everything between them (the reference's "fp32 islands",
 // block.rs:24-42) stays in fp32.
-// Pair of a weight matrix: the caller's pre-split copy when there is one, else split here into the workspace.
-static pmb_status weight_pair(cudaStream_t st, const Weights16* wx, bool in_proj, const float* src, int64_t rows, int64_t cols,
-                              uint16_t* hi, uint16_t* lo, Pair16* out) {
-  if (wx && wx->pairs) { *out = in_proj ? Pair16{wx->in_proj, wx->in_lo, cols} : Pair16{wx->out_proj, wx->out_lo, cols}; return PMB_OK; }
-  PMB_TRY(split_pair16(st, src, rows, cols, cols, hi, lo, cols));
-  *out = Pair16{hi, lo, cols};
-  return PMB_OK;
+// Pair of a weight matrix: the caller's pre-split copy, or the workspace's arrays, into which `todo` then splits it.
+struct Splits {
+  SplitItem it[4];
+  int n = 0;
+  void add(const float* src, int64_t count, uint16_t* hi, uint16_t* lo) { it[n++] = SplitItem{src, count, hi, lo}; }
+  pmb_status run(cudaStream_t st) { return n ? split_pairs_flat(st, it, n) : PMB_OK; }
+};
+static Pair16 weight_pair(const Weights16* wx, bool in_proj, const float* src, int64_t rows, int64_t cols, uint16_t* hi, uint16_t* lo, Splits* todo) {
+  if (wx && wx->pairs) return in_proj ? Pair16{wx->in_proj, wx->in_lo, cols} : Pair16{wx->out_proj, wx->out_lo, cols};
+  todo->add(src, rows * cols, hi, lo);
+  return Pair16{hi, lo, cols};
 }
 
 // x_pair_ready: the (hi, lo) pair of x is already in the workspace (written by the GEMM that produced x)
@@ -226,9 +230,10 @@ static pmb_status block_fwd_core(cudaStream_t st, const Dims& d, const pmb_block
   const bool pr = !w16 && block_uses_pairs(d);
   if (w16) PMB_TRY(gemm_bf16(st, 0, 0, d.M, d.J, d.D, x, d.D, w16->in_proj, d.J, w.xzd, d.J, nullptr, 0));
   else if (pr) {
-    Pair16 win;
-    if (!x_pair_ready) PMB_TRY(split_pair16(st, static_cast<const float*>(x), d.M, d.D, d.D, w.x_hi, w.x_lo, d.D));
-    PMB_TRY(weight_pair(st, wx, true, p.in_proj_weight, d.D, d.J, w.win_hi, w.win_lo, &win));
+    Splits todo;
+    if (!x_pair_ready) todo.add(static_cast<const float*>(x), (int64_t)d.M * d.D, w.x_hi, w.x_lo);
+    const Pair16 win = weight_pair(wx, true, p.in_proj_weight, d.D, d.J, w.win_hi, w.win_lo, &todo);
+    PMB_TRY(todo.run(st));
     PMB_TRY(gemm_pairs(st, 0, 0, d.M, d.J, d.D, Pair16{w.x_hi, w.x_lo, d.D}, win, w.xzd, d.J, nullptr));
   }
   else PMB_TRY(gemm(st, 0, 0, d.M, d.J, d.D, static_cast<const float*>(x), d.D, p.in_proj_weight, d.J, w.xzd, d.J, nullptr, 0));
@@ -294,6 +299,7 @@ pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, 
   const Weights16* w16 = storage_is_bf16(wx) ? wx : nullptr;
   const bool pr = !w16 && block_uses_pairs(d);
   BlockWs w{};
+  Pair16 wout{nullptr, nullptr, 0};
   const bool plain = block_plain16(d, w16 != nullptr), by_chunks = scan_by_chunks(d, w16 != nullptr, false);
   // (the backward of a stack whose blocks keep the FMA contractions amplifies any difference between the forward's scan and its own)
   const bool as_backward = backward_follows && !w16 && !block_uses_chain_bwd(d, false, wx && wx->pairs);
@@ -304,9 +310,11 @@ pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, 
       return fail(PMB_ERR_WORKSPACE, "block workspace too small (%zu < %zu)", ws_bytes, block_ws_bytes(d, w16 != nullptr));
     if (w16) PMB_TRY(gemm_bf16(st, 0, 0, d.M, d.J, d.D, x, d.D, w16->in_proj, d.J, f.xzd, d.J, nullptr, 0));
     else if (pr) {
-      Pair16 win;
-      if (!x_pair_ready) PMB_TRY(split_pair16(st, static_cast<const float*>(x), d.M, d.D, d.D, f.x_hi, f.x_lo, d.D));
-      PMB_TRY(weight_pair(st, wx, true, p.in_proj_weight, d.D, d.J, f.win_hi, f.win_lo, &win));
+      Splits todo;
+      if (!x_pair_ready) todo.add(static_cast<const float*>(x), (int64_t)d.M * d.D, f.x_hi, f.x_lo);
+      const Pair16 win = weight_pair(wx, true, p.in_proj_weight, d.D, d.J, f.win_hi, f.win_lo, &todo);
+      wout = weight_pair(wx, false, p.out_proj_weight, d.I, d.D, f.wout_hi, f.wout_lo, &todo);
+      PMB_TRY(todo.run(st));
       PMB_TRY(gemm_pairs(st, 0, 0, d.M, d.J, d.D, Pair16{f.x_hi, f.x_lo, d.D}, win, f.xzd, d.J, nullptr));
     }
     else PMB_TRY(gemm(st, 0, 0, d.M, d.J, d.D, static_cast<const float*>(x), d.D, p.in_proj_weight, d.J, f.xzd, d.J, nullptr, 0));
@@ -327,8 +335,11 @@ pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, 
   }
   if (w16) PMB_TRY(gemm_bf16(st, 0, 0, d.M, d.D, d.I, w.normed16, d.I, w16->out_proj, d.D, out, d.D, residual, 1));
   else if (pr) {
-    Pair16 wout;
-    PMB_TRY(weight_pair(st, wx, false, p.out_proj_weight, d.I, d.D, w.wout_hi, w.wout_lo, &wout));
+    if (!wout.hi) {
+      Splits todo;
+      wout = weight_pair(wx, false, p.out_proj_weight, d.I, d.D, w.wout_hi, w.wout_lo, &todo);
+      PMB_TRY(todo.run(st));
+    }
     // the next block reads this output as its in_proj operand: its pair leaves the epilogue (into the x pair of the
     // one forward slot, which this block's own in_proj has long finished reading)
     PairGemm e{0, 0, d.M, d.D, d.I, Pair16{w.normed_hi, w.normed_lo, d.I}, wout, static_cast<float*>(out), d.D, static_cast<const float*>(residual)};
@@ -370,8 +381,10 @@ static pmb_status block_grads(cudaStream_t st, const Dims& d, const pmb_block_pa
   Pair16 wout{}, dop{w.dout_hi, w.dout_lo, d.D};
   if (pr) {
     // (the block above wrote the pair of its dx, which is this block's dout, from its last GEMM's epilogue)
-    if (!dout_pair_ready) PMB_TRY(split_pair16(st, static_cast<const float*>(dout), d.M, d.D, d.D, w.dout_hi, w.dout_lo, d.D));
-    PMB_TRY(weight_pair(st, wx, false, p.out_proj_weight, d.I, d.D, w.wout_hi, w.wout_lo, &wout));
+    Splits todo;
+    if (!dout_pair_ready) todo.add(static_cast<const float*>(dout), (int64_t)d.M * d.D, w.dout_hi, w.dout_lo);
+    wout = weight_pair(wx, false, p.out_proj_weight, d.I, d.D, w.wout_hi, w.wout_lo, &todo);
+    PMB_TRY(todo.run(st));
     // dnormed heads the critical chain of this block: it stays on the caller's stream; only dW_out is deferred
     if (gl) PMB_TRY(gemm_pairs(st, 0, 1, d.M, d.I, d.D, dop, wout, w.dnormed, d.I, nullptr));
   }

@@ -162,6 +162,9 @@ pmb_status read_clear_device_status_bf16(unsigned int* word);
 struct Pair16 { const uint16_t* hi; const uint16_t* lo; int64_t ld; };
 pmb_status split_pair16(cudaStream_t st, const float* src, int64_t rows, int64_t cols, int64_t ld, uint16_t* hi, uint16_t* lo,
                         int64_t ld16);
+// up to four contiguous arrays in one launch (n a multiple of 4, pair arrays 8-byte aligned)
+struct SplitItem { const float* src; int64_t n; uint16_t* hi; uint16_t* lo; };
+pmb_status split_pairs_flat(cudaStream_t st, const SplitItem* items, int n);
 // same, but writes only columns [0, cols) of each destination row and leaves the rest of the pitch untouched
 pmb_status split_pair16_strided(cudaStream_t st, const float* src, int64_t rows, int64_t cols, int64_t ld, uint16_t* hi, uint16_t* lo,
                                 int64_t ld16);
