@@ -113,8 +113,8 @@ int32_t pmb_selftest_device_once(void);
  * tiles (cta_group::2): both operands are split into (hi, lo) bf16 pairs (hi + lo carries 16 mantissa bits) and each
  * k-step issues hi*hi + lo*hi + hi*lo with kind::f16, fp32 accumulation.  Error ~1e-5 of the result's scale (the
  * 3xTF32 kernels: ~1e-6), about twice their speed.  Auto takes the pair engine when the operands are 16-byte aligned
- * with row lengths that are multiples of 8 (a persistent kernel of 256x256 CTA-pair tiles when M > 128 and the product
- * has at least 18 such tiles -- PMB_GEMM_PAIR_MIN changes the 18 -- else the persistent single-CTA kernel), else 3xTF32
+ * with row lengths that are multiples of 8 (a persistent kernel of 256x256 or 256x128 CTA-pair tiles when M > 128 and the
+ * product has at least 4 of the wide ones -- PMB_GEMM_PAIR_MIN changes the 4 -- else the persistent single-CTA kernel), else 3xTF32
  * when its alignment rules hold, else FMA; the environment variable
  * PMB_GEMM_ENGINE=tf32 keeps auto off engine 4, =simt forces FMA.  Engine 4 keeps the split operands in a
  * library-owned scratch buffer that grows on demand (cudaMalloc inside the call); pmb_gemm_reserve_scratch() sizes it
@@ -175,10 +175,11 @@ pmb_status pmb_ssd_scan_bwd(void* stream, int32_t batch, int32_t seqlen, int32_t
 /* Scan with bf16 inputs and fp32 state (the reference upcasts to F32 around Ops::ssd_scan, block.rs:203-208):
  * x, b, c, y and dy, dx, db, dc are contiguous bf16 (B,T,H,P) / (B,T,G,N); a, da and the states are fp32.
  * The backward reads x, b, c from the workspace the forward left behind (keep it untouched in between).
- * With d_head 64, d_state 64 or 128, block_len a multiple of 128 and at most 64 chunks per sequence the bf16 tensors
- * are the tensor-core operands as they are (one kind::f16 MMA per product; cumulative sums, decay factors, chunk
- * states and accumulators in fp32; y and dx written as bf16 by the kernels that form them) and the eight bf16
- * pointers must be 16-byte aligned.  Other shapes widen to fp32, run the fp32 scan and round the results. */
+ * With d_head up to 64 and d_state up to 128 (multiples of 8) the bf16 tensors are the tensor-core operands as they are, at
+ * any length; cumulative sums, decay factors, states and accumulators are fp32, and y and the gradients are written as bf16 by the
+ * kernels that form them.  What is formed on the way (masked tiles, scaled rows, states) enters the products rounded to bf16 when
+ * d_head is 64, d_state 64 or 128, block_len a multiple of 128 and at most 64 chunks make a sequence -- the eight bf16 pointers
+ * must then be 16-byte aligned -- and as (hi, lo) bf16 pairs otherwise.  Other shapes widen to fp32, run the fp32 scan and round. */
 size_t pmb_ssd_workspace_bytes_bf16(int32_t batch, int32_t seqlen, int32_t n_heads, int32_t d_head,
                                     int32_t d_state, int32_t n_groups, int32_t block_len);
 pmb_status pmb_ssd_scan_fwd_bf16(void* stream, int32_t batch, int32_t seqlen, int32_t n_heads, int32_t d_head,
@@ -238,8 +239,8 @@ pmb_status pmb_mamba2_block_bwd(void* stream, const pmb_mamba2_config* cfg, cons
  * fp32 and the caller supplies bf16 copies of the two projection weights (pmb_cast_f32_to_bf16, refreshed whenever
  * the fp32 masters change).  The projections run as bf16 GEMMs with fp32 accumulation; conv, softplus, exp, the
  * scan's recurrence (cumulative sums, decay factors, chunk states, accumulators) and the norm run in fp32 as in the
- * reference; on the shapes the fused scan kernels take (block_len a multiple of 128, d_state = d_head = 64) the
- * scan's tensor-core products read their operands rounded to bf16.  Parameter gradients are fp32.  Needs d_model,
+ * reference; with d_state = d_head = 64 and whole chunks of 128 or 256 tokens the scan's tensor-core products read their
+ * operands rounded to bf16, elsewhere as (hi, lo) bf16 pairs.  Parameter gradients are fp32.  Needs d_model,
  * d_inner and in_proj_dim to be multiples of 8. */
 size_t pmb_mamba2_block_workspace_bytes_bf16(const pmb_mamba2_config* cfg, int32_t batch, int32_t seqlen);
 pmb_status pmb_mamba2_block_fwd_bf16(void* stream, const pmb_mamba2_config* cfg, const pmb_block_params* params,

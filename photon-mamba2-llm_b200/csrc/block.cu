@@ -94,7 +94,7 @@ static size_t slab_floats(const Dims& d) {
 // heads narrower than 64) the two forms are further apart than fp32 results of one call may move.
 static bool block_uses_chain_bwd(const Dims& d, bool bf16, bool in_model) {
   const bool dims = bf16 ? !ssd_plain16_shape(d.P, d.N, d.Q) && d.D % 8 == 0 && d.J % 8 == 0 && d.I % 8 == 0 : block_uses_pairs(d);
-  const bool close = bf16 || in_model || ssd_fused_supported(d.P, d.N, d.Q, true) || d.Q <= (d.P >= 64 ? 256 : 64);
+  const bool close = bf16 || in_model || ssd_fused_supported(d.P, d.N, d.Q) || d.Q <= (d.P >= 64 ? 256 : 64);
   return dims && close && ssd_chain_enabled() && ssd_chain_bwd_shape(d.P, d.N, true) && d.I <= 2048;
 }
 

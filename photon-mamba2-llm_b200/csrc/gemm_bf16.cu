@@ -1163,15 +1163,18 @@ static double makespan(Group* g, int n, int slots) {
   const int clusters = (int)(tiles < slots ? tiles : slots);
   set_lead(g, n, clusters);
   if (tiles > 8 * slots) return total / clusters > most ? total / clusters : most;
+  // the first cluster of the round (and the first one without a long tile) has the most to do: tiles are in order of their length
   double worst = 0.0;
-  for (int c = 0; c < clusters; ++c) {
+  for (int i = 0; i < 2; ++i) {
+    const int c = i ? g->lead : 0;
+    if (i && (c == 0 || c >= clusters)) continue;
     double t = 0.0;
     for (int j = 0;; ++j) {
       const int id = pair_tile_at(*g, c, clusters, j);
       if (id >= tiles) break;
-      int base = 0, i = 0;
-      while (id >= base + g->pr[i].tiles) base += g->pr[i++].tiles;
-      t += tile_cost(g->pr[i]);
+      int base = 0, k = 0;
+      while (id >= base + g->pr[k].tiles) base += g->pr[k++].tiles;
+      t += tile_cost(g->pr[k]);
     }
     if (t > worst) worst = t;
   }

@@ -952,7 +952,7 @@ void ssd_ws_take(Arena& ar, int B, int T, int H, int P, int N, int G, int Q, Ssd
   SsdWs& w = *wp;
   const int nc = T / Q;
   const bool tcshape = Q % 64 == 0 && N % 32 == 0 && P % 64 == 0;
-  const bool fz = ssd_fused_supported(P, N, Q, true) && fused_enabled();
+  const bool fz = ssd_fused_supported(P, N, Q) && fused_enabled();
   const size_t hp = (size_t)B * T * H * P, gn = (size_t)B * T * 2 * G * N, stn = (size_t)B * nc * H * N * P, qq = (size_t)B * nc * G * Q * Q;
   if (part & 1) {
     w.S = ar.take<float>((size_t)B * H * T);
@@ -1128,7 +1128,7 @@ pmb_status ssd_fwd(cudaStream_t st, const SsdIn& in, const float* init_state, fl
   const double tok = (double)p.B * p.T;
   const bool tc = ssd_tc_supported(in) && (ldy % 4 == 0) && (reinterpret_cast<uintptr_t>(y) % 16 == 0);
   // the intra-chunk chain C B^T -> mask -> x x~ (+ the carried-state term) as one tcgen05 kernel on bf16 pairs
-  const bool fz = tc && fused_enabled() && ssd_fused_supported(p.P, p.N, p.Q, true);
+  const bool fz = tc && fused_enabled() && ssd_fused_supported(p.P, p.N, p.Q);
   SsdIn in_tc = in;
   bool xt_ready = false;
   {
@@ -1202,7 +1202,7 @@ __global__ void __launch_bounds__(256) dys_pair_kernel(const float* __restrict__
 bool ssd_bwd_takes_pairs(const SsdIn& in, const float* dy, int64_t lddy, const SsdGrads& g) {
   const bool tc = ssd_tc_supported(in) && (lddy % 4 == 0) && (reinterpret_cast<uintptr_t>(dy) % 16 == 0) && (g.lddbc % 4 == 0) &&
                   ((reinterpret_cast<uintptr_t>(g.db) | reinterpret_cast<uintptr_t>(g.dc)) % 16 == 0);
-  return tc && fused_enabled() && ssd_fused_supported(in.P, in.N, in.Q, true) && (g.lddx % 4 == 0) && (reinterpret_cast<uintptr_t>(g.dx) % 16 == 0);
+  return tc && fused_enabled() && ssd_fused_supported(in.P, in.N, in.Q) && (g.lddx % 4 == 0) && (reinterpret_cast<uintptr_t>(g.dx) % 16 == 0);
 }
 
 pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy, const float* dy, int64_t lddy,
@@ -1264,7 +1264,7 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
   }
   else if (tc) {
     // (a forward that took the fused kernel left no C B^T behind: form it now)
-    if (fused_enabled() && ssd_fused_supported(p.P, p.N, p.Q, true)) PMB_TRY(ssd_tc_cb(st, in, ws));
+    if (fused_enabled() && ssd_fused_supported(p.P, p.N, p.Q)) PMB_TRY(ssd_tc_cb(st, in, ws));
     PMB_TRY(ssd_tc_dx(st, in, dy, lddy, ws));
   }
   else PMB_TRY(run_op(st, "ssd_bwd_dx", make_op<OpDx>(p, p.Q, p.P), nbch, 2.0 * tok * p.H * p.P * (p.Q + p.N)));

@@ -96,10 +96,8 @@ struct Params {
   int H, hpg, Q, nc, nb, T, N;
   const float* S;
   float* out; int64_t ldo;
-  uint16_t* out16;          // when set: the result goes here as bf16 (same row pitch, in elements) instead of to `out`
   const float* x; int64_t ldx; const float* D;
   float* off_out;           // mode 0, optional: (B,T,H,P) the carried-state part of y, exp(S_t) C_t h_prev
-  uint16_t* off_out16;      // the same as bf16 (one of the two at most)
   float* csum; float* esum; // mode 1: (B,T,H)  c_s = sum_{t>s} W[t,s];  e_s = exp(S_end - S_s) <x~_s, B_s dh>
   float* rpart;             // mode 1: (B*nc*H, nb, Q)  partial row sums r_t = sum_{s<t} W[t,s] over the s of one row block
   unsigned int* status;
@@ -482,15 +480,6 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
             od[j] = make_float4(fac * __uint_as_float(a2[4 * j]), fac * __uint_as_float(a2[4 * j + 1]), fac * __uint_as_float(a2[4 * j + 2]),
                                 fac * __uint_as_float(a2[4 * j + 3]));
         }
-        if (MODE == 0 && p.off_out16) {
-          uint2* od = reinterpret_cast<uint2*>(p.off_out16 + (trow * p.H + h) * (int64_t)P + c0);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const __nv_bfloat162 b0 = __floats2bfloat162_rn(fac * __uint_as_float(a2[4 * j]), fac * __uint_as_float(a2[4 * j + 1]));
-            const __nv_bfloat162 b1 = __floats2bfloat162_rn(fac * __uint_as_float(a2[4 * j + 2]), fac * __uint_as_float(a2[4 * j + 3]));
-            od[j] = make_uint2(*reinterpret_cast<const uint32_t*>(&b0), *reinterpret_cast<const uint32_t*>(&b1));
-          }
-        }
         if (MODE == 1) {
           // this row of the x~ tile: 64-element block c0 / 64, 16-byte chunks (c0 % 64) / 8 .. + 3, swizzled
           const uint8_t* xrow = base_ptr + (rop_s - base) + GE::XR_OFF + (c0 >> 6) * T128 + (r_local >> 3) * 1024 + (r_local & 7) * 128;
@@ -511,7 +500,6 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
           }
         }
         float4* dst = reinterpret_cast<float4*>(p.out + trow * p.ldo + h * P + c0);
-        uint2* dst16 = reinterpret_cast<uint2*>(p.out16 + trow * p.ldo + h * P + c0);
         const float4* xs = (MODE == 0 && p.D) ? reinterpret_cast<const float4*>(p.x + trow * p.ldx + h * P + c0) : nullptr;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -524,12 +512,7 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
             const float4 q = (c0 == 32 * grp) ? xpre[j] : xs[j];
             o.x = fmaf(dv, q.x, o.x); o.y = fmaf(dv, q.y, o.y); o.z = fmaf(dv, q.z, o.z); o.w = fmaf(dv, q.w, o.w);
           }
-          if (p.out16) {
-            const __nv_bfloat162 b0 = __floats2bfloat162_rn(o.x, o.y), b1 = __floats2bfloat162_rn(o.z, o.w);
-            dst16[j] = make_uint2(*reinterpret_cast<const uint32_t*>(&b0), *reinterpret_cast<const uint32_t*>(&b1));
-          } else {
-            dst[j] = o;
-          }
+          dst[j] = o;
         }
       }
     }
@@ -635,8 +618,8 @@ static pmb_status launch(cudaStream_t st, const FusedArgs& a) {
   if (NS == 1) { ms.rop[1] = ms.rop[0]; ms.cop[1] = ms.cop[0]; ms.v[1] = ms.v[0]; ms.st[1] = ms.st[0]; ms.xr[1] = ms.xr[0]; }
   Params p{};
   p.H = a.H; p.hpg = a.H / a.G; p.Q = a.Q; p.nc = nc; p.nb = a.Q / RB; p.T = a.T; p.N = a.N;
-  p.S = a.S; p.out = a.out; p.out16 = a.out16; p.ldo = a.ldo; p.x = a.x; p.ldx = a.ldx; p.D = a.D;
-  p.off_out = a.off_out; p.off_out16 = a.off_out16; p.csum = a.csum; p.esum = a.esum; p.rpart = a.rpart;
+  p.S = a.S; p.out = a.out; p.ldo = a.ldo; p.x = a.x; p.ldx = a.ldx; p.D = a.D;
+  p.off_out = a.off_out; p.csum = a.csum; p.esum = a.esum; p.rpart = a.rpart;
   p.status = status_ptr();
   PMB_SMEM_OPT_IN(GE::SMEM, ssd_fused_kernel<MODE, NS, NK, PB>);
   if (GE::CTAS > 1) {      // two CTAs per SM need the largest shared-memory carve-out
@@ -654,44 +637,27 @@ static pmb_status launch(cudaStream_t st, const FusedArgs& a) {
   return PMB_OK;
 }
 
-template <int MODE, int NS>
-static pmb_status pick(cudaStream_t st, const FusedArgs& a) {
-  const int nk = a.N / 64, pb = a.P / 64;
-  if (nk == 1 && pb == 1) return launch<MODE, NS, 1, 1>(st, a);
-  if (NS == 1) {      // plain bf16 operands are half the size: the wider shapes fit as well
-    if (nk == 2 && pb == 1) return launch<MODE, 1, 2, 1>(st, a);
-    if (nk == 1 && pb == 2) return launch<MODE, 1, 1, 2>(st, a);
-    if (nk == 2 && pb == 2) return launch<MODE, 1, 2, 2>(st, a);
-  }
-  return fail(PMB_ERR_UNSUPPORTED, "ssd_fused: d_state %d / d_head %d not supported", a.N, a.P);
-}
-
 }  // namespace sf
 
-bool ssd_fused_supported(int P, int N, int Q, bool pairs) {
-  if (Q % sf::RB != 0 || Q > sf::MAXQ) return false;
-  if (!(N == 64 || N == 128) || !(P == 64 || P == 128)) return false;
-  if (pairs && !(N == 64 && P == 64)) return false;     // the backward's plan (two resident row operands) fits pairs at 64 x 64 only
-  return true;
-}
+bool ssd_fused_supported(int P, int N, int Q) { return Q % sf::RB == 0 && Q <= sf::MAXQ && N == 64 && P == 64; }
 
 pmb_status ssd_fused(cudaStream_t st, int mode, const FusedArgs& a) {
   const bool pairs = a.c.lo != nullptr;
-  if (!ssd_fused_supported(a.P, a.N, a.Q, pairs) || a.T % a.Q != 0 || a.H % a.G != 0)
+  if (!ssd_fused_supported(a.P, a.N, a.Q) || a.T % a.Q != 0 || a.H % a.G != 0)
     return fail(PMB_ERR_UNSUPPORTED, "ssd_fused: unsupported shape (P=%d N=%d Q=%d)", a.P, a.N, a.Q);
   if ((a.b.lo != nullptr) != pairs || (a.v.lo != nullptr) != pairs || (a.state.lo != nullptr) != pairs || (mode == 1 && (a.xt.lo != nullptr) != pairs))
     return fail(PMB_ERR_ARG, "ssd_fused: operands must be all pairs or all plain bf16");
   if (mode == 1 && (!a.xt.hi || !a.csum || !a.esum || !a.rpart)) return fail(PMB_ERR_ARG, "ssd_fused: mode 1 needs x~ and the three sum outputs");
   if ((int64_t)a.B * a.T >= (1LL << 31) || (int64_t)a.B * (a.T / a.Q) * a.H * a.N >= (1LL << 31))
     return fail(PMB_ERR_SHAPE, "ssd_fused: too many rows for 32-bit tile coordinates");
-  if (!a.out && !a.out16) return fail(PMB_ERR_ARG, "ssd_fused: no output");
-  if ((a.ldo & 3) || ((reinterpret_cast<uintptr_t>(a.out) | reinterpret_cast<uintptr_t>(a.out16)) & 15) || (a.D && ((a.ldx & 3) || (reinterpret_cast<uintptr_t>(a.x) & 15))))
+  if (!a.out) return fail(PMB_ERR_ARG, "ssd_fused: no output");
+  if ((a.ldo & 3) || (reinterpret_cast<uintptr_t>(a.out) & 15) || (a.D && ((a.ldx & 3) || (reinterpret_cast<uintptr_t>(a.x) & 15))))
     return fail(PMB_ERR_SHAPE, "ssd_fused: output and x rows must be 16-byte aligned");
   const double tok = (double)a.B * a.T;
   // algorithmic work: G per head (2 Q N), masked product (2 Q P) over the causal half (counted in full), state term (2 N P)
   ProfScope prof(st, mode == 0 ? "ssd_fused_y" : "ssd_fused_dx", 2.0 * tok * a.H * ((double)a.Q * (a.N + a.P) + (double)a.N * a.P), 0.0);
-  if (mode == 0) return pairs ? sf::pick<0, 2>(st, a) : sf::pick<0, 1>(st, a);
-  return pairs ? sf::pick<1, 2>(st, a) : sf::pick<1, 1>(st, a);
+  if (mode == 0) return pairs ? sf::launch<0, 2, 1, 1>(st, a) : sf::launch<0, 1, 1, 1>(st, a);
+  return pairs ? sf::launch<1, 2, 1, 1>(st, a) : sf::launch<1, 1, 1, 1>(st, a);
 }
 
 }  // namespace pmb

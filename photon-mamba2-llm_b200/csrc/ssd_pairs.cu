@@ -6,8 +6,8 @@
 //   dC[t,n]      = sum_{s<=t} dG[t,s] B[s,n] + sum_h sum_p dYs_h[t,p] h_prev_h[n,p]
 //   dB[s,n]      = sum_{t>=s} dG[t,s] C[t,n] + sum_h sum_p xs_h[s,p]  dh_h[n,p]
 // (mamba2/ssd_ops.rs:201-234 and its autograd compute the same quantities op by op.)
-// Shapes: block_len % 128 == 0, d_state = d_head = 64 with (hi, lo) pairs; with plain bf16 operands (no lo arrays in
-// the workspace: the bf16-input scan) d_state may also be 128.  Other shapes keep the 3xTF32 / FMA engines.
+// Shapes: block_len % 128 == 0, d_state = d_head = 64; with (hi, lo) pairs, or on the hi halves alone (bf16-storage blocks).  Other
+// shapes keep the 3xTF32 / FMA engines.
 #include "common.cuh"
 #include "kernels.h"
 #include "pair_bgemm.cuh"
