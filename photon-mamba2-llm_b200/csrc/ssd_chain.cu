@@ -641,11 +641,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       if (i > 0 && !p.state_only) ok = __all_sync(0xffffffffu, wait(HFREE, (uint32_t)(i - 1), 256u));
       if (!ok) break;
       const int64_t so = (((int64_t)bb * ncht + i0 / NB + i) * p.H + h) * NP + (int64_t)nr * p.P;
-      if (ND == 1 && p.hprev && active) {
-#pragma unroll
-        for (int q = 0; q < PW / 4; ++q)
-          if (4 * q < p.P) *reinterpret_cast<float4*>(p.hprev + so + 4 * q) = make_float4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
-      }
       if (tile && !p.state_only) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {                       // eight 16-byte chunks of the row
@@ -655,15 +650,28 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
           const uint32_t a = h_s + (uint32_t)(nr * 128 + ((c ^ (nr & 7)) << 4));
           st_shared_v4(a, hi[0], hi[1], hi[2], hi[3]);
           if (ND == 2) st_shared_v4(a + NK * T64, lo[0], lo[1], lo[2], lo[3]);
-          if (p.hp_hi && active && 8 * c < p.P) {
-            *reinterpret_cast<uint4*>(p.hp_hi + so + 8 * c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            if (ND == 2) *reinterpret_cast<uint4*>(p.hp_lo + so + 8 * c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-          }
         }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(HRDY));
+      // (what a backward keeps goes out after the operand tile, under the products that read it)
+      if (p.hp_hi && active && !p.state_only) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          if (8 * c >= p.P) continue;
+          uint32_t hi[4], lo[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) split2(hv[8 * c + 2 * e], hv[8 * c + 2 * e + 1], hi[e], lo[e], ND == 2);
+          *reinterpret_cast<uint4*>(p.hp_hi + so + 8 * c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+          if (ND == 2) *reinterpret_cast<uint4*>(p.hp_lo + so + 8 * c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        }
+      }
+      if (ND == 1 && p.hprev && active) {
+#pragma unroll
+        for (int q = 0; q < PW / 4; ++q)
+          if (4 * q < p.P) *reinterpret_cast<float4*>(p.hprev + so + 4 * q) = make_float4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
+      }
       ok = __all_sync(0xffffffffu, wait(SRDY + (i % NSB), (uint32_t)(i / NSB), 512u) && wait(UFULL, (uint32_t)i, 512u));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
