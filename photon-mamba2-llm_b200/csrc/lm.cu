@@ -280,7 +280,9 @@ struct pmb_lm {
   float* saved = nullptr;     // (L+1) x (M, D)
   float* dhidden = nullptr;   // (M, D)
   float* logits = nullptr;    // (tile_rows, Vp)
-  float* logits2 = nullptr;   // bf16 storage, long products: a second tile, so that dhidden of one runs under the next one's kernels
+  // bf16 storage, long products: a second tile, so that dhidden of one runs under the next one's kernels.  It lies in the blocks'
+  // workspace, which is idle between the two passes over the stack, or is an allocation of its own where that is too small.
+  float *logits2 = nullptr, *logits2_own = nullptr;
   float* row_loss = nullptr;  // (M)
   float* loss = nullptr;      // scalar
   unsigned int* bad = nullptr;
@@ -414,8 +416,13 @@ static pmb_status lm_create_impl(const pmb_mamba2_config* cfg, int L0, int L1, i
     lm->ce_inplace = ((size_t)vocab * 4 <= (size_t)CE_MAX_SMEM) ? 1 : 0;
     if (!lm->ce_inplace) ok = ok && alloc((void**)&lm->dlogits16, (size_t)lm->tile_rows * lm->Vp * 2);
     else if (d.M > lm->tile_rows && head_lane_clusters(lm->tile_rows, d.D, vocab)) {
-      ok = ok && alloc((void**)&lm->logits2, (size_t)lm->tile_rows * lm->Vp * 4);
-      pair_bytes += (size_t)lm->tile_rows * lm->Vp * 4;
+      const size_t bytes = (size_t)lm->tile_rows * lm->Vp * 4;
+      if (lm->ws_bytes >= bytes) lm->logits2 = static_cast<float*>(lm->ws);
+      else {
+        ok = ok && alloc((void**)&lm->logits2_own, bytes);
+        lm->logits2 = lm->logits2_own;
+        pair_bytes += bytes;
+      }
     }
   }
   if (L1 > 0) {
@@ -470,7 +477,7 @@ extern "C" void pmb_lm_destroy(pmb_lm* lm) {
   if (!lm) return;
   cudaFree(lm->params); cudaFree(lm->grads); cudaFree(lm->saved); cudaFree(lm->dhidden); cudaFree(lm->logits);
   cudaFree(lm->row_loss); cudaFree(lm->loss); cudaFree(lm->bad); cudaFree(lm->ids); cudaFree(lm->targets); cudaFree(lm->ws); cudaFree(lm->params16); cudaFree(lm->dlogits16);
-  cudaFree(lm->params_hi); cudaFree(lm->params_lo); cudaFree(lm->dlog_hi); cudaFree(lm->dlog_lo); cudaFree(lm->hid_hi); cudaFree(lm->hid_lo); cudaFree(lm->dh_part); cudaFree(lm->logits2);
+  cudaFree(lm->params_hi); cudaFree(lm->params_lo); cudaFree(lm->dlog_hi); cudaFree(lm->dlog_lo); cudaFree(lm->hid_hi); cudaFree(lm->hid_lo); cudaFree(lm->dh_part); cudaFree(lm->logits2_own);
   cudaFree(lm->gather); cudaFree(lm->l1_pair); cudaFree(lm->saved1); cudaFree(lm->pooled); cudaFree(lm->dpool); cudaFree(lm->dh1); cudaFree(lm->hsum);
   delete lm;
 }
@@ -492,7 +499,7 @@ extern "C" void pmb_lm_activation_detail(const pmb_lm* lm, int64_t* h_out3) {
   h_out3[0] = (int64_t)((size_t)lm->d.M * lm->d.D * esz * (lm->L0 + 1) + (lm->L1 > 0 ? (size_t)lm->d1.M * lm->d.D * esz * (lm->L1 + 1) : 0));                          // stored for backward: block inputs
   h_out3[1] = (int64_t)lm->ws_bytes;                                                              // transient: one block's workspace
   h_out3[2] = (int64_t)((size_t)lm->tile_rows * lm->Vp * (lm->ce_inplace ? 4 : (lm->bf16 ? 6 : (lm->pairs ? 8 : 4))) + (size_t)lm->d.M * lm->d.D * esz +
-                        (lm->logits2 ? (size_t)lm->tile_rows * lm->Vp * 4 : 0) +
+                        (lm->logits2_own ? (size_t)lm->tile_rows * lm->Vp * 4 : 0) +
                         (lm->pairs ? (size_t)lm->tile_rows * lm->d.D * 4 : 0));  // transient: logits tile (+ its gradient's pair), d(hidden)
 }
 extern "C" const float* pmb_lm_loss_device(const pmb_lm* lm) { return lm ? lm->loss : nullptr; }
