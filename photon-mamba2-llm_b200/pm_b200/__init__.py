@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes as C
 import pathlib
+import threading
 from dataclasses import dataclass
 
 import torch
@@ -520,7 +521,7 @@ class Mamba2Block:
         self._ws = None
         self._cfg = C.byref(config.c())
         self._params_c, self._params_key = None, None
-        self._step_ws = {}
+        self._step_ws = threading.local()
         self.refresh_weights()
 
     def refresh_weights(self):
@@ -590,16 +591,25 @@ class Mamba2Block:
         return {"ssm_state": torch.zeros(batch, cfg.n_heads, cfg.d_state, cfg.d_head, device=device),
                 "conv_window": torch.zeros(batch, cfg.xbc_dim, cfg.d_conv - 1, device=device)}
 
+    def _step_workspace(self, stream, batch, device):
+        """Scratch of one step, kept per (device, stream, batch): steps on several streams may overlap.  Each thread has its own: the
+        launches of two threads' steps on one stream may interleave.  A captured step takes memory of the capture's pool, which lives
+        as long as the graph: what is kept here goes when a ninth key comes, and a replay would write to memory of another tensor."""
+        if torch.cuda.is_current_stream_capturing():
+            return torch.empty(lib.pmb_mamba2_step_workspace_bytes(self._cfg, batch), device=device, dtype=torch.uint8)
+        kept = self._step_ws.__dict__
+        ws = kept.get((device, stream, batch))
+        if ws is None:
+            if len(kept) >= 8:
+                del kept[next(iter(kept))]
+            ws = kept[(device, stream, batch)] = torch.empty(lib.pmb_mamba2_step_workspace_bytes(self._cfg, batch), device=device, dtype=torch.uint8)
+        return ws
+
     def step(self, x_t, state):
         """`Mamba2Block::step`: x_t (B,1,D); the state dict is updated in place and returned."""
         B = x_t.shape[0]
         stream = _stream()
-        ws = self._step_ws.get((stream, B))          # one workspace per stream: steps on several streams may overlap
-        if ws is None:
-            n = lib.pmb_mamba2_step_workspace_bytes(self._cfg, B)
-            if len(self._step_ws) >= 8:
-                self._step_ws.clear()
-            ws = self._step_ws[(stream, B)] = torch.empty(n, device=x_t.device, dtype=torch.uint8)
+        ws = self._step_workspace(stream, B, x_t.device)
         y = torch.empty_like(x_t)
         _check(lib.pmb_mamba2_step(stream, self._cfg, self._params_struct(), B, _dev(x_t, "x_t").data_ptr(),
                                    state["ssm_state"].data_ptr(), state["conv_window"].data_ptr(), y.data_ptr(),

@@ -1,0 +1,101 @@
+"""What a block object keeps on the host between calls: the library is replaced by a recorder, no kernel is launched."""
+import threading
+
+import pytest
+import torch
+
+
+class Recorder:
+    """Stands in for the library: notes the workspace that each step was handed."""
+
+    def __init__(self):
+        self.steps = []
+        self.inside = threading.Barrier(1)
+
+    def pmb_mamba2_step_workspace_bytes(self, cfg, batch):
+        return 256 * batch
+
+    def pmb_mamba2_step(self, stream, cfg, params, batch, x, state, window, y, ws, n):
+        self.steps.append((threading.get_ident(), ws, n))
+        self.inside.wait(10)
+        return 0
+
+
+@pytest.fixture
+def pm(monkeypatch):
+    import __graft_entry__ as ge
+    ge.build()
+    import pm_b200
+    monkeypatch.setattr(pm_b200, "lib", Recorder())
+    monkeypatch.setattr(pm_b200, "_dev", lambda t, name: t)
+    monkeypatch.setattr(pm_b200, "_stream", lambda: 7)
+    pm_b200.capturing = False
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: pm_b200.capturing)
+    yield pm_b200
+    del pm_b200.capturing
+
+
+def make(pm):
+    cfg = pm.Mamba2Config(d_model=16, d_state=8, d_head=8, n_heads=2)
+    return pm.Mamba2Block(cfg, {k: torch.ones(s) for k, s in cfg.param_shapes().items()})
+
+
+def step(blk, batch=2, device="cpu"):
+    blk.step(torch.zeros(batch, 1, 16, device=device), blk.zero_state(batch, device))
+
+
+def test_captured_step_owns_its_workspace(pm):
+    blk = make(pm)
+    step(blk)                        # warm-up on the stream that captures
+    pm.capturing = True
+    held = []
+    empty = torch.empty
+    pm_ws = []
+
+    def keep(*a, **k):               # (what the capture's pool does: memory handed out inside it stays with the graph)
+        t = empty(*a, **k)
+        held.append(t)
+        pm_ws.append(t.data_ptr())
+        return t
+    torch.empty = keep
+    try:
+        step(blk)
+    finally:
+        torch.empty = empty
+        pm.capturing = False
+    captured = pm.lib.steps[-1][1]
+    assert captured in pm_ws
+    for batch in (2, *range(3, 14)):  # more keys than the object keeps, and the captured one's again
+        step(blk, batch)
+    step(blk)
+    assert captured not in [ws for _, ws, _ in pm.lib.steps[2:]] and pm.lib.steps[0][1] != captured
+    assert all(n == 256 * b for (_, _, n), b in zip(pm.lib.steps, (2, 2, 2, *range(3, 14), 2)))
+
+
+def test_kept_workspaces_are_reused_and_bounded(pm):
+    blk = make(pm)
+    for _ in range(2):
+        step(blk)
+    assert pm.lib.steps[0][1] == pm.lib.steps[1][1]
+    for batch in range(1, 40):
+        step(blk, batch)
+    assert len(blk._step_ws.__dict__) <= 8
+
+
+def test_threads_do_not_share_a_workspace(pm):
+    blk = make(pm)
+    pm.lib.inside = threading.Barrier(2)             # both calls are inside the library at the same time
+    threads = [threading.Thread(target=step, args=(blk,)) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    (a, wa, _), (b, wb, _) = pm.lib.steps
+    assert a != b and wa != wb
+
+
+def test_devices_do_not_share_a_workspace(pm):
+    blk = make(pm)
+    step(blk)
+    step(blk, device="meta")                         # (data_ptr() of a meta tensor is 0)
+    assert pm.lib.steps[0][1] != 0 and pm.lib.steps[1][1] == 0

@@ -111,6 +111,35 @@ def test_decode_batches(pm, B, D, H, P, N, G):
     assert pm.device_status() == 0
 
 
+# a captured step is replayed after the block has stepped at more batch sizes than it keeps workspaces for, and after memory has been
+# handed out again
+def test_captured_decode_outlives_other_batches(pm):
+    D, H, P, N, B = 64, 4, 32, 16, 3
+    cfg, p, blk = _block(pm, D, H, P, N, 1, 64, torch.float32)
+    start = {"ssm_state": randn((B, H, N, P), 7, 0.3).cuda(), "conv_window": randn((B, cfg.xbc_dim, 3), 8, 0.5).cuda()}
+    x, st = randn((B, 1, D), 20).cuda(), {k: v.clone() for k, v in start.items()}
+    want, _ = blk.step(x, {k: v.clone() for k, v in start.items()})
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        blk.step(x, {k: v.clone() for k, v in start.items()})              # warm-up on the stream that captures
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        y, _ = blk.step(x, st)
+    for stream in (side, torch.cuda.current_stream()):
+        with torch.cuda.stream(stream):
+            for batch in range(1, 12):
+                blk.step(randn((batch, 1, D), batch).cuda(), blk.zero_state(batch))
+            guards = [torch.full((64 * k,), 7, dtype=torch.uint8, device="cuda") for k in range(1, 200)]
+    torch.cuda.synchronize()
+    for k in st:
+        st[k].copy_(start[k])
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and pm.device_status() == 0
+    assert all(bool((g == 7).all()) for g in guards)
+
+
 # the bf16-input scan off the 128-token grid keeps everything but its outputs at fp32 precision: lengths around a step, segments,
 # narrow heads and states, one and two halves of d_state, tensors that start off a 16-byte boundary
 @pytest.mark.parametrize("B,T", [(1, 1), (2, 127), (1, 129), (3, 200), (1, 700)])
