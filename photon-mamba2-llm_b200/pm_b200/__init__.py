@@ -519,7 +519,7 @@ class Mamba2Block:
             raise PmbError(2, f"compute dtype {compute_dtype} is not supported")
         self.bf16 = compute_dtype == torch.bfloat16
         self._ws = None
-        self._cfg = C.byref(config.c())
+        self._cfg_c, self._cfg_key = None, None
         self._params_c, self._params_key = None, None
         self._step_ws = threading.local()
         self.refresh_weights()
@@ -529,6 +529,22 @@ class Mamba2Block:
         if self.bf16:
             self.w_in16 = to_bf16(self.params["in_proj_weight"])
             self.w_out16 = to_bf16(self.params["out_proj_weight"])
+
+    def __getstate__(self):
+        """A copy or a pickle leaves out what belongs to this object alone: the C views and the workspaces."""
+        return {**self.__dict__, "_ws": None, "_cfg_c": None, "_cfg_key": None, "_params_c": None, "_params_key": None, "_step_ws": None}
+
+    def __setstate__(self, state):
+        self.__dict__.update(state, _step_ws=threading.local())
+
+    def _config_struct(self):
+        """The C view of the configuration, rebuilt when one of its values was changed."""
+        c = self.config
+        key = (c.d_model, c.d_state, c.d_head, c.n_heads, c.n_groups, c.d_conv, c.block_len, c.rmsnorm_eps)
+        if key != self._cfg_key:
+            self._step_ws = threading.local()        # (the sizes of steps' workspaces follow from it)
+            self._cfg_c, self._cfg_key = c.c(), key
+        return C.byref(self._cfg_c)
 
     def _params_struct(self):
         """The C view of the parameters, rebuilt when one of the tensors was replaced."""
@@ -544,9 +560,9 @@ class Mamba2Block:
             raise PmbError(2, f"{name}: expected a contiguous {want} CUDA tensor, got {t.dtype}")
         return t
 
-    def _workspace(self, B, T, device):
+    def _workspace(self, cfg, B, T, device):
         fn = lib.pmb_mamba2_block_workspace_bytes_bf16 if self.bf16 else lib.pmb_mamba2_block_workspace_bytes
-        n = fn(self._cfg, B, T)
+        n = fn(cfg, B, T)
         if n == 0:
             raise PmbError(1, lib.pmb_last_error().decode())
         if self._ws is None or self._ws.numel() < n:
@@ -555,33 +571,35 @@ class Mamba2Block:
 
     def forward(self, x, residual=None):
         B, T, D = x.shape
-        ws = self._workspace(B, T, x.device)
+        cfg = self._config_struct()
+        ws = self._workspace(cfg, B, T, x.device)
         out = torch.empty_like(x)
         ps = self._params_struct()
         self._io(x, "x")
         if self.bf16:
-            _check(lib.pmb_mamba2_block_fwd_bf16(_stream(), self._cfg, ps, self.w_in16.data_ptr(),
+            _check(lib.pmb_mamba2_block_fwd_bf16(_stream(), cfg, ps, self.w_in16.data_ptr(),
                                                  self.w_out16.data_ptr(), B, T, x.data_ptr(), _ptr(residual), out.data_ptr(),
                                                  ws.data_ptr(), ws.numel()))
         else:
-            _check(lib.pmb_mamba2_block_fwd(_stream(), self._cfg, ps, B, T, x.data_ptr(),
+            _check(lib.pmb_mamba2_block_fwd(_stream(), cfg, ps, B, T, x.data_ptr(),
                                             _ptr(residual), out.data_ptr(), ws.data_ptr(), ws.numel()))
         return out
 
     def backward(self, x, dout, dx_accum=None):
         """Recomputes the block from `x` and returns (dx, {param gradients})."""
         B, T, D = x.shape
-        ws = self._workspace(B, T, x.device)
+        cfg = self._config_struct()
+        ws = self._workspace(cfg, B, T, x.device)
         dx = torch.empty_like(x)
         grads = {k: torch.empty_like(v) for k, v in self.params.items()}
         ps, gs = self._params_struct(), _params_struct(grads)
         self._io(x, "x"); self._io(dout, "dout")
         if self.bf16:
-            _check(lib.pmb_mamba2_block_bwd_bf16(_stream(), self._cfg, ps, self.w_in16.data_ptr(),
+            _check(lib.pmb_mamba2_block_bwd_bf16(_stream(), cfg, ps, self.w_in16.data_ptr(),
                                                  self.w_out16.data_ptr(), B, T, x.data_ptr(), dout.data_ptr(), _ptr(dx_accum),
                                                  dx.data_ptr(), C.byref(gs), ws.data_ptr(), ws.numel()))
         else:
-            _check(lib.pmb_mamba2_block_bwd(_stream(), self._cfg, ps, B, T, x.data_ptr(),
+            _check(lib.pmb_mamba2_block_bwd(_stream(), cfg, ps, B, T, x.data_ptr(),
                                             dout.data_ptr(), _ptr(dx_accum), dx.data_ptr(), C.byref(gs),
                                             ws.data_ptr(), ws.numel()))
         return dx, grads
@@ -591,27 +609,27 @@ class Mamba2Block:
         return {"ssm_state": torch.zeros(batch, cfg.n_heads, cfg.d_state, cfg.d_head, device=device),
                 "conv_window": torch.zeros(batch, cfg.xbc_dim, cfg.d_conv - 1, device=device)}
 
-    def _step_workspace(self, stream, batch, device):
+    def _step_workspace(self, cfg, stream, batch, device):
         """Scratch of one step, kept per (device, stream, batch): steps on several streams may overlap.  Each thread has its own: the
         launches of two threads' steps on one stream may interleave.  A captured step takes memory of the capture's pool, which lives
         as long as the graph: what is kept here goes when a ninth key comes, and a replay would write to memory of another tensor."""
         if torch.cuda.is_current_stream_capturing():
-            return torch.empty(lib.pmb_mamba2_step_workspace_bytes(self._cfg, batch), device=device, dtype=torch.uint8)
+            return torch.empty(lib.pmb_mamba2_step_workspace_bytes(cfg, batch), device=device, dtype=torch.uint8)
         kept = self._step_ws.__dict__
         ws = kept.get((device, stream, batch))
         if ws is None:
             if len(kept) >= 8:
                 del kept[next(iter(kept))]
-            ws = kept[(device, stream, batch)] = torch.empty(lib.pmb_mamba2_step_workspace_bytes(self._cfg, batch), device=device, dtype=torch.uint8)
+            ws = kept[(device, stream, batch)] = torch.empty(lib.pmb_mamba2_step_workspace_bytes(cfg, batch), device=device, dtype=torch.uint8)
         return ws
 
     def step(self, x_t, state):
         """`Mamba2Block::step`: x_t (B,1,D); the state dict is updated in place and returned."""
         B = x_t.shape[0]
-        stream = _stream()
-        ws = self._step_workspace(stream, B, x_t.device)
+        stream, cfg = _stream(), self._config_struct()
+        ws = self._step_workspace(cfg, stream, B, x_t.device)
         y = torch.empty_like(x_t)
-        _check(lib.pmb_mamba2_step(stream, self._cfg, self._params_struct(), B, _dev(x_t, "x_t").data_ptr(),
+        _check(lib.pmb_mamba2_step(stream, cfg, self._params_struct(), B, _dev(x_t, "x_t").data_ptr(),
                                    state["ssm_state"].data_ptr(), state["conv_window"].data_ptr(), y.data_ptr(),
                                    ws.data_ptr(), ws.numel()))
         return y, state

@@ -1,4 +1,6 @@
 """What a block object keeps on the host between calls: the library is replaced by a recorder, no kernel is launched."""
+import copy
+import pickle
 import threading
 
 import pytest
@@ -16,6 +18,7 @@ class Recorder:
         return 256 * batch
 
     def pmb_mamba2_step(self, stream, cfg, params, batch, x, state, window, y, ws, n):
+        self.config, self.params = cfg._obj, params._obj
         self.steps.append((threading.get_ident(), ws, n))
         self.inside.wait(10)
         return 0
@@ -99,3 +102,23 @@ def test_devices_do_not_share_a_workspace(pm):
     step(blk)
     step(blk, device="meta")                         # (data_ptr() of a meta tensor is 0)
     assert pm.lib.steps[0][1] != 0 and pm.lib.steps[1][1] == 0
+
+
+def test_block_can_be_copied_and_pickled(pm):
+    blk = make(pm)
+    step(blk)
+    for twin in (copy.deepcopy(blk), pickle.loads(pickle.dumps(blk)), copy.copy(blk)):
+        step(twin)
+        own = {k: getattr(pm.lib.params, k) for k in pm.PARAM_ORDER}
+        assert own == {k: v.data_ptr() for k, v in twin.params.items()}
+        assert pm.lib.steps[-1][1] != pm.lib.steps[0][1]             # workspaces stay with the object they came from
+        assert twin.config == blk.config and pm.lib.config.d_model == 16
+
+
+def test_edited_configuration_counts(pm):
+    blk = make(pm)
+    step(blk)
+    assert pm.lib.config.rmsnorm_eps == pytest.approx(1e-5)
+    blk.config.rmsnorm_eps = 1e-3
+    step(blk)
+    assert pm.lib.config.rmsnorm_eps == pytest.approx(1e-3)
