@@ -157,6 +157,8 @@ __global__ void __launch_bounds__(GV_THREADS) gemv_kernel(const GemvArgs a) {
 // in_proj, so that 268 MB of state at batch 256 stream with every load of a CTA in flight.  Writes g = (C h + D x) silu(z)
 // and the sum of g^2 over the head.
 constexpr int STEP_THREADS = 256;
+// floats that B and C take in front of the partial outputs, which are stored 16 bytes at a time
+__host__ __device__ constexpr int bc_floats(int N) { return (2 * N + 3) & ~3; }
 struct StateArgs {
   const float* act; const float* dt; const float* z; int64_t ldz; const float* a_log; const float* D;
   float* state; float* g; float* ss; int H, G, N, P, X, I;
@@ -166,7 +168,7 @@ __global__ void __launch_bounds__(STEP_THREADS) state_step_kernel(const StateArg
   extern __shared__ __align__(16) float sh[];             // B (N), C (N), partial outputs (rows x P)
   __shared__ float red[32];
   const int bh = blockIdx.x, h = bh % s.H, b = bh / s.H, g = h / (s.H / s.G);
-  float* Bs = sh; float* Cs = sh + s.N; float* part = sh + 2 * s.N;
+  float* Bs = sh; float* Cs = sh + s.N; float* part = sh + bc_floats(s.N);
   const int pw = s.P / 4, nsl = STEP_THREADS / pw, p4 = threadIdx.x % pw, sl = threadIdx.x / pw;
   float4* st = reinterpret_cast<float4*>(s.state + (int64_t)bh * s.N * s.P);
   float4 hv[ITER];
@@ -586,7 +588,7 @@ static pmb_status launch_state_step(cudaStream_t st, const Dims& d, const dec::S
   const bool vec4 = (d.P % 4 == 0) && (d.P / 4 <= dec::STEP_THREADS) && (dec::STEP_THREADS % (d.P / 4) == 0) && (d.X % 4 == 0) && (d.I % 4 == 0) &&
                     (reinterpret_cast<uintptr_t>(s.state) % 16 == 0);
   const int pw = vec4 ? d.P / 4 : (d.P < dec::STEP_THREADS ? d.P : dec::STEP_THREADS), nsl = dec::STEP_THREADS / pw;
-  const size_t shm = (size_t)(2 * d.N + nsl * d.P) * sizeof(float);
+  const size_t shm = (size_t)((vec4 ? dec::bc_floats(d.N) : 2 * d.N) + nsl * d.P) * sizeof(float);
   if (shm > 48 * 1024) return fail(PMB_ERR_SHAPE, "mamba2_step: d_state/d_head too large for the step kernel");
   const int iter = (int)cdiv(d.N, nsl);
   ProfScope prof(st, "decode_ssm_step", 0.0, 8.0 * d.B * d.H * d.N * d.P);

@@ -93,9 +93,9 @@ def test_block_bf16_weight_gradient_splits(pm, B, T):
 
 
 # batch sizes around the switch from streamed FMA to tensor-core projections and its tile widths; widths with ragged column
-# tiles; the last two are served by the general kernels
+# tiles; the last ones are served by the general kernels, or have an odd d_state per head under the vectorised state step
 @pytest.mark.parametrize("B", [1, 2, 3, 5, 9, 16, 17, 33, 70, 130, 300])
-@pytest.mark.parametrize("D,H,P,N,G", [(64, 4, 32, 16, 1), (72, 6, 24, 40, 6), (200, 8, 64, 128, 1), (36, 3, 5, 7, 1)])
+@pytest.mark.parametrize("D,H,P,N,G", [(64, 4, 32, 16, 1), (72, 6, 24, 40, 6), (200, 8, 64, 128, 1), (36, 3, 5, 7, 1), (64, 2, 8, 7, 2), (64, 4, 8, 5, 4)])
 def test_decode_batches(pm, B, D, H, P, N, G):
     cfg, p, blk = _block(pm, D, H, P, N, G, 64, torch.float32)
     st = blk.zero_state(B)
