@@ -143,14 +143,15 @@ inline pmb_status make_dims(const pmb_mamba2_config* c, int batch, int seqlen, D
 
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.0f / (1.0f + __expf(-x)); }
 // 1 / d for d >= 1: one Newton step with a fused residual on the hardware's approximation, which rounds to nearest there (Markstein,
-// IBM J. Res. Dev. 34(1), 1990).  Equal to 1.0f / d for every float from 1 to 8e37 (all of them compared on the GPU); 0 above, where
-// the quotient is below 1.3e-38.  No branch for special operands, so the reciprocals of neighbouring
-// elements overlap: the kernels that take several sigmoids per thread and row were bound by that chain.
+// IBM J. Res. Dev. 34(1), 1990).  Equal to 1.0f / d for every float from 1 to 8e37 (all of them were compared on the GPU once;
+// test_gpu_primitives.py compares four million); 0 above, where the quotient is below 1.3e-38; NaN for NaN.  No branch for special
+// operands, so the reciprocals of neighbouring elements overlap: the kernels that take several sigmoids per thread and row were
+// bound by that chain.
 __device__ __forceinline__ float rcp_ge1(float d) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
   r = fmaf(r, fmaf(-d, r, 1.0f), r);
-  return d < 8e37f ? r : 0.0f;
+  return d >= 8e37f ? 0.0f : r;
 }
 __device__ __forceinline__ float sigmoid_acc(float x) { return rcp_ge1(1.0f + expf(-x)); }
 // softplus in the reference's stable form max(x,0)+log(1+exp(-|x|)) (pm-candle ops_impl.rs:123-133)

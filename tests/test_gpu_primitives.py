@@ -32,6 +32,25 @@ def test_unary_and_binary(pm):
         pm.binary("add", x.cuda(), y[:, :10].contiguous().cuda())
 
 
+def test_sigmoid_of_special_values(pm):
+    x = torch.tensor([float("nan"), float("inf"), float("-inf"), -100.0, -89.0, 0.0, -0.0, 100.0])
+    got = pm.unary("sigmoid", x.cuda()).cpu()
+    assert torch.isnan(got[0])
+    assert torch.equal(got[1:], torch.tensor([1.0, 0.0, 0.0, 0.0, 0.5, 0.5, 1.0]))
+    assert torch.isnan(pm.unary("silu", x[:1].cuda())).all()
+
+
+def test_sigmoid_reciprocal_equals_the_division(pm):
+    """The reciprocal of 1 + exp(-x), which the kernels take without a division, against the division on the same denominators:
+    four million of them from 1 + 6e-8 to 8e37, in every binade, bit by bit."""
+    g = torch.Generator().manual_seed(11)
+    x = torch.cat([torch.rand(1 << 21, generator=g) * 105.0 - 87.2, torch.rand(1 << 21, generator=g) * 24.0 - 8.0]).cuda()
+    d = pm.unary("add_scalar", pm.unary("exp", -x), 1.0)
+    keep = d < 8e37
+    assert int(keep.sum()) > x.numel() - 100 and float(d[keep].max()) > 5e37 and float(d.min()) < 1.0001
+    assert torch.equal(pm.unary("sigmoid", x)[keep], pm.binary("div", torch.ones_like(d), d)[keep])
+
+
 def test_views_as_strided_copies(pm):
     x = randn((4, 6, 10), 3)
     xc = x.cuda()
