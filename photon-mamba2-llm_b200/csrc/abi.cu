@@ -332,7 +332,7 @@ extern "C" pmb_status pmb_ssd_scan_fwd_bf16(void* stream, int32_t batch, int32_t
     Scan16Ws w16;
     if (ssd16_ws_layout(batch, seqlen, n_heads, d_head, d_state, n_groups, block_len, d_ws, ws_bytes, &w16) == 0)
       return fail(PMB_ERR_WORKSPACE, "ssd bf16 workspace too small");
-    if (w16.plain && (reinterpret_cast<uintptr_t>(d_x) | reinterpret_cast<uintptr_t>(d_b) | reinterpret_cast<uintptr_t>(d_c) | reinterpret_cast<uintptr_t>(d_y)) & 15)
+    if (w16.whole && (reinterpret_cast<uintptr_t>(d_x) | reinterpret_cast<uintptr_t>(d_b) | reinterpret_cast<uintptr_t>(d_c) | reinterpret_cast<uintptr_t>(d_y)) & 15)
       return fail(PMB_ERR_SHAPE, "ssd_scan_fwd_bf16: x, b, c and y must be 16-byte aligned");
     return ssd16_fwd(static_cast<cudaStream_t>(stream), batch, seqlen, n_heads, d_head, d_state, n_groups, d_x, d_a, d_b, d_c,
                      d_init_state, d_y, d_final_state, w16);
@@ -361,7 +361,7 @@ extern "C" pmb_status pmb_ssd_scan_bwd_bf16(void* stream, int32_t batch, int32_t
     Scan16Ws w16;
     if (ssd16_ws_layout(batch, seqlen, n_heads, d_head, d_state, n_groups, block_len, d_ws, ws_bytes, &w16) == 0)
       return fail(PMB_ERR_WORKSPACE, "ssd bf16 workspace too small");
-    if (w16.plain && (reinterpret_cast<uintptr_t>(d_dy) | reinterpret_cast<uintptr_t>(d_dx) | reinterpret_cast<uintptr_t>(d_db) | reinterpret_cast<uintptr_t>(d_dc)) & 15)
+    if (w16.whole && (reinterpret_cast<uintptr_t>(d_dy) | reinterpret_cast<uintptr_t>(d_dx) | reinterpret_cast<uintptr_t>(d_db) | reinterpret_cast<uintptr_t>(d_dc)) & 15)
       return fail(PMB_ERR_SHAPE, "ssd_scan_bwd_bf16: dy, dx, db and dc must be 16-byte aligned");
     return ssd16_bwd(static_cast<cudaStream_t>(stream), batch, seqlen, n_heads, d_head, d_state, n_groups, d_dy, d_dx, d_da, d_db, d_dc, w16);
   }

@@ -96,10 +96,11 @@ void ssd_ws_take(Arena& ar, int B, int T, int H, int P, int N, int G, int Q, Ssd
 // The scan on bf16 inputs as they are (bf16 tensor-core operands, fp32 recurrence; no fp32 staging copies): any length, d_head up to
 // 64 and d_state up to 128 in multiples of 8.
 struct Scan16Ws {
-  bool plain;                          // what is formed on the way is rounded to bf16 (whole chunks of 128 tokens at d_head 64)
+  bool whole;                          // whole chunks of 128 tokens at d_head 64: the callers' tensors are 16-byte aligned
+  bool plain;                          // what is formed on the way is rounded to bf16 (most of those shapes)
   float* S; uint16_t *x, *b, *c;       // kept for the backward
   uint16_t *hp_hi, *hp_lo, *dh_hi, *dh_lo;
-  uint16_t *t0, *t1, *g0, *g1;         // landing buffers for tensors that are not 16-byte aligned (not with `plain`)
+  uint16_t *t0, *t1, *g0, *g1;         // landing buffers for tensors that are not 16-byte aligned (not with `whole`)
   float *init, *last, *seg, *part;
 };
 bool ssd16_supported(int B, int T, int H, int P, int N, int G, int Q);

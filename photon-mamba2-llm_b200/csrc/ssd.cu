@@ -1403,15 +1403,26 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
 // ---------------------------------------------------------------------------------------------
 // The scan on bf16 inputs as they are (mamba2/block.rs:203-208: x, B, C in bf16, the recurrence in fp32).  x, B, C and dY go to
 // the tensor cores as plain bf16 operands, a, S, the states and every accumulator stay fp32, y and the gradients leave the kernels
-// as bf16.  On whole chunks of 128 tokens at d_head 64 the operands formed on the way (masked tiles, scaled x and dY, states) are
-// rounded to bf16 too; on every other shape they are (hi, lo) pairs, so that nothing but the outputs is rounded to bf16.
+// as bf16.  On whole chunks of 128 or 256 tokens at d_head 64 (ssd16_plain) the operands formed on the way (masked tiles, scaled x and
+// dY, states) are rounded to bf16 too; on every other shape they are (hi, lo) pairs, so that nothing but the outputs is rounded to bf16.
 // Measured, forward and backward: 16 x 8192 tokens, 32 heads of 128 x 64: 7.01 ms chunk by chunk (16 launches), 3.22 ms as chains (5);
 // 5 x 1474 tokens, 16 heads: 4443 us widened to fp32 for the FMA contractions, 234 us.
 // ---------------------------------------------------------------------------------------------
 
-// rounds what is formed on the way to bf16
-static bool ssd16_plain(int T, int P, int N, int Q) {
+// Whole chunks of 128 tokens at d_head 64: the callers' tensors must be 16-byte aligned.  (More than 64 chunks were never part of this:
+// such sequences keep pairs of what is formed on the way, and with them da at 1.5e-6 instead of 4e-4.)
+static bool ssd16_whole(int T, int P, int N, int Q) {
   return P == 64 && (N == 64 || N == 128) && Q % 128 == 0 && Q <= PREP_MAX_Q && T / Q <= SCAN_DOT_MAX_NC;
+}
+// Rounds what is formed on the way to bf16.  A state enters the products of every step of 128 tokens, not of every chunk, and each time
+// its rounding adds to da (fp32; everything else leaves as bf16 and does not notice): with k steps to a chunk the error is up to sqrt(k) of
+// what rounding once per chunk leaves, and a sequence of one chunk has no need of any.  Error of da against fp64, 8 heads of 64 x 64, rounded
+// once per chunk / once per step / on pairs: 256 tokens in one chunk 2.4e-6 / 2.3e-4 / 1.5e-6; two chunks of 256 2.6e-4 / 3.7e-4 /
+// 1.5e-6; four 3.2e-4 / 4.2e-4 / 1.5e-6, and 1.25 times as large on longer sequences; eight chunks of 512 2.4e-4 / 4.2e-4 / 1.5e-6.  Pairs take
+// 13 to 37 % longer (2 x 512 tokens, 8 heads of 64 x 64: 64 -> 72 us; 16 x 8192, 32 heads of 128 x 64: 3.15 -> 4.31 ms).  They serve
+// chunks of more than two steps and sequences of at most two chunks of two steps; the others stay within 1.4 of one rounding per chunk.
+static bool ssd16_plain(int T, int P, int N, int Q) {
+  return ssd16_whole(T, P, N, Q) && (Q == SCAN_STEP || (Q == 2 * SCAN_STEP && T / Q > 2));
 }
 bool ssd16_supported(int B, int T, int H, int P, int N, int G, int Q) {
   return ssd_chain_enabled() && ssd_chain_shape(P, N) && (int64_t)B * T < (1LL << 31) && (int64_t)B * cdiv(T, SCAN_STEP) < (1LL << 31);
@@ -1421,13 +1432,14 @@ size_t ssd16_ws_layout(int B, int T, int H, int P, int N, int G, int Q, void* ba
   Arena ar(base, bytes);
   Scan16Ws w{};
   const size_t hp = (size_t)B * T * H * P, gn = (size_t)B * T * G * N, np = (size_t)B * H * N * P, stn = np * cdiv(T, SCAN_STEP);
+  w.whole = ssd16_whole(T, P, N, Q);
   w.plain = ssd16_plain(T, P, N, Q);
   w.S = ar.take<float>((size_t)B * T * H);
   w.x = ar.take<uint16_t>(hp);
   w.b = ar.take<uint16_t>(gn); w.c = ar.take<uint16_t>(gn);
   w.hp_hi = ar.take<uint16_t>(stn); w.dh_hi = ar.take<uint16_t>(stn);
-  if (!w.plain) {
-    w.hp_lo = ar.take<uint16_t>(stn); w.dh_lo = ar.take<uint16_t>(stn);
+  if (!w.plain) { w.hp_lo = ar.take<uint16_t>(stn); w.dh_lo = ar.take<uint16_t>(stn); }
+  if (!w.whole) {
     w.t0 = ar.take<uint16_t>(hp); w.t1 = ar.take<uint16_t>(hp); w.g0 = ar.take<uint16_t>(gn); w.g1 = ar.take<uint16_t>(gn);
   }
   w.init = ar.take<float>(np); w.last = ar.take<float>(np);

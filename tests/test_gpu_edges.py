@@ -171,6 +171,26 @@ def test_scan_bf16_lengths(pm, B, T, P, N, G, off):
             assert_close(got, want, tol=tol, what=what)
 
 
+# chunks of several steps: a state is rounded to bf16 between the steps only where that leaves da (fp32) about as far off as one rounding
+# per chunk does; a single chunk, two chunks of two steps and chunks of more steps keep da and the state at fp32 precision
+@pytest.mark.parametrize("T,Q", [(256, 256), (512, 256), (384, 384), (768, 384), (1024, 512), (1024, 1024)])
+@pytest.mark.parametrize("N,G", [(64, 1), (128, 4)])
+def test_scan_bf16_chunks_of_several_steps(pm, T, Q, N, G):
+    B, H, P = 2, 4, 64
+    x, b, c, dy = randn((B, T, H, P), 1).bfloat16(), randn((B, T, G, N), 2).bfloat16(), randn((B, T, G, N), 3).bfloat16(), randn((B, T, H, P), 4).bfloat16()
+    a = -torch.nn.functional.softplus(randn((B, T, H), 5) - 2.0)
+    scan = pm.SsdScanBf16(x.cuda(), a.cuda(), b.cuda(), c.cuda(), Q)
+    y, last = scan.forward(want_final_state=True)
+    dx, da, db, dc = scan.backward(dy.cuda())
+    assert pm.device_status() == 0
+    leaves = [t.double().requires_grad_(True) for t in (x, a, b, c)]
+    ref, last_ref = orc.ssd_scan_chunked(leaves[0], leaves[1], *(t.expand(B, T, H, N) for t in leaves[2:]), Q, return_final_state=True)
+    ref.backward(dy.double())
+    for got, want, tol, what in ((y.float(), ref, 5e-3, "y"), (last, last_ref, 1e-4, "final state"), (dx.float(), leaves[0].grad, 5e-3, "dx"),
+                                 (da, leaves[1].grad, 1e-4, "da"), (db.float(), leaves[2].grad, 5e-3, "db"), (dc.float(), leaves[3].grad, 5e-3, "dc")):
+        assert_close(got, want, tol=tol, what=what)
+
+
 # the CTA-pair GEMM's ways of storing a result: ragged edges (odd widths, rows past the last whole tile), fp32 and bf16, a residual
 # loaded ahead, a result added onto C, and the two tile widths (few tiles with a long K take the narrow one on pairs)
 @pytest.mark.parametrize("M,N,K", [(2048, 768, 1536), (1100, 1411, 200), (300, 4616, 72)])
