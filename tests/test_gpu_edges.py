@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from oracle import mamba2_oracle as orc
-from util import assert_close, randn, tol_for
+from util import FP32_TOL, assert_close, randn, tol_for
 
 pytestmark = pytest.mark.gpu
 
@@ -56,12 +56,13 @@ def test_block_forward_lengths(pm, B, T, P, N, G):
     assert_close(out, orc.block_forward(p, cfg, x), what=f"B={B} T={T} P={P} N={N} G={G}")
 
 
-# the same for the backward, with sequences long enough to be walked in segments
+# the same for the backward, with sequences long enough to be walked in segments (eight heads: in_proj's width is a multiple of 8 and
+# the chain kernels serve the backward; four: the FMA contractions)
 @pytest.mark.parametrize("B,T", [(1, 1), (2, 17), (1, 127), (2, 128), (3, 129), (1, 256), (1, 640), (2, 1024)])
-@pytest.mark.parametrize("P,N,G", [(64, 64, 1), (32, 16, 1), (64, 64, 4), (64, 24, 1)])
-def test_block_backward_lengths(pm, B, T, P, N, G):
-    D, H = 64, 4
-    cfg, p, blk = _block(pm, D, H, P, N, G, 128 if P == 64 else 64, torch.float32)
+@pytest.mark.parametrize("P,N,G,H", [(64, 64, 1, 4), (64, 64, 1, 8), (32, 16, 1, 4), (32, 16, 1, 8), (64, 64, 4, 4), (64, 64, 8, 8), (64, 24, 1, 4), (64, 24, 1, 8), (48, 40, 1, 8)])
+def test_block_backward_lengths(pm, B, T, P, N, G, H):
+    D, Q = 64, 128 if P == 64 else 64
+    cfg, p, blk = _block(pm, D, H, P, N, G, Q, torch.float32)
     x, cot = randn((B, T, D), 5), randn((B, T, D), 6)
     dx, grads = blk.backward(x.cuda(), cot.cuda())
     torch.cuda.synchronize()
@@ -69,10 +70,12 @@ def test_block_backward_lengths(pm, B, T, P, N, G):
     leaves = {k: v.clone().requires_grad_(True) for k, v in p.items()}
     xr = x.clone().requires_grad_(True)
     orc.block_forward(leaves, cfg, xr).backward(cot)
+    chunk = Q if T % Q == 0 else T
+    chain = H == 8 and (chunk <= (256 if P == 64 else 64) or (P == N == 64 and chunk % 128 == 0))
     assert_close(dx, xr.grad, what="dx")
     for k, g in grads.items():
         if T > 1 or k != "a_log":      # (one token: d(a_log) is exactly zero)
-            assert_close(g, leaves[k].grad, tol=tol_for(k), what=k)
+            assert_close(g, leaves[k].grad, tol=FP32_TOL if chain else tol_for(k), what=k)
 
 
 # token counts at which the weight gradients of the bf16-storage block split K or not, with and without whole tiles

@@ -15,9 +15,10 @@ FP32_TOL = 1e-4
 
 
 # The gradients of a_log and dt_bias are sums over all tokens of S-weighted differences of nearly equal terms (row
-# sums minus column sums of dM o M).  On the shapes the fused tensor-core scan takes (block_len % 128 == 0, d_state =
-# d_head = 64) both sums come from the same registers (csrc/ssd_fused.cu) and the two tensors get the bar of every
-# other tensor (`fused=True`).  The fp32 FMA engine that serves the remaining (small or ragged) shapes forms the
+# sums minus column sums of dM o M).  The tensor-core scans take both sums from the same registers (csrc/ssd_chain_bwd.cu,
+# which serves fp32 blocks whose widths are multiples of 8 with chunks of up to 256 tokens, or 64 with heads narrower than 64;
+# csrc/ssd_fused.cu, which serves the scan operator at block_len % 128 == 0, d_state = d_head = 64), and there the two tensors get
+# the bar of every other tensor (`fused=True`).  The fp32 FMA engine that serves the remaining shapes forms the
 # difference from y and dx~ instead and is held to 5e-4 there (the reference's own cross-backend SSD gradient tests
 # use 1e-3, crates/pm-cuda/tests/grad_ssd.rs:62-227).
 CANCELLATION_TOL = 5e-4
