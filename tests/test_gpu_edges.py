@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from oracle import mamba2_oracle as orc
-from util import FP32_TOL, assert_close, randn, tol_for
+from util import FP32_TOL, assert_close, block_params, cuda_params, randn, tol_for
 
 pytestmark = pytest.mark.gpu
 
@@ -192,6 +192,47 @@ def test_scan_bf16_chunks_of_several_steps(pm, T, Q, N, G):
     for got, want, tol, what in ((y.float(), ref, 5e-3, "y"), (last, last_ref, 1e-4, "final state"), (dx.float(), leaves[0].grad, 5e-3, "dx"),
                                  (da, leaves[1].grad, 1e-4, "da"), (db.float(), leaves[2].grad, 5e-3, "db"), (dc.float(), leaves[3].grad, 5e-3, "dc")):
         assert_close(got, want, tol=tol, what=what)
+
+
+# bf16 storage with a long vocabulary: the gradient of a row tile's hidden rows runs on a stream of its own under the next tile, and the
+# tiles alternate between two buffers.  Four whole tiles and a remainder; the second buffer in the blocks' workspace, or (small blocks) of
+# its own.  Everything on one stream, eagerly and as a graph replay, is the same sums in the same order.
+@pytest.mark.parametrize("D,H,P,N,Q,own", [(64, 8, 8, 8, 32, True), (256, 8, 64, 64, 128, False)])
+def test_lm_head_lane(pm, D, H, P, N, Q, own):
+    B, T, V = 9, 512, 8200
+    cfg = orc.Mamba2Config(d_model=D, d_state=N, d_head=P, n_heads=H, n_groups=1, d_conv=4, block_len=Q)
+    p, embed = block_params(cfg, seed=61), randn((V, D), 13, 0.3)
+    lm = pm.FlatMamba(pm.Mamba2Config(d_model=D, d_state=N, d_head=P, n_heads=H, n_groups=1, d_conv=4, block_len=Q), 1, V, B, T, compute_dtype=torch.bfloat16)
+    lm.load(embed.cuda(), [cuda_params(p)])
+    tile = 1024 * V * 4
+    assert (lm.activation_detail["lm_head_transient"] >= 2 * tile) == own and (lm.activation_detail["block_workspace"] >= tile) == (not own)
+    graph = lm.capture_step()
+    n_embed = V * D
+    for seed in range(3):
+        ids, tg, _ = orc.lcg_batch(17 + seed, B, T, V)
+        pm.set_concurrency(False)
+        try:
+            loss = lm.step_device(ids.cuda(), tg.cuda()).clone()
+        finally:
+            pm.set_concurrency(True)
+        want = lm.flat_grads.clone()
+        if seed == 0:
+            er, leaves = embed.clone().requires_grad_(True), {k: v.clone().requires_grad_(True) for k, v in p.items()}
+            ref = orc.lm_loss(er, [leaves], cfg, ids, tg)
+            ref.backward()
+            assert abs(float(loss) - float(ref)) < 2e-2 * float(ref)
+            ge, gl = lm.grads()
+            assert_close(ge, er.grad, tol=2e-2, what="embed")
+            for k in ("in_proj_weight", "out_proj_weight", "norm_weight"):
+                assert_close(gl[0][k], leaves[k].grad, tol=2e-2, what=k)
+        for run in (lm.step_device, lm.step_device, graph, graph):
+            lm.flat_grads.zero_()
+            assert torch.equal(run(ids.cuda(), tg.cuda()).reshape(-1), loss.reshape(-1))
+            assert torch.equal(lm.flat_grads[n_embed:], want[n_embed:])
+            assert_close(lm.flat_grads[:n_embed], want[:n_embed], tol=1e-6, what="embed")      # (its token rows are added atomically)
+    assert pm.device_status() == 0
+    del graph
+    lm.close()
 
 
 # the CTA-pair GEMM's ways of storing a result: ragged edges (odd widths, rows past the last whole tile), fp32 and bf16, a residual
