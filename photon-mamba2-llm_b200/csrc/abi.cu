@@ -2,6 +2,8 @@
 #include <cstdio>
 #include <cstdlib>
 #include <initializer_list>
+#include <map>
+#include <mutex>
 #include "common.cuh"
 #include "kernels.h"
 #include "ssd_tc.h"
@@ -42,8 +44,18 @@ pmb_status gemm(cudaStream_t st, int ta, int tb, int64_t M, int64_t N, int64_t K
   return gemm_simt(st, ta, tb, M, N, K, A, lda, B, ldb, C, ldc, R);
 }
 
-static SideLane g_lanes[64][7];
+static cudaStream_t g_lane_streams[64][7];
+static std::mutex g_lane_mu;
 static int g_lanes_enabled = 1;   // pmb_set_concurrency(0): every caller gets no lane and runs its chains on the one stream
+
+// The streams are shared by all threads, the events belong to one: between a thread's record of an event and its wait for it another
+// thread, on another stream of its caller's, would record the same event, and the first one's lane would start too early.  (Work that
+// shares a lane's stream is in that stream's order, which is at most more order than was asked for.)
+struct ThreadLanes {
+  std::map<int, SideLane> lanes;  // [device * 7 + lane]
+  ~ThreadLanes() { for (auto& l : lanes) for (cudaEvent_t e : l.second.ev) if (e) cudaEventDestroy(e); }
+};
+static thread_local ThreadLanes t_lanes;
 
 pmb_status get_side_lane(int idx, SideLane** out) {
   *out = nullptr;
@@ -51,15 +63,20 @@ pmb_status get_side_lane(int idx, SideLane** out) {
   int dev = 0;
   PMB_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64 || idx < 0 || idx >= 7) return PMB_OK;
-  SideLane& l = g_lanes[dev][idx];
+  SideLane& l = t_lanes.lanes[dev * 7 + idx];
   if (!l.s) {
-    // lanes that carry the critical chain of the stack backward (6: gradient kernels of the current block, 0: the
-    // scan backward's second chain, 5: its dB branch) get the highest stream priority, so that their CTAs are placed ahead of the
-    // recompute-ahead and the deferred GEMMs whenever an SM frees up
-    int least = 0, greatest = 0;
-    PMB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    PMB_CUDA(cudaStreamCreateWithPriority(&l.s, cudaStreamNonBlocking, (idx == 0 || idx == 5 || idx == 6) ? greatest : least));
-    for (int i = 0; i < 6; ++i) PMB_CUDA(cudaEventCreateWithFlags(&l.ev[i], cudaEventDisableTiming));
+    std::lock_guard<std::mutex> lock(g_lane_mu);
+    cudaStream_t& s = g_lane_streams[dev][idx];
+    if (!s) {
+      // lanes that carry the critical chain of the stack backward (6: gradient kernels of the current block, 0: the
+      // scan backward's second chain, 5: its dB branch) get the highest stream priority, so that their CTAs are placed ahead of the
+      // recompute-ahead and the deferred GEMMs whenever an SM frees up
+      int least = 0, greatest = 0;
+      PMB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+      PMB_CUDA(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, (idx == 0 || idx == 5 || idx == 6) ? greatest : least));
+    }
+    for (cudaEvent_t& e : l.ev) if (!e) PMB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    l.s = s;
   }
   *out = &l;
   return PMB_OK;

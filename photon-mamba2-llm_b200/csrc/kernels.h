@@ -4,8 +4,8 @@
 
 namespace pmb {
 
-// ---- abi.cu: side streams for kernels that do not depend on each other.  One stream and six events per (device,
-// lane index), created on first use (so the first call should come before any stream capture).  lane 0: scan
+// ---- abi.cu: side streams for kernels that do not depend on each other.  One stream per (device, lane index) and six events per
+// thread of it, created on first use (so a thread's first call should come before any stream capture).  lane 0: scan
 // backward chains; 1: gradient GEMMs of a block that are off the critical path; 2: scan forward; 3: recompute-ahead;
 // 4: embedding-table gradient (fp32) or gradient of the hidden rows (bf16) of the LM head; 5: unused; 6: the gradient kernels of the stack backward (high priority,
 // like lane 0).  *out stays NULL past device 63.

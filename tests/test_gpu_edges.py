@@ -1,5 +1,7 @@
 """GPU tests of the kernel variants at the sizes where their tiling or dispatch changes: edges of tiles, remainders,
 the smallest and largest sizes of a rule.  Oracle or plain fp32 / fp64 torch as the reference."""
+import threading
+
 import pytest
 import torch
 
@@ -233,6 +235,34 @@ def test_lm_head_lane(pm, D, H, P, N, Q, own):
     assert pm.device_status() == 0
     del graph
     lm.close()
+
+
+# two threads with a block and a stream each share the library's internal streams, not the events that order them
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_blocks_on_two_threads(pm, dtype):
+    work = []
+    for k, (B, T) in enumerate([(2, 512), (1, 700)]):
+        cfg, p, blk = _block(pm, 128, 8, 64, 64, 1, 128, dtype, seed=3 + k)
+        x, cot = (randn((B, T, 128), s + k).cuda().to(dtype) for s in (5, 15))
+        dx, grads = blk.backward(x, cot)
+        work.append((blk, x, cot, dx, grads))
+    torch.cuda.synchronize()
+    off = [[], []]
+
+    def run(k):
+        blk, x, cot, dx, grads = work[k]
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(40):
+                got, g = blk.backward(x, cot)
+                off[k].append((got != dx).any() | torch.stack([(g[n] != grads[n]).any() for n in g]).any())
+            torch.cuda.current_stream().synchronize()
+    threads = [threading.Thread(target=run, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert [len(o) for o in off] == [40, 40] and not any(bool(o) for k in off for o in k)
+    assert pm.device_status() == 0
 
 
 # the CTA-pair GEMM's ways of storing a result: ragged edges (odd widths, rows past the last whole tile), fp32 and bf16, a residual
