@@ -564,15 +564,13 @@ namespace pmb { namespace hb { pmb_status pair_operand_map(CUtensorMap* map, con
 
 template <int NB>
 static pmb_status skinny_nb(cudaStream_t st, const uint16_t* hi, const uint16_t* lo, int64_t B, int64_t K, int64_t J, const float* W, float* slab, int splits) {
-  static unsigned int* status[PMB_MAX_DEVICES] = {nullptr};
-  int dev = 0;
-  PMB_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= PMB_MAX_DEVICES) dev = 0;
-  if (!status[dev]) PMB_CUDA(cudaGetSymbolAddress((void**)&status[dev], g_decode_status));
+  static unsigned int* known[PMB_MAX_DEVICES] = {nullptr};
+  unsigned int* status = tcx::status_address(g_decode_status, known);
+  if (!status) return fail(PMB_ERR_CUDA, "decode: no status word on this device");
   dec::SkMaps ms{};
   PMB_TRY(hb::pair_operand_map(&ms.x[0], hi, K, B, K, dec::SK_BK, NB));
   PMB_TRY(hb::pair_operand_map(&ms.x[1], lo, K, B, K, dec::SK_BK, NB));
-  dec::SkArgs a{W, J, (int)K, (int)J, (int)B, (int)cdiv(cdiv(K, dec::SK_BK), splits), slab, status[dev]};
+  dec::SkArgs a{W, J, (int)K, (int)J, (int)B, (int)cdiv(cdiv(K, dec::SK_BK), splits), slab, status};
   PMB_SMEM_OPT_IN(dec::SkGeo<NB>::SMEM, dec::skinny_gemm_kernel<NB>);
   ProfScope prof(st, "decode_gemm", 2.0 * B * K * J, 4.0 * ((double)K * J + (double)splits * B * J));
   return launch_pdl(st, dec::skinny_gemm_kernel<NB>, dim3((unsigned)cdiv(J, 128), (unsigned)splits, (unsigned)cdiv(B, NB)), dec::SK_THREADS, dec::SkGeo<NB>::SMEM, ms, a);

@@ -88,12 +88,8 @@ pmb_status get_map(CUtensorMap* out, const float* base, int64_t d0, int64_t d1, 
 }
 
 unsigned int* status_ptr() {
-  static unsigned int* ptr[64] = {nullptr};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  if (!ptr[dev]) cudaGetSymbolAddress((void**)&ptr[dev], g_small_status);
-  return ptr[dev];
+  static unsigned int* known[PMB_MAX_DEVICES] = {nullptr};
+  return tcx::status_address(g_small_status, known);
 }
 
 }  // namespace

@@ -45,8 +45,6 @@ using namespace tcx;
 constexpr int L = SCAN_STEP, PW = 64, T128 = L * 128, T64 = 64 * 128;
 constexpr int W_MASK = 4, W_XF = 12, W_ST = 20, NTHREADS = 32 * 24, XF_THREADS = 256;
 // (shares of the block's 80 x 768 registers: 72, 2 x 80, 2 x 72 and 104 per thread of the six warpgroups)
-template <int R> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
-template <int R> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
 
 template <int NI, int ND, int NK>
 struct Geo {
@@ -84,33 +82,8 @@ struct Params {
   unsigned int* status;
 };
 
-__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo, bool want_lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  if (want_lo) {
-    const float2 hf = __bfloat1622float2(h);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(a - hf.x, b - hf.y);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
-  }
-}
-__device__ __forceinline__ void st_shared_v2(uint32_t a, uint32_t x, uint32_t y) {
-  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(a), "r"(x), "r"(y) : "memory");
-}
-__device__ __forceinline__ void st_shared_v4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
-  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
-}
 __device__ __forceinline__ uint32_t ld_shared(uint32_t a) { uint32_t v; asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
 __device__ __forceinline__ float2 bf2(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
-      : "memory");
-}
-__device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {
-  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(src) : "memory");
-}
 
 // On entry every lane holds its row's values for 16 consecutive columns; on exit lane l holds the sum of column l & 15 over the
 // warp's 32 rows.  Fixed order.
@@ -728,12 +701,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
 
 // ---- host side -------------------------------------------------------------------------------------------
 static unsigned int* status_ptr() {
-  static unsigned int* ptr[PMB_MAX_DEVICES] = {nullptr};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= PMB_MAX_DEVICES) dev = 0;
-  if (!ptr[dev]) cudaGetSymbolAddress((void**)&ptr[dev], g_chain_bwd_status);
-  return ptr[dev];
+  static unsigned int* known[PMB_MAX_DEVICES] = {nullptr};
+  return status_address(g_chain_bwd_status, known);
 }
 
 template <int NI, int ND, int NK, bool IN16>

@@ -119,17 +119,6 @@ __device__ __forceinline__ float warp_column_sums(float (&v)[32], int lane) {
   return v[0];
 }
 
-// two fp32 values -> packed bf16x2 of their high parts (round to nearest even) and of the remainders
-__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo, bool want_lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  if (want_lo) {
-    const float2 hf = __bfloat1622float2(h);
-    const __nv_bfloat162 l = __floats2bfloat162_rn(a - hf.x, b - hf.y);
-    lo = *reinterpret_cast<const uint32_t*>(&l);
-  }
-}
-
 template <int MODE, int NS, int NK, int PB>
 __global__ void __launch_bounds__(NTHREADS, (Geo<MODE, NS, NK, PB>::CTAS))
 ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
@@ -588,12 +577,8 @@ pmb_status bf16_map4(CUtensorMap* out, const uint16_t* base, int64_t d0, int64_t
 }
 
 static unsigned int* status_ptr() {
-  static unsigned int* ptr[PMB_MAX_DEVICES] = {nullptr};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= PMB_MAX_DEVICES) dev = 0;
-  if (!ptr[dev]) cudaGetSymbolAddress((void**)&ptr[dev], g_fused_status);
-  return ptr[dev];
+  static unsigned int* known[PMB_MAX_DEVICES] = {nullptr};
+  return status_address(g_fused_status, known);
 }
 
 template <int MODE, int NS, int NK, int PB>

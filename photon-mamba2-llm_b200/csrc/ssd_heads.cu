@@ -61,12 +61,6 @@ struct Params {
   unsigned int* status;
 };
 
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
-      : "memory");
-}
 __device__ __forceinline__ uint32_t pack2(float a, float b) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&v);
@@ -367,12 +361,8 @@ __global__ void __launch_bounds__(256) heads_sum_kernel(const float* __restrict_
 }
 
 static unsigned int* status_ptr() {
-  static unsigned int* ptr[PMB_MAX_DEVICES] = {nullptr};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= PMB_MAX_DEVICES) dev = 0;
-  if (!ptr[dev]) cudaGetSymbolAddress((void**)&ptr[dev], g_heads_status);
-  return ptr[dev];
+  static unsigned int* known[PMB_MAX_DEVICES] = {nullptr};
+  return status_address(g_heads_status, known);
 }
 
 template <int NI, int ND>

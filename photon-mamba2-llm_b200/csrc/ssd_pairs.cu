@@ -188,12 +188,8 @@ template <class Op>
 Op mk(const PP& p, int Mdim, int Ndim) { Op op{}; op.p = p; op.Mdim = Mdim; op.Ndim = Ndim; return op; }
 
 unsigned int* status_ptr() {
-  static unsigned int* ptr[PMB_MAX_DEVICES] = {nullptr};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= PMB_MAX_DEVICES) dev = 0;
-  if (!ptr[dev]) cudaGetSymbolAddress((void**)&ptr[dev], g_pairs_status);
-  return ptr[dev];
+  static unsigned int* known[PMB_MAX_DEVICES] = {nullptr};
+  return tcx::status_address(g_pairs_status, known);
 }
 
 // logical map i of the set <- the (hi, lo) arrays of one operand

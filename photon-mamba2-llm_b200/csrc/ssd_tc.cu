@@ -404,12 +404,8 @@ Op mk(const TcP& p, int Mdim, int Ndim) { Op op{}; op.p = p; op.Mdim = Mdim; op.
 
 // device address of this device's status word (looked up once per device)
 unsigned int* status_ptr() {
-  static unsigned int* ptr[64] = {nullptr};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  if (!ptr[dev]) cudaGetSymbolAddress((void**)&ptr[dev], g_ssd_tc_status);
-  return ptr[dev];
+  static unsigned int* known[PMB_MAX_DEVICES] = {nullptr};
+  return tcx::status_address(g_ssd_tc_status, known);
 }
 
 }  // namespace
