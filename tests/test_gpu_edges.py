@@ -1,5 +1,8 @@
 """GPU tests of the kernel variants at the sizes where their tiling or dispatch changes: edges of tiles, remainders,
 the smallest and largest sizes of a rule.  Oracle or plain fp32 / fp64 torch as the reference."""
+import pathlib
+import subprocess
+import sys
 import threading
 
 import pytest
@@ -263,6 +266,35 @@ def test_blocks_on_two_threads(pm, dtype):
         t.join()
     assert [len(o) for o in off] == [40, 40] and not any(bool(o) for k in off for o in k)
     assert pm.device_status() == 0
+
+
+FIRST_CALLS = """
+import threading, torch, pm_b200 as pm
+cfg = pm.Mamba2Config(d_model=64, d_state=64, d_head=64, n_heads=8, block_len=128)
+g = torch.Generator().manual_seed(1)
+params = {k: (0.1 * torch.randn(s, generator=g)).cuda() for k, s in cfg.param_shapes().items()}
+x = torch.randn(2, 256, 64, generator=g).cuda()
+torch.cuda.synchronize()
+start, got = threading.Barrier(6), [None] * 6
+def first(k):
+    blk = pm.Mamba2Block(cfg, params)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        start.wait()
+        got[k] = (blk.forward(x), *blk.backward(x, x)[1].values())
+        torch.cuda.current_stream().synchronize()
+threads = [threading.Thread(target=first, args=(k,)) for k in range(6)]
+[t.start() for t in threads]; [t.join() for t in threads]
+assert all(g is not None and all(torch.equal(a, b) for a, b in zip(g, got[0])) for g in got), got
+assert pm.device_status() == 0
+print("same")
+"""
+
+
+# what the library sets up on first use (the driver's entry point, internal streams, kernel attributes, tensor maps), asked for by six
+# threads at the same time in a process of its own
+def test_first_calls_on_several_threads(pm):
+    r = subprocess.run([sys.executable, "-c", FIRST_CALLS], cwd=pathlib.Path(pm.__file__).parent.parent, capture_output=True, text=True, timeout=200)
+    assert r.returncode == 0 and r.stdout.strip() == "same", r.stderr[-2000:]
 
 
 # the CTA-pair GEMM's ways of storing a result: ragged edges (odd widths, rows past the last whole tile), fp32 and bf16, a residual
