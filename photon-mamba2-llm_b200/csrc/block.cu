@@ -88,10 +88,12 @@ static size_t slab_floats(const Dims& d) {
 // The scan of a block that has a backward runs as ssd_chain.cu / ssd_chain_bwd.cu / ssd_heads.cu on (hi, lo) pairs: every
 // sequence length, d_state and d_head up to 64.  (bf16 blocks whose operands are plain bf16, and d_state 128, keep the kernels
 // that work chunk by chunk.)
-// Long chunks off the 128-token grid (a sequence that no chunk divides is one chunk) in fp32 outside of a model keep the FMA
-// contractions: those form d(a_log) and d(dt_bias) as <dY, y> - <x~, dx~>, whose rounding grows with the chunk (5e-4 of the
-// gradient's norm against fp64 at 3 x 700 tokens, where the sums of the chain kernel are off by 2e-5); from 256 tokens on (64 with
-// heads narrower than 64) the two forms are further apart than fp32 results of one call may move.
+// Chunks (a sequence that no chunk divides is one) of more than 256 tokens, or 64 with heads narrower than 64, other than multiples of
+// 128 at 64 x 64, keep the FMA contractions in fp32 outside of a model.  Theirs is not the better result: they form d(a_log) and d(dt_bias) as
+// <dY, y> - <x~, dx~>, whose rounding grows with the chunk (from fp64, relative to the gradient's norm: 1e-4 at 200 tokens, 2e-4 to 8e-4 at
+// 1000 to 1337; the sums of the chain kernel 1e-5 to 2.5e-5; all other gradients are equally far off), nor the faster one (forward and backward
+// of 2 x 1337 tokens, 24 heads of 64 x 64: 2395 us, 519 as chains; a stack of five on 2 x 740: 7.2 ms, 1.9).  They stay because those two
+// gradients of a call would move by that much, more than fp32 results are expected to between two builds (2e-4).
 static bool block_uses_chain_bwd(const Dims& d, bool bf16, bool in_model) {
   const bool dims = bf16 ? !ssd_plain16_shape(d.P, d.N, d.Q) && d.D % 8 == 0 && d.J % 8 == 0 && d.I % 8 == 0 : block_uses_pairs(d);
   const bool close = bf16 || in_model || ssd_fused_supported(d.P, d.N, d.Q) || d.Q <= (d.P >= 64 ? 256 : 64);
@@ -301,7 +303,7 @@ pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, 
   BlockWs w{};
   Pair16 wout{nullptr, nullptr, 0};
   const bool plain = block_plain16(d, w16 != nullptr), by_chunks = scan_by_chunks(d, w16 != nullptr, false);
-  // (the backward of a stack whose blocks keep the FMA contractions amplifies any difference between the forward's scan and its own)
+  // (a stack whose blocks keep the FMA contractions scans with them in the forward too: its gradients are those of the forward that it ran)
   const bool as_backward = backward_follows && !w16 && !block_uses_chain_bwd(d, false, wx && wx->pairs);
   if (ssd_chain_enabled() && ssd_chain_shape(d.P, d.N) && !by_chunks && !as_backward) {
     // nothing is kept for a backward: the scan is one kernel that takes dt_raw, x and the B | C pair as the conv left them

@@ -1,7 +1,7 @@
 // One-token recurrent decode (Mamba2Block::step, crates/pm-core/src/mamba2/block.rs:278-417):
 // rolling conv window + h <- exp(A dt) h + dt (B (x) x), y = C h + D x, gate, norm, out_proj.
 //
-// The weights (fp32) and the state are read once per token and that is the whole cost, so no pass copies them: up to 16
+// The weights (fp32) and the state are read once per token and that is most of the cost at both ends, so no pass copies them: up to 16
 // sequences the projections are FMA kernels that stream the weight rows (three launches: in_proj + conv step + dt, state
 // step + gate, norm + out_proj), beyond that a tensor-core kernel that turns each weight tile into a bf16 pair on its way
 // through shared memory.  The launches are chained with programmatic dependent launch: a kernel is placed while its predecessor
@@ -610,8 +610,10 @@ extern "C" pmb_status pmb_mamba2_step(void* stream, const pmb_mamba2_config* cfg
   const bool vec = d.J % 4 == 0 && d.D % 4 == 0 && d.I % 4 == 0 && al(p->in_proj_weight) && al(p->out_proj_weight);
   dec::StepIn si{d.B, d.D, d.I, d.X, d.J, d.H, d.G, d.N, d.P, d.K, p->conv1d_weight, p->conv1d_bias, p->dt_bias, d_conv_window, w.z, d.I, w.act, w.dt};
   const dec::StateArgs sa{w.act, w.dt, w.z, d.I, p->a_log, p->d_skip, d_ssm_state, w.g, w.ss, d.H, d.G, d.N, d.P, d.X, d.I};
-  // up to 16 sequences FMA on streamed weights is below the launch overhead of anything larger; beyond, its 64 FMA per
-  // weight and more would bound it
+  // Up to 16 sequences the products are fp32 FMA (y 2e-7 of its norm from fp64), beyond on bf16 pairs (7e-6).  Where the line
+  // lies is a matter of that precision, not of time.  us per step, FMA / tensor cores (24 heads of 64 x 64 at d_model 768; 32 of 64 x 128
+  // at d_model 2048): 1 sequence 14.2 / 19.0, 19.6 / 26.6; 2: 18.1 / 19.8, 26.6 / 28.3; 4: 22.5 / 20.3, 35.3 / 28.4; 8: 32.9 / 22.1, 50.0 / 29.0;
+  // 16: 55.3 / 22.6, 81.0 / 31.1; 17: 22.9 and 31.6.  (From five on the inputs' stores to shared memory go 8 or 16 ways to a bank.)
   if (vec && d.B <= 16 && gemv_smem(d.B, d.D) <= GEMV_MAX_SMEM && gemv_smem(d.B, d.I) <= GEMV_MAX_SMEM) {
     dec::GemvArgs a{};
     a.B = d.B; a.K = d.D; a.N = d.J; a.W = p->in_proj_weight; a.ldw = d.J; a.in = d_x_t; a.ldin = d.D; a.st = si;

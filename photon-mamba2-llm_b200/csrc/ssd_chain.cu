@@ -23,7 +23,7 @@
 // plain operands, 8200 with pairs; two warps of the role per scheduler, so the chains inside a warp count).  The code
 // is kept small (rolled loops): at 130 KB of straight-line code every role waited for instruction fetches and a step took twice
 // as long.  Measured at 24 heads of 64 x 64: 23 us for 4 x 512 tokens on pairs, 147 us for 8 x 2048 on plain operands in chunks of
-// 256, 53 us for 1 x 1337 on pairs; the four kernels it replaces there (prepare, states, state pass, masked product) took 52 and
+// 256, 31 us (two launches over segments) for 1 x 1337 on pairs; the four kernels it replaces there (prepare, states, state pass, masked product) took 52 and
 // 290 us, the FMA contractions that served the odd length 590 us.  Every mbarrier wait is bounded; on expiry the CTA raises the status
 // word, every role stops issuing work, copies in flight are waited for (bounded) and TMEM is freed on the way out.
 #include <cuda_bf16.h>

@@ -1,5 +1,5 @@
 // Backward of the chunked SSD scan along a sequence as one kernel: the adjoint of ssd_chain.cu's forward except for the three
-// sums over heads (dG, dC, dB), which ssd_pairs.cu forms next to it.  One CTA owns one (batch, head) and walks its steps of 128
+// sums over heads (dG, dC, dB), which ssd_heads.cu forms after it.  One CTA owns one (batch, head) and walks its steps of 128
 // tokens from the last to the first with the state's adjoint dh in registers.
 //
 // Per step (rows s, columns t of the masked tile; S = inclusive cumulative sum of a in the step; h = state entering it, as the forward

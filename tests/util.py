@@ -16,7 +16,7 @@ FP32_TOL = 1e-4
 
 # The gradients of a_log and dt_bias are sums over all tokens of S-weighted differences of nearly equal terms (row
 # sums minus column sums of dM o M).  The tensor-core scans take both sums from the same registers (csrc/ssd_chain_bwd.cu,
-# which serves fp32 blocks whose widths are multiples of 8 with chunks of up to 256 tokens, or 64 with heads narrower than 64;
+# which serves fp32 blocks whose widths are multiples of 8 with chunks of up to 256 tokens (64 with heads narrower than 64);
 # csrc/ssd_fused.cu, which serves the scan operator at block_len % 128 == 0, d_state = d_head = 64), and there the two tensors get
 # the bar of every other tensor (`fused=True`).  The fp32 FMA engine that serves the remaining shapes forms the
 # difference from y and dx~ instead and is held to 5e-4 there (the reference's own cross-backend SSD gradient tests
