@@ -119,6 +119,23 @@ def test_decode_batches(pm, B, D, H, P, N, G):
     assert pm.device_status() == 0
 
 
+# more sequences than a grid has rows, on the general and on the tensor-core route of the projections
+@pytest.mark.parametrize("D,H,P,N", [(16, 1, 8, 4), (16, 2, 4, 7)])
+def test_decode_many_sequences(pm, D, H, P, N):
+    B = 65537
+    cfg, p, blk = _block(pm, D, H, P, N, 1, 64, torch.float32)
+    st = blk.zero_state(B)
+    ref = {"ssm_state": randn((B, H, N, P), 7, 0.3), "conv_window": randn((B, cfg.xbc_dim, 3), 8, 0.5)}
+    st["ssm_state"].copy_(ref["ssm_state"]); st["conv_window"].copy_(ref["conv_window"])
+    x = randn((B, 1, D), 20)
+    y, st = blk.step(x.cuda(), st)
+    y_ref, ref = orc.block_step(p, cfg, x, ref)
+    assert_close(y, y_ref, what="y")
+    assert_close(st["ssm_state"], ref["ssm_state"], what="state")
+    assert_close(st["conv_window"], ref["conv_window"], what="window")
+    assert pm.device_status() == 0
+
+
 # a captured step is replayed after the block has stepped at more batch sizes than it keeps workspaces for, and after memory has been
 # handed out again
 def test_captured_decode_outlives_other_batches(pm):
