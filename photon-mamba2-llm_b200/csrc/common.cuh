@@ -22,12 +22,15 @@ inline pmb_status fail(pmb_status st, const char* fmt, ...) {
   return st;
 }
 
+// (A refused call's error is taken back from the runtime, or the next launch check of this thread would report it again.)
 #define PMB_CUDA(expr)                                                                         \
   do {                                                                                         \
     cudaError_t e__ = (expr);                                                                  \
-    if (e__ != cudaSuccess)                                                                    \
+    if (e__ != cudaSuccess) {                                                                  \
+      cudaGetLastError();                                                                      \
       return pmb::fail(PMB_ERR_CUDA, "%s failed: %s (%s:%d)", #expr, cudaGetErrorString(e__),  \
                        __FILE__, __LINE__);                                                    \
+    }                                                                                          \
   } while (0)
 
 #define PMB_TRY(expr)                   \

@@ -769,7 +769,7 @@ extern "C" pmb_status pmb_lm_step_device_dp(pmb_lm* lm, void* stream, const int6
     const size_t need = (size_t)n * ((size_t)lm->d.M * lm->d.D * sizeof(float) + (size_t)lm->d.M * sizeof(int64_t));
     if (lm->gather_bytes < need) {     // first data-parallel step (make it outside stream capture)
       cudaFree(lm->gather); lm->gather = nullptr; lm->gather_bytes = 0;
-      if (cudaMalloc(&lm->gather, need) != cudaSuccess) { lm->split_table = 0; return fail(PMB_ERR_CUDA, "lm_step_device_dp: cannot allocate the gather buffer"); }
+      if (cudaMalloc(&lm->gather, need) != cudaSuccess) { cudaGetLastError(); lm->split_table = 0; return fail(PMB_ERR_CUDA, "lm_step_device_dp: cannot allocate the gather buffer"); }
       lm->gather_bytes = need;
     }
   }

@@ -314,6 +314,13 @@ def test_first_calls_on_several_threads(pm):
     assert r.returncode == 0 and r.stdout.strip() == "same", r.stderr[-2000:]
 
 
+# an allocation that the driver refuses fails the call that asked for it, and no later one
+def test_refused_call_does_not_fail_the_next(pm):
+    assert pm.lib.pmb_gemm_reserve_scratch(1 << 60) != 0
+    a, b = randn((64, 32), 1).cuda(), randn((32, 64), 2).cuda()
+    assert_close(pm.matmul(a, b), a.double() @ b.double(), tol=3e-5, what="product")
+
+
 # the CTA-pair GEMM's ways of storing a result: ragged edges (odd widths, rows past the last whole tile), fp32 and bf16, a residual
 # loaded ahead, a result added onto C, and the two tile widths (few tiles with a long K take the narrow one on pairs)
 @pytest.mark.parametrize("M,N,K", [(2048, 768, 1536), (1100, 1411, 200), (300, 4616, 72)])
