@@ -180,7 +180,8 @@ pmb_status pmb_ssd_scan_bwd(void* stream, int32_t batch, int32_t seqlen, int32_t
  * kernels that form them.  What is formed on the way (masked tiles, scaled rows, states) enters the products rounded to bf16 when
  * d_head is 64, d_state 64 or 128, and 2 to 64 chunks of 128 tokens or 3 to 64 chunks of 256 make a sequence (one chunk of 128 needs
  * no state), and as (hi, lo) bf16 pairs otherwise.  With d_head 64, d_state 64 or 128, block_len a multiple of 128 up to 1024 and at
- * most 64 chunks the eight bf16 pointers must be 16-byte aligned.  Other shapes widen to fp32, run the fp32 scan and round. */
+ * most 64 chunks the eight bf16 pointers must be 16-byte aligned.  On all other shapes the final state is formed in fp32 throughout.  Shapes beyond
+ * d_head 64 or d_state 128 widen to fp32, run the fp32 scan and round. */
 size_t pmb_ssd_workspace_bytes_bf16(int32_t batch, int32_t seqlen, int32_t n_heads, int32_t d_head,
                                     int32_t d_state, int32_t n_groups, int32_t block_len);
 pmb_status pmb_ssd_scan_fwd_bf16(void* stream, int32_t batch, int32_t seqlen, int32_t n_heads, int32_t d_head,

@@ -196,6 +196,23 @@ def test_scan_bf16_lengths(pm, B, T, P, N, G, off):
             assert_close(got, want, tol=tol, what=what)
 
 
+# the state that the bf16-input scan hands on is formed in fp32 off the whole chunks (whole ones round what they form): fp32 sums of up to
+# 700 decaying terms stay within 2e-6 of fp64, sums of bf16 pairs are 5e-6 off.
+@pytest.mark.parametrize("B,T", [(1, 1), (2, 127), (1, 129), (3, 200), (1, 700)])
+@pytest.mark.parametrize("P,N,G,off", [(64, 64, 1, 0), (64, 128, 4, 0), (32, 16, 1, 0), (8, 40, 1, 3)])
+def test_scan_bf16_final_state_in_fp32(pm, B, T, P, N, G, off):
+    H = 4
+    x, b, c = randn((B, T, H, P), 1).bfloat16(), randn((B, T, G, N), 2).bfloat16(), randn((B, T, G, N), 3).bfloat16()
+    a = -torch.nn.functional.softplus(randn((B, T, H), 5) - 2.0)
+    init = torch.cat([torch.zeros(off), randn((B, H, N, P), 6).flatten()]).cuda()[off:].view(B, H, N, P)
+    be, ce = (t.double().expand(B, T, H, N) for t in (b, c))
+    for i0 in (None, init):
+        _, want = orc.ssd_scan_chunked(x.double(), a.double(), be, ce, T, initial_state=None if i0 is None else i0.cpu().double(), return_final_state=True)
+        _, last = pm.SsdScanBf16(x.cuda(), a.cuda(), b.cuda(), c.cuda(), 128).forward(init_state=i0, want_final_state=True)
+        assert pm.device_status() == 0
+        assert_close(last, want, tol=2e-6, what="final state")
+
+
 # chunks of several steps: a state is rounded to bf16 between the steps only where that leaves da (fp32) about as far off as one rounding
 # per chunk does; a single chunk, two chunks of two steps and chunks of more steps keep da and the state at fp32 precision
 @pytest.mark.parametrize("T,Q", [(256, 256), (512, 256), (384, 384), (768, 384), (1024, 512), (1024, 1024)])
