@@ -504,6 +504,19 @@ def gated_rmsnorm_bwd_static(dout, y, z, w, rstd):
 # Mamba2Block
 # ------------------------------------------------------------------------------------------------
 
+def _kept_workspace(holder, n, device):
+    """The scratch that `holder` keeps between calls, at least n bytes.  It belongs to one thread and stream: a call from another one
+    gets a new one (what is still running keeps the old one's memory, which the allocator hands out again on that stream only).  A
+    captured call takes memory of the capture's pool, which lives as long as the graph: the kept one goes when a larger call comes, and a
+    replay would write to memory of another tensor."""
+    if torch.cuda.is_current_stream_capturing():
+        return torch.empty(n, device=device, dtype=torch.uint8)
+    owner, kept = (device, _stream(), threading.get_ident()), holder._ws
+    if kept is None or kept[0] != owner or kept[1].numel() < n:
+        kept = holder._ws = (owner, torch.empty(n, device=device, dtype=torch.uint8))
+    return kept[1]
+
+
 class Mamba2Block:
     """One block: parameters are a dict of fp32 CUDA tensors in `PARAM_ORDER`."""
 
@@ -522,6 +535,7 @@ class Mamba2Block:
         self._cfg_c, self._cfg_key = None, None
         self._params_c, self._params_key = None, None
         self._step_ws = threading.local()
+        self._config_struct()
         self.refresh_weights()
 
     def refresh_weights(self):
@@ -539,11 +553,9 @@ class Mamba2Block:
 
     def _config_struct(self):
         """The C view of the configuration, rebuilt when one of its values was changed."""
-        c = self.config
-        key = (c.d_model, c.d_state, c.d_head, c.n_heads, c.n_groups, c.d_conv, c.block_len, c.rmsnorm_eps)
-        if key != self._cfg_key:
+        if vars(self.config) != self._cfg_key:
             self._step_ws = threading.local()        # (the sizes of steps' workspaces follow from it)
-            self._cfg_c, self._cfg_key = c.c(), key
+            self._cfg_c, self._cfg_key = self.config.c(), dict(vars(self.config))
         return C.byref(self._cfg_c)
 
     def _params_struct(self):
@@ -565,9 +577,7 @@ class Mamba2Block:
         n = fn(cfg, B, T)
         if n == 0:
             raise PmbError(1, lib.pmb_last_error().decode())
-        if self._ws is None or self._ws.numel() < n:
-            self._ws = torch.empty(n, device=device, dtype=torch.uint8)
-        return self._ws
+        return _kept_workspace(self, n, device)
 
     def forward(self, x, residual=None):
         B, T, D = x.shape
@@ -649,25 +659,27 @@ class ContextEncoder:
             arr[i] = _params_struct(p)
         return arr
 
+    def _workspace(self, B, T, device):
+        return _kept_workspace(self, lib.pmb_stack_workspace_bytes(C.byref(self.config.c()), B, T), device)   # two forward slots: recompute one block ahead
+
     def forward_checkpointed(self, x):
         B, T, D = x.shape
         L = len(self.layers)
-        n = lib.pmb_stack_workspace_bytes(C.byref(self.config.c()), B, T)   # two forward slots: recompute one block ahead
-        if self._ws is None or self._ws.numel() < n:
-            self._ws = torch.empty(n, device=x.device, dtype=torch.uint8)
+        ws = self._workspace(B, T, x.device)
         saved = torch.empty(L + 1, B, T, D, device=x.device, dtype=torch.float32)
         saved[0].copy_(x)
         _check(lib.pmb_stack_fwd_ckpt(_stream(), C.byref(self.config.c()), L, self._arrays(self.layers), B, T,
-                                      saved.data_ptr(), self._ws.data_ptr(), self._ws.numel()))
+                                      saved.data_ptr(), ws.data_ptr(), ws.numel()))
         return saved[L], saved
 
     def checkpoint_backward(self, saved, dhidden, on_layer_done=None):
         L, B, T, D = saved.shape[0] - 1, saved.shape[1], saved.shape[2], saved.shape[3]
         grads = [{k: torch.empty_like(v) for k, v in p.items()} for p in self.layers]
+        ws = self._workspace(B, T, saved.device)
         dh = dhidden.clone()
         cb = LAYER_CALLBACK(on_layer_done) if on_layer_done else C.cast(None, LAYER_CALLBACK)
         _check(lib.pmb_stack_bwd(_stream(), C.byref(self.config.c()), L, self._arrays(self.layers), self._arrays(grads),
-                                 B, T, saved.data_ptr(), dh.data_ptr(), self._ws.data_ptr(), self._ws.numel(), cb, None))
+                                 B, T, saved.data_ptr(), dh.data_ptr(), ws.data_ptr(), ws.numel(), cb, None))
         return dh, grads
 
 

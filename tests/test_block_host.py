@@ -17,6 +17,22 @@ class Recorder:
     def pmb_mamba2_step_workspace_bytes(self, cfg, batch):
         return 256 * batch
 
+    def pmb_mamba2_block_workspace_bytes(self, cfg, batch, seqlen):
+        return 64 * batch * seqlen
+
+    pmb_stack_workspace_bytes = pmb_mamba2_block_workspace_bytes
+
+    def pmb_mamba2_block_fwd(self, stream, cfg, params, batch, seqlen, x, residual, out, ws, n):
+        self.steps.append((threading.get_ident(), ws, n))
+        self.inside.wait(10)
+        return 0
+
+    def pmb_stack_fwd_ckpt(self, stream, cfg, layers, params, batch, seqlen, saved, ws, n):
+        return self.pmb_mamba2_block_fwd(stream, cfg, params, batch, seqlen, saved, None, None, ws, n)
+
+    def pmb_stack_bwd(self, stream, cfg, layers, params, grads, batch, seqlen, saved, dh, ws, n, cb, user):
+        return self.pmb_mamba2_block_fwd(stream, cfg, params, batch, seqlen, saved, None, None, ws, n)
+
     def pmb_mamba2_step(self, stream, cfg, params, batch, x, state, window, y, ws, n):
         self.config, self.params = cfg._obj, params._obj
         self.steps.append((threading.get_ident(), ws, n))
@@ -31,11 +47,13 @@ def pm(monkeypatch):
     import pm_b200
     monkeypatch.setattr(pm_b200, "lib", Recorder())
     monkeypatch.setattr(pm_b200, "_dev", lambda t, name: t)
-    monkeypatch.setattr(pm_b200, "_stream", lambda: 7)
+    monkeypatch.setattr(pm_b200.Mamba2Block, "_io", lambda self, t, name: t)
+    pm_b200.on_stream = 7
+    monkeypatch.setattr(pm_b200, "_stream", lambda: pm_b200.on_stream)
     pm_b200.capturing = False
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: pm_b200.capturing)
     yield pm_b200
-    del pm_b200.capturing
+    del pm_b200.capturing, pm_b200.on_stream
 
 
 def make(pm):
@@ -122,3 +140,51 @@ def test_edited_configuration_counts(pm):
     blk.config.rmsnorm_eps = 1e-3
     step(blk)
     assert pm.lib.config.rmsnorm_eps == pytest.approx(1e-3)
+
+
+def calls(pm, kind):
+    """A function that makes one call of the kind at a sequence length, and the object that keeps its workspace."""
+    blk = make(pm)
+    if kind == "block":
+        return lambda T: blk.forward(torch.zeros(1, T, 16))
+    enc = pm.ContextEncoder(blk.config, [blk.params])
+    if kind == "stack":
+        return lambda T: enc.forward_checkpointed(torch.zeros(1, T, 16))
+    return lambda T: enc.checkpoint_backward(torch.zeros(2, 1, T, 16), torch.zeros(1, T, 16))
+
+
+@pytest.mark.parametrize("kind", ["block", "stack", "stack backward"])
+def test_block_and_stack_workspaces(pm, kind):
+    call = calls(pm, kind)
+    used = lambda: pm.lib.steps[-1][1:]
+    call(8)
+    first = used()
+    call(4)
+    assert used() == first == (first[0], 64 * 8)     # kept, and large enough for less
+    held, empty = [], torch.empty
+    torch.empty = lambda *a, **k: held.append(empty(*a, **k)) or held[-1]
+    try:
+        pm.capturing = True
+        call(8)
+    finally:
+        torch.empty, pm.capturing = empty, False
+    captured = used()[0]
+    assert captured != first[0] and captured in [t.data_ptr() for t in held]
+    call(8)
+    assert used() == first
+    call(16)                                         # grows
+    assert used()[1] == 64 * 16 and used()[0] != captured
+    pm.on_stream = 9
+    call(4)
+    assert used()[1] == 64 * 4                       # another stream: not the large one, which stream 7 may still use
+
+
+def test_block_workspace_on_two_threads(pm):
+    call = calls(pm, "block")
+    pm.lib.inside = threading.Barrier(2)
+    threads = [threading.Thread(target=call, args=(8,)) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert pm.lib.steps[0][1] != pm.lib.steps[1][1]
