@@ -61,7 +61,7 @@ pmb_status cast_f32_bf16(cudaStream_t st, const float* src, uint16_t* dst, int64
 }
 
 struct BlockWs {
-  float *xzd, *act, *dt, *y, *rstd, *normed, *Aneg;
+  float *xzd, *act, *dt, *y, *y_plain, *rstd, *normed, *Aneg;      // y_plain: y without the skip term, where the scan's backward reads it
   SsdWs ssd;
   float *seg, *seg_bwd;          // states (and their adjoints) of the segments that few long sequences are cut into
   int nseg;
@@ -117,6 +117,7 @@ static size_t block_ws_layout(const Dims& d, void* base, size_t bytes, BlockWs* 
     f.act = ar.take<float>((size_t)d.M * d.X);
     f.dt = ar.take<float>((size_t)d.M * d.H);
     f.y = ar.take<float>(mi);
+    f.y_plain = !chain && ssd_wants_plain_y(d.P, d.N, d.Q) ? ar.take<float>(mi) : nullptr;
     f.rstd = ar.take<float>((size_t)d.M);
     f.normed = ar.take<float>(pairs ? 0 : mi);       // with pair GEMMs the normalised output only exists as a pair
     f.Aneg = ar.take<float>((size_t)d.H);
@@ -181,6 +182,7 @@ static SsdIn ssd_inputs(const Dims& d, const pmb_block_params& p, const BlockWs&
   in.dt = w.dt; in.A = w.Aneg; in.a = nullptr;
   in.b = w.act + d.I; in.c = w.act + d.I + d.G * d.N; in.ldbc = d.X;
   in.D = p.d_skip;
+  in.y_plain = w.y_plain;
   return in;
 }
 

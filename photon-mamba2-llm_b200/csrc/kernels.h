@@ -51,6 +51,9 @@ struct SsdIn {
   const float* a;         // (B,T,H), used when dt == NULL
   const float* b; const float* c; int64_t ldbc;
   const float* D;         // (H) skip weights or NULL:  y += D[h] * x
+  // y without the skip term, (B,T,H,P) or NULL.  Written by a forward and read by a backward that forms dS from <dY, y - D x> (every engine but
+  // the fused pairs): where D x outweighs the rest of y the subtraction leaves nothing of it.
+  float* y_plain = nullptr;
   bool dys_ready = false; // backward: ws.dys = dY exp(S) was already written by the caller
   bool dy_pair_ready = false;  // backward: ws.dy_hi / dy_lo (the pair of dY) were already written by the caller
   bool bc_pair_ready = false;  // forward: ws.bc_hi / bc_lo (the pairs of B | C) were already written by the caller
@@ -90,6 +93,7 @@ struct SsdWs {            // persistent between fwd and bwd of one scan
   float* rpart;              // (B,nc,H,Q/128,Q) partial row sums of W (fused backward)
 };
 size_t ssd_ws_layout(int B, int T, int H, int P, int N, int G, int Q, void* base, size_t bytes, SsdWs* out);
+bool ssd_wants_plain_y(int P, int N, int Q);      // shapes whose backward reads y_plain
 // the same buffers taken from a caller's arena in two parts: bit 0 = forward-written / backward-read, bit 1 = backward only
 struct Arena;
 void ssd_ws_take(Arena& ar, int B, int T, int H, int P, int N, int G, int Q, SsdWs* w, int part);

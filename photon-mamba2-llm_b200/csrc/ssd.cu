@@ -9,7 +9,7 @@
 //             dx~ = (CB o L)^T dY + exp(S_end - S_s) B_s dh
 //             dG = sum_heads L o (dY x~^T);  dC = dG B + sum_h exp(S_t) dY_t h_prev^T;
 //             dB = dG^T C + sum_h exp(S_end - S_s) x~_s dh^T
-//             dS_t = <dY_t, Y_t> - <x~_t, dx~_t>, dS_{Q-1} += <dh, h_next>;  da = reverse cumsum(dS)
+//             dS_t = <dY_t, Y_t> - <x~_t, dx~_t>, dS_{Q-1} += <dh, h_next>;  da = reverse cumsum(dS)   (Y without the skip term)
 // The reference computes the same quantities with ~40 primitive ops and autograd
 // (crates/pm-core/src/mamba2/ssd_ops.rs:167-284); nothing of size (Q,Q) per head is stored here.
 //
@@ -32,9 +32,9 @@ struct SsdP {
   const float* b; const float* c; int64_t ldbc;
   const float* D;
   float* S; float* hprev; float* hlast; float* CB; float* dh; float* dG; float* dxt;
-  const float* y; int64_t ldy;
+  const float* y; int64_t ldy; bool skip_in_y;
   const float* dy; int64_t lddy;
-  float* yout; int64_t ldyo;
+  float* yout; int64_t ldyo; float* yplain;
   float* db; float* dc; int64_t lddbc;
 
   __device__ __forceinline__ int64_t tok(int bb, int cc, int q) const { return (int64_t)bb * T + (int64_t)cc * Q + q; }
@@ -133,6 +133,7 @@ struct OpScan {
   __device__ float seg_scale(int, int, int) const { return 1.0f; }
   __device__ bool seg_active(int) const { return true; }
   __device__ void store(int m, int n, float v) const {
+    if (p.yplain) p.yplain[((cx.t0 + m) * p.H + cx.h) * p.P + n] = v;
     if (p.D) v = fmaf(p.D[cx.h], p.x[(cx.t0 + m) * p.ldx + cx.h * p.P + n], v);
     p.yout[(cx.t0 + m) * p.ldyo + cx.h * p.P + n] = v;
   }
@@ -593,13 +594,13 @@ __global__ void ssd_rowdots_kernel(SsdP p, float* __restrict__ dx, int64_t lddx,
   int64_t total = (int64_t)p.B * p.T * p.H;
   if (w >= total) return;
   int h = (int)(w % p.H); int64_t tk = w / p.H;
-  float dtv = p.dtv(tk, h), Dv = p.D ? p.D[h] : 0.0f;
+  float dtv = p.dtv(tk, h), Dv = p.D ? p.D[h] : 0.0f, Dy = p.skip_in_y ? Dv : 0.0f;
   float s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
   for (int pp = lane; pp < p.P; pp += 32) {
     float xv = p.x[tk * p.ldx + h * p.P + pp];
     float dxt = p.dxt[tk * (int64_t)(p.H * p.P) + h * p.P + pp];
     float dyv = p.dy[tk * p.lddy + h * p.P + pp];
-    float yv = p.y[tk * p.ldy + h * p.P + pp] - Dv * xv;
+    float yv = p.y[tk * p.ldy + h * p.P + pp] - Dy * xv;
     s1 = fmaf(dxt, xv, s1);
     s2 = fmaf(dyv, yv, s2);
     s3 = fmaf(dyv, xv, s3);
@@ -683,7 +684,7 @@ __global__ void __launch_bounds__(PREP_THREADS) chunk_rows_finish_kernel(SsdP p,
   __shared__ float s_ddtx[PREP_MAX_Q], s_dS[PREP_MAX_Q], s_dD[PREP_MAX_Q], s_dt[PREP_MAX_Q], wsum[PREP_THREADS / 32], red[32];
   const int w = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int h = w % p.H, bc = w / p.H, cc = bc % p.nc, bb = bc / p.nc;
-  const float Dv = p.D ? p.D[h] : 0.0f;
+  const float Dv = p.D ? p.D[h] : 0.0f, Dy = p.skip_in_y ? Dv : 0.0f;
   const int64_t tok0 = p.tok(bb, cc, 0);
   const int P4 = p.P >> 2;
   // phase 1: a half-warp per row, float4 lanes (P <= 64) or strided lanes beyond
@@ -699,7 +700,7 @@ __global__ void __launch_bounds__(PREP_THREADS) chunk_rows_finish_kernel(SsdP p,
         const float4 dxt = reinterpret_cast<const float4*>(p.dxt + tk * (int64_t)(p.H * p.P) + h * p.P)[j];
         const float4 dyv = reinterpret_cast<const float4*>(p.dy + tk * p.lddy + h * p.P)[j];
         float4 yv = reinterpret_cast<const float4*>(p.y + tk * p.ldy + h * p.P)[j];
-        yv.x -= Dv * xv.x; yv.y -= Dv * xv.y; yv.z -= Dv * xv.z; yv.w -= Dv * xv.w;
+        yv.x -= Dy * xv.x; yv.y -= Dy * xv.y; yv.z -= Dy * xv.z; yv.w -= Dy * xv.w;
         s1 = fmaf(dxt.x, xv.x, fmaf(dxt.y, xv.y, fmaf(dxt.z, xv.z, fmaf(dxt.w, xv.w, s1))));
         s2 = fmaf(dyv.x, yv.x, fmaf(dyv.y, yv.y, fmaf(dyv.z, yv.z, fmaf(dyv.w, yv.w, s2))));
         s3 = fmaf(dyv.x, xv.x, fmaf(dyv.y, xv.y, fmaf(dyv.z, xv.z, fmaf(dyv.w, xv.w, s3))));
@@ -1064,6 +1065,7 @@ bool ssd_chain_enabled() {
   static const bool simt = [] { const char* e = getenv("PMB_SSD_ENGINE"); return e && strcmp(e, "simt") == 0; }();
   return fused_enabled() && !simt;
 }
+bool ssd_wants_plain_y(int P, int N, int Q) { return !(ssd_chain_enabled() && ssd_fused_supported(P, N, Q)); }
 bool ssd_plain16_shape(int P, int N, int Q) { return P == 64 && N == 64 && (Q == 128 || Q == 256); }
 
 // x~[b,t,h,:] = x[b,t,h,:] * dt[b,t,h] as a bf16 pair (only when the fused cumsum kernel did not already write it)
@@ -1123,7 +1125,7 @@ pmb_status ssd_fwd(cudaStream_t st, const SsdIn& in, const float* init_state, fl
                    const SsdWs& ws) {
   SsdP p;
   PMB_TRY(fill_params(in, ws, &p));
-  p.yout = y; p.ldyo = ldy;
+  p.yout = y; p.ldyo = ldy; p.yplain = in.y_plain;
   int nbch = p.B * p.nc * p.H, nbcg = p.B * p.nc * p.G;
   const double tok = (double)p.B * p.T;
   const bool tc = ssd_tc_supported(in) && (ldy % 4 == 0) && (reinterpret_cast<uintptr_t>(y) % 16 == 0);
@@ -1209,7 +1211,7 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
                    const SsdGrads& g, const SsdWs& ws) {
   SsdP p;
   PMB_TRY(fill_params(in, ws, &p));
-  p.y = y; p.ldy = ldy; p.dy = dy; p.lddy = lddy; p.db = g.db; p.dc = g.dc; p.lddbc = g.lddbc;
+  p.y = in.y_plain ? in.y_plain : y; p.ldy = in.y_plain ? (int64_t)in.H * in.P : ldy; p.skip_in_y = in.D && !in.y_plain; p.dy = dy; p.lddy = lddy; p.db = g.db; p.dc = g.dc; p.lddbc = g.lddbc;
   int nbch = p.B * p.nc * p.H, nbcg = p.B * p.nc * p.G;
   int64_t rows = (int64_t)p.B * p.T * p.H;
   float* ddt_x = ws.rows; float* dS = ws.rows + rows; float* dDrow = ws.rows + 2 * rows; float* dsend = ws.rows + 3 * rows;

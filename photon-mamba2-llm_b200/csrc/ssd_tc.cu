@@ -33,7 +33,7 @@ struct TcP {
   const float* dt; const float* D;
   const float* S;
   const float* dy; int64_t lddy;
-  float* y; int64_t ldy;
+  float* y; int64_t ldy; float* yplain;
   float* hprev; float* dh; float* CB; float* dG; float* dxt; float* part;
   const float* xs;   // (B,T,H,P)  x * dt * exp(S_end - S_t)
   const float* dys;  // (B,T,H,P)  dY * exp(S_t)
@@ -210,6 +210,11 @@ struct TcScan {
     if (MODE == 0) {
       const int64_t row = t.tok0 + m;
       float4* dst = reinterpret_cast<float4*>(p.y + row * p.ldy + t.h * p.P + nb);
+      if (p.yplain) {
+        float4* pl = reinterpret_cast<float4*>(p.yplain + (row * p.H + t.h) * p.P + nb);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) pl[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      }
       if (p.D) {
         const float dv = p.D[t.h];
         const float4* xs = reinterpret_cast<const float4*>(p.x + row * p.ldx + t.h * p.P + nb);
@@ -506,7 +511,7 @@ pmb_status ssd_tc_state(cudaStream_t st, const SsdIn& in, const SsdWs& ws) {
 
 pmb_status ssd_tc_scan(cudaStream_t st, const SsdIn& in, float* y, int64_t ldy, const SsdWs& ws) {
   TcP p = make_p(in, ws);
-  p.y = y; p.ldy = ldy;
+  p.y = y; p.ldy = ldy; p.yplain = in.y_plain;
   MapSet ms{};
   int64_t tok = (int64_t)p.B * p.T;
   PMB_TRY(get_map(&ms.m[0], ws.CB, p.Q, (int64_t)p.B * p.nc * p.G * p.Q, 1, p.Q, (int64_t)p.Q * p.Q, 32, 128, false));

@@ -83,6 +83,24 @@ def test_block_backward_lengths(pm, B, T, P, N, G, H):
             assert_close(g, leaves[k].grad, tol=FP32_TOL if chain else tol_for(k), what=k)
 
 
+# inputs of the size that a model's embeddings have, where D x outweighs the scan's part of y a thousand times: d(a_log) and d(dt_bias) do not
+# go through y - D x, on the FMA contractions (odd widths, ragged lengths, d_head beyond 64), 3xTF32 (d_state 128 on whole chunks), and the chains
+@pytest.mark.parametrize("P,N,H,T,Q", [(64, 128, 8, 256, 128), (64, 128, 8, 300, 128), (64, 64, 8, 300, 128), (64, 64, 6, 256, 128), (32, 16, 4, 200, 64), (24, 40, 6, 128, 64),
+                                       (128, 64, 4, 128, 64), (5, 7, 3, 60, 32)])
+def test_block_gradients_of_small_inputs(pm, P, N, H, T, Q):
+    D, B = 64, 2
+    cfg, p, blk = _block(pm, D, H, P, N, 1, Q, torch.float32)
+    x, cot = randn((B, T, D), 5, 0.02), randn((B, T, D), 6, 1e-3)
+    dx, grads = blk.backward(x.cuda(), cot.cuda())
+    assert pm.device_status() == 0
+    leaves = {k: v.double().requires_grad_(True) for k, v in p.items()}
+    xr = x.double().requires_grad_(True)
+    orc.block_forward(leaves, cfg, xr).backward(cot.double())
+    assert_close(dx, xr.grad, what="dx")
+    for k, g in grads.items():
+        assert_close(g, leaves[k].grad, tol=tol_for(k), what=k)
+
+
 # token counts at which the weight gradients of the bf16-storage block split K or not, with and without whole tiles
 @pytest.mark.parametrize("B,T", [(1, 40), (1, 1100), (3, 1024)])
 def test_block_bf16_weight_gradient_splits(pm, B, T):
