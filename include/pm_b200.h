@@ -232,8 +232,8 @@ pmb_status pmb_gated_rmsnorm_bwd_static(void* stream, int64_t rows, int32_t widt
  * bf16 pairs of their fp32 operands (16 mantissa bits; engine 4 of pmb_gemm_f32).  So do the products inside the scan: in the forward with
  * d_head up to 64 and d_state up to 128, multiples of 8; in the backward with both up to 64, d_model, d_inner (at most 2048) and in_proj_dim
  * multiples of 8, and chunks of at most 256 tokens (64 with d_head below 64; any multiple of 128 with both at 64).  Elsewhere the scan uses
- * fp32 FMA or 3xTF32.  One block measured against fp64: output and gradients 5e-6 to 2e-5 of their norm; d(a_log) and d(dt_bias) up to 8e-4 where
- * the backward's scan is FMA. */
+ * fp32 FMA or 3xTF32.  One block measured against fp64: output and gradients 5e-6 to 2e-5 of their norm; d(a_log) and d(dt_bias), where the
+ * backward's scan is FMA or 3xTF32, 1.5e-5 to 1.4e-4 in models (pmb_lm_*) and up to 1e-3 (inputs of unit size) or 3e-3 (half that) here. */
 size_t pmb_mamba2_block_workspace_bytes(const pmb_mamba2_config* cfg, int32_t batch, int32_t seqlen);
 pmb_status pmb_mamba2_block_fwd(void* stream, const pmb_mamba2_config* cfg, const pmb_block_params* params,
                                 int32_t batch, int32_t seqlen, const float* d_x, const float* d_residual,

@@ -90,13 +90,13 @@ static size_t slab_floats(const Dims& d) {
 // that work chunk by chunk.)
 // Chunks (a sequence that no chunk divides is one) of more than 256 tokens, or 64 with heads narrower than 64, other than multiples of
 // 128 at 64 x 64, keep the FMA contractions in fp32 outside of a model.  Theirs is not the better result: they form d(a_log) and d(dt_bias) as
-// <dY, y> - <x~, dx~>, whose rounding grows with the chunk (from fp64, relative to the gradient's norm: 1e-4 at 200 tokens, 2e-4 to 8e-4 at
-// 1000 to 1337; the sums of the chain kernel 1e-5 to 2.5e-5; all other gradients are equally far off), nor the faster one (forward and backward
-// of 2 x 1337 tokens, 24 heads of 64 x 64: 2395 us, 519 as chains; a stack of five on 2 x 740: 7.2 ms, 1.9).  They stay because those two
-// gradients of a call would move by that much, more than fp32 results are expected to between two builds (2e-4).
-static bool block_uses_chain_bwd(const Dims& d, bool bf16, bool in_model) {
+// <dY, y - D x> - <x~, dx~>, 1e-4 of their norm from fp64 on unit-size inputs of 200 tokens and 2e-4 to 8e-4 at 1000 to 1337 (the chain kernels'
+// sums 1e-5 to 2.5e-5; all other gradients are equally far off; for smaller inputs see outweighed in ssd.cu), nor the faster one (forward and
+// backward of 2 x 1337 tokens, 24 heads of 64 x 64: 2395 us, 514 as chains; a stack of five on 2 x 740: 7.2 ms, 1.9).  They stay because those
+// two gradients of a call would move by that much, more than fp32 results are expected to between two builds (2e-4).
+static bool block_uses_chain_bwd(const Dims& d, bool bf16) {
   const bool dims = bf16 ? !ssd_plain16_shape(d.P, d.N, d.Q) && d.D % 8 == 0 && d.J % 8 == 0 && d.I % 8 == 0 : block_uses_pairs(d);
-  const bool close = bf16 || in_model || ssd_fused_supported(d.P, d.N, d.Q) || d.Q <= (d.P >= 64 ? 256 : 64);
+  const bool close = bf16 || d.in_model || ssd_fused_supported(d.P, d.N, d.Q) || d.Q <= (d.P >= 64 ? 256 : 64);
   return dims && close && ssd_chain_enabled() && ssd_chain_bwd_shape(d.P, d.N, true) && d.I <= 2048;
 }
 
@@ -108,7 +108,7 @@ static bool block_uses_chain_bwd(const Dims& d, bool bf16, bool in_model) {
 static size_t block_ws_layout(const Dims& d, void* base, size_t bytes, BlockWs* out, bool bf16 = false, int nslots = 1, int slot = 0, bool presplit = false) {
   Arena ar(base, bytes);
   BlockWs w{};
-  const bool pairs = !bf16 && block_uses_pairs(d), chain = block_uses_chain_bwd(d, bf16, presplit);
+  const bool pairs = !bf16 && block_uses_pairs(d), chain = block_uses_chain_bwd(d, bf16);
   const size_t hp = (size_t)d.M * d.I, steps_np = (size_t)d.B * cdiv(d.T, SCAN_STEP) * d.H * d.N * d.P;
   const size_t md = (size_t)d.M * d.D, mi = (size_t)d.M * d.I, mj = (size_t)d.M * d.J, dj = (size_t)d.D * d.J, id = (size_t)d.I * d.D;
   for (int sl = 0; sl < nslots; ++sl) {
@@ -175,7 +175,7 @@ static size_t block_ws_layout(const Dims& d, void* base, size_t bytes, BlockWs* 
 size_t block_ws_bytes(const Dims& d, bool bf16) { return block_ws_layout(d, nullptr, 0, nullptr, bf16); }
 size_t stack_ws_bytes(const Dims& d, bool bf16, bool presplit) { return block_ws_layout(d, nullptr, 0, nullptr, bf16, 2, 0, presplit); }
 
-static SsdIn ssd_inputs(const Dims& d, const pmb_block_params& p, const BlockWs& w) {
+static SsdIn ssd_inputs(const Dims& d, const pmb_block_params& p, const BlockWs& w, bool bf16) {
   SsdIn in{};
   in.B = d.B; in.T = d.T; in.H = d.H; in.P = d.P; in.N = d.N; in.G = d.G; in.Q = d.Q;
   in.x = w.act; in.ldx = d.X;
@@ -183,6 +183,7 @@ static SsdIn ssd_inputs(const Dims& d, const pmb_block_params& p, const BlockWs&
   in.b = w.act + d.I; in.c = w.act + d.I + d.G * d.N; in.ldbc = d.X;
   in.D = p.d_skip;
   in.y_plain = w.y_plain;
+  in.y_plain_rarely = !bf16 && !d.in_model;
   return in;
 }
 
@@ -246,10 +247,10 @@ static pmb_status block_fwd_core(cudaStream_t st, const Dims& d, const pmb_block
   ConvPairOut bc{};
   // (bf16 storage: the scan reads the hi halves alone, so the lo halves are not written)
   if (w.ssd.bc_hi) bc = ConvPairOut{w.ssd.bc_hi, w16 ? nullptr : w.ssd.bc_lo, d.I, 2 * d.G * d.N};
-  const bool chain = block_uses_chain_bwd(d, w16 != nullptr, wx && wx->pairs);
+  const bool chain = block_uses_chain_bwd(d, w16 != nullptr);
   if (chain) bc.lo = w.ssd.bc_lo;
   PMB_TRY(conv_silu_dt_fwd(st, d, w.xzd, p.conv1d_weight, p.conv1d_bias, p.dt_bias, w.act, nullptr, w.ssd.bc_hi ? &bc : nullptr));
-  SsdIn sin = ssd_inputs(d, p, w);
+  SsdIn sin = ssd_inputs(d, p, w, w16 != nullptr);
   if (chain) {
     ChainArgs a = chain_inputs(d, p, w.xzd, w.act, w.ssd.bc_hi, w.ssd.bc_lo, w.y);
     a.S_out = w.ssd.S; a.dt_out = w.dt; a.A_out = w.Aneg; a.hp_hi = w.ssd.hp_hi; a.hp_lo = w.ssd.hp_lo; a.seg = w.seg;
@@ -306,7 +307,7 @@ pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, 
   Pair16 wout{nullptr, nullptr, 0};
   const bool plain = block_plain16(d, w16 != nullptr), by_chunks = scan_by_chunks(d, w16 != nullptr, false);
   // (a stack whose blocks keep the FMA contractions scans with them in the forward too: its gradients are those of the forward that it ran)
-  const bool as_backward = backward_follows && !w16 && !block_uses_chain_bwd(d, false, wx && wx->pairs);
+  const bool as_backward = backward_follows && !w16 && !block_uses_chain_bwd(d, false);
   if (ssd_chain_enabled() && ssd_chain_shape(d.P, d.N) && !by_chunks && !as_backward) {
     // nothing is kept for a backward: the scan is one kernel that takes dt_raw, x and the B | C pair as the conv left them
     FwdWs f{};
@@ -422,11 +423,11 @@ static pmb_status block_grads(cudaStream_t st, const Dims& d, const pmb_block_pa
   // dY exp(S) for the scan backward when the tensor-core scan will run.
   uint16_t* ph = pr ? w.dxzd_hi : (w16 ? w.dxzd16 : nullptr);   // bf16 storage: plain bf16 rounding, no low part
   uint16_t* pl = pr ? w.dxzd_lo : nullptr;
-  SsdIn sin = ssd_inputs(d, p, w);
+  SsdIn sin = ssd_inputs(d, p, w, w16 != nullptr);
   sin.plain16 = w16 != nullptr;
   NormBwdExtra ex{};
   ex.dz_hi = ph; ex.dz_lo = pl;
-  const bool chain = block_uses_chain_bwd(d, w16 != nullptr, wx && wx->pairs);
+  const bool chain = block_uses_chain_bwd(d, w16 != nullptr);
   if (!chain && (pr || w16) && ssd_tc_supported(sin) && (d.P % 4 == 0)) {
     ex.S = w.ssd.S; ex.H = d.H; ex.P = d.P; ex.T = d.T; sin.dys_ready = true;
     if (w.ssd.dy_hi) {   // the scan backward runs on bf16 pairs: dY and dY exp(S) leave the norm backward as pairs

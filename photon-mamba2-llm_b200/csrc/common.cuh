@@ -117,6 +117,7 @@ struct Arena {
 
 struct Dims {
   int B, T, D, N, P, H, G, K, Q, I, X, J, nc;
+  bool in_model = false;      // a block of a model handle (lm.cu)
   int64_t M;  // tokens
   float eps;
 };

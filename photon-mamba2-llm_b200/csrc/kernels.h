@@ -54,6 +54,7 @@ struct SsdIn {
   // y without the skip term, (B,T,H,P) or NULL.  Written by a forward and read by a backward that forms dS from <dY, y - D x> (every engine but
   // the fused pairs): where D x outweighs the rest of y the subtraction leaves nothing of it.
   float* y_plain = nullptr;
+  bool y_plain_rarely = false;    // backward: only for rows in which D x outweighs the rest of y by far (outweighed in ssd.cu)
   bool dys_ready = false; // backward: ws.dys = dY exp(S) was already written by the caller
   bool dy_pair_ready = false;  // backward: ws.dy_hi / dy_lo (the pair of dY) were already written by the caller
   bool bc_pair_ready = false;  // forward: ws.bc_hi / bc_lo (the pairs of B | C) were already written by the caller

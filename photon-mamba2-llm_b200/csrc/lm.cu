@@ -348,6 +348,7 @@ static pmb_status lm_create_impl(const pmb_mamba2_config* cfg, int L0, int L1, i
   *out = nullptr;
   Dims d;
   PMB_TRY(make_dims(cfg, batch, seqlen, &d));
+  d.in_model = true;
   if (bf16_storage && ((d.D % 8) || (d.J % 8) || (d.I % 8)))
     return fail(PMB_ERR_SHAPE, "lm_create: bf16 storage needs d_model, d_inner and in_proj_dim to be multiples of 8");
   if (L0 <= 0 || L1 < 0 || vocab <= 0) return fail(PMB_ERR_SHAPE, "lm_create: layer counts and vocab must be positive");
@@ -360,6 +361,7 @@ static pmb_status lm_create_impl(const pmb_mamba2_config* cfg, int L0, int L1, i
   if (L1 > 0) {
     pmb_status s1 = make_dims(cfg, batch, seqlen / group, &lm->d1);
     if (s1 != PMB_OK) { delete lm; return s1; }
+    lm->d1.in_model = true;
   }
   lm->Vp = (int)align_up((size_t)vocab, 64);
   int tile_cap = LM_TILE_ROWS;

@@ -32,7 +32,7 @@ struct SsdP {
   const float* b; const float* c; int64_t ldbc;
   const float* D;
   float* S; float* hprev; float* hlast; float* CB; float* dh; float* dG; float* dxt;
-  const float* y; int64_t ldy; bool skip_in_y;
+  const float* y; int64_t ldy; bool skip_in_y; const float* yp;      // yp: y without the skip term, for the rows that want it
   const float* dy; int64_t lddy;
   float* yout; int64_t ldyo; float* yplain;
   float* db; float* dc; int64_t lddbc;
@@ -585,6 +585,13 @@ static pmb_status launch_state_scan(cudaStream_t st, const SsdP& p, float* buf, 
   return PMB_OK;
 }
 
+// fp32 blocks outside of a model take <dY, y - D x> except in rows (one token and head) that this holds for: there D x is more than 48 times what
+// the scan adds per unit of dt (of dt, because heads with a small dt have a small y on any input), and the difference has lost most of y.
+// Inputs of unit size have next to no such rows and keep their results, which <dY, y> throughout would move by up to 8e-4 in d(a_log) and
+// d(dt_bias).  From fp64 those two are off by (8 heads of 64 x 64, 2 x 1000 tokens; y - D x everywhere / in the other rows): inputs
+// of size 1: 6.7e-4 / 5.9e-4; 0.5: 2.8e-3 / 2.9e-3; 0.2: 2.6e-2 / 2.6e-3; 0.1: 0.10 / 2.2e-4; 0.02: 0.78 / 7.8e-5.
+__device__ __forceinline__ bool outweighed(float skip_sq, float y_sq, float dt) { return skip_sq * dt * dt > 48.0f * 48.0f * y_sq; }
+
 // One warp per (b,t,h): row dot products and dx.
 //   ddt_x = <dx~, x>;  dS = <dY, Y - D x> - dt * ddt_x;  dDrow = <dY, x>;  dx = dx~ * dt + D * dY
 __global__ void ssd_rowdots_kernel(SsdP p, float* __restrict__ dx, int64_t lddx, float* __restrict__ ddt_x,
@@ -595,7 +602,7 @@ __global__ void ssd_rowdots_kernel(SsdP p, float* __restrict__ dx, int64_t lddx,
   if (w >= total) return;
   int h = (int)(w % p.H); int64_t tk = w / p.H;
   float dtv = p.dtv(tk, h), Dv = p.D ? p.D[h] : 0.0f, Dy = p.skip_in_y ? Dv : 0.0f;
-  float s1 = 0.0f, s2 = 0.0f, s3 = 0.0f;
+  float s1 = 0.0f, s2 = 0.0f, s3 = 0.0f, s2p = 0.0f, yy = 0.0f, kk = 0.0f;
   for (int pp = lane; pp < p.P; pp += 32) {
     float xv = p.x[tk * p.ldx + h * p.P + pp];
     float dxt = p.dxt[tk * (int64_t)(p.H * p.P) + h * p.P + pp];
@@ -604,9 +611,17 @@ __global__ void ssd_rowdots_kernel(SsdP p, float* __restrict__ dx, int64_t lddx,
     s1 = fmaf(dxt, xv, s1);
     s2 = fmaf(dyv, yv, s2);
     s3 = fmaf(dyv, xv, s3);
+    if (p.yp) {
+      const float q = p.yp[(tk * p.H + h) * p.P + pp], k = Dv * xv;
+      s2p = fmaf(dyv, q, s2p); yy = fmaf(q, q, yy); kk = fmaf(k, k, kk);
+    }
     dx[tk * lddx + h * p.P + pp] = fmaf(dxt, dtv, Dv * dyv);
   }
   s1 = warp_sum(s1); s2 = warp_sum(s2); s3 = warp_sum(s3);
+  if (p.yp) {
+    s2p = warp_sum(s2p); yy = warp_sum(yy); kk = warp_sum(kk);
+    if (outweighed(kk, yy, dtv)) s2 = s2p;
+  }
   if (lane == 0) {
     ddt_x[w] = s1;
     dS[w] = s2 - dtv * s1;
@@ -691,7 +706,7 @@ __global__ void __launch_bounds__(PREP_THREADS) chunk_rows_finish_kernel(SsdP p,
   const int sub = lane >> 4, l16 = lane & 15;
   for (int t0 = wid * 2; t0 < p.Q; t0 += (PREP_THREADS / 32) * 2) {
     const int t = t0 + sub;
-    float s1 = 0.0f, s2 = 0.0f, s3 = 0.0f, dtv = 1.0f;
+    float s1 = 0.0f, s2 = 0.0f, s3 = 0.0f, s2p = 0.0f, yy = 0.0f, kk = 0.0f, dtv = 1.0f;
     if (t < p.Q) {
       const int64_t tk = tok0 + t;
       dtv = p.dtv(tk, h);
@@ -700,6 +715,13 @@ __global__ void __launch_bounds__(PREP_THREADS) chunk_rows_finish_kernel(SsdP p,
         const float4 dxt = reinterpret_cast<const float4*>(p.dxt + tk * (int64_t)(p.H * p.P) + h * p.P)[j];
         const float4 dyv = reinterpret_cast<const float4*>(p.dy + tk * p.lddy + h * p.P)[j];
         float4 yv = reinterpret_cast<const float4*>(p.y + tk * p.ldy + h * p.P)[j];
+        if (p.yp) {
+          const float4 q = reinterpret_cast<const float4*>(p.yp + (tk * p.H + h) * p.P)[j];
+          const float4 k = make_float4(Dv * xv.x, Dv * xv.y, Dv * xv.z, Dv * xv.w);
+          s2p = fmaf(dyv.x, q.x, fmaf(dyv.y, q.y, fmaf(dyv.z, q.z, fmaf(dyv.w, q.w, s2p))));
+          yy = fmaf(q.x, q.x, fmaf(q.y, q.y, fmaf(q.z, q.z, fmaf(q.w, q.w, yy))));
+          kk = fmaf(k.x, k.x, fmaf(k.y, k.y, fmaf(k.z, k.z, fmaf(k.w, k.w, kk))));
+        }
         yv.x -= Dy * xv.x; yv.y -= Dy * xv.y; yv.z -= Dy * xv.z; yv.w -= Dy * xv.w;
         s1 = fmaf(dxt.x, xv.x, fmaf(dxt.y, xv.y, fmaf(dxt.z, xv.z, fmaf(dxt.w, xv.w, s1))));
         s2 = fmaf(dyv.x, yv.x, fmaf(dyv.y, yv.y, fmaf(dyv.z, yv.z, fmaf(dyv.w, yv.w, s2))));
@@ -711,6 +733,13 @@ __global__ void __launch_bounds__(PREP_THREADS) chunk_rows_finish_kernel(SsdP p,
 #pragma unroll
     for (int o = 8; o > 0; o >>= 1) {        // sums within each half-warp
       s1 += __shfl_xor_sync(0xffffffffu, s1, o); s2 += __shfl_xor_sync(0xffffffffu, s2, o); s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+    }
+    if (p.yp) {
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        s2p += __shfl_xor_sync(0xffffffffu, s2p, o); yy += __shfl_xor_sync(0xffffffffu, yy, o); kk += __shfl_xor_sync(0xffffffffu, kk, o);
+      }
+      if (outweighed(kk, yy, dtv)) s2 = s2p;
     }
     if (t < p.Q && l16 == 0) { s_ddtx[t] = s1; s_dS[t] = s2 - dtv * s1; s_dD[t] = s3; s_dt[t] = dtv; }
   }
@@ -1211,7 +1240,8 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
                    const SsdGrads& g, const SsdWs& ws) {
   SsdP p;
   PMB_TRY(fill_params(in, ws, &p));
-  p.y = in.y_plain ? in.y_plain : y; p.ldy = in.y_plain ? (int64_t)in.H * in.P : ldy; p.skip_in_y = in.D && !in.y_plain; p.dy = dy; p.lddy = lddy; p.db = g.db; p.dc = g.dc; p.lddbc = g.lddbc;
+  const bool plain = in.y_plain && !in.y_plain_rarely;
+  p.y = plain ? in.y_plain : y; p.ldy = plain ? (int64_t)in.H * in.P : ldy; p.skip_in_y = in.D && !plain; p.yp = plain ? nullptr : in.y_plain; p.dy = dy; p.lddy = lddy; p.db = g.db; p.dc = g.dc; p.lddbc = g.lddbc;
   int nbch = p.B * p.nc * p.H, nbcg = p.B * p.nc * p.G;
   int64_t rows = (int64_t)p.B * p.T * p.H;
   float* ddt_x = ws.rows; float* dS = ws.rows + rows; float* dDrow = ws.rows + 2 * rows; float* dsend = ws.rows + 3 * rows;

@@ -101,6 +101,30 @@ def test_block_gradients_of_small_inputs(pm, P, N, H, T, Q):
         assert_close(g, leaves[k].grad, tol=tol_for(k), what=k)
 
 
+# the same in a model, whose token embeddings are of that size: every engine of the scan's backward, fp32 and bf16 storage (2e-2 as for any
+# bf16 gradient)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("P,N,H,T,Q", [(64, 128, 8, 256, 128), (64, 128, 8, 300, 128), (32, 16, 8, 200, 64), (24, 40, 8, 128, 64), (32, 16, 4, 200, 64), (128, 64, 8, 128, 64)])
+def test_model_decay_gradients(pm, dtype, P, N, H, T, Q):
+    D, B, V, L = 128, 2, 200, 2
+    if dtype == torch.bfloat16 and H % 8:
+        pytest.skip("bf16 storage wants widths that are multiples of 8")
+    cfg = orc.Mamba2Config(d_model=D, d_state=N, d_head=P, n_heads=H, n_groups=1, d_conv=4, block_len=Q)
+    layers, embed = [block_params(cfg, seed=61 + l) for l in range(L)], randn((V, D), 13, 0.02)
+    lm = pm.FlatMamba(pm.Mamba2Config(d_model=D, d_state=N, d_head=P, n_heads=H, n_groups=1, d_conv=4, block_len=Q), L, V, B, T, compute_dtype=dtype)
+    lm.load(embed.cuda(), [cuda_params(p) for p in layers])
+    ids, tg, _ = orc.lcg_batch(17, B, T, V)
+    lm.step_device(ids.cuda(), tg.cuda())
+    er, ls = embed.double().requires_grad_(True), [{k: v.double().requires_grad_(True) for k, v in p.items()} for p in layers]
+    orc.lm_loss(er, ls, cfg, ids, tg, cdt=torch.float64).backward()
+    assert pm.device_status() == 0
+    _, gl = lm.grads()
+    for l in range(L):
+        for k in ("a_log", "dt_bias", "in_proj_weight", "d_skip"):
+            assert_close(gl[l][k], ls[l][k].grad, tol=tol_for(k) if dtype == torch.float32 else 2e-2, what=f"layer {l} {k}")
+    lm.close()
+
+
 # token counts at which the weight gradients of the bf16-storage block split K or not, with and without whole tiles
 @pytest.mark.parametrize("B,T", [(1, 40), (1, 1100), (3, 1024)])
 def test_block_bf16_weight_gradient_splits(pm, B, T):

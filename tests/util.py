@@ -19,8 +19,8 @@ FP32_TOL = 1e-4
 # which serves fp32 blocks whose widths are multiples of 8 with chunks of up to 256 tokens (64 with heads narrower than 64);
 # csrc/ssd_fused.cu, which serves the scan operator at block_len % 128 == 0, d_state = d_head = 64), and there the two tensors get
 # the bar of every other tensor (`fused=True`).  The fp32 FMA engine that serves the remaining shapes forms the
-# difference from y and dx~ instead and is held to 5e-4 there (the reference's own cross-backend SSD gradient tests
-# use 1e-3, crates/pm-cuda/tests/grad_ssd.rs:62-227).
+# difference from y and dx~ instead and is held to 5e-4 there on the tests' inputs (the reference's own cross-backend SSD
+# gradient tests use 1e-3, crates/pm-cuda/tests/grad_ssd.rs:62-227).
 CANCELLATION_TOL = 5e-4
 
 # One 24-layer step: every tensor carries the rounding of ~150 bf16-pair GEMMs in sequence (16 mantissa bits per
