@@ -387,7 +387,7 @@ gemm_bf16_kernel(const __grid_constant__ Group g, const int total_tiles, unsigne
   // advances it by total_tiles per replay).  sched == NULL: CTA b takes tiles b, b + gridDim.x, ...
   auto ticket_tile = [&](unsigned long long t) { return (int)gridDim.x + (int)((t - ticket0) % (unsigned long long)total_tiles); };
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
@@ -646,7 +646,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ Group g) {
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(tiles_ptr + STAGES * STAGE_BYTES + 8 * (2 * STAGES + 1));
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int m0 = (tile / q.tiles_n) * 256 + (int)rank * TBM;     // this CTA's rows of A and of the output
   const int n0 = (tile % q.tiles_n) * BN2;                      // the pair's columns; this CTA loads B columns n0 + rank*128 ..
   const int nb0 = n0 + (int)rank * BNH;
@@ -787,6 +787,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ Group g) {
 // inside `if (lane == 0)`, 791 us = 1390 TFLOP/s with one elected lane of a converged warp and one commit for both CTAs); at K = 768 the
 // 256 KB of fp32 that a tile writes.  Four epilogue warps were the limit there: products with a bf16 residual 67 -> 40 us, the two
 // gradients of in_proj at 16384 tokens 165 -> 129, of the tied head per 1024 rows 339 -> 254.
+// The warp index is a shuffle's result, so that the roles' branches are uniform to the compiler: 2 % of the training steps' products.
 // The CTA-pair kernel above as a tile loop: cluster c works on tiles c, c + clusters, ...; the operand ring keeps
 // running across tiles; the accumulator alternates between two TMEM buffers of BN2 columns, so each CTA drains its
 // 128 rows of tile i (through the same TMA-store epilogue as the single-CTA kernel) while the leader issues tile
@@ -828,7 +829,7 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
   auto r_bar = [&](int w, int slot) { return bars + 8u * (2 * STAGES + 4 + NSLOT * w + slot); };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(tiles_ptr + STAGES * STAGE_BYTES + EPI + 8 * (2 * STAGES + 4 + PairPCfg<SPLIT, BN2>::EPI_WARPS * NSLOT));
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }

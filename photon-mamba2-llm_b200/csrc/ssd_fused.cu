@@ -143,7 +143,7 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
   float* rsum = sS + MAXQ;                              // mode 1: [NGRP][2][NEPI][CW] column sums of W per warp
   float* xchg = rsum + 2 * NGRP * NEPI * CW;            // mode 1: [2][RB] second group's row sums, handed to the first
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int bch = (int)blockIdx.x;                      // (b * nc + chunk) * H + head
   // the row blocks with the most column blocks are scheduled first
   const int rb = MODE == 0 ? p.nb - 1 - (int)blockIdx.y : (int)blockIdx.y;

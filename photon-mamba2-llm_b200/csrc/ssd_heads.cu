@@ -14,7 +14,8 @@
 // 11 %); warps wait for TMEM loads, each of which is followed at once by its wait, with five warps to a scheduler.
 // Measured at 24 heads of 64 x 64 on pairs, 4 x 512 tokens: 18 us + 3 us for the sum of the shares; the three contractions and their
 // sums that it replaces took 45 us and read copies of dY and x~ scaled by the decays that are not made any more.  bf16, 32 heads of 128 x 64, 16 x 8192 tokens: 836 us with two
-// stages, 820 with three (3.2 GB of operands; the contractions it replaces: 1070 us).
+// stages, 820 with three, 670 since the warp index is a shuffle's result (uniform branches and descriptors) and a wait looks at its barrier first
+// (3.2 GB of operands; the contractions it replaces: 1070 us).
 #include <cuda_bf16.h>
 #include "tc_common.cuh"
 #include "kernels.h"
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
   volatile uint32_t* abort_flag = tmem_slot + 1;
   float* sS = reinterpret_cast<float*>(bar_ptr + 256);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   int id = (int)blockIdx.x;
   const int split = id % p.nsplit; id /= p.nsplit;
   const int tile = id;
@@ -118,6 +119,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
 
   auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
   auto wait = [&](int b, uint32_t parity, unsigned int code) -> bool {
+    if (mbar_wait(bar(b), parity & 1u, 1u)) return true;
     if (*abort_flag) return false;
     if (mbar_wait(bar(b), parity & 1u)) return true;
     give_up(code);
