@@ -6,7 +6,7 @@
 //   x~[s,:] = x[s,:] dt[s],  xs[s,:] = x~[s,:] exp(S_end - S_s)             transform warps -> shared memory (bf16 operands)
 //   G = C B^T   (128 x 128)                                                 tensor core, TMEM
 //   M[t,s] = G[t,s] exp(S_t - S_s) [s <= t]                                 mask warps, TMEM -> registers -> TMEM over G
-//   y[t,:] = M x~ + exp(S_t) C_t h + D x[t,:]                               tensor core, mask warps' epilogue
+//   y[t,:] = M x~ + exp(S_t) C_t h + D x[t,:]                               tensor core, output warps
 //   h <- exp(S_end) h + B^T xs                                              tensor core, state warps' registers
 // S, xs and h can also be kept per chunk of two steps (plain bf16 operands): the second step's rows then see the first
 // one's columns through a masked tile of their own and h as it entered the chunk.
@@ -15,16 +15,23 @@
 // any length: rows past the end arrive as zeros (TMA fills them per batch) and carry a = 0.  d_state up to 128 and d_head
 // up to 64, in multiples of 8: the 64-wide tiles are zero-filled beyond them.
 //
-// warp 0 = TMA producer (B and C tiles), 1 = MMA issuer, 4..11 = two mask groups of four warps (columns 0-63 / 64-127 of
-// the masked tile; then one half of the output columns each), 12..19 = transform, 20..23 = state.  The MMA issuer runs
-// G one step ahead, the mask warps mask step i + 1 before they drain step i, and the only chain from step to step is
-// h -> h (a few hundred clocks), so the roles overlap.
-// What bounds it: the instructions of the mask warps (mask 2500-2900 clocks, drain and store 3500 of a step of about 6600 with
-// plain operands, 8200 with pairs; two warps of the role per scheduler, so the chains inside a warp count).  The code
-// is kept small (rolled loops): at 130 KB of straight-line code every role waited for instruction fetches and a step took twice
-// as long.  Measured at 24 heads of 64 x 64: 23 us for 4 x 512 tokens on pairs, 147 us for 8 x 2048 on plain operands in chunks of
-// 256, 31 us (two launches over segments) for 1 x 1337 on pairs; the four kernels it replaces there (prepare, states, state pass, masked product) took 52 and
-// 290 us, the FMA contractions that served the odd length 590 us.  Every mbarrier wait is bounded; on expiry the CTA raises the status
+// warp 0 = TMA loads (B, C, bf16 x), 1 = products of the masked tile (G one item ahead, M x~), 2 = products of the state (C h, U), 3 = TMA
+// stores, 4..11 = two mask groups of four warps, then twelve warps of output and transform (eight and four; on fp32 pairs, whose
+// transform rounds every element twice, four and eight), 24..27 = state.
+// What bounds it: no pipe and no memory level.  A step takes 9100 warp instructions at d_state 128 on plain operands, issued in 41 % of the
+// cycles; every role is a chain of TMEM loads, shared memory and arithmetic with two warps of it on a scheduler.  What shaped the roles are
+// clocks read inside a step of 16 x 8192 tokens, 32 heads of 128 x 64, bf16 (927 us when masking and output were one role and one warp issued
+// all products, 700 now):
+//  - the products are issued by two warps: with one, its waits and the issue took 5000 of a step's 5200 clocks.  The warp index comes from a
+//    shuffle, so that the roles' branches and the descriptors are uniform to the compiler (742 -> 711 us, this kernel alone);
+//  - B and C are given back before the masked product waits for the mask, so that the next tiles (2200 clocks) land while it is masked;
+//  - bf16 x is the operand x~ as it is and comes by TMA: copied by the transform warps, their few pieces in flight took 4200 clocks a step;
+//  - a and dt are requested two chunks ahead (a head's tokens are a line apart), and below the diagonal the masked tile takes one
+//    exponential per row and block of 32 columns instead of one per element (not where M is rounded for a stream of bf16 values: those
+//    results are what they were).
+// Measured at 24 heads of 64 x 64: 23.4 us for 4 x 512 tokens on pairs (23.9 before the above), 141 us for 8 x 2048 on plain operands in chunks
+// of 256 with all that a chunk-by-chunk backward reads (188), 31 us (two launches over segments) for 1 x 1337 on pairs.  Every mbarrier wait is
+// bounded; on expiry the CTA raises the status
 // word, every role stops issuing work, copies in flight are waited for (bounded) and TMEM is freed on the way out.
 #include <cuda_bf16.h>
 #include <mutex>
@@ -52,13 +59,15 @@ constexpr int L = SCAN_STEP;            // tokens per step (= the MMA's M)
 constexpr int PW = 64;                  // width of the head tile
 constexpr int T128 = L * 128;           // bytes of a 128-row x 64-element bf16 tile (128-byte rows)
 constexpr int T64 = 64 * 128;
-// Six warpgroups; setmaxnreg shares the block's 80 x 768 registers out by what a role keeps live (40 + 2 x 88 + 2 x 72 + 120 per
-// thread of the six groups).
-constexpr int W_MASK = 4, W_XF = 12, W_ST = 20, NWARPS = 24, NTHREADS = 32 * NWARPS, XF_THREADS = 256;
+// Seven warpgroups: 0 loads, stores and MMAs, 1 and 2 mask, then three of output and transform warps, 6 state.  setmaxnreg shares the
+// block's 72 x 896 registers out by what a role keeps live.  Per thread: 40, 2 x 64 or 72, then 96 + 2 x 64 or 2 x 72 + 72, and 104.
+constexpr int W_MASK = 4, W_OUT = 12, W_ST = 24, NWARPS = 28, NTHREADS = 32 * NWARPS;
 
 // NB = 128-token blocks per chunk: S, the decay of xs and the state are relative to chunks of NB blocks.
-template <int NI, int ND, int NK, int NB>
+template <int NI, int ND, int NK, int NB, bool XIN16>
 struct Geo {
+  // fp32 pairs spend most on the transform (two roundings of every element, twice), the others on the output
+  static constexpr int OUTW = NI == 2 ? 4 : 8, XFW = 12 - OUTW, XF_THREADS = 32 * XFW;
   static constexpr int BT = NI * NK * T128;              // B (or C) of a step
   static constexpr int STAGE = 2 * BT;                   // [B | C]
   static constexpr int XT = NI * T128;                   // x~
@@ -67,29 +76,34 @@ struct Geo {
   static constexpr bool BIG = NI * NK == 4;              // pairs at d_state 128: one stage of B | C is all that fits
   static constexpr int STG = BIG ? 1 : 2;
   static constexpr int XB = ND == 1 ? 2 : 1;
-  static constexpr int NSB = NB == 1 ? XB + 1 : 2;       // copies of S: a chunk's S is read until its last tile has been masked
+  // copies of S: a chunk's S is read until its last tile has been masked and its output scaled, which the transform warps know of the
+  // step XB + 2 (two blocks to a chunk: the chunk three) before the one they begin (see there)
+  static constexpr int NSB = NB == 1 ? XB + 2 : 3;
   static_assert(NB == 1 || (STG == 2 && XB == 2), "both blocks of a chunk are resident");
   static constexpr int TILES = STG * STAGE + XB * XBUF + HB;
-  static constexpr int AHEAD = BIG ? 0 : (ND * NK >= 2 ? 3 : 4);              // 16-byte pieces of x that every transform thread has in flight
-  static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 256 /*barriers*/ + NSB * NB * L * 4 + (BIG ? 4 : 8) * NB * L /*row factors*/ + AHEAD * XF_THREADS * 16;
+  // fp32 x: 16-byte pieces that every transform thread has in flight (bf16 x is copied into the operand tile as it is)
+  static constexpr int AHEAD = BIG || XIN16 ? 0 : ND == 2 ? 3 : 16;
+  // (BIG: no room for column factors and half of the alignment slack; shared memory starts 1024-byte aligned where nothing static
+  // precedes it, and the kernel checks)
+  static constexpr int SLOT = (BIG ? 1 : 2) * L, SLACK = BIG ? 512 : 1024;    // floats per copy of S: [S | column factors]
+  static constexpr int SMEM = TILES + SLACK + 256 /*barriers*/ + NSB * SLOT * 4 + (BIG ? 4 : 8) * NB * L /*row factors*/ + AHEAD * XF_THREADS * 16;
 };
 
-struct Maps { CUtensorMap b[2], c[2], xt, xs; };         // [0] = hi (or the plain bf16 tensor), [1] = lo
+struct Maps { CUtensorMap b[2], c[2], x, xt, xs; };      // [0] = hi (or the plain bf16 tensor), [1] = lo; x = bf16 x
 
 struct Params {
   int T, H, hpg, N, P, nsteps;
-  const float* x; const uint16_t* x16; int64_t ldx;
+  const float* x; int64_t ldx;                           // fp32
   const float* dt_raw; int64_t ld_raw; const float* dt_bias; const float* a_log;   // raw mode: dt and A are formed here
   const float* dt; const float* A; const float* a;                                 // (dt, A) or a alone
   const float* D;
   const float* init;                                     // (B,H,N,P) or NULL
   float* y; uint16_t* y16; int64_t ldy;
   float* dt_out; float* A_out; float* S_out;             // optional from here on: what a backward reads
-  uint16_t* x_keep;                                      // (B,T,H,P) copy of x16
   uint16_t *hp_hi, *hp_lo;                               // (B,nsteps,H,N,P)
   float* last;                                           // (B,H,N,P)
   // plain operands, for a backward that works chunk by chunk: state entering each chunk in fp32, exp(S) C h of every token, and
-  // (store_ops) x~ and xs as the kernel formed them
+  // (store_ops) x~ and xs as the kernel formed them.  bf16 x: store_ops leaves a copy of it.
   float *hprev, *yoff;
   int store_ops;
   int nseg, per;                                         // segments of a sequence, steps per segment
@@ -100,40 +114,45 @@ struct Params {
 
 template <int NI, int ND, int NK, int NB, bool XIN16>
 __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid_constant__ Maps maps, const Params p) {
-  using GE = Geo<NI, ND, NK, NB>;
-  constexpr int STG = GE::STG, XB = GE::XB, NSB = GE::NSB;
-  extern __shared__ uint8_t smem_raw[];
+  using GE = Geo<NI, ND, NK, NB, XIN16>;
+  constexpr int STG = GE::STG, XB = GE::XB, NSB = GE::NSB, OUTW = GE::OUTW, XFW = GE::XFW, XF_THREADS = GE::XF_THREADS, W_XF = W_OUT + OUTW;
+  // the masked tile by factors of blocks instead of an exponential per element: not where the rounding of M to bf16 is part of a stream
+  // of bf16 values (the storage blocks on plain operands: each flipped rounding would grow through the layers behind it)
+  constexpr bool FACT = NB == 1 && !GE::BIG && (ND == 2 || XIN16);
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
+  if (base - raw > (uint32_t)GE::SLACK) { if (threadIdx.x == 0) atomicOr(p.status, 4096u); return; }
   uint8_t* base_ptr = smem_raw + (base - raw);
   const uint32_t ring_s = base, xbuf_s = ring_s + STG * GE::STAGE, h_s = xbuf_s + XB * GE::XBUF, bars = h_s + GE::HB;
-  enum { FULL = 0, EMPTY = 2, XRDY = 4, XFREE = 6, SRDY = 8 /*4*/, GFULL = 12, MRDY = 14, UFULL = 16, UFREE, HRDY, HFREE, ACCFULL, ACCFREE, NBAR };
-  static_assert(8 * NBAR + 16 + 48 <= 256, "barrier block");
+  enum { FULL = 0, EMPTY = 2, XRDY = 4, XFREE = 6, SRDY = 8 /*4*/, GFULL = 12, MRDY = 14, UFULL = 16, UFREE, HRDY, HFREE, ACCFULL, ACCFREE, XIN = 22 /*2*/, NBAR = 24 };
+  static_assert(8 * NBAR + 8 + 48 <= 256 && NSB <= 4, "barrier block");
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
   uint8_t* bar_ptr = base_ptr + (bars - base);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 8 * NBAR);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  float* wsum = reinterpret_cast<float*>(bar_ptr + 8 * NBAR + 16);
+  float* wsum = reinterpret_cast<float*>(bar_ptr + 8 * NBAR + 8);
   float* sEnd = wsum + 8;                                   // S_end of the last four chunks
-  float* sS = reinterpret_cast<float*>(bar_ptr + 256);
-  float2* sfac = reinterpret_cast<float2*>(sS + NSB * NB * L);   // (dt, exp(S_end - S)) of the step's rows
-  float* sdt = sS + NSB * NB * L;                                // BIG: dt alone, the last kilobyte is not there
+  float* sS = reinterpret_cast<float*>(bar_ptr + 256);      // [NSB][S | FACT: exp(S_q - S), q = last token of the token's 32]
+  float2* sfac = reinterpret_cast<float2*>(sS + NSB * GE::SLOT);    // (dt, exp(S_end - S)) of the step's rows
+  float* sdt = sS + NSB * GE::SLOT;                                 // BIG: dt alone, the last kilobyte is not there
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int bh = (int)blockIdx.x / p.nseg, seg = (int)blockIdx.x % p.nseg;
   const int h = bh % p.H, bb = bh / p.H, g = h / p.hpg;
   const int i0 = seg * p.per, toff = i0 * L;               // first step and token of this CTA's segment
   const int n = min(p.per, p.nsteps - i0);
   const int64_t tokb = (int64_t)bb * p.T;
   if (threadIdx.x == 0) {
+    const int mmas = p.state_only ? 1 : 2;                  // warps that issue products
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bar(FULL + i), 1); mbar_init(bar(EMPTY + i), 1);
-      mbar_init(bar(XRDY + i), 8); mbar_init(bar(XFREE + i), ND == 1 && p.store_ops ? 2 : 1);
+      mbar_init(bar(FULL + i), 1); mbar_init(bar(EMPTY + i), mmas);
+      mbar_init(bar(XIN + i), 1); mbar_init(bar(XRDY + i), XFW); mbar_init(bar(XFREE + i), mmas + (p.store_ops ? 1 : 0));
       mbar_init(bar(GFULL + i), 1); mbar_init(bar(MRDY + i), 8);
     }
-    for (int i = 0; i < 4; ++i) mbar_init(bar(SRDY + i), 8);
+    for (int i = 0; i < 4; ++i) mbar_init(bar(SRDY + i), XFW);
     mbar_init(bar(UFULL), 1); mbar_init(bar(UFREE), 4); mbar_init(bar(HRDY), 4); mbar_init(bar(HFREE), 1);
-    mbar_init(bar(ACCFULL), 1); mbar_init(bar(ACCFREE), 8);
+    mbar_init(bar(ACCFULL), 2); mbar_init(bar(ACCFREE), OUTW);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -151,6 +170,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
   // bounded waits that also end as soon as another role of the CTA has given up
   auto wait = [&](int b, uint32_t parity, unsigned int code) -> bool {
+    if (mbar_wait(bar(b), parity & 1u, 1u)) return true;
     if (*abort_flag) return false;
     if (mbar_wait(bar(b), parity & 1u)) return true;
     give_up(code);
@@ -162,7 +182,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   if (warp == 0) {
     // ---------------- TMA producer: B and C tiles of each step ----------------
     if (lane == 0) {
-      int issued = 0;
+      int issued = 0, xissued = 0;
       for (int i = 0; i < n; ++i) {
         const int s = i % STG;
         if (!wait(EMPTY + s, (uint32_t)(i / STG) ^ 1u, 1u)) break;
@@ -176,18 +196,27 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
             if (!p.state_only) tma_load_4d(dst + GE::BT + (sp * NK + kt) * T128, &maps.c[sp], 64 * kt, toff + i * L, g, bb, bar(FULL + s));
           }
         issued = i + 1;
+        if (XIN16) {                                         // bf16 x is the operand tile x~ as it is
+          const int xb = i % XB;
+          if (!wait(XFREE + xb, (uint32_t)(i / XB) ^ 1u, 2048u)) break;
+          mbar_expect_tx(bar(XIN + xb), T128);
+          tma_load_4d(xbuf_s + xb * GE::XBUF, &maps.x, 0, toff + i * L, h, bb, bar(XIN + xb));
+          xissued = i + 1;
+        }
       }
-      if (*abort_flag)
+      if (*abort_flag) {
         for (int i = (issued > STG ? issued - STG : 0); i < issued; ++i) mbar_wait(bar(FULL + i % STG), (uint32_t)((i / STG) & 1));
+        for (int i = (xissued > XB ? xissued - XB : 0); i < xissued; ++i) mbar_wait(bar(XIN + i % XB), (uint32_t)((i / XB) & 1));
+      }
     }
-  } else if (ND == 1 && warp == 3 && p.store_ops) {
+  } else if ((XIN16 || ND == 1) && warp == 3 && p.store_ops) {
     // ---------------- x~ and xs go out as they lie in shared memory ----------------
     if (lane == 0) {
       for (int i = 0; i < n; ++i) {
         const int xb = i % XB;
-        if (!wait(XRDY + xb, (uint32_t)(i / XB), 1024u)) break;
+        if (!wait((XIN16 ? XIN : XRDY) + xb, (uint32_t)(i / XB), 1024u)) break;
         tma_store_4d(&maps.xt, xbuf_s + xb * GE::XBUF, 0, toff + i * L, h, bb);
-        tma_store_4d(&maps.xs, xbuf_s + xb * GE::XBUF + GE::XT, 0, toff + i * L, h, bb);
+        if (!XIN16) tma_store_4d(&maps.xs, xbuf_s + xb * GE::XBUF + GE::XT, 0, toff + i * L, h, bb);
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         mbar_arrive(bar(XFREE + xb));
@@ -195,11 +224,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer (the whole warp waits; one elected lane issues) ----------------
+    // ---------------- products of the masked tile: G and M x~ (the whole warp waits; one elected lane issues) ----------------
     const uint32_t dh = desc_hi(1024, 2);
     const uint32_t id_g = idesc_bf16(0, 0, L, L);            // G: both operands K-major
-    const uint32_t id_v = idesc_bf16(0, 1, L, PW);           // x x~, x h: B operand MN-major
-    const uint32_t id_u = idesc_bf16(1, 1, L, PW);           // B^T xs: both operands MN-major
+    const uint32_t id_v = idesc_bf16(0, 1, L, PW);           // x x~: B operand MN-major
     auto all = [&](bool v) -> bool { return __all_sync(0xffffffffu, v); };
     // G of the item (block k, earlier or same block kb of its chunk) into buffer m & 1
     auto mma_g = [&](int m, int k, int kb) -> bool {
@@ -216,33 +244,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
             mma_split<NI, NI>(tG + (uint32_t)((m & 1) * L), c0 + o, (NK * T128) >> 4, b0 + o, (NK * T128) >> 4, dh, id_g, (kt | q) ? 1u : 0u);
           }
         umma_commit(bar(GFULL + (m & 1)));
+        if (NB == 1 || k % NB > 0) umma_commit(bar(EMPTY + kb % STG));      // (that block's B and C have been in their last G)
       }
       __syncwarp();
       return true;
     };
-    if (p.state_only) {
-      for (int k = 0; k < n; ++k) {
-        const int s = k % STG, xb = k % XB;
-        if (!all(wait(FULL + s, (uint32_t)(k / STG), 2u) && wait(XRDY + xb, (uint32_t)(k / XB), 4u) && (k == 0 || wait(UFREE, (uint32_t)(k - 1), 4u)))) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (elect_one()) {
-          const uint32_t b0 = desc_lo(ring_s + s * GE::STAGE, T128), xs0 = desc_lo(xbuf_s + xb * GE::XBUF + GE::XT, T128);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const uint32_t o = (uint32_t)(q * 2048) >> 4;
-            mma_split<NI, ND>(tU, b0 + o, (NK * T128) >> 4, xs0 + o, T128 >> 4, dh, id_u, q ? 1u : 0u);
-          }
-          umma_commit(bar(UFULL)); umma_commit(bar(XFREE + xb)); umma_commit(bar(EMPTY + s));
-        }
-        __syncwarp();
-      }
-    }
     bool ok = !p.state_only && mma_g(0, 0, 0);
     int m = 0;                                               // item: (block, column block), the diagonal one last
 #pragma unroll 1
     for (int k = 0; k < n && ok; ++k) {
-      const int s = k % STG, xb = k % XB, rb = k % NB, c = k / NB;
-      if (STG == 1 && k > 0 && !(ok = mma_g(m, k, k))) break;
+      const int xb = k % XB, rb = k % NB;
 #pragma unroll 1
       for (int cb = 0; cb <= rb; ++cb, ++m) {
         if (STG == 2) {                                      // one item ahead
@@ -250,24 +261,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
           else if (k + 1 < n) ok = mma_g(m + 1, k + 1, k + 1 - (k + 1) % NB);
           if (!ok) break;
         }
-        if (cb == 0) {
-          // acc2 = C h
-          if (!(ok = all(wait(HRDY, (uint32_t)c, 8u) && (k == 0 || wait(ACCFREE, (uint32_t)(k - 1), 8u))))) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          if (elect_one()) {
-            const uint32_t c0 = desc_lo(ring_s + s * GE::STAGE + GE::BT, 16), h0 = desc_lo(h_s, T64);
-#pragma unroll
-            for (int kt = 0; kt < NK; ++kt)
-#pragma unroll
-              for (int q = 0; q < 4; ++q)
-                mma_split<NI, ND>(tA2, c0 + ((uint32_t)(kt * T128 + q * 32) >> 4), (NK * T128) >> 4, h0 + ((uint32_t)(kt * T64 + q * 2048) >> 4), (NK * T64) >> 4, dh, id_v,
-                      (kt | q) ? 1u : 0u);
-            if (rb == NB - 1 || k + 1 == n) umma_commit(bar(HFREE));
-          }
-          __syncwarp();
-        }
         // acc1 += M x~, the masked tile read from TMEM: per 32 columns [hi: 16 | lo: 16], 8 columns per k-step of 16
-        if (!(ok = all((cb < rb || wait(XRDY + xb, (uint32_t)(k / XB), 4u)) && wait(MRDY + (m & 1), (uint32_t)(m >> 1), 16u)))) break;
+        if (!(ok = all((cb < rb || wait((XIN16 ? XIN : XRDY) + xb, (uint32_t)(k / XB), 4u)) && (cb > 0 || k == 0 || wait(ACCFREE, (uint32_t)(k - 1), 8u)) &&
+                       wait(MRDY + (m & 1), (uint32_t)(m >> 1), 16u)))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t xt0 = desc_lo(xbuf_s + ((k - rb + cb) % XB) * GE::XBUF, T128);
         if (elect_one()) {
@@ -278,186 +274,233 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
             mma_split_ts<ND, NI>(tA1, ta, 16u, vb, T128 >> 4, dh, id_v, acc);
           }
           if (cb == rb) umma_commit(bar(ACCFULL));
-          else umma_commit(bar(XFREE + (k - rb + cb) % XB));      // (the earlier block of the chunk is done with)
+          if (cb < rb || rb == NB - 1) umma_commit(bar(XFREE + (k - rb + cb) % XB));      // (that block of the chunk is done with)
         }
         __syncwarp();
+        if (STG == 1 && k + 1 < n) ok = mma_g(m + 1, k + 1, k + 1);
       }
-      if (!ok) break;
+    }
+  } else if (warp == 2) {
+    // ---------------- products of the state: C h and U (a warp of their own: the waits and the issue of one warp took 5000 of a
+    // step's 5200 clocks) ----------------
+    const uint32_t dh = desc_hi(1024, 2);
+    const uint32_t id_v = idesc_bf16(0, 1, L, PW);           // x h: B operand MN-major
+    const uint32_t id_u = idesc_bf16(1, 1, L, PW);           // B^T xs: both operands MN-major
+    auto all = [&](bool v) -> bool { return __all_sync(0xffffffffu, v); };
+    bool ok = true;
+#pragma unroll 1
+    for (int k = 0; k < n && ok; ++k) {
+      const int s = k % STG, xb = k % XB, rb = k % NB, c = k / NB;
+      // acc2 = C h
+      auto carried = [&]() -> bool {
+                if (!all(wait(FULL + s, (uint32_t)(k / STG), 4u) && wait(HRDY, (uint32_t)c, 8u) && (k == 0 || wait(ACCFREE, (uint32_t)(k - 1), 8u)))) return false;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (elect_one()) {
+                  const uint32_t c0 = desc_lo(ring_s + s * GE::STAGE + GE::BT, 16), h0 = desc_lo(h_s, T64);
+        #pragma unroll
+                  for (int kt = 0; kt < NK; ++kt)
+        #pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                      mma_split<NI, ND>(tA2, c0 + ((uint32_t)(kt * T128 + q * 32) >> 4), (NK * T128) >> 4, h0 + ((uint32_t)(kt * T64 + q * 2048) >> 4), (NK * T64) >> 4, dh, id_v,
+                            (kt | q) ? 1u : 0u);
+                  umma_commit(bar(ACCFULL));
+          if (XB == 2) umma_commit(bar(EMPTY + s));
+                  if (rb == NB - 1 || k + 1 == n) umma_commit(bar(HFREE));
+                }
+                __syncwarp();
+        return true;
+      };
       // U (+)= B^T xs: the chunk's contribution to the state
-      if (!(ok = all(rb > 0 || c == 0 || wait(UFREE, (uint32_t)(c - 1), 4u)))) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (elect_one()) {
-        // (M = 128 over one or two 64-wide blocks of d_state; with one block the second reads the tile behind it and
-        // its rows of U are never looked at)
-        const uint32_t b0 = desc_lo(ring_s + s * GE::STAGE, T128), xs0 = desc_lo(xbuf_s + xb * GE::XBUF + GE::XT, T128);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const uint32_t o = (uint32_t)(q * 2048) >> 4;
-          mma_split<NI, ND>(tU, b0 + o, (NK * T128) >> 4, xs0 + o, T128 >> 4, dh, id_u, (q | rb) ? 1u : 0u);
-        }
-        if (rb == NB - 1 || k + 1 == n) umma_commit(bar(UFULL));
-        if (rb == NB - 1) umma_commit(bar(XFREE + xb));
-        umma_commit(bar(EMPTY + s));
-      }
-      __syncwarp();
+      auto update = [&]() -> bool {
+                    if (!all(wait(FULL + s, (uint32_t)(k / STG), 4u) && wait(XRDY + xb, (uint32_t)(k / XB), 4u) &&
+                             (rb > 0 || c == 0 || wait(UFREE, (uint32_t)(c - 1), 4u)))) return false;
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              if (elect_one()) {
+                // (M = 128 over one or two 64-wide blocks of d_state; with one block the second reads the tile behind it and
+                // its rows of U are never looked at)
+                const uint32_t b0 = desc_lo(ring_s + s * GE::STAGE, T128), xs0 = desc_lo(xbuf_s + xb * GE::XBUF + GE::XT, T128);
+        #pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                  const uint32_t o = (uint32_t)(q * 2048) >> 4;
+                  mma_split<NI, ND>(tU, b0 + o, (NK * T128) >> 4, xs0 + o, T128 >> 4, dh, id_u, (q | rb) ? 1u : 0u);
+                }
+                if (rb == NB - 1 || k + 1 == n) umma_commit(bar(UFULL));
+                umma_commit(bar(XFREE + xb));
+          if (XB == 1 || p.state_only) umma_commit(bar(EMPTY + s));
+              }
+              __syncwarp();
+        return true;
+      };
+      // (two buffers of x: xs has been there for a while, and the state's chain does not wait for C h; one: xs is being formed)
+      ok = p.state_only ? update() : XB == 2 ? update() && carried() : carried() && update();
     }
   }
-  } else if (warp < W_XF) {
-    // ---------------- mask groups, then epilogue of the step before ----------------
-    regs_inc<88>();
+  } else if (warp < W_OUT) {
+    // ---------------- mask groups: blocks of 32 columns, group g those of index g and g + 2 ----------------
+    if (NI == 2) regs_dec<64>();
     const int quarter = warp & 3, grp = (warp - W_MASK) >> 2, r_local = quarter * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     bool ok = !p.state_only;
-    const float dv = p.D ? p.D[h] : 0.0f;
-    // the accumulators are drained in fragments of 16 rows x 8 columns (a quad of lanes holds 8 columns of a row: whole
-    // 32-byte sectors per store), so a thread's output rows are er + {0, 8, 16, 24} and not the row that it masks
-    const int er = quarter * 32 + (lane >> 2), ec = (lane & 3) * 2;
-    float fac[4] = {0.0f, 0.0f, 0.0f, 0.0f};                // exp(S) of those rows in the step whose epilogue is due
-    int k = 0, rb = 0, cb = 0;                              // this item: block k = block rb of its chunk, column block cb
-    // item after item; after the first tile of a block has been masked, the block before it is drained
-    for (int m = 0; k <= n; ++m) {
-      float fnext[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      const bool first = cb == 0;
-      if (ok && k < n) {
-        const int c = k / NB;
-        const float* S = sS + (c % NSB) * NB * L;
-        const bool got = wait(SRDY + (c % NSB), (uint32_t)(c / NSB), 32u) && wait(GFULL + (m & 1), (uint32_t)(m >> 1), 32u);
-        ok = __all_sync(0xffffffffu, got);
-        if (ok) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const float* Sc = S + cb * L;                      // S of the tile's columns
-          const float S_row = S[rb * L + r_local];
-          if (first) {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) fnext[e] = __expf(S[rb * L + er + 8 * e]);
-          }
-          const int c0 = grp * 64;
-          const uint32_t tg = tG + lane_addr + (uint32_t)((m & 1) * L + c0);
-          const bool above = cb == rb && grp == 1 && quarter < 2;       // every column of this half is past every row of this warp
-          const bool below = cb < rb || (grp == 0 && quarter >= 2);      // no column of this half is past any row of this warp
+    int k = 0, rb = 0, kc = 0;                              // this item: block k = block rb of its chunk, column block kc
 #pragma unroll 1
-          for (int half = 0; half < 2; ++half) {
-            uint32_t mh[16], ml[16];
-            if (above) {
+    for (int m = 0; k < n && ok; ++m) {
+      const int c = k / NB;
+      const float* S = sS + (c % NSB) * GE::SLOT;
+      ok = __all_sync(0xffffffffu, wait(SRDY + (c % NSB), (uint32_t)(c / NSB), 32u) && wait(GFULL + (m & 1), (uint32_t)(m >> 1), 32u));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int diag = NB == 1 || kc == rb ? quarter : 4;   // the block of 32 columns that the diagonal crosses (none: all are before every row)
+      const float S_row = S[rb * L + r_local];
+      S += kc * L;                                          // of the columns
+#pragma unroll 1
+      for (int cb = grp; cb < 4; cb += 2) {
+        const uint32_t tg = tG + lane_addr + (uint32_t)((m & 1) * L + 32 * cb);
+        uint32_t mh[16], ml[16];
+        if (cb > diag) {                                 // every column is past every row of this warp
 #pragma unroll
-              for (int e = 0; e < 16; ++e) { mh[e] = 0u; ml[e] = 0u; }
-            } else {
-              uint32_t r[32];
-              tmem_ld32(tg + (uint32_t)(half * 32), r);
+          for (int e = 0; e < 16; ++e) { mh[e] = 0u; ml[e] = 0u; }
+        } else {
+          uint32_t r[32];
+          tmem_ld32(tg, r);
+          if (FACT && cb < diag) {
+            // every column is before every row: exp(S_t - S_s) = exp(S_t - S_q) exp(S_q - S_s) with q the block's last column
+            const float rf = __expf(S_row - S[32 * cb + 31]);
 #pragma unroll
-              for (int e2 = 0; e2 < 16; ++e2) {
-                const int col = c0 + half * 32 + 2 * e2;
-                const float2 sv = *reinterpret_cast<const float2*>(Sc + col);
-                float m0 = __uint_as_float(r[2 * e2]) * __expf(S_row - sv.x), m1 = __uint_as_float(r[2 * e2 + 1]) * __expf(S_row - sv.y);
-                if (!below) { m0 = col <= r_local ? m0 : 0.0f; m1 = col + 1 <= r_local ? m1 : 0.0f; }
-                ml[e2] = 0u;
-                split2(m0, m1, mh[e2], ml[e2], ND == 2);
-              }
+            for (int e4 = 0; e4 < 8; ++e4) {
+              const float4 cf = *reinterpret_cast<const float4*>(S + L + 32 * cb + 4 * e4);
+              ml[2 * e4] = ml[2 * e4 + 1] = 0u;
+              split2(__uint_as_float(r[4 * e4]) * (rf * cf.x), __uint_as_float(r[4 * e4 + 1]) * (rf * cf.y), mh[2 * e4], ml[2 * e4], ND == 2);
+              split2(__uint_as_float(r[4 * e4 + 2]) * (rf * cf.z), __uint_as_float(r[4 * e4 + 3]) * (rf * cf.w), mh[2 * e4 + 1], ml[2 * e4 + 1], ND == 2);
             }
-            tmem_st16(tg + (uint32_t)(half * 32), mh);
-            if (ND == 2) tmem_st16(tg + (uint32_t)(half * 32 + 16), ml);
+          } else {
+#pragma unroll
+            for (int e2 = 0; e2 < 16; ++e2) {
+              const float2 sv = *reinterpret_cast<const float2*>(S + 32 * cb + 2 * e2);
+              float m0 = __uint_as_float(r[2 * e2]) * __expf(S_row - sv.x), m1 = __uint_as_float(r[2 * e2 + 1]) * __expf(S_row - sv.y);
+              if (FACT || cb == diag) { m0 = 2 * e2 <= lane ? m0 : 0.0f; m1 = 2 * e2 + 1 <= lane ? m1 : 0.0f; }
+              ml[e2] = 0u;
+              split2(m0, m1, mh[e2], ml[e2], ND == 2);
+            }
           }
-          tmem_wait_st();
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(MRDY + (m & 1)));
         }
+        tmem_st16(tg, mh);
+        if (ND == 2) tmem_st16(tg + 16u, ml);
       }
-      if (ok && first && k > 0) {
-        const int i = k;
-        const int col = h * p.P + 32 * grp + ec;
-        float2 x[4][2];                                     // the skip term's x of one 16-row half
-        auto fetch_x = [&](int rh) {
+      tmem_wait_st();
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(MRDY + (m & 1)));
+      if (kc == rb) { ++k; rb = rb + 1 == NB ? 0 : rb + 1; kc = 0; } else ++kc;
+    }
+  } else if (warp < W_XF) {
+    // ---------------- output: drains the accumulators of a step while the next one is masked ----------------
+    constexpr int NG = 8 / OUTW;                            // halves of the output columns that a warp takes
+    if (NG == 2) regs_inc<96>();
+    const int quarter = warp & 3, grp = NG == 1 ? (warp - W_OUT) >> 2 : 0;
+    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+    const float dv = p.D ? p.D[h] : 0.0f;
+    // fragments of 16 rows x 8 columns (a quad of lanes holds 8 columns of a row: whole 32-byte sectors per store): this thread's
+    // output rows are er + {0, 8, 16, 24}
+    const int er = quarter * 32 + (lane >> 2), cw = 32 * grp, col = h * p.P + cw + (lane & 3) * 2;
+    bool ok = !p.state_only;
+#pragma unroll 1
+    for (int k = 0; k < n && ok; ++k) {
+      const int c = k / NB;
+      const float* S = sS + (c % NSB) * GE::SLOT + (k % NB) * L;
+      const int t0 = toff + k * L + er;
+      float2 o[2][4 * NG][2];                               // [16-row half][8-column group][row, row + 8]
+      auto fetch_x = [&](int rh, int q, int e) -> float2 {  // the skip term's x
+        const int t = t0 + 16 * rh + 8 * e;
+        return p.D && t < p.T && cw + 8 * q < p.P ? *reinterpret_cast<const float2*>(p.x + (tokb + t) * p.ldx + col + 8 * q) : make_float2(0.0f, 0.0f);
+      };
+      if (!XIN16 && NG == 1) {                              // (requested ahead of the accumulators)
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int t = toff + (i - 1) * L + er + 16 * rh + 8 * e;
-            const float* xr = p.x + (tokb + t) * p.ldx + col;
+        for (int rh = 0; rh < 2; ++rh)
 #pragma unroll
-            for (int q = 0; q < 4; ++q)
-              x[q][e] = p.D && t < p.T && 32 * grp + 8 * q < p.P ? *reinterpret_cast<const float2*>(xr + 8 * q) : make_float2(0.0f, 0.0f);
-          }
-        };
-        fetch_x(0);                                         // (requested ahead of the accumulators)
-        ok = __all_sync(0xffffffffu, wait(ACCFULL, (uint32_t)(i - 1), 64u));
-        if (ok) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          // both accumulators into registers, combined, and handed back before anything waits for memory
-          float2 o[2][4][2];                                // [16-row half][8-column group][row, row + 8]
+          for (int e = 0; e < 2; ++e)
 #pragma unroll
-          for (int rh = 0; rh < 2; ++rh)
+            for (int q = 0; q < 4; ++q) o[rh][q][e] = fetch_x(rh, q, e);
+      }
+      ok = __all_sync(0xffffffffu, wait(SRDY + (c % NSB), (uint32_t)(c / NSB), 64u));
+      if (!ok) break;
+      float f[4];
 #pragma unroll
-            for (int c16 = 0; c16 < 2; ++c16) {
-              uint32_t a1[8], a2[8];
-              const uint32_t ta = lane_addr + ((uint32_t)(16 * rh) << 16) + (uint32_t)(32 * grp + 16 * c16);
-              tmem_ld16x256_x2(tA1 + ta, a1);
-              tmem_ld16x256_x2(tA2 + ta, a2);
-              tmem_wait_ld();
+      for (int e = 0; e < 4; ++e) f[e] = __expf(S[er + 8 * e]);
+      ok = __all_sync(0xffffffffu, wait(ACCFULL, (uint32_t)k, 64u));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-              for (int q = 0; q < 2; ++q)
+      for (int rh = 0; rh < 2; ++rh)
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                  const float f = fac[2 * rh + e];
-                  if (NI == 1 && !XIN16 && p.yoff) {
-                    const int t = toff + (i - 1) * L + er + 16 * rh + 8 * e;
-                    if (t < p.T && 32 * grp + 16 * c16 + 8 * q < p.P)
-                      *reinterpret_cast<float2*>(p.yoff + (tokb + t) * (int64_t)(p.H * p.P) + col + 16 * c16 + 8 * q) =
-                          make_float2(f * __uint_as_float(a2[4 * q + 2 * e]), f * __uint_as_float(a2[4 * q + 2 * e + 1]));
-                  }
-                  o[rh][2 * c16 + q][e] = make_float2(fmaf(f, __uint_as_float(a2[4 * q + 2 * e]), __uint_as_float(a1[4 * q + 2 * e])),
-                                                      fmaf(f, __uint_as_float(a2[4 * q + 2 * e + 1]), __uint_as_float(a1[4 * q + 2 * e + 1])));
-                }
-            }
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(ACCFREE));
+        for (int c16 = 0; c16 < 2 * NG; ++c16) {
+          uint32_t a1[8], a2[8];
+          const uint32_t ta = lane_addr + ((uint32_t)(16 * rh) << 16) + (uint32_t)(cw + 16 * c16);
+          tmem_ld16x256_x2(tA1 + ta, a1);
+          tmem_ld16x256_x2(tA2 + ta, a2);
+          tmem_wait_ld();
 #pragma unroll
-          for (int rh = 0; rh < 2; ++rh) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-#pragma unroll
-              for (int e = 0; e < 2; ++e) { o[rh][q][e].x = fmaf(dv, x[q][e].x, o[rh][q][e].x); o[rh][q][e].y = fmaf(dv, x[q][e].y, o[rh][q][e].y); }
-            if (rh == 0) fetch_x(1);
+          for (int q = 0; q < 2; ++q)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const int t = toff + (i - 1) * L + er + 16 * rh + 8 * e;
-              if (!p.y16 && t < p.T) {
-                float* yr = p.y + (tokb + t) * p.ldy + col;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) if (32 * grp + 8 * q < p.P) *reinterpret_cast<float2*>(yr + 8 * q) = o[rh][q][e];
+              const int r = 4 * q + 2 * e;
+              float2& v = o[rh][2 * c16 + q][e];
+              if (ND == 1 && !XIN16 && p.yoff) {
+                const int t = t0 + 16 * rh + 8 * e;
+                if (t < p.T && cw + 16 * c16 + 8 * q < p.P)
+                  *reinterpret_cast<float2*>(p.yoff + (tokb + t) * (int64_t)(p.H * p.P) + col + 16 * c16 + 8 * q) =
+                      make_float2(f[2 * rh + e] * __uint_as_float(a2[r]), f[2 * rh + e] * __uint_as_float(a2[r + 1]));
               }
-              if (p.y16) {
-                // neighbouring lanes swap halves, so that a lane writes four columns and a quad one whole sector
+              const float u0 = fmaf(f[2 * rh + e], __uint_as_float(a2[r]), __uint_as_float(a1[r])), u1 = fmaf(f[2 * rh + e], __uint_as_float(a2[r + 1]), __uint_as_float(a1[r + 1]));
+              v = XIN16 || NG == 2 ? make_float2(u0, u1) : make_float2(fmaf(dv, v.x, u0), fmaf(dv, v.y, u1));
+            }
+        }
+      // handed back before anything waits for memory
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(ACCFREE));
 #pragma unroll
-                for (int q = 0; q < 4; q += 2) {
-                  uint32_t v0, v1, z;
-                  split2(o[rh][q][e].x, o[rh][q][e].y, v0, z, false); split2(o[rh][q + 1][e].x, o[rh][q + 1][e].y, v1, z, false);
-                  const bool odd = lane & 1;
-                  const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
-                  const uint2 w = odd ? make_uint2(got, v1) : make_uint2(v0, got);
-                  // even lanes: columns ec .. ec + 3 of the first eight; odd lanes: ec - 2 .. ec + 1 of the second
-                  if (t < p.T && 32 * grp + 8 * (q + (odd ? 1 : 0)) < p.P)
-                    *reinterpret_cast<uint2*>(p.y16 + (tokb + t) * p.ldy + col + 8 * q + (odd ? 6 : 0)) = w;
-                }
-              }
+      for (int rh = 0; rh < 2; ++rh)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int t = t0 + 16 * rh + 8 * e;
+          if (!XIN16) {
+            if (NG == 2) {
+              float2 x[4 * NG];
+#pragma unroll
+              for (int q = 0; q < 4 * NG; ++q) x[q] = fetch_x(rh, q, e);
+#pragma unroll
+              for (int q = 0; q < 4 * NG; ++q) o[rh][q][e] = make_float2(fmaf(dv, x[q].x, o[rh][q][e].x), fmaf(dv, x[q].y, o[rh][q][e].y));
+            }
+            if (t < p.T) {
+              float* yr = p.y + (tokb + t) * p.ldy + col;
+#pragma unroll
+              for (int q = 0; q < 4 * NG; ++q) if (cw + 8 * q < p.P) *reinterpret_cast<float2*>(yr + 8 * q) = o[rh][q][e];
+            }
+          } else {
+            // neighbouring lanes swap halves, so that a lane writes four columns and a quad one whole sector
+#pragma unroll
+            for (int q = 0; q < 4 * NG; q += 2) {
+              uint32_t v0, v1, z;
+              split2(o[rh][q][e].x, o[rh][q][e].y, v0, z, false); split2(o[rh][q + 1][e].x, o[rh][q + 1][e].y, v1, z, false);
+              const bool odd = lane & 1;
+              const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
+              const uint2 w = odd ? make_uint2(got, v1) : make_uint2(v0, got);
+              // even lanes: the lane's columns and the next two of the first eight; odd lanes: the two before and its own of the second
+              if (t < p.T && cw + 8 * (q + (odd ? 1 : 0)) < p.P)
+                *reinterpret_cast<uint2*>(p.y16 + (tokb + t) * p.ldy + col + 8 * q + (odd ? 6 : 0)) = w;
             }
           }
         }
-      }
-      if (first) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) fac[e] = fnext[e];
-      }
-      if (cb == rb) { ++k; rb = rb + 1 == NB ? 0 : rb + 1; cb = 0; } else ++cb;
     }
   } else if (warp < W_ST) {
     // ---------------- transform: S of the step, x -> x~ and xs ----------------
-    regs_dec<72>();
+    if (XFW == 8) regs_dec<64>();
     const int wx = warp - W_XF, tid = threadIdx.x - 32 * W_XF;
     const float Ah = p.dt_raw ? -expf(p.a_log[h]) : (p.dt ? p.A[h] : 1.0f);
     const float bias = p.dt_raw ? p.dt_bias[h] : 0.0f;
     if (p.dt_raw && p.A_out && bb == 0 && tid == 0) p.A_out[h] = Ah;
     constexpr int LPR = XIN16 ? 8 : 16;                     // lanes per row, 16 bytes each
-    constexpr int RPI = 8 * (32 / LPR), NIT = L / RPI;      // rows per pass of the eight warps, passes
+    constexpr int RPI = XFW * (32 / LPR), NIT = L / RPI;    // rows per pass of the role, passes
     constexpr int EPL = XIN16 ? 8 : 4;                      // elements per lane
     const int j = lane % LPR, r0 = wx * (32 / LPR) + lane / LPR;
     const bool jcol = EPL * j < p.P;
@@ -467,9 +510,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     // (cp.async; no barrier; rows past the end arrive as zeros)
     constexpr int RING = GE::AHEAD > 0 ? GE::AHEAD : 1;
     const uint32_t xring = smem_u32(sfac + NB * L) + (uint32_t)tid * 16u;
-    const char* src = XIN16 ? reinterpret_cast<const char*>(p.x16 + (tokb + toff + r0) * p.ldx + h * p.P + (jcol ? EPL * j : 0))
-                            : reinterpret_cast<const char*>(p.x + (tokb + toff + r0) * p.ldx + h * p.P + (jcol ? EPL * j : 0));
-    const int64_t sstep = (int64_t)RPI * p.ldx * (XIN16 ? 2 : 4);
+    const char* src = reinterpret_cast<const char*>(p.x + (tokb + toff + r0) * p.ldx + h * p.P + (jcol ? EPL * j : 0));
+    const int64_t sstep = (int64_t)RPI * p.ldx * 4;
     int frow = toff + r0;                                          // row of the next piece to request
     auto request = [&](uint32_t slot) {
       const bool in = frow < p.T && jcol;
@@ -478,62 +520,80 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       frow += RPI;
       if (frow < p.T) src += sstep;                         // (the address stays inside the tensor)
     };
-    auto fetch_a = [&](int c) -> float {                    // of this thread's token of chunk c
-      const int t = toff + c * NB * L + tid;
-      if (tid >= NB * L || t >= p.T) return 0.0f;
-      const int64_t tk = tokb + t;
-      if (p.dt_raw) return p.dt_raw[tk * p.ld_raw + h];
-      return p.dt ? p.dt[tk * p.H + h] : p.a[tk * p.H + h];
+    constexpr int TPT = NB * L > XF_THREADS ? NB * L / XF_THREADS : 1;      // tokens of a chunk per thread
+    float av[TPT], an[TPT];                                 // requested two chunks ahead: the tokens of a head are a line apart
+    auto fetch_a = [&](int c, float (&av)[TPT]) {           // of this thread's tokens of chunk c
+#pragma unroll
+      for (int u = 0; u < TPT; ++u) {
+        const int t = toff + c * NB * L + u * XF_THREADS + tid;
+        const int64_t tk = tokb + t;
+        av[u] = 0.0f;
+        if (tid < NB * L && t < p.T) av[u] = p.dt_raw ? p.dt_raw[tk * p.ld_raw + h] : p.dt ? p.dt[tk * p.H + h] : p.a[tk * p.H + h];
+      }
     };
     if (GE::AHEAD > 0) {
-      if (frow >= p.T) { src = XIN16 ? reinterpret_cast<const char*>(p.x16) : reinterpret_cast<const char*>(p.x); }
+      if (frow >= p.T) src = reinterpret_cast<const char*>(p.x);
 #pragma unroll 1
       for (int q = 0; q < RING; ++q) request((uint32_t)q * (XF_THREADS * 16));
     }
-    float av = fetch_a(0);
+    fetch_a(0, av);
+    fetch_a(1, an);
     uint32_t slot = 0;
     bool ok = true;
     for (int i = 0; i < n; ++i) {
       const int c = i / NB, rb = i % NB;
-      float* S = sS + (c % NSB) * NB * L;
+      float* S = sS + (c % NSB) * GE::SLOT;
       if (rb == 0) {
         // S of the chunk.  A warp that gave up keeps reaching the named barriers: it skips the work, not the barrier.
-        const int t = toff + c * NB * L + tid;
-        const bool in = tid < NB * L && t < p.T;
-        float dtv = 1.0f, v = av;
-        if (p.dt_raw) { dtv = in ? softplus_acc(av + bias) : 0.0f; v = Ah * dtv; }
-        else if (p.dt) { dtv = av; v = Ah * av; }
+        float dtv[TPT], v[TPT];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) { const float u = __shfl_up_sync(0xffffffffu, v, o); if (lane >= o) v += u; }
-        if (lane == 31 && tid < NB * L) wsum[wx] = v;
-        asm volatile("bar.sync 4, 256;" ::: "memory");
+        for (int u = 0; u < TPT; ++u) {
+          const bool in = toff + c * NB * L + u * XF_THREADS + tid < p.T;
+          dtv[u] = 1.0f; v[u] = av[u];
+          if (p.dt_raw) { dtv[u] = in ? softplus_acc(av[u] + bias) : 0.0f; v[u] = Ah * dtv[u]; }
+          else if (p.dt) { dtv[u] = av[u]; v[u] = Ah * av[u]; }
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) { const float w = __shfl_up_sync(0xffffffffu, v[u], o); if (lane >= o) v[u] += w; }
+          if (lane == 31 && tid < NB * L) wsum[u * XFW + wx] = v[u];
+        }
+        asm volatile("bar.sync 4, %0;" ::"n"(XF_THREADS) : "memory");
         if (tid < NB * L) {
-          float off = 0.0f, send = 0.0f;                    // fixed order
+          float off[TPT], send = 0.0f;                      // fixed order
 #pragma unroll
-          for (int q = 0; q < 4 * NB; ++q) { if (q == wx) off = send; send += wsum[q]; }
-          v += off;
-          if (tid == NB * L - 1) v = send;
-          // (nobody reads the buffer's old content any more: this thread has waited for the last products of the step, with
-          // two operand buffers of the second last, before the block before this one; those products read tiles masked with it)
-          S[tid] = v;
-          if (GE::BIG) sdt[tid] = dtv; else sfac[tid] = make_float2(dtv, __expf(send - v));
-          if (tid == NB * L - 1) sEnd[c & 3] = send;
-          if (in) {
-            if (p.S_out && !p.state_only) p.S_out[((int64_t)bb * p.H + h) * p.T + t] = v;
-            if (p.dt_out && !p.state_only) p.dt_out[(tokb + t) * p.H + h] = dtv;
+          for (int q = 0; q < 4 * NB; ++q) { if (q % XFW == wx) off[q / XFW] = send; send += wsum[q]; }
+          // (nobody reads the buffer's old content any more: in the step before this one the thread has waited for the products of step
+          // i - 1 - XB, which follow the masking of that step and the draining of the one before, and with it of everything earlier)
+#pragma unroll
+          for (int u = 0; u < TPT; ++u) {
+            const int q = u * XF_THREADS + tid, t = toff + c * NB * L + q;
+            v[u] += off[u];
+            if (q == NB * L - 1) v[u] = send;
+            S[q] = v[u];
+            if (FACT) S[L + q] = __expf(__shfl_sync(0xffffffffu, v[u], 31) - v[u]);
+            if (GE::BIG) sdt[q] = dtv[u]; else sfac[q] = make_float2(dtv[u], __expf(send - v[u]));
+            if (q == NB * L - 1) sEnd[c & 3] = send;
+            if (t < p.T) {
+              if (p.S_out && !p.state_only) p.S_out[((int64_t)bb * p.H + h) * p.T + t] = v[u];
+              if (p.dt_out && !p.state_only) p.dt_out[(tokb + t) * p.H + h] = dtv[u];
+            }
           }
         }
-        asm volatile("bar.sync 4, 256;" ::: "memory");
+        asm volatile("bar.sync 4, %0;" ::"n"(XF_THREADS) : "memory");
         if (lane == 0) mbar_arrive(bar(SRDY + (c % NSB)));
-        if (i + NB < n) av = fetch_a(c + 1);
+#pragma unroll
+        for (int u = 0; u < TPT; ++u) av[u] = an[u];
+        if (i + 2 * NB < n) fetch_a(c + 2, an);
       }
-      if (ok && i >= XB) ok = __all_sync(0xffffffffu, wait(XFREE + (i % XB), (uint32_t)(i / XB - 1), 128u));
+      if (ok && XIN16) ok = __all_sync(0xffffffffu, wait(XIN + (i % XB), (uint32_t)(i / XB), 128u));
+      else if (ok && i >= XB) ok = __all_sync(0xffffffffu, wait(XFREE + (i % XB), (uint32_t)(i / XB - 1), 128u));
       if (ok) {
         uint32_t dst = xbuf_s + (i % XB) * GE::XBUF + place;
-#pragma unroll 2
+#pragma unroll (XIN16 ? 4 : 2)
         for (int it = 0; it < NIT; ++it, dst += RPI * 128) {
           uint4 xq = make_uint4(0u, 0u, 0u, 0u);
-          if (GE::AHEAD > 0) {
+          if (XIN16) {
+            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(xq.x), "=r"(xq.y), "=r"(xq.z), "=r"(xq.w) : "r"(dst));
+          } else if (GE::AHEAD > 0) {
             asm volatile("cp.async.wait_group %0;" ::"n"(RING - 1) : "memory");
             asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(xq.x), "=r"(xq.y), "=r"(xq.z), "=r"(xq.w) : "r"(xring + slot) : "memory");
           } else {
@@ -547,12 +607,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
             uint32_t s4[4], k4[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) split2(__uint_as_float(in4[e] << 16) * f.y, __uint_as_float(in4[e] & 0xffff0000u) * f.y, s4[e], k4[e], ND == 2);
-            st_shared_v4(dst, in4[0], in4[1], in4[2], in4[3]);
             st_shared_v4(dst + GE::XT, s4[0], s4[1], s4[2], s4[3]);
             if (ND == 2) st_shared_v4(dst + GE::XT + T128, k4[0], k4[1], k4[2], k4[3]);
-            // (the backward of the bf16 scan is not handed x again)
-            const int row = toff + i * L + it * RPI + r0;
-            if (p.x_keep && !p.state_only && jcol && row < p.T) *reinterpret_cast<uint4*>(p.x_keep + (tokb + row) * p.ldx + h * p.P + EPL * j) = xq;
           } else {
             const float f0 = __uint_as_float(xq.x) * f.x, f1 = __uint_as_float(xq.y) * f.x, f2 = __uint_as_float(xq.z) * f.x, f3 = __uint_as_float(xq.w) * f.x;
             uint32_t h0, h1, l0 = 0u, l1 = 0u, g0, g1, k0 = 0u, k1 = 0u;
@@ -579,7 +635,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     asm volatile("cp.async.wait_all;" ::: "memory");
   } else {
     // ---------------- state: h in registers (thread = row n of the state) ----------------
-    regs_inc<120>();
+    regs_inc<104>();
     const int quarter = warp & 3, nr = quarter * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const bool active = nr < p.N;                           // rows past d_state hold zeros
@@ -687,7 +743,7 @@ static unsigned int* status_ptr() {
 
 template <int NI, int ND, int NK, int NB, bool XIN16>
 static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
-  using GE = Geo<NI, ND, NK, NB>;
+  using GE = Geo<NI, ND, NK, NB, XIN16>;
   static_assert(GE::SMEM <= 227 * 1024, "shared-memory plan");
   static_assert(XIN16 ? NI == 1 : NI == ND, "fp32 tensors take pairs throughout or not at all");
   Maps ms{};
@@ -698,16 +754,18 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
   }
   Params p{};
   p.T = a.T; p.H = a.H; p.hpg = a.H / a.G; p.N = a.N; p.P = a.P; p.nsteps = (int)cdiv(a.T, L);
-  p.x = a.x; p.x16 = a.x16; p.ldx = a.ldx;
+  p.x = a.x; p.ldx = a.ldx;
   p.dt_raw = a.dt_raw; p.ld_raw = a.ld_raw; p.dt_bias = a.dt_bias; p.a_log = a.a_log; p.dt = a.dt; p.A = a.A; p.a = a.a; p.D = a.D;
   p.init = a.init; p.y = a.y; p.y16 = a.y16; p.ldy = a.ldy; p.dt_out = a.dt_out; p.A_out = a.A_out; p.S_out = a.S_out;
-  p.hprev = a.hprev; p.yoff = a.yoff; p.store_ops = a.xt != nullptr;
-  if (p.store_ops) {
+  p.hprev = a.hprev; p.yoff = a.yoff;
+  uint16_t* const keep = XIN16 ? a.x_keep : a.xt;
+  if (XIN16) PMB_TRY(sf::bf16_map4(&ms.x, a.x16, a.P, a.T, a.H, a.B, a.ldx, a.P, a.T * a.ldx, 64, L));
+  if (keep) {
     const int64_t hp = (int64_t)a.H * a.P;
-    PMB_TRY(sf::bf16_map4(&ms.xt, a.xt, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
-    PMB_TRY(sf::bf16_map4(&ms.xs, a.xs, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
+    PMB_TRY(sf::bf16_map4(&ms.xt, keep, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
+    if (!XIN16) PMB_TRY(sf::bf16_map4(&ms.xs, a.xs, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
   }
-  p.x_keep = a.x_keep; p.hp_hi = a.hp_hi; p.hp_lo = a.hp_lo; p.last = a.last; p.status = status_ptr();
+  p.hp_hi = a.hp_hi; p.hp_lo = a.hp_lo; p.last = a.last; p.status = status_ptr();
   p.nseg = 1; p.per = p.nsteps;
   if (NB == 1 && a.seg) {
     p.nseg = ssd_chain_segments(a.B, a.T, a.H, &p.per);
@@ -721,6 +779,7 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
     PMB_LAUNCHED();
     p.state_only = 0;
   }
+  p.store_ops = keep != nullptr;
   ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
   PMB_LAUNCHED();
   return PMB_OK;

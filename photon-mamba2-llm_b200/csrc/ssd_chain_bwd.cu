@@ -14,15 +14,22 @@
 // The row and column sums of W come from the same registers, so that the near-total cancellation in sum_t S_t dS_t (the gradient of
 // A) is between identically rounded numbers; <dY, y> - <x~, dx~> from separately rounded products loses it.
 //
-// warp 0 = TMA loads (B, C, h), 1 = MMA issuer, 2 = per-token gradients (da / ddt and the per-head sums), 3 = TMA stores of the bf16
-// operands x~ and dY that the sums over heads read, 4..11 = two mask groups (columns 0-63 / 64-127; then half of the output
-// columns each), 12..19 = transform (x -> x~, dY -> dY and dY exp(S), all into shared memory), 20..23 = state.
-// What bounds it: the mask warps (masked tile and sums of W, then three accumulators drained against x~ and dY), about 10 us per step;
-// GT and dMT of the next step form under the epilogue, the state chain and the loads under the masks.
-// Measured at 24 heads of 64 x 64 on pairs: 42 us for 4 x 512 tokens (the d(states) product, reverse pass, masked product and row
-// kernel it replaces: 118 us), 30 us for 2 x 384, 76 us for 2 x 1000 (1.7 ms of FMA contractions with ssd_heads.cu's share).
+// <dx~_s, x~_s>, which the gradient of dt needs, is the same sum over t >= s plus e_s: W's row sum with its diagonal.
+//
+// warp 0 = TMA loads (B, C, h, bf16 x and dY), 1 = products of the masked tile (GT, dMT, MT dY), 2 = per-token gradients (da / ddt and the
+// per-head sums), 3 = products of the state (B dh, C h, U) and TMA stores of the operands x~ and dY that the sums over heads read, 4..11 = two
+// mask groups of four warps, then the output of the same step, 12..19 = transform (x -> x~, dY -> dY and dY exp(S), into shared memory; bf16
+// x and dY are operands as they are), 20..23 = state.
+// What bounds it: instructions and their chains, 16800 warp instructions a step at d_state 128, issued in 43 % of the cycles.  On plain
+// operands mask (4100 clocks), MT dY and output (2300) follow one another; on pairs, whose one buffer of x~ and dY has to be drained first, the
+// transform (6500) comes on top.  Warps of their own for the output (28 of 72 registers) were no faster: 1317 us against 1271 for
+// 16 x 8192 tokens, 32 heads of 128 x 64 (1412 with one MMA warp, sums by 16 shuffles per 16 columns and an exponential per element), nor x and dY
+// prefetched into registers (50 us for 4 x 512 tokens, 24 heads of 64 x 64, on pairs) or read again by the output (49).
+// Measured at 24 heads of 64 x 64 on pairs: 43 us for 4 x 512 tokens (the d(states) product, reverse pass, masked product and row
+// kernel it replaces: 118 us), 31 us for 2 x 384, 76 us for 2 x 1000 (1.7 ms of FMA contractions with ssd_heads.cu's share).
 // Every mbarrier wait is bounded, as in the forward.
 #include <cuda_bf16.h>
+#include <type_traits>
 #include "tc_common.cuh"
 #include "kernels.h"
 #include "ssd_fused.h"
@@ -44,9 +51,9 @@ using namespace tcx;
 
 constexpr int L = SCAN_STEP, PW = 64, T128 = L * 128, T64 = 64 * 128;
 constexpr int W_MASK = 4, W_XF = 12, W_ST = 20, NTHREADS = 32 * 24, XF_THREADS = 256;
-// (shares of the block's 80 x 768 registers: 72, 2 x 80, 2 x 72 and 104 per thread of the six warpgroups)
+// (shares of the block's 80 x 768 registers: 56, 2 x 88, 2 x 72 and 104 per thread of the six warpgroups)
 
-template <int NI, int ND, int NK>
+template <int NI, int ND, int NK, bool IN16>
 struct Geo {
   static constexpr int BT = NI * NK * T128;              // B (or C)
   static constexpr int HT = ND * NK * T64;               // h, dh: rows n of 128 bytes
@@ -55,19 +62,20 @@ struct Geo {
   static constexpr int XBUF = 2 * XT + ND * T128;        // [x~ | dY | dY exp(S)]
   static constexpr int XB = ND == 1 ? 2 : 1;
   static constexpr int NSB = XB + 2;
-  static constexpr int AHEAD = 2;                        // pieces of x and of dY that a transform thread has in flight
+  static constexpr int AHEAD = IN16 ? 0 : 2;             // fp32: pieces of x and of dY that a transform thread has in flight (bf16: the tiles are copied as they are)
   static constexpr int TILES = STAGE + XB * XBUF + HT;
-  static constexpr int ROWS = 12 * L;                    // per-row sums: [2 groups] of W, e, f, <dx~, x~>; [4 quarters] column sums of W
-  static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 512 /*barriers, small sums*/ + (2 * NSB * L + 2 * ROWS) * 4 + 2 * AHEAD * XF_THREADS * 16;
+  static constexpr int ROWS = 11 * L;                    // per-row sums: [2 groups] of W, e, f; W[s,s]; [4 quarters] column sums of W
+  static constexpr int SLOT = 3 * L;                     // a step's [S | dt | column factors]
+  static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 512 /*barriers, small sums*/ + (NSB * SLOT + 2 * ROWS) * 4 + 2 * AHEAD * XF_THREADS * 16;
 };
 
-struct Maps { CUtensorMap b[2], c[2], h[2], xt[2], dy[2]; };      // [0] = hi (or the plain bf16 tensor), [1] = lo
+struct Maps { CUtensorMap b[2], c[2], h[2], xt[2], dy[2]; };      // [0] = hi (or the plain bf16 tensor), [1] = lo; bf16: xt and dy are the inputs
 
 struct Params {
   int T, H, hpg, N, P, nsteps;
   const float* S;                                        // (B,H,T)
-  const float* x; const uint16_t* x16; int64_t ldx;
-  const float* dy; const uint16_t* dy16; int64_t lddy;
+  const float* x; int64_t ldx;                           // fp32
+  const float* dy; int64_t lddy;
   const float* dt; const float* A;                       // (B,T,H), (H); NULL: x~ = x and da is the result
   const float* D;
   float* dx; uint16_t* dx16; int64_t lddx;
@@ -85,25 +93,25 @@ struct Params {
 __device__ __forceinline__ uint32_t ld_shared(uint32_t a) { uint32_t v; asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a)); return v; }
 __device__ __forceinline__ float2 bf2(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
 
-// On entry every lane holds its row's values for 16 consecutive columns; on exit lane l holds the sum of column l & 15 over the
-// warp's 32 rows.  Fixed order.
-__device__ __forceinline__ float warp_column_sums16(float (&v)[16], int lane) {
+// On entry v[2 o + c] is a lane's sum over its four rows of column 8 o + 2 (lane & 3) + c of 32; on exit the lane returns the sum over the
+// warp's 32 rows of the column column_of(lane).  Fixed order.
+__device__ __forceinline__ float warp_column_sums32(float (&v)[8], int lane) {
 #pragma unroll
-  for (int w = 8; w >= 1; w >>= 1) {
-    const bool upper = (lane & w) != 0;
+  for (int w = 4; w >= 1; w >>= 1) {
+    const bool upper = (lane & (4 * w)) != 0;
 #pragma unroll
     for (int k = 0; k < w; ++k) {
-      const float keep = upper ? v[k + w] : v[k];
-      const float send = upper ? v[k] : v[k + w];
-      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+      const float keep = upper ? v[k + w] : v[k], send = upper ? v[k] : v[k + w];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, 4 * w);
     }
   }
-  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
+  return v[0];
 }
+__device__ __forceinline__ int column_of(int lane) { return 8 * (lane >> 3) + 2 * (lane & 3) + ((lane >> 2) & 1); }
 
 template <int NI, int ND, int NK, bool IN16>
 __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
-  using GE = Geo<NI, ND, NK>;
+  using GE = Geo<NI, ND, NK, IN16>;
   constexpr int XB = GE::XB, NSB = GE::NSB;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -111,27 +119,28 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
   uint8_t* base_ptr = smem_raw + (base - raw);
   const uint32_t b_s = base, c_s = b_s + GE::BT, hin_s = c_s + GE::BT, xbuf_s = base + GE::STAGE, dh_s = xbuf_s + XB * GE::XBUF, bars = dh_s + GE::HT;
   enum { FULL = 0, EMPTY, XRDY /*2*/, XFREE = XRDY + 2 /*2*/, SRDY = XFREE + 2 /*4*/, GFULL = SRDY + 4, MRDY, ACCFULL, ACCFREE, UFULL, UFREE, HRDY, HFREE,
-         RRDY /*2*/, RFREE = RRDY + 2 /*2*/, NBAR = RFREE + 2 };
-  static_assert(8 * NBAR + 16 + 64 <= 512 && NSB <= 4, "barrier block");
+         RRDY /*2*/, RFREE = RRDY + 2 /*2*/, XIN = RFREE + 2 /*2*/, NBAR = XIN + 2 };
+  static_assert(8 * NBAR + 16 + 80 <= 512 && NSB <= 4, "barrier block");
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
   uint8_t* bar_ptr = base_ptr + (bars - base);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 8 * NBAR);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   float* ddw = reinterpret_cast<float*>(bar_ptr + 8 * NBAR + 16);      // [2 steps][4 state warps] <dh, h>
   float* dDw = ddw + 8;                                                // [8 transform warps] <dY, x>
-  float* sS = reinterpret_cast<float*>(bar_ptr + 512);                 // [NSB] S and dt of a step's tokens
-  float* sRows = sS + 2 * NSB * L;                                     // [2 steps] per-row sums
+  float* sWend = dDw + 8;                                              // [4 transform warps] S of their last token
+  float* sS = reinterpret_cast<float*>(bar_ptr + 512);                 // [NSB] S, dt and column factor exp(S_t - S_q) of a step's tokens, q = the last one before the token's 32
+  float* sRows = sS + NSB * GE::SLOT;                                     // [2 steps] per-row sums
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int bh = (int)blockIdx.x / p.nseg, seg = (int)blockIdx.x % p.nseg;
   const int h = bh % p.H, bb = bh / p.H, g = h / p.hpg;
   const int n = min(p.per, p.nsteps - seg * p.per), last = seg * p.per + n - 1;      // steps of this CTA's segment, the last one of them
   const int64_t tokb = (int64_t)bb * p.T;
   if (threadIdx.x == 0) {
-    mbar_init(bar(FULL), 1); mbar_init(bar(EMPTY), p.state_only ? 1 : 5);
-    for (int i = 0; i < 2; ++i) { mbar_init(bar(XRDY + i), 8); mbar_init(bar(XFREE + i), p.state_only ? 1 : 10); mbar_init(bar(RRDY + i), 12); mbar_init(bar(RFREE + i), 1); }
+    mbar_init(bar(FULL), 1); mbar_init(bar(EMPTY), p.state_only ? 1 : 6);
+    for (int i = 0; i < 2; ++i) { mbar_init(bar(XIN + i), 1); mbar_init(bar(XRDY + i), 8); mbar_init(bar(XFREE + i), p.state_only ? 1 : IN16 ? 10 : 11); mbar_init(bar(RRDY + i), 12); mbar_init(bar(RFREE + i), 1); }
     for (int i = 0; i < 4; ++i) mbar_init(bar(SRDY + i), 8);
-    mbar_init(bar(GFULL), 1); mbar_init(bar(MRDY), 8); mbar_init(bar(ACCFULL), 1); mbar_init(bar(ACCFREE), 8);
+    mbar_init(bar(GFULL), 1); mbar_init(bar(MRDY), 8); mbar_init(bar(ACCFULL), 2); mbar_init(bar(ACCFREE), 8);
     mbar_init(bar(UFULL), 1); mbar_init(bar(UFREE), 4); mbar_init(bar(HRDY), 4); mbar_init(bar(HFREE), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -150,6 +159,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
   auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
   // bounded waits that also end as soon as another role of the CTA has given up
   auto wait = [&](int b, uint32_t parity, unsigned int code) -> bool {
+    if (mbar_wait(bar(b), parity & 1u, 1u)) return true;
     if (*abort_flag) return false;
     if (mbar_wait(bar(b), parity & 1u)) return true;
     give_up(code);
@@ -159,13 +169,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
 
   // k = 0, 1, ... counts the steps as they are walked; step last - k of the sequence
   if (warp < W_MASK) {
-    regs_dec<72>();
+    regs_dec<56>();
     if (warp == 0) {
       // ---------------- TMA producer: B, C and the entering state ----------------
       if (lane == 0) {
         int issued = 0;
+        int xissued = 0;
+        // bf16: the operand tiles x~ and dY are the inputs as they are (two buffers: room for a step's is there before that for its other tiles)
+        auto xload = [&](int k) -> bool {
+          const int xb = k % XB;
+          if (!wait(XFREE + xb, (uint32_t)(k / XB) ^ 1u, 4096u)) return false;
+          mbar_expect_tx(bar(XIN + xb), (p.state_only ? 1 : 2) * T128);
+          if (!p.state_only) tma_load_4d(xbuf_s + xb * GE::XBUF, &maps.xt[0], 0, (last - k) * L, h, bb, bar(XIN + xb));
+          tma_load_4d(xbuf_s + xb * GE::XBUF + GE::XT, &maps.dy[0], 0, (last - k) * L, h, bb, bar(XIN + xb));
+          xissued = k + 1;
+          return true;
+        };
         for (int k = 0; k < n; ++k) {
           const int i = last - k;
+          if (IN16 && XB == 2 && !xload(k)) break;
           if (!wait(EMPTY, (uint32_t)k ^ 1u, 1u)) break;
           mbar_expect_tx(bar(FULL), p.state_only ? GE::BT : GE::STAGE);
 #pragma unroll
@@ -180,86 +202,121 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
               if (!p.state_only) tma_load_4d(hin_s + (sp * NK + kt) * T64, &maps.h[sp], 0, 64 * kt, h, bb * p.nsteps + i, bar(FULL));
           }
           issued = k + 1;
+          if (IN16 && XB == 1 && !xload(k)) break;
         }
         if (*abort_flag && issued > 0) mbar_wait(bar(FULL), (uint32_t)((issued - 1) & 1));
+        if (IN16 && *abort_flag)
+          for (int k = (xissued > XB ? xissued - XB : 0); k < xissued; ++k) mbar_wait(bar(XIN + k % XB), (uint32_t)((k / XB) & 1));
       }
-    } else if (warp == 1) {
-      // ---------------- MMA issuer (the whole warp waits; one elected lane issues) ----------------
+    } else if (warp == 1 || warp == 3) {
+      // ---------------- MMA issuers (the whole warp waits; one elected lane issues) ----------------
       const uint32_t dhi = desc_hi(1024, 2);
       const uint32_t id_g = idesc_bf16(0, 0, L, L);            // both operands K-major
       const uint32_t id_v = idesc_bf16(0, 1, L, PW);           // B operand MN-major
       const uint32_t id_u = idesc_bf16(1, 1, L, PW);           // both operands MN-major
       const uint32_t BS = (NK * T128) >> 4, HS = (NK * T64) >> 4, XS = T128 >> 4;      // from a hi tile to its lo tile
-      bool ok = true;
+      bool ok = !(warp == 1 && p.state_only);
 #pragma unroll 1
       for (int k = 0; k < n && ok; ++k) {
         const int xb = k % XB;
         const uint32_t xt_s = xbuf_s + xb * GE::XBUF, dy_s = xt_s + GE::XT, dys_s = dy_s + GE::XT;
-        if (!(ok = all(wait(FULL, (uint32_t)k, 2u) && wait(XRDY + xb, (uint32_t)(k / XB), 2u)))) break;
+        auto xready = [&]() -> bool { return all(wait(XRDY + xb, (uint32_t)(k / XB), 2u) && (!IN16 || wait(XIN + xb, (uint32_t)(k / XB), 2u))); };
+        if (!(ok = all(wait(FULL, (uint32_t)k, 2u)))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (!p.state_only) {
-        // (both accumulators were read by the mask warps before they reported the last tile; the products that read the masked
-        // tile over GT were issued before this)
-        if (elect_one()) {
-          const uint32_t b0 = desc_lo(b_s, 16), c0 = desc_lo(c_s, 16), x0 = desc_lo(xt_s, 16), y0 = desc_lo(dy_s, 16);
+        if (warp == 1) {
+          // the masked tile's: GT and dMT (both accumulators were read by the mask warps before they reported the last tile; the products that
+          // read the masked tile over GT were issued before this)
+          if (elect_one()) {
+            const uint32_t b0 = desc_lo(b_s, 16), c0 = desc_lo(c_s, 16);
 #pragma unroll
-          for (int kt = 0; kt < NK; ++kt)
+            for (int kt = 0; kt < NK; ++kt)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const uint32_t o = (uint32_t)(kt * T128 + q * 32) >> 4;
-              mma_split<NI, NI>(tG, b0 + o, BS, c0 + o, BS, dhi, id_g, (kt | q) ? 1u : 0u);
-            }
-#pragma unroll
-          for (int q = 0; q < 4; ++q) mma_split<NI, NI>(tM, x0 + 2 * q, XS, y0 + 2 * q, XS, dhi, id_g, q ? 1u : 0u);
-          umma_commit(bar(GFULL));
-        }
-        __syncwarp();
-        }
-        // U = C^T (exp(S) dY): the step's contribution to the state's adjoint (with one 64-wide block of d_state the second half
-        // of M reads the tile behind it and its rows of U are never looked at)
-        if (!(ok = all(k == 0 || wait(UFREE, (uint32_t)(k - 1), 4u)))) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (elect_one()) {
-          const uint32_t c0 = desc_lo(c_s, T128), y0 = desc_lo(dys_s, T128);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) mma_split<NI, ND>(tU, c0 + ((uint32_t)(q * 2048) >> 4), BS, y0 + ((uint32_t)(q * 2048) >> 4), XS, dhi, id_u, q ? 1u : 0u);
-          umma_commit(bar(UFULL));
-          if (p.state_only) { umma_commit(bar(EMPTY)); umma_commit(bar(XFREE + xb)); }
-        }
-        __syncwarp();
-        if (p.state_only) continue;
-        // B dh and C h
-        if (!(ok = all(wait(HRDY, (uint32_t)k, 8u) && (k == 0 || wait(ACCFREE, (uint32_t)(k - 1), 8u))))) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (elect_one()) {
-          const uint32_t b0 = desc_lo(b_s, 16), c0 = desc_lo(c_s, 16), d0 = desc_lo(dh_s, T64), h0 = desc_lo(hin_s, T64);
-#pragma unroll
-          for (int kt = 0; kt < NK; ++kt)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const uint32_t oa = (uint32_t)(kt * T128 + q * 32) >> 4, ob = (uint32_t)(kt * T64 + q * 2048) >> 4;
-              mma_split<NI, ND>(tA2, b0 + oa, BS, d0 + ob, HS, dhi, id_v, (kt | q) ? 1u : 0u);
-              mma_split<NI, ND>(tA3, c0 + oa, BS, h0 + ob, HS, dhi, id_v, (kt | q) ? 1u : 0u);
-            }
-          umma_commit(bar(HFREE));
-          umma_commit(bar(EMPTY));
-        }
-        __syncwarp();
-        // MT dY, the masked tile read from TMEM: per 16 columns [hi: 8 | lo: 8]
-        if (!(ok = all(wait(MRDY, (uint32_t)k, 16u)))) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (elect_one()) {
-          const uint32_t y0 = desc_lo(dy_s, T128);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            const uint32_t ta = tG + (uint32_t)(16 * q), vb = y0 + ((uint32_t)(q * 2048) >> 4);
-            mma_split_ts<ND, NI>(tA1, ta, 8u, vb, XS, dhi, id_v, q ? 1u : 0u);
+              for (int q = 0; q < 4; ++q) {
+                const uint32_t o = (uint32_t)(kt * T128 + q * 32) >> 4;
+                mma_split<NI, NI>(tG, b0 + o, BS, c0 + o, BS, dhi, id_g, (kt | q) ? 1u : 0u);
+              }
+            umma_commit(bar(EMPTY));
           }
-          umma_commit(bar(ACCFULL));
-          umma_commit(bar(XFREE + xb));
+          __syncwarp();
+          if (!(ok = xready())) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (elect_one()) {
+            const uint32_t x0 = desc_lo(xt_s, 16), y0 = desc_lo(dy_s, 16);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) mma_split<NI, NI>(tM, x0 + 2 * q, XS, y0 + 2 * q, XS, dhi, id_g, q ? 1u : 0u);
+            umma_commit(bar(GFULL));
+          }
+          __syncwarp();
+          // MT dY, the masked tile read from TMEM: per 32 columns [hi: 16 | lo: 16], 8 columns per k-step of 16
+          if (!(ok = all((k == 0 || wait(ACCFREE, (uint32_t)(k - 1), 8u)) && wait(MRDY, (uint32_t)k, 16u)))) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (elect_one()) {
+            const uint32_t y0 = desc_lo(dy_s, T128);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+              const uint32_t ta = tG + (uint32_t)((q >> 1) * 32 + (q & 1) * 8), vb = y0 + ((uint32_t)(q * 2048) >> 4);
+              mma_split_ts<ND, NI>(tA1, ta, 16u, vb, XS, dhi, id_v, q ? 1u : 0u);
+            }
+            umma_commit(bar(ACCFULL));
+            umma_commit(bar(XFREE + xb));
+          }
+          __syncwarp();
+        } else {
+          // the state's: B dh and C h, and U
+          auto carried = [&]() -> bool {
+                        if (!all(wait(HRDY, (uint32_t)k, 8u) && (k == 0 || wait(ACCFREE, (uint32_t)(k - 1), 8u)))) return false;
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        if (elect_one()) {
+                          const uint32_t b0 = desc_lo(b_s, 16), c0 = desc_lo(c_s, 16), d0 = desc_lo(dh_s, T64), h0 = desc_lo(hin_s, T64);
+            #pragma unroll
+                          for (int kt = 0; kt < NK; ++kt)
+            #pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                              const uint32_t oa = (uint32_t)(kt * T128 + q * 32) >> 4, ob = (uint32_t)(kt * T64 + q * 2048) >> 4;
+                              mma_split<NI, ND>(tA2, b0 + oa, BS, d0 + ob, HS, dhi, id_v, (kt | q) ? 1u : 0u);
+                              mma_split<NI, ND>(tA3, c0 + oa, BS, h0 + ob, HS, dhi, id_v, (kt | q) ? 1u : 0u);
+                            }
+                          umma_commit(bar(ACCFULL));
+                          umma_commit(bar(HFREE));
+              if (XB == 2) umma_commit(bar(EMPTY));
+                        }
+                        __syncwarp();
+            return true;
+          };
+          auto update = [&]() -> bool {
+                      if (!(xready() && all(k == 0 || wait(UFREE, (uint32_t)(k - 1), 4u)))) return false;
+                      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                      // U = C^T (exp(S) dY): the step's contribution to the state's adjoint (with one 64-wide block of d_state the second half
+                      // of M reads the tile behind it and its rows of U are never looked at)
+                      if (elect_one()) {
+                        const uint32_t cm = desc_lo(c_s, T128), y0 = desc_lo(dys_s, T128);
+            #pragma unroll
+                        for (int q = 0; q < 8; ++q) mma_split<NI, ND>(tU, cm + ((uint32_t)(q * 2048) >> 4), BS, y0 + ((uint32_t)(q * 2048) >> 4), XS, dhi, id_u, q ? 1u : 0u);
+                        umma_commit(bar(UFULL)); umma_commit(bar(XFREE + xb));
+              if (XB == 1 || p.state_only) umma_commit(bar(EMPTY));
+                      }
+                      __syncwarp();
+            return true;
+          };
+          // (two buffers: exp(S) dY has been there for a while, and the state's chain does not wait for the draining; one: it is being formed)
+          if (!(ok = p.state_only ? update() : XB == 2 ? update() && carried() : carried() && update())) break;
+          if (!IN16 && !p.state_only && lane == 0) {
+            // x~ and dY go out as the operands that the sums over heads read
+            if (p.store_ops) {
+#pragma unroll
+              for (int sp = 0; sp < NI; ++sp) {
+                tma_store_4d(&maps.xt[sp], xt_s + sp * T128, 0, (last - k) * L, h, bb);
+                tma_store_4d(&maps.dy[sp], dy_s + sp * T128, 0, (last - k) * L, h, bb);
+              }
+              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+              asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            }
+            mbar_arrive(bar(XFREE + xb));
+          }
+          __syncwarp();
         }
-        __syncwarp();
       }
+      if (!IN16 && warp == 3 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     } else if (p.state_only) {
     } else if (warp == 2) {
       // ---------------- per-token gradients (lane = four consecutive tokens) ----------------
@@ -270,12 +327,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
         const int i = last - k;
         if (!all(wait(SRDY + (k % NSB), (uint32_t)(k / NSB), 1024u) && wait(RRDY + (k & 1), (uint32_t)(k >> 1), 1024u))) break;
         const float4* R = reinterpret_cast<const float4*>(sRows + (k & 1) * GE::ROWS) + lane;
-        const float* S = sS + (k % NSB) * 2 * L;
+        const float* S = sS + (k % NSB) * GE::SLOT;
         const float4 S4 = reinterpret_cast<const float4*>(S)[lane], dt4 = reinterpret_cast<const float4*>(S + L)[lane];
         const float send = S[L - 1];
         auto two = [&](int a) { const float4 u = R[a * 32], v = R[(a + 1) * 32]; return make_float4(u.x + v.x, u.y + v.y, u.z + v.z, u.w + v.w); };
-        const float4 r4 = two(0), e4 = two(2), f4 = two(4), q4 = two(6), ca = two(8), cb = two(10);
-        const float Sv[4] = {S4.x, S4.y, S4.z, S4.w}, dtv[4] = {dt4.x, dt4.y, dt4.z, dt4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
+        const float4 r4 = two(0), e4 = two(2), f4 = two(4), w4 = R[6 * 32], ca = two(7), cb = two(9);
+        const float Sv[4] = {S4.x, S4.y, S4.z, S4.w}, dtv[4] = {dt4.x, dt4.y, dt4.z, dt4.w};
+        float qv[4] = {r4.x + w4.x, r4.y + w4.y, r4.z + w4.z, r4.w + w4.w};      // <dx~_s, x~_s> = sum_{t >= s} W[s,t] + e_s
         float d[4] = {ca.x + cb.x - r4.x, ca.y + cb.y - r4.y, ca.z + cb.z - r4.z, ca.w + cb.w - r4.w};
         const float ev[4] = {e4.x, e4.y, e4.z, e4.w}, fv[4] = {f4.x, f4.y, f4.z, f4.w};
         float es = 0.0f;
@@ -283,6 +341,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
         for (int j = 0; j < 4; ++j) {
           const float e = __expf(send - Sv[j]) * ev[j];
           es += e;
+          qv[j] += e;
           d[j] += __expf(Sv[j]) * fv[j] - e;
         }
         es = warp_sum(es);
@@ -321,167 +380,209 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
         // (row of `part`: segment by segment of a sequence)
         if (lane == 0) { const int64_t o = ((int64_t)bb * p.nseg + seg) * p.H + h; p.part[o] = accA; p.part[2 * p.part_pitch + o] = accB; }
       }
-    } else {
-      // ---------------- stores of the operands that the sums over heads read ----------------
-      if (lane == 0) {
-        for (int k = 0; k < n; ++k) {
-          const int xb = k % XB, i = last - k;
-          if (!wait(XRDY + xb, (uint32_t)(k / XB), 2048u)) break;
-          if (p.store_ops) {
-#pragma unroll
-            for (int sp = 0; sp < NI; ++sp) {
-              tma_store_4d(&maps.xt[sp], xbuf_s + xb * GE::XBUF + sp * T128, 0, i * L, h, bb);
-              tma_store_4d(&maps.dy[sp], xbuf_s + xb * GE::XBUF + GE::XT + sp * T128, 0, i * L, h, bb);
-            }
-            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-          }
-          mbar_arrive(bar(XFREE + xb));
-        }
-        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-      }
     }
   } else if (warp < W_XF) {
-    // ---------------- mask groups, then the epilogue of the same step ----------------
-
-    const int quarter = warp & 3, grp = (warp - W_MASK) >> 2, r_local = quarter * 32 + lane;
+    regs_inc<88>();
+    const int quarter = warp & 3, grp = (warp - W_MASK) >> 2;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const bool dtm = p.dt != nullptr;
     const float dv = p.D ? p.D[h] : 0.0f;
-    const int er = quarter * 32 + (lane >> 2), ec = (lane & 3) * 2;
-    bool ok = !p.state_only;
-    for (int k = 0; k < n && ok; ++k) {
-      const int xb = k % XB, i = last - k;
+    const int er = quarter * 32 + (lane >> 2), ec = (lane & 3) * 2, cw = 32 * grp;
+    constexpr int PPR = 2;                                  // output pieces of 16 rows
+    // ---------------- output of a step: half of the columns, in pieces of 16 rows x 16 columns, fragments of 16 x 8 (whole 32-byte
+    // sectors per store) ----------------
+    auto output = [&](int k) -> bool {
       float* R = sRows + (k & 1) * GE::ROWS;
-      const float* S = sS + (k % NSB) * 2 * L;
-      ok = all((k < 2 || wait(RFREE + (k & 1), (uint32_t)((k >> 1) - 1), 32u)) && wait(SRDY + (k % NSB), (uint32_t)(k / NSB), 32u) &&
-               wait(GFULL, (uint32_t)k, 32u));
-      if (!ok) break;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      {
-        const float S_row = S[r_local];
-        float rsum = 0.0f;
-#pragma unroll 1
-        for (int ch = 0; ch < 4; ++ch) {
-          const int c0 = grp * 64 + ch * 16;
-          uint32_t m[16];
-          float cs = 0.0f;
-          if (c0 + 15 < quarter * 32) {                     // every column is before every row of this warp
+      const float* S = sS + (k % NSB) * GE::SLOT;
+      const int xb = k % XB, i = last - k;
+      const uint32_t xt_s = xbuf_s + xb * GE::XBUF, dy_s = xt_s + GE::XT;
+      auto fetch = [&](int pc, float2 (&xo)[2][2], float2 (&yo)[2][2]) {
+        const int rh = pc / PPR, c16 = pc % PPR;
 #pragma unroll
-            for (int e = 0; e < 16; ++e) m[e] = 0u;
-          } else {
-            uint32_t gr[16], dr[16];
-            tmem_ld16(tG + lane_addr + (uint32_t)c0, gr);
-            tmem_ld16(tM + lane_addr + (uint32_t)c0, dr);
-            tmem_wait_ld();
-            float w[16];
+        for (int q = 0; q < 2; ++q)
 #pragma unroll
-            for (int e2 = 0; e2 < 8; ++e2) {
-              const int col = c0 + 2 * e2;
-              const float2 sv = *reinterpret_cast<const float2*>(S + col);
-              float m0 = __uint_as_float(gr[2 * e2]) * __expf(sv.x - S_row), m1 = __uint_as_float(gr[2 * e2 + 1]) * __expf(sv.y - S_row);
-              m0 = col >= r_local ? m0 : 0.0f;
-              m1 = col + 1 >= r_local ? m1 : 0.0f;
-              w[2 * e2] = col > r_local ? m0 * __uint_as_float(dr[2 * e2]) : 0.0f;
-              w[2 * e2 + 1] = col + 1 > r_local ? m1 * __uint_as_float(dr[2 * e2 + 1]) : 0.0f;
-              rsum += w[2 * e2];
-              rsum += w[2 * e2 + 1];
-              split2(m0, m1, m[e2], m[8 + e2], ND == 2);
-              if (ND == 1) m[8 + e2] = 0u;
+          for (int e = 0; e < 2; ++e) {
+            const uint32_t at = (uint32_t)((er + 16 * rh + 8 * e) * 128) + (uint32_t)(((4 * grp + 2 * c16 + q) ^ (lane >> 2)) << 4) + (uint32_t)((lane & 3) * 4);
+            xo[q][e] = bf2(ld_shared(xt_s + at)); yo[q][e] = bf2(ld_shared(dy_s + at));
+            if (NI == 2) {
+              const float2 xl = bf2(ld_shared(xt_s + T128 + at)), yl = bf2(ld_shared(dy_s + T128 + at));
+              xo[q][e].x += xl.x; xo[q][e].y += xl.y; yo[q][e].x += yl.x; yo[q][e].y += yl.y;
             }
-            cs = warp_column_sums16(w, lane);
           }
-          tmem_st16(tG + lane_addr + (uint32_t)c0, m);
-          if (lane < 16) R[(8 + quarter) * L + c0 + lane] = cs;
-        }
-        R[grp * L + r_local] = rsum;
-        tmem_wait_st();
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(MRDY));
-      }
-      // epilogue: fragments of 16 rows x 8 columns (whole 32-byte sectors per store)
-      ok = all(wait(XRDY + xb, (uint32_t)(k / XB), 64u) && wait(ACCFULL, (uint32_t)k, 64u));
-      if (!ok) break;
+      };
+      if (!all(wait((IN16 ? XIN : XRDY) + xb, (uint32_t)(k / XB), 64u) && wait(ACCFULL, (uint32_t)k, 64u))) return false;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const float send = S[L - 1];
-      const uint32_t xt_s = xbuf_s + xb * GE::XBUF, dy_s = xt_s + GE::XT;
-      const int colb = h * p.P + 32 * grp + ec;
+      float fx[2], dtr[2], es[2], fs[2];
 #pragma unroll 1
-      for (int rh = 0; rh < 2; ++rh) {
-        float fx[2], dtr[2], es[2] = {0.0f, 0.0f}, fs[2] = {0.0f, 0.0f}, qs[2] = {0.0f, 0.0f};
+      for (int pc0 = 0; pc0 < 2 * PPR; pc0 += 2) {
+        if (pc0 % PPR == 0) {
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          fx[e] = __expf(send - S[er + 16 * rh + 8 * e]);
-          dtr[e] = dtm ? S[L + er + 16 * rh + 8 * e] : 1.0f;
+          for (int e = 0; e < 2; ++e) {
+            const int row = er + 16 * (pc0 / PPR) + 8 * e;
+            fx[e] = __expf(send - S[row]);
+            dtr[e] = dtm ? S[L + row] : 1.0f;
+            es[e] = fs[e] = 0.0f;
+          }
         }
-        float2 o[4][2];
 #pragma unroll
-        for (int c16 = 0; c16 < 2; ++c16) {
+        for (int u = 0; u < 2; ++u) {
+          const int pc = pc0 + u, rh = pc / PPR, c16 = pc % PPR;
+          float2 xn[2][2], yn[2][2];                        // [8-column group][row, row + 8]
+          fetch(pc, xn, yn);
           uint32_t a1[8], a2[8], a3[8];
-          const uint32_t ta = lane_addr + ((uint32_t)(16 * rh) << 16) + (uint32_t)(32 * grp + 16 * c16);
+          const uint32_t ta = lane_addr + ((uint32_t)(16 * rh) << 16) + (uint32_t)(cw + 16 * c16);
           tmem_ld16x256_x2(tA1 + ta, a1);
           tmem_ld16x256_x2(tA2 + ta, a2);
           tmem_ld16x256_x2(tA3 + ta, a3);
           tmem_wait_ld();
+          float2 o[2][2];
 #pragma unroll
           for (int q = 0; q < 2; ++q)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const uint32_t at = (uint32_t)((er + 16 * rh + 8 * e) * 128) + (uint32_t)(((4 * grp + 2 * c16 + q) ^ (lane >> 2)) << 4) + (uint32_t)((lane & 3) * 4);
-              float2 xv = bf2(ld_shared(xt_s + at)), yv = bf2(ld_shared(dy_s + at));
-              if (NI == 2) {
-                const float2 xl = bf2(ld_shared(xt_s + T128 + at)), yl = bf2(ld_shared(dy_s + T128 + at));
-                xv.x += xl.x; xv.y += xl.y; yv.x += yl.x; yv.y += yl.y;
-              }
               const int r = 4 * q + 2 * e;
+              const float2 yv = yn[q][e], xv = xn[q][e];
               const float u0 = __uint_as_float(a2[r]), u1 = __uint_as_float(a2[r + 1]);
               const float d0 = fmaf(fx[e], u0, __uint_as_float(a1[r])), d1 = fmaf(fx[e], u1, __uint_as_float(a1[r + 1]));
               es[e] = fmaf(u0, xv.x, fmaf(u1, xv.y, es[e]));
               fs[e] = fmaf(__uint_as_float(a3[r]), yv.x, fmaf(__uint_as_float(a3[r + 1]), yv.y, fs[e]));
-              qs[e] = fmaf(d0, xv.x, fmaf(d1, xv.y, qs[e]));
-              o[2 * c16 + q][e] = make_float2(fmaf(d0, dtr[e], dv * yv.x), fmaf(d1, dtr[e], dv * yv.y));
+              o[q][e] = make_float2(fmaf(d0, dtr[e], dv * yv.x), fmaf(d1, dtr[e], dv * yv.y));
             }
-        }
-        if (rh == 1) {
-          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-          __syncwarp();
-          if (lane == 0) { mbar_arrive(bar(ACCFREE)); mbar_arrive(bar(XFREE + xb)); }
-        }
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-#pragma unroll
-          for (int s = 1; s < 4; s <<= 1) {                 // the quad of lanes that shares a row
-            es[e] += __shfl_xor_sync(0xffffffffu, es[e], s);
-            fs[e] += __shfl_xor_sync(0xffffffffu, fs[e], s);
-            qs[e] += __shfl_xor_sync(0xffffffffu, qs[e], s);
+          if (pc == 2 * PPR - 1) {
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) { mbar_arrive(bar(ACCFREE)); mbar_arrive(bar(XFREE + xb)); }
           }
-          const int row = er + 16 * rh + 8 * e;
-          if ((lane & 3) == 0) { R[(2 + grp) * L + row] = es[e]; R[(4 + grp) * L + row] = fs[e]; R[(6 + grp) * L + row] = qs[e]; }
-          const int t = i * L + row;
-          if (!IN16) {
-            if (t < p.T) {
-              float* dr = p.dx + (tokb + t) * p.lddx + colb;
 #pragma unroll
-              for (int q = 0; q < 4; ++q) if (32 * grp + 8 * q < p.P) *reinterpret_cast<float2*>(dr + 8 * q) = o[q][e];
-            }
-          } else {
-            // neighbouring lanes swap halves, so that a lane writes four columns and a quad one whole sector
+          for (int e = 0; e < 2; ++e) {
+            const int t = i * L + er + 16 * rh + 8 * e;
+            if (!IN16) {
+              if (t < p.T) {
+                float* dr = p.dx + (tokb + t) * p.lddx + h * p.P + cw + 16 * c16 + ec;
 #pragma unroll
-            for (int q = 0; q < 4; q += 2) {
+                for (int q = 0; q < 2; ++q) if (cw + 16 * c16 + 8 * q < p.P) *reinterpret_cast<float2*>(dr + 8 * q) = o[q][e];
+              }
+            } else {
+              // neighbouring lanes swap halves, so that a lane writes four columns and a quad one whole sector
               uint32_t v0, v1, z;
-              split2(o[q][e].x, o[q][e].y, v0, z, false); split2(o[q + 1][e].x, o[q + 1][e].y, v1, z, false);
+              split2(o[0][e].x, o[0][e].y, v0, z, false); split2(o[1][e].x, o[1][e].y, v1, z, false);
               const bool odd = lane & 1;
               const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? v0 : v1, 1);
               const uint2 wv = odd ? make_uint2(got, v1) : make_uint2(v0, got);
-              if (t < p.T && 32 * grp + 8 * (q + (odd ? 1 : 0)) < p.P)
-                *reinterpret_cast<uint2*>(p.dx16 + (tokb + t) * p.lddx + colb + 8 * q + (odd ? 6 : 0)) = wv;
+              if (t < p.T && cw + 16 * c16 + (odd ? 8 : 0) < p.P)
+                *reinterpret_cast<uint2*>(p.dx16 + (tokb + t) * p.lddx + h * p.P + cw + 16 * c16 + ec + (odd ? 6 : 0)) = wv;
             }
+          }
+        }
+        if (pc0 % PPR == PPR - 2) {
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+#pragma unroll
+            for (int w = 1; w < 4; w <<= 1) {               // the quad of lanes that shares a row
+              es[e] += __shfl_xor_sync(0xffffffffu, es[e], w);
+              fs[e] += __shfl_xor_sync(0xffffffffu, fs[e], w);
+            }
+            const int row = er + 16 * (pc0 / PPR) + 8 * e;
+            if ((lane & 3) == 0) { R[(2 + grp) * L + row] = es[e]; R[(4 + grp) * L + row] = fs[e]; }
           }
         }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(RRDY + (k & 1)));
+      return true;
+    };
+    // ---------------- mask groups: blocks of 32 columns, group g those of index g and g + 2 ----------------
+    // Fragments of 16 rows x 8 columns: a lane holds rows fr + {0, 8, 16, 24} of the warp's 32 and two adjacent columns of every eight, so
+    // a column's sum over the warp takes four additions in the lane and three exchanges of a halving number of columns.
+    const int fr = lane >> 2, fc = 2 * (lane & 3);
+    bool ok = !p.state_only;
+#pragma unroll 1
+    for (int k = 0; k < n && ok; ++k) {
+      float* R = sRows + (k & 1) * GE::ROWS;
+      const float* S = sS + (k % NSB) * GE::SLOT;
+      ok = all((k < 2 || wait(RFREE + (k & 1), (uint32_t)((k >> 1) - 1), 32u)) && wait(SRDY + (k % NSB), (uint32_t)(k / NSB), 32u) &&
+               wait(GFULL, (uint32_t)k, 32u));
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      float Sr[4], rs[4] = {0.0f, 0.0f, 0.0f, 0.0f};        // rows fr + 8 e
+#pragma unroll
+      for (int e = 0; e < 4; ++e) Sr[e] = S[quarter * 32 + fr + 8 * e];
+#pragma unroll 1
+      for (int cb = grp; cb < 4; cb += 2) {
+        const uint32_t tb = lane_addr + (uint32_t)(32 * cb);
+        float cs[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) cs[e] = 0.0f;
+        if (cb < quarter) {                                 // every column is before every row of this warp
+          uint32_t z[16];
+#pragma unroll
+          for (int e = 0; e < 16; ++e) z[e] = 0u;
+          tmem_st16(tG + tb, z);
+          if (ND == 2) tmem_st16(tG + tb + 16u, z);
+        } else {
+          // past the diagonal (every column past every row): exp(S_t - S_s) = exp(S_t - S_q) exp(S_q - S_s), q = the last token before the columns
+          auto block = [&](auto diagonal) {
+            constexpr bool DIAG = decltype(diagonal)::value;
+            float rf[4];
+            if (!DIAG) {
+              const float sq = S[32 * cb - 1];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) rf[e] = __expf(sq - Sr[e]);
+            }
+            const float* Sc = S + (DIAG ? 0 : 2 * L) + 32 * cb + fc;      // S, or the columns' factors
+#pragma unroll
+            for (int rh = 0; rh < 2; ++rh) {
+              const uint32_t at = tb + ((uint32_t)(16 * rh) << 16);
+              uint32_t gr[16], dr[16], mh[8], ml[8];
+              tmem_ld16x256_x4(tG + at, gr);
+              tmem_ld16x256_x4(tM + at, dr);
+              tmem_wait_ld();
+#pragma unroll
+              for (int o = 0; o < 4; ++o) {
+                const float2 sv = *reinterpret_cast<const float2*>(Sc + 8 * o);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                  const int r = 4 * o + 2 * e;
+                  float m0, m1, w0, w1;
+                  if (!DIAG) {
+                    m0 = __uint_as_float(gr[r]) * (rf[2 * rh + e] * sv.x); m1 = __uint_as_float(gr[r + 1]) * (rf[2 * rh + e] * sv.y);
+                    w0 = m0 * __uint_as_float(dr[r]); w1 = m1 * __uint_as_float(dr[r + 1]);
+                  } else {
+                    const int d = 8 * o + fc - (fr + 8 * e + 16 * rh);    // column - row
+                    m0 = __uint_as_float(gr[r]) * __expf(sv.x - Sr[2 * rh + e]); m1 = __uint_as_float(gr[r + 1]) * __expf(sv.y - Sr[2 * rh + e]);
+                    m0 = d >= 0 ? m0 : 0.0f; m1 = d >= -1 ? m1 : 0.0f;
+                    w0 = d >= 0 ? m0 * __uint_as_float(dr[r]) : 0.0f; w1 = d >= -1 ? m1 * __uint_as_float(dr[r + 1]) : 0.0f;
+                    if (o == 2 * rh + e && (d == 0 || d == -1)) {          // (the diagonal lies in the fragments on it)
+                      R[6 * L + quarter * 32 + fr + 8 * o] = d == 0 ? w0 : w1;
+                      if (d == 0) w0 = 0.0f; else w1 = 0.0f;
+                    }
+                  }
+                  rs[2 * rh + e] += w0 + w1;
+                  cs[2 * o] += w0; cs[2 * o + 1] += w1;
+                  ml[2 * o + e] = 0u;
+                  split2(m0, m1, mh[2 * o + e], ml[2 * o + e], ND == 2);
+                }
+              }
+              tmem_st16x128_x4(tG + at, mh);
+              if (ND == 2) tmem_st16x128_x4(tG + at + 16u, ml);
+            }
+          };
+          if (cb == quarter) block(std::true_type{}); else block(std::false_type{});
+        }
+        R[(7 + quarter) * L + 32 * cb + column_of(lane)] = cb < quarter ? 0.0f : warp_column_sums32(cs, lane);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        rs[e] += __shfl_xor_sync(0xffffffffu, rs[e], 1);
+        rs[e] += __shfl_xor_sync(0xffffffffu, rs[e], 2);
+        if ((lane & 3) == e) R[grp * L + quarter * 32 + fr + 8 * e] = rs[e];
+      }
+      tmem_wait_st();
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar(MRDY));
+      ok = output(k);
     }
   } else if (warp < W_ST) {
     // ---------------- transform: x -> x~, dY -> dY and dY exp(S) ----------------
@@ -489,7 +590,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
     const int wx = warp - W_XF, tid = threadIdx.x - 32 * W_XF;
     const bool dtm = p.dt != nullptr;
     constexpr int LPR = IN16 ? 8 : 16;                      // lanes per row, 16 bytes each
-    constexpr int RPI = 8 * (32 / LPR), NIT = L / RPI;      // rows per pass of the eight warps, passes
+    constexpr int RPI = 8 * (32 / LPR), NIT = L / RPI;    // rows per pass of the role, passes
     constexpr int EPL = IN16 ? 8 : 4;                       // elements per lane
     constexpr int AHEAD = GE::AHEAD;
     const int j = lane % LPR, r0 = wx * (32 / LPR) + lane / LPR;
@@ -499,18 +600,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
     // barrier; rows past the end and columns past d_head arrive as zeros)
     const uint32_t ring = smem_u32(sRows + 2 * GE::ROWS) + (uint32_t)tid * 16u;
     constexpr uint32_t SLOT = 2 * XF_THREADS * 16;          // [x | dY]
-    const int esz = IN16 ? 2 : 4;
-    const char* xsrc = (IN16 ? reinterpret_cast<const char*>(p.x16) : reinterpret_cast<const char*>(p.x)) + (int64_t)(h * p.P + (jcol ? EPL * j : 0)) * esz;
-    const char* ysrc = (IN16 ? reinterpret_cast<const char*>(p.dy16) : reinterpret_cast<const char*>(p.dy)) + (int64_t)(h * p.P + (jcol ? EPL * j : 0)) * esz;
-    int rk = 0, rit = 0;                                    // the next piece to request: step and pass
+    constexpr int esz = 4;
+    const char* xsrc = reinterpret_cast<const char*>(p.x) + (int64_t)(h * p.P + (jcol ? EPL * j : 0)) * esz;
+    const char* ysrc = reinterpret_cast<const char*>(p.dy) + (int64_t)(h * p.P + (jcol ? EPL * j : 0)) * esz;
+    int rrow = last * L + r0, rit = 0;                      // row and pass of the next piece to request; rows are walked up inside a step
     auto request = [&](uint32_t slot) {
-      if (rk < n) {
-        const int row = (last - rk) * L + rit * RPI + r0;
-        const bool in = row < p.T && jcol;
-        const int64_t tk = tokb + (row < p.T ? row : p.T - 1);      // (the address stays inside the tensor)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + slot), "l"(xsrc + tk * p.ldx * esz), "r"(in ? 16 : 0) : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + slot + XF_THREADS * 16), "l"(ysrc + tk * p.lddy * esz), "r"(in ? 16 : 0) : "memory");
-        if (++rit == NIT) { rit = 0; ++rk; }
+      if (rrow >= (last - n + 1) * L) {
+        const bool in = rrow < p.T && jcol;
+        const int64_t tk = tokb + (rrow < p.T ? rrow : p.T - 1);      // (the address stays inside the tensor)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + slot), "l"(xsrc + tk * (p.ldx * esz)), "r"(in ? 16 : 0) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + slot + XF_THREADS * 16), "l"(ysrc + tk * (p.lddy * esz)), "r"(in ? 16 : 0) : "memory");
+        rrow += RPI;
+        if (++rit == NIT) { rit = 0; rrow -= 2 * L; }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -522,6 +623,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       s_next = Sg[t < p.T ? t : p.T - 1];                   // (a = 0 past the end)
       if (dtm) d_next = t < p.T ? p.dt[(tokb + t) * p.H + h] : 0.0f;
     };
+    if (!IN16)
 #pragma unroll 1
     for (int q = 0; q < AHEAD; ++q) request((uint32_t)q * SLOT);
     fetch_s(0);
@@ -530,21 +632,30 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
     bool ok = true;
     for (int k = 0; k < n; ++k) {
       const int xb = k % XB;
-      float* S = sS + (k % NSB) * 2 * L;
-      if (ok && k >= XB) ok = all(wait(XFREE + xb, (uint32_t)(k / XB - 1), 128u));
-      // (whoever reads the ring's old entry has finished: NSB - XB - 1 steps lie between it and the step just freed)
-      if (ok && tid < L) { S[tid] = s_next; S[L + tid] = d_next; }
-      asm volatile("bar.sync 4, 256;" ::: "memory");        // (a warp that gave up keeps reaching the named barrier)
+      float* S = sS + (k % NSB) * GE::SLOT;
+      if (ok && IN16) ok = all(wait(XIN + xb, (uint32_t)(k / XB), 128u));
+      else if (ok && k >= XB) ok = all(wait(XFREE + xb, (uint32_t)(k / XB - 1), 128u));
+      // (whoever reads the ring's old entry, of step k - NSB, has finished: the products of step k - XB, whose buffer was just freed, follow
+      // the draining of step k - XB - 1 and its row sums wait for nobody that is further behind)
+      const float sv = s_next;
+      if (ok && tid < L) { S[tid] = sv; S[L + tid] = d_next; }
+      if (lane == 31 && tid < L) sWend[wx] = sv;
+      asm volatile("bar.sync 4, %0;" ::"n"(256) : "memory");        // (a warp that gave up keeps reaching the named barriers)
+      if (ok && tid < L) S[2 * L + tid] = __expf(sv - sWend[wx > 0 ? wx - 1 : 0]);
+      asm volatile("bar.sync 4, %0;" ::"n"(256) : "memory");
       if (!ok) continue;
       if (lane == 0) mbar_arrive(bar(SRDY + (k % NSB)));
       fetch_s(k + 1);
       uint32_t dst = xbuf_s + xb * GE::XBUF + place;
-#pragma unroll 2
+#pragma unroll (IN16 ? 4 : 2)
       for (int it = 0; it < NIT; ++it, dst += RPI * 128) {
-        uint4 xq, yq;
-        asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD - 1) : "memory");
+        uint4 xq = make_uint4(0u, 0u, 0u, 0u), yq;
+        if (IN16) asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(yq.x), "=r"(yq.y), "=r"(yq.z), "=r"(yq.w) : "r"(dst + GE::XT));
+        else {
+        asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD > 0 ? AHEAD - 1 : 0) : "memory");
         asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(xq.x), "=r"(xq.y), "=r"(xq.z), "=r"(xq.w) : "r"(ring + slot) : "memory");
         asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(yq.x), "=r"(yq.y), "=r"(yq.z), "=r"(yq.w) : "r"(ring + slot + XF_THREADS * 16) : "memory");
+        }
         const int row = it * RPI + r0;
         const float f = __expf(S[row]);
         if (IN16) {
@@ -552,8 +663,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
           uint32_t s4[4], k4[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) { const float2 v = bf2(y4[e]); split2(v.x * f, v.y * f, s4[e], k4[e], ND == 2); }
-          st_shared_v4(dst, xq.x, xq.y, xq.z, xq.w);
-          st_shared_v4(dst + GE::XT, yq.x, yq.y, yq.z, yq.w);
           st_shared_v4(dst + 2 * GE::XT, s4[0], s4[1], s4[2], s4[3]);
           if (ND == 2) st_shared_v4(dst + 2 * GE::XT + T128, k4[0], k4[1], k4[2], k4[3]);
         } else {
@@ -573,8 +682,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
 #pragma unroll
           for (int e = 0; e < 4; ++e) dD = fmaf(xv[e], yv[e], dD);
         }
-        request(slot);                                      // (this pass has consumed the slot)
-        slot = slot + SLOT == AHEAD * SLOT ? 0u : slot + SLOT;
+        if (!IN16) {
+          request(slot);                                    // (this pass has consumed the slot)
+          slot = slot + SLOT == AHEAD * SLOT ? 0u : slot + SLOT;
+        }
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
@@ -660,7 +771,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       ok = all(wait(SRDY + (k % NSB), (uint32_t)(k / NSB), 512u) && wait(UFULL, (uint32_t)k, 512u));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const float send = sS[(k % NSB) * 2 * L + L - 1], dec = __expf(send);
+      const float send = sS[(k % NSB) * GE::SLOT + L - 1], dec = __expf(send);
       stot += send;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
@@ -707,7 +818,7 @@ static unsigned int* status_ptr() {
 
 template <int NI, int ND, int NK, bool IN16>
 static pmb_status launch(cudaStream_t st, const ChainBwdArgs& a) {
-  using GE = Geo<NI, ND, NK>;
+  using GE = Geo<NI, ND, NK, IN16>;
   static_assert(GE::SMEM <= 227 * 1024, "shared-memory plan");
   static_assert(IN16 ? NI == 1 : NI == ND, "fp32 tensors take pairs throughout");
   const int n = (int)cdiv(a.T, L);
@@ -718,14 +829,18 @@ static pmb_status launch(cudaStream_t st, const ChainBwdArgs& a) {
     PMB_TRY(sf::bf16_map4(&ms.b[sp], lo ? a.b.lo : a.b.hi, a.N, a.T, a.G, a.B, a.b.pitch, a.N, (int64_t)a.T * a.b.pitch, 64, L));
     PMB_TRY(sf::bf16_map4(&ms.c[sp], lo ? a.c.lo : a.c.hi, a.N, a.T, a.G, a.B, a.c.pitch, a.N, (int64_t)a.T * a.c.pitch, 64, L));
     PMB_TRY(sf::bf16_map4(&ms.h[sp], lod ? a.hp_lo : a.hp_hi, a.P, a.N, a.H, (int64_t)a.B * n, a.P, st_h, a.H * st_h, 64, 64));
-    if (a.xt_hi) {
+    if (IN16 && !sp) {
+      PMB_TRY(sf::bf16_map4(&ms.xt[0], a.x16, a.P, a.T, a.H, a.B, a.ldx, a.P, a.T * a.ldx, 64, L));
+      PMB_TRY(sf::bf16_map4(&ms.dy[0], a.dy16, a.P, a.T, a.H, a.B, a.lddy, a.P, a.T * a.lddy, 64, L));
+    }
+    if (!IN16 && a.xt_hi) {
       PMB_TRY(sf::bf16_map4(&ms.xt[sp], lo ? a.xt_lo : a.xt_hi, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
       PMB_TRY(sf::bf16_map4(&ms.dy[sp], lo ? a.dyo_lo : a.dyo_hi, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
     }
   }
   Params p{};
   p.T = a.T; p.H = a.H; p.hpg = a.H / a.G; p.N = a.N; p.P = a.P; p.nsteps = n;
-  p.S = a.S; p.x = a.x; p.x16 = a.x16; p.ldx = a.ldx; p.dy = a.dy; p.dy16 = a.dy16; p.lddy = a.lddy; p.dt = a.dt; p.A = a.A; p.D = a.D;
+  p.S = a.S; p.x = a.x; p.ldx = a.ldx; p.dy = a.dy; p.lddy = a.lddy; p.dt = a.dt; p.A = a.A; p.D = a.D;
   p.dx = a.dx; p.dx16 = a.dx16; p.lddx = a.lddx; p.store_ops = a.xt_hi != nullptr; p.dh_hi = a.dh_hi; p.dh_lo = a.dh_lo; p.da = a.da;
   p.raw_hi = a.raw_hi; p.raw_lo = a.raw_lo; p.ld_raw = a.ld_raw; p.raw_col = a.raw_col; p.part = a.part; p.status = status_ptr();
   p.nseg = 1; p.per = n;

@@ -421,3 +421,23 @@ def test_conv_backward_strips(pm, B, T, K, H, P, N):
     dxzd, dw, db = pm.conv_silu_bwd(cfg, xzd.detach().cuda(), w.detach().cuda(), b.detach().cuda(), dact.cuda())
     for got, want, what in ((dxzd[..., I:I + X], xzd.grad[..., I:I + X], "dx"), (dw, w.grad, "dw"), (db, b.grad, "db")):
         assert_close(got, want, tol=1e-5, what=what)
+
+
+# decays that underflow inside a step of 128 tokens: the scan's masked tiles are formed by factors of 32-token blocks, each of which is a
+# decay of its own.  bf16 inputs (rounded and kept as pairs), ragged and whole lengths, segments; as in the tests above.
+@pytest.mark.parametrize("T,Q", [(128, 128), (200, 128), (512, 128), (1500, 256), (2048, 256)])
+@pytest.mark.parametrize("N,strength", [(64, 3.0), (128, 30.0)])
+def test_scan_bf16_strong_decay(pm, T, Q, N, strength):
+    B, H, P = 1, 4, 64
+    x, b, c, dy = randn((B, T, H, P), 1).bfloat16(), randn((B, T, 1, N), 2).bfloat16(), randn((B, T, 1, N), 3).bfloat16(), randn((B, T, H, P), 4).bfloat16()
+    a = -strength * torch.nn.functional.softplus(randn((B, T, H), 5) - 1.0)
+    scan = pm.SsdScanBf16(x.cuda(), a.cuda(), b.cuda(), c.cuda(), Q)
+    y = scan.forward()
+    dx, da, db, dc = scan.backward(dy.cuda())
+    assert pm.device_status() == 0
+    leaves = [t.double().requires_grad_(True) for t in (x, a, b, c)]
+    orc.ssd_scan_chunked(leaves[0], leaves[1], *(t.expand(B, T, H, N) for t in leaves[2:]), Q if T % Q == 0 else T).backward(dy.double())
+    ref = orc.ssd_scan_chunked(*(t.detach() for t in leaves[:2]), *(t.detach().expand(B, T, H, N) for t in leaves[2:]), Q if T % Q == 0 else T)
+    for got, want, tol, what in ((y.float(), ref, 5e-3, "y"), (dx.float(), leaves[0].grad, 5e-3, "dx"), (da, leaves[1].grad, 1e-3, "da"),
+                                 (db.float(), leaves[2].grad, 5e-3, "db"), (dc.float(), leaves[3].grad, 5e-3, "dc")):
+        assert_close(got, want, tol=tol, what=what)
