@@ -93,6 +93,35 @@ struct DeviceOnce {
     }                                                                                                            \
   } while (0)
 
+// Programmatic dependent launch.  A kernel launched with launch_pdl may be placed, and run what it does before pdl_wait(), while the kernel
+// before it in the stream is still at work: from the point on at which every CTA of that one has called pdl_launch() or ended.  pdl_wait()
+// returns when the kernels it depends on have completed and their memory is visible, so every thread calls it before it touches memory that
+// any other kernel writes or reads; a kernel then completes after all its predecessors, as without this.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A kernel that is placed early holds its registers and shared memory while it waits.  Where another stream has work for those SMs that costs
+// more than the launch it hides: inside a PdlPause launches of this thread are ordinary ones.
+inline thread_local int g_pdl_paused = 0;
+struct PdlPause {
+  const bool on;
+  explicit PdlPause(bool pause) : on(pause) { g_pdl_paused += on; }
+  ~PdlPause() { g_pdl_paused -= on; }
+  PdlPause(const PdlPause&) = delete;
+  PdlPause& operator=(const PdlPause&) = delete;
+};
+template <class... Params, class... Args>
+inline pmb_status launch_pdl(cudaStream_t st, void (*kernel)(Params...), dim3 grid, unsigned block, size_t smem, const Args&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = g_pdl_paused ? 0 : 1;
+  PMB_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
+  PMB_LAUNCHED();
+  return PMB_OK;
+}
+
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 

@@ -28,8 +28,6 @@ pmb_status read_clear_device_status_decode(unsigned int* word) {
 
 namespace dec {
 
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // conv window (B,X,K-1) fp32: oldest column first (state.rs:31-51).  Shifts the window and returns silu(conv).
 __device__ __forceinline__ float conv_step(float* __restrict__ win, const float* __restrict__ w, float bias, float xn, int K) {
@@ -519,20 +517,6 @@ extern "C" size_t pmb_mamba2_step_workspace_bytes(const pmb_mamba2_config* cfg, 
   Dims d;
   if (make_dims(cfg, batch, 1, &d) != PMB_OK) return 0;
   return step_ws_layout(d, nullptr, 0, nullptr);
-}
-
-// launch with programmatic dependence on the kernel before it (see the head of the file)
-template <class... Params, class... Args>
-static pmb_status launch_pdl(cudaStream_t st, void (*kernel)(Params...), dim3 grid, unsigned block, size_t smem, Args... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid; cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr; cfg.numAttrs = 1;
-  PMB_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
-  PMB_LAUNCHED();
-  return PMB_OK;
 }
 
 constexpr size_t GEMV_MAX_SMEM = 200 * 1024;

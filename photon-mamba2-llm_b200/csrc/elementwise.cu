@@ -103,6 +103,8 @@ template <int K>
 __global__ void __launch_bounds__(CONV_STRIP_THREADS) conv_silu_fwd_strip_kernel(const float* __restrict__ xzd, int64_t ldx, int col0,
                                                                                  const float* __restrict__ w, const float* __restrict__ bias,
                                                                                  float* __restrict__ act, int X, int T, int run, ConvPairOut po) {
+  pdl_launch();
+  pdl_wait();
   const int c = (blockIdx.x * 8 + (threadIdx.x & 7)) * 4;
   const int tblocks = (T + CONV_SLICES * run - 1) / (CONV_SLICES * run);
   const int b = blockIdx.y / tblocks, t0 = (blockIdx.y % tblocks) * (CONV_SLICES * run) + (threadIdx.x >> 3) * run;
@@ -112,6 +114,8 @@ __global__ void __launch_bounds__(CONV_STRIP_THREADS) conv_silu_fwd_strip_kernel
 template <int K>
 __global__ void __launch_bounds__(128) conv_silu_fwd_kernel(const float* __restrict__ xzd, int64_t ldx, int col0, const float* __restrict__ w,
                                                             const float* __restrict__ bias, float* __restrict__ act, int X, int T, int run) {
+  pdl_launch();
+  pdl_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int tblocks = (T + run - 1) / run;
   const int b = blockIdx.y / tblocks, t0 = (blockIdx.y % tblocks) * run;
@@ -139,12 +143,11 @@ static pmb_status launch_conv_fwd_k(cudaStream_t st, const Dims& d, const float*
   }
   if (vec) {
     dim3 grid((unsigned)cdiv(d.X, 32), (unsigned)(d.B * cdiv(d.T, CONV_SLICES * run)));
-    conv_silu_fwd_strip_kernel<K><<<grid, CONV_STRIP_THREADS, 0, st>>>(xzd, d.J, d.I, w, b, act, d.X, d.T, run, po);
+    PMB_TRY(launch_pdl(st, conv_silu_fwd_strip_kernel<K>, grid, CONV_STRIP_THREADS, 0, xzd, d.J, d.I, w, b, act, d.X, d.T, run, po));
   } else {
     dim3 grid((unsigned)cdiv(d.X, 128), (unsigned)(d.B * cdiv(d.T, run)));
-    conv_silu_fwd_kernel<K><<<grid, 128, 0, st>>>(xzd, d.J, d.I, w, b, act, d.X, d.T, run);
+    PMB_TRY(launch_pdl(st, conv_silu_fwd_kernel<K>, grid, 128, 0, xzd, d.J, d.I, w, b, act, d.X, d.T, run));
   }
-  PMB_LAUNCHED();
   return PMB_OK;
 }
 
@@ -295,6 +298,8 @@ __global__ void __launch_bounds__(128) conv_silu_bwd_kernel(const float* __restr
                                                             const float* __restrict__ dact, float* __restrict__ dxzd,
                                                             float* __restrict__ partial, int X, int T, int run,
                                                             uint16_t* __restrict__ pair_hi, uint16_t* __restrict__ pair_lo) {
+  pdl_launch();
+  pdl_wait();
   int c = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (c >= X) return;
   int tblocks = (T + run - 1) / run;
@@ -321,6 +326,8 @@ __global__ void __launch_bounds__(CONV_STRIP_THREADS, 7) conv_silu_bwd_strip_ker
                                                                   const float* __restrict__ dact, float* __restrict__ dxzd,
                                                                   float* __restrict__ partial, int X, int T, int run,
                                                                   uint16_t* __restrict__ pair_hi, uint16_t* __restrict__ pair_lo) {
+  pdl_launch();
+  pdl_wait();
   constexpr int NV = 2 * K + 2, NW = CONV_STRIP_THREADS / 32;
   __shared__ float red[NW][16][NV];
   __shared__ __align__(16) uint8_t stage[CONV_BWD_AHEAD * CONV_BWD_SLOT];
@@ -388,13 +395,12 @@ static pmb_status launch_conv_bwd_k(cudaStream_t st, const Dims& d, const float*
   const int run = strip ? conv_run(d, CONV_BWD_SLICES) : conv_run(d);
   if (strip) {
     if constexpr (K <= 4)
-      conv_silu_bwd_strip_kernel<K><<<dim3((unsigned)cdiv(d.X, 32), rows), CONV_STRIP_THREADS, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, run, pair_hi, pair_lo);
+      PMB_TRY(launch_pdl(st, conv_silu_bwd_strip_kernel<K>, dim3((unsigned)cdiv(d.X, 32), rows), CONV_STRIP_THREADS, 0, xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, run, pair_hi, pair_lo));
   } else if (vec) {
-    conv_silu_bwd_kernel<K, 4><<<dim3((unsigned)cdiv(d.X / 4, 128), rows), 128, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, run, pair_hi, pair_lo);
+    PMB_TRY(launch_pdl(st, conv_silu_bwd_kernel<K, 4>, dim3((unsigned)cdiv(d.X / 4, 128), rows), 128, 0, xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, run, pair_hi, pair_lo));
   } else {
-    conv_silu_bwd_kernel<K, 1><<<dim3((unsigned)cdiv(d.X, 128), rows), 128, 0, st>>>(xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, run, pair_hi, pair_lo);
+    PMB_TRY(launch_pdl(st, conv_silu_bwd_kernel<K, 1>, dim3((unsigned)cdiv(d.X, 128), rows), 128, 0, xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, run, pair_hi, pair_lo));
   }
-  PMB_LAUNCHED();
   return PMB_OK;
 }
 
@@ -417,10 +423,8 @@ pmb_status conv_silu_bwd(cudaStream_t st, const Dims& d, const float* xzd, const
   const int64_t rows = conv_bwd_partial_rows(d, conv_bwd_strip_ok(d, xzd, dact, dxzd));
   cudaStream_t rs = st;
   if (red) { PMB_TRY(order_after(st, red->ev[4], red->s)); rs = red->s; }
-  column_sum_kernel<<<(unsigned)cdiv(d.X * d.K, 32), 32 * COLSUM_LANES, 0, rs>>>(partial, rows, d.X * d.K, dw);
-  PMB_LAUNCHED();
-  column_sum_kernel<<<(unsigned)cdiv(d.X, 32), 32 * COLSUM_LANES, 0, rs>>>(partial + rows * d.X * d.K, rows, d.X, db);
-  PMB_LAUNCHED();
+  PMB_TRY(launch_pdl(rs, column_sum_kernel, dim3((unsigned)cdiv(d.X * d.K, 32)), 32 * COLSUM_LANES, 0, partial, rows, d.X * d.K, dw));
+  PMB_TRY(launch_pdl(rs, column_sum_kernel, dim3((unsigned)cdiv(d.X, 32)), 32 * COLSUM_LANES, 0, partial + rows * d.X * d.K, rows, d.X, db));
   return PMB_OK;
 }
 
@@ -436,6 +440,8 @@ __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_fwd_kernel(const f
                                                                          float* __restrict__ out, float* __restrict__ rstd,
                                                                          int width, float eps, uint16_t* __restrict__ out_hi,
                                                                          uint16_t* __restrict__ out_lo) {
+  pdl_launch();
+  pdl_wait();
   __shared__ float red[32];
   int64_t row = blockIdx.x;
   const float* yr = y + row * width;
@@ -492,6 +498,8 @@ __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_fwd_vec_kernel(con
                                                                              float* __restrict__ out, float* __restrict__ rstd,
                                                                              int width, float eps, uint16_t* __restrict__ out_hi,
                                                                              uint16_t* __restrict__ out_lo, int64_t rows, int nrows) {
+  pdl_launch();
+  pdl_wait();
   __shared__ float red[2][32];
   const int nvec = width >> 2;
   const int64_t r0 = (int64_t)blockIdx.x * nrows;
@@ -566,13 +574,11 @@ pmb_status gated_rmsnorm_fwd(cudaStream_t st, int64_t rows, int width, float eps
     // four to eight blocks share an SM; with fewer rows than fill it that way every row has a block
     const int nr = (int)cdiv(rows, 148 * 6);
     const unsigned nblk = (unsigned)cdiv(rows, nr);
-    if (per == 1) gated_rmsnorm_fwd_vec_kernel<1><<<nblk, threads, 0, st>>>(y, z, ldz, w, out, rstd, width, eps, out_hi, out_lo, rows, nr);
-    else gated_rmsnorm_fwd_vec_kernel<2><<<nblk, threads, 0, st>>>(y, z, ldz, w, out, rstd, width, eps, out_hi, out_lo, rows, nr);
-    PMB_LAUNCHED();
+    if (per == 1) PMB_TRY(launch_pdl(st, gated_rmsnorm_fwd_vec_kernel<1>, dim3((unsigned)nblk), threads, 0, y, z, ldz, w, out, rstd, width, eps, out_hi, out_lo, rows, nr));
+    else PMB_TRY(launch_pdl(st, gated_rmsnorm_fwd_vec_kernel<2>, dim3((unsigned)nblk), threads, 0, y, z, ldz, w, out, rstd, width, eps, out_hi, out_lo, rows, nr));
     return PMB_OK;
   }
-  gated_rmsnorm_fwd_kernel<<<(unsigned)rows, NORM_THREADS, 0, st>>>(y, z, ldz, w, out, rstd, width, eps, out_hi, out_lo);
-  PMB_LAUNCHED();
+  PMB_TRY(launch_pdl(st, gated_rmsnorm_fwd_kernel, dim3((unsigned)rows), NORM_THREADS, 0, y, z, ldz, w, out, rstd, width, eps, out_hi, out_lo));
   return PMB_OK;
 }
 
@@ -586,6 +592,8 @@ __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_bwd_kernel(const f
                                                                          const float* __restrict__ w, const float* __restrict__ rstd,
                                                                          float* __restrict__ dy, float* __restrict__ dz, int64_t lddz,
                                                                          float* __restrict__ dw_partial, int64_t rows, int width) {
+  pdl_launch();
+  pdl_wait();
   __shared__ float red[32];
   float dwacc[NORM_MAX_PER_THREAD];
 #pragma unroll
@@ -641,6 +649,8 @@ __global__ void __launch_bounds__(NORM_THREADS, 3) gated_rmsnorm_bwd_vec_kernel(
                                                                              float* __restrict__ dy, float* __restrict__ dz, int64_t lddz,
                                                                              float* __restrict__ dw_partial, int64_t rows, int width, int nrows,
                                                                              NormBwdExtra ex) {
+  pdl_launch();
+  pdl_wait();
   __shared__ float red[2][32];
   const int nvec = width >> 2;
   float4 dwacc[PER], wv[PER];
@@ -716,6 +726,8 @@ __global__ void __launch_bounds__(NORM_THREADS, 3) gated_rmsnorm_bwd_vec_kernel(
 // (four loads in flight) and the lanes' sums are added in a fixed order (deterministic).  The columns alone give few blocks, so
 // what counts is the length of a lane's chain of loads: 23 us for 4096 rows of 1536 columns with 8 lanes.
 __global__ void __launch_bounds__(32 * COLSUM_LANES) column_sum_kernel(const float* __restrict__ partial, int64_t rows, int cols, float* __restrict__ out) {
+  pdl_launch();
+  pdl_wait();
   __shared__ float sh[COLSUM_LANES][33];
   int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   int j = blockIdx.x * 32 + tx;
@@ -758,16 +770,14 @@ pmb_status gated_rmsnorm_bwd(cudaStream_t st, int64_t rows, int width, const flo
     int64_t nr = cdiv(rows, 8 * 148);
     if (nr < NORM_ROWS) nr = NORM_ROWS;
     nblk = cdiv(rows, nr);
-    if (per == 1) gated_rmsnorm_bwd_vec_kernel<1><<<(unsigned)nblk, threads, 0, st>>>(dout, y, z, ldz, w, rstd, dy, dz, lddz, partial, rows, width, (int)nr, ex);
-    else gated_rmsnorm_bwd_vec_kernel<2><<<(unsigned)nblk, threads, 0, st>>>(dout, y, z, ldz, w, rstd, dy, dz, lddz, partial, rows, width, (int)nr, ex);
+    if (per == 1) PMB_TRY(launch_pdl(st, gated_rmsnorm_bwd_vec_kernel<1>, dim3((unsigned)nblk), threads, 0, dout, y, z, ldz, w, rstd, dy, dz, lddz, partial, rows, width, (int)nr, ex));
+    else PMB_TRY(launch_pdl(st, gated_rmsnorm_bwd_vec_kernel<2>, dim3((unsigned)nblk), threads, 0, dout, y, z, ldz, w, rstd, dy, dz, lddz, partial, rows, width, (int)nr, ex));
   } else {
-    gated_rmsnorm_bwd_kernel<<<(unsigned)nblk, NORM_THREADS, 0, st>>>(dout, y, z, ldz, w, rstd, dy, dz, lddz, partial, rows, width);
+    PMB_TRY(launch_pdl(st, gated_rmsnorm_bwd_kernel, dim3((unsigned)nblk), NORM_THREADS, 0, dout, y, z, ldz, w, rstd, dy, dz, lddz, partial, rows, width));
   }
-  PMB_LAUNCHED();
   cudaStream_t rs = st;
   if (red) { PMB_TRY(order_after(st, red->ev[4], red->s)); rs = red->s; }
-  column_sum_kernel<<<(unsigned)cdiv(width, 32), 32 * COLSUM_LANES, 0, rs>>>(partial, nblk, width, dw);
-  PMB_LAUNCHED();
+  PMB_TRY(launch_pdl(rs, column_sum_kernel, dim3((unsigned)cdiv(width, 32)), 32 * COLSUM_LANES, 0, partial, nblk, width, dw));
   return PMB_OK;
 }
 
@@ -818,8 +828,7 @@ pmb_status gated_rmsnorm_bwd_static(cudaStream_t st, int64_t rows, int width, co
 }
 
 pmb_status column_sum(cudaStream_t st, const float* partial, int64_t rows, int cols, float* out) {
-  column_sum_kernel<<<(unsigned)cdiv(cols, 32), 32 * COLSUM_LANES, 0, st>>>(partial, rows, cols, out);
-  PMB_LAUNCHED();
+  PMB_TRY(launch_pdl(st, column_sum_kernel, dim3((unsigned)cdiv(cols, 32)), 32 * COLSUM_LANES, 0, partial, rows, cols, out));
   return PMB_OK;
 }
 

@@ -409,6 +409,8 @@ gemm_bf16_kernel(const __grid_constant__ Group g, const int total_tiles, unsigne
   else asm volatile("bar.sync 1, %0;" ::"n"(NTHREADS) : "memory");
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = warp == 0 ? 0u : *tmem_slot;
+  pdl_launch();
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -848,6 +850,8 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
   cluster_sync_all();     // both CTAs' barriers are initialised before either signals the other's
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
+  pdl_launch();
+  pdl_wait();
 
   if (warp == 0) {
     // (the whole warp waits, one elected lane issues)
@@ -1266,13 +1270,12 @@ pmb_status gemm_bf16_group(cudaStream_t st, const PlainGemm* gs, int n, int max_
     }
     const unsigned grid = 2u * (unsigned)(clusters < slots ? clusters : slots);
     set_lead(&g, n, (int)(grid / 2));
-    gemm_bf16_pairp_kernel<false, 256><<<grid, (PairPCfg<false, 256>::THREADS), PairPCfg<false, 256>::SMEM_BYTES, st>>>(g, (int)clusters);
+    PMB_TRY(launch_pdl(st, gemm_bf16_pairp_kernel<false, 256>, grid, (PairPCfg<false, 256>::THREADS), PairPCfg<false, 256>::SMEM_BYTES, g, (int)clusters));
   } else {
     unsigned long long t0 = 0;
     unsigned long long* sc = sched_counter(st, tiles, &t0);
-    gemm_bf16_kernel<false><<<persistent_grid(tiles), NTHREADS, Cfg<false>::SMEM_BYTES, st>>>(g, (int)tiles, sc, t0);
+    PMB_TRY(launch_pdl(st, gemm_bf16_kernel<false>, dim3((unsigned)(persistent_grid(tiles))), NTHREADS, Cfg<false>::SMEM_BYTES, g, (int)tiles, sc, t0));
   }
-  PMB_LAUNCHED();
   return PMB_OK;
 }
 
@@ -1284,6 +1287,8 @@ pmb_status gemm_bf16(cudaStream_t st, int ta, int tb, int64_t M, int64_t N, int6
 
 // out = sum of n slabs, fixed order; `pitch` elements apart, `elems` each; out fp32 or bf16
 __global__ void __launch_bounds__(256) sum_slabs_kernel(const float* __restrict__ part, int n, int64_t pitch, int64_t elems, void* __restrict__ out, int out_bf16) {
+  pdl_launch();
+  pdl_wait();
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (i >= elems) return;
   float4 a = *reinterpret_cast<const float4*>(part + i);
@@ -1298,8 +1303,7 @@ __global__ void __launch_bounds__(256) sum_slabs_kernel(const float* __restrict_
 pmb_status sum_slabs(cudaStream_t st, const float* part, int n, int64_t pitch, int64_t elems, void* out, int out_bf16) {
   if (elems & 3) return fail(PMB_ERR_SHAPE, "sum_slabs: the element count must be a multiple of 4");
   ProfScope prof(st, "splitk_sum", 0.0, (4.0 * n + (out_bf16 ? 2.0 : 4.0)) * elems);
-  sum_slabs_kernel<<<(unsigned)cdiv(elems / 4, 256), 256, 0, st>>>(part, n, pitch, elems, out, out_bf16);
-  PMB_LAUNCHED();
+  PMB_TRY(launch_pdl(st, sum_slabs_kernel, dim3((unsigned)cdiv(elems / 4, 256)), 256, 0, part, n, pitch, elems, out, out_bf16));
   return PMB_OK;
 }
 
@@ -1308,6 +1312,8 @@ pmb_status sum_slabs(cudaStream_t st, const float* part, int n, int64_t pitch, i
 // One thread = 4 consecutive columns of the pair; columns in [cols, ld16) are written as zero.
 __global__ void split_pair16_kernel(const float* __restrict__ src, int64_t rows, int64_t cols, int64_t ld,
                                     uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, int64_t ld16, int vec) {
+  pdl_launch();
+  pdl_wait();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   int64_t c4 = ld16 / 4;
   if (i >= rows * c4) return;
@@ -1336,8 +1342,7 @@ pmb_status split_pair16(cudaStream_t st, const float* src, int64_t rows, int64_t
     return fail(PMB_ERR_ARG, "split_pair16: the pair needs 16-byte aligned bases and a row pitch that is a multiple of 8");
   const int vec = ((reinterpret_cast<uintptr_t>(src) & 15) == 0 && (ld & 3) == 0) ? 1 : 0;
   ProfScope prof(st, "split_f32_bf16x2", 0.0, 8.0 * rows * cols);
-  split_pair16_kernel<<<(unsigned)cdiv(rows * (ld16 / 4), 256), 256, 0, st>>>(src, rows, cols, ld, hi, lo, ld16, vec);
-  PMB_LAUNCHED();
+  PMB_TRY(launch_pdl(st, split_pair16_kernel, dim3((unsigned)cdiv(rows * (ld16 / 4), 256)), 256, 0, src, rows, cols, ld, hi, lo, ld16, vec));
   return PMB_OK;
 }
 
@@ -1347,6 +1352,8 @@ pmb_status split_pair16(cudaStream_t st, const float* src, int64_t rows, int64_t
 struct SplitGroup { SplitItem it[4]; int first[4]; };      // first[i]: block at which item i starts
 template <int U>
 __global__ void __launch_bounds__(256) split_flat_kernel(const SplitGroup g) {
+  pdl_launch();
+  pdl_wait();
   int w = 0;
 #pragma unroll
   for (int i = 1; i < 4; ++i) if ((int)blockIdx.x >= g.first[i]) w = i;
@@ -1386,9 +1393,8 @@ pmb_status split_pairs_flat(cudaStream_t st, const SplitItem* items, int n) {
   }
   if (blocks > 0x7ffffffe) return fail(PMB_ERR_SHAPE, "split_pairs_flat: too large");
   ProfScope prof(st, "split_f32_bf16x2", 0.0, 8.0 * total);
-  if (U == 4) split_flat_kernel<4><<<(unsigned)blocks, 256, 0, st>>>(g);
-  else split_flat_kernel<1><<<(unsigned)blocks, 256, 0, st>>>(g);
-  PMB_LAUNCHED();
+  if (U == 4) PMB_TRY(launch_pdl(st, split_flat_kernel<4>, dim3((unsigned)blocks), 256, 0, g));
+  else PMB_TRY(launch_pdl(st, split_flat_kernel<1>, dim3((unsigned)blocks), 256, 0, g));
   return PMB_OK;
 }
 
@@ -1396,6 +1402,8 @@ pmb_status split_pairs_flat(cudaStream_t st, const SplitItem* items, int n) {
 // sources can share one pair buffer side by side.
 __global__ void split_pair16_cols_kernel(const float* __restrict__ src, int64_t rows, int64_t cols, int64_t ld,
                                          uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, int64_t ld16) {
+  pdl_launch();
+  pdl_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t c4 = cols / 4;
   if (i >= rows * c4) return;
@@ -1408,8 +1416,7 @@ pmb_status split_pair16_strided(cudaStream_t st, const float* src, int64_t rows,
                                 int64_t ld16) {
   if ((cols & 3) || (ld16 & 3) || ld16 < cols || ((reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 7))
     return fail(PMB_ERR_ARG, "split_pair16_strided: column count and pitch must be multiples of 4, destinations 8-byte aligned");
-  split_pair16_cols_kernel<<<(unsigned)cdiv(rows * (cols / 4), 256), 256, 0, st>>>(src, rows, cols, ld, hi, lo, ld16);
-  PMB_LAUNCHED();
+  PMB_TRY(launch_pdl(st, split_pair16_cols_kernel, dim3((unsigned)cdiv(rows * (cols / 4), 256)), 256, 0, src, rows, cols, ld, hi, lo, ld16));
   return PMB_OK;
 }
 
@@ -1504,12 +1511,11 @@ pmb_status gemm_pairs_group(cudaStream_t st, const PairGemm* gs, int n, int tile
       set_lead(&g, n, (int)(grid / 2));
       if (pair_mode == 4) {
         PMB_SMEM_OPT_IN((PairPCfg<true, 256>::SMEM_BYTES), gemm_bf16_pairp_kernel<true, 256>);
-        gemm_bf16_pairp_kernel<true, 256><<<grid, (PairPCfg<true, 256>::THREADS), PairPCfg<true, 256>::SMEM_BYTES, st>>>(g, (int)clusters);
+        PMB_TRY(launch_pdl(st, gemm_bf16_pairp_kernel<true, 256>, grid, (PairPCfg<true, 256>::THREADS), PairPCfg<true, 256>::SMEM_BYTES, g, (int)clusters));
       } else {
         PMB_SMEM_OPT_IN((PairPCfg<true, 128>::SMEM_BYTES), gemm_bf16_pairp_kernel<true, 128>);
-        gemm_bf16_pairp_kernel<true, 128><<<grid, (PairPCfg<true, 128>::THREADS), PairPCfg<true, 128>::SMEM_BYTES, st>>>(g, (int)clusters);
+        PMB_TRY(launch_pdl(st, gemm_bf16_pairp_kernel<true, 128>, grid, (PairPCfg<true, 128>::THREADS), PairPCfg<true, 128>::SMEM_BYTES, g, (int)clusters));
       }
-      PMB_LAUNCHED();
       return PMB_OK;
     }
     ProfScope prof(st, pair_mode == 2 ? "gemm_bf16x2_pair256" : "gemm_bf16x2_pair128", flops, bytes);
@@ -1522,9 +1528,8 @@ pmb_status gemm_pairs_group(cudaStream_t st, const PairGemm* gs, int n, int tile
   {
     unsigned long long t0 = 0;
     unsigned long long* sc = sched_counter(st, total, &t0);
-    gemm_bf16_kernel<true><<<persistent_grid(total), NTHREADS, Cfg<true>::SMEM_BYTES, st>>>(g, (int)total, sc, t0);
+    PMB_TRY(launch_pdl(st, gemm_bf16_kernel<true>, dim3((unsigned)(persistent_grid(total))), NTHREADS, Cfg<true>::SMEM_BYTES, g, (int)total, sc, t0));
   }
-  PMB_LAUNCHED();
   return PMB_OK;
 }
 

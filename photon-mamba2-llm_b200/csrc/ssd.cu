@@ -918,6 +918,8 @@ __global__ void __launch_bounds__(ROWS_THREADS, 3) chunk_rows_finish_w_kernel(Ss
 // fixed order; d_a_log = A dA.  (One thread per head walked the rows in 16 us at 64 rows.)
 __global__ void __launch_bounds__(128) head_finish_kernel(const float* __restrict__ part, int rows, int H, const float* __restrict__ A, float* __restrict__ dA,
                                    float* __restrict__ dD, float* __restrict__ d_dt_bias, float* __restrict__ d_a_log) {
+  pdl_launch();
+  pdl_wait();
   const int h = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (h >= H) return;
   float a = 0.0f, d = 0.0f, b = 0.0f;
@@ -935,8 +937,7 @@ __global__ void __launch_bounds__(128) head_finish_kernel(const float* __restric
 }
 
 pmb_status ssd_head_finish(cudaStream_t st, const float* part, int rows, int H, const float* A, float* dA, float* dD, float* d_dt_bias, float* d_a_log) {
-  head_finish_kernel<<<(unsigned)cdiv(H, 4), 128, 0, st>>>(part, rows, H, A, dA, dD, d_dt_bias, d_a_log);
-  PMB_LAUNCHED();
+  PMB_TRY(launch_pdl(st, head_finish_kernel, dim3((unsigned)cdiv(H, 4)), 128, 0, part, rows, H, A, dA, dD, d_dt_bias, d_a_log));
   return PMB_OK;
 }
 
@@ -1322,9 +1323,8 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
   auto head_sums = [&](cudaStream_t s) -> pmb_status {   // part = [dA partials (B*nc,H)] [dD partials (B*nc,H)] [d_dt_bias partials]
     if (!in.dt) return PMB_OK;
     if (fz) {
-      head_finish_kernel<<<(unsigned)cdiv(p.H, 4), 128, 0, s>>>(ws.part, p.B * p.nc, p.H, in.A, g.dA, g.dD, g.raw.hi ? g.raw.d_dt_bias : nullptr,
-                                                                  g.raw.hi ? g.raw.d_a_log : nullptr);
-      PMB_LAUNCHED();
+      PMB_TRY(launch_pdl(s, head_finish_kernel, dim3((unsigned)cdiv(p.H, 4)), 128, 0, ws.part, p.B * p.nc, p.H, in.A, g.dA, g.dD, g.raw.hi ? g.raw.d_dt_bias : nullptr,
+                                                                  g.raw.hi ? g.raw.d_a_log : nullptr));
       return PMB_OK;
     }
     PMB_TRY(column_sum(s, ws.part, (int64_t)p.B * p.nc, p.H, g.dA));

@@ -165,6 +165,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  pdl_launch();
+  pdl_wait();
   const uint32_t tG = tmem, tA1 = tmem + 256, tA2 = tmem + 320, tU = tmem + 384;
 
   auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
@@ -775,13 +777,11 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
   const unsigned grid = (unsigned)((int64_t)a.B * a.H * p.nseg);
   if (p.nseg > 1) {
     p.state_only = 1;
-    ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
-    PMB_LAUNCHED();
+    PMB_TRY(launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>, grid, NTHREADS, GE::SMEM, ms, p));
     p.state_only = 0;
   }
   p.store_ops = keep != nullptr;
-  ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
-  PMB_LAUNCHED();
+  PMB_TRY(launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>, grid, NTHREADS, GE::SMEM, ms, p));
   return PMB_OK;
 }
 

@@ -154,6 +154,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  pdl_launch();
+  pdl_wait();
   const uint32_t tG = tmem, tM = tmem + 128, tA1 = tmem + 256, tA2 = tmem + 320, tA3 = tmem + 384, tU = tmem + 448;
 
   auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
@@ -853,12 +855,10 @@ static pmb_status launch(cudaStream_t st, const ChainBwdArgs& a) {
   const unsigned grid = (unsigned)((int64_t)a.B * a.H * p.nseg);
   if (p.nseg > 1) {
     p.state_only = 1;
-    ssd_chain_bwd_kernel<NI, ND, NK, IN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
-    PMB_LAUNCHED();
+    PMB_TRY(launch_pdl(st, ssd_chain_bwd_kernel<NI, ND, NK, IN16>, grid, NTHREADS, GE::SMEM, ms, p));
     p.state_only = 0;
   }
-  ssd_chain_bwd_kernel<NI, ND, NK, IN16><<<grid, NTHREADS, GE::SMEM, st>>>(ms, p);
-  PMB_LAUNCHED();
+  PMB_TRY(launch_pdl(st, ssd_chain_bwd_kernel<NI, ND, NK, IN16>, grid, NTHREADS, GE::SMEM, ms, p));
   return PMB_OK;
 }
 

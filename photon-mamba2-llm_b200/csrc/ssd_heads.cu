@@ -113,6 +113,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  pdl_launch();
+  pdl_wait();
   const uint32_t tM = tmem, tC = tmem + 256, tB = tmem + 384;
   // the stage that dG goes over: the one the last head of the first pass was in
   const uint32_t dg_s = GE::OWN_DG ? base + GE::STG * GE::STAGE : base + (uint32_t)((nh - 1) & 1) * GE::STAGE;
@@ -342,6 +344,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
 
 // Adds the shares of the splits in a fixed order; four columns per thread.
 __global__ void __launch_bounds__(256) heads_sum_kernel(const float* __restrict__ part, Params p, int64_t total) {
+  pdl_launch();
+  pdl_wait();
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= total) return;
   const int n4 = p.N / 4, c = (int)(q % n4); int64_t r = q / n4;
@@ -389,12 +393,10 @@ static pmb_status launch(cudaStream_t st, const HeadsArgs& a, int nsplit) {
   p.S = a.S; p.dc = a.dc; p.db = a.db; p.ld = a.ld; p.dc16 = a.dc16; p.db16 = a.db16; p.part = a.part; p.status = status_ptr();
   const int64_t tiles = (int64_t)a.B * n * a.G;
   PMB_SMEM_OPT_IN(GE::SMEM, ssd_heads_kernel<NI, ND>);
-  ssd_heads_kernel<NI, ND><<<(unsigned)(tiles * nsplit), NTHREADS, GE::SMEM, st>>>(ms, p);
-  PMB_LAUNCHED();
+  PMB_TRY(launch_pdl(st, ssd_heads_kernel<NI, ND>, dim3((unsigned)((tiles * nsplit))), NTHREADS, GE::SMEM, ms, p));
   if (nsplit > 1) {
     const int64_t total = tiles * 2 * L * (a.N / 4);
-    heads_sum_kernel<<<(unsigned)cdiv(total, 256), 256, 0, st>>>(a.part, p, total);
-    PMB_LAUNCHED();
+    PMB_TRY(launch_pdl(st, heads_sum_kernel, dim3((unsigned)cdiv(total, 256)), 256, 0, a.part, p, total));
   }
   return PMB_OK;
 }

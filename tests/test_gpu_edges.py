@@ -441,3 +441,24 @@ def test_scan_bf16_strong_decay(pm, T, Q, N, strength):
     for got, want, tol, what in ((y.float(), ref, 5e-3, "y"), (dx.float(), leaves[0].grad, 5e-3, "dx"), (da, leaves[1].grad, 1e-3, "da"),
                                  (db.float(), leaves[2].grad, 5e-3, "db"), (dc.float(), leaves[3].grad, 5e-3, "dc")):
         assert_close(got, want, tol=tol, what=what)
+
+
+# kernels that start while the one before them in the stream is still at work wait for it before they touch memory: calls one after the
+# other on buffers that each of them overwrites give what they give one at a time (the sums have fixed orders: equal bits)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D,H,P,N,B,T,Q", [(128, 8, 32, 16, 2, 128, 64), (256, 8, 64, 64, 2, 300, 128), (768, 24, 64, 64, 1, 640, 256)])
+def test_calls_one_after_the_other(pm, dtype, D, H, P, N, B, T, Q):
+    _, _, blk = _block(pm, D, H, P, N, 1, Q, dtype)
+    xs, cots = [randn((B, T, D), 5 + i).cuda().to(dtype) for i in range(4)], [randn((B, T, D), 15 + i).cuda().to(dtype) for i in range(4)]
+
+    def call(i):
+        return blk.forward(xs[i], residual=xs[i]), *blk.backward(xs[i], cots[i])
+    want = []
+    for i in range(4):
+        want.append(call(i))
+        torch.cuda.synchronize()
+    for _ in range(5):
+        for i, got in enumerate([call(i) for i in range(4)]):
+            assert torch.equal(got[0], want[i][0]) and torch.equal(got[1], want[i][1])
+            assert all(torch.equal(got[2][k], want[i][2][k]) for k in got[2])
+    assert pm.device_status() == 0
