@@ -182,11 +182,14 @@ template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // Epilogue of one tile for one epilogue warp: its 32 rows (row0 ..) x `ncols` columns (n0 ..) of the accumulator at
-// `tmem_acc` (lane offset included).  Results that meet the TMA rules leave through the warp's NSLOT swizzled staging slots of 32
-// rows of 128 bytes (32 fp32 or 64 bf16 columns) and TMA stores.  The residual blocks are TMA-loaded into the slots: the first NSLOT
-// of a tile by prefetch(), while its products still run (four slots hold all of a 256-wide bf16 tile), further ones as soon as
-// a slot's store has read it.  Everything else is stored row by row.  `pc` and `rph` carry the slot in turn and the residual
-// barriers' phases across tiles.
+// `tmem_acc` (lane offset included).  fp32 results that meet the TMA rules go out from the accumulator's fragments as whole 32-byte
+// sectors, and so do their bf16 pairs; the residual's fragments are in registers, the first 32 columns' requested by prefetch() while
+// the products still run, the others 32 columns ahead.  (Through one staging slot per warp the second block's residual waited for the first
+// one's store: 2048 x 768 x 1536 on pairs with residual and pair output, a tile per cluster, 28 us, 17.6 without either.)  bf16 results
+// and fp32 ones that are added onto C leave through the warp's NSLOT swizzled staging slots of 32 rows of 128 bytes (32 fp32 or 64 bf16
+// columns) and TMA stores; a bf16 residual is TMA-loaded into the slots: the first NSLOT blocks of a tile by prefetch(), further
+// ones as soon as a slot's store has read it.  Everything else is stored row by row.  `pc` and `rph` carry the slot in turn and the
+// residual barriers' phases across tiles.
 __device__ __forceinline__ void tma_add_2d(const CUtensorMap* map, uint32_t src, int c0, int c1) {
   asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%1, %2}], [%3];"
                ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(src) : "memory");
@@ -195,15 +198,33 @@ template <int NSLOT>
 struct Epilogue {
   uint32_t slot0, rbar0;                     // the warp's slots and their residual barriers (8 bytes apart)
   uint32_t pc = 0, rph = 0, loading = 0;     // (loading: lane 0's record of the slots with a load in flight)
-  __device__ __forceinline__ bool loads(const Params& p) const { return p.tma_out && p.R && !p.red; }
+  uint2 rr[16];                              // fp32 residual of the next 32 columns, as fragments
+  __device__ __forceinline__ bool loads(const Params& p) const { return p.tma_out && p.R && p.out_bf16; }
+  // residual fragments of 32 columns from c0 on (rows and columns outside of the matrix: zeros)
+  __device__ __forceinline__ void fetch(const Params& p, int row0, int n0, int c0, int lane) {
+    const int r = row0 + (lane >> 2), c = n0 + c0 + (lane & 3) * 2;
+    const float* base = static_cast<const float*>(p.R) + (int64_t)r * p.ldc + c;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int dr = 16 * (i >> 1) + 8 * (e & 1), dc = 16 * (i & 1) + 8 * (e >> 1);
+        const float* at = base + (int64_t)dr * p.ldc + dc;
+        uint2 v = make_uint2(0u, 0u);
+        if (r + dr < p.M && c + dc + 1 < p.N) v = *reinterpret_cast<const uint2*>(at);
+        else if (r + dr < p.M && c + dc < p.N) v.x = __float_as_uint(*at);
+        rr[4 * i + e] = v;
+      }
+  }
   __device__ __forceinline__ void load(const Problem& q, uint32_t slot, int c, int row0) {
     mbar_expect_tx(rbar0 + 8u * slot, EPI_SLOT_BYTES);
     tma_load_2d(slot0 + slot * EPI_SLOT_BYTES, &q.mR, c, row0, rbar0 + 8u * slot);
     loading |= 1u << slot;
   }
   __device__ __forceinline__ void prefetch(const Problem& q, const Params& p, int row0, int n0, int ncols, int lane) {
+    if (p.tma_out && p.R && !p.out_bf16 && !p.red) { fetch(p, row0, n0, 0, lane); return; }
     if (!loads(p) || row0 >= p.M || n0 >= p.N || lane != 0) return;
-    const int bw = p.out_bf16 ? 64 : 32, end = min(ncols, p.N - n0);
+    const int bw = 64, end = min(ncols, p.N - n0);
     bulk_wait_read<0>();
     for (int i = 0; i < NSLOT && i * bw < end; ++i) load(q, (pc + i) % NSLOT, n0 + i * bw, row0);
   }
@@ -226,8 +247,8 @@ struct Epilogue {
     }
     if (row0 >= p.M) return;
     const bool res = loads(p);
-    if (!res && !p.red && !p.e_hi && !p.out_bf16) {
-      // nothing to add and fp32: 16 x 8 fragments go out as they are, a quad of lanes one whole 32-byte sector, and nobody waits
+    if (!p.red && !p.out_bf16) {
+      // 16 x 8 fragments go out as they are, a quad of lanes one whole 32-byte sector, and nobody waits
       const int r = row0 + (lane >> 2), c = n0 + (lane & 3) * 2;
       float* base = static_cast<float*>(p.C) + (int64_t)(rowoff + r) * p.ldc + c;
 #pragma unroll 1
@@ -236,6 +257,18 @@ struct Epilogue {
 #pragma unroll
         for (int i = 0; i < 4; ++i) tmem_ld16x256_x2(tmem_acc + ((uint32_t)(16 * (i >> 1)) << 16) + (uint32_t)(c0 + 16 * (i & 1)), v[i]);
         tmem_wait_ld();
+        if (p.R) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              uint32_t* w = &v[i][4 * (e >> 1) + 2 * (e & 1)];
+              w[0] = __float_as_uint(__uint_as_float(w[0]) + __uint_as_float(rr[4 * i + e].x));
+              w[1] = __float_as_uint(__uint_as_float(w[1]) + __uint_as_float(rr[4 * i + e].y));
+            }
+          if (c0 + 32 < ncols && n0 + c0 + 32 < p.N) fetch(p, row0, n0, c0 + 32, lane);
+        }
+        const bool whole = row0 + 32 <= p.M && n0 + c0 + 32 <= p.N;
         auto put = [&](bool inside) {
 #pragma unroll
           for (int i = 0; i < 4; ++i)
@@ -248,7 +281,31 @@ struct Epilogue {
               else if (r + dr < p.M && c + dc < p.N) *at = __uint_as_float(o.x);
             }
         };
-        if (row0 + 32 <= p.M && n0 + c0 + 32 <= p.N) put(true); else put(false);
+        if (whole) put(true); else put(false);
+        if (p.e_hi) {
+          // the same values as a (hi, lo) bf16 pair: neighbouring lanes swap halves, so that a lane has four columns of one of two octets
+          const bool odd = lane & 1;
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int row = r + 16 * (i >> 1) + 8 * e, c16 = n0 + c0 + 16 * (i & 1);
+              uint32_t h0, l0, h1, l1;
+              split2(__uint_as_float(v[i][2 * e]), __uint_as_float(v[i][2 * e + 1]), h0, l0, true);
+              split2(__uint_as_float(v[i][4 + 2 * e]), __uint_as_float(v[i][4 + 2 * e + 1]), h1, l1, true);
+              const uint32_t gh = __shfl_xor_sync(0xffffffffu, odd ? h0 : h1, 1), gl = __shfl_xor_sync(0xffffffffu, odd ? l0 : l1, 1);
+              const uint2 h = odd ? make_uint2(gh, h1) : make_uint2(h0, gh), l = odd ? make_uint2(gl, l1) : make_uint2(l0, gl);
+              const int col = c16 + ((lane & 3) * 2) + (odd ? 6 : 0);      // first of the lane's four columns
+              if (row >= p.M) continue;
+              uint16_t* eh = p.e_hi + (int64_t)row * p.lde + col;
+              uint16_t* el = p.e_lo + (int64_t)row * p.lde + col;
+              if (whole || col + 4 <= p.N) { *reinterpret_cast<uint2*>(eh) = h; *reinterpret_cast<uint2*>(el) = l; }
+              else
+                for (int j = 0; j < 4 && col + j < p.N; ++j) {
+                  eh[j] = (uint16_t)((j < 2 ? h.x : h.y) >> (16 * (j & 1))); el[j] = (uint16_t)((j < 2 ? l.x : l.y) >> (16 * (j & 1)));
+                }
+            }
+        }
       }
       return;
     }
@@ -286,42 +343,6 @@ struct Epilogue {
             asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
           }
           continue;
-        }
-        if (landed) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float4 v;
-            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                         : "r"(sbase + (uint32_t)((j ^ (lane & 7)) * 16)));
-            r[4 * j] = __float_as_uint(__uint_as_float(r[4 * j]) + v.x);
-            r[4 * j + 1] = __float_as_uint(__uint_as_float(r[4 * j + 1]) + v.y);
-            r[4 * j + 2] = __float_as_uint(__uint_as_float(r[4 * j + 2]) + v.z);
-            r[4 * j + 3] = __float_as_uint(__uint_as_float(r[4 * j + 3]) + v.w);
-          }
-        }
-        if (p.e_hi) {
-          // the same values as a (hi, lo) bf16 pair, straight from registers: 64 contiguous bytes per row and array
-          const int m = row0 + lane;
-          if (m < p.M) {
-            uint16_t* eh = p.e_hi + (int64_t)m * p.lde + n0 + c0;
-            uint16_t* el = p.e_lo + (int64_t)m * p.lde + n0 + c0;
-            if (n0 + c0 + 32 <= p.N) {
-#pragma unroll
-              for (int j = 0; j < 32; j += 8) {
-                uint32_t h[8], l[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) split_bf16_pair(__uint_as_float(r[j + e]), h[e], l[e]);
-                *reinterpret_cast<uint4*>(eh + j) = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
-                *reinterpret_cast<uint4*>(el + j) = make_uint4(l[0] | (l[1] << 16), l[2] | (l[3] << 16), l[4] | (l[5] << 16), l[6] | (l[7] << 16));
-              }
-            } else {
-              for (int j = 0; j < 32 && n0 + c0 + j < p.N; ++j) {
-                uint32_t h, l;
-                split_bf16_pair(__uint_as_float(r[j]), h, l);
-                eh[j] = (uint16_t)h; el[j] = (uint16_t)l;
-              }
-            }
-          }
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j)
