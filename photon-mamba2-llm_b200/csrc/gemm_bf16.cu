@@ -6,6 +6,7 @@
 // 32 KiB per stage) and the ring is 6 deep.  K-major tiles: 128-byte rows, 128-byte swizzle.  MN-major
 // tiles: blocks of 64 elements along M/N, 64 k-rows of 128 bytes per block, same swizzle.
 // Every mbarrier wait is bounded; on expiry the kernel raises the device status word and drains.
+#include <algorithm>
 #include <climits>
 #include <cstdint>
 #include <cstdlib>
@@ -143,7 +144,8 @@ __device__ __forceinline__ void store_row_piece(const Params& p, int m, int nb, 
 // pr[1].tiles on the second, and so on (unused entries have tiles == 0).
 // Two products whose tile counts each fill the 148 SMs badly (weight-gradient and data-gradient of one projection)
 // then share the machine instead of running as two ragged waves.
-struct Problem { CUtensorMap mA, mB, mAlo, mBlo, mC, mR; Params p; int tiles_n; int tiles_mn; int tiles; };
+// (On the CTA-pair kernel a product can be two problems: columns from n_begin up to n_end each, in tiles of their own width.)
+struct Problem { CUtensorMap mA, mB, mAlo, mBlo, mC, mR; Params p; int tiles_n; int tiles_mn; int tiles; int n_begin, n_end; };
 constexpr int MAX_GROUP = 4;
 // Order of the tiles on the persistent CTA-pair kernel.  lead == 0: cluster c takes tiles c, c + clusters, ...  lead > 0 (fewer
 // than the clusters): the first `lead` tiles are the long ones (weight gradients: K is the token count) and take one cluster
@@ -888,7 +890,7 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
       const Params& p = q.p;
       split_of(q, &tile, &kt0, &kt1);
       const int m0 = (tile / q.tiles_n) * 256 + (int)rank * TBM, bnh = p.bn >> 1;      // (tiles of bn <= BN2 columns)
-      const int nb0 = (tile % q.tiles_n) * p.bn + (int)rank * bnh;
+      const int nb0 = q.n_begin + (tile % q.tiles_n) * p.bn + (int)rank * bnh;
       const uint32_t tx = 2u * (uint32_t)(STAGE_BYTES - (SPLIT ? 2 : 1) * (BNH - bnh) * TBK * 2);
       const bool amn = p.a_mn_major, bmn = p.b_mn_major, wide = BNH > 64 && bnh > 64;
       for (int kt = kt0; kt < kt1; ++kt) {
@@ -991,7 +993,7 @@ gemm_bf16_pairp_kernel(const __grid_constant__ Group g, const int total_tiles) {
       const Problem& q = g.pr[pick_problem(g, tid, &tile)];
       const Params& p = q.p;
       const int rowoff = split_of(q, &tile, &kt0, &kt1) * p.slab_rows;
-      const int m0 = (tile / q.tiles_n) * 256 + (int)rank * TBM, cw = p.bn >> 1, n0 = (tile % q.tiles_n) * p.bn + chalf * cw;
+      const int m0 = (tile / q.tiles_n) * 256 + (int)rank * TBM, cw = p.bn >> 1, n0 = q.n_begin + (tile % q.tiles_n) * p.bn + chalf * cw;
       const int b = it & 1;
       est.prefetch(q, p, m0 + quarter * 32, n0, cw, lane);
       const bool acc_ok = __all_sync(0xffffffffu, mbar_wait_idle(acc_full(b), ((uint32_t)it >> 1) & 1u));
@@ -1073,7 +1075,6 @@ static pmb_status make_out_maps(Problem* q, int slabs = 1) {
   PMB_TRY(make_map(&q->mC, p.C, p.N, slabs > 1 ? (int64_t)slabs * p.slab_rows : p.M, p.ldc, 32, 32, true));
   // (one addend per element and launch, so the order of the additions is as it was: C, then the product)
   p.red = p.R == p.C && slabs == 1 && !p.e_hi;
-  if (p.R && !p.red) PMB_TRY(make_map(&q->mR, p.R, p.N, p.M, p.ldc, 32, 32, true));
   p.tma_out = 1;
   return PMB_OK;
 }
@@ -1172,7 +1173,8 @@ static void set_lead(Group* g, int n, int clusters) {
 static void set_tiles(Problem* q, int bn) {
   const int splits = (int)cdiv(ktiles(q->p.K), q->p.kt_per);
   q->p.bn = bn;
-  q->tiles_n = (int)cdiv(q->p.N, bn);
+  if (q->n_end == 0) q->n_end = q->p.N;
+  q->tiles_n = (int)cdiv(q->n_end - q->n_begin, bn);
   q->tiles_mn = (int)(cdiv(q->p.M, 256) * q->tiles_n);
   q->tiles = q->tiles_mn * splits;
 }
@@ -1218,6 +1220,74 @@ static void choose_widths(Group* g, int n, int slots) {
     if (mask == 0 || t < 0.9 * best) { best = t; pick = mask; }
   }
   for (int i = 0; i < n; ++i) set_tiles(&g->pr[i], (pick >> i) & 1 ? 128 : 256);
+}
+
+// The longest cluster's work, cluster by cluster.
+static double makespan_exact(Group* g, int n, int slots) {
+  int tiles = 0;
+  for (int i = 0; i < n; ++i) tiles += g->pr[i].tiles;
+  const int clusters = tiles < slots ? tiles : slots;
+  set_lead(g, n, clusters);
+  double worst = 0.0;
+  for (int c = 0; c < clusters; ++c) {
+    double t = 0.0;
+    for (int j = 0;; ++j) {
+      const int id = pair_tile_at(*g, c, clusters, j);
+      if (id >= tiles) break;
+      int base = 0, k = 0;
+      while (id >= base + g->pr[k].tiles) base += g->pr[k++].tiles;
+      t += tile_cost(g->pr[k]);
+    }
+    if (t > worst) worst = t;
+  }
+  return worst;
+}
+
+// A few rounds of tiles leave the last one partly empty whatever the width: one product's columns then go to tiles of 256 up to a column and
+// of 128 from there on, where that brings the longest cluster down by a fourteenth (2048 x 3224 x 768 on pairs: 104 tiles of 256 columns are
+// two rounds on 74 clusters, 30.1 us; 64 and 80 of 128 are one and a half).  The answer depends on the shapes alone and is kept (256 of
+// them).  Returns the number of problems.
+struct CutKey {
+  int n, slots; int64_t v[3 * MAX_GROUP];
+  bool operator<(const CutKey& o) const { return n != o.n ? n < o.n : slots != o.slots ? slots < o.slots : std::lexicographical_compare(v, v + 3 * MAX_GROUP, o.v, o.v + 3 * MAX_GROUP); }
+};
+struct Cut { int which, at; };
+static int cut_widths(Group* g, int n, int slots) {
+  int64_t tiles = 0;
+  for (int i = 0; i < n; ++i) tiles += g->pr[i].tiles;
+  if (n >= MAX_GROUP || tiles <= slots || tiles > 4 * slots) return n;
+  static std::map<CutKey, Cut> known;
+  static std::mutex mu;
+  CutKey key{};
+  key.n = n; key.slots = slots;
+  for (int i = 0; i < n; ++i) { key.v[3 * i] = g->pr[i].p.M; key.v[3 * i + 1] = g->pr[i].p.N; key.v[3 * i + 2] = (int64_t)g->pr[i].p.kt_per << 32 | g->pr[i].p.K; }
+  auto apply = [&](const Cut& c, Group* to) {
+    for (int i = n; i > c.which; --i) to->pr[i] = to->pr[i - 1];
+    Problem &a = to->pr[c.which], &b = to->pr[c.which + 1];
+    a.n_begin = 0; a.n_end = c.at; b.n_begin = c.at; b.n_end = b.p.N;
+    set_tiles(&a, 256); set_tiles(&b, 128);
+  };
+  Cut best{-1, 0};
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = known.find(key);
+    if (it != known.end()) best = it->second;
+    else {
+      double t0 = makespan_exact(g, n, slots) * (13.0 / 14.0);
+      for (int i = 0; i < n; ++i)
+        for (int at = 256; at < g->pr[i].p.N; at += 256) {
+          Group h = *g;
+          apply(Cut{i, at}, &h);
+          const double t = makespan_exact(&h, n + 1, slots);
+          if (t < t0) { t0 = t; best = Cut{i, at}; }
+        }
+      if (known.size() >= 256) known.clear();
+      known.emplace(key, best);
+    }
+  }
+  if (best.which < 0) return n;
+  apply(best, g);
+  return n + 1;
 }
 
 }  // namespace hb
@@ -1513,14 +1583,16 @@ pmb_status gemm_pairs_group(cudaStream_t st, const PairGemm* gs, int n, int tile
   for (int i = 0; i < n; ++i) if ((gs[i].emit.hi || gs[i].ksplit > 1) && pair_mode <= 2) pair_mode = 0;      // (the one-tile-per-cluster kernels do not write the pair output)
   if (pair_mode) {
     const int64_t slots = persistent_grid(148) / 2;
-    if (pair_mode == 4) choose_widths(&g, n, (int)slots);
+    int np = n;
+    if (pair_mode == 4) { choose_widths(&g, n, (int)slots); np = cut_widths(&g, n, (int)slots); }
     else for (int i = 0; i < n; ++i) set_tiles(&g.pr[i], pair_mode == 2 ? 256 : 128);
     PMB_SMEM_OPT_IN((PairCfg<true, 256>::SMEM_BYTES), gemm_bf16_pair_kernel<true, 256>);
     PMB_SMEM_OPT_IN((PairCfg<true, 128>::SMEM_BYTES), gemm_bf16_pair_kernel<true, 128>);
     int64_t clusters = 0;
-    for (int i = 0; i < n; ++i) {
-      const PairGemm& e = gs[i];
+    for (int i = 0, of = 0; i < np; ++i) {
       Problem& q = g.pr[i];
+      if (i > 0 && q.n_begin == 0) ++of;                     // (the product that the problem is of)
+      const PairGemm& e = gs[of];
       // B boxes of the pair kernels are half a tile tall (K-major tiles); MN-major boxes stay 64 columns wide
       const int half = q.p.bn / 2;
       if (e.tb) { PMB_TRY(make_map(&q.mB, e.B.hi, e.K, e.N, e.B.ld, TBK, half)); PMB_TRY(make_map(&q.mBlo, e.B.lo, e.K, e.N, e.B.ld, TBK, half)); }
@@ -1529,7 +1601,7 @@ pmb_status gemm_pairs_group(cudaStream_t st, const PairGemm* gs, int n, int tile
     if (pair_mode >= 3) {
       ProfScope prof(st, "gemm_bf16x2", flops, bytes);
       const unsigned grid = 2u * (unsigned)(clusters < slots ? clusters : slots);
-      set_lead(&g, n, (int)(grid / 2));
+      set_lead(&g, np, (int)(grid / 2));
       if (pair_mode == 4) {
         PMB_SMEM_OPT_IN((PairPCfg<true, 256>::SMEM_BYTES), gemm_bf16_pairp_kernel<true, 256>);
         PMB_TRY(launch_pdl(st, gemm_bf16_pairp_kernel<true, 256>, grid, (PairPCfg<true, 256>::THREADS), PairPCfg<true, 256>::SMEM_BYTES, g, (int)clusters));

@@ -443,6 +443,17 @@ def test_scan_bf16_strong_decay(pm, T, Q, N, strength):
         assert_close(got, want, tol=tol, what=what)
 
 
+# products whose columns go to tiles of two widths: two rounds of tiles, a cut inside and one before the last tile, B in either order, a residual
+@pytest.mark.parametrize("M,N,K", [(2048, 3224, 768), (1337, 3224, 136), (1000, 5000, 64)])
+@pytest.mark.parametrize("tb,res", [(False, False), (True, True)])
+def test_gemm_columns_cut(pm, M, N, K, tb, res):
+    a, b, r = randn((M, K), 1).cuda(), randn((N, K) if tb else (K, N), 2).cuda(), randn((M, N), 3).cuda()
+    out = pm.matmul(a, b, trans_b=tb, residual=r if res else None)
+    assert pm.device_status() == 0
+    want = a.double() @ (b.T if tb else b).double() + (r.double() if res else 0.0)
+    assert_close(out, want, tol=3e-5, what=f"{M}x{N}x{K}")
+
+
 # kernels that start while the one before them in the stream is still at work wait for it before they touch memory: calls one after the
 # other on buffers that each of them overwrites give what they give one at a time (the sums have fixed orders: equal bits)
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
