@@ -7,8 +7,8 @@
 // through shared memory.  The launches are chained with programmatic dependent launch: a kernel is placed while its predecessor
 // runs, requests the weights or state it will need, and only then waits.  (A kernel that waits does so for everything enqueued
 // before, because its predecessor did.)
-// Measured: 1 sequence at d_model 768, 24 heads of 64 x 64: 71 -> 16 us a step (host included; splitting both weights into
-// pairs on every call and GEMM tiles of 128 rows before); 256 at d_model 2048, 32 heads of 64 x 128: 228 -> 145 us, of which the
+// Measured: 1 sequence at d_model 768, 24 heads of 64 x 64: 71 -> 16 -> 14.2 us a step, which is the host's time for it (splitting both
+// weights into pairs on every call and GEMM tiles of 128 rows before; 10.1 when replayed from a graph); 256 at d_model 2048, 32 heads of 64 x 128: 228 -> 145 us, of which the
 // state takes 81 (537 MB, 6.6 TB/s).
 #include <cuda_bf16.h>
 #include "common.cuh"
@@ -58,48 +58,69 @@ __device__ __forceinline__ void in_proj_column(const StepIn& s, int b, int j, fl
 }
 
 // ---- up to 16 sequences: out[b, j] = sum_k in[b, k] W[k, j] on FMA ------------------------------------------------------------
-// CTA = 32 columns: 8 lanes x 16 bytes across a weight row, 32 rows in flight per pass (8 warps x 4), 8 passes requested at
-// once; the inputs sit in shared memory as [k][b].  OUT = 0: in_proj with the conv step and softplus in the epilogue.
-// OUT = 1: out_proj of the gated, normalised y (g y silu(z) and its per-head sums of squares come from the state kernel).
-constexpr int GV_THREADS = 256, GV_COLS = 32, GV_AHEAD = 8;
+// CTA = 4 CW columns: CW lanes x 16 bytes across a weight row, a thread takes four adjacent rows at a time (one 16-byte read of a
+// sequence's inputs, which sit in shared memory as they lie in memory, serves 16 products) and has GV_GROUPS such groups in flight.
+// What bounds it is the chain launch, inputs, weights, reduction, and beyond four sequences the fetching of the inputs by every CTA.
+// Inputs interleaved by sequence, stored a float at a time 8 or 16 ways to a bank, and tiles of 32 columns took, in us per step (24 heads
+// of 64 x 64 at d_model 768): 2 sequences 20.5, 4: 25.2, 8: 36.2, 16: 56.7; now 14.1, 14.6, 18.4, 27.2 (32 heads of 64 x 128 at 2048: 1 sequence 31.6 -> 21.1, 8: 60.8 -> 31.4, 16: 94.7 -> 48.1).
+// OUT = 0: in_proj with the conv step and softplus in the epilogue.
+// OUT = 1: out_proj of the gated, normalised y (g = y silu(z) and its per-head sums of squares come from the state kernel; the row's
+// rstd is one factor of the result).
+constexpr int GV_THREADS = 256, GV_GROUPS = 3;
 struct GemvArgs {
   int B, K, N; const float* W; int64_t ldw;
-  const float* in; int64_t ldin;                         // OUT 0: x_t
-  const float* g; const float* ss; int H; const float* norm_w; float eps;   // OUT 1
+  const float* in;                                       // OUT 0: x_t (B, K); OUT 1: g
+  bool in_vec;                                           // `in` (and norm_w) can be read 16 bytes at a time
+  const float* ss; int H; const float* norm_w; float eps;   // OUT 1
   float* out; StepIn st;
 };
-template <int BT, int OUT>
+template <int BT, int OUT, int CW>
 __global__ void __launch_bounds__(GV_THREADS) gemv_kernel(const GemvArgs a) {
-  extern __shared__ __align__(16) float sx[];             // [K][BT], then the partial sums [8][BT][32]
+  constexpr int COLS = 4 * CW, PASS = 4 * (GV_THREADS / CW);                 // columns; weight rows of one group of all threads
+  extern __shared__ __align__(16) float sx[];             // [BT][K], then the partial sums [8][BT][COLS]
   __shared__ float rs[16];
-  const int tid = threadIdx.x, tx = tid & 7, ks = tid >> 3, warp = tid >> 5, lane = tid & 31;
-  const int j = blockIdx.x * GV_COLS + 4 * tx;
-  const bool jin = j < a.N;                               // (N is a multiple of 4)
-  const float* wp = a.W + (int64_t)ks * a.ldw + (jin ? j : 0);
-  float4 w[GV_AHEAD];
-  auto request = [&](int k0) {
+  const int tid = threadIdx.x, tx = tid % CW, k4 = 4 * (tid / CW), warp = tid >> 5, lane = tid & 31;
+  const int j = blockIdx.x * COLS + 4 * tx;
+  const bool jin = j < a.N;                               // (N and K are multiples of 4)
+  const float* wp = a.W + (int64_t)k4 * a.ldw + (jin ? j : 0);
+  float4 w[GV_GROUPS][4];
+  auto request = [&](int u, int k0) {
 #pragma unroll
-    for (int u = 0; u < GV_AHEAD; ++u) {
-      const int k = k0 + 32 * u + ks;
-      w[u] = jin && k < a.K ? __ldg(reinterpret_cast<const float4*>(wp + (int64_t)(k0 + 32 * u) * a.ldw)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
+    for (int r = 0; r < 4; ++r)
+      w[u][r] = jin && k0 + k4 < a.K ? __ldg(reinterpret_cast<const float4*>(wp + (int64_t)(k0 + r) * a.ldw)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   };
-  request(0);                                             // (weights do not depend on the kernel before)
-  pdl_launch();
-  pdl_wait();
-  if (OUT == 1) {
-    if (tid < BT) {
-      float t = 0.0f;
-      if (tid < a.B) for (int h = 0; h < a.H; ++h) t += a.ss[(int64_t)tid * a.H + h];       // fixed order
-      rs[tid] = 1.0f / sqrtf(t / (float)a.K + a.eps);
+  // in_proj follows whatever the caller put in the stream, which may have written the weights and the state: it waits first, and only
+  // then lets the state kernel in, which reads the state before its own wait.  What out_proj requests is older than the step.
+  if (OUT == 0) { pdl_wait(); pdl_launch(); }
+#pragma unroll
+  for (int u = 0; u < GV_GROUPS; ++u) request(u, u * PASS);
+  if (OUT == 1) { pdl_launch(); pdl_wait(); }
+  const int kq = a.K >> 2;
+#pragma unroll 4
+  for (int i = tid; i < kq * BT; i += GV_THREADS) {
+    const int b = BT == 1 ? 0 : i / kq, k = 4 * (i - b * kq);
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (b < a.B) {
+      const float* p = a.in + (int64_t)b * a.K + k;
+      float4 n = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+      if (a.in_vec) {
+        v = *reinterpret_cast<const float4*>(p);
+        if (OUT == 1) n = __ldg(reinterpret_cast<const float4*>(a.norm_w + k));
+      } else {
+        v = make_float4(p[0], p[1], p[2], p[3]);
+        if (OUT == 1) n = make_float4(a.norm_w[k], a.norm_w[k + 1], a.norm_w[k + 2], a.norm_w[k + 3]);
+      }
+      if (OUT == 1) { v.x *= n.x; v.y *= n.y; v.z *= n.z; v.w *= n.w; }
     }
-    __syncthreads();
+    *reinterpret_cast<float4*>(sx + b * a.K + k) = v;
   }
-  for (int i = tid; i < a.K * BT; i += GV_THREADS) {
-    const int b = i / a.K, k = i - b * a.K;               // (lanes along k: coalesced)
-    float v = 0.0f;
-    if (b < a.B) v = OUT == 0 ? a.in[b * a.ldin + k] : a.g[(int64_t)b * a.K + k] * rs[b] * a.norm_w[k];
-    sx[k * BT + b] = v;
+  if (OUT == 1) {
+    for (int b = warp; b < a.B; b += GV_THREADS / 32) {
+      float t = 0.0f;
+      for (int h = lane; h < a.H; h += 32) t += a.ss[(int64_t)b * a.H + h];
+      t = warp_sum(t);
+      if (lane == 0) rs[b] = 1.0f / sqrtf(t / (float)a.K + a.eps);
+    }
   }
   __syncthreads();
   float acc[BT][4];
@@ -107,46 +128,46 @@ __global__ void __launch_bounds__(GV_THREADS) gemv_kernel(const GemvArgs a) {
   for (int b = 0; b < BT; ++b)
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[b][e] = 0.0f;
-  for (int k0 = 0; k0 < a.K; k0 += 32 * GV_AHEAD) {
-    float4 c[GV_AHEAD];
+  for (int k0 = 0; k0 < a.K; k0 += GV_GROUPS * PASS) {
 #pragma unroll
-    for (int u = 0; u < GV_AHEAD; ++u) c[u] = w[u];
-    if (k0 + 32 * GV_AHEAD < a.K) request(k0 + 32 * GV_AHEAD);
-#pragma unroll
-    for (int u = 0; u < GV_AHEAD; ++u) {
-      const int k = k0 + 32 * u + ks;
+    for (int u = 0; u < GV_GROUPS; ++u) {
+      const int k = k0 + u * PASS + k4;
       if (k < a.K) {
 #pragma unroll
         for (int b = 0; b < BT; ++b) {
-          const float xv = sx[k * BT + b];
-          acc[b][0] = fmaf(xv, c[u].x, acc[b][0]); acc[b][1] = fmaf(xv, c[u].y, acc[b][1]);
-          acc[b][2] = fmaf(xv, c[u].z, acc[b][2]); acc[b][3] = fmaf(xv, c[u].w, acc[b][3]);
+          const float4 xv = *reinterpret_cast<const float4*>(sx + b * a.K + k);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const float xr = r == 0 ? xv.x : (r == 1 ? xv.y : (r == 2 ? xv.z : xv.w));
+            acc[b][0] = fmaf(xr, w[u][r].x, acc[b][0]); acc[b][1] = fmaf(xr, w[u][r].y, acc[b][1]);
+            acc[b][2] = fmaf(xr, w[u][r].z, acc[b][2]); acc[b][3] = fmaf(xr, w[u][r].w, acc[b][3]);
+          }
         }
       }
+      request(u, k0 + (GV_GROUPS + u) * PASS);
     }
   }
 #pragma unroll
   for (int b = 0; b < BT; ++b)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      acc[b][e] += __shfl_xor_sync(0xffffffffu, acc[b][e], 8);
-      acc[b][e] += __shfl_xor_sync(0xffffffffu, acc[b][e], 16);
-    }
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+      for (int m = CW; m < 32; m *= 2) acc[b][e] += __shfl_xor_sync(0xffffffffu, acc[b][e], m);
   __syncthreads();
   float* red = sx;
-  if (lane < 8) {
+  if (lane < CW) {
 #pragma unroll
-    for (int b = 0; b < BT; ++b) *reinterpret_cast<float4*>(red + (warp * BT + b) * GV_COLS + 4 * lane) = make_float4(acc[b][0], acc[b][1], acc[b][2], acc[b][3]);
+    for (int b = 0; b < BT; ++b) *reinterpret_cast<float4*>(red + (warp * BT + b) * COLS + 4 * lane) = make_float4(acc[b][0], acc[b][1], acc[b][2], acc[b][3]);
   }
   __syncthreads();
-  for (int i = tid; i < BT * GV_COLS; i += GV_THREADS) {
-    const int b = i / GV_COLS, col = blockIdx.x * GV_COLS + i % GV_COLS;
+  for (int i = tid; i < BT * COLS; i += GV_THREADS) {
+    const int b = i / COLS, col = blockIdx.x * COLS + i % COLS;
     if (b >= a.B || col >= a.N) continue;
     float v = 0.0f;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) v += red[(q * BT + b) * GV_COLS + i % GV_COLS];
+    for (int q = 0; q < 8; ++q) v += red[(q * BT + b) * COLS + i % COLS];
     if (OUT == 0) in_proj_column(a.st, b, col, v);
-    else a.out[(int64_t)b * a.N + col] = v;
+    else a.out[(int64_t)b * a.N + col] = v * rs[b];
   }
 }
 
@@ -522,27 +543,27 @@ extern "C" size_t pmb_mamba2_step_workspace_bytes(const pmb_mamba2_config* cfg, 
 constexpr size_t GEMV_MAX_SMEM = 200 * 1024;
 static int gemv_tile(int B) { return B > 8 ? 16 : (B > 4 ? 8 : (B > 2 ? 4 : (B > 1 ? 2 : 1))); }
 static size_t gemv_smem(int B, int K) {
-  const size_t bt = (size_t)gemv_tile(B), a = (size_t)K * bt, b = 8 * bt * dec::GV_COLS;
+  const size_t bt = (size_t)gemv_tile(B), a = (size_t)K * bt, b = 8 * bt * 32;      // (32: the widest tile's columns)
   return (a > b ? a : b) * sizeof(float);
 }
-template <int BT, int OUT>
-static pmb_status gemv_bt(cudaStream_t st, const dec::GemvArgs& a, bool pdl) {
-  PMB_SMEM_OPT_IN(GEMV_MAX_SMEM, dec::gemv_kernel<BT, OUT>);
-  const unsigned grid = (unsigned)cdiv(a.N, dec::GV_COLS);
-  const size_t smem = gemv_smem(a.B, a.K);
-  if (pdl) return launch_pdl(st, dec::gemv_kernel<BT, OUT>, dim3(grid), dec::GV_THREADS, smem, a);
-  dec::gemv_kernel<BT, OUT><<<grid, dec::GV_THREADS, smem, st>>>(a);
-  PMB_LAUNCHED();
-  return PMB_OK;
+template <int BT, int OUT, int CW>
+static pmb_status gemv_cw(cudaStream_t st, const dec::GemvArgs& a) {
+  PMB_SMEM_OPT_IN(GEMV_MAX_SMEM, dec::gemv_kernel<BT, OUT, CW>);
+  return launch_pdl(st, dec::gemv_kernel<BT, OUT, CW>, dim3((unsigned)cdiv(a.N, 4 * CW)), dec::GV_THREADS, gemv_smem(a.B, a.K), a);
 }
 template <int OUT>
-static pmb_status gemv(cudaStream_t st, const dec::GemvArgs& a, bool pdl) {
+static pmb_status gemv(cudaStream_t st, const dec::GemvArgs& a) {
+  // Tiles of 16 columns for in_proj and of 8 for out_proj, which has fewer and longer ones: more CTAs, and most or all of a thread's
+  // weights requested at once.  With 16 sequences a CTA holds 64 bytes of inputs per k, which every CTA has to fetch: twice the width.
+  // us per step with tiles of 32/32, 32/16, 16/16, 16/8, 8/8 (24 heads of 64 x 64 at d_model 768): 4 sequences 17.3, 16.1, 15.6, 14.6, 16.1;
+  // 8: 23.0, 20.4, 18.8, 18.4, 22.5; 16: 30.0, 27.1, 29.8, 28.3, 32.4; (32 heads of 64 x 128 at 2048) 1: 23.7, 22.4, 20.6, 21.0, 22.9;
+  // 8: 38.7, 35.4, 34.2, 31.4, 38.1; 16: 53.1, 48.2, 53.3, 65.1, 78.6.
   switch (gemv_tile(a.B)) {
-    case 1: return gemv_bt<1, OUT>(st, a, pdl);
-    case 2: return gemv_bt<2, OUT>(st, a, pdl);
-    case 4: return gemv_bt<4, OUT>(st, a, pdl);
-    case 8: return gemv_bt<8, OUT>(st, a, pdl);
-    default: return gemv_bt<16, OUT>(st, a, pdl);
+    case 1: return gemv_cw<1, OUT, OUT ? 2 : 4>(st, a);
+    case 2: return gemv_cw<2, OUT, OUT ? 2 : 4>(st, a);
+    case 4: return gemv_cw<4, OUT, OUT ? 2 : 4>(st, a);
+    case 8: return gemv_cw<8, OUT, OUT ? 2 : 4>(st, a);
+    default: return gemv_cw<16, OUT, OUT ? 4 : 8>(st, a);
   }
 }
 
@@ -598,17 +619,17 @@ extern "C" pmb_status pmb_mamba2_step(void* stream, const pmb_mamba2_config* cfg
   const dec::StateArgs sa{w.act, w.dt, w.z, d.I, p->a_log, p->d_skip, d_ssm_state, w.g, w.ss, d.H, d.G, d.N, d.P, d.X, d.I};
   // Up to 16 sequences the products are fp32 FMA (y 2e-7 of its norm from fp64), beyond on bf16 pairs (7e-6).  Where the line
   // lies is a matter of that precision, not of time.  us per step, FMA / tensor cores (24 heads of 64 x 64 at d_model 768; 32 of 64 x 128
-  // at d_model 2048): 1 sequence 14.2 / 19.0, 19.6 / 26.6; 2: 18.1 / 19.8, 26.6 / 28.3; 4: 22.5 / 20.3, 35.3 / 28.4; 8: 32.9 / 22.1, 50.0 / 29.0;
-  // 16: 55.3 / 22.6, 81.0 / 31.1; 17: 22.9 and 31.6.  (From five on the inputs' stores to shared memory go 8 or 16 ways to a bank.)
+  // at d_model 2048): 1 sequence 14.2 / 19.0, 21.1 / 26.6; 2: 14.1 / 19.8, 23.9 / 28.3; 4: 14.6 / 20.3, 28.3 / 28.4; 8: 18.4 / 22.1, 31.4 / 29.0;
+  // 16: 27.2 / 22.6, 48.1 / 31.1; 17: 22.9 and 31.6.
   if (vec && d.B <= 16 && gemv_smem(d.B, d.D) <= GEMV_MAX_SMEM && gemv_smem(d.B, d.I) <= GEMV_MAX_SMEM) {
     dec::GemvArgs a{};
-    a.B = d.B; a.K = d.D; a.N = d.J; a.W = p->in_proj_weight; a.ldw = d.J; a.in = d_x_t; a.ldin = d.D; a.st = si;
-    { ProfScope prof(st, "decode_in_proj", 2.0 * d.B * d.D * d.J, 4.0 * d.D * d.J); PMB_TRY(gemv<0>(st, a, false)); }
+    a.B = d.B; a.K = d.D; a.N = d.J; a.W = p->in_proj_weight; a.ldw = d.J; a.in = d_x_t; a.in_vec = al(d_x_t); a.st = si;
+    { ProfScope prof(st, "decode_in_proj", 2.0 * d.B * d.D * d.J, 4.0 * d.D * d.J); PMB_TRY(gemv<0>(st, a)); }
     PMB_TRY(launch_state_step(st, d, sa));
     dec::GemvArgs o{};
-    o.B = d.B; o.K = d.I; o.N = d.D; o.W = p->out_proj_weight; o.ldw = d.D; o.g = w.g; o.ss = w.ss; o.H = d.H; o.norm_w = p->norm_weight; o.eps = d.eps; o.out = d_y_t;
+    o.B = d.B; o.K = d.I; o.N = d.D; o.W = p->out_proj_weight; o.ldw = d.D; o.in = w.g; o.in_vec = al(w.g) && al(p->norm_weight); o.ss = w.ss; o.H = d.H; o.norm_w = p->norm_weight; o.eps = d.eps; o.out = d_y_t;
     ProfScope prof(st, "decode_out_proj", 2.0 * d.B * d.D * d.I, 4.0 * d.D * d.I);
-    return gemv<1>(st, o, true);
+    return gemv<1>(st, o);
   }
   const bool tc = vec && d.D % 8 == 0 && d.I % 8 == 0;
   int n_in = 1;

@@ -161,6 +161,27 @@ def test_decode_batches(pm, B, D, H, P, N, G):
     assert pm.device_status() == 0
 
 
+# weight rows that take a thread more than one pass of its groups, with a remainder, on both products; offset 1: the token and the norm's
+# weight off the 16-byte grid
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("B", [1, 2, 4, 8, 16])
+def test_decode_long_rows(pm, B, offset):
+    def off_grid(t):
+        return torch.cat([t.new_zeros(offset), t.flatten()])[offset:].view(t.shape)
+
+    D, H, P, N = 1028, 13, 128, 12
+    cfg, p, blk = _block(pm, D, H, P, N, 1, 64, torch.float32)
+    blk.params["norm_weight"] = off_grid(blk.params["norm_weight"])
+    ref = {"ssm_state": randn((B, H, N, P), 7, 0.3), "conv_window": randn((B, cfg.xbc_dim, 3), 8, 0.5)}
+    st = {k: v.cuda() for k, v in ref.items()}
+    x = randn((B, 1, D), 20)
+    y, st = blk.step(off_grid(x.cuda()), st)
+    y_ref, ref = orc.block_step(p, cfg, x, ref)
+    assert_close(y, y_ref, what="y")
+    assert_close(st["ssm_state"], ref["ssm_state"], what="state")
+    assert_close(st["conv_window"], ref["conv_window"], what="window")
+
+
 # more sequences than a grid has rows, on the general and on the tensor-core route of the projections
 @pytest.mark.parametrize("D,H,P,N", [(16, 1, 8, 4), (16, 2, 4, 7)])
 def test_decode_many_sequences(pm, D, H, P, N):
