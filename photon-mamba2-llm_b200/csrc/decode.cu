@@ -6,7 +6,9 @@
 // step + gate, norm + out_proj), beyond that a tensor-core kernel that turns each weight tile into a bf16 pair on its way
 // through shared memory.  The launches are chained with programmatic dependent launch: a kernel is placed while its predecessor
 // runs, requests the weights or state it will need, and only then waits.  (A kernel that waits does so for everything enqueued
-// before, because its predecessor did.)
+// before, because its predecessor did.)  What is requested early has to be older than the step: so in_proj, which may follow any kernel
+// and be placed while several are at work, reads nothing before its wait, and the kernel in front of the state step lets that one in only
+// after its own wait.
 // Measured: 1 sequence at d_model 768, 24 heads of 64 x 64: 71 -> 16 -> 14.2 us a step, which is the host's time for it (splitting both
 // weights into pairs on every call and GEMM tiles of 128 rows before; 10.1 when replayed from a graph); 256 at d_model 2048, 32 heads of 64 x 128: 228 -> 145 us, of which the
 // state takes 81 (537 MB, 6.6 TB/s).
@@ -296,7 +298,7 @@ template <int NB> struct SkGeo {
   static constexpr int SMEM = SK_STAGES * STAGE + 1024 + 256;
 };
 struct SkMaps { CUtensorMap x[2]; };
-struct SkArgs { const float* W; int64_t ldw; int K, J, B, kt_per; float* slab; unsigned int* status; };
+struct SkArgs { const float* W; int64_t ldw; int K, J, B, kt_per; bool early; float* slab; unsigned int* status; };    // early: W is older than the kernel before
 
 template <int NB>
 __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid_constant__ SkMaps maps, const SkArgs a) {
@@ -336,7 +338,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
   };
   if (warp == 0) {
     if (lane == 0) {
-      pdl_wait();                                          // (x comes from the kernel before; the weights do not)
+      pdl_wait();                                          // (x comes from the kernel before)
       int issued = 0;
       for (int kt = kt0; kt < kt1; ++kt) {
         const int it = kt - kt0, s = it % SK_STAGES;
@@ -418,6 +420,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(WFULL + s));
     };
+    if (!a.early) pdl_wait();
     request(kt0, wa);
     request(kt0 + 1, wb);
     for (int kt = kt0; kt < kt1 && ok; kt += 2) {
@@ -454,8 +457,8 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
 // ends; a linear grid costs a division, 0.5 us of 30 at 24 sequences)
 constexpr int FINISH_Y = 65535;
 __global__ void __launch_bounds__(256) in_proj_finish_kernel(const float* __restrict__ slab, int n, StepIn s) {
-  pdl_launch();
   pdl_wait();
+  pdl_launch();                                            // (in this order: the state step reads the state before it waits)
   const int j = (int)(blockIdx.x * blockDim.x + threadIdx.x), b = (int)(blockIdx.y + blockIdx.z * FINISH_Y);
   if (j >= s.J || b >= s.B) return;
   const float* p = slab + (int64_t)b * s.J + j;
@@ -570,23 +573,23 @@ static pmb_status gemv(cudaStream_t st, const dec::GemvArgs& a) {
 namespace pmb { namespace hb { pmb_status pair_operand_map(CUtensorMap* map, const uint16_t* base, int64_t inner, int64_t outer, int64_t ld, int box_inner, int box_outer); } }
 
 template <int NB>
-static pmb_status skinny_nb(cudaStream_t st, const uint16_t* hi, const uint16_t* lo, int64_t B, int64_t K, int64_t J, const float* W, float* slab, int splits) {
+static pmb_status skinny_nb(cudaStream_t st, const uint16_t* hi, const uint16_t* lo, int64_t B, int64_t K, int64_t J, const float* W, bool early, float* slab, int splits) {
   static unsigned int* known[PMB_MAX_DEVICES] = {nullptr};
   unsigned int* status = tcx::status_address(g_decode_status, known);
   if (!status) return fail(PMB_ERR_CUDA, "decode: no status word on this device");
   dec::SkMaps ms{};
   PMB_TRY(hb::pair_operand_map(&ms.x[0], hi, K, B, K, dec::SK_BK, NB));
   PMB_TRY(hb::pair_operand_map(&ms.x[1], lo, K, B, K, dec::SK_BK, NB));
-  dec::SkArgs a{W, J, (int)K, (int)J, (int)B, (int)cdiv(cdiv(K, dec::SK_BK), splits), slab, status};
+  dec::SkArgs a{W, J, (int)K, (int)J, (int)B, (int)cdiv(cdiv(K, dec::SK_BK), splits), early, slab, status};
   PMB_SMEM_OPT_IN(dec::SkGeo<NB>::SMEM, dec::skinny_gemm_kernel<NB>);
   ProfScope prof(st, "decode_gemm", 2.0 * B * K * J, 4.0 * ((double)K * J + (double)splits * B * J));
   return launch_pdl(st, dec::skinny_gemm_kernel<NB>, dim3((unsigned)cdiv(J, 128), (unsigned)splits, (unsigned)cdiv(B, NB)), dec::SK_THREADS, dec::SkGeo<NB>::SMEM, ms, a);
 }
-static pmb_status skinny(cudaStream_t st, const uint16_t* hi, const uint16_t* lo, int64_t B, int64_t K, int64_t J, const float* W, float* slab, int splits) {
-  if (B > 128) return skinny_nb<256>(st, hi, lo, B, K, J, W, slab, splits);
-  if (B > 64) return skinny_nb<128>(st, hi, lo, B, K, J, W, slab, splits);
-  if (B > 32) return skinny_nb<64>(st, hi, lo, B, K, J, W, slab, splits);
-  return skinny_nb<32>(st, hi, lo, B, K, J, W, slab, splits);
+static pmb_status skinny(cudaStream_t st, const uint16_t* hi, const uint16_t* lo, int64_t B, int64_t K, int64_t J, const float* W, bool early, float* slab, int splits) {
+  if (B > 128) return skinny_nb<256>(st, hi, lo, B, K, J, W, early, slab, splits);
+  if (B > 64) return skinny_nb<128>(st, hi, lo, B, K, J, W, early, slab, splits);
+  if (B > 32) return skinny_nb<64>(st, hi, lo, B, K, J, W, early, slab, splits);
+  return skinny_nb<32>(st, hi, lo, B, K, J, W, early, slab, splits);
 }
 
 static pmb_status launch_state_step(cudaStream_t st, const Dims& d, const dec::StateArgs& s) {
@@ -636,7 +639,7 @@ extern "C" pmb_status pmb_mamba2_step(void* stream, const pmb_mamba2_config* cfg
   if (tc) {
     n_in = skinny_splits(d.B, d.J, d.D);
     PMB_TRY(split_pair16(st, d_x_t, d.B, d.D, d.D, w.x_hi, w.x_lo, d.D));
-    PMB_TRY(skinny(st, w.x_hi, w.x_lo, d.B, d.D, d.J, p->in_proj_weight, w.slab, n_in));
+    PMB_TRY(skinny(st, w.x_hi, w.x_lo, d.B, d.D, d.J, p->in_proj_weight, false, w.slab, n_in));
   } else {
     PMB_TRY(gemm(st, 0, 0, d.B, d.J, d.D, d_x_t, d.D, p->in_proj_weight, d.J, w.slab, d.J, nullptr, 0));
   }
@@ -650,6 +653,6 @@ extern "C" pmb_status pmb_mamba2_step(void* stream, const pmb_mamba2_config* cfg
   if (!tc) return gemm(st, 0, 0, d.B, d.D, d.I, w.normed, d.I, p->out_proj_weight, d.D, d_y_t, d.D, nullptr, 0);
   const int n_out = skinny_splits(d.B, d.D, d.I);
   const bool direct = n_out == 1 || !al(d_y_t);
-  PMB_TRY(skinny(st, w.n_hi, w.n_lo, d.B, d.I, d.D, p->out_proj_weight, direct ? d_y_t : w.slab, direct ? 1 : n_out));
+  PMB_TRY(skinny(st, w.n_hi, w.n_lo, d.B, d.I, d.D, p->out_proj_weight, true, direct ? d_y_t : w.slab, direct ? 1 : n_out));
   return direct ? PMB_OK : sum_slabs(st, w.slab, n_out, (int64_t)d.B * d.D, (int64_t)d.B * d.D, d_y_t, 0);
 }

@@ -182,6 +182,33 @@ def test_decode_long_rows(pm, B, offset):
     assert_close(st["conv_window"], ref["conv_window"], what="window")
 
 
+# steps that follow one another without a pause read what the step before wrote, and weights that a product just wrote: the same bits as with
+# the device idle in between; the projections on FMA, on the tensor cores and on the general kernels
+@pytest.mark.parametrize("B,D", [(1, 128), (16, 128), (40, 128), (400, 128), (400, 132)])
+def test_decode_steps_back_to_back(pm, B, D):
+    cfg, p, blk = _block(pm, D, 4, 64, 64, 1, 64, torch.float32)
+    x = [randn((B, 1, D), 20 + i).cuda() for i in range(12)]
+    eye, w = torch.eye(D, device="cuda"), [randn(tuple(blk.params["in_proj_weight"].shape), 40 + i, 0.1).cuda() for i in range(3)]
+
+    def run(pause):
+        st, ys = blk.zero_state(B), []
+        for i, xt in enumerate(x):
+            if i % 4 == 3:
+                pm.matmul(eye, w[i // 4], out=blk.params["in_proj_weight"])
+                pause()
+            y, st = blk.step(xt, st)
+            pause()
+            ys.append(y)
+        torch.cuda.synchronize()
+        return ys + [st["ssm_state"], st["conv_window"]]
+
+    first = blk.params["in_proj_weight"].clone()
+    want = run(torch.cuda.synchronize)
+    blk.params["in_proj_weight"].copy_(first)
+    for got, ref in zip(run(lambda: None), want):
+        assert torch.equal(got, ref)
+
+
 # more sequences than a grid has rows, on the general and on the tensor-core route of the projections
 @pytest.mark.parametrize("D,H,P,N", [(16, 1, 8, 4), (16, 2, 4, 7)])
 def test_decode_many_sequences(pm, D, H, P, N):
