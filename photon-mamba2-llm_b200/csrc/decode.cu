@@ -10,7 +10,7 @@
 // and be placed while several are at work, reads nothing before its wait, and the kernel in front of the state step lets that one in only
 // after its own wait.
 // Measured: 1 sequence at d_model 768, 24 heads of 64 x 64: 71 -> 16 -> 14.2 us a step, which is the host's time for it (splitting both
-// weights into pairs on every call and GEMM tiles of 128 rows before; 10.1 when replayed from a graph); 256 at d_model 2048, 32 heads of 64 x 128: 228 -> 145 us, of which the
+// weights into pairs on every call and GEMM tiles of 128 rows before; 10.1 when replayed from a graph); 256 at d_model 2048, 32 heads of 64 x 128: 228 -> 145 -> 130 us, of which the
 // state takes 81 (537 MB, 6.6 TB/s).
 #include <cuda_bf16.h>
 #include "common.cuh"
@@ -182,8 +182,17 @@ constexpr int STEP_THREADS = 256;
 __host__ __device__ constexpr int bc_floats(int N) { return (2 * N + 3) & ~3; }
 struct StateArgs {
   const float* act; const float* dt; const float* z; int64_t ldz; const float* a_log; const float* D;
-  float* state; float* g; float* ss; int H, G, N, P, X, I;
+  const float* norm_w;
+  float* state; float* g; uint16_t* hi; uint16_t* lo; float* ss; int H, G, N, P, X, I;      // hi: g norm_w as a (hi, lo) pair instead of g
 };
+// the gated output of one (b, i)
+__device__ __forceinline__ void store_gated(const StateArgs& s, int b, int i, float gv) {
+  const int64_t o = (int64_t)b * s.I + i;
+  if (!s.hi) { s.g[o] = gv; return; }
+  uint32_t h, l;
+  split_bf16_pair(gv * s.norm_w[i], h, l);
+  s.hi[o] = (uint16_t)h; s.lo[o] = (uint16_t)l;
+}
 template <int ITER>
 __global__ void __launch_bounds__(STEP_THREADS) state_step_kernel(const StateArgs s) {
   extern __shared__ __align__(16) float sh[];             // B (N), C (N), partial outputs (rows x P)
@@ -233,7 +242,7 @@ __global__ void __launch_bounds__(STEP_THREADS) state_step_kernel(const StateArg
     y = fmaf(Dh, arow[h * s.P + p], y);
     const float zv = s.z[b * s.ldz + h * s.P + p];
     const float gv = y * zv * sigmoid_acc(zv);
-    s.g[(int64_t)b * s.I + h * s.P + p] = gv;
+    store_gated(s, b, h * s.P + p, gv);
     q = fmaf(gv, gv, q);
   }
   const float tot = block_sum(q, red);
@@ -278,7 +287,7 @@ __global__ void __launch_bounds__(STEP_THREADS) state_step_any_kernel(const Stat
     y = fmaf(s.D[h], arow[h * s.P + p], y);
     const float zv = s.z[b * s.ldz + h * s.P + p];
     const float gv = y * zv * sigmoid_acc(zv);
-    s.g[(int64_t)b * s.I + h * s.P + p] = gv;
+    store_gated(s, b, h * s.P + p, gv);
     q = fmaf(gv, gv, q);
   }
   const float tot = block_sum(q, red);
@@ -290,6 +299,9 @@ __global__ void __launch_bounds__(STEP_THREADS) state_step_any_kernel(const Stat
 // once per NB sequences.  Eight warps load the fp32 weight tile (64 k x 128 j, whole 512-byte rows, the next tile requested
 // while this one is converted), split it into a bf16 pair and store it as the MN-major operand; x arrives as a pair by TMA.
 // lo*hi + hi*lo + hi*hi as in every fp32 product here.  K is split over CTAs so that the launch fills the machine once.
+// XC: x in fp32, converted by the same warps, for in_proj up to 64 sequences; a launch and a pass less (17 sequences, 24 heads: 25.3 -> 20.5 us a
+// step together with the norm's, which out_finish_kernel took over).  With more sequences the conversion in every CTA would cost more
+// than the pass: it grows with the tile, the weights' does not.
 using namespace tcx;
 constexpr int SK_BK = 64, SK_CONV = 8, SK_THREADS = 64 + 32 * SK_CONV, SK_STAGES = 2;
 template <int NB> struct SkGeo {
@@ -298,9 +310,19 @@ template <int NB> struct SkGeo {
   static constexpr int SMEM = SK_STAGES * STAGE + 1024 + 256;
 };
 struct SkMaps { CUtensorMap x[2]; };
-struct SkArgs { const float* W; int64_t ldw; int K, J, B, kt_per; bool early; float* slab; unsigned int* status; };    // early: W is older than the kernel before
+__device__ __forceinline__ void pairs8(const float4 (&w)[2], uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+  const float v[8] = {w[0].x, w[0].y, w[0].z, w[0].w, w[1].x, w[1].y, w[1].z, w[1].w};
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const __nv_bfloat162 hh = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+    const float2 hf = __bfloat1622float2(hh);
+    const __nv_bfloat162 ll = __floats2bfloat162_rn(v[2 * e] - hf.x, v[2 * e + 1] - hf.y);
+    hi[e] = *reinterpret_cast<const uint32_t*>(&hh); lo[e] = *reinterpret_cast<const uint32_t*>(&ll);
+  }
+}
+struct SkArgs { const float* W; int64_t ldw; const float* x; int K, J, B, kt_per; bool early; float* slab; unsigned int* status; };    // early: W is older than the kernel before
 
-template <int NB>
+template <int NB, bool XC>
 __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid_constant__ SkMaps maps, const SkArgs a) {
   using GE = SkGeo<NB>;
   extern __shared__ uint8_t smem_raw[];
@@ -310,7 +332,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 8 * NBAR);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;    // (uniform to the compiler)
   const int j0 = (int)blockIdx.x * 128, b0 = (int)blockIdx.z * NB;
   const int kt_all = (a.K + SK_BK - 1) / SK_BK, kt0 = (int)blockIdx.y * a.kt_per, kt1 = min(kt_all, kt0 + a.kt_per);
   if (threadIdx.x == 0) {
@@ -337,7 +359,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
     return false;
   };
   if (warp == 0) {
-    if (lane == 0) {
+    if (!XC && lane == 0) {
       pdl_wait();                                          // (x comes from the kernel before)
       int issued = 0;
       for (int kt = kt0; kt < kt1; ++kt) {
@@ -357,7 +379,7 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
     for (int kt = kt0; kt < kt1; ++kt) {
       const int it = kt - kt0, s = it % SK_STAGES;
       const uint32_t ph = (uint32_t)(it / SK_STAGES);
-      if (!__all_sync(0xffffffffu, wait(XFULL + s, ph, 2u) && wait(WFULL + s, ph, 2u))) break;
+      if (!__all_sync(0xffffffffu, (XC || wait(XFULL + s, ph, 2u)) && wait(WFULL + s, ph, 2u))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (elect_one()) {
         const uint32_t st = base + s * GE::STAGE;
@@ -389,21 +411,33 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
         w[i][1] = in && in1 ? __ldcs(reinterpret_cast<const float4*>(src + 4)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
     };
+    constexpr int XR = XC ? NB / 32 : 1;                               // x: eight columns k of rows xr + 32 i
+    const int xq = ct & 7, xr = ct >> 3;
+    float4 xa[XR][2], xb[XR][2];
+    auto request_x = [&](int kt, float4 (&x)[XR][2]) {
+#pragma unroll
+      for (int i = 0; i < XR; ++i) {
+        const int b = b0 + xr + 32 * i, k = kt * SK_BK + 8 * xq;       // (K is a multiple of 8)
+        const float* src = a.x + (int64_t)b * a.K + k;
+        const bool in = kt < kt1 && k < a.K && b < a.B;
+        x[i][0] = in ? *reinterpret_cast<const float4*>(src) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        x[i][1] = in ? *reinterpret_cast<const float4*>(src + 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+    };
     bool ok = true;
     // converts one tile into its stage and requests the tile two further on into the registers it came from
-    auto convert = [&](int kt, float4 (&w)[4][2]) {
+    auto convert = [&](int kt, float4 (&w)[4][2], float4 (&x)[XR][2]) {
       const int it = kt - kt0, s = it % SK_STAGES;
       uint32_t hi[4][4], lo[4][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float v[8] = {w[i][0].x, w[i][0].y, w[i][0].z, w[i][0].w, w[i][1].x, w[i][1].y, w[i][1].z, w[i][1].w};
+        pairs8(w[i], hi[i], lo[i]);
+      }
+      uint32_t xh[XR][4], xl[XR][4];
+      if (XC) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const __nv_bfloat162 hh = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
-          const float2 hf = __bfloat1622float2(hh);
-          const __nv_bfloat162 ll = __floats2bfloat162_rn(v[2 * e] - hf.x, v[2 * e + 1] - hf.y);
-          hi[i][e] = *reinterpret_cast<const uint32_t*>(&hh); lo[i][e] = *reinterpret_cast<const uint32_t*>(&ll);
-        }
+        for (int i = 0; i < XR; ++i) pairs8(x[i], xh[i], xl[i]);
+        request_x(kt + 2, x);
       }
       request(kt + 2, w);
       ok = __all_sync(0xffffffffu, ok && wait(EMPTY + s, (uint32_t)(it / SK_STAGES) ^ 1u, 4u));
@@ -416,16 +450,26 @@ __global__ void __launch_bounds__(SK_THREADS, 1) skinny_gemm_kernel(const __grid
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(o), "r"(hi[i][0]), "r"(hi[i][1]), "r"(hi[i][2]), "r"(hi[i][3]) : "memory");
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(o + GE::WT), "r"(lo[i][0]), "r"(lo[i][1]), "r"(lo[i][2]), "r"(lo[i][3]) : "memory");
       }
+      if (XC) {
+#pragma unroll
+        for (int i = 0; i < XR; ++i) {
+          const int r = xr + 32 * i;
+          const uint32_t o = base + s * GE::STAGE + 2 * GE::WT + (uint32_t)(r * 128 + ((xq ^ (r & 7)) << 4));
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(o), "r"(xh[i][0]), "r"(xh[i][1]), "r"(xh[i][2]), "r"(xh[i][3]) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(o + GE::XT), "r"(xl[i][0]), "r"(xl[i][1]), "r"(xl[i][2]), "r"(xl[i][3]) : "memory");
+        }
+      }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(WFULL + s));
     };
-    if (!a.early) pdl_wait();
+    if (XC || !a.early) pdl_wait();
     request(kt0, wa);
     request(kt0 + 1, wb);
+    if (XC) { request_x(kt0, xa); request_x(kt0 + 1, xb); }
     for (int kt = kt0; kt < kt1 && ok; kt += 2) {
-      convert(kt, wa);
-      if (kt + 1 < kt1 && ok) convert(kt + 1, wb);
+      convert(kt, wa, xa);
+      if (kt + 1 < kt1 && ok) convert(kt + 1, wb, xb);
     }
     ok = __all_sync(0xffffffffu, ok && wait(ACC, 0u, 8u));
     if (ok) {
@@ -461,6 +505,18 @@ __global__ void __launch_bounds__(256) in_proj_finish_kernel(const float* __rest
   pdl_launch();                                            // (in this order: the state step reads the state before it waits)
   const int j = (int)(blockIdx.x * blockDim.x + threadIdx.x), b = (int)(blockIdx.y + blockIdx.z * FINISH_Y);
   if (j >= s.J || b >= s.B) return;
+  // what the column's conv step needs is requested with the slabs (11.7 -> 10.7 us for 256 sequences, 2304 channels)
+  const int c = j - s.I;
+  const bool conv4 = s.K == 4 && c >= 0 && c < s.X;
+  float* win = s.window + ((int64_t)b * s.X + (conv4 ? c : 0)) * (s.K - 1);
+  float t3[3], w4[4], bias = 0.0f;
+  if (conv4) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) t3[k] = win[k];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w4[k] = __ldg(s.conv_w + 4 * c + k);
+    if (s.conv_b) bias = __ldg(s.conv_b + c);
+  }
   const float* p = slab + (int64_t)b * s.J + j;
   const int64_t pitch = (int64_t)s.B * s.J;
   float v = 0.0f;
@@ -471,12 +527,18 @@ __global__ void __launch_bounds__(256) in_proj_finish_kernel(const float* __rest
 #pragma unroll
     for (int u = 0; u < 4; ++u) v += t[u];
   }
+  if (conv4) {
+    win[0] = t3[1]; win[1] = t3[2]; win[2] = v;
+    const float u = fmaf(w4[3], v, fmaf(w4[2], t3[2], fmaf(w4[1], t3[1], fmaf(w4[0], t3[0], bias))));
+    s.act[(int64_t)b * s.X + c] = u * sigmoid_acc(u);
+    return;
+  }
   in_proj_column(s, b, j, v);
 }
 
-// g rstd w as a (hi, lo) pair (I a multiple of 8 then) or, hi == NULL, in fp32
-__global__ void __launch_bounds__(256) norm_kernel(const float* __restrict__ g, const float* __restrict__ ss, const float* __restrict__ w, uint16_t* __restrict__ hi,
-                                                   uint16_t* __restrict__ lo, float* __restrict__ out, int I, int H, float eps) {
+// g rstd w, for the general product
+__global__ void __launch_bounds__(256) norm_kernel(const float* __restrict__ g, const float* __restrict__ ss, const float* __restrict__ w, float* __restrict__ out, int I, int H,
+                                                   float eps) {
   __shared__ float rs;
   const int64_t b = blockIdx.x;
   pdl_launch();
@@ -488,14 +550,34 @@ __global__ void __launch_bounds__(256) norm_kernel(const float* __restrict__ g, 
   }
   __syncthreads();
   const float r = rs;
-  if (!hi) {
-    for (int i = threadIdx.x; i < I; i += blockDim.x) out[b * I + i] = g[b * I + i] * r * w[i];
-    return;
+  for (int i = threadIdx.x; i < I; i += blockDim.x) out[b * I + i] = g[b * I + i] * r * w[i];
+}
+
+// y[b] = rstd[b] (sum of out_proj's slabs); grid: sequences x 1024 columns (D is a multiple of 8).  The state step writes the pair of
+// g norm_w, so that no pass stands between it and out_proj (5.6 us of 138 at 256 sequences, 32 heads of 64 x 128).
+__global__ void __launch_bounds__(256) out_finish_kernel(const float* __restrict__ slab, int n, const float* __restrict__ ss, float* __restrict__ y, bool vec, int64_t BD, int D,
+                                                         int I, int H, float eps) {
+  const int64_t b = blockIdx.x;
+  const int j = (int)(blockIdx.y * 1024 + 4 * threadIdx.x);
+  pdl_launch();
+  pdl_wait();
+  const bool in = j < D;
+  const float* p = slab + b * D + (in ? j : 0);
+  float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float t = 0.0f;
+  for (int h = threadIdx.x & 31; h < H; h += 32) t += ss[b * H + h];
+  for (int q = 0; q < n; q += 4) {
+    float4 f[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) f[u] = q + u < n ? *reinterpret_cast<const float4*>(p + (q + u) * BD) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) { v.x += f[u].x; v.y += f[u].y; v.z += f[u].z; v.w += f[u].w; }
   }
-  for (int i = 4 * threadIdx.x; i < I; i += 4 * blockDim.x) {
-    const float4 v = *reinterpret_cast<const float4*>(g + b * I + i);
-    store_pair4(hi + b * I + i, lo + b * I + i, v.x * r * w[i], v.y * r * w[i + 1], v.z * r * w[i + 2], v.w * r * w[i + 3]);
-  }
+  const float r = 1.0f / sqrtf(warp_sum(t) / (float)I + eps);
+  if (!in) return;
+  float* o = y + b * D + j;
+  if (vec) *reinterpret_cast<float4*>(o) = make_float4(v.x * r, v.y * r, v.z * r, v.w * r);
+  else { o[0] = v.x * r; o[1] = v.y * r; o[2] = v.z * r; o[3] = v.w * r; }
 }
 
 }  // namespace dec
@@ -572,24 +654,27 @@ static pmb_status gemv(cudaStream_t st, const dec::GemvArgs& a) {
 
 namespace pmb { namespace hb { pmb_status pair_operand_map(CUtensorMap* map, const uint16_t* base, int64_t inner, int64_t outer, int64_t ld, int box_inner, int box_outer); } }
 
-template <int NB>
-static pmb_status skinny_nb(cudaStream_t st, const uint16_t* hi, const uint16_t* lo, int64_t B, int64_t K, int64_t J, const float* W, bool early, float* slab, int splits) {
+// x in fp32 (K a multiple of 8, on the 16-byte grid) or, x == NULL, as the pair (hi, lo)
+template <int NB, bool XC>
+static pmb_status skinny_nb(cudaStream_t st, const float* x, const uint16_t* hi, const uint16_t* lo, int64_t B, int64_t K, int64_t J, const float* W, bool early, float* slab, int splits) {
   static unsigned int* known[PMB_MAX_DEVICES] = {nullptr};
   unsigned int* status = tcx::status_address(g_decode_status, known);
   if (!status) return fail(PMB_ERR_CUDA, "decode: no status word on this device");
   dec::SkMaps ms{};
-  PMB_TRY(hb::pair_operand_map(&ms.x[0], hi, K, B, K, dec::SK_BK, NB));
-  PMB_TRY(hb::pair_operand_map(&ms.x[1], lo, K, B, K, dec::SK_BK, NB));
-  dec::SkArgs a{W, J, (int)K, (int)J, (int)B, (int)cdiv(cdiv(K, dec::SK_BK), splits), early, slab, status};
-  PMB_SMEM_OPT_IN(dec::SkGeo<NB>::SMEM, dec::skinny_gemm_kernel<NB>);
+  if (!XC) {
+    PMB_TRY(hb::pair_operand_map(&ms.x[0], hi, K, B, K, dec::SK_BK, NB));
+    PMB_TRY(hb::pair_operand_map(&ms.x[1], lo, K, B, K, dec::SK_BK, NB));
+  }
+  dec::SkArgs a{W, J, x, (int)K, (int)J, (int)B, (int)cdiv(cdiv(K, dec::SK_BK), splits), early, slab, status};
+  PMB_SMEM_OPT_IN(dec::SkGeo<NB>::SMEM, dec::skinny_gemm_kernel<NB, XC>);
   ProfScope prof(st, "decode_gemm", 2.0 * B * K * J, 4.0 * ((double)K * J + (double)splits * B * J));
-  return launch_pdl(st, dec::skinny_gemm_kernel<NB>, dim3((unsigned)cdiv(J, 128), (unsigned)splits, (unsigned)cdiv(B, NB)), dec::SK_THREADS, dec::SkGeo<NB>::SMEM, ms, a);
+  return launch_pdl(st, dec::skinny_gemm_kernel<NB, XC>, dim3((unsigned)cdiv(J, 128), (unsigned)splits, (unsigned)cdiv(B, NB)), dec::SK_THREADS, dec::SkGeo<NB>::SMEM, ms, a);
 }
-static pmb_status skinny(cudaStream_t st, const uint16_t* hi, const uint16_t* lo, int64_t B, int64_t K, int64_t J, const float* W, bool early, float* slab, int splits) {
-  if (B > 128) return skinny_nb<256>(st, hi, lo, B, K, J, W, early, slab, splits);
-  if (B > 64) return skinny_nb<128>(st, hi, lo, B, K, J, W, early, slab, splits);
-  if (B > 32) return skinny_nb<64>(st, hi, lo, B, K, J, W, early, slab, splits);
-  return skinny_nb<32>(st, hi, lo, B, K, J, W, early, slab, splits);
+static pmb_status skinny(cudaStream_t st, const float* x, const uint16_t* hi, const uint16_t* lo, int64_t B, int64_t K, int64_t J, const float* W, bool early, float* slab, int splits) {
+  if (B > 128) return skinny_nb<256, false>(st, nullptr, hi, lo, B, K, J, W, early, slab, splits);
+  if (B > 64) return skinny_nb<128, false>(st, nullptr, hi, lo, B, K, J, W, early, slab, splits);
+  if (B > 32) return x ? skinny_nb<64, true>(st, x, hi, lo, B, K, J, W, early, slab, splits) : skinny_nb<64, false>(st, x, hi, lo, B, K, J, W, early, slab, splits);
+  return x ? skinny_nb<32, true>(st, x, hi, lo, B, K, J, W, early, slab, splits) : skinny_nb<32, false>(st, x, hi, lo, B, K, J, W, early, slab, splits);
 }
 
 static pmb_status launch_state_step(cudaStream_t st, const Dims& d, const dec::StateArgs& s) {
@@ -618,13 +703,15 @@ extern "C" pmb_status pmb_mamba2_step(void* stream, const pmb_mamba2_config* cfg
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto al = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) == 0; };
   const bool vec = d.J % 4 == 0 && d.D % 4 == 0 && d.I % 4 == 0 && al(p->in_proj_weight) && al(p->out_proj_weight);
+  const bool fma = vec && d.B <= 16 && gemv_smem(d.B, d.D) <= GEMV_MAX_SMEM && gemv_smem(d.B, d.I) <= GEMV_MAX_SMEM;
+  const bool tc = !fma && vec && d.D % 8 == 0 && d.I % 8 == 0;
   dec::StepIn si{d.B, d.D, d.I, d.X, d.J, d.H, d.G, d.N, d.P, d.K, p->conv1d_weight, p->conv1d_bias, p->dt_bias, d_conv_window, w.z, d.I, w.act, w.dt};
-  const dec::StateArgs sa{w.act, w.dt, w.z, d.I, p->a_log, p->d_skip, d_ssm_state, w.g, w.ss, d.H, d.G, d.N, d.P, d.X, d.I};
+  const dec::StateArgs sa{w.act, w.dt, w.z, d.I, p->a_log, p->d_skip, p->norm_weight, d_ssm_state, w.g, tc ? w.n_hi : nullptr, w.n_lo, w.ss, d.H, d.G, d.N, d.P, d.X, d.I};
   // Up to 16 sequences the products are fp32 FMA (y 2e-7 of its norm from fp64), beyond on bf16 pairs (7e-6).  Where the line
   // lies is a matter of that precision, not of time.  us per step, FMA / tensor cores (24 heads of 64 x 64 at d_model 768; 32 of 64 x 128
   // at d_model 2048): 1 sequence 14.2 / 19.0, 21.1 / 26.6; 2: 14.1 / 19.8, 23.9 / 28.3; 4: 14.6 / 20.3, 28.3 / 28.4; 8: 18.4 / 22.1, 31.4 / 29.0;
   // 16: 27.2 / 22.6, 48.1 / 31.1; 17: 22.9 and 31.6.
-  if (vec && d.B <= 16 && gemv_smem(d.B, d.D) <= GEMV_MAX_SMEM && gemv_smem(d.B, d.I) <= GEMV_MAX_SMEM) {
+  if (fma) {
     dec::GemvArgs a{};
     a.B = d.B; a.K = d.D; a.N = d.J; a.W = p->in_proj_weight; a.ldw = d.J; a.in = d_x_t; a.in_vec = al(d_x_t); a.st = si;
     { ProfScope prof(st, "decode_in_proj", 2.0 * d.B * d.D * d.J, 4.0 * d.D * d.J); PMB_TRY(gemv<0>(st, a)); }
@@ -634,12 +721,12 @@ extern "C" pmb_status pmb_mamba2_step(void* stream, const pmb_mamba2_config* cfg
     ProfScope prof(st, "decode_out_proj", 2.0 * d.B * d.D * d.I, 4.0 * d.D * d.I);
     return gemv<1>(st, o);
   }
-  const bool tc = vec && d.D % 8 == 0 && d.I % 8 == 0;
   int n_in = 1;
   if (tc) {
     n_in = skinny_splits(d.B, d.J, d.D);
-    PMB_TRY(split_pair16(st, d_x_t, d.B, d.D, d.D, w.x_hi, w.x_lo, d.D));
-    PMB_TRY(skinny(st, w.x_hi, w.x_lo, d.B, d.D, d.J, p->in_proj_weight, false, w.slab, n_in));
+    const bool x32 = d.B <= 64 && al(d_x_t);
+    if (!x32) PMB_TRY(split_pair16(st, d_x_t, d.B, d.D, d.D, w.x_hi, w.x_lo, d.D));
+    PMB_TRY(skinny(st, x32 ? d_x_t : nullptr, w.x_hi, w.x_lo, d.B, d.D, d.J, p->in_proj_weight, false, w.slab, n_in));
   } else {
     PMB_TRY(gemm(st, 0, 0, d.B, d.J, d.D, d_x_t, d.D, p->in_proj_weight, d.J, w.slab, d.J, nullptr, 0));
   }
@@ -647,12 +734,14 @@ extern "C" pmb_status pmb_mamba2_step(void* stream, const pmb_mamba2_config* cfg
   PMB_TRY(launch_pdl(st, dec::in_proj_finish_kernel, dim3((unsigned)cdiv(d.J, 256), (unsigned)(d.B < dec::FINISH_Y ? d.B : dec::FINISH_Y), (unsigned)cdiv(d.B, dec::FINISH_Y)), 256, 0,
                      static_cast<const float*>(w.slab), n_in, si)); }
   PMB_TRY(launch_state_step(st, d, sa));
-  { ProfScope prof(st, "decode_norm", 0.0, 8.0 * d.B * d.I);
-  PMB_TRY(launch_pdl(st, dec::norm_kernel, dim3((unsigned)d.B), 256, 0, static_cast<const float*>(w.g), static_cast<const float*>(w.ss), p->norm_weight, tc ? w.n_hi : nullptr,
-                     w.n_lo, w.normed, d.I, d.H, d.eps)); }
-  if (!tc) return gemm(st, 0, 0, d.B, d.D, d.I, w.normed, d.I, p->out_proj_weight, d.D, d_y_t, d.D, nullptr, 0);
+  if (!tc) {
+    { ProfScope prof(st, "decode_norm", 0.0, 8.0 * d.B * d.I);
+    PMB_TRY(launch_pdl(st, dec::norm_kernel, dim3((unsigned)d.B), 256, 0, static_cast<const float*>(w.g), static_cast<const float*>(w.ss), p->norm_weight, w.normed, d.I, d.H, d.eps)); }
+    return gemm(st, 0, 0, d.B, d.D, d.I, w.normed, d.I, p->out_proj_weight, d.D, d_y_t, d.D, nullptr, 0);
+  }
   const int n_out = skinny_splits(d.B, d.D, d.I);
-  const bool direct = n_out == 1 || !al(d_y_t);
-  PMB_TRY(skinny(st, w.n_hi, w.n_lo, d.B, d.I, d.D, p->out_proj_weight, true, direct ? d_y_t : w.slab, direct ? 1 : n_out));
-  return direct ? PMB_OK : sum_slabs(st, w.slab, n_out, (int64_t)d.B * d.D, (int64_t)d.B * d.D, d_y_t, 0);
+  PMB_TRY(skinny(st, nullptr, w.n_hi, w.n_lo, d.B, d.I, d.D, p->out_proj_weight, true, w.slab, n_out));
+  ProfScope prof(st, "decode_out_sum", 0.0, 4.0 * d.B * d.D * (n_out + 1.0));
+  return launch_pdl(st, dec::out_finish_kernel, dim3((unsigned)d.B, (unsigned)cdiv(d.D, 1024)), 256, 0, static_cast<const float*>(w.slab), n_out, static_cast<const float*>(w.ss), d_y_t,
+                    al(d_y_t), (int64_t)d.B * d.D, d.D, d.I, d.H, d.eps);
 }

@@ -161,15 +161,15 @@ def test_decode_batches(pm, B, D, H, P, N, G):
     assert pm.device_status() == 0
 
 
-# weight rows that take a thread more than one pass of its groups, with a remainder, on both products; offset 1: the token and the norm's
-# weight off the 16-byte grid
+# weight rows that take a thread more than one pass of its groups, with a remainder, on both products; beyond 16 sequences the two widths
+# that convert the token themselves, with a part of a tile at the end; offset 1: the token and the norm's weight off the 16-byte grid
 @pytest.mark.parametrize("offset", [0, 1])
-@pytest.mark.parametrize("B", [1, 2, 4, 8, 16])
-def test_decode_long_rows(pm, B, offset):
+@pytest.mark.parametrize("B,D", [(1, 1028), (2, 1028), (4, 1028), (8, 1028), (16, 1028), (17, 1032), (32, 1032), (50, 1032), (64, 1032)])
+def test_decode_long_rows(pm, B, D, offset):
     def off_grid(t):
         return torch.cat([t.new_zeros(offset), t.flatten()])[offset:].view(t.shape)
 
-    D, H, P, N = 1028, 13, 128, 12
+    H, P, N = 13, 128, 12
     cfg, p, blk = _block(pm, D, H, P, N, 1, 64, torch.float32)
     blk.params["norm_weight"] = off_grid(blk.params["norm_weight"])
     ref = {"ssm_state": randn((B, H, N, P), 7, 0.3), "conv_window": randn((B, cfg.xbc_dim, 3), 8, 0.5)}
