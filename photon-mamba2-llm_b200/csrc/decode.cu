@@ -10,7 +10,7 @@
 // and be placed while several are at work, reads nothing before its wait, and the kernel in front of the state step lets that one in only
 // after its own wait.
 // Measured: 1 sequence at d_model 768, 24 heads of 64 x 64: 71 -> 16 -> 14.2 us a step, which is the host's time for it (splitting both
-// weights into pairs on every call and GEMM tiles of 128 rows before; 10.1 when replayed from a graph); 256 at d_model 2048, 32 heads of 64 x 128: 228 -> 145 -> 130 us, of which the
+// weights into pairs on every call and GEMM tiles of 128 rows before; 10.1 when replayed from a graph); 256 at d_model 2048, 32 heads of 64 x 128: 228 -> 145 -> 127 us, of which the
 // state takes 81 (537 MB, 6.6 TB/s).
 #include <cuda_bf16.h>
 #include "common.cuh"
@@ -594,7 +594,7 @@ struct StepWs {
 
 // K splits of the tensor-core projection: one wave of CTAs, at least two k-tiles each
 static int skinny_splits(int64_t B, int64_t J, int64_t K) {
-  const int64_t nb = B > 128 ? 256 : (B > 64 ? 128 : (B > 32 ? 64 : 32));
+  const int64_t nb = B > 64 ? 128 : (B > 32 ? 64 : 32);
   const int64_t ctas = cdiv(J, 128) * cdiv(B, nb), kt = cdiv(K, dec::SK_BK);
   int64_t sp = 148 / ctas;
   if (sp > kt / 2) sp = kt / 2;
@@ -670,8 +670,9 @@ static pmb_status skinny_nb(cudaStream_t st, const float* x, const uint16_t* hi,
   ProfScope prof(st, "decode_gemm", 2.0 * B * K * J, 4.0 * ((double)K * J + (double)splits * B * J));
   return launch_pdl(st, dec::skinny_gemm_kernel<NB, XC>, dim3((unsigned)cdiv(J, 128), (unsigned)splits, (unsigned)cdiv(B, NB)), dec::SK_THREADS, dec::SkGeo<NB>::SMEM, ms, a);
 }
+// 128 sequences to a tile and no more: two of them take half the K splits of one of 256, so half the sums go through memory (256 sequences,
+// us per step: 24 heads at d_model 768 69.0 with 256, 65.4 with 128, 67.5 with 64; 32 heads at 2048 129.4, 127.1 and 145; 8 heads at 512 38.9, 33.1, 31.5).
 static pmb_status skinny(cudaStream_t st, const float* x, const uint16_t* hi, const uint16_t* lo, int64_t B, int64_t K, int64_t J, const float* W, bool early, float* slab, int splits) {
-  if (B > 128) return skinny_nb<256, false>(st, nullptr, hi, lo, B, K, J, W, early, slab, splits);
   if (B > 64) return skinny_nb<128, false>(st, nullptr, hi, lo, B, K, J, W, early, slab, splits);
   if (B > 32) return x ? skinny_nb<64, true>(st, x, hi, lo, B, K, J, W, early, slab, splits) : skinny_nb<64, false>(st, x, hi, lo, B, K, J, W, early, slab, splits);
   return x ? skinny_nb<32, true>(st, x, hi, lo, B, K, J, W, early, slab, splits) : skinny_nb<32, false>(st, x, hi, lo, B, K, J, W, early, slab, splits);
