@@ -143,8 +143,7 @@ static size_t block_ws_layout(const Dims& d, void* base, size_t bytes, BlockWs* 
   if (chain) {
     w.ssd.xt_hi = ar.take<uint16_t>(hp); w.ssd.xt_lo = ar.take<uint16_t>(hp); w.ssd.dy_hi = ar.take<uint16_t>(hp); w.ssd.dy_lo = ar.take<uint16_t>(hp);
     w.ssd.dh_hi = ar.take<uint16_t>(steps_np); w.ssd.dh_lo = ar.take<uint16_t>(steps_np);
-    int per = 0;
-    w.nseg = ssd_chain_segments(d.B, d.T, d.H, &per);
+    w.nseg = ssd_chain_plan(d.B, d.T, d.H).nseg;
     w.ssd.part = ar.take<float>((size_t)3 * d.B * w.nseg * d.H);
     w.seg_bwd = ar.take<float>(ssd_chain_seg_floats(d.B, d.T, d.H, d.P, d.N));
     w.ssd.splitk = ar.take<float>(ssd_heads_part_floats(d.B, d.T, d.H, d.N, d.G));

@@ -106,9 +106,9 @@ struct Params {
   // (store_ops) x~ and xs as the kernel formed them.  bf16 x: store_ops leaves a copy of it.
   float *hprev, *yoff;
   int store_ops;
-  int nseg, per;                                         // segments of a sequence, steps per segment
+  int whole, nseg, per;                                  // chains walked in one piece; segments of the others, steps per segment (see ChainPlan)
   int state_only;                                        // first of two passes over segments: only seg_h and seg_d are formed
-  float *seg_h, *seg_d;                                  // (B*H,nseg,N,P), (B*H,nseg): state that a segment leaves when it starts from none, decay over it
+  float *seg_h, *seg_d;                                  // (B*H-whole,nseg,N,P), (B*H-whole,nseg): state that a segment leaves when it starts from none, decay over it
   unsigned int* status;
 };
 
@@ -138,10 +138,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   float* sdt = sS + NSB * GE::SLOT;                                 // BIG: dt alone, the last kilobyte is not there
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int bh = (int)blockIdx.x / p.nseg, seg = (int)blockIdx.x % p.nseg;
+  // blocks: the chains in one piece, then the others segment by segment (the first of two passes has these alone)
+  const int cut = (int)blockIdx.x - (p.state_only ? 0 : p.whole), nseg = cut < 0 ? 1 : p.nseg, per = cut < 0 ? p.nsteps : p.per;
+  const int bh = cut < 0 ? (int)blockIdx.x : p.whole + cut / nseg, seg = cut < 0 ? 0 : cut % nseg;
+  if (p.state_only && seg + 1 == nseg) return;             // (nobody starts from what the last one leaves)
   const int h = bh % p.H, bb = bh / p.H, g = h / p.hpg;
-  const int i0 = seg * p.per, toff = i0 * L;               // first step and token of this CTA's segment
-  const int n = min(p.per, p.nsteps - i0);
+  const int i0 = seg * per, toff = i0 * L;                 // first step and token of this CTA's segment
+  const int n = min(per, p.nsteps - i0);
   const int64_t tokb = (int64_t)bb * p.T;
   if (threadIdx.x == 0) {
     const int mmas = p.state_only ? 1 : 2;                  // warps that issue products
@@ -165,8 +168,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  pdl_launch();
-  pdl_wait();
+  // A chain in one piece needs nothing from the first pass, which lets this kernel in only after its own wait.
+  if (p.state_only) { pdl_wait(); pdl_launch(); } else { pdl_launch(); if (cut >= 0 || p.nseg == 1) pdl_wait(); }
   const uint32_t tG = tmem, tA1 = tmem + 256, tA2 = tmem + 320, tU = tmem + 384;
 
   auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
@@ -652,8 +655,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     }
     if (!p.state_only && active)
       for (int j = 0; j < seg; ++j) {                       // what the segments before this one leave
-        const float* F = p.seg_h + ((int64_t)bh * p.nseg + j) * NP + (int64_t)nr * p.P;
-        const float dj = p.seg_d[bh * p.nseg + j];
+        const int64_t row = cut - seg + j;
+        const float* F = p.seg_h + row * NP + (int64_t)nr * p.P;
+        const float dj = p.seg_d[row];
 #pragma unroll
         for (int q = 0; q < PW / 4; ++q) {
           if (4 * q >= p.P) continue;
@@ -721,7 +725,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       if (lane == 0) mbar_arrive(bar(UFREE));
     }
     if (ok && p.state_only && nr == 0) p.seg_d[blockIdx.x] = __expf(stot);
-    float* const leave = p.state_only ? p.seg_h + (int64_t)blockIdx.x * NP : p.last && seg + 1 == p.nseg ? p.last + (int64_t)bh * NP : nullptr;
+    float* const leave = p.state_only ? p.seg_h + (int64_t)blockIdx.x * NP : p.last && seg + 1 == nseg ? p.last + (int64_t)bh * NP : nullptr;
     if (ok && leave && active) {
       float* dst = leave + (int64_t)nr * p.P;
 #pragma unroll
@@ -768,20 +772,19 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
     if (!XIN16) PMB_TRY(sf::bf16_map4(&ms.xs, a.xs, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
   }
   p.hp_hi = a.hp_hi; p.hp_lo = a.hp_lo; p.last = a.last; p.status = status_ptr();
-  p.nseg = 1; p.per = p.nsteps;
-  if (NB == 1 && a.seg) {
-    p.nseg = ssd_chain_segments(a.B, a.T, a.H, &p.per);
-    p.seg_h = a.seg; p.seg_d = a.seg + (size_t)a.B * a.H * p.nseg * a.N * a.P;
-  }
+  const int chains = a.B * a.H;
+  const ChainPlan plan = NB == 1 && a.seg ? ssd_chain_plan(a.B, a.T, a.H) : ChainPlan{chains, 1, p.nsteps};
+  p.whole = plan.whole; p.nseg = plan.nseg; p.per = plan.per;
+  const unsigned cut = (unsigned)((chains - p.whole) * p.nseg);      // blocks of segments
+  if (cut) { p.seg_h = a.seg; p.seg_d = a.seg + (size_t)cut * a.N * a.P; }
   PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>);
-  const unsigned grid = (unsigned)((int64_t)a.B * a.H * p.nseg);
-  if (p.nseg > 1) {
+  if (cut) {
     p.state_only = 1;
-    PMB_TRY(launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>, grid, NTHREADS, GE::SMEM, ms, p));
+    PMB_TRY(launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>, cut, NTHREADS, GE::SMEM, ms, p));
     p.state_only = 0;
   }
   p.store_ops = keep != nullptr;
-  PMB_TRY(launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>, grid, NTHREADS, GE::SMEM, ms, p));
+  PMB_TRY(launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>, (unsigned)p.whole + cut, NTHREADS, GE::SMEM, ms, p));
   return PMB_OK;
 }
 
@@ -791,17 +794,21 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
 // a first pass that only forms the state each segment leaves (about a quarter of a step's time).  Two steps per segment at least;
 // under four steps the second launch costs what the cut saves.  Measured at
 // 8 heads of 64 x 64, 1 x 2048 tokens: a block's forward 137 us uncut, 90 us in eight segments; training step of four layers 1588 and 934 us.
-int ssd_chain_segments(int B, int T, int H, int* per) {
-  const int n = (int)cdiv(T, SCAN_STEP), most = (int)(148 / ((int64_t)B * H > 148 ? 149 : (int64_t)B * H));
-  int nseg = most < n / 2 ? most : n / 2;
-  if (nseg < 2 || n < 4) { *per = n; return 1; }
-  *per = (int)cdiv(n, nseg);
-  return (int)cdiv(n, *per);
+// With more chains than SMs the same goes for those of the last round: the others need nothing from the first pass and start beside it.  From
+// three segments on, forward and backward of the bf16 scan: 160 chains of 64 x 64, 1000 tokens 220 -> 188 us, 192 of 64 x 128, 2048 tokens
+// 352 -> 330; an fp32 prefill of 5 x 1200 tokens, 32 heads, 364 -> 352.  With two, 208 chains of 64 x 64 took 67 us forward instead of 59 and
+// 113 backward instead of 118, 512 of 64 x 128 241 and 513 instead of 211 and 514: the first pass takes what the last round gives.
+ChainPlan ssd_chain_plan(int B, int T, int H) {
+  const int64_t chains = (int64_t)B * H;
+  const int n = (int)cdiv(T, SCAN_STEP), rest = (int)(chains % 148 ? chains % 148 : 148);
+  const int most = 148 / rest, nseg = most < n / 2 ? most : n / 2;
+  if (n < 4 || nseg < (chains > 148 ? 3 : 2)) return ChainPlan{(int)chains, 1, n};
+  const int per = (int)cdiv(n, nseg);
+  return ChainPlan{(int)(chains - rest), (int)cdiv(n, per), per};
 }
 size_t ssd_chain_seg_floats(int B, int T, int H, int P, int N) {
-  int per = 0;
-  const int nseg = ssd_chain_segments(B, T, H, &per);
-  return nseg > 1 ? (size_t)B * H * nseg * ((size_t)N * P + 1) : 0;
+  const ChainPlan plan = ssd_chain_plan(B, T, H);
+  return plan.nseg > 1 ? ((size_t)B * H - plan.whole) * plan.nseg * ((size_t)N * P + 1) : 0;
 }
 
 pmb_status ssd_chain_fwd(cudaStream_t st, const ChainArgs& a) {

@@ -47,7 +47,9 @@ struct ChainArgs {
   uint16_t *xt, *xs;                           // ... and the operands x~ and xs, (B,T,H,P)
   float* seg = nullptr;                        // ssd_chain_seg_floats() floats: lets few long sequences be walked in segments (blocks == 1)
 };
-int ssd_chain_segments(int B, int T, int H, int* per);      // segments of a sequence; *per = steps of each (the last may have fewer)
+// The first `whole` chains (b, h) are walked in one piece, each of the others in `nseg` segments of `per` steps (the last may have fewer).
+struct ChainPlan { int whole, nseg, per; };
+ChainPlan ssd_chain_plan(int B, int T, int H);
 size_t ssd_chain_seg_floats(int B, int T, int H, int P, int N);
 inline bool ssd_chain_shape(int P, int N) { return P > 0 && P <= 64 && P % 8 == 0 && N > 0 && N <= 128 && N % 8 == 0; }
 bool ssd_chain_enabled();      // false when PMB_SSD_FUSED=0 or PMB_SSD_ENGINE=simt

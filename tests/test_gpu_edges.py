@@ -521,3 +521,48 @@ def test_calls_one_after_the_other(pm, dtype, D, H, P, N, B, T, Q):
             assert torch.equal(got[0], want[i][0]) and torch.equal(got[1], want[i][1])
             assert all(torch.equal(got[2][k], want[i][2][k]) for k in got[2])
     assert pm.device_status() == 0
+
+
+# more chains than the machine has SMs: those of a last round that fills less than a third of it are walked in segments beside the others
+# (one chain more than a round, a few, just under a third; just over and two full rounds, which stay whole)
+@pytest.mark.parametrize("B,H", [(149, 1), (19, 8), (24, 8), (25, 8), (37, 8)])
+@pytest.mark.parametrize("T", [770, 896])
+def test_scan_last_round_in_segments(pm, B, H, T):
+    P, N, G = 16, 24, 1
+    x, b, c, dy = randn((B, T, H, P), 1).bfloat16(), randn((B, T, G, N), 2).bfloat16(), randn((B, T, G, N), 3).bfloat16(), randn((B, T, H, P), 4).bfloat16()
+    a = -torch.nn.functional.softplus(randn((B, T, H), 5) - 2.0)
+    init = randn((B, H, N, P), 6)
+    scan = pm.SsdScanBf16(x.cuda(), a.cuda(), b.cuda(), c.cuda(), 128)
+    y, last = scan.forward(init_state=init.cuda(), want_final_state=True)
+    scan.forward()
+    dx, da, db, dc = scan.backward(dy.cuda())
+    torch.cuda.synchronize()
+    assert pm.device_status() == 0
+    leaves = [t.float().requires_grad_(True) for t in (x, a, b, c)]
+    be, ce = (t.expand(B, T, H, N) for t in leaves[2:])
+    orc.ssd_scan_chunked(leaves[0], leaves[1], be, ce, T // 7, return_final_state=True)[0].backward(dy.float())
+    with torch.no_grad():
+        ref, ref_last = orc.ssd_scan_chunked(leaves[0], leaves[1], be, ce, T // 7, initial_state=init, return_final_state=True)
+    for got, want, tol, what in ((y.float(), ref, 5e-3, "y"), (last, ref_last, 5e-3, "final state"), (dx.float(), leaves[0].grad, 5e-3, "dx"), (da, leaves[1].grad, 5e-3, "da"),
+                                 (db.float(), leaves[2].grad, 5e-3, "db"), (dc.float(), leaves[3].grad, 5e-3, "dc")):
+        assert_close(got, want, tol=tol, what=what)
+
+
+@pytest.mark.parametrize("B", [19, 24])
+def test_block_last_round_in_segments(pm, B):
+    D, H, P, N, T, Q = 64, 8, 16, 16, 770, 64
+    cfg, p, blk = _block(pm, D, H, P, N, 1, Q, torch.float32)
+    x, cot = randn((B, T, D), 5), randn((B, T, D), 6)
+    out = blk.forward(x.cuda())
+    dx, grads = blk.backward(x.cuda(), cot.cuda())
+    torch.cuda.synchronize()
+    assert pm.device_status() == 0
+    leaves = {k: v.clone().requires_grad_(True) for k, v in p.items()}
+    xr = x.clone().requires_grad_(True)
+    ref = orc.block_forward(leaves, cfg, xr)
+    ref.backward(cot)
+    assert_close(out, ref.detach(), what="out")
+    assert_close(dx, xr.grad, what="dx")
+    for k, g in grads.items():
+        # (the sums for a_log and dt_bias cancel over 15000 tokens: 1.9e-4 and 2.2e-4 from fp64 also with 144 chains, which stay whole)
+        assert_close(g, leaves[k].grad, tol=5e-4 if k in ("a_log", "dt_bias") else FP32_TOL, what=k)
