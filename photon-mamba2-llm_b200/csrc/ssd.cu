@@ -789,14 +789,16 @@ __global__ void __launch_bounds__(PREP_THREADS) chunk_rows_finish_kernel(SsdP p,
 // goes through y - D x or through two separately rounded matrix products.  da = reverse cumsum(dS);
 // ddt = <dx~, x> + A da;  dx = dx~ dt + D dY;  per-chunk partials of dA and dD.
 struct WSums { const float* rpart; const float* csum; const float* esum; const float* yoff; int nb; };
-// Each half-warp has two rows in flight per pass (all loads of both rows are issued before the first use), and three CTAs share an
-// SM: while one sums over its chunk another streams.  16384 tokens, 24 heads: 159 us with two CTAs, 127 with three (500 MB).
+// A half-warp takes one row per pass and asks for its next one before (cp.async, slots of the thread's own, no barrier); five CTAs share an
+// SM: while one sums over its chunk another streams.  Bound by HBM, rows of 256 bytes of four tensors (16384 tokens, 24 heads, 500 MB): 159 us
+// with two rows per pass in registers and two CTAs, 127 with three; two rows ahead in shared memory and three CTAs 116, one row and three
+// CTAs 122, four 106, five 107 (8192 tokens: 46, 43, 43, 45, 44).
 constexpr int ROWS_THREADS = 256;
-__global__ void __launch_bounds__(ROWS_THREADS, 3) chunk_rows_finish_w_kernel(SsdP p, WSums ws, float* __restrict__ dx, int64_t lddx,
+__global__ void __launch_bounds__(ROWS_THREADS, 5) chunk_rows_finish_w_kernel(SsdP p, WSums ws, float* __restrict__ dx, int64_t lddx,
                                                                            const float* __restrict__ dd, float* __restrict__ da_out,
                                                                            float* __restrict__ ddt_out, float* __restrict__ part,
                                                                            SsdGrads::RawDt raw) {
-  __shared__ float s_ddtx[PREP_MAX_Q], s_dS[PREP_MAX_Q], s_dD[PREP_MAX_Q], s_dt[PREP_MAX_Q], s_e[PREP_MAX_Q], wsum[ROWS_THREADS / 32], red[32];
+  __shared__ float wsum[ROWS_THREADS / 32], red[32];
   constexpr int NHW = ROWS_THREADS / 16;
   const int w = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int h = w % p.H, bc = w / p.H, cc = bc % p.nc, bb = bc / p.nc;
@@ -805,57 +807,52 @@ __global__ void __launch_bounds__(ROWS_THREADS, 3) chunk_rows_finish_w_kernel(Ss
   const int P4 = p.P >> 2;
   const int hw = tid >> 4, l16 = lane & 15;
   const int64_t hp = (int64_t)p.H * p.P;
-  for (int tb = 0; tb < p.Q; tb += 2 * NHW) {
-    const int t[2] = {tb + hw, tb + NHW + hw};
-    float s1[2] = {0.0f, 0.0f}, s2[2] = {0.0f, 0.0f}, s3[2] = {0.0f, 0.0f}, dtv[2] = {1.0f, 1.0f};
-    float rr[2] = {0.0f, 0.0f}, cs[2] = {0.0f, 0.0f}, es[2] = {0.0f, 0.0f};
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      if (t[u] < p.Q) {
-        const int64_t tk = tok0 + t[u];
-        dtv[u] = p.dtv(tk, h);
-        if (l16 == 0) {
-          const int64_t idx = tk * p.H + h;
-          for (int rb = 0; rb <= t[u] / 128; ++rb) rr[u] += ws.rpart[((int64_t)w * ws.nb + rb) * p.Q + t[u]];   // row blocks whose rows s can be < t
-          cs[u] = ws.csum[idx]; es[u] = ws.esum[idx];
-        }
+  extern __shared__ __align__(16) float4 rring[];           // [pass % 2][x, dx~, dY, yoff][thread], then five values per row of the chunk
+  float4* const own = rring + tid;
+  float* const s_ddtx = reinterpret_cast<float*>(rring + 8 * ROWS_THREADS);
+  float *const s_dS = s_ddtx + p.Q, *const s_dD = s_dS + p.Q, *const s_dt = s_dD + p.Q, *const s_e = s_dt + p.Q;
+  auto fetch = [&](int t) {
+    if (t < p.Q && l16 < P4) {
+      const int64_t tk = tok0 + t;
+      const uint32_t d = (uint32_t)__cvta_generic_to_shared(own + (t / NHW % 2) * 4 * ROWS_THREADS);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(p.x + tk * p.ldx + h * p.P + 4 * l16) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * ROWS_THREADS), "l"(p.dxt + tk * hp + h * p.P + 4 * l16) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 32 * ROWS_THREADS), "l"(p.dy + tk * p.lddy + h * p.P + 4 * l16) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 48 * ROWS_THREADS), "l"(ws.yoff + tk * hp + h * p.P + 4 * l16) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(hw);
+  for (int tb = 0; tb < p.Q; tb += NHW) {
+    const int t = tb + hw;
+    const int64_t tk = tok0 + t;
+    float s1 = 0.0f, s2 = 0.0f, s3 = 0.0f, dtv = 1.0f, rr = 0.0f, cs = 0.0f, es = 0.0f;
+    if (t < p.Q) {
+      dtv = p.dtv(tk, h);
+      if (l16 == 0) {
+        const int64_t idx = tk * p.H + h;
+        for (int rb = 0; rb <= t / 128; ++rb) rr += ws.rpart[((int64_t)w * ws.nb + rb) * p.Q + t];   // row blocks whose rows s can be < t
+        cs = ws.csum[idx]; es = ws.esum[idx];
       }
     }
-    for (int j = l16; j < P4; j += 16) {
-      float4 xv[2], dxt[2], dyv[2], yo[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (t[u] < p.Q) {
-          const int64_t tk = tok0 + t[u];
-          xv[u] = reinterpret_cast<const float4*>(p.x + tk * p.ldx + h * p.P)[j];
-          dxt[u] = reinterpret_cast<const float4*>(p.dxt + tk * hp + h * p.P)[j];
-          dyv[u] = reinterpret_cast<const float4*>(p.dy + tk * p.lddy + h * p.P)[j];
-          yo[u] = reinterpret_cast<const float4*>(ws.yoff + tk * hp + h * p.P)[j];
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (t[u] < p.Q) {
-          const int64_t tk = tok0 + t[u];
-          s1[u] = fmaf(dxt[u].x, xv[u].x, fmaf(dxt[u].y, xv[u].y, fmaf(dxt[u].z, xv[u].z, fmaf(dxt[u].w, xv[u].w, s1[u]))));
-          s2[u] = fmaf(dyv[u].x, yo[u].x, fmaf(dyv[u].y, yo[u].y, fmaf(dyv[u].z, yo[u].z, fmaf(dyv[u].w, yo[u].w, s2[u]))));
-          s3[u] = fmaf(dyv[u].x, xv[u].x, fmaf(dyv[u].y, xv[u].y, fmaf(dyv[u].z, xv[u].z, fmaf(dyv[u].w, xv[u].w, s3[u]))));
-          reinterpret_cast<float4*>(dx + tk * lddx + h * p.P)[j] =
-              make_float4(fmaf(dxt[u].x, dtv[u], Dv * dyv[u].x), fmaf(dxt[u].y, dtv[u], Dv * dyv[u].y), fmaf(dxt[u].z, dtv[u], Dv * dyv[u].z),
-                          fmaf(dxt[u].w, dtv[u], Dv * dyv[u].w));
-        }
-      }
+    fetch(t + NHW);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    if (t < p.Q && l16 < P4) {
+      const float4* const in = own + (t / NHW % 2) * 4 * ROWS_THREADS;
+      const float4 xv = in[0], dxt = in[ROWS_THREADS], dyv = in[2 * ROWS_THREADS], yo = in[3 * ROWS_THREADS];
+      s1 = fmaf(dxt.x, xv.x, fmaf(dxt.y, xv.y, fmaf(dxt.z, xv.z, dxt.w * xv.w)));
+      s2 = fmaf(dyv.x, yo.x, fmaf(dyv.y, yo.y, fmaf(dyv.z, yo.z, dyv.w * yo.w)));
+      s3 = fmaf(dyv.x, xv.x, fmaf(dyv.y, xv.y, fmaf(dyv.z, xv.z, dyv.w * xv.w)));
+      reinterpret_cast<float4*>(dx + tk * lddx + h * p.P)[l16] =
+          make_float4(fmaf(dxt.x, dtv, Dv * dyv.x), fmaf(dxt.y, dtv, Dv * dyv.y), fmaf(dxt.z, dtv, Dv * dyv.z), fmaf(dxt.w, dtv, Dv * dyv.w));
     }
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) {
-        s1[u] += __shfl_xor_sync(0xffffffffu, s1[u], o); s2[u] += __shfl_xor_sync(0xffffffffu, s2[u], o); s3[u] += __shfl_xor_sync(0xffffffffu, s3[u], o);
-      }
-      if (t[u] < p.Q && l16 == 0) {
-        s_ddtx[t[u]] = s1[u]; s_dD[t[u]] = s3[u]; s_dt[t[u]] = dtv[u]; s_e[t[u]] = es[u];
-        s_dS[t[u]] = ((rr[u] - cs[u]) + s2[u]) - es[u];
-      }
+    for (int o = 8; o > 0; o >>= 1) {
+      s1 += __shfl_xor_sync(0xffffffffu, s1, o); s2 += __shfl_xor_sync(0xffffffffu, s2, o); s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+    }
+    if (t < p.Q && l16 == 0) {
+      s_ddtx[t] = s1; s_dD[t] = s3; s_dt[t] = dtv; s_e[t] = es;
+      s_dS[t] = ((rr - cs) + s2) - es;
     }
   }
   __syncthreads();
@@ -1308,7 +1305,9 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
                           reinterpret_cast<uintptr_t>(g.dx) | reinterpret_cast<uintptr_t>(p.dxt)) % 16 == 0);
     if (fz) {
       WSums wsm{ws.rpart, ws.csum, ws.esum, ws.yoff, p.Q / 128};
-      chunk_rows_finish_w_kernel<<<(unsigned)nbch, ROWS_THREADS, 0, st>>>(p, wsm, g.dx, g.lddx, dsend, g.da, g.ddt, ws.part, in.dt ? g.raw : SsdGrads::RawDt{});
+      const int ring = 8 * 16 * ROWS_THREADS + 5 * 4 * p.Q;
+      PMB_SMEM_OPT_IN(8 * 16 * ROWS_THREADS + 5 * 4 * PREP_MAX_Q, chunk_rows_finish_w_kernel);
+      chunk_rows_finish_w_kernel<<<(unsigned)nbch, ROWS_THREADS, ring, st>>>(p, wsm, g.dx, g.lddx, dsend, g.da, g.ddt, ws.part, in.dt ? g.raw : SsdGrads::RawDt{});
       PMB_LAUNCHED();
     } else if (vec_ok && nbch <= 4 * 148 && p.Q <= PREP_MAX_Q) {
       chunk_rows_finish_kernel<<<(unsigned)nbch, PREP_THREADS, 0, st>>>(p, g.dx, g.lddx, dsend, g.da, g.ddt, ws.part);
