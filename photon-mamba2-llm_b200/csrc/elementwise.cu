@@ -14,7 +14,8 @@ __global__ void column_sum_kernel(const float* __restrict__ partial, int64_t row
 // registers and the next CONV_AHEAD rows on their way, so that every global access is a coalesced vector access and each input
 // row is read (run+K-1)/run times.  Bound by HBM.  A CTA of the vector kernels is 16 runs of 8 channel quads (128-byte strips of
 // its rows): no thread is idle for any channel count that is a multiple of 32.
-// Measured at 8 x 2048 tokens of 1664 channels: forward 68 us with runs of 8 all requested up front, 49 now;
+// Measured at 8 x 2048 tokens of 1664 channels: forward 68 us with runs of 8 all requested up front, 49 with the next four rows in registers,
+// 41 now: they wait in shared memory (cp.async), which leaves room for more CTAs (eight rows 41, pairs of channels 42); at 8 x 1024 16.4 and 13.9;
 // backward 131 us, 110 with four channels per thread and the next four rows in registers (170 of them, three CTAs per SM), 82 now: two channels
 // (72 registers, seven CTAs), the next eight rows in shared memory (cp.async).  At 4 x 512 tokens 20.7 and 18.6 us, at 2 x 128 of 544 channels
 // 7.7 and 5.6.
@@ -43,7 +44,7 @@ __device__ __forceinline__ void conv_load(const float* p, float (&o)[VEC]) {
 template <int K, int VEC>
 __device__ __forceinline__ void conv_fwd_thread(const float* __restrict__ xzd, int64_t ldx, int col0, const float* __restrict__ w,
                                                 const float* __restrict__ bias, float* __restrict__ act, int X, int T,
-                                                const ConvPairOut& po, int c, int b, int t0, int t1) {
+                                                const ConvPairOut& po, int c, int b, int t0, int t1, uint32_t slots = 0) {
   float wr[VEC][K], br[VEC], win[VEC][K];
 #pragma unroll
   for (int v = 0; v < VEC; ++v) {
@@ -62,14 +63,22 @@ __device__ __forceinline__ void conv_fwd_thread(const float* __restrict__ xzd, i
 #pragma unroll
     for (int v = 0; v < VEC; ++v) win[v][k] = o[v];
   }
-  float ring[CONV_AHEAD][VEC];
+  // four channels: the next rows wait in slots of the thread's own in shared memory (cp.async, no barrier) and not in registers
+  constexpr bool STAGED = VEC == 4;
+  constexpr uint32_t PITCH = CONV_STRIP_THREADS * 16;
+  float ring[STAGED ? 1 : CONV_AHEAD][VEC];
+  uint32_t slot = slots;
   const float* nx = src + (int64_t)t0 * ldx;                  // the next row to request
-  auto request = [&](int t, float (&o)[VEC]) {
-    if (t < t1) conv_load<VEC>(nx, o);
+  auto request = [&](int t, int q) {
+    if (STAGED) {
+      if (t < t1) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot), "l"(nx) : "memory");
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      slot = slot + PITCH == slots + CONV_AHEAD * PITCH ? slots : slot + PITCH;
+    } else if (t < t1) conv_load<VEC>(nx, ring[q]);
     nx += ldx;
   };
 #pragma unroll
-  for (int q = 0; q < CONV_AHEAD; ++q) request(t0 + q, ring[q]);
+  for (int q = 0; q < CONV_AHEAD; ++q) request(t0 + q, q);
   float* dst = act + ((int64_t)b * T + t0) * X + c;
   int64_t o16 = ((int64_t)b * T + t0) * po.width + (c - po.col0);
   const bool pair = VEC == 4 && po.hi && c >= po.col0;        // the B | C columns also go out as a bf16 pair (operands of the scan)
@@ -79,9 +88,13 @@ __device__ __forceinline__ void conv_fwd_thread(const float* __restrict__ xzd, i
       const int t = tb + q;
       if (t >= t1) break;
       float o[VEC];
+      if (STAGED) {                                          // (the slot that is due is the one to request into)
+        asm volatile("cp.async.wait_group %0;" ::"n"(CONV_AHEAD - 1) : "memory");
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(o[0]), "=f"(o[1 % VEC]), "=f"(o[2 % VEC]), "=f"(o[3 % VEC]) : "r"(slot) : "memory");
+      }
 #pragma unroll
-      for (int v = 0; v < VEC; ++v) win[v][K - 1] = ring[q][v];
-      request(t + CONV_AHEAD, ring[q]);
+      for (int v = 0; v < VEC; ++v) win[v][K - 1] = STAGED ? o[v] : ring[STAGED ? 0 : q][v];
+      request(t + CONV_AHEAD, q);
 #pragma unroll
       for (int v = 0; v < VEC; ++v) {
         float u = br[v];
@@ -105,10 +118,12 @@ __global__ void __launch_bounds__(CONV_STRIP_THREADS) conv_silu_fwd_strip_kernel
                                                                                  float* __restrict__ act, int X, int T, int run, ConvPairOut po) {
   pdl_launch();
   pdl_wait();
+  __shared__ __align__(16) float4 rows[CONV_AHEAD][CONV_STRIP_THREADS];
   const int c = (blockIdx.x * 8 + (threadIdx.x & 7)) * 4;
   const int tblocks = (T + CONV_SLICES * run - 1) / (CONV_SLICES * run);
   const int b = blockIdx.y / tblocks, t0 = (blockIdx.y % tblocks) * (CONV_SLICES * run) + (threadIdx.x >> 3) * run;
-  if (c < X && t0 < T) conv_fwd_thread<K, 4>(xzd, ldx, col0, w, bias, act, X, T, po, c, b, t0, min(t0 + run, T));
+  if (c < X && t0 < T)
+    conv_fwd_thread<K, 4>(xzd, ldx, col0, w, bias, act, X, T, po, c, b, t0, min(t0 + run, T), (uint32_t)__cvta_generic_to_shared(&rows[0][threadIdx.x]));
 }
 // any channel count and alignment
 template <int K>

@@ -455,17 +455,20 @@ def test_gemm_pair_tiles_on_pairs(pm, M, N, K):
     assert_close(out, a.double() @ b.double(), tol=3e-5, what=f"{M}x{N}x{K}")
 
 
-# the conv backward's strips: 8 runs of 8, 16 or 32 steps to a CTA, two channels per thread, the next eight rows in shared memory (the oracle's
-# fp32 sums in another order: 1e-5 of the largest)
+# the conv's strips: 16 runs (backward 8) of 8, 16 or 32 steps to a CTA, four (two) channels per thread, the next four (eight) rows in shared
+# memory (the oracle's fp32 sums in another order: 1e-5 of the largest)
 @pytest.mark.parametrize("K", [2, 3, 4])
 @pytest.mark.parametrize("B,T", [(1, 1), (2, 7), (1, 8), (1, 63), (2, 65), (3, 300), (40, 260)])
 @pytest.mark.parametrize("H,P,N", [(4, 4, 4), (4, 16, 8), (8, 16, 16)])
-def test_conv_backward_strips(pm, B, T, K, H, P, N):
+def test_conv_strips(pm, B, T, K, H, P, N):
     cfg = pm.Mamba2Config(d_model=32, d_state=N, d_head=P, n_heads=H, n_groups=1, d_conv=K, block_len=T)
     I, X, J = cfg.d_inner, cfg.xbc_dim, cfg.in_proj_dim
     xzd, w, b, dact = randn((B, T, J), 1).requires_grad_(True), randn((X, 1, K), 2, 0.5).requires_grad_(True), randn((X,), 3, 0.1).requires_grad_(True), randn((B, T, X), 5)
     conv = torch.nn.functional.conv1d(xzd[..., I:I + X].transpose(1, 2), w, None, padding=K - 1, groups=X) + b.reshape(-1, 1)
-    (orc.silu(conv[..., :T].transpose(1, 2)) * dact).sum().backward()
+    want = orc.silu(conv[..., :T].transpose(1, 2))
+    act, _ = pm.conv_silu_dt_fwd(cfg, xzd.detach().cuda(), w.detach().cuda(), b.detach().cuda(), torch.zeros(H).cuda())
+    assert_close(act, want, tol=1e-5, what="act")
+    (want * dact).sum().backward()
     dxzd, dw, db = pm.conv_silu_bwd(cfg, xzd.detach().cuda(), w.detach().cuda(), b.detach().cuda(), dact.cuda())
     for got, want, what in ((dxzd[..., I:I + X], xzd.grad[..., I:I + X], "dx"), (dw, w.grad, "dw"), (db, b.grad, "db")):
         assert_close(got, want, tol=1e-5, what=what)
