@@ -528,12 +528,6 @@ __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_fwd_vec_kernel(con
       if (i < nvec) { yn[n] = reinterpret_cast<const float4*>(y + row * width)[i]; zn[n] = reinterpret_cast<const float4*>(z + row * ldz)[i]; }
     }
   };
-  auto split = [](float v, uint32_t& h, uint32_t& l) {   // (hi, lo) bf16 pair, round to nearest even
-    const uint32_t u = __float_as_uint(v);
-    h = (u + 0x7fffu + ((u >> 16) & 1u)) >> 16;
-    const uint32_t ul = __float_as_uint(v - __uint_as_float(h << 16));
-    l = (ul + 0x7fffu + ((ul >> 16) & 1u)) >> 16;
-  };
   if (r0 < r1) request(r0);
   for (int64_t row = r0; row < r1; ++row) {
   float4 g[PER];
@@ -556,12 +550,7 @@ __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_fwd_vec_kernel(con
       const float4 wv = reinterpret_cast<const float4*>(w)[i];
       const float4 v = make_float4(g[n].x * r * wv.x, g[n].y * r * wv.y, g[n].z * r * wv.z, g[n].w * r * wv.w);
       if (out) reinterpret_cast<float4*>(out + row * width)[i] = v;
-      if (out_hi) {
-        uint32_t h[4], l[4];
-        split(v.x, h[0], l[0]); split(v.y, h[1], l[1]); split(v.z, h[2], l[2]); split(v.w, h[3], l[3]);
-        reinterpret_cast<uint2*>(out_hi + row * width)[i] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
-        if (out_lo) reinterpret_cast<uint2*>(out_lo + row * width)[i] = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
-      }
+      if (out_hi) store_pair4(out_hi + row * width + 4 * i, out_lo ? out_lo + row * width + 4 * i : nullptr, v.x, v.y, v.z, v.w);
     }
   }
   }
@@ -654,9 +643,10 @@ __global__ void __launch_bounds__(NORM_THREADS) gated_rmsnorm_bwd_kernel(const f
 
 // float4 variant of the backward.  Optional extras (see NormBwdExtra): dz as a (hi, lo) bf16 pair instead of fp32, and dY exp(S) for
 // the scan backward.  Bound by HBM (reads of dout, y, z, writes of dy and the bf16 copies).  A block walks `nrows` rows
-// with its share of dw in registers: few long blocks leave few partial sums (one row of them per block), and the three to five blocks
-// that share an SM cover each other's loads (two blocks per SM with the next row requested ahead: 145 us, three: 181).
-// Measured at 16384 rows of 1536 with plain bf16 copies (550 MB): 136 us + 60 us of partial sums with four rows per block, 117 us + 3 now.
+// with its share of dw in registers: few long blocks leave few partial sums (one row of them per block), and the blocks that share an SM
+// cover each other's loads; the next row is asked for before this one's sum (in registers, with room for two blocks: 145 us).
+// Measured at 16384 rows of 1536 with plain bf16 copies (550 MB): 136 us + 60 us of partial sums with four rows per block, 117 us + 3 with
+// fourteen, 97 now with the next row in shared memory (104 when registers are held to four blocks; one row more ahead 114); 8192 rows: 39 and 32.
 template <int PER>
 __global__ void __launch_bounds__(NORM_THREADS, 3) gated_rmsnorm_bwd_vec_kernel(const float* __restrict__ dout, const float* __restrict__ y,
                                                                              const float* __restrict__ z, int64_t ldz,
@@ -677,20 +667,35 @@ __global__ void __launch_bounds__(NORM_THREADS, 3) gated_rmsnorm_bwd_vec_kernel(
   }
   const int64_t r0 = (int64_t)blockIdx.x * nrows;
   const int64_t r1 = r0 + nrows < rows ? r0 + nrows : rows;
-  for (int64_t row = r0; row < r1; ++row) {
-    const float r = rstd[row];
-    float4 zv[PER], yv[PER], dn[PER], gv[PER], sv[PER];
-    float dot = 0.0f;
+  // the next row waits in slots of the thread's own (cp.async, no barrier): [z, y, dout][PER][thread]
+  __shared__ __align__(16) float4 next[3 * PER * NORM_THREADS];
+  float4* const own = next + threadIdx.x;
+  auto fetch = [&](int64_t row) {
 #pragma unroll
     for (int n = 0; n < PER; ++n) {
       const int i = threadIdx.x + n * blockDim.x;
-      zv[n] = yv[n] = dn[n] = make_float4(0, 0, 0, 0);
-      if (i < nvec) {
-        zv[n] = reinterpret_cast<const float4*>(z + row * ldz)[i];
-        yv[n] = reinterpret_cast<const float4*>(y + row * width)[i];
-        dn[n] = reinterpret_cast<const float4*>(dout + row * width)[i];
-      }
+      if (i >= nvec || row >= r1) continue;
+      const uint32_t d = (uint32_t)__cvta_generic_to_shared(own + n * NORM_THREADS);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(z + row * ldz + 4 * i) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * PER * NORM_THREADS), "l"(y + row * width + 4 * i) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 32 * PER * NORM_THREADS), "l"(dout + row * width + 4 * i) : "memory");
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(r0);
+  float rnext = r0 < r1 ? rstd[r0] : 0.0f;
+  for (int64_t row = r0; row < r1; ++row) {
+    const float r = rnext;
+    if (row + 1 < r1) rnext = rstd[row + 1];
+    float4 zv[PER], yv[PER], dn[PER], gv[PER], sv[PER];
+    float dot = 0.0f;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+    for (int n = 0; n < PER; ++n) {
+      zv[n] = yv[n] = dn[n] = make_float4(0, 0, 0, 0);
+      if (threadIdx.x + n * blockDim.x < nvec) { zv[n] = own[n * NORM_THREADS]; yv[n] = own[(PER + n) * NORM_THREADS]; dn[n] = own[(2 * PER + n) * NORM_THREADS]; }
+    }
+    fetch(row + 1);
 #pragma unroll
     for (int n = 0; n < PER; ++n) {
       sv[n] = make_float4(sigmoid_acc(zv[n].x), sigmoid_acc(zv[n].y), sigmoid_acc(zv[n].z), sigmoid_acc(zv[n].w));

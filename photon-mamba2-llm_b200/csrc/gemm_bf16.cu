@@ -341,7 +341,7 @@ struct Epilogue {
             }
             uint32_t o[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) o[e] = (uint32_t)float_to_bf16_bits(v[2 * e]) | ((uint32_t)float_to_bf16_bits(v[2 * e + 1]) << 16);
+            for (int e = 0; e < 4; ++e) o[e] = bf16_of_two(v[2 * e], v[2 * e + 1]);
             asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
           }
           continue;

@@ -152,12 +152,6 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_pair_inplace_kernel(
   auto request = [&](const float* row, int i) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(srow_s + 16u * (uint32_t)i), "l"(row + 4 * i) : "memory");
   };
-  auto split = [](float v, uint32_t& h, uint32_t& l) {
-    uint32_t u = __float_as_uint(v);
-    h = (u + 0x7fffu + ((u >> 16) & 1u)) >> 16;
-    uint32_t ul = __float_as_uint(v - __uint_as_float(h << 16));
-    l = (ul + 0x7fffu + ((ul >> 16) & 1u)) >> 16;
-  };
   int64_t r = blockIdx.x;
   for (int i = threadIdx.x; i < V4; i += CE_THREADS) request(logits + r * ld, i);
   float vt = tail < V ? logits[r * ld + tail] : 0.0f;
@@ -199,15 +193,13 @@ __global__ void __launch_bounds__(CE_THREADS) cross_entropy_pair_inplace_kernel(
       if (more) request(next, i);
       const int c = 4 * i;
       float g[4] = {e.x * inv, e.y * inv, e.z * inv, e.w * inv};
-      uint32_t h[4], l4[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) { if (c + k == tg) g[k] -= 1.0f; split(g[k] * inv_rows, h[k], l4[k]); }
-      *reinterpret_cast<uint2*>(hi + c) = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
-      if (write_lo) *reinterpret_cast<uint2*>(lo + c) = make_uint2(l4[0] | (l4[1] << 16), l4[2] | (l4[3] << 16));
+      for (int k = 0; k < 4; ++k) { if (c + k == tg) g[k] -= 1.0f; g[k] *= inv_rows; }
+      store_pair4(hi + c, write_lo ? lo + c : nullptr, g[0], g[1], g[2], g[3]);
     }
     if (tail < V) {
       uint32_t h, l1;
-      split((srow[tail] * inv - (tail == tg ? 1.0f : 0.0f)) * inv_rows, h, l1);
+      split_bf16_pair((srow[tail] * inv - (tail == tg ? 1.0f : 0.0f)) * inv_rows, h, l1);
       hi[tail] = (uint16_t)h; if (write_lo) lo[tail] = (uint16_t)l1;
     }
   }
