@@ -106,9 +106,10 @@ struct Params {
   // (store_ops) x~ and xs as the kernel formed them.  bf16 x: store_ops leaves a copy of it.
   float *hprev, *yoff;
   int store_ops;
-  int whole, nseg, per;                                  // chains walked in one piece; segments of the others, steps per segment (see ChainPlan)
+  int first, nseg, per, div;                             // first chain of this launch; segments of a sequence, steps per segment, blocks per chain
+  int late;                                              // needs nothing from the kernel before, which lets this one in after its own wait: waits when it is done
   int state_only;                                        // first of two passes over segments: only seg_h and seg_d are formed
-  float *seg_h, *seg_d;                                  // (B*H-whole,nseg,N,P), (B*H-whole,nseg): state that a segment leaves when it starts from none, decay over it
+  float *seg_h, *seg_d;                                  // (B*H-whole,nseg-1,N,P), (B*H-whole,nseg-1): state that a segment leaves when it starts from none, decay over it (nobody reads the last one's)
   unsigned int* status;
 };
 
@@ -138,13 +139,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   float* sdt = sS + NSB * GE::SLOT;                                 // BIG: dt alone, the last kilobyte is not there
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  // blocks: the chains in one piece, then the others segment by segment (the first of two passes has these alone)
-  const int cut = (int)blockIdx.x - (p.state_only ? 0 : p.whole), nseg = cut < 0 ? 1 : p.nseg, per = cut < 0 ? p.nsteps : p.per;
-  const int bh = cut < 0 ? (int)blockIdx.x : p.whole + cut / nseg, seg = cut < 0 ? 0 : cut % nseg;
-  if (p.state_only && seg + 1 == nseg) return;             // (nobody starts from what the last one leaves)
+  const int bh = p.first + (int)blockIdx.x / p.div, seg = (int)blockIdx.x % p.div;
   const int h = bh % p.H, bb = bh / p.H, g = h / p.hpg;
-  const int i0 = seg * per, toff = i0 * L;                 // first step and token of this CTA's segment
-  const int n = min(per, p.nsteps - i0);
+  const int i0 = seg * p.per, toff = i0 * L;               // first step and token of this CTA's segment
+  const int n = min(p.per, p.nsteps - i0);
   const int64_t tokb = (int64_t)bb * p.T;
   if (threadIdx.x == 0) {
     const int mmas = p.state_only ? 1 : 2;                  // warps that issue products
@@ -168,8 +166,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  // A chain in one piece needs nothing from the first pass, which lets this kernel in only after its own wait.
-  if (p.state_only) { pdl_wait(); pdl_launch(); } else { pdl_launch(); if (cut >= 0 || p.nseg == 1) pdl_wait(); }
+  if (!p.late) pdl_wait();
+  pdl_launch();
   const uint32_t tG = tmem, tA1 = tmem + 256, tA2 = tmem + 320, tU = tmem + 384;
 
   auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
@@ -655,7 +653,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     }
     if (!p.state_only && active)
       for (int j = 0; j < seg; ++j) {                       // what the segments before this one leave
-        const int64_t row = cut - seg + j;
+        const int64_t row = (int64_t)(bh - p.first) * (p.nseg - 1) + j;
         const float* F = p.seg_h + row * NP + (int64_t)nr * p.P;
         const float dj = p.seg_d[row];
 #pragma unroll
@@ -725,7 +723,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       if (lane == 0) mbar_arrive(bar(UFREE));
     }
     if (ok && p.state_only && nr == 0) p.seg_d[blockIdx.x] = __expf(stot);
-    float* const leave = p.state_only ? p.seg_h + (int64_t)blockIdx.x * NP : p.last && seg + 1 == nseg ? p.last + (int64_t)bh * NP : nullptr;
+    float* const leave = p.state_only ? p.seg_h + (int64_t)blockIdx.x * NP : p.last && seg + 1 == p.nseg ? p.last + (int64_t)bh * NP : nullptr;
     if (ok && leave && active) {
       float* dst = leave + (int64_t)nr * p.P;
 #pragma unroll
@@ -739,6 +737,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
   }
+  if (p.late) pdl_wait();                                  // (a kernel completes after those before it)
 }
 
 // ---- host side -------------------------------------------------------------------------------------------
@@ -774,17 +773,23 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
   p.hp_hi = a.hp_hi; p.hp_lo = a.hp_lo; p.last = a.last; p.status = status_ptr();
   const int chains = a.B * a.H;
   const ChainPlan plan = NB == 1 && a.seg ? ssd_chain_plan(a.B, a.T, a.H) : ChainPlan{chains, 1, p.nsteps};
-  p.whole = plan.whole; p.nseg = plan.nseg; p.per = plan.per;
-  const unsigned cut = (unsigned)((chains - p.whole) * p.nseg);      // blocks of segments
+  const unsigned cut = (unsigned)((chains - plan.whole) * plan.nseg);      // blocks of segments
   if (cut) { p.seg_h = a.seg; p.seg_d = a.seg + (size_t)cut * a.N * a.P; }
   PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>);
+  auto run = [&](unsigned blocks) { return launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>, blocks, NTHREADS, GE::SMEM, ms, p); };
+  // the segments' states, the segments, and beside both the chains in one piece
   if (cut) {
-    p.state_only = 1;
-    PMB_TRY(launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>, cut, NTHREADS, GE::SMEM, ms, p));
-    p.state_only = 0;
+    p.first = plan.whole; p.nseg = plan.nseg; p.per = plan.per;
+    p.state_only = 1; p.div = plan.nseg - 1;
+    PMB_TRY(run(cut / p.nseg * p.div));
+    p.state_only = 0; p.div = plan.nseg;
   }
   p.store_ops = keep != nullptr;
-  PMB_TRY(launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>, (unsigned)p.whole + cut, NTHREADS, GE::SMEM, ms, p));
+  if (cut) PMB_TRY(run(cut));
+  if (plan.whole) {
+    p.first = 0; p.nseg = p.div = 1; p.per = p.nsteps; p.late = cut > 0;
+    PMB_TRY(run((unsigned)plan.whole));
+  }
   return PMB_OK;
 }
 
@@ -801,7 +806,7 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
 ChainPlan ssd_chain_plan(int B, int T, int H) {
   const int64_t chains = (int64_t)B * H;
   const int n = (int)cdiv(T, SCAN_STEP), rest = (int)(chains % 148 ? chains % 148 : 148);
-  const int most = 148 / rest, nseg = most < n / 2 ? most : n / 2;
+  const int most = chains > 148 && rest < 5 ? 32 : 148 / rest, nseg = most < n / 2 ? most : n / 2;      // (32: ChainBwdArgs.part)
   if (n < 4 || nseg < (chains > 148 ? 3 : 2)) return ChainPlan{(int)chains, 1, n};
   const int per = (int)cdiv(n, nseg);
   return ChainPlan{(int)(chains - rest), (int)cdiv(n, per), per};

@@ -84,9 +84,11 @@ struct Params {
   float* da;                                             // (B,T,H)
   uint16_t *raw_hi, *raw_lo; int64_t ld_raw; int raw_col;                  // dt mode: gradient before the softplus as a bf16 pair (raw_lo may be NULL)
   float* part; int64_t part_pitch;                       // dt mode: per (b, h) sums for dA, dD and d_dt_bias, `part_pitch` apart
-  int whole, nseg, per;                                  // chains walked in one piece; segments of the others, steps per segment (see ChainPlan)
+  int first, nseg, per, div;                             // first chain of this launch; segments of a sequence, steps per segment, blocks per chain
+  int late;                                              // needs nothing from the kernel before, which lets this one in after its own wait: waits when it is done
+  int rows, fill;                                        // rows of `part` per (b, h); of them a block writes its own, a chain in one piece all (zeros: no more than a warp has lanes)
   int state_only;                                        // first of two passes over segments: only seg_h and seg_d are formed
-  float *seg_h, *seg_d;                                  // (B*H-whole,nseg,N,P), (B*H-whole,nseg): adjoint that a segment hands back when it receives none, decay over it
+  float *seg_h, *seg_d;                                  // (B*H-whole,nseg-1,N,P), (B*H-whole,nseg-1): adjoint that a segment hands back when it receives none, decay over it (nobody receives the first one's)
   unsigned int* status;
 };
 
@@ -132,12 +134,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
   float* sRows = sS + NSB * GE::SLOT;                                     // [2 steps] per-row sums
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  // blocks: the chains in one piece, then the others segment by segment (the first of two passes has these alone)
-  const int cut = (int)blockIdx.x - (p.state_only ? 0 : p.whole), nseg = cut < 0 ? 1 : p.nseg, per = cut < 0 ? p.nsteps : p.per;
-  const int bh = cut < 0 ? (int)blockIdx.x : p.whole + cut / nseg, seg = cut < 0 ? 0 : cut % nseg;
-  if (p.state_only && seg == 0) return;                    // (nobody receives what the first one hands back)
+  const int bh = p.first + (int)blockIdx.x / p.div, seg = (int)blockIdx.x % p.div + p.nseg - p.div;
   const int h = bh % p.H, bb = bh / p.H, g = h / p.hpg;
-  const int n = min(per, p.nsteps - seg * per), last = seg * per + n - 1;      // steps of this CTA's segment, the last one of them
+  const int n = min(p.per, p.nsteps - seg * p.per), last = seg * p.per + n - 1;      // steps of this CTA's segment, the last one of them
   const int64_t tokb = (int64_t)bb * p.T;
   if (threadIdx.x == 0) {
     mbar_init(bar(FULL), 1); mbar_init(bar(EMPTY), p.state_only ? 1 : 6);
@@ -157,8 +156,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  // A chain in one piece needs nothing from the first pass, which lets this kernel in only after its own wait.
-  if (p.state_only) { pdl_wait(); pdl_launch(); } else { pdl_launch(); if (cut >= 0 || p.nseg == 1) pdl_wait(); }
+  if (!p.late) pdl_wait();
+  pdl_launch();
   const uint32_t tG = tmem, tM = tmem + 128, tA1 = tmem + 256, tA2 = tmem + 320, tA3 = tmem + 384, tU = tmem + 448;
 
   auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
@@ -383,11 +382,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       if (dtm) {
         accA = warp_sum(accA); accB = warp_sum(accB);
         // (row of `part`: segment by segment of a sequence; a chain in one piece fills its rows with zeros)
-        if (lane == 0)
-          for (int j = seg; j < (cut < 0 ? p.nseg : seg + 1); ++j) {
-            const int64_t o = ((int64_t)bb * p.nseg + j) * p.H + h;
-            p.part[o] = j == seg ? accA : 0.0f; p.part[2 * p.part_pitch + o] = j == seg ? accB : 0.0f;
-          }
+        if (lane < p.fill) {
+          const int64_t o = ((int64_t)bb * p.rows + seg + lane) * p.H + h;
+          p.part[o] = lane == 0 ? accA : 0.0f; p.part[2 * p.part_pitch + o] = lane == 0 ? accB : 0.0f;
+        }
       }
     }
   } else if (warp < W_XF) {
@@ -715,8 +713,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
 #pragma unroll
     for (int q = 0; q < PW; ++q) hv[q] = 0.0f;
     if (!p.state_only && active)
-      for (int j = nseg - 1; j > seg; --j) {                // what the segments after this one hand back
-        const int64_t row = cut - seg + j;
+      for (int j = p.nseg - 1; j > seg; --j) {              // what the segments after this one hand back
+        const int64_t row = (int64_t)(bh - p.first) * (p.nseg - 1) + j - 1;
         const float* F = p.seg_h + row * NP + (int64_t)nr * p.P;
         const float dj = p.seg_d[row];
 #pragma unroll
@@ -809,15 +807,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (threadIdx.x == 0 && p.part && !p.state_only) {
+  if ((int)threadIdx.x < p.fill && p.part && !p.state_only) {
     float t = 0.0f;                                         // fixed order
     for (int q = 0; q < 8; ++q) t += dDw[q];
-    for (int j = seg; j < (cut < 0 ? p.nseg : seg + 1); ++j) p.part[p.part_pitch + ((int64_t)bb * p.nseg + j) * p.H + h] = j == seg ? t : 0.0f;
+    p.part[p.part_pitch + ((int64_t)bb * p.rows + seg + threadIdx.x) * p.H + h] = threadIdx.x == 0 ? t : 0.0f;
   }
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
   }
+  if (p.late) pdl_wait();                                  // (a kernel completes after those before it)
 }
 
 // ---- host side -------------------------------------------------------------------------------------------
@@ -855,17 +854,23 @@ static pmb_status launch(cudaStream_t st, const ChainBwdArgs& a) {
   p.raw_hi = a.raw_hi; p.raw_lo = a.raw_lo; p.ld_raw = a.ld_raw; p.raw_col = a.raw_col; p.part = a.part; p.status = status_ptr();
   const int chains = a.B * a.H;
   const ChainPlan plan = a.seg ? ssd_chain_plan(a.B, a.T, a.H) : ChainPlan{chains, 1, n};
-  p.whole = plan.whole; p.nseg = plan.nseg; p.per = plan.per;
-  const unsigned cut = (unsigned)((chains - p.whole) * p.nseg);      // blocks of segments
+  const unsigned cut = (unsigned)((chains - plan.whole) * plan.nseg);      // blocks of segments
   if (cut) { p.seg_h = a.seg; p.seg_d = a.seg + (size_t)cut * a.N * a.P; }
-  p.part_pitch = (int64_t)chains * p.nseg;
+  p.rows = plan.nseg; p.fill = 1; p.part_pitch = (int64_t)chains * plan.nseg;
   PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_bwd_kernel<NI, ND, NK, IN16>);
+  auto run = [&](unsigned blocks) { return launch_pdl(st, ssd_chain_bwd_kernel<NI, ND, NK, IN16>, blocks, NTHREADS, GE::SMEM, ms, p); };
+  // the segments' adjoints, the segments, and beside both the chains in one piece
   if (cut) {
-    p.state_only = 1;
-    PMB_TRY(launch_pdl(st, ssd_chain_bwd_kernel<NI, ND, NK, IN16>, cut, NTHREADS, GE::SMEM, ms, p));
-    p.state_only = 0;
+    p.first = plan.whole; p.nseg = plan.nseg; p.per = plan.per;
+    p.state_only = 1; p.div = plan.nseg - 1;
+    PMB_TRY(run(cut / p.nseg * p.div));
+    p.state_only = 0; p.div = plan.nseg;
+    PMB_TRY(run(cut));
   }
-  PMB_TRY(launch_pdl(st, ssd_chain_bwd_kernel<NI, ND, NK, IN16>, (unsigned)p.whole + cut, NTHREADS, GE::SMEM, ms, p));
+  if (plan.whole) {
+    p.first = 0; p.nseg = p.div = 1; p.per = n; p.late = cut > 0; p.fill = plan.nseg;
+    PMB_TRY(run((unsigned)plan.whole));
+  }
   return PMB_OK;
 }
 
