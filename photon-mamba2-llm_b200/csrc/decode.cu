@@ -711,7 +711,7 @@ extern "C" pmb_status pmb_mamba2_step(void* stream, const pmb_mamba2_config* cfg
   // Up to 16 sequences the products are fp32 FMA (y 2e-7 of its norm from fp64), beyond on bf16 pairs (7e-6).  Where the line
   // lies is a matter of that precision, not of time.  us per step, FMA / tensor cores (24 heads of 64 x 64 at d_model 768; 32 of 64 x 128
   // at d_model 2048): 1 sequence 14.2 / 19.0, 21.1 / 26.6; 2: 14.1 / 19.8, 23.9 / 28.3; 4: 14.6 / 20.3, 28.3 / 28.4; 8: 18.4 / 22.1, 31.4 / 29.0;
-  // 16: 27.2 / 22.6, 48.1 / 31.1; 17: 22.9 and 31.6.
+  // 16: 27.2 / 22.6, 48.1 / 31.1; 17: 22.9 and 31.6 (20.5 and 30.4 since that side's steps take two launches less).
   if (fma) {
     dec::GemvArgs a{};
     a.B = d.B; a.K = d.D; a.N = d.J; a.W = p->in_proj_weight; a.ldw = d.J; a.in = d_x_t; a.in_vec = al(d_x_t); a.st = si;

@@ -813,6 +813,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ Group g) {
 // 256 KB of fp32 that a tile writes.  Four epilogue warps were the limit there: products with a bf16 residual 67 -> 40 us, the two
 // gradients of in_proj at 16384 tokens 165 -> 129, of the tied head per 1024 rows 339 -> 254.
 // The warp index is a shuffle's result, so that the roles' branches are uniform to the compiler: 2 % of the training steps' products.
+// Plain products of 16384 x 4096 x 768 take 65 us without an epilogue, 66 with the accumulators read, 82 with bf16 results, 104 with fp32
+// ones: the results' bytes at HBM's rate on top of the products, however they leave (fragments, slots and TMA, whole lines through shared
+// memory) and whenever (paced over the next tile, clusters staggered).  Tiles of 512 columns, one pass over A for both accumulators: 107 and 130.
 // The CTA-pair kernel above as a tile loop: cluster c works on tiles c, c + clusters, ...; the operand ring keeps
 // running across tiles; the accumulator alternates between two TMEM buffers of BN2 columns, so each CTA drains its
 // 128 rows of tile i (through the same TMA-store epilogue as the single-CTA kernel) while the leader issues tile
