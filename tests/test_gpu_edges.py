@@ -551,6 +551,46 @@ def test_scan_last_round_in_segments(pm, B, H, T):
         assert_close(got, want, tol=tol, what=what)
 
 
+# the launches of such a call overlap one another and the next call's: the same bits as with the device idle in between, and in a graph
+@pytest.mark.parametrize("B", [19, 24])
+def test_scans_in_segments_back_to_back(pm, B):
+    T, H, P, N = 896, 8, 16, 24
+    scans = []
+    for k in range(2):
+        x, b, c, dy = (randn(sh, 10 * k + i).bfloat16().cuda() for i, sh in enumerate([(B, T, H, P), (B, T, 1, N), (B, T, 1, N), (B, T, H, P)]))
+        a = -torch.nn.functional.softplus(randn((B, T, H), 10 * k + 5) - 2.0).cuda()
+        scans.append((pm.SsdScanBf16(x, a, b, c, 128), dy))
+
+    def run(pause):
+        out = []
+        for _ in range(3):
+            for scan, dy in scans:
+                out.append(scan.forward())
+                pause()
+                out.extend(scan.backward(dy))
+                pause()
+        torch.cuda.synchronize()
+        return out
+
+    want = run(torch.cuda.synchronize)
+    for got, ref in zip(run(lambda: None), want):
+        assert torch.equal(got, ref)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        for scan, dy in scans:
+            scan.forward(); scan.backward(dy)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        out = [t for scan, dy in scans for t in (scan.forward(), *scan.backward(dy))]
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    for got, ref in zip(out, want):
+        assert torch.equal(got, ref)
+    assert pm.device_status() == 0
+
+
 @pytest.mark.parametrize("B", [19, 24])
 def test_block_last_round_in_segments(pm, B):
     D, H, P, N, T, Q = 64, 8, 16, 16, 770, 64
