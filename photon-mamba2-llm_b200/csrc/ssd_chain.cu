@@ -86,7 +86,7 @@ struct Geo {
   static constexpr int AHEAD = BIG || XIN16 ? 0 : ND == 2 ? 3 : 16;
   // (BIG: no room for column factors and half of the alignment slack; shared memory starts 1024-byte aligned where nothing static
   // precedes it, and the kernel checks)
-  static constexpr int SLOT = (BIG ? 1 : 2) * L, SLACK = BIG ? 512 : 1024;    // floats per copy of S: [S | column factors]
+  static constexpr int SLOT = BIG ? L : 2 * L + 4, SLACK = BIG ? 512 : 1024;    // floats per copy of S: [S | column factors | what they refer to]
   static constexpr int SMEM = TILES + SLACK + 256 /*barriers*/ + NSB * SLOT * 4 + (BIG ? 4 : 8) * NB * L /*row factors*/ + AHEAD * XF_THREADS * 16;
 };
 
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   volatile uint32_t* abort_flag = tmem_slot + 1;
   float* wsum = reinterpret_cast<float*>(bar_ptr + 8 * NBAR + 8);
   float* sEnd = wsum + 8;                                   // S_end of the last four chunks
-  float* sS = reinterpret_cast<float*>(bar_ptr + 256);      // [NSB][S | FACT: exp(S_q - S), q = last token of the token's 32]
+  float* sS = reinterpret_cast<float*>(bar_ptr + 256);      // [NSB][S | FACT: exp(m - S), m = smallest S of the token's 32 | FACT: the four m]
   float2* sfac = reinterpret_cast<float2*>(sS + NSB * GE::SLOT);    // (dt, exp(S_end - S)) of the step's rows
   float* sdt = sS + NSB * GE::SLOT;                                 // BIG: dt alone, the last kilobyte is not there
 
@@ -367,8 +367,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
           uint32_t r[32];
           tmem_ld32(tg, r);
           if (FACT && cb < diag) {
-            // every column is before every row: exp(S_t - S_s) = exp(S_t - S_q) exp(S_q - S_s) with q the block's last column
-            const float rf = __expf(S_row - S[32 * cb + 31]);
+            // every column is before every row: exp(S_t - S_s) = exp(S_t - m) exp(m - S_s), m as below where the factors are formed
+            const float rf = __expf(S_row - S[2 * L + cb]);
 #pragma unroll
             for (int e4 = 0; e4 < 8; ++e4) {
               const float4 cf = *reinterpret_cast<const float4*>(S + L + 32 * cb + 4 * e4);
@@ -573,7 +573,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
             v[u] += off[u];
             if (q == NB * L - 1) v[u] = send;
             S[q] = v[u];
-            if (FACT) S[L + q] = __expf(__shfl_sync(0xffffffffu, v[u], 31) - v[u]);
+            if (FACT) {
+              // m = the smallest S of the 32 columns, their last where a <= 0.  Where a is positive for a while (bf16 x comes with any a)
+              // S can rise and fall by more than fp32's exponent inside a step: no factor exp(m - S_s) is above 1, and exp(S_t - m)
+              // overflows only where an exponential of the row does.
+              const float m = warp_min(v[u]);
+              S[L + q] = __expf(m - v[u]);
+              if (lane == 0) S[2 * L + q / 32] = m;
+            }
             if (GE::BIG) sdt[q] = dtv[u]; else sfac[q] = make_float2(dtv[u], __expf(send - v[u]));
             if (q == NB * L - 1) sEnd[c & 3] = send;
             if (t < p.T) {

@@ -65,7 +65,7 @@ struct Geo {
   static constexpr int AHEAD = IN16 ? 0 : 2;             // fp32: pieces of x and of dY that a transform thread has in flight (bf16: the tiles are copied as they are)
   static constexpr int TILES = STAGE + XB * XBUF + HT;
   static constexpr int ROWS = 11 * L;                    // per-row sums: [2 groups] of W, e, f; W[s,s]; [4 quarters] column sums of W
-  static constexpr int SLOT = 3 * L;                     // a step's [S | dt | column factors]
+  static constexpr int SLOT = 3 * L + 4;                 // a step's [S | dt | column factors | what they refer to]
   static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 512 /*barriers, small sums*/ + (NSB * SLOT + 2 * ROWS) * 4 + 2 * AHEAD * XF_THREADS * 16;
 };
 
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
   float* ddw = reinterpret_cast<float*>(bar_ptr + 8 * NBAR + 16);      // [2 steps][4 state warps] <dh, h>
   float* dDw = ddw + 8;                                                // [8 transform warps] <dY, x>
   float* sWend = dDw + 8;                                              // [4 transform warps] S of their last token
-  float* sS = reinterpret_cast<float*>(bar_ptr + 512);                 // [NSB] S, dt and column factor exp(S_t - S_q) of a step's tokens, q = the last one before the token's 32
+  float* sS = reinterpret_cast<float*>(bar_ptr + 512);                 // [NSB] S, dt and column factor exp(S_t - m) of a step's tokens, m = the largest S of the token's 32 and of the token before them; the four m
   float* sRows = sS + NSB * GE::SLOT;                                     // [2 steps] per-row sums
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -528,14 +528,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
           tmem_st16(tG + tb, z);
           if (ND == 2) tmem_st16(tG + tb + 16u, z);
         } else {
-          // past the diagonal (every column past every row): exp(S_t - S_s) = exp(S_t - S_q) exp(S_q - S_s), q = the last token before the columns
+          // past the diagonal (every column past every row): exp(S_t - S_s) = exp(S_t - m) exp(m - S_s), m as below where the factors are formed
           auto block = [&](auto diagonal) {
             constexpr bool DIAG = decltype(diagonal)::value;
             float rf[4];
             if (!DIAG) {
-              const float sq = S[32 * cb - 1];
+              const float m = S[3 * L + cb];
 #pragma unroll
-              for (int e = 0; e < 4; ++e) rf[e] = __expf(sq - Sr[e]);
+              for (int e = 0; e < 4; ++e) rf[e] = __expf(m - Sr[e]);
             }
             const float* Sc = S + (DIAG ? 0 : 2 * L) + 32 * cb + fc;      // S, or the columns' factors
 #pragma unroll
@@ -648,7 +648,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       if (ok && tid < L) { S[tid] = sv; S[L + tid] = d_next; }
       if (lane == 31 && tid < L) sWend[wx] = sv;
       asm volatile("bar.sync 4, %0;" ::"n"(256) : "memory");        // (a warp that gave up keeps reaching the named barriers)
-      if (ok && tid < L) S[2 * L + tid] = __expf(sv - sWend[wx > 0 ? wx - 1 : 0]);
+      if (ok && tid < L) {
+        // m = the largest S of the 32 columns and of the token before them, that token's where a <= 0: as in the forward, no factor
+        // exp(S_t - m) is above 1, and exp(m - S_s) overflows only where an exponential of the row does
+        const float m = fmaxf(sWend[wx > 0 ? wx - 1 : 0], warp_max(sv));
+        S[2 * L + tid] = __expf(sv - m);
+        if (lane == 0) S[3 * L + wx] = m;
+      }
       asm volatile("bar.sync 4, %0;" ::"n"(256) : "memory");
       if (!ok) continue;
       if (lane == 0) mbar_arrive(bar(SRDY + (k % NSB)));

@@ -96,6 +96,17 @@ __device__ __forceinline__ void st_shared_v2(uint32_t a, uint32_t x, uint32_t y)
 __device__ __forceinline__ void st_shared_v4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
+// smallest and largest value of a warp
+__device__ __forceinline__ float warp_min(float v) {
+  float r;
+  asm volatile("redux.sync.min.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float warp_max(float v) {
+  float r;
+  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
+  return r;
+}
 // two fp32 values -> packed bf16x2 of their high parts (round to nearest even) and of the remainders
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo, bool want_lo) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);

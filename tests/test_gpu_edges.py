@@ -494,6 +494,33 @@ def test_scan_bf16_strong_decay(pm, T, Q, N, strength):
         assert_close(got, want, tol=tol, what=what)
 
 
+# a that is positive for a while: inside a step S rises (falls) by `rise` and comes back, so that the factors of a block beyond 88 are inf and 0
+# where the rows outside have ordinary exponentials.  Rows inside the excursion overflow and are left out, as are dx of the rise and y of the
+# fall, whose states do.  bf16 inputs (rounded and kept as pairs), ragged and whole lengths, segments; bf16 results as in the tests above.
+@pytest.mark.parametrize("T,Q", [(128, 128), (200, 128), (512, 128), (1500, 256)])
+@pytest.mark.parametrize("N", [64, 128])
+@pytest.mark.parametrize("rise", [12.0, 30.0, 100.0])
+def test_scan_bf16_positive_a(pm, T, Q, N, rise):
+    B, H, P = 1, 4, 64
+    x, b, c, dy = randn((B, T, H, P), 1).bfloat16(), randn((B, T, 1, N), 2).bfloat16(), randn((B, T, 1, N), 3).bfloat16(), randn((B, T, H, P), 4).bfloat16()
+    for sign, first, end, what in ((1.0, 20, 40, "y"), (-1.0, 70, 100, "dx")):
+        a = -torch.nn.functional.softplus(randn((B, T, H), 5) - 2.0)
+        out = torch.ones(T, dtype=torch.bool)
+        for t0 in range(0, T - end, 128):
+            a[:, t0 + first] += sign * rise
+            a[:, t0 + end] -= sign * rise
+            out[t0 + first:t0 + end] = False
+        scan = pm.SsdScanBf16(x.cuda(), a.cuda(), b.cuda(), c.cuda(), Q)
+        got = scan.forward()
+        xd = x.double().requires_grad_(True)
+        want = orc.ssd_scan_chunked(xd, a.double(), *(t.double().expand(B, T, H, N) for t in (b, c)), Q if T % Q == 0 else T)
+        if what == "dx":
+            got = scan.backward(dy.cuda())[0]
+            want, = torch.autograd.grad(want, xd, dy.double())
+        assert pm.device_status() == 0
+        assert_close(got.float()[:, out], want.detach()[:, out], tol=5e-3, what=what)
+
+
 # products whose columns go to tiles of two widths: two rounds of tiles, a cut inside and one before the last tile, B in either order, a residual
 @pytest.mark.parametrize("M,N,K", [(2048, 3224, 768), (1337, 3224, 136), (1000, 5000, 64)])
 @pytest.mark.parametrize("tb,res", [(False, False), (True, True)])
