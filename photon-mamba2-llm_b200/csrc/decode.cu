@@ -592,9 +592,21 @@ struct StepWs {
   float* normed;
 };
 
-// K splits of the tensor-core projection: one wave of CTAs, at least two k-tiles each
+// Sequences per tile of the tensor-core projection.  128 where the SMs are shared by K splits: two tiles of 128 take half the splits of one
+// of 256, so half the sums go through memory.  256 where there is one split either way and tiles of 128 need a second round, and where they
+// leave one split of 24 k-tiles or more.  Each weight is converted once per tile.  What 256 gives of a step in us, for in_proj and out_proj
+// by tiles of 128 (k-tiles): 24 heads of 64 x 64 at d_model 768, 256 sequences -1.5 with 52 (12), -2.4 with 12 (24); 640 -5.4 with 130,
+// -3.3 with 30; 768 +6.1 with 156; 2048 (417) +4.1 with 416, +6.1 with 96; 32 heads of 64 x 128 at 2048, 256 sequences -2.9 with 70 (32), -4.5
+// with 32 (32); 512 -0.5 with 140, -0.6 with 64; 768 (357) +11.8 with 210, +7.4 with 96; 8 heads of 64 x 64 at 256, 1024 sequences -2.3 with 80
+// (4); 2048 +2.7 with 160.  (64 at 256 sequences: 67.5, 145 and 31.5 where 128 took 65.4, 127.1 and 33.1.)
+static int64_t skinny_tile(int64_t B, int64_t J, int64_t K) {
+  const int64_t tiles = cdiv(J, 128) * cdiv(B, 128);
+  if (B > 128 && (tiles > 148 || (tiles > 74 && K >= 24 * dec::SK_BK))) return 256;
+  return B > 64 ? 128 : (B > 32 ? 64 : 32);
+}
+// K splits: one wave of CTAs, at least two k-tiles each
 static int skinny_splits(int64_t B, int64_t J, int64_t K) {
-  const int64_t nb = B > 64 ? 128 : (B > 32 ? 64 : 32);
+  const int64_t nb = skinny_tile(B, J, K);
   const int64_t ctas = cdiv(J, 128) * cdiv(B, nb), kt = cdiv(K, dec::SK_BK);
   int64_t sp = 148 / ctas;
   if (sp > kt / 2) sp = kt / 2;
@@ -670,11 +682,11 @@ static pmb_status skinny_nb(cudaStream_t st, const float* x, const uint16_t* hi,
   ProfScope prof(st, "decode_gemm", 2.0 * B * K * J, 4.0 * ((double)K * J + (double)splits * B * J));
   return launch_pdl(st, dec::skinny_gemm_kernel<NB, XC>, dim3((unsigned)cdiv(J, 128), (unsigned)splits, (unsigned)cdiv(B, NB)), dec::SK_THREADS, dec::SkGeo<NB>::SMEM, ms, a);
 }
-// 128 sequences to a tile and no more: two of them take half the K splits of one of 256, so half the sums go through memory (256 sequences,
-// us per step: 24 heads at d_model 768 69.0 with 256, 65.4 with 128, 67.5 with 64; 32 heads at 2048 129.4, 127.1 and 145; 8 heads at 512 38.9, 33.1, 31.5).
 static pmb_status skinny(cudaStream_t st, const float* x, const uint16_t* hi, const uint16_t* lo, int64_t B, int64_t K, int64_t J, const float* W, bool early, float* slab, int splits) {
-  if (B > 64) return skinny_nb<128, false>(st, nullptr, hi, lo, B, K, J, W, early, slab, splits);
-  if (B > 32) return x ? skinny_nb<64, true>(st, x, hi, lo, B, K, J, W, early, slab, splits) : skinny_nb<64, false>(st, x, hi, lo, B, K, J, W, early, slab, splits);
+  const int64_t nb = skinny_tile(B, J, K);
+  if (nb == 256) return skinny_nb<256, false>(st, nullptr, hi, lo, B, K, J, W, early, slab, splits);
+  if (nb == 128) return skinny_nb<128, false>(st, nullptr, hi, lo, B, K, J, W, early, slab, splits);
+  if (nb == 64) return x ? skinny_nb<64, true>(st, x, hi, lo, B, K, J, W, early, slab, splits) : skinny_nb<64, false>(st, x, hi, lo, B, K, J, W, early, slab, splits);
   return x ? skinny_nb<32, true>(st, x, hi, lo, B, K, J, W, early, slab, splits) : skinny_nb<32, false>(st, x, hi, lo, B, K, J, W, early, slab, splits);
 }
 

@@ -161,6 +161,22 @@ def test_decode_batches(pm, B, D, H, P, N, G):
     assert pm.device_status() == 0
 
 
+# as many sequences as tiles of 128 of them fit on the SMs at once (in_proj has nine column tiles), and one more, which is alone in a tile of
+# 256; as many as leave out_proj two splits of its 24 k-tiles (seven column tiles), and one more
+@pytest.mark.parametrize("B,D,H,P", [(2048, 200, 8, 64), (2049, 200, 8, 64), (1280, 800, 24, 64), (1281, 800, 24, 64)])
+def test_decode_tiles_of_many_sequences(pm, B, D, H, P):
+    N = 16
+    cfg, p, blk = _block(pm, D, H, P, N, 1, 64, torch.float32)
+    ref = {"ssm_state": randn((B, H, N, P), 7, 0.3), "conv_window": randn((B, cfg.xbc_dim, 3), 8, 0.5)}
+    x = randn((B, 1, D), 20)
+    y, st = blk.step(x.cuda(), {k: v.cuda() for k, v in ref.items()})
+    y_ref, ref = orc.block_step(p, cfg, x, ref)
+    assert_close(y, y_ref, what="y")
+    assert_close(st["ssm_state"], ref["ssm_state"], what="state")
+    assert_close(st["conv_window"], ref["conv_window"], what="window")
+    assert pm.device_status() == 0
+
+
 # weight rows that take a thread more than one pass of its groups, with a remainder, on both products; beyond 16 sequences the two widths
 # that convert the token themselves, with a part of a tile at the end; offset 1: the token and the norm's weight off the 16-byte grid
 @pytest.mark.parametrize("offset", [0, 1])
