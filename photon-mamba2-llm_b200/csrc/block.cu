@@ -193,16 +193,18 @@ static ChainArgs chain_inputs(const Dims& d, const pmb_block_params& p, const fl
   return a;
 }
 
-// bf16-storage blocks on whole chunks: plain bf16 operands, and few long sequences scanned chunk by chunk instead of as chains.  (Plain
-// bf16 chunks keep the rounding of the kernels that work chunk by chunk, so their sequences are not cut into segments.  One step of a
-// chain takes 3.5 us; those kernels 30 us and 0.1 us per step of a head.  Where a backward follows the chain also writes what that reads:
-// 7.7 us per step against 30 us and 0.07.  Long-context step 49.09 -> 47.14 ms; with the first line, blocks of 48 chains of twelve steps
-// lost 4 %.)
+// bf16-storage blocks on whole chunks: plain bf16 operands, and few long sequences scanned chunk by chunk instead of as chains, which are
+// not cut into segments here (a chain's S, state and xs go by chunks of two steps where the chunk has them).  What a chain's steps take, one
+// after the other, beyond a fixed cost, against the chunk-by-chunk kernels' time per step of a head; where a backward follows, the chain also
+// writes what that reads.  Fitted to 130 shapes of 8 to 32 heads, 512 to 8192 tokens: the slower side is taken by at most 1.3 % of a block's
+// forward and 0.6 % of its backward.  us, chains / chunk by chunk: forward 1 x 1024 tokens, 8 heads 53 / 46, 32 heads 70 / 75; 1 x 2048,
+// 24 heads 103 / 99; 2 x 2048, 24 heads 126 / 143; 4 x 2048, 8 heads 106 / 102; backward 1 x 512, 8 heads 115 / 114, 24 heads 156 / 162;
+// 2 x 2048, 24 heads 419 / 409, 32 heads 486 / 497; 4 x 4096, 24 heads 1194 / 1297.
 static bool block_plain16(const Dims& d, bool bf16) { return bf16 && ssd_plain16_shape(d.P, d.N, d.Q); }
 static bool scan_by_chunks(const Dims& d, bool bf16, bool keep) {
   const double steps = (double)cdiv(d.T, SCAN_STEP), chains = (double)d.B * d.H;
   if (!block_plain16(d, bf16)) return false;
-  return keep ? 7.7 * steps * (chains > 148.0 ? chains / 148.0 : 1.0) > 30.0 + 0.07 * chains * steps : 3.5 * steps > 30.0 + 0.1 * chains * steps;
+  return (keep ? 4.4 : 3.0) * steps > 12.0 + 0.07 * chains * steps;
 }
 
 // Steps 1-8 of Mamba2Block::forward (block.rs:143-222): everything up to the normalised gate output.

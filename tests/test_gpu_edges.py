@@ -142,6 +142,27 @@ def test_block_bf16_weight_gradient_splits(pm, B, T):
         assert_close(grads[k], leaves[k].grad, tol=2e-2, what=k)
 
 
+# bf16 storage on whole chunks, on either side of the lines between the scan as chains and chunk by chunk: both as chains, the recompute chunk by
+# chunk, both chunk by chunk; chunks of one and two steps.  Tolerances of the tests above.
+@pytest.mark.parametrize("B,T", [(5, 512), (1, 512), (1, 1024)])
+@pytest.mark.parametrize("Q", [128, 256])
+def test_block_bf16_chains_or_chunks(pm, B, T, Q):
+    cfg, p, blk = _block(pm, 64, 8, 64, 64, 1, Q, torch.bfloat16)
+    x, cot = randn((B, T, 64), 5).bfloat16(), randn((B, T, 64), 6).bfloat16()
+    out = blk.forward(x.cuda())
+    dx, grads = blk.backward(x.cuda(), cot.cuda())
+    torch.cuda.synchronize()
+    assert pm.device_status() == 0
+    leaves = {k: v.clone().requires_grad_(True) for k, v in p.items()}
+    xr = x.float().requires_grad_(True)
+    ref = orc.block_forward(leaves, cfg, xr)
+    ref.backward(cot.float())
+    assert_close(out.float(), ref, tol=2e-2, what="out")
+    assert_close(dx.float(), xr.grad, tol=3e-2, what="dx")
+    for k, v in leaves.items():
+        assert_close(grads[k], v.grad, tol=2e-2, what=k)
+
+
 # batch sizes around the switch from streamed FMA to tensor-core projections and its tile widths; widths with ragged column
 # tiles; the last ones are served by the general kernels, or have an odd d_state per head under the vectorised state step
 @pytest.mark.parametrize("B", [1, 2, 3, 5, 9, 16, 17, 33, 70, 130, 300])
