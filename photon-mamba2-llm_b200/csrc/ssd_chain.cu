@@ -86,7 +86,10 @@ struct Geo {
   static constexpr int AHEAD = BIG || XIN16 ? 0 : ND == 2 ? 3 : 16;
   // (BIG: no room for column factors and half of the alignment slack; shared memory starts 1024-byte aligned where nothing static
   // precedes it, and the kernel checks)
-  static constexpr int SLOT = BIG ? L : 2 * L + 4, SLACK = BIG ? 512 : 1024;    // floats per copy of S: [S | column factors | what they refer to]
+  // the masked tile by factors of blocks instead of an exponential per element: not where the rounding of M to bf16 is part of a stream
+  // of bf16 values (the storage blocks on plain operands: each flipped rounding would grow through the layers behind it)
+  static constexpr bool FACT = NB == 1 && !BIG && (ND == 2 || XIN16);
+  static constexpr int SLOT = FACT ? 2 * L + 4 : BIG ? L : 2 * L, SLACK = BIG ? 512 : 1024;    // floats per copy of S: [S | column factors | what they refer to]
   static constexpr int SMEM = TILES + SLACK + 256 /*barriers*/ + NSB * SLOT * 4 + (BIG ? 4 : 8) * NB * L /*row factors*/ + AHEAD * XF_THREADS * 16;
 };
 
@@ -117,10 +120,8 @@ struct Params {
 template <int NI, int ND, int NK, int NB, bool XIN16>
 __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid_constant__ Maps maps, const Params p) {
   using GE = Geo<NI, ND, NK, NB, XIN16>;
+  constexpr bool FACT = GE::FACT;
   constexpr int STG = GE::STG, XB = GE::XB, NSB = GE::NSB, OUTW = GE::OUTW, XFW = GE::XFW, XF_THREADS = GE::XF_THREADS, W_XF = W_OUT + OUTW;
-  // the masked tile by factors of blocks instead of an exponential per element: not where the rounding of M to bf16 is part of a stream
-  // of bf16 values (the storage blocks on plain operands: each flipped rounding would grow through the layers behind it)
-  constexpr bool FACT = NB == 1 && !GE::BIG && (ND == 2 || XIN16);
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
