@@ -89,8 +89,9 @@ struct Geo {
   // the masked tile by factors of blocks instead of an exponential per element: not where the rounding of M to bf16 is part of a stream
   // of bf16 values (the storage blocks on plain operands: each flipped rounding would grow through the layers behind it)
   static constexpr bool FACT = NB == 1 && !BIG && (ND == 2 || XIN16);
-  static constexpr int SLOT = FACT ? 2 * L + 4 : BIG ? L : 2 * L, SLACK = BIG ? 512 : 1024;    // floats per copy of S: [S | column factors | what they refer to]
-  static constexpr int SMEM = TILES + SLACK + 256 /*barriers*/ + NSB * SLOT * 4 + (BIG ? 4 : 8) * NB * L /*row factors*/ + AHEAD * XF_THREADS * 16;
+  static constexpr int BARS = XIN16 ? 320 : 256;         // bytes of barriers and small sums
+  static constexpr int SLOT = (BIG ? 1 : 2) * L, SLACK = BIG ? 512 : 1024;    // floats per copy of S: [S | column factors]
+  static constexpr int SMEM = TILES + SLACK + BARS + NSB * SLOT * 4 + (BIG ? 4 : 8) * NB * L /*row factors*/ + AHEAD * XF_THREADS * 16;
 };
 
 struct Maps { CUtensorMap b[2], c[2], x, xt, xs; };      // [0] = hi (or the plain bf16 tensor), [1] = lo; x = bf16 x
@@ -129,14 +130,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   uint8_t* base_ptr = smem_raw + (base - raw);
   const uint32_t ring_s = base, xbuf_s = ring_s + STG * GE::STAGE, h_s = xbuf_s + XB * GE::XBUF, bars = h_s + GE::HB;
   enum { FULL = 0, EMPTY = 2, XRDY = 4, XFREE = 6, SRDY = 8 /*4*/, GFULL = 12, MRDY = 14, UFULL = 16, UFREE, HRDY, HFREE, ACCFULL, ACCFREE, XIN = 22 /*2*/, NBAR = 24 };
-  static_assert(8 * NBAR + 8 + 48 <= 256 && NSB <= 4, "barrier block");
+  static_assert(8 * NBAR + 8 + 48 + (XIN16 ? 64 : 0) <= GE::BARS && NSB <= 4, "barrier block");
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
   uint8_t* bar_ptr = base_ptr + (bars - base);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 8 * NBAR);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   float* wsum = reinterpret_cast<float*>(bar_ptr + 8 * NBAR + 8);
   float* sEnd = wsum + 8;                                   // S_end of the last four chunks
-  float* sS = reinterpret_cast<float*>(bar_ptr + 256);      // [NSB][S | FACT: exp(m - S), m = smallest S of the token's 32 | FACT: the four m]
+  float* sM = sEnd + 4;                                     // XIN16: [NSB][4] smallest S of 32 tokens
+  float* sS = reinterpret_cast<float*>(bar_ptr + GE::BARS); // [NSB][S | FACT: exp(m - S), m = smallest S of the token's 32]
   float2* sfac = reinterpret_cast<float2*>(sS + NSB * GE::SLOT);    // (dt, exp(S_end - S)) of the step's rows
   float* sdt = sS + NSB * GE::SLOT;                                 // BIG: dt alone, the last kilobyte is not there
 
@@ -369,7 +371,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
           tmem_ld32(tg, r);
           if (FACT && cb < diag) {
             // every column is before every row: exp(S_t - S_s) = exp(S_t - m) exp(m - S_s), m as below where the factors are formed
-            const float rf = __expf(S_row - S[2 * L + cb]);
+            const float rf = __expf(S_row - (XIN16 ? sM[(c % NSB) * 4 + cb] : S[32 * cb + 31]));
 #pragma unroll
             for (int e4 = 0; e4 < 8; ++e4) {
               const float4 cf = *reinterpret_cast<const float4*>(S + L + 32 * cb + 4 * e4);
@@ -578,9 +580,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
               // m = the smallest S of the 32 columns, their last where a <= 0.  Where a is positive for a while (bf16 x comes with any a)
               // S can rise and fall by more than fp32's exponent inside a step: no factor exp(m - S_s) is above 1, and exp(S_t - m)
               // overflows only where an exponential of the row does.
-              const float m = warp_min(v[u]);
+              const float m = XIN16 ? warp_min(v[u]) : __shfl_sync(0xffffffffu, v[u], 31);
               S[L + q] = __expf(m - v[u]);
-              if (lane == 0) S[2 * L + q / 32] = m;
+              if (XIN16 && lane == 0) sM[(c % NSB) * 4 + q / 32] = m;
             }
             if (GE::BIG) sdt[q] = dtv[u]; else sfac[q] = make_float2(dtv[u], __expf(send - v[u]));
             if (q == NB * L - 1) sEnd[c & 3] = send;

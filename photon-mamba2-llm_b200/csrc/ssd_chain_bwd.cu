@@ -65,7 +65,7 @@ struct Geo {
   static constexpr int AHEAD = IN16 ? 0 : 2;             // fp32: pieces of x and of dY that a transform thread has in flight (bf16: the tiles are copied as they are)
   static constexpr int TILES = STAGE + XB * XBUF + HT;
   static constexpr int ROWS = 11 * L;                    // per-row sums: [2 groups] of W, e, f; W[s,s]; [4 quarters] column sums of W
-  static constexpr int SLOT = 3 * L + 4;                 // a step's [S | dt | column factors | what they refer to]
+  static constexpr int SLOT = 3 * L;                     // a step's [S | dt | column factors]
   static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 512 /*barriers, small sums*/ + (NSB * SLOT + 2 * ROWS) * 4 + 2 * AHEAD * XF_THREADS * 16;
 };
 
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
   const uint32_t b_s = base, c_s = b_s + GE::BT, hin_s = c_s + GE::BT, xbuf_s = base + GE::STAGE, dh_s = xbuf_s + XB * GE::XBUF, bars = dh_s + GE::HT;
   enum { FULL = 0, EMPTY, XRDY /*2*/, XFREE = XRDY + 2 /*2*/, SRDY = XFREE + 2 /*4*/, GFULL = SRDY + 4, MRDY, ACCFULL, ACCFREE, UFULL, UFREE, HRDY, HFREE,
          RRDY /*2*/, RFREE = RRDY + 2 /*2*/, XIN = RFREE + 2 /*2*/, NBAR = XIN + 2 };
-  static_assert(8 * NBAR + 16 + 80 <= 512 && NSB <= 4, "barrier block");
+  static_assert(8 * NBAR + 16 + 80 + 64 <= 512 && NSB <= 4, "barrier block");
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
   uint8_t* bar_ptr = base_ptr + (bars - base);
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bar_ptr + 8 * NBAR);
@@ -130,7 +130,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
   float* ddw = reinterpret_cast<float*>(bar_ptr + 8 * NBAR + 16);      // [2 steps][4 state warps] <dh, h>
   float* dDw = ddw + 8;                                                // [8 transform warps] <dY, x>
   float* sWend = dDw + 8;                                              // [4 transform warps] S of their last token
-  float* sS = reinterpret_cast<float*>(bar_ptr + 512);                 // [NSB] S, dt and column factor exp(S_t - m) of a step's tokens, m = the largest S of the token's 32 and of the token before them; the four m
+  float* sM = sWend + 4;                                               // IN16: [NSB][4] m of 32 tokens
+  float* sS = reinterpret_cast<float*>(bar_ptr + 512);                 // [NSB] S, dt and column factor exp(S_t - m) of a step's tokens, m = the largest S of the token's 32 and of the one before them
   float* sRows = sS + NSB * GE::SLOT;                                     // [2 steps] per-row sums
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
@@ -533,7 +534,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
             constexpr bool DIAG = decltype(diagonal)::value;
             float rf[4];
             if (!DIAG) {
-              const float m = S[3 * L + cb];
+              const float m = IN16 ? sM[(k % NSB) * 4 + cb] : S[32 * cb - 1];
 #pragma unroll
               for (int e = 0; e < 4; ++e) rf[e] = __expf(m - Sr[e]);
             }
@@ -651,9 +652,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       if (ok && tid < L) {
         // m = the largest S of the 32 columns and of the token before them, that token's where a <= 0: as in the forward, no factor
         // exp(S_t - m) is above 1, and exp(m - S_s) overflows only where an exponential of the row does
-        const float m = fmaxf(sWend[wx > 0 ? wx - 1 : 0], warp_max(sv));
+        float m = sWend[wx > 0 ? wx - 1 : 0];
+        if (IN16) m = fmaxf(m, warp_max(sv));
         S[2 * L + tid] = __expf(sv - m);
-        if (lane == 0) S[3 * L + wx] = m;
+        if (IN16 && lane == 0) sM[(k % NSB) * 4 + wx] = m;
       }
       asm volatile("bar.sync 4, %0;" ::"n"(256) : "memory");
       if (!ok) continue;
