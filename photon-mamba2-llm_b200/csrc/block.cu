@@ -596,10 +596,13 @@ pmb_status stack_bwd(cudaStream_t st, const Dims& d, int n_layers, const pmb_blo
     return PMB_OK;
   }
   // Dependent launches hide what a kernel does before its first load: a training step of 2 x 128 tokens takes 309 us with them, 372 without.
-  // Where one projection fills the machine a kernel that is placed early keeps the other stream's kernels off its SM: two-level step of
-  // 8 x 1024 tokens 17.1 ms with them, 16.3 without; 4 x 512 tokens 9.81 and 9.76.  (Where nothing runs beside it they stay up to two rounds of tiles, then
-  // the kernels are too long to notice: 8 x 2048 tokens 45.3 and 44.7 ms.)
-  const PdlPause pause(tiles256(d.M, d.J) > 74);
+  // But a kernel that is placed early holds its SMs while it waits, and a GEMM wants two whole ones to a tile: from some 60 tiles of a
+  // projection on, a recompute whose scan is chains, which want a whole SM each too, finds no room beside a waiting GEMM and the kernel in front
+  // of it.  What ordinary launches in here add to a training step of 12 layers, by tiles; d_model 256 to 768, sequences of 512 to 2048 tokens:
+  // fp32 18-40 -2.4 to +0.5 %, 52-60 +2 to +6, 72-80 -1.3 to +3.6, 104-140 -1.4 to +2, 144-156 -0.7 to -5.8, 208-416 -4.8 to +3;
+  // bf16 as chains 26-60 -3.2 to +3.8, 72-80 -1.8 to -10.2, 104-140 -1.9 to +3, 144-156 +1.9 to -7.7, 208-832 -1.1 to -5.8; bf16 chunk by chunk
+  // 18-20 -1 to -4.8, 72-80 +4 to +7, 144 -0.1, 208 -2.5.
+  const PdlPause pause(tiles256(d.M, d.J) > (!bf ? 74 : scan_by_chunks(d, true, true) ? 140 : 60));
   // events: ev[0], ev[1] = recompute into slot 0 / 1 finished;  ev[2], ev[3] = gradient kernels reading slot 0 / 1 finished
   cudaStream_t sr = rl->s;
   // The gradient kernels run on a high-priority internal stream (the caller's stream has the lowest priority a

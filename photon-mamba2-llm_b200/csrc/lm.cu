@@ -555,7 +555,10 @@ extern "C" pmb_status pmb_lm_step_device(pmb_lm* lm, void* stream, const int64_t
   const uint16_t* table16 = h16 ? lm->params16 + lm->off[0] : nullptr;
   const bool prs = lm->pairs != 0;
   const Weights16* w16 = (h16 || prs) ? lm->lw16.data() : nullptr;
-  const PdlPause pause(cdiv(M, 256) * cdiv(d.J, 256) > 148);      // (see stack_bwd)
+  // (See stack_bwd.  Where nothing runs beside it a step keeps them up to two rounds of tiles on 148 SMs; then the kernels are too long to notice and
+  // the head's second stream is kept from its SMs.  Ordinary launches throughout against those of the stack's backward alone: 144-156 tiles 0 to +4 %,
+  // 208-288 -0.6 to +2.4, 320-832 -0.7 to -1.8.)
+  const PdlPause pause(cdiv(M, 256) * cdiv(d.J, 256) > 296);
   // the fp32 masters may have been updated by the optimizer since the last step: refresh their pairs
   if (prs) { const SplitItem all{lm->params, lm->n_params, lm->params_hi, lm->params_lo}; PMB_TRY(split_pairs_flat(st, &all, 1)); }
   const Pair16 table_p{prs ? lm->params_hi + lm->off[0] : nullptr, prs ? lm->params_lo + lm->off[0] : nullptr, D};
