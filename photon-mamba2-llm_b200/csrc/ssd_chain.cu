@@ -111,7 +111,7 @@ struct Params {
   // (store_ops) x~ and xs as the kernel formed them.  bf16 x: store_ops leaves a copy of it.
   float *hprev, *yoff;
   int store_ops;
-  int first, nseg, per, div;                             // first chain of this launch; segments of a sequence, steps per segment, blocks per chain
+  int first, nseg, per;                                  // first chain of this launch (grid: chains x segments); segments of a sequence, steps per segment
   int late;                                              // needs nothing from the kernel before, which lets this one in after its own wait: waits when it is done
   int state_only;                                        // first of two passes over segments: only seg_h and seg_d are formed
   float *seg_h, *seg_d;                                  // (B*H-whole,nseg-1,N,P), (B*H-whole,nseg-1): state that a segment leaves when it starts from none, decay over it (nobody reads the last one's)
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   float* sdt = sS + NSB * GE::SLOT;                                 // BIG: dt alone, the last kilobyte is not there
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int bh = p.first + (int)blockIdx.x / p.div, seg = (int)blockIdx.x % p.div;
+  const int bh = p.first + (int)blockIdx.x, seg = (int)blockIdx.y;
   const int h = bh % p.H, bb = bh / p.H, g = h / p.hpg;
   const int i0 = seg * p.per, toff = i0 * L;               // first step and token of this CTA's segment
   const int n = min(p.per, p.nsteps - i0);
@@ -733,8 +733,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(UFREE));
     }
-    if (ok && p.state_only && nr == 0) p.seg_d[blockIdx.x] = __expf(stot);
-    float* const leave = p.state_only ? p.seg_h + (int64_t)blockIdx.x * NP : p.last && seg + 1 == p.nseg ? p.last + (int64_t)bh * NP : nullptr;
+    const int64_t row = (int64_t)blockIdx.x * gridDim.y + blockIdx.y;
+    if (ok && p.state_only && nr == 0) p.seg_d[row] = __expf(stot);
+    float* const leave = p.state_only ? p.seg_h + row * NP : p.last && seg + 1 == p.nseg ? p.last + (int64_t)bh * NP : nullptr;
     if (ok && leave && active) {
       float* dst = leave + (int64_t)nr * p.P;
 #pragma unroll
@@ -787,19 +788,19 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
   const unsigned cut = (unsigned)((chains - plan.whole) * plan.nseg);      // blocks of segments
   if (cut) { p.seg_h = a.seg; p.seg_d = a.seg + (size_t)cut * a.N * a.P; }
   PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>);
-  auto run = [&](unsigned blocks) { return launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>, blocks, NTHREADS, GE::SMEM, ms, p); };
+  auto run = [&](int count, int segments) { return launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>, dim3((unsigned)count, (unsigned)segments), NTHREADS, GE::SMEM, ms, p); };
   // the segments' states, the segments, and beside both the chains in one piece
   if (cut) {
     p.first = plan.whole; p.nseg = plan.nseg; p.per = plan.per;
-    p.state_only = 1; p.div = plan.nseg - 1;
-    PMB_TRY(run(cut / p.nseg * p.div));
-    p.state_only = 0; p.div = plan.nseg;
+    p.state_only = 1;
+    PMB_TRY(run(chains - plan.whole, plan.nseg - 1));
+    p.state_only = 0;
   }
   p.store_ops = keep != nullptr;
-  if (cut) PMB_TRY(run(cut));
+  if (cut) PMB_TRY(run(chains - plan.whole, plan.nseg));
   if (plan.whole) {
-    p.first = 0; p.nseg = p.div = 1; p.per = p.nsteps; p.late = cut > 0;
-    PMB_TRY(run((unsigned)plan.whole));
+    p.first = 0; p.nseg = 1; p.per = p.nsteps; p.late = cut > 0;
+    PMB_TRY(run(plan.whole, 1));
   }
   return PMB_OK;
 }

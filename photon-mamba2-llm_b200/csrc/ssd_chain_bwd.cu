@@ -84,7 +84,7 @@ struct Params {
   float* da;                                             // (B,T,H)
   uint16_t *raw_hi, *raw_lo; int64_t ld_raw; int raw_col;                  // dt mode: gradient before the softplus as a bf16 pair (raw_lo may be NULL)
   float* part; int64_t part_pitch;                       // dt mode: per (b, h) sums for dA, dD and d_dt_bias, `part_pitch` apart
-  int first, nseg, per, div;                             // first chain of this launch; segments of a sequence, steps per segment, blocks per chain
+  int first, nseg, per;                                  // first chain of this launch (grid: chains x segments); segments of a sequence, steps per segment
   int late;                                              // needs nothing from the kernel before, which lets this one in after its own wait: waits when it is done
   int rows, fill;                                        // rows of `part` per (b, h); of them a block writes its own, a chain in one piece all (zeros: no more than a warp has lanes)
   int state_only;                                        // first of two passes over segments: only seg_h and seg_d are formed
@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
   float* sRows = sS + NSB * GE::SLOT;                                     // [2 steps] per-row sums
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int bh = p.first + (int)blockIdx.x / p.div, seg = (int)blockIdx.x % p.div + p.nseg - p.div;
+  const int bh = p.first + (int)blockIdx.x, seg = (int)blockIdx.y + p.state_only;
   const int h = bh % p.H, bb = bh / p.H, g = h / p.hpg;
   const int n = min(p.per, p.nsteps - seg * p.per), last = seg * p.per + n - 1;      // steps of this CTA's segment, the last one of them
   const int64_t tokb = (int64_t)bb * p.T;
@@ -804,8 +804,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       if (lane == 0) mbar_arrive(bar(UFREE));
     }
     if (ok && p.state_only) {
-      if (nr == 0) p.seg_d[blockIdx.x] = __expf(stot);
-      float* dst = p.seg_h + (int64_t)blockIdx.x * NP + (int64_t)nr * p.P;
+      const int64_t row = (int64_t)blockIdx.x * gridDim.y + blockIdx.y;
+      if (nr == 0) p.seg_d[row] = __expf(stot);
+      float* dst = p.seg_h + row * NP + (int64_t)nr * p.P;
       if (active) {
 #pragma unroll
         for (int q = 0; q < PW / 4; ++q)
@@ -866,18 +867,18 @@ static pmb_status launch(cudaStream_t st, const ChainBwdArgs& a) {
   if (cut) { p.seg_h = a.seg; p.seg_d = a.seg + (size_t)cut * a.N * a.P; }
   p.rows = plan.nseg; p.fill = 1; p.part_pitch = (int64_t)chains * plan.nseg;
   PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_bwd_kernel<NI, ND, NK, IN16>);
-  auto run = [&](unsigned blocks) { return launch_pdl(st, ssd_chain_bwd_kernel<NI, ND, NK, IN16>, blocks, NTHREADS, GE::SMEM, ms, p); };
+  auto run = [&](int count, int segments) { return launch_pdl(st, ssd_chain_bwd_kernel<NI, ND, NK, IN16>, dim3((unsigned)count, (unsigned)segments), NTHREADS, GE::SMEM, ms, p); };
   // the segments' adjoints, the segments, and beside both the chains in one piece
   if (cut) {
     p.first = plan.whole; p.nseg = plan.nseg; p.per = plan.per;
-    p.state_only = 1; p.div = plan.nseg - 1;
-    PMB_TRY(run(cut / p.nseg * p.div));
-    p.state_only = 0; p.div = plan.nseg;
-    PMB_TRY(run(cut));
+    p.state_only = 1;
+    PMB_TRY(run(chains - plan.whole, plan.nseg - 1));
+    p.state_only = 0;
+    PMB_TRY(run(chains - plan.whole, plan.nseg));
   }
   if (plan.whole) {
-    p.first = 0; p.nseg = p.div = 1; p.per = n; p.late = cut > 0; p.fill = plan.nseg;
-    PMB_TRY(run((unsigned)plan.whole));
+    p.first = 0; p.nseg = 1; p.per = n; p.late = cut > 0; p.fill = plan.nseg;
+    PMB_TRY(run(plan.whole, 1));
   }
   return PMB_OK;
 }
