@@ -61,7 +61,7 @@ struct Geo {
   static constexpr int XT = NI * T128;                   // x~ (or dY)
   static constexpr int XBUF = 2 * XT + ND * T128;        // [x~ | dY | dY exp(S)]
   static constexpr int XB = ND == 1 ? 2 : 1;
-  static constexpr int NSB = XB + 2;
+  static constexpr int NSB = 4;                          // copies of S: see the transform warps
   static constexpr int AHEAD = IN16 ? 0 : 2;             // fp32: pieces of x and of dY that a transform thread has in flight (bf16: the tiles are copied as they are)
   static constexpr int TILES = STAGE + XB * XBUF + HT;
   static constexpr int ROWS = 11 * L;                    // per-row sums: [2 groups] of W, e, f; W[s,s]; [4 quarters] column sums of W
@@ -641,10 +641,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
     for (int k = 0; k < n; ++k) {
       const int xb = k % XB;
       float* S = sS + (k % NSB) * GE::SLOT;
-      if (ok && IN16) ok = all(wait(XIN + xb, (uint32_t)(k / XB), 128u));
-      else if (ok && k >= XB) ok = all(wait(XFREE + xb, (uint32_t)(k / XB - 1), 128u));
-      // (whoever reads the ring's old entry, of step k - NSB, has finished: the products of step k - XB, whose buffer was just freed, follow
-      // the draining of step k - XB - 1 and its row sums wait for nobody that is further behind)
+      if (IN16 && ok) ok = all(wait(XIN + xb, (uint32_t)(k / XB), 128u));
+      // fp32: S is formed ahead of the wait for the one buffer of x, whose transform is what every step waits for.  (Whoever reads the copy's old
+      // entry, of step k - 4, has finished: the buffer of step k - 2 has been waited for, by fp32 in the step before, by bf16's loads here.
+      // It is free when that step has been masked, for which the masks wait for the row sums of step k - 4, and when its product U
+      // is done, which waits for the state warps' end of step k - 3.)
       const float sv = s_next;
       if (ok && tid < L) { S[tid] = sv; S[L + tid] = d_next; }
       if (lane == 31 && tid < L) sWend[wx] = sv;
@@ -661,6 +662,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       if (!ok) continue;
       if (lane == 0) mbar_arrive(bar(SRDY + (k % NSB)));
       fetch_s(k + 1);
+      if (!IN16 && k >= XB && !(ok = all(wait(XFREE + xb, (uint32_t)(k / XB - 1), 128u)))) continue;
       uint32_t dst = xbuf_s + xb * GE::XBUF + place;
 #pragma unroll (IN16 ? 4 : 2)
       for (int it = 0; it < NIT; ++it, dst += RPI * 128) {
