@@ -300,42 +300,41 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       const int s = k % STG, xb = k % XB, rb = k % NB, c = k / NB;
       // acc2 = C h
       auto carried = [&]() -> bool {
-                if (!all(wait(FULL + s, (uint32_t)(k / STG), 4u) && wait(HRDY, (uint32_t)c, 8u) && (k == 0 || wait(ACCFREE, (uint32_t)(k - 1), 8u)))) return false;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (elect_one()) {
-                  const uint32_t c0 = desc_lo(ring_s + s * GE::STAGE + GE::BT, 16), h0 = desc_lo(h_s, T64);
-        #pragma unroll
-                  for (int kt = 0; kt < NK; ++kt)
-        #pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                      mma_split<NI, ND>(tA2, c0 + ((uint32_t)(kt * T128 + q * 32) >> 4), (NK * T128) >> 4, h0 + ((uint32_t)(kt * T64 + q * 2048) >> 4), (NK * T64) >> 4, dh, id_v,
-                            (kt | q) ? 1u : 0u);
-                  umma_commit(bar(ACCFULL));
+        if (!all(wait(FULL + s, (uint32_t)(k / STG), 4u) && wait(HRDY, (uint32_t)c, 8u) && (k == 0 || wait(ACCFREE, (uint32_t)(k - 1), 8u)))) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (elect_one()) {
+          const uint32_t c0 = desc_lo(ring_s + s * GE::STAGE + GE::BT, 16), h0 = desc_lo(h_s, T64);
+#pragma unroll
+          for (int kt = 0; kt < NK; ++kt)
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              mma_split<NI, ND>(tA2, c0 + ((uint32_t)(kt * T128 + q * 32) >> 4), (NK * T128) >> 4, h0 + ((uint32_t)(kt * T64 + q * 2048) >> 4), (NK * T64) >> 4, dh, id_v,
+                                (kt | q) ? 1u : 0u);
+          umma_commit(bar(ACCFULL));
           if (XB == 2) umma_commit(bar(EMPTY + s));
-                  if (rb == NB - 1 || k + 1 == n) umma_commit(bar(HFREE));
-                }
-                __syncwarp();
+          if (rb == NB - 1 || k + 1 == n) umma_commit(bar(HFREE));
+        }
+        __syncwarp();
         return true;
       };
       // U (+)= B^T xs: the chunk's contribution to the state
       auto update = [&]() -> bool {
-                    if (!all(wait(FULL + s, (uint32_t)(k / STG), 4u) && wait(XRDY + xb, (uint32_t)(k / XB), 4u) &&
-                             (rb > 0 || c == 0 || wait(UFREE, (uint32_t)(c - 1), 4u)))) return false;
-              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              if (elect_one()) {
-                // (M = 128 over one or two 64-wide blocks of d_state; with one block the second reads the tile behind it and
-                // its rows of U are never looked at)
-                const uint32_t b0 = desc_lo(ring_s + s * GE::STAGE, T128), xs0 = desc_lo(xbuf_s + xb * GE::XBUF + GE::XT, T128);
-        #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                  const uint32_t o = (uint32_t)(q * 2048) >> 4;
-                  mma_split<NI, ND>(tU, b0 + o, (NK * T128) >> 4, xs0 + o, T128 >> 4, dh, id_u, (q | rb) ? 1u : 0u);
-                }
-                if (rb == NB - 1 || k + 1 == n) umma_commit(bar(UFULL));
-                umma_commit(bar(XFREE + xb));
+        if (!all(wait(FULL + s, (uint32_t)(k / STG), 4u) && wait(XRDY + xb, (uint32_t)(k / XB), 4u) && (rb > 0 || c == 0 || wait(UFREE, (uint32_t)(c - 1), 4u)))) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (elect_one()) {
+          // (M = 128 over one or two 64-wide blocks of d_state; with one block the second reads the tile behind it and
+          // its rows of U are never looked at)
+          const uint32_t b0 = desc_lo(ring_s + s * GE::STAGE, T128), xs0 = desc_lo(xbuf_s + xb * GE::XBUF + GE::XT, T128);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const uint32_t o = (uint32_t)(q * 2048) >> 4;
+            mma_split<NI, ND>(tU, b0 + o, (NK * T128) >> 4, xs0 + o, T128 >> 4, dh, id_u, (q | rb) ? 1u : 0u);
+          }
+          if (rb == NB - 1 || k + 1 == n) umma_commit(bar(UFULL));
+          umma_commit(bar(XFREE + xb));
           if (XB == 1 || p.state_only) umma_commit(bar(EMPTY + s));
-              }
-              __syncwarp();
+        }
+        __syncwarp();
         return true;
       };
       // (two buffers of x: xs has been there for a while, and the state's chain does not wait for C h; one: xs is being formed)

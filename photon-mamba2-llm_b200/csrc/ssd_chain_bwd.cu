@@ -269,38 +269,38 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
         } else {
           // the state's: B dh and C h, and U
           auto carried = [&]() -> bool {
-                        if (!all(wait(HRDY, (uint32_t)k, 8u) && (k == 0 || wait(ACCFREE, (uint32_t)(k - 1), 8u)))) return false;
-                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        if (elect_one()) {
-                          const uint32_t b0 = desc_lo(b_s, 16), c0 = desc_lo(c_s, 16), d0 = desc_lo(dh_s, T64), h0 = desc_lo(hin_s, T64);
-            #pragma unroll
-                          for (int kt = 0; kt < NK; ++kt)
-            #pragma unroll
-                            for (int q = 0; q < 4; ++q) {
-                              const uint32_t oa = (uint32_t)(kt * T128 + q * 32) >> 4, ob = (uint32_t)(kt * T64 + q * 2048) >> 4;
-                              mma_split<NI, ND>(tA2, b0 + oa, BS, d0 + ob, HS, dhi, id_v, (kt | q) ? 1u : 0u);
-                              mma_split<NI, ND>(tA3, c0 + oa, BS, h0 + ob, HS, dhi, id_v, (kt | q) ? 1u : 0u);
-                            }
-                          umma_commit(bar(ACCFULL));
-                          umma_commit(bar(HFREE));
+            if (!all(wait(HRDY, (uint32_t)k, 8u) && (k == 0 || wait(ACCFREE, (uint32_t)(k - 1), 8u)))) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (elect_one()) {
+              const uint32_t b0 = desc_lo(b_s, 16), c0 = desc_lo(c_s, 16), d0 = desc_lo(dh_s, T64), h0 = desc_lo(hin_s, T64);
+#pragma unroll
+              for (int kt = 0; kt < NK; ++kt)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                  const uint32_t oa = (uint32_t)(kt * T128 + q * 32) >> 4, ob = (uint32_t)(kt * T64 + q * 2048) >> 4;
+                  mma_split<NI, ND>(tA2, b0 + oa, BS, d0 + ob, HS, dhi, id_v, (kt | q) ? 1u : 0u);
+                  mma_split<NI, ND>(tA3, c0 + oa, BS, h0 + ob, HS, dhi, id_v, (kt | q) ? 1u : 0u);
+                }
+              umma_commit(bar(ACCFULL));
+              umma_commit(bar(HFREE));
               if (XB == 2) umma_commit(bar(EMPTY));
-                        }
-                        __syncwarp();
+            }
+            __syncwarp();
             return true;
           };
           auto update = [&]() -> bool {
-                      if (!(xready() && all(k == 0 || wait(UFREE, (uint32_t)(k - 1), 4u)))) return false;
-                      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                      // U = C^T (exp(S) dY): the step's contribution to the state's adjoint (with one 64-wide block of d_state the second half
-                      // of M reads the tile behind it and its rows of U are never looked at)
-                      if (elect_one()) {
-                        const uint32_t cm = desc_lo(c_s, T128), y0 = desc_lo(dys_s, T128);
-            #pragma unroll
-                        for (int q = 0; q < 8; ++q) mma_split<NI, ND>(tU, cm + ((uint32_t)(q * 2048) >> 4), BS, y0 + ((uint32_t)(q * 2048) >> 4), XS, dhi, id_u, q ? 1u : 0u);
-                        umma_commit(bar(UFULL)); umma_commit(bar(XFREE + xb));
+            if (!(xready() && all(k == 0 || wait(UFREE, (uint32_t)(k - 1), 4u)))) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // U = C^T (exp(S) dY): the step's contribution to the state's adjoint (with one 64-wide block of d_state the second half
+            // of M reads the tile behind it and its rows of U are never looked at)
+            if (elect_one()) {
+              const uint32_t cm = desc_lo(c_s, T128), y0 = desc_lo(dys_s, T128);
+#pragma unroll
+              for (int q = 0; q < 8; ++q) mma_split<NI, ND>(tU, cm + ((uint32_t)(q * 2048) >> 4), BS, y0 + ((uint32_t)(q * 2048) >> 4), XS, dhi, id_u, q ? 1u : 0u);
+              umma_commit(bar(UFULL)); umma_commit(bar(XFREE + xb));
               if (XB == 1 || p.state_only) umma_commit(bar(EMPTY));
-                      }
-                      __syncwarp();
+            }
+            __syncwarp();
             return true;
           };
           // (two buffers: exp(S) dY has been there for a while, and the state's chain does not wait for the draining; one: it is being formed)
@@ -396,7 +396,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
     const bool dtm = p.dt != nullptr;
     const float dv = p.D ? p.D[h] : 0.0f;
     const int er = quarter * 32 + (lane >> 2), ec = (lane & 3) * 2, cw = 32 * grp;
-    constexpr int PPR = 2;                                  // output pieces of 16 rows
     // ---------------- output of a step: half of the columns, in pieces of 16 rows x 16 columns, fragments of 16 x 8 (whole 32-byte
     // sectors per store) ----------------
     auto output = [&](int k) -> bool {
@@ -404,8 +403,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       const float* S = sS + (k % NSB) * GE::SLOT;
       const int xb = k % XB, i = last - k;
       const uint32_t xt_s = xbuf_s + xb * GE::XBUF, dy_s = xt_s + GE::XT;
-      auto fetch = [&](int pc, float2 (&xo)[2][2], float2 (&yo)[2][2]) {
-        const int rh = pc / PPR, c16 = pc % PPR;
+      auto fetch = [&](int rh, int c16, float2 (&xo)[2][2], float2 (&yo)[2][2]) {
 #pragma unroll
         for (int q = 0; q < 2; ++q)
 #pragma unroll
@@ -423,21 +421,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       const float send = S[L - 1];
       float fx[2], dtr[2], es[2], fs[2];
 #pragma unroll 1
-      for (int pc0 = 0; pc0 < 2 * PPR; pc0 += 2) {
-        if (pc0 % PPR == 0) {
+      for (int rh = 0; rh < 2; ++rh) {                      // 16 rows, in two pieces
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int row = er + 16 * (pc0 / PPR) + 8 * e;
-            fx[e] = __expf(send - S[row]);
-            dtr[e] = dtm ? S[L + row] : 1.0f;
-            es[e] = fs[e] = 0.0f;
-          }
+        for (int e = 0; e < 2; ++e) {
+          const int row = er + 16 * rh + 8 * e;
+          fx[e] = __expf(send - S[row]);
+          dtr[e] = dtm ? S[L + row] : 1.0f;
+          es[e] = fs[e] = 0.0f;
         }
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int pc = pc0 + u, rh = pc / PPR, c16 = pc % PPR;
+        for (int c16 = 0; c16 < 2; ++c16) {
           float2 xn[2][2], yn[2][2];                        // [8-column group][row, row + 8]
-          fetch(pc, xn, yn);
+          fetch(rh, c16, xn, yn);
           uint32_t a1[8], a2[8], a3[8];
           const uint32_t ta = lane_addr + ((uint32_t)(16 * rh) << 16) + (uint32_t)(cw + 16 * c16);
           tmem_ld16x256_x2(tA1 + ta, a1);
@@ -457,7 +452,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
               fs[e] = fmaf(__uint_as_float(a3[r]), yv.x, fmaf(__uint_as_float(a3[r + 1]), yv.y, fs[e]));
               o[q][e] = make_float2(fmaf(d0, dtr[e], dv * yv.x), fmaf(d1, dtr[e], dv * yv.y));
             }
-          if (pc == 2 * PPR - 1) {
+          if (rh == 1 && c16 == 1) {
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) { mbar_arrive(bar(ACCFREE)); mbar_arrive(bar(XFREE + xb)); }
@@ -483,17 +478,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
             }
           }
         }
-        if (pc0 % PPR == PPR - 2) {
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
+        for (int e = 0; e < 2; ++e) {
 #pragma unroll
-            for (int w = 1; w < 4; w <<= 1) {               // the quad of lanes that shares a row
-              es[e] += __shfl_xor_sync(0xffffffffu, es[e], w);
-              fs[e] += __shfl_xor_sync(0xffffffffu, fs[e], w);
-            }
-            const int row = er + 16 * (pc0 / PPR) + 8 * e;
-            if ((lane & 3) == 0) { R[(2 + grp) * L + row] = es[e]; R[(4 + grp) * L + row] = fs[e]; }
+          for (int w = 1; w < 4; w <<= 1) {                 // the quad of lanes that shares a row
+            es[e] += __shfl_xor_sync(0xffffffffu, es[e], w);
+            fs[e] += __shfl_xor_sync(0xffffffffu, fs[e], w);
           }
+          const int row = er + 16 * rh + 8 * e;
+          if ((lane & 3) == 0) { R[(2 + grp) * L + row] = es[e]; R[(4 + grp) * L + row] = fs[e]; }
         }
       }
       __syncwarp();
@@ -608,16 +601,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
     // barrier; rows past the end and columns past d_head arrive as zeros)
     const uint32_t ring = smem_u32(sRows + 2 * GE::ROWS) + (uint32_t)tid * 16u;
     constexpr uint32_t SLOT = 2 * XF_THREADS * 16;          // [x | dY]
-    constexpr int esz = 4;
-    const char* xsrc = reinterpret_cast<const char*>(p.x) + (int64_t)(h * p.P + (jcol ? EPL * j : 0)) * esz;
-    const char* ysrc = reinterpret_cast<const char*>(p.dy) + (int64_t)(h * p.P + (jcol ? EPL * j : 0)) * esz;
+    const char* xsrc = reinterpret_cast<const char*>(p.x) + (int64_t)(h * p.P + (jcol ? EPL * j : 0)) * 4;
+    const char* ysrc = reinterpret_cast<const char*>(p.dy) + (int64_t)(h * p.P + (jcol ? EPL * j : 0)) * 4;
     int rrow = last * L + r0, rit = 0;                      // row and pass of the next piece to request; rows are walked up inside a step
     auto request = [&](uint32_t slot) {
       if (rrow >= (last - n + 1) * L) {
         const bool in = rrow < p.T && jcol;
         const int64_t tk = tokb + (rrow < p.T ? rrow : p.T - 1);      // (the address stays inside the tensor)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + slot), "l"(xsrc + tk * (p.ldx * esz)), "r"(in ? 16 : 0) : "memory");
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + slot + XF_THREADS * 16), "l"(ysrc + tk * (p.lddy * esz)), "r"(in ? 16 : 0) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + slot), "l"(xsrc + tk * (p.ldx * 4)), "r"(in ? 16 : 0) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ring + slot + XF_THREADS * 16), "l"(ysrc + tk * (p.lddy * 4)), "r"(in ? 16 : 0) : "memory");
         rrow += RPI;
         if (++rit == NIT) { rit = 0; rrow -= 2 * L; }
       }
@@ -631,9 +623,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       s_next = Sg[t < p.T ? t : p.T - 1];                   // (a = 0 past the end)
       if (dtm) d_next = t < p.T ? p.dt[(tokb + t) * p.H + h] : 0.0f;
     };
-    if (!IN16)
+    if (!IN16) {
 #pragma unroll 1
-    for (int q = 0; q < AHEAD; ++q) request((uint32_t)q * SLOT);
+      for (int q = 0; q < AHEAD; ++q) request((uint32_t)q * SLOT);
+    }
     fetch_s(0);
     uint32_t slot = 0;
     float dD = 0.0f;
@@ -667,11 +660,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
 #pragma unroll (IN16 ? 4 : 2)
       for (int it = 0; it < NIT; ++it, dst += RPI * 128) {
         uint4 xq = make_uint4(0u, 0u, 0u, 0u), yq;
-        if (IN16) asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(yq.x), "=r"(yq.y), "=r"(yq.z), "=r"(yq.w) : "r"(dst + GE::XT));
-        else {
-        asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD > 0 ? AHEAD - 1 : 0) : "memory");
-        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(xq.x), "=r"(xq.y), "=r"(xq.z), "=r"(xq.w) : "r"(ring + slot) : "memory");
-        asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(yq.x), "=r"(yq.y), "=r"(yq.z), "=r"(yq.w) : "r"(ring + slot + XF_THREADS * 16) : "memory");
+        if (IN16) {
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(yq.x), "=r"(yq.y), "=r"(yq.z), "=r"(yq.w) : "r"(dst + GE::XT));
+        } else {
+          asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD > 0 ? AHEAD - 1 : 0) : "memory");
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(xq.x), "=r"(xq.y), "=r"(xq.z), "=r"(xq.w) : "r"(ring + slot) : "memory");
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(yq.x), "=r"(yq.y), "=r"(yq.z), "=r"(yq.w) : "r"(ring + slot + XF_THREADS * 16) : "memory");
         }
         const int row = it * RPI + r0;
         const float f = __expf(S[row]);
@@ -741,50 +735,50 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
     for (int k = 0; k < n && ok; ++k) {
       const int i = last - k;
       if (!p.state_only) {
-      if (k > 0) ok = all(wait(HFREE, (uint32_t)(k - 1), 256u));
-      if (!ok) break;
-      const int64_t so = (((int64_t)bb * p.nsteps + i) * p.H + h) * NP + (int64_t)nr * p.P;
-      if (tile) {
+        if (k > 0) ok = all(wait(HFREE, (uint32_t)(k - 1), 256u));
+        if (!ok) break;
+        const int64_t so = (((int64_t)bb * p.nsteps + i) * p.H + h) * NP + (int64_t)nr * p.P;
+        if (tile) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {                       // eight 16-byte chunks of the row
-          uint32_t hi[4], lo[4] = {0u, 0u, 0u, 0u};
+          for (int c = 0; c < 8; ++c) {                       // eight 16-byte chunks of the row
+            uint32_t hi[4], lo[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
-          for (int e = 0; e < 4; ++e) split2(hv[8 * c + 2 * e], hv[8 * c + 2 * e + 1], hi[e], lo[e], ND == 2);
-          const uint32_t a = dh_s + (uint32_t)(nr * 128 + ((c ^ (nr & 7)) << 4));
-          st_shared_v4(a, hi[0], hi[1], hi[2], hi[3]);
-          if (ND == 2) st_shared_v4(a + NK * T64, lo[0], lo[1], lo[2], lo[3]);
-          if (active && 8 * c < p.P) {
-            *reinterpret_cast<uint4*>(p.dh_hi + so + 8 * c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            if (ND == 2) *reinterpret_cast<uint4*>(p.dh_lo + so + 8 * c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            for (int e = 0; e < 4; ++e) split2(hv[8 * c + 2 * e], hv[8 * c + 2 * e + 1], hi[e], lo[e], ND == 2);
+            const uint32_t a = dh_s + (uint32_t)(nr * 128 + ((c ^ (nr & 7)) << 4));
+            st_shared_v4(a, hi[0], hi[1], hi[2], hi[3]);
+            if (ND == 2) st_shared_v4(a + NK * T64, lo[0], lo[1], lo[2], lo[3]);
+            if (active && 8 * c < p.P) {
+              *reinterpret_cast<uint4*>(p.dh_hi + so + 8 * c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+              if (ND == 2) *reinterpret_cast<uint4*>(p.dh_lo + so + 8 * c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            }
           }
         }
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar(HRDY));
-      // <dh, h>
-      ok = all(wait(FULL, (uint32_t)k, 512u) && (k < 2 || wait(RFREE + (k & 1), (uint32_t)((k >> 1) - 1), 512u)));
-      if (!ok) break;
-      float dot = 0.0f;
-      if (active) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(HRDY));
+        // <dh, h>
+        ok = all(wait(FULL, (uint32_t)k, 512u) && (k < 2 || wait(RFREE + (k & 1), (uint32_t)((k >> 1) - 1), 512u)));
+        if (!ok) break;
+        float dot = 0.0f;
+        if (active) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const uint32_t a = hin_s + (uint32_t)(nr * 128 + ((c ^ (nr & 7)) << 4));
-          uint32_t v[4];
+          for (int c = 0; c < 8; ++c) {
+            const uint32_t a = hin_s + (uint32_t)(nr * 128 + ((c ^ (nr & 7)) << 4));
+            uint32_t v[4];
 #pragma unroll
-          for (int sp = 0; sp < ND; ++sp) {
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a + sp * NK * T64) : "memory");
+            for (int sp = 0; sp < ND; ++sp) {
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(a + sp * NK * T64) : "memory");
 #pragma unroll
-            for (int e = 0; e < 4; ++e) { const float2 u = bf2(v[e]); dot = fmaf(u.x, hv[8 * c + 2 * e], fmaf(u.y, hv[8 * c + 2 * e + 1], dot)); }
+              for (int e = 0; e < 4; ++e) { const float2 u = bf2(v[e]); dot = fmaf(u.x, hv[8 * c + 2 * e], fmaf(u.y, hv[8 * c + 2 * e + 1], dot)); }
+            }
           }
         }
-      }
-      dot = warp_sum(dot);
-      if (lane == 0) {
-        ddw[(k & 1) * 4 + quarter] = dot;
-        mbar_arrive(bar(RRDY + (k & 1)));
-        mbar_arrive(bar(EMPTY));
-      }
+        dot = warp_sum(dot);
+        if (lane == 0) {
+          ddw[(k & 1) * 4 + quarter] = dot;
+          mbar_arrive(bar(RRDY + (k & 1)));
+          mbar_arrive(bar(EMPTY));
+        }
       }
       ok = all(wait(SRDY + (k % NSB), (uint32_t)(k / NSB), 512u) && wait(UFULL, (uint32_t)k, 512u));
       if (!ok) break;
