@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       float* S = sS + (c % NSB) * GE::SLOT;
       if (rb == 0) {
         // S of the chunk.  A warp that gave up keeps reaching the named barriers: it skips the work, not the barrier.
-        float dtv[TPT], v[TPT];
+        float dtv[TPT], v[TPT], least[TPT];
 #pragma unroll
         for (int u = 0; u < TPT; ++u) {
           const bool in = toff + c * NB * L + u * XF_THREADS + tid < p.T;
@@ -561,6 +561,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
 #pragma unroll
           for (int o = 1; o < 32; o <<= 1) { const float w = __shfl_up_sync(0xffffffffu, v[u], o); if (lane >= o) v[u] += w; }
           if (lane == 31 && tid < NB * L) wsum[u * XFW + wx] = v[u];
+          if (FACT && XIN16) least[u] = warp_min(v[u]);     // (on its way while the warps meet)
         }
         asm volatile("bar.sync 4, %0;" ::"n"(XF_THREADS) : "memory");
         if (tid < NB * L) {
@@ -579,7 +580,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
               // m = the smallest S of the 32 columns, their last where a <= 0.  Where a is positive for a while (bf16 x comes with any a)
               // S can rise and fall by more than fp32's exponent inside a step: no factor exp(m - S_s) is above 1, and exp(S_t - m)
               // overflows only where an exponential of the row does.
-              const float m = XIN16 ? warp_min(v[u]) : __shfl_sync(0xffffffffu, v[u], 31);
+              const float m = XIN16 ? least[u] + off[u] : __shfl_sync(0xffffffffu, v[u], 31);
               S[L + q] = __expf(m - v[u]);
               if (XIN16 && lane == 0) sM[(c % NSB) * 4 + q / 32] = m;
             }

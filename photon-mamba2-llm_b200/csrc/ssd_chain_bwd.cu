@@ -642,12 +642,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       const float sv = s_next;
       if (ok && tid < L) { S[tid] = sv; S[L + tid] = d_next; }
       if (lane == 31 && tid < L) sWend[wx] = sv;
+      const float most = IN16 && tid < L ? warp_max(sv) : sv;       // (on its way while the warps meet)
       asm volatile("bar.sync 4, %0;" ::"n"(256) : "memory");        // (a warp that gave up keeps reaching the named barriers)
       if (ok && tid < L) {
         // m = the largest S of the 32 columns and of the token before them, that token's where a <= 0: as in the forward, no factor
         // exp(S_t - m) is above 1, and exp(m - S_s) overflows only where an exponential of the row does
         float m = sWend[wx > 0 ? wx - 1 : 0];
-        if (IN16) m = fmaxf(m, warp_max(sv));
+        if (IN16) m = fmaxf(m, most);
         S[2 * L + tid] = __expf(sv - m);
         if (IN16 && lane == 0) sM[(k % NSB) * 4 + wx] = m;
       }
