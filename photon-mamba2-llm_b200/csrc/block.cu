@@ -87,8 +87,8 @@ static size_t slab_floats(const Dims& d) {
 // 128 at 64 x 64, keep the FMA contractions in fp32 outside of a model.  Theirs is not the better result: they form d(a_log) and d(dt_bias) as
 // <dY, y - D x> - <x~, dx~>, 1e-4 of their norm from fp64 on unit-size inputs of 200 tokens and 2e-4 to 8e-4 at 1000 to 1337 (the chain kernels'
 // sums 1e-5 to 2.5e-5; all other gradients are equally far off; for smaller inputs see outweighed in ssd.cu), nor the faster one (forward and
-// backward of 2 x 1337 tokens, 24 heads of 64 x 64: 2395 us, 514 as chains; a stack of five on 2 x 740: 7.2 ms, 1.9).  They stay because those
-// two gradients of a call would move by that much, more than fp32 results are expected to between two builds (2e-4).
+// backward of 2 x 1337 tokens, 24 heads of 64 x 64: 2395 us, 514 as chains; a stack of five on 2 x 740: 7.2 ms, 1.9).  That they stay is a choice
+// and no bound: fp32 results are held to 2e-4 between two builds, and those two gradients of a call would move by up to four times that, towards fp64.
 static bool block_uses_chain_bwd(const Dims& d, bool bf16) {
   const bool dims = bf16 ? !ssd_plain16_shape(d.P, d.N, d.Q) && d.D % 8 == 0 && d.J % 8 == 0 && d.I % 8 == 0 : block_uses_pairs(d);
   const bool close = bf16 || d.in_model || ssd_fused_supported(d.P, d.N, d.Q) || d.Q <= (d.P >= 64 ? 256 : 64);
@@ -194,7 +194,7 @@ static ChainArgs chain_inputs(const Dims& d, const pmb_block_params& p, const fl
 }
 
 // bf16-storage blocks on whole chunks: plain bf16 operands, and few long sequences scanned chunk by chunk instead of as chains, which are
-// not cut into segments here (a chain's S, state and xs go by chunks of two steps where the chunk has them).  What a chain's steps take, one
+// not cut into segments here (that is built for S and states by steps, not by chunks of two, and would round other sums).  What a chain's steps take, one
 // after the other, beyond a fixed cost, against the chunk-by-chunk kernels' time per step of a head; where a backward follows, the chain also
 // writes what that reads.  Fitted to 130 shapes of 8 to 32 heads, 512 to 8192 tokens: the slower side is taken by at most 1.3 % of a block's
 // forward and 0.6 % of its backward.  us, chains / chunk by chunk: forward 1 x 1024 tokens, 8 heads 53 / 46, 32 heads 70 / 75; 1 x 2048,

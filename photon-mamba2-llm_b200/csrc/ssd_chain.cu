@@ -18,21 +18,21 @@
 // warp 0 = TMA loads (B, C, bf16 x), 1 = products of the masked tile (G one item ahead, M x~), 2 = products of the state (C h, U), 3 = TMA
 // stores, 4..11 = two mask groups of four warps, then twelve warps of output and transform (eight and four; on fp32 pairs, whose
 // transform rounds every element twice, four and eight), 24..27 = state.
-// What bounds it: no pipe and no memory level.  A step takes 9100 warp instructions at d_state 128 on plain operands, issued in 41 % of the
+// What bounds it: no pipe and no memory level.  A step takes 8000 warp instructions at d_state 128 on plain operands, issued in 41 % of the
 // cycles; every role is a chain of TMEM loads, shared memory and arithmetic with two warps of it on a scheduler.  What shaped the roles are
 // clocks read inside a step of 16 x 8192 tokens, 32 heads of 128 x 64, bf16 (927 us when masking and output were one role and one warp issued
-// all products, 700 now):
+// all products, 720 now):
 //  - the products are issued by two warps: with one, its waits and the issue took 5000 of a step's 5200 clocks.  The warp index comes from a
 //    shuffle, so that the roles' branches and the descriptors are uniform to the compiler (742 -> 711 us, this kernel alone);
 //  - B and C are given back before the masked product waits for the mask, so that the next tiles (2200 clocks) land while it is masked;
 //  - bf16 x is the operand x~ as it is and comes by TMA: copied by the transform warps, their few pieces in flight took 4200 clocks a step;
 //  - a and dt are requested two chunks ahead (a head's tokens are a line apart), and below the diagonal the masked tile takes one
-//    exponential per row and block of 32 columns instead of one per element (not where M is rounded for a stream of bf16 values: those
-//    results are what they were);
-//  - the kernel's 63 KB are about what the instruction cache holds for seven roles: an early return and a few selects by block, 72 KB, cost 8 %.
-// Measured at 24 heads of 64 x 64: 23.4 us for 4 x 512 tokens on pairs (23.9 before the above), 141 us for 8 x 2048 on plain operands in chunks
-// of 256 with all that a chunk-by-chunk backward reads (188), 31 us (two launches over segments) for 1 x 1337 on pairs.  Every mbarrier wait is
-// bounded; on expiry the CTA raises the status
+//    exponential per row and block of 32 columns instead of one per element (not where M is rounded for a stream of bf16 values, see FACT);
+//  - the kernel's 63 KB are about what the instruction cache holds for seven roles: an early return and a few selects by block, 72 KB, cost 8 %;
+//  - the segment is the grid's y and not a remainder that stays in a register: on pairs its spills cost 10 % (24.6 -> 22.2 us at 4 x 512).
+// Measured at 24 heads of 64 x 64: 22 us for 4 x 512 tokens on pairs, 25 with what a backward reads (23.9 and 26 before the above); 8 x 2048 on
+// plain operands in chunks of 256, 119 us, and 166 with all that a chunk-by-chunk backward reads (their mean 188); 31 us (two launches over
+// segments) for 1 x 1337 on pairs.  Every mbarrier wait is bounded; on expiry the CTA raises the status
 // word, every role stops issuing work, copies in flight are waited for (bounded) and TMEM is freed on the way out.
 #include <cuda_bf16.h>
 #include <mutex>
@@ -86,8 +86,9 @@ struct Geo {
   static constexpr int AHEAD = BIG || XIN16 ? 0 : ND == 2 ? 3 : 16;
   // (BIG: no room for column factors and half of the alignment slack; shared memory starts 1024-byte aligned where nothing static
   // precedes it, and the kernel checks)
-  // the masked tile by factors of blocks instead of an exponential per element: not where the rounding of M to bf16 is part of a stream
-  // of bf16 values (the storage blocks on plain operands: each flipped rounding would grow through the layers behind it)
+  // The masked tile by factors of blocks instead of an exponential per element.  Not for storage blocks on plain operands, whose M is rounded to
+  // bf16 in a stream of bf16 values: a flipped rounding grows through the layers behind it, so that the gradients of two builds would differ
+  // by as much as bf16 storage itself puts them off (2e-2).  That is a choice for results that repeat; neither form is nearer to fp64.
   static constexpr bool FACT = NB == 1 && !BIG && (ND == 2 || XIN16);
   static constexpr int BARS = XIN16 ? 320 : 256;         // bytes of barriers and small sums
   static constexpr int SLOT = (BIG ? 1 : 2) * L, SLACK = BIG ? 512 : 1024;    // floats per copy of S: [S | column factors]

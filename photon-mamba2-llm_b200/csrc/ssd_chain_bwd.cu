@@ -20,13 +20,13 @@
 // per-head sums), 3 = products of the state (B dh, C h, U) and TMA stores of the operands x~ and dY that the sums over heads read, 4..11 = two
 // mask groups of four warps, then the output of the same step, 12..19 = transform (x -> x~, dY -> dY and dY exp(S), into shared memory; bf16
 // x and dY are operands as they are), 20..23 = state.
-// What bounds it: instructions and their chains, 16800 warp instructions a step at d_state 128, issued in 43 % of the cycles.  On plain
+// What bounds it: instructions and their chains, 15000 warp instructions a step at d_state 128, issued in 44 % of the cycles.  On plain
 // operands mask (4100 clocks), MT dY and output (2300) follow one another; on pairs, whose one buffer of x~ and dY has to be drained first, the
 // transform (6500) comes on top.  Warps of their own for the output (28 of 72 registers) were no faster: 1317 us against 1271 for
 // 16 x 8192 tokens, 32 heads of 128 x 64 (1412 with one MMA warp, sums by 16 shuffles per 16 columns and an exponential per element), nor x and dY
 // prefetched into registers (50 us for 4 x 512 tokens, 24 heads of 64 x 64, on pairs) or read again by the output (49).
-// Measured at 24 heads of 64 x 64 on pairs: 43 us for 4 x 512 tokens (the d(states) product, reverse pass, masked product and row
-// kernel it replaces: 118 us), 31 us for 2 x 384, 76 us for 2 x 1000 (1.7 ms of FMA contractions with ssd_heads.cu's share).
+// Measured at 24 heads of 64 x 64 on pairs: 45 us for 4 x 512 tokens (the d(states) product, reverse pass, masked product and row
+// kernel it replaces: 118 us), 31 us for 2 x 384, 53 us in segments for 2 x 1000 (1.7 ms of FMA contractions with ssd_heads.cu's share).
 // Every mbarrier wait is bounded, as in the forward.
 #include <cuda_bf16.h>
 #include <type_traits>

@@ -10,11 +10,11 @@
 //
 // warp 0 = TMA, 1 = MMA issuer, 2 = S of the heads, 4..11 = dG (64 columns per thread), 12..15 = dC, 16..19 = dB (64 columns per
 // thread).  Two or three operand stages, two sets of accumulators: the products of the next head run under the sums of this one.
-// What bounds it: latency.  No pipe or memory level is near its limit at 32 heads of 128 x 64 (issue slots 40 %, DRAM 44 %, exponentials
-// 11 %); warps wait for TMEM loads, each of which is followed at once by its wait, with five warps to a scheduler.
+// What bounds it: latency.  No pipe or memory level is near its limit at 32 heads of 128 x 64 (issue slots 46 %, DRAM 51 %, exponentials
+// 16 %); warps wait for TMEM loads, each of which is followed at once by its wait, with five warps to a scheduler.
 // Measured at 24 heads of 64 x 64 on pairs, 4 x 512 tokens: 18 us + 3 us for the sum of the shares; the three contractions and their
 // sums that it replaces took 45 us and read copies of dY and x~ scaled by the decays that are not made any more.  bf16, 32 heads of 128 x 64, 16 x 8192 tokens: 836 us with two
-// stages, 820 with three, 670 since the warp index is a shuffle's result (uniform branches and descriptors) and a wait looks at its barrier first
+// stages, 820 with three, 680 since the warp index is a shuffle's result (uniform branches and descriptors) and a wait looks at its barrier first
 // (3.2 GB of operands; the contractions it replaces: 1070 us).
 #include <cuda_bf16.h>
 #include "tc_common.cuh"
