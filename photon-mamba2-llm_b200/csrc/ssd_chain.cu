@@ -88,7 +88,7 @@ struct Geo {
   // precedes it, and the kernel checks)
   // The masked tile by factors of blocks instead of an exponential per element.  Not for storage blocks on plain operands, whose M is rounded to
   // bf16 in a stream of bf16 values: a flipped rounding grows through the layers behind it, so that the gradients of two builds would differ
-  // by as much as bf16 storage itself puts them off (2e-2).  That is a choice for results that repeat; neither form is nearer to fp64.
+  // by as much as bf16 storage itself puts them off (2e-2).  That is a choice, for results that repeat.
   static constexpr bool FACT = NB == 1 && !BIG && (ND == 2 || XIN16);
   static constexpr int BARS = XIN16 ? 320 : 256;         // bytes of barriers and small sums
   static constexpr int SLOT = (BIG ? 1 : 2) * L, SLACK = BIG ? 512 : 1024;    // floats per copy of S: [S | column factors]
