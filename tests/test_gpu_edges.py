@@ -492,10 +492,10 @@ def test_gemm_pair_tiles_on_pairs(pm, M, N, K):
     assert_close(out, a.double() @ b.double(), tol=3e-5, what=f"{M}x{N}x{K}")
 
 
-# the conv's strips: 16 runs (backward 8) of 8, 16 or 32 steps to a CTA, four (two) channels per thread, the next four (eight) rows in shared
-# memory (the oracle's fp32 sums in another order: 1e-5 of the largest)
+# the conv's strips: 16 runs (backward 8) of 8, 16 or 32 steps to a CTA (130 and 240 sequences of 160 channels), four (two) channels per
+# thread, the next four (eight) rows in shared memory (the oracle's fp32 sums in another order: 1e-5 of the largest)
 @pytest.mark.parametrize("K", [2, 3, 4])
-@pytest.mark.parametrize("B,T", [(1, 1), (2, 7), (1, 8), (1, 63), (2, 65), (3, 300), (40, 260)])
+@pytest.mark.parametrize("B,T", [(1, 1), (2, 7), (1, 8), (1, 63), (2, 65), (3, 300), (40, 260), (130, 260), (240, 260)])
 @pytest.mark.parametrize("H,P,N", [(4, 4, 4), (4, 16, 8), (8, 16, 16)])
 def test_conv_strips(pm, B, T, K, H, P, N):
     cfg = pm.Mamba2Config(d_model=32, d_state=N, d_head=P, n_heads=H, n_groups=1, d_conv=K, block_len=T)
@@ -559,7 +559,7 @@ def test_scan_bf16_positive_a(pm, T, Q, N, rise):
 
 
 # products whose columns go to tiles of two widths: two rounds of tiles, a cut inside and one before the last tile, B in either order, a residual
-@pytest.mark.parametrize("M,N,K", [(2048, 3224, 768), (1337, 3224, 136), (1000, 5000, 64)])
+@pytest.mark.parametrize("M,N,K", [(2048, 3224, 768), (1337, 3224, 136), (1000, 5000, 64), (14630, 296, 64)])
 @pytest.mark.parametrize("tb,res", [(False, False), (True, True)])
 def test_gemm_columns_cut(pm, M, N, K, tb, res):
     a, b, r = randn((M, K), 1).cuda(), randn((N, K) if tb else (K, N), 2).cuda(), randn((M, N), 3).cuda()
