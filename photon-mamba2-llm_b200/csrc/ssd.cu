@@ -1297,7 +1297,17 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
     }
   }
   if (lane) PMB_CUDA(cudaEventRecord(lane->ev[2], st));       // dh is ready (dB reads it)
-  if (fz) {
+  if (fz && in.plain16) {
+    // (the B / C / x~ operands were written by the forward of this scan and are still in the workspace)
+    const FusedArgs fa = fused_args(in, ws);
+    DxArgs da{};
+    da.B = in.B; da.T = in.T; da.H = in.H; da.P = in.P; da.N = in.N; da.G = in.G; da.Q = in.Q;
+    da.S = ws.S; da.dt = in.dt; da.A = in.A; da.D = in.D; da.b = fa.b; da.c = fa.c;
+    da.xt = ws.xt_hi; da.dy16 = ws.dy_hi; da.dh = ws.dh_hi;
+    da.x = in.x; da.ldx = in.ldx; da.dy = dy; da.lddy = lddy; da.yoff = ws.yoff; da.dx = g.dx; da.lddx = g.lddx;
+    da.dd = dsend; da.rpart = ws.rpart; da.sums = p.dxt; da.part = ws.part; da.raw = g.raw;
+    PMB_TRY(ssd_dx(st, da));
+  } else if (fz) {
     // dY as a bf16 pair (the B / C / x~ pairs were written by the forward of this scan and are still in the workspace)
     FusedArgs fa = fused_args(in, ws);
     fa.v = Op16{ws.dy_hi, in.plain16 ? nullptr : ws.dy_lo, (int64_t)p.H * p.P};
@@ -1313,7 +1323,7 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
     PMB_TRY(ssd_tc_dx(st, in, dy, lddy, ws));
   }
   else PMB_TRY(run_op(st, "ssd_bwd_dx", make_op<OpDx>(p, p.Q, p.P), nbch, 2.0 * tok * p.H * p.P * (p.Q + p.N)));
-  {
+  if (!(fz && in.plain16)) {
     ProfScope prof(st, "ssd_bwd_rows", 0.0, 4.0 * tok * p.H * (5.0 * p.P + 8.0));
     const bool vec_ok = (p.P % 4 == 0) && (p.ldx % 4 == 0) && (p.ldy % 4 == 0) && (p.lddy % 4 == 0) && (g.lddx % 4 == 0) &&
                         ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.y) | reinterpret_cast<uintptr_t>(p.dy) |

@@ -5,14 +5,13 @@
 //   1. G = R K^T on the tensor core into one of two TMEM buffers (R = the CTA's 128 rows of C, K = 64 rows of B in
 //      mode 0; the roles of B and C swap in mode 1), K = d_state;
 //   2. four warps read G from TMEM (thread = row), multiply by exp(S_row - S_col) with the causal test in fp32
-//      registers, and write the masked tile into shared memory as a K-major bf16 operand (hi and lo halves of the
-//      fp32 value in pair mode);
+//      registers, and write the masked tile back over G as a bf16 operand (hi and lo halves of the fp32 value in pair mode);
 //   3. acc1 += masked tile x V (V = 64 rows of x~ in mode 0, of dY in mode 1; MN-major) on the tensor core;
 // while step 2 of block j runs, the tensor core already computes step 1 of block j+1.  The carried-state term
 // (C h_prev in mode 0, B dh in mode 1) goes to a second accumulator and is scaled per row in the epilogue, which
 // also adds the skip term D x (mode 0).  C B^T never reaches HBM and no operand is rescaled in shared memory.
 //
-// Mode 1 (backward) also forms, from the same registers, the quantity the gradient of the decay needs.  With
+// Mode 1 (backward; on pairs: ssd_dx.cu is the one on plain operands) also forms, from the same registers, the quantity the gradient of the decay needs.  With
 // dM[t,s] = <dY_t, x~_s> (one more MMA per column block: the x~ rows of the CTA times the dY tile already in shared
 // memory) and W[t,s] = dM[t,s] G[t,s] exp(S_t - S_s) for s < t, the gradient w.r.t. the in-chunk cumulative sum is
 // dS_k = sum_s W[k,s] - sum_t W[t,k] (+ the carried-state terms).  Row sums over t (thread-private) and column sums
@@ -63,7 +62,6 @@ constexpr int MAXQ = 1024;
 //   ROP    the CTA's row operand, resident: NS x NK tiles of 128 x 64
 //   ring   STAGES slots of [K operand: NS x NK tiles of 64 x 64 | V: NS x PB tiles of 64 x 64]; slot use 0 carries the
 //          carried-state tile (NS x NK x PB tiles of 64 x 64, never larger than a slot) instead of a column block
-//   MOP    MB buffers of the masked tile: NS tiles of 128 x 64
 template <int MODE, int NS, int NK, int PB>
 struct Geo {
   static constexpr int ROP = NS * NK * T128 + (MODE == 1 ? NS * PB * T128 : 0);   // mode 1: + the x~ rows of the CTA
@@ -72,22 +70,18 @@ struct Geo {
   static constexpr int V = NS * PB * T64;
   static constexpr int STAGE = COP + V;
   static constexpr int ST = NS * NK * PB * T64;
-  // TM: the masked tile goes back into TMEM over G and is the A operand of the second product from there, so there
+  // The masked tile goes back into TMEM over G and is the A operand of the second product from there, so there
   // are no masked-tile buffers in shared memory.  Mode 0: two CTAs then fit on an SM.  Mode 1 stays at one CTA per SM
-  // (384 TMEM columns, two resident row operands) and gains only the shorter hand-over (measured: 3.5 % of the
-  // kernel with pairs, nothing with plain bf16 operands, which keep the shared-memory tile).
-  static constexpr bool TM = (MODE == 0) || (NS == 2);
-  static constexpr int MOP1 = TM ? 0 : NS * T128;
+  // (384 TMEM columns, two resident row operands) and gains only the shorter hand-over (measured: 3.5 % of the kernel).
   static constexpr int BUDGET = MODE == 0 ? 104 * 1024 : 218 * 1024;
-  static constexpr int MB = (ROP + 2 * MOP1 + 2 * STAGE <= BUDGET) ? 2 : 1;
-  static constexpr int REM = BUDGET - ROP - MB * MOP1;
+  static constexpr int REM = BUDGET - ROP;
   static constexpr int STAGES = REM / STAGE >= 4 ? 4 : REM / STAGE;
-  static constexpr bool FITS = STAGES >= 2 && ST <= STAGE && MB == 2;   // (one masked-tile buffer per mask group)
-  static constexpr int TILES = ROP + STAGES * STAGE + MB * MOP1;
+  static constexpr bool FITS = STAGES >= 2 && ST <= STAGE;
+  static constexpr int TILES = ROP + STAGES * STAGE;
   static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 256 /*barriers*/ + MAXQ * 4 /*S of the chunk*/ +
                               (MODE == 1 ? (2 * NGRP * NEPI * CW + 2 * RB) * 4 : 0) /*column sums of W, group exchange*/;
   static constexpr int TMEM_COLS = ((MODE == 1 ? 4 : 2) * CW + 2 * 64 * PB) <= 256 ? 256 : 512;
-  static constexpr int CTAS = (TM && TMEM_COLS == 256) ? 2 : 1;      // CTAs per SM the plan is sized for
+  static constexpr int CTAS = TMEM_COLS == 256 ? 2 : 1;      // CTAs per SM the plan is sized for
 };
 
 struct Maps { CUtensorMap rop[2], cop[2], v[2], st[2], xr[2]; };   // [0] = hi (or the plain bf16 tensor), [1] = lo
@@ -123,17 +117,15 @@ template <int MODE, int NS, int NK, int PB>
 __global__ void __launch_bounds__(NTHREADS, (Geo<MODE, NS, NK, PB>::CTAS))
 ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
   using GE = Geo<MODE, NS, NK, PB>;
-  constexpr int STAGES = GE::STAGES, MB = GE::MB, P = 64 * PB;
+  constexpr int STAGES = GE::STAGES, P = 64 * PB;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - raw);
   const uint32_t rop_s = base;
   const uint32_t ring_s = rop_s + GE::ROP;
-  const uint32_t mop_s = ring_s + STAGES * GE::STAGE;
-  const uint32_t bars = mop_s + MB * GE::MOP1;
-  enum { R_FULL = 0, LD_FULL = 1, LD_EMPTY = LD_FULL + STAGES, G_FULL = LD_EMPTY + STAGES, G_FREE = G_FULL + 2,
-         M_READY = G_FREE + 2, M_FREE = M_READY + MB, ACC_FULL = M_FREE + MB, NBAR = ACC_FULL + 1 };
+  const uint32_t bars = ring_s + STAGES * GE::STAGE;
+  enum { R_FULL = 0, LD_FULL = 1, LD_EMPTY = LD_FULL + STAGES, G_FULL = LD_EMPTY + STAGES, M_READY = G_FULL + 2, ACC_FULL = M_READY + 2, NBAR };
   static_assert(8 * NBAR + 8 <= 256, "barrier block");
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
   uint8_t* bar_ptr = base_ptr + (bars - base);
@@ -155,8 +147,7 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
   if (threadIdx.x == 0) {
     mbar_init(bar(R_FULL), 1);
     for (int s = 0; s < STAGES; ++s) { mbar_init(bar(LD_FULL + s), 1); mbar_init(bar(LD_EMPTY + s), 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(bar(G_FULL + i), 1); mbar_init(bar(G_FREE + i), NEPI); }
-    for (int i = 0; i < MB; ++i) { mbar_init(bar(M_READY + i), NEPI); mbar_init(bar(M_FREE + i), 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(bar(G_FULL + i), 1); mbar_init(bar(M_READY + i), NEPI); }
     mbar_init(bar(ACC_FULL), 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -280,8 +271,7 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
       auto mma_g = [&](int jj) -> bool {
         const int it = jj + 1, s = it % STAGES;
         if (!wait_all(LD_FULL + s, (uint32_t)((it / STAGES) & 1), 2u)) return false;
-        // (TM: the buffer's previous content, masked tile jj - 2, was read by a product issued before this one)
-        if (!GE::TM && jj >= 2 && !wait_all(G_FREE + (jj & 1), (uint32_t)(((jj >> 1) - 1) & 1), 4u)) return false;
+        // (the buffer's previous content, masked tile jj - 2, was read by a product issued before this one)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t cop = ring_s + s * GE::STAGE;
         const uint32_t r0 = lo_k(rop_s), c0d = lo_k(cop);
@@ -310,12 +300,11 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
       ok = ok && mma_g(0);
       if (ok && ncb > 1) ok = mma_g(1);
       for (int jj = 0; jj < ncb && ok; ++jj) {
-        const int mb = jj % MB, s = (jj + 1) % STAGES;
-        if (!wait_all(M_READY + mb, (uint32_t)((jj / MB) & 1), 8u)) { ok = false; break; }
+        const int mb = jj & 1, s = (jj + 1) % STAGES;
+        if (!wait_all(M_READY + mb, (uint32_t)((jj >> 1) & 1), 8u)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t m0d = lo_k(mop_s + mb * GE::MOP1), v0d = lo_mn(ring_s + s * GE::STAGE + GE::COP);
+        const uint32_t v0d = lo_mn(ring_s + s * GE::STAGE + GE::COP);
         if (elect_one()) {
-        if (GE::TM) {
           // masked tile in TMEM, in place of G: per 32 k of the block [hi: 16 columns | lo: 16 columns], 8 columns per k-step
           const uint32_t bs = (PB * T64) >> 4;
 #pragma unroll
@@ -331,13 +320,7 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
               mma_f16_ts_h(tA1, ta, vb, dh, id_v, acc);
             }
           }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            kstep(tA1, m0d + ((k * 32) >> 4), T128 >> 4, v0d + ((k * 2048) >> 4), (PB * T64) >> 4, id_v, (jj | k) ? 1u : 0u);
-        }
-        umma_commit(bar(LD_EMPTY + s));
-        umma_commit(bar(M_FREE + mb));
+          umma_commit(bar(LD_EMPTY + s));
         }
         __syncwarp();
         if (jj + 2 < ncb && !mma_g(jj + 2)) { ok = false; break; }
@@ -346,7 +329,7 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
       __syncwarp();
     }
   } else {
-    // ---------------- mask (TMEM -> registers -> shared-memory operand), then epilogue ----------------
+    // ---------------- mask (TMEM -> registers -> TMEM), then epilogue ----------------
     const int quarter = warp & 3;                       // the TMEM lane quarter this warp may read
     const int grp = (warp - 2) >> 2;                    // mask group: column blocks jj with jj % 2 == grp
     const int r_local = quarter * 32 + lane;
@@ -365,12 +348,9 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
     // work, not the barrier), so the four warps of a group can never wait for one another unboundedly.
     for (int jj = grp; jj < ncb; jj += NGRP) {
       const int c0 = (cb0 + jj) * CW, mb = jj & 1, use = jj >> 1;       // use-th block of this group's buffers
-      bool got = ok && wait_idle(G_FULL + mb, (uint32_t)(use & 1), 16u);
-      if (!GE::TM && got && use >= 1) got = wait_idle(M_FREE + mb, (uint32_t)((use - 1) & 1), 32u);
-      ok = __all_sync(0xffffffffu, got);
+      ok = __all_sync(0xffffffffu, ok && wait_idle(G_FULL + mb, (uint32_t)(use & 1), 16u));
       if (ok) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        uint8_t* mrow = base_ptr + (mop_s - base) + mb * GE::MOP1 + (r_local >> 3) * 1024 + (r_local & 7) * 128;
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           uint32_t r[32];
@@ -382,10 +362,9 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
 #pragma unroll
             for (int e = 0; e < 32; ++e) wv[e] = __uint_as_float(d[e]);
           }
-          uint32_t mh[16], ml[16];                  // TM: this half's packed hi / lo values
+          uint32_t mh[16], ml[16];                  // this half's packed hi / lo values
 #pragma unroll
           for (int q8 = 0; q8 < 4; ++q8) {
-            uint32_t hi[4], lo[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
             for (int e2 = 0; e2 < 4; ++e2) {
               const int e = q8 * 8 + 2 * e2;
@@ -403,32 +382,22 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
                 wv[e + 1] = col + 1 > row ? wv[e + 1] * m1 : 0.0f;
                 c_acc += wv[e] + wv[e + 1];
               }
-              split2(m0, m1, hi[e2], lo[e2], NS == 2);
-            }
-            if (GE::TM) {
-#pragma unroll
-              for (int e2 = 0; e2 < 4; ++e2) { mh[q8 * 4 + e2] = hi[e2]; ml[q8 * 4 + e2] = lo[e2]; }
-            } else {
-              const int sw = ((half * 4 + q8) ^ (r_local & 7)) << 4;     // 128-byte swizzle of the 16-byte chunk
-              *reinterpret_cast<uint4*>(mrow + sw) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-              if (NS == 2) *reinterpret_cast<uint4*>(mrow + T128 + sw) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+              ml[q8 * 4 + e2] = 0u;
+              split2(m0, m1, mh[q8 * 4 + e2], ml[q8 * 4 + e2], NS == 2);
             }
           }
-          if (GE::TM) {
-            // over the 32 columns of G just read: [hi of these 32 k | lo of these 32 k]
-            tmem_st16(tG + lane_addr + (uint32_t)(mb * CW + half * 32), mh);
-            if (NS == 2) tmem_st16(tG + lane_addr + (uint32_t)(mb * CW + half * 32 + 16), ml);
-          }
+          // over the 32 columns of G just read: [hi of these 32 k | lo of these 32 k]
+          tmem_st16(tG + lane_addr + (uint32_t)(mb * CW + half * 32), mh);
+          if (NS == 2) tmem_st16(tG + lane_addr + (uint32_t)(mb * CW + half * 32 + 16), ml);
           if (MODE == 1) {
             // column sums of W over this warp's 32 rows: lane l ends up with column half*32 + l
             rsum[(((grp * 2) + (use & 1)) * NEPI + quarter) * CW + half * 32 + lane] = warp_column_sums(wv, lane);
           }
         }
-        if (GE::TM) tmem_wait_st();
+        tmem_wait_st();
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        if (!GE::TM) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) { if (!GE::TM) mbar_arrive(bar(G_FREE + mb)); mbar_arrive(bar(M_READY + mb)); }
+        if (lane == 0) mbar_arrive(bar(M_READY + mb));
       }
       if (MODE == 1) {
         if (grp == 0) asm volatile("bar.sync 1, %0;" ::"n"(32 * NEPI) : "memory");
@@ -624,6 +593,8 @@ static pmb_status launch(cudaStream_t st, const FusedArgs& a) {
 
 }  // namespace sf
 
+unsigned int* ssd_fused_status() { return sf::status_ptr(); }
+
 bool ssd_fused_supported(int P, int N, int Q) { return Q % sf::RB == 0 && Q <= sf::MAXQ && N == 64 && P == 64; }
 
 pmb_status ssd_fused(cudaStream_t st, int mode, const FusedArgs& a) {
@@ -642,7 +613,7 @@ pmb_status ssd_fused(cudaStream_t st, int mode, const FusedArgs& a) {
   // algorithmic work: G per head (2 Q N), masked product (2 Q P) over the causal half (counted in full), state term (2 N P)
   ProfScope prof(st, mode == 0 ? "ssd_fused_y" : "ssd_fused_dx", 2.0 * tok * a.H * ((double)a.Q * (a.N + a.P) + (double)a.N * a.P), 0.0);
   if (mode == 0) return pairs ? sf::launch<0, 2, 1, 1>(st, a) : sf::launch<0, 1, 1, 1>(st, a);
-  return pairs ? sf::launch<1, 2, 1, 1>(st, a) : sf::launch<1, 1, 1, 1>(st, a);
+  return pairs ? sf::launch<1, 2, 1, 1>(st, a) : fail(PMB_ERR_UNSUPPORTED, "ssd_fused: the backward on plain operands is ssd_dx");
 }
 
 }  // namespace pmb

@@ -105,6 +105,24 @@ bool ssd_fused_supported(int P, int N, int Q);
 //         plus csum, esum, rpart (see FusedArgs)
 pmb_status ssd_fused(cudaStream_t st, int mode, const FusedArgs& a);
 
+// ---- the backward on plain bf16 operands (ssd_dx.cu): chunks of 128 or 256 tokens at d_state = d_head = 64
+struct DxArgs {
+  int B, T, H, P, N, G, Q;
+  const float* S; const float* dt; const float* A; const float* D;      // D = NULL: no skip term
+  Op16 b, c;               // as in FusedArgs
+  const uint16_t *xt, *dy16, *dh;   // x~ and dY (B,T,H,P); adjoint of the state leaving each chunk (B,T/Q,H,N,P)
+  const float* x; int64_t ldx; const float* dy; int64_t lddy;
+  const float* yoff;       // (B,T,H,P) exp(S_t) C_t h_prev
+  float* dx; int64_t lddx; // dx~ dt + D dY
+  const float* dd;         // (B*T/Q,H) <dh, h_prev>
+  float *rpart, *sums;     // scratch: (B*T/Q*H, Q/128, Q) and ssd_dx_sum_floats() floats
+  float* part;             // 3 x (B*T/Q,H): sums for dA, dD, d_dt_bias
+  SsdGrads::RawDt raw;     // gradient before the softplus (hi alone)
+};
+size_t ssd_dx_sum_floats(int B, int T, int H);
+pmb_status ssd_dx(cudaStream_t st, const DxArgs& a);
+
+unsigned int* ssd_fused_status();
 pmb_status read_clear_device_status_fused(unsigned int* word);
 pmb_status read_clear_device_status_pairs(unsigned int* word);
 

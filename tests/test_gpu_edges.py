@@ -696,3 +696,22 @@ def test_two_level_widths(pm, D, dtype):
     assert_close(lm.view(lm.flat_grads, -2), wr.grad, tol=tol, what="d_wproj")
     assert pm.device_status() == 0
     lm.close()
+
+
+# the backward of whole chunks on plain operands (csrc/ssd_dx.cu): one and several row blocks to a chunk, one chunk, B and C per head, more
+# CTAs than fit the machine at once, and a decay that underflows inside a block of columns.  bf16 operands and storage: 2e-2.
+@pytest.mark.parametrize("B,T,Q", [(1, 128, 128), (2, 256, 256), (2, 768, 128), (3, 1024, 256), (2, 4096, 256)])
+@pytest.mark.parametrize("G,decay", [(1, 0.0), (1, 3.0), (8, 0.0)])
+def test_block_bf16_backward_of_chunks(pm, B, T, Q, G, decay):
+    cfg, p, blk = _block(pm, 256, 8, 64, 64, G, Q, torch.bfloat16)
+    p["a_log"] = p["a_log"] + decay
+    blk = pm.Mamba2Block(blk.config, {k: v.cuda() for k, v in p.items()}, compute_dtype=torch.bfloat16)
+    x, cot = randn((B, T, 256), 32).bfloat16(), randn((B, T, 256), 33).bfloat16()
+    leaves = {k: v.clone().requires_grad_(True) for k, v in p.items()}
+    xr = x.float().requires_grad_(True)
+    orc.block_forward(leaves, cfg, xr).backward(cot.float())
+    dx, grads = blk.backward(x.cuda(), cot.cuda())
+    assert_close(dx.float(), xr.grad, tol=2e-2, what="dx")
+    for k, v in leaves.items():
+        assert_close(grads[k], v.grad, tol=2e-2, what=k)
+    assert pm.device_status() == 0
