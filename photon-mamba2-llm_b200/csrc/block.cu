@@ -255,7 +255,7 @@ static pmb_status block_fwd_core(cudaStream_t st, const Dims& d, const pmb_block
     // the backward reads S, the states, x~, xs and the carried part of y: the chain leaves them on its way
     ChainArgs a = chain_inputs(d, p, w.xzd, w.act, w.ssd.bc_hi, nullptr, w.y);
     a.blocks = d.Q / SCAN_STEP;
-    a.S_out = w.ssd.S; a.dt_out = w.dt; a.A_out = w.Aneg; a.hp_hi = w.ssd.hp_hi; a.hprev = w.ssd.hprev; a.yoff = w.ssd.yoff; a.xt = w.ssd.xt_hi; a.xs = w.ssd.xs_hi;
+    a.S_out = w.ssd.S; a.dt_out = w.dt; a.A_out = w.Aneg; a.hp_hi = w.ssd.hp_hi; a.hprev = w.ssd.hprev; a.xt = w.ssd.xt_hi; a.xs = w.ssd.xs_hi;
     PMB_TRY(ssd_chain_fwd(st, a));
   } else {
   sin.plain16 = w16 != nullptr;

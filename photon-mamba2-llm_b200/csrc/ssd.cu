@@ -1221,7 +1221,7 @@ pmb_status ssd_fwd(cudaStream_t st, const SsdIn& in, const float* init_state, fl
     fa.v = Op16{ws.xt_hi, in.plain16 ? nullptr : ws.xt_lo, (int64_t)p.H * p.P};
     fa.state = Op16{ws.hp_hi, in.plain16 ? nullptr : ws.hp_lo, p.P};
     fa.out = y; fa.ldo = ldy; fa.x = in.x; fa.ldx = in.ldx; fa.D = in.D;
-    fa.off_out = ws.yoff;
+    fa.off_out = in.plain16 ? nullptr : ws.yoff;
     PMB_TRY(ssd_fused(st, 0, fa));
   }
   else if (tc) PMB_TRY(ssd_tc_scan(st, in, y, ldy, ws));
@@ -1303,8 +1303,8 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
     DxArgs da{};
     da.B = in.B; da.T = in.T; da.H = in.H; da.P = in.P; da.N = in.N; da.G = in.G; da.Q = in.Q;
     da.S = ws.S; da.dt = in.dt; da.A = in.A; da.D = in.D; da.b = fa.b; da.c = fa.c;
-    da.xt = ws.xt_hi; da.dy16 = ws.dy_hi; da.dh = ws.dh_hi;
-    da.x = in.x; da.ldx = in.ldx; da.dy = dy; da.lddy = lddy; da.yoff = ws.yoff; da.dx = g.dx; da.lddx = g.lddx;
+    da.xt = ws.xt_hi; da.dy16 = ws.dy_hi; da.hp = ws.hp_hi; da.dh = ws.dh_hi;
+    da.x = in.x; da.ldx = in.ldx; da.dy = dy; da.lddy = lddy; da.dx = g.dx; da.lddx = g.lddx;
     da.dd = dsend; da.rpart = ws.rpart; da.sums = p.dxt; da.part = ws.part; da.raw = g.raw;
     PMB_TRY(ssd_dx(st, da));
   } else if (fz) {

@@ -108,9 +108,9 @@ struct Params {
   float* dt_out; float* A_out; float* S_out;             // optional from here on: what a backward reads
   uint16_t *hp_hi, *hp_lo;                               // (B,nsteps,H,N,P)
   float* last;                                           // (B,H,N,P)
-  // plain operands, for a backward that works chunk by chunk: state entering each chunk in fp32, exp(S) C h of every token, and
-  // (store_ops) x~ and xs as the kernel formed them.  bf16 x: store_ops leaves a copy of it.
-  float *hprev, *yoff;
+  // plain operands, for a backward that works chunk by chunk: state entering each chunk in fp32, and (store_ops) x~ and xs as the
+  // kernel formed them.  bf16 x: store_ops leaves a copy of it.
+  float* hprev;
   int store_ops;
   int first, nseg, per;                                  // first chain of this launch (grid: chains x segments); segments of a sequence, steps per segment
   int late;                                              // needs nothing from the kernel before, which lets this one in after its own wait: waits when it is done
@@ -451,12 +451,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
             for (int e = 0; e < 2; ++e) {
               const int r = 4 * q + 2 * e;
               float2& v = o[rh][2 * c16 + q][e];
-              if (ND == 1 && !XIN16 && p.yoff) {
-                const int t = t0 + 16 * rh + 8 * e;
-                if (t < p.T && cw + 16 * c16 + 8 * q < p.P)
-                  *reinterpret_cast<float2*>(p.yoff + (tokb + t) * (int64_t)(p.H * p.P) + col + 16 * c16 + 8 * q) =
-                      make_float2(f[2 * rh + e] * __uint_as_float(a2[r]), f[2 * rh + e] * __uint_as_float(a2[r + 1]));
-              }
               const float u0 = fmaf(f[2 * rh + e], __uint_as_float(a2[r]), __uint_as_float(a1[r])), u1 = fmaf(f[2 * rh + e], __uint_as_float(a2[r + 1]), __uint_as_float(a1[r + 1]));
               v = XIN16 || NG == 2 ? make_float2(u0, u1) : make_float2(fmaf(dv, v.x, u0), fmaf(dv, v.y, u1));
             }
@@ -775,7 +769,7 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
   p.x = a.x; p.ldx = a.ldx;
   p.dt_raw = a.dt_raw; p.ld_raw = a.ld_raw; p.dt_bias = a.dt_bias; p.a_log = a.a_log; p.dt = a.dt; p.A = a.A; p.a = a.a; p.D = a.D;
   p.init = a.init; p.y = a.y; p.y16 = a.y16; p.ldy = a.ldy; p.dt_out = a.dt_out; p.A_out = a.A_out; p.S_out = a.S_out;
-  p.hprev = a.hprev; p.yoff = a.yoff;
+  p.hprev = a.hprev;
   uint16_t* const keep = XIN16 ? a.x_keep : a.xt;
   if (XIN16) PMB_TRY(sf::bf16_map4(&ms.x, a.x16, a.P, a.T, a.H, a.B, a.ldx, a.P, a.T * a.ldx, 64, L));
   if (keep) {
@@ -837,7 +831,7 @@ pmb_status ssd_chain_fwd(cudaStream_t st, const ChainArgs& a) {
   if (!al16(a.x) || !al16(a.x16) || !al16(a.y) || !al16(a.y16) || !al16(a.init) || (a.ldx & (a.x16 ? 7 : 3)) || (a.ldy & 3))
     return fail(PMB_ERR_SHAPE, "ssd_chain: x, y and state rows must be 16-byte aligned");
   if (!pairs && !a.x16 && a.N > 64) return fail(PMB_ERR_UNSUPPORTED, "ssd_chain: fp32 x with plain bf16 B and C takes d_state up to 64");
-  if ((a.hprev || a.yoff || a.xt) && (pairs || a.x16 || a.seg || (a.xt != nullptr) != (a.xs != nullptr))) return fail(PMB_ERR_ARG, "ssd_chain: the chunk outputs go with fp32 x on plain operands");
+  if ((a.hprev || a.xt) && (pairs || a.x16 || a.seg || (a.xt != nullptr) != (a.xs != nullptr))) return fail(PMB_ERR_ARG, "ssd_chain: the chunk outputs go with fp32 x on plain operands");
   const double tok = (double)a.B * a.T;
   // G and the masked product over the causal half of a step, the state update and the carried-state product
   ProfScope prof(st, "ssd_chain_fwd", tok * a.H * ((double)SCAN_STEP * (a.N + a.P) + 4.0 * a.N * a.P), 0.0);

@@ -25,21 +25,20 @@ using namespace tcx;
 constexpr int RB = 128, CW = 64, NMASKW = 8, NMASK = 32 * NMASKW, NTHREADS = 64 + NMASK;
 constexpr int PW = 64, MAXQ = 256;
 constexpr int T128 = RB * 128, T64 = CW * 128;
-constexpr int STAGES = 2, STAGE = 2 * T64;                  // [C | dY] of a column block; slot use 0 carries the state tile
+constexpr int STAGES = 2, STAGE = 2 * T64;                  // [C | dY] of a column block; slot use 0 carries the state tiles, [dh | h]
 constexpr int TILES = 2 * T128 + STAGES * STAGE + 2 * T128; // [B | x~], ring, two masked tiles
 constexpr int NSUM = 5;                                     // per row: sum of W over t, e, <dx~, x>, <dY, exp(S) C h>, <dY, x>
 constexpr int SMEM = TILES + 1024 + 256 + (MAXQ + 4 * MAXQ + 2 * NSUM * RB) * 4;
 constexpr int TMEM_COLS = 256;
 static_assert(2 * (SMEM + 1024) <= 227 * 1024, "two CTAs per SM");
 
-struct Maps { CUtensorMap b, x, c, dy, st; };
+struct Maps { CUtensorMap b, x, c, cr, dy, st, hp; };       // cr: C in tiles of 128 rows
 struct Params {
   int H, hpg, Q, nc, nb, T;
   const float* S;
   const float* dt;
   const float* x; int64_t ldx;
   const float* dy; int64_t lddy;
-  const float* yoff;
   const float* D;
   float* dx; int64_t lddx;
   float* rpart;                                             // (B*nc*H, nb, Q)
@@ -81,7 +80,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) ssd_dx_kernel(const __grid_consta
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* base_ptr = smem_raw + (base - raw);
   const uint32_t b_s = base, x_s = b_s + T128, ring_s = x_s + T128, mop_s = ring_s + STAGES * STAGE, bars = mop_s + 2 * T128;
-  enum { R_FULL = 0, LD_FULL = 1, LD_EMPTY = LD_FULL + STAGES, G_FULL = LD_EMPTY + STAGES, G_FREE, M_READY, M_FREE = M_READY + 2, ACC_FULL = M_FREE + 2, NBAR };
+  enum { R_FULL = 0, F_FULL, LD_FULL, LD_EMPTY = LD_FULL + STAGES, G_FULL = LD_EMPTY + STAGES, G_FREE, M_READY, M_FREE = M_READY + 2, ACC_FULL = M_FREE + 2, NBAR };
   static_assert(8 * NBAR + 8 <= 256, "barrier block");
   auto bar = [&](int i) { return bars + 8u * (uint32_t)i; };
   uint8_t* bar_ptr = base_ptr + (bars - base);
@@ -97,7 +96,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) ssd_dx_kernel(const __grid_consta
   const int tok0 = bc * p.Q;                                // first token of the chunk (T = nc * Q)
   const int cb0 = 2 * rb, ncb = p.Q / CW - cb0;
   if (threadIdx.x == 0) {
-    mbar_init(bar(R_FULL), 1);
+    mbar_init(bar(R_FULL), 1); mbar_init(bar(F_FULL), 1);
     for (int s = 0; s < STAGES; ++s) { mbar_init(bar(LD_FULL + s), 1); mbar_init(bar(LD_EMPTY + s), 1); }
     mbar_init(bar(G_FULL), 1); mbar_init(bar(G_FREE), NMASKW);
     for (int i = 0; i < 2; ++i) { mbar_init(bar(M_READY + i), NMASKW); mbar_init(bar(M_FREE + i), 1); }
@@ -134,17 +133,19 @@ __global__ void __launch_bounds__(NTHREADS, 2) ssd_dx_kernel(const __grid_consta
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      mbar_expect_tx(bar(R_FULL), 2 * T128);
+      mbar_expect_tx(bar(R_FULL), 3 * T128);
       tma_load_3d(b_s, &maps.b, 0, tok0 + RB * rb, g, bar(R_FULL));
       tma_load_3d(x_s, &maps.x, 0, tok0 + RB * rb, h, bar(R_FULL));
+      tma_load_3d(mop_s, &maps.cr, 0, tok0 + RB * rb, g, bar(R_FULL));      // (over the first masked tile, which waits for its product)
       int issued = 0;
       for (int it = 0; it <= ncb; ++it) {
         const int s = it % STAGES;
         if (!wait(LD_EMPTY + s, (uint32_t)(it / STAGES) ^ 1u, 1u)) break;
         const uint32_t dst = ring_s + s * STAGE;
         if (it == 0) {
-          mbar_expect_tx(bar(LD_FULL + s), T64);
+          mbar_expect_tx(bar(LD_FULL + s), STAGE);
           tma_load_3d(dst, &maps.st, 0, bch * PW, 0, bar(LD_FULL + s));
+          tma_load_3d(dst + T64, &maps.hp, 0, bch * PW, 0, bar(LD_FULL + s));
         } else {
           const int row0 = tok0 + CW * (cb0 + it - 1);
           mbar_expect_tx(bar(LD_FULL + s), STAGE);
@@ -169,8 +170,12 @@ __global__ void __launch_bounds__(NTHREADS, 2) ssd_dx_kernel(const __grid_consta
     bool ok = wait_all(R_FULL, 0u, 2u) && wait_all(LD_FULL + 0, 0u, 2u);
     if (ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t s0 = desc_lo(ring_s, T64);
+      const uint32_t s0 = desc_lo(ring_s, T64), h0 = desc_lo(ring_s + T64, T64), c0 = desc_lo(mop_s, 16);
       if (elect_one()) {
+        // C h, where the first product of a masked tile will land once the mask warps have read it
+#pragma unroll
+        for (int k = 0; k < 4; ++k) mma_f16_h(tA1, c0 + ((k * 32) >> 4), dh, h0 + ((k * 2048) >> 4), dh, id_v, k ? 1u : 0u);
+        umma_commit(bar(F_FULL));
 #pragma unroll
         for (int k = 0; k < 4; ++k) mma_f16_h(tA2, b0 + ((k * 32) >> 4), dh, s0 + ((k * 2048) >> 4), dh, id_v, k ? 1u : 0u);
         umma_commit(bar(LD_EMPTY + 0));
@@ -218,20 +223,48 @@ __global__ void __launch_bounds__(NTHREADS, 2) ssd_dx_kernel(const __grid_consta
     const int grp = (warp - 2) >> 2;                        // half of a block's (and of the output's) columns
     const int tid = (int)threadIdx.x - 64, r_local = quarter * 32 + lane, row0 = rb * RB + quarter * 32;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-    const int64_t HP = (int64_t)p.H * PW;
+    // fragments: this thread's rows are er + {0, 8, 16, 24}, its columns cw + 8 o + {0, 1}
+    const int er = quarter * 32 + (lane >> 2), cw = 32 * grp + (lane & 3) * 2;
+    const int64_t tkr = (int64_t)tok0 + rb * RB + er;
+    const int col = h * PW + cw;
+    float2 dyf[4][4];                                       // dY of all four rows, on its way while the first operands are
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+      for (int o = 0; o < 4; ++o) dyf[e][o] = *reinterpret_cast<const float2*>(p.dy + (tkr + 8 * e) * p.lddy + col + 8 * o);
     {
       const float* Sp = p.S + ((int64_t)bb * p.H + h) * p.T + (int64_t)cc * p.Q;
       if (tid < p.Q) sS[tid] = Sp[tid];
-      // the epilogue's rows on their way into L2: a thread has one line of each tensor
-      const int64_t tk = (int64_t)tok0 + rb * RB + (tid >> 1);
-      const int c = h * PW + 32 * (tid & 1);
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(p.x + tk * p.ldx + c));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(p.dy + tk * p.lddy + c));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(p.yoff + tk * HP + c));
+      // the epilogue's rows of x on their way into L2, a line per thread
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(p.x + ((int64_t)tok0 + rb * RB + (tid >> 1)) * p.ldx + h * PW + 32 * (tid & 1)));
       asm volatile("bar.sync 3, %0;" ::"n"(NMASK) : "memory");
     }
     const float S_row = sS[rb * RB + r_local];
-    bool ok = true;
+    bool ok = __all_sync(0xffffffffu, wait_idle(F_FULL, 0u, 64u));
+    if (ok) {
+      // f_t = <dY_t, exp(S_t) C_t h> of the same 128 tokens
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int rh = 0; rh < 2; ++rh) {
+        uint32_t a[16];
+        tmem_ld16x256_x4(tA1 + lane_addr + ((uint32_t)(16 * rh) << 16) + (uint32_t)(32 * grp), a);
+        tmem_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float fs = __expf(sS[rb * RB + er + 16 * rh + 8 * e]);
+          float f = 0.0f;
+#pragma unroll
+          for (int o = 0; o < 4; ++o) {
+            const float2 dy = dyf[2 * rh + e][o];
+            f = fmaf(dy.x, fs * __uint_as_float(a[4 * o + 2 * e]), fmaf(dy.y, fs * __uint_as_float(a[4 * o + 2 * e + 1]), f));
+          }
+          f += __shfl_xor_sync(0xffffffffu, f, 1);
+          f += __shfl_xor_sync(0xffffffffu, f, 2);
+          if ((lane & 3) == 0) xchg[(grp * NSUM + 3) * RB + er + 16 * rh + 8 * e] = f;
+        }
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
     float c_acc = 0.0f;                                     // sum over t > s of W[t,s] for this thread's row s, this half's columns
     // (nothing in this loop waits for another warp but through the bounded waits, so a warp that gave up just leaves it)
 #pragma unroll 1
@@ -286,12 +319,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) ssd_dx_kernel(const __grid_consta
       if (lane == 0) mbar_arrive(bar(M_READY + mb));
       colsum[quarter * MAXQ + c0 + lane] = warp_column_sums(wv, lane);
     }
-    // fragments: this thread's rows are er + {0, 8, 16, 24}, its columns cw + 8 o + {0, 1}
-    const int er = quarter * 32 + (lane >> 2), cw = 32 * grp + (lane & 3) * 2;
     const float Dv = p.D ? p.D[h] : 0.0f;
-    const int64_t tkr = (int64_t)tok0 + rb * RB + er;
-    const int col = h * PW + cw;
-    float2 xv[2][4], dyv[2][4], yo[2][4];
+    float2 xv[2][4], dyv[2][4];
     float dtv[2];
     auto fetch = [&](int rh) {
 #pragma unroll
@@ -302,7 +331,6 @@ __global__ void __launch_bounds__(NTHREADS, 2) ssd_dx_kernel(const __grid_consta
         for (int o = 0; o < 4; ++o) {
           xv[e][o] = *reinterpret_cast<const float2*>(p.x + tk * p.ldx + col + 8 * o);
           dyv[e][o] = *reinterpret_cast<const float2*>(p.dy + tk * p.lddy + col + 8 * o);
-          yo[e][o] = *reinterpret_cast<const float2*>(p.yoff + tk * HP + col + 8 * o);
         }
       }
     };
@@ -316,7 +344,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) ssd_dx_kernel(const __grid_consta
       const uint8_t* xt = base_ptr + (x_s - base);
 #pragma unroll 1
       for (int rh = 0; rh < 2; ++rh) {
-        float es[2] = {0.0f, 0.0f}, s1[2] = {0.0f, 0.0f}, s2[2] = {0.0f, 0.0f}, s3[2] = {0.0f, 0.0f}, fac[2];
+        float es[2] = {0.0f, 0.0f}, s1[2] = {0.0f, 0.0f}, s3[2] = {0.0f, 0.0f}, fac[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) fac[e] = __expf(S_end - sS[rb * RB + er + 16 * rh + 8 * e]);
 #pragma unroll
@@ -336,9 +364,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) ssd_dx_kernel(const __grid_consta
               const uint32_t xp = *reinterpret_cast<const uint32_t*>(xt + rl * 128 + (((4 * grp + o) ^ (rl & 7)) << 4) + (lane & 3) * 4);
               es[e] = fmaf(__uint_as_float(xp << 16), b0, fmaf(__uint_as_float(xp & 0xffff0000u), b1, es[e]));
               const float v0 = fmaf(fac[e], b0, __uint_as_float(a1[r])), v1 = fmaf(fac[e], b1, __uint_as_float(a1[r + 1]));
-              const float2 xx = xv[e][o], dy = dyv[e][o], yy = yo[e][o];
+              const float2 xx = xv[e][o], dy = dyv[e][o];
               s1[e] = fmaf(v0, xx.x, fmaf(v1, xx.y, s1[e]));
-              s2[e] = fmaf(dy.x, yy.x, fmaf(dy.y, yy.y, s2[e]));
               s3[e] = fmaf(dy.x, xx.x, fmaf(dy.y, xx.y, s3[e]));
               *reinterpret_cast<float2*>(p.dx + (tkr + 16 * rh + 8 * e) * p.lddx + col + 8 * o) = make_float2(fmaf(v0, dtv[e], Dv * dy.x), fmaf(v1, dtv[e], Dv * dy.y));
             }
@@ -349,10 +376,10 @@ __global__ void __launch_bounds__(NTHREADS, 2) ssd_dx_kernel(const __grid_consta
 #pragma unroll
           for (int o = 1; o <= 2; o <<= 1) {
             es[e] += __shfl_xor_sync(0xffffffffu, es[e], o); s1[e] += __shfl_xor_sync(0xffffffffu, s1[e], o);
-            s2[e] += __shfl_xor_sync(0xffffffffu, s2[e], o); s3[e] += __shfl_xor_sync(0xffffffffu, s3[e], o);
+            s3[e] += __shfl_xor_sync(0xffffffffu, s3[e], o);
           }
-          const float v = (lane & 3) == 0 ? es[e] * fac[e] : (lane & 3) == 1 ? s1[e] : (lane & 3) == 2 ? s2[e] : s3[e];
-          xchg[(grp * NSUM + 1 + (lane & 3)) * RB + er + 16 * rh + 8 * e] = v;
+          const int which = lane & 3;
+          if (which < 3) xchg[(grp * NSUM + (which == 2 ? 4 : 1 + which)) * RB + er + 16 * rh + 8 * e] = which == 0 ? es[e] * fac[e] : which == 1 ? s1[e] : s3[e];
         }
       }
     }
@@ -425,12 +452,14 @@ pmb_status ssd_dx(cudaStream_t st, const DxArgs& a) {
   sdx::Maps ms{};
   PMB_TRY(sf::bf16_map3(&ms.b, a.b.hi, 64, tok, a.G, a.b.pitch, 64, 64, sdx::RB));
   PMB_TRY(sf::bf16_map3(&ms.c, a.c.hi, 64, tok, a.G, a.c.pitch, 64, 64, sdx::CW));
+  PMB_TRY(sf::bf16_map3(&ms.cr, a.c.hi, 64, tok, a.G, a.c.pitch, 64, 64, sdx::RB));
   PMB_TRY(sf::bf16_map3(&ms.x, a.xt, 64, tok, a.H, HP, 64, 64, sdx::RB));
   PMB_TRY(sf::bf16_map3(&ms.dy, a.dy16, 64, tok, a.H, HP, 64, 64, sdx::CW));
   PMB_TRY(sf::bf16_map3(&ms.st, a.dh, 64, (int64_t)chunks * a.H * 64, 1, 64, 64 * 64, 64, sdx::CW));
+  PMB_TRY(sf::bf16_map3(&ms.hp, a.hp, 64, (int64_t)chunks * a.H * 64, 1, 64, 64 * 64, 64, sdx::CW));
   sdx::Params p{};
   p.H = a.H; p.hpg = a.H / a.G; p.Q = a.Q; p.nc = nc; p.nb = a.Q / sdx::RB; p.T = a.T;
-  p.S = a.S; p.dt = a.dt; p.x = a.x; p.ldx = a.ldx; p.dy = a.dy; p.lddy = a.lddy; p.yoff = a.yoff; p.D = a.D; p.dx = a.dx; p.lddx = a.lddx;
+  p.S = a.S; p.dt = a.dt; p.x = a.x; p.ldx = a.ldx; p.dy = a.dy; p.lddy = a.lddy; p.D = a.D; p.dx = a.dx; p.lddx = a.lddx;
   p.rpart = a.rpart; p.sums = a.sums; p.status = ssd_fused_status();
   {
     ProfScope prof(st, "ssd_dx", 2.0 * tok * a.H * 64 * (3.0 * a.Q + 64), 0.0);

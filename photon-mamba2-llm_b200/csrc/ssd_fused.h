@@ -43,7 +43,7 @@ struct ChainArgs {
   uint16_t* x_keep;                            // copy of x16, (B,T,H,P)
   uint16_t *hp_hi, *hp_lo;                     // state entering each step, (B,steps,H,N,P)
   float* last;                                 // (B,H,N,P)
-  float *hprev, *yoff;                         // plain operands with fp32 x: (B,chunks,H,N,P) state entering each chunk, (B,T,H,P) exp(S) C h
+  float *hprev;                                // plain operands with fp32 x: (B,chunks,H,N,P) state entering each chunk
   uint16_t *xt, *xs;                           // ... and the operands x~ and xs, (B,T,H,P)
   float* seg = nullptr;                        // ssd_chain_seg_floats() floats: lets few long sequences be walked in segments (blocks == 1)
 };
@@ -110,9 +110,8 @@ struct DxArgs {
   int B, T, H, P, N, G, Q;
   const float* S; const float* dt; const float* A; const float* D;      // D = NULL: no skip term
   Op16 b, c;               // as in FusedArgs
-  const uint16_t *xt, *dy16, *dh;   // x~ and dY (B,T,H,P); adjoint of the state leaving each chunk (B,T/Q,H,N,P)
+  const uint16_t *xt, *dy16, *hp, *dh;   // x~ and dY (B,T,H,P); state entering each chunk and adjoint of the one leaving it (B,T/Q,H,N,P)
   const float* x; int64_t ldx; const float* dy; int64_t lddy;
-  const float* yoff;       // (B,T,H,P) exp(S_t) C_t h_prev
   float* dx; int64_t lddx; // dx~ dt + D dY
   const float* dd;         // (B*T/Q,H) <dh, h_prev>
   float *rpart, *sums;     // scratch: (B*T/Q*H, Q/128, Q) and ssd_dx_sum_floats() floats
