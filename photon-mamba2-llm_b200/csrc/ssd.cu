@@ -1033,7 +1033,7 @@ void ssd_ws_take(Arena& ar, int B, int T, int H, int P, int N, int G, int Q, Ssd
         // pair path: dC and dB run side by side, each with its own partial tiles
         size_t dbc2 = (size_t)2 * ssd_pairs_dbc_nsplit(B, T, H, N, G, Q) * nbcg * Q * N;
         if (dbc2 > need) need = dbc2;
-        size_t dgp2 = (size_t)ssd_pairs_dg_nsplit(B, T, H, G, Q) * nbcg * Q * Q;
+        size_t dgp2 = (size_t)ssd_dg_nsplit(B, T, H, G, Q) * nbcg * Q * Q;
         if (dgp2 > need) need = dgp2;
       }
       w.splitk = ar.take<float>(need);
@@ -1376,8 +1376,8 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
   if (fz) {
     {
       ProfScope prof(sb, "ssd_bwd_dg_pair", 2.0 * tok * p.H * p.Q * p.P, 0.0);
-      const int nsg = ssd_pairs_dg_nsplit(p.B, p.T, p.H, p.G, p.Q);
-      PMB_TRY(ssd_pairs_dg(sb, in, ws, nsg));
+      const int nsg = ssd_dg_nsplit(p.B, p.T, p.H, p.G, p.Q);
+      PMB_TRY(ssd_dg(sb, in, ws, nsg));
       PMB_TRY(reduce(nsg, p.Q, 0, ws.dG, 0, 128));
     }
     const int ns = ssd_pairs_dbc_nsplit(p.B, p.T, p.H, p.N, p.G, p.Q);

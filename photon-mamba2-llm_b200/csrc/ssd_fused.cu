@@ -27,6 +27,7 @@
 // column blocks), so the mask work of two blocks and the tensor-core work of a third overlap.  Every mbarrier wait is bounded; on
 // expiry the CTA raises the status word, stops issuing work, and leaves through the common exit (TMEM freed).
 #include <cuda_bf16.h>
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 #include "tc_common.cuh"
@@ -494,10 +495,9 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
 
 // ---- host side -------------------------------------------------------------------------------------------
 struct MapKey {
-  const void* base; int rank; int64_t d[4], s[3]; int b0, b1;
+  const void* base; int rank; int64_t d[5], s[4]; int b[5];
   bool operator==(const MapKey& o) const {
-    return base == o.base && rank == o.rank && d[0] == o.d[0] && d[1] == o.d[1] && d[2] == o.d[2] && d[3] == o.d[3] && s[0] == o.s[0] && s[1] == o.s[1] &&
-           s[2] == o.s[2] && b0 == o.b0 && b1 == o.b1;
+    return base == o.base && rank == o.rank && std::equal(d, d + 5, o.d) && std::equal(s, s + 4, o.s) && std::equal(b, b + 5, o.b);
   }
 };
 struct MapKeyHash {
@@ -506,32 +506,31 @@ struct MapKeyHash {
     auto mix = [&](int64_t v) { h ^= std::hash<int64_t>()(v) + 0x9e3779b97f4a7c15ULL + (h << 6) + (h >> 2); };
     for (int64_t v : k.d) mix(v);
     for (int64_t v : k.s) mix(v);
-    mix(k.b0); mix(k.b1); mix(k.rank);
+    for (int v : k.b) mix(v);
+    mix(k.rank);
     return h;
   }
 };
 static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> g_maps;   // shared by all devices and host threads
 static std::mutex g_maps_mu;
 
-static pmb_status bf16_map(CUtensorMap* out, const uint16_t* base, int rank, int64_t d0, int64_t d1, int64_t d2, int64_t d3, int64_t s0, int64_t s1, int64_t s2, int b0, int b1) {
-  MapKey key{base, rank, {d0, d1, d2, d3}, {s0, s1, s2}, b0, b1};
+static pmb_status bf16_map(CUtensorMap* out, const MapKey& key) {
   std::lock_guard<std::mutex> lock(g_maps_mu);
   auto it = g_maps.find(key);
   if (it == g_maps.end()) {
     if (g_maps.size() > 8192) g_maps.clear();
     EncodeTiledFn enc = get_encode();
     if (!enc) return fail(PMB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    cuuint64_t dims[4] = {(cuuint64_t)d0, (cuuint64_t)d1, (cuuint64_t)d2, (cuuint64_t)d3};
-    cuuint64_t strides[3] = {(cuuint64_t)s0 * 2, (cuuint64_t)s1 * 2, (cuuint64_t)s2 * 2};
-    cuuint32_t box[4] = {(cuuint32_t)b0, (cuuint32_t)b1, 1, 1};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
+    cuuint64_t dims[5], strides[4];
+    cuuint32_t box[5], estr[5] = {1, 1, 1, 1, 1};
+    for (int i = 0; i < 5; ++i) { dims[i] = (cuuint64_t)key.d[i]; box[i] = (cuuint32_t)key.b[i]; if (i < 4) strides[i] = (cuuint64_t)key.s[i] * 2; }
     CUtensorMap m;
-    CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<uint16_t*>(base), dims, strides, box, estr,
+    CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)key.rank, const_cast<void*>(key.base), dims, strides, box, estr,
                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
-      return fail(PMB_ERR_CUDA, "cuTensorMapEncodeTiled (bf16, rank %d) failed with code %d (dims %lld %lld %lld %lld, pitches %lld %lld %lld)", rank, (int)r,
-                  (long long)d0, (long long)d1, (long long)d2, (long long)d3, (long long)s0, (long long)s1, (long long)s2);
+      return fail(PMB_ERR_CUDA, "cuTensorMapEncodeTiled (bf16, rank %d) failed with code %d (dims %lld %lld %lld %lld, pitches %lld %lld %lld)", key.rank, (int)r, (long long)key.d[0],
+                  (long long)key.d[1], (long long)key.d[2], (long long)key.d[3], (long long)key.s[0], (long long)key.s[1], (long long)key.s[2]);
     it = g_maps.emplace(key, m).first;
   }
   *out = it->second;
@@ -539,10 +538,13 @@ static pmb_status bf16_map(CUtensorMap* out, const uint16_t* base, int rank, int
 }
 // (a map's rank has to be the rank of the copies that use it)
 pmb_status bf16_map3(CUtensorMap* out, const uint16_t* base, int64_t d0, int64_t d1, int64_t d2, int64_t s0, int64_t s1, int b0, int b1) {
-  return bf16_map(out, base, 3, d0, d1, d2, 1, s0, s1, 0, b0, b1);
+  return bf16_map(out, MapKey{base, 3, {d0, d1, d2, 1, 1}, {s0, s1, 0, 0}, {b0, b1, 1, 1, 1}});
 }
 pmb_status bf16_map4(CUtensorMap* out, const uint16_t* base, int64_t d0, int64_t d1, int64_t d2, int64_t d3, int64_t s0, int64_t s1, int64_t s2, int b0, int b1) {
-  return bf16_map(out, base, 4, d0, d1, d2, d3, s0, s1, s2, b0, b1);
+  return bf16_map(out, MapKey{base, 4, {d0, d1, d2, d3, 1}, {s0, s1, s2, 0}, {b0, b1, 1, 1, 1}});
+}
+pmb_status bf16_map_rows8(CUtensorMap* out, const uint16_t* base, int64_t d0, int64_t tokens, int64_t H, int64_t pitch, int64_t head) {
+  return bf16_map(out, MapKey{base, 5, {d0, 8, tokens / 32, 4, H}, {pitch, 32 * pitch, 8 * pitch, head}, {64, 8, 4, 4, 1}});
 }
 
 static unsigned int* status_ptr() {

@@ -128,8 +128,9 @@ pmb_status read_clear_device_status_pairs(unsigned int* word);
 // ---- the other contractions of the scan on the same bf16 pairs (ssd_pairs.cu; shapes of ssd_fused_supported(pairs)):
 // states / dstates (per head), dG (summed over the heads of a group, decay mask folded in registers), dC / dB.
 pmb_status ssd_pairs_state(cudaStream_t st, const SsdIn& in, const SsdWs& ws, int mode);      // 0: chunk states, 1: d(states)
-int ssd_pairs_dg_nsplit(int B, int T, int H, int G, int Q);
-pmb_status ssd_pairs_dg(cudaStream_t st, const SsdIn& in, const SsdWs& ws, int nsplit);       // -> ws.dg_hi/lo (nsplit == 1) or ws.splitk partials
+// dG (ssd_dg.cu)
+int ssd_dg_nsplit(int B, int T, int H, int G, int Q);
+pmb_status ssd_dg(cudaStream_t st, const SsdIn& in, const SsdWs& ws, int nsplit);       // -> ws.dg_hi/lo (nsplit == 1) or ws.splitk partials
 int ssd_pairs_dbc_nsplit(int B, int T, int H, int N, int G, int Q);
 // mode 0: dC, 1: dB; `part` = where the head-split partial tiles go (nsplit * B * nc * G * Q * N floats)
 pmb_status ssd_pairs_dbc(cudaStream_t st, const SsdIn& in, const SsdWs& ws, int mode, float* out, int64_t ld, int nsplit, float* part);
@@ -140,6 +141,9 @@ pmb_status bf16_map3(CUtensorMap* out, const uint16_t* base, int64_t d0, int64_t
 // cached rank-4 bf16 tensor map of a token-major operand: dims (d0 contiguous, T tokens with pitch s0, d2 heads / groups
 // with pitch s1, B sequences with pitch s2), box (b0, b1, 1, 1).  A box that reaches past the end of a sequence (or past
 // d0) is filled with zeros there, never with the next sequence's rows.
+// cached map of 128 token rows (tokens a multiple of 32, 64 columns from 0) that a copy deals to a tile in groups of eight: tile row
+// 32 q + 8 i + r = token row 32 i + 8 q + r; coordinates (0, 0, first row / 32, 0, head)
+pmb_status bf16_map_rows8(CUtensorMap* out, const uint16_t* base, int64_t d0, int64_t tokens, int64_t H, int64_t pitch, int64_t head);
 pmb_status bf16_map4(CUtensorMap* out, const uint16_t* base, int64_t d0, int64_t T, int64_t d2, int64_t B, int64_t s0, int64_t s1, int64_t s2, int b0, int b1);
 }
 

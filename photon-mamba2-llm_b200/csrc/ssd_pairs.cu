@@ -1,8 +1,7 @@
-// The contractions of the chunked SSD scan other than the fused intra-chunk kernel, on bf16 pairs that their
+// The contractions of the chunked SSD scan other than the intra-chunk kernels and dG, on bf16 pairs that their
 // producers already wrote (pair_bgemm_kernel: TMA -> tensor core, no rescaling in shared memory):
 //   states[n,p]  = sum_q B[q,n] xs[q,p]           xs  = x dt exp(S_end - S_q)   (chunk-prepare kernel)
 //   dstate[n,p]  = sum_t C[t,n] dYs[t,p]          dYs = dY exp(S_t)             (gated-norm backward)
-//   dG[t,s]      = sum_{h in group} exp(S_h,t - S_h,s) [s<=t] sum_p dY_h[t,p] x~_h[s,p]
 //   dC[t,n]      = sum_{s<=t} dG[t,s] B[s,n] + sum_h sum_p dYs_h[t,p] h_prev_h[n,p]
 //   dB[s,n]      = sum_{t>=s} dG[t,s] C[t,n] + sum_h sum_p xs_h[s,p]  dh_h[n,p]
 // (mamba2/ssd_ops.rs:201-234 and its autograd compute the same quantities op by op.)
@@ -37,16 +36,10 @@ struct PP {
   uint16_t* dg_hi; uint16_t* dg_lo;
 };
 
-constexpr int MAX_Q = 1024;
-
 // ---- states (MODE 0) / dstates (MODE 1): maps 0 = B or C (MN-major: n contiguous, token rows), 1 = xs or dYs (MN-major)
 template <int NS_>
 struct PState {
   static constexpr int BN = 64, NS = NS_;
-  static constexpr bool SEG_EPI = false;
-  static constexpr int AUX_FLOATS = 0;
-  float* aux;
-  __device__ void stage(int, int) {}
   PP p; int Mdim, Ndim;
   int h, g, tok0; float* out;
   __device__ bool init(int batch, int, int) {
@@ -59,71 +52,10 @@ struct PState {
   __device__ void seg(int, int, int, int& kt0, int& kt1, int& am, int& bm, int& amn, int& bmn) const { kt0 = 0; kt1 = p.Q / 64; am = 0; bm = 1; amn = 1; bmn = 1; }
   __device__ void a_coord(int, int kt, int m0, int& c0, int& c1, int& c2) const { c0 = m0; c1 = tok0 + kt * 64; c2 = g; }
   __device__ void b_coord(int, int kt, int n0, int& c0, int& c1, int& c2) const { c0 = n0; c1 = tok0 + kt * 64; c2 = h; }
-  __device__ void seg_accumulate(int, int, int, const float (&)[32], float (&)[32]) const {}
-  __device__ void stage_seg(int, int, int) {}
   __device__ void store(int m, int nb, const float (&v)[32]) const {
     float4* dst = reinterpret_cast<float4*>(out + (int64_t)m * p.P + nb);
 #pragma unroll
     for (int j = 0; j < 8; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-  }
-};
-
-// ---- dG: one segment per head (K = d_head), folded with that head's decay mask in registers.
-// maps 0 = dY (K-major rows t), 1 = x~ (K-major rows s)
-template <int NS_>
-struct PDG {
-  static constexpr int BN = 128, NS = NS_;
-  static constexpr bool SEG_EPI = true;
-  static constexpr int AUX_FLOATS = 2 * MAX_Q;   // two halves of S (Q), one per segment in flight
-  float* aux;
-  __device__ void stage(int, int) {}
-  PP p; int Mdim, Ndim;
-  int bb, cc, g, split, tok0; int64_t obase;
-  __device__ void stage_seg(int s, int tid, int nthr) {
-    const int h = head_of(s);
-    float* dst = aux + (s & 1) * p.Q;
-    const float* sp = p.S + ((int64_t)bb * p.H + h) * p.T + (int64_t)cc * p.Q;
-    for (int q = tid; q < p.Q; q += nthr) dst[q] = sp[q];
-  }
-  __device__ bool init(int batch, int m0, int n0) {
-    if (n0 > m0 + pbg::BM - 1) return false;                  // above the diagonal
-    split = batch % p.nsplit; batch /= p.nsplit;
-    g = batch % p.G; const int bc = batch / p.G; cc = bc % p.nc; bb = bc / p.nc;
-    tok0 = bc * p.Q;
-    obase = (p.nsplit > 1 ? (int64_t)blockIdx.z : (int64_t)batch) * p.Q * p.Q;
-    return true;
-  }
-  __device__ int nseg() const { return (p.hpg - split + p.nsplit - 1) / p.nsplit; }
-  __device__ int head_of(int s) const { return g * p.hpg + split + s * p.nsplit; }
-  __device__ void seg(int, int, int, int& kt0, int& kt1, int& am, int& bm, int& amn, int& bmn) const { kt0 = 0; kt1 = p.P / 64; am = 0; bm = 1; amn = 0; bmn = 0; }
-  __device__ void a_coord(int s, int kt, int m0, int& c0, int& c1, int& c2) const { c0 = kt * 64; c1 = tok0 + m0; c2 = head_of(s); }
-  __device__ void b_coord(int s, int kt, int n0, int& c0, int& c1, int& c2) const { c0 = kt * 64; c1 = tok0 + n0; c2 = head_of(s); }
-  __device__ void seg_accumulate(int s, int m, int nb, const float (&v)[32], float (&acc)[32]) const {
-    if (m >= p.Q || nb > m) return;
-    const float* sv = aux + (s & 1) * p.Q;
-    const float sm = sv[m];
-#pragma unroll
-    for (int j = 0; j < 32; j += 4) {
-      const float4 s4 = *reinterpret_cast<const float4*>(sv + nb + j);
-      const float ss[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float w = (nb + j + e <= m) ? __expf(sm - ss[e]) : 0.0f;
-        acc[j + e] = fmaf(v[j + e], w, acc[j + e]);
-      }
-    }
-  }
-  __device__ void store(int m, int nb, const float (&v)[32]) const {
-    const int64_t o = obase + (int64_t)m * p.Q + nb;
-    if (p.nsplit > 1) {
-      float4* dst = reinterpret_cast<float4*>(p.part + o);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        store_pair4(p.dg_hi + o + 4 * j, NS == 2 ? p.dg_lo + o + 4 * j : nullptr, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-    }
   }
 };
 
@@ -132,10 +64,6 @@ struct PDG {
 template <int MODE, int NS_>
 struct PDBC {
   static constexpr int BN = 64, NS = NS_;
-  static constexpr bool SEG_EPI = false;
-  static constexpr int AUX_FLOATS = 0;
-  float* aux;
-  __device__ void stage(int, int) {}
   PP p; int Mdim, Ndim;
   int bb, cc, g, split, nh, tok0, dgrow0; float* pout;
   __device__ bool init(int batch, int, int) {
@@ -167,8 +95,6 @@ struct PDBC {
     if (split == 0 && s == 0) { c0 = n0; c1 = tok0 + kt * 64; c2 = g; }
     else { c0 = kt * 64; c1 = ((bb * p.nc + cc) * p.H + head_of(s)) * p.N + n0; c2 = 0; }
   }
-  __device__ void seg_accumulate(int, int, int, const float (&)[32], float (&)[32]) const {}
-  __device__ void stage_seg(int, int, int) {}
   __device__ void store(int m, int nb, const float (&v)[32]) const {
     float* base = p.nsplit > 1 ? pout + (int64_t)m * Ndim + nb : p.out + (int64_t)(tok0 + m) * p.ld + g * p.N + nb;
     float4* dst = reinterpret_cast<float4*>(base);
@@ -226,31 +152,13 @@ pmb_status ssd_pairs_state(cudaStream_t st, const SsdIn& in, const SsdWs& ws_in,
 
 // Head-split factor of a per-group contraction with `ctas` CTAs per split: as many splits as fit the machine in ONE wave
 // (one CTA more than that costs a second wave), then the fewest splits that give the same number of heads per CTA
-// (fewer partial tiles to write and add up).  The 128-wide dG tiles run one CTA per SM, the 64-wide ones two.
+// (fewer partial tiles to write and add up).
 static int pick_head_split(int64_t ctas, int hpg, int ctas_per_sm) {
   int want = (int)((ctas_per_sm * 148) / (ctas > 0 ? ctas : 1));
   if (want < 1) want = 1;
   if (want > hpg) want = hpg;
   const int per = (hpg + want - 1) / want;        // heads per CTA at that split
   return (hpg + per - 1) / per;
-}
-
-int ssd_pairs_dg_nsplit(int B, int T, int H, int G, int Q) {
-  const int nbcg = B * (T / Q) * G, hpg = H / G, qt = Q / pbg::BM;
-  return pick_head_split((int64_t)nbcg * (qt * (qt + 1) / 2), hpg, pbg::Geometry<PDG<2>::BN, 2>::CTAS_PER_SM);
-}
-
-pmb_status ssd_pairs_dg(cudaStream_t st, const SsdIn& in, const SsdWs& ws_in, int nsplit) {
-  const SsdWs ws = in.plain16 ? hi_only(ws_in) : ws_in;
-  PP p = make_pp(in, ws);
-  p.nsplit = nsplit;
-  const int64_t tok = (int64_t)p.B * p.T, hp = (int64_t)p.H * p.P;
-  MapSet ms{};
-  PMB_TRY(set_map(&ms, 0, ws.dy_hi, ws.dy_lo, p.P, tok, p.H, hp, p.P, 64, 128));
-  PMB_TRY(set_map(&ms, 1, ws.xt_hi, ws.xt_lo, p.P, tok, p.H, hp, p.P, 64, 128));
-  for (int i = 4; i < 8; ++i) ms.m[i] = ms.m[0];
-  if (!ws.dy_lo) return pbg::launch(st, ms, mk<PDG<1>>(p, p.Q, p.Q), p.B * p.nc * p.G * nsplit, status_ptr());
-  return pbg::launch(st, ms, mk<PDG<2>>(p, p.Q, p.Q), p.B * p.nc * p.G * nsplit, status_ptr());
 }
 
 int ssd_pairs_dbc_nsplit(int B, int T, int H, int N, int G, int Q) {
