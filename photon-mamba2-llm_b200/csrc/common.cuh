@@ -187,6 +187,16 @@ __device__ __forceinline__ float rcp_ge1(float d) {
   return d >= 8e37f ? 0.0f : r;
 }
 __device__ __forceinline__ float sigmoid_acc(float x) { return rcp_ge1(1.0f + expf(-x)); }
+// two fp32 values in one operation, each rounded as by the scalar one
+typedef unsigned long long F2;
+__device__ __forceinline__ F2 pack2(float a, float b) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float2 unpack2(F2 v) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v)); return r; }
+__device__ __forceinline__ F2 add2(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+__device__ __forceinline__ F2 neg2(F2 v) { return v ^ 0x8000000080000000ull; }
+// 2^x with results below 2^-126 as zero
+__device__ __forceinline__ float ex2_ftz(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
 // softplus in the reference's stable form max(x,0)+log(1+exp(-|x|)) (pm-candle ops_impl.rs:123-133)
 __device__ __forceinline__ float softplus_acc(float x) { return fmaxf(x, 0.0f) + log1pf(expf(-fabsf(x))); }
 
@@ -234,6 +244,14 @@ __device__ __forceinline__ void store_pair4(uint16_t* hi, uint16_t* lo, float a,
   const uint32_t h0 = bf16_of_two(a, b), h1 = bf16_of_two(c, d);
   *reinterpret_cast<uint2*>(hi) = make_uint2(h0, h1);
   if (lo) *reinterpret_cast<uint2*>(lo) = make_uint2(bf16_rest_of_two(a, b, h0), bf16_rest_of_two(c, d, h1));
+}
+// four consecutive floats as two pairs
+struct Quad { F2 a, b; };
+__device__ __forceinline__ Quad load_quad(const float* p) { const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p); return Quad{v.x, v.y}; }
+__device__ __forceinline__ void store_quad(float* p, const Quad& v) { *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v.a, v.b); }
+__device__ __forceinline__ void store_pair4(uint16_t* hi, uint16_t* lo, const Quad& v) {
+  const float2 a = unpack2(v.a), b = unpack2(v.b);
+  store_pair4(hi, lo, a.x, a.y, b.x, b.y);
 }
 
 }  // namespace pmb

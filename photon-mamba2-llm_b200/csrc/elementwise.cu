@@ -16,27 +16,37 @@ __global__ void column_sum_kernel(const float* __restrict__ partial, int64_t row
 // its rows): no thread is idle for any channel count that is a multiple of 32.
 // Measured at 8 x 2048 tokens of 1664 channels: forward 68 us with runs of 8 all requested up front, 49 with the next four rows in registers,
 // 41 now: they wait in shared memory (cp.async), which leaves room for more CTAs (eight rows 41, pairs of channels 42); at 8 x 1024 16.4 and 13.9;
-// backward 131 us, 110 with four channels per thread and the next four rows in registers (170 of them, three CTAs per SM), 82 now: two channels
-// (72 registers, seven CTAs), the next eight rows in shared memory (cp.async).  At 4 x 512 tokens 20.7 and 18.6 us, at 2 x 128 of 544 channels
-// 7.7 and 5.6.
+// backward (plain bf16 result) 131 us, 110 with four channels per thread and the next four rows in registers (170 of them, three CTAs per SM), 82 with
+// two channels and the next eight rows in shared memory, 57 now: that one was bound by issue (87 warp instructions per element in 79 % of the
+// issue slots), so four channels go as two pairs of packed fp32 operations, with the next four rows in shared memory (128 registers); its bytes
+// alone take 42.  At 8 x 1024 45 and 34, at 4 x 512 with a (hi, lo) result 24 and 19, at 2 x 128 of 544 channels 5.6 and 5.7.  Sigmoids stay
+// scalar: an exponential of pairs was faster but 12 % further from fp64, and its flipped roundings grew past what two builds agree to.
 // ---------------------------------------------------------------------------------------------
 constexpr int CONV_AHEAD = 4;
 constexpr int CONV_SLICES = 16;
 constexpr int CONV_STRIP_THREADS = CONV_SLICES * 8;
-// The backward's threads own two channels: 8 runs of 16 channel pairs to a CTA.
-constexpr int CONV_BWD_SLICES = 8, CONV_BWD_AHEAD = 8, CONV_BWD_SLOT = 2 * CONV_STRIP_THREADS * 8;      // (a slot: a row of both inputs)
 
 // Steps per run: 32 where that still gives eight CTAs per SM (the halo of K - 1 rows is then a tenth), else 16 or 8.
-static int conv_run(const Dims& d, int slices = CONV_SLICES) {
+static int conv_run(const Dims& d) {
   for (int run = 32; run > 8; run >>= 1)
-    if (cdiv(d.X, 32) * d.B * cdiv(d.T, slices * run) >= 148 * 8) return run;
+    if (cdiv(d.X, 32) * d.B * cdiv(d.T, CONV_SLICES * run) >= 148 * 8) return run;
   return 8;
+}
+
+// weights and bias of channels [c, c + 4), as two pairs
+template <int K>
+__device__ __forceinline__ void conv_weights(const float* __restrict__ w, const float* __restrict__ bias, int c, F2 (&wr)[2][K], F2 (&br)[2]) {
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    br[v] = bias ? pack2(bias[c + 2 * v], bias[c + 2 * v + 1]) : 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) wr[v][k] = pack2(w[(c + 2 * v) * K + k], w[(c + 2 * v + 1) * K + k]);
+  }
 }
 
 template <int VEC>
 __device__ __forceinline__ void conv_load(const float* p, float (&o)[VEC]) {
   if (VEC == 4) { const float4 q = *reinterpret_cast<const float4*>(p); o[0] = q.x; o[1 % VEC] = q.y; o[2 % VEC] = q.z; o[3 % VEC] = q.w; }
-  else if (VEC == 2) { const float2 q = *reinterpret_cast<const float2*>(p); o[0] = q.x; o[1 % VEC] = q.y; }
   else o[0] = *p;
 }
 
@@ -199,7 +209,7 @@ __device__ __forceinline__ void conv_bwd_thread(const float* __restrict__ xzd, i
                                                 const float* __restrict__ bias, const float* __restrict__ dact,
                                                 float* __restrict__ dxzd, int X, int T, uint16_t* __restrict__ pair_hi,
                                                 uint16_t* __restrict__ pair_lo, int c, int b, int t0, int t1,
-                                                float (&dwacc)[VEC][K], float (&dbacc)[VEC], uint32_t ring = 0) {
+                                                float (&dwacc)[VEC][K], float (&dbacc)[VEC]) {
   float wr[VEC][K], br[VEC];
 #pragma unroll
   for (int v = 0; v < VEC; ++v) {
@@ -229,25 +239,15 @@ __device__ __forceinline__ void conv_bwd_thread(const float* __restrict__ xzd, i
   // Walk t from t0 to t1-1+(K-1): du[t] is needed by dxbc[t-(K-1) .. t]; du beyond the sequence end is 0.
   const int tend = t1 + K - 1;
   const int tl = min(tend, T);                                 // rows that exist
-  // two channels: the next rows wait in slots of the thread's own in shared memory (cp.async, no barrier) and not in registers
-  constexpr bool STAGED = VEC == 2;
-  float xr[STAGED ? 1 : CONV_AHEAD][VEC], dr[STAGED ? 1 : CONV_AHEAD][VEC];
-  uint32_t slot = 0;
+  float xr[CONV_AHEAD][VEC], dr[CONV_AHEAD][VEC];
   const float* nx = src + (int64_t)t0 * ldx;
   const float* nd = dact + ((int64_t)b * T + t0) * X + c;
   auto request = [&](int t, int q) {
-    if (STAGED) {
-      if (t < tl) {
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(ring + slot), "l"(nx) : "memory");
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(ring + slot + CONV_STRIP_THREADS * 8), "l"(nd) : "memory");
-      }
-      asm volatile("cp.async.commit_group;" ::: "memory");
-      slot = slot + CONV_BWD_SLOT == CONV_BWD_AHEAD * CONV_BWD_SLOT ? 0u : slot + CONV_BWD_SLOT;
-    } else if (t < tl) { conv_load<VEC>(nx, xr[q]); conv_load<VEC>(nd, dr[q]); }
+    if (t < tl) { conv_load<VEC>(nx, xr[q]); conv_load<VEC>(nd, dr[q]); }
     nx += ldx; nd += X;
   };
 #pragma unroll
-  for (int q = 0; q < (STAGED ? CONV_BWD_AHEAD : CONV_AHEAD); ++q) request(t0 + q, q);
+  for (int q = 0; q < CONV_AHEAD; ++q) request(t0 + q, q);
   int64_t off = ((int64_t)b * T + t0 - (K - 1)) * ldx + col0 + c;      // of row t - (K - 1)
   for (int tb = t0; tb < tend; tb += CONV_AHEAD) {
 #pragma unroll
@@ -256,13 +256,8 @@ __device__ __forceinline__ void conv_bwd_thread(const float* __restrict__ xzd, i
       if (t >= tend) break;
       float xn[VEC], dn[VEC], g[VEC];
 #pragma unroll
-      for (int v = 0; v < VEC; ++v) { xn[v] = xr[STAGED ? 0 : q][v]; dn[v] = dr[STAGED ? 0 : q][v]; }
-      if (STAGED) {                                          // (the slot that is due is the one to request into)
-        asm volatile("cp.async.wait_group %0;" ::"n"(CONV_BWD_AHEAD - 1) : "memory");
-        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(xn[0]), "=f"(xn[1 % VEC]) : "r"(ring + slot) : "memory");
-        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(dn[0]), "=f"(dn[1 % VEC]) : "r"(ring + slot + CONV_STRIP_THREADS * 8) : "memory");
-      }
-      request(t + (STAGED ? CONV_BWD_AHEAD : CONV_AHEAD), q);
+      for (int v = 0; v < VEC; ++v) { xn[v] = xr[q][v]; dn[v] = dr[q][v]; }
+      request(t + CONV_AHEAD, q);
 #pragma unroll
       for (int v = 0; v < VEC; ++v) {
 #pragma unroll
@@ -290,14 +285,8 @@ __device__ __forceinline__ void conv_bwd_thread(const float* __restrict__ xzd, i
       if (t - (K - 1) >= t0) {
         if (pair_hi) {       // the gradient is only a GEMM operand: write it as a (hi, lo) bf16 pair with the same pitch
           if (VEC == 4) store_pair4(pair_hi + off, pair_lo ? pair_lo + off : nullptr, g[0], g[1 % VEC], g[2 % VEC], g[3 % VEC]);
-          else if (VEC == 2) {
-            uint32_t h0, l0, h1, l1;
-            split_bf16_pair(g[0], h0, l0); split_bf16_pair(g[1 % VEC], h1, l1);
-            *reinterpret_cast<uint32_t*>(pair_hi + off) = h0 | (h1 << 16);
-            if (pair_lo) *reinterpret_cast<uint32_t*>(pair_lo + off) = l0 | (l1 << 16);
-          } else { uint32_t h, l; split_bf16_pair(g[0], h, l); pair_hi[off] = (uint16_t)h; if (pair_lo) pair_lo[off] = (uint16_t)l; }
+          else { uint32_t h, l; split_bf16_pair(g[0], h, l); pair_hi[off] = (uint16_t)h; if (pair_lo) pair_lo[off] = (uint16_t)l; }
         } else if (VEC == 4) *reinterpret_cast<float4*>(dxzd + off) = make_float4(g[0], g[1 % VEC], g[2 % VEC], g[3 % VEC]);
-        else if (VEC == 2) *reinterpret_cast<float2*>(dxzd + off) = make_float2(g[0], g[1 % VEC]);
         else dxzd[off] = g[0];
       }
       off += ldx;
@@ -332,57 +321,127 @@ __global__ void __launch_bounds__(128) conv_silu_bwd_kernel(const float* __restr
   }
 }
 
-// The same work with the parameter-gradient partials summed inside the CTA: one partial row entry per channel and CTA instead of
-// one per thread, which at a few thousand tokens moved more partial sums than data.  Sums run in a fixed order (shuffles, then the
-// warps in order).
+// The same work on four channels as two pairs, up to four taps, with the parameter-gradient partials summed inside the CTA: one partial row
+// entry per channel and CTA instead of one per thread, which at a few thousand tokens moved more partial sums than data.  Sums run in a
+// fixed order (shuffles, then the warps in order).
 template <int K>
-__global__ void __launch_bounds__(CONV_STRIP_THREADS, 7) conv_silu_bwd_strip_kernel(const float* __restrict__ xzd, int64_t ldx, int col0,
+__global__ void __launch_bounds__(CONV_STRIP_THREADS, 4) conv_silu_bwd_strip_kernel(const float* __restrict__ xzd, int64_t ldx, int col0,
                                                                   const float* __restrict__ w, const float* __restrict__ bias,
                                                                   const float* __restrict__ dact, float* __restrict__ dxzd,
                                                                   float* __restrict__ partial, int X, int T, int run,
                                                                   uint16_t* __restrict__ pair_hi, uint16_t* __restrict__ pair_lo) {
   pdl_launch();
   pdl_wait();
-  constexpr int NV = 2 * K + 2, NW = CONV_STRIP_THREADS / 32;
-  __shared__ float red[NW][16][NV];
-  __shared__ __align__(16) uint8_t stage[CONV_BWD_AHEAD * CONV_BWD_SLOT];
-  const uint32_t ring = (uint32_t)__cvta_generic_to_shared(stage) + threadIdx.x * 8;
-  const int tx = threadIdx.x & 15, slice = threadIdx.x >> 4, warp = threadIdx.x >> 5;
-  const int c = (blockIdx.x * 16 + tx) * 2;
-  const int tblocks = (T + CONV_BWD_SLICES * run - 1) / (CONV_BWD_SLICES * run);
+  constexpr int NV = 4 * K + 4, NW = CONV_STRIP_THREADS / 32;
+  __shared__ float red[NW][8][NV];
+  __shared__ __align__(16) float4 stage[CONV_AHEAD][2][CONV_STRIP_THREADS];
+  const int tx = threadIdx.x & 7, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int c = (blockIdx.x * 8 + tx) * 4;
+  const int tblocks = (T + CONV_SLICES * run - 1) / (CONV_SLICES * run);
   const int b = blockIdx.y / tblocks;
-  const int t0 = (blockIdx.y % tblocks) * (CONV_BWD_SLICES * run) + slice * run;
-  float dwacc[2][K], dbacc[2];
+  const int t0 = (blockIdx.y % tblocks) * (CONV_SLICES * run) + (threadIdx.x >> 3) * run;
+  F2 dwacc[2][K], dbacc[2] = {0, 0};
+#pragma unroll
+  for (int k = 0; k < K; ++k) dwacc[0][k] = dwacc[1][k] = 0;
+  if (c < X && t0 < T) {
+    const int t1 = min(t0 + run, T), tend = t1 + K - 1, tl = min(tend, T);      // rows [t0, tl) are read: du[t] is needed by dxbc[t-(K-1) .. t]
+    F2 wr[2][K], br[2], xin[2][K], dus[2][K];                // xbc and du of [t-(K-1), t]
+    conv_weights<K>(w, bias, c, wr, br);
+    const float* src = xzd + (int64_t)b * T * ldx + col0 + c;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const int t = t0 - K + k;
+      const Quad v = k > 0 && t >= 0 ? load_quad(src + (int64_t)t * ldx) : Quad{0, 0};
+      xin[0][k] = v.a; xin[1][k] = v.b;
+      dus[0][k] = dus[1][k] = 0;
+    }
+    // the next rows wait in slots of the thread's own in shared memory (cp.async, no barrier) and not in registers
+    constexpr uint32_t HALF = CONV_STRIP_THREADS * 16, PITCH = 2 * HALF;
+    const uint32_t slots = (uint32_t)__cvta_generic_to_shared(&stage[0][0][threadIdx.x]);
+    const float *nx = src + (int64_t)t0 * ldx, *nd = dact + ((int64_t)b * T + t0) * X + c;
+    auto request = [&](int t, uint32_t slot) {
+      if (t < tl) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot), "l"(nx) : "memory");
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + HALF), "l"(nd) : "memory");
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      nx += ldx; nd += X;
+    };
+#pragma unroll
+    for (int q = 0; q < CONV_AHEAD; ++q) request(t0 + q, slots + q * PITCH);
+    int64_t off = ((int64_t)b * T + t0 - (K - 1)) * ldx + col0 + c;      // of row t - (K - 1)
+    const F2 one = pack2(1.0f, 1.0f), neg = pack2(-1.0f, -1.0f);
+    for (int tb = t0; tb < tend; tb += CONV_AHEAD) {
+#pragma unroll
+      for (int q = 0; q < CONV_AHEAD; ++q) {
+        const int t = tb + q;
+        if (t >= tend) break;
+        const uint32_t slot = slots + q * PITCH;              // (the slot that is due is the one to request into)
+        F2 xn[2], dn[2];
+        asm volatile("cp.async.wait_group %0;" ::"n"(CONV_AHEAD - 1) : "memory");
+        asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(xn[0]), "=l"(xn[1]) : "r"(slot) : "memory");
+        asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(dn[0]), "=l"(dn[1]) : "r"(slot + HALF) : "memory");
+        request(t + CONV_AHEAD, slot);
+        Quad g;
+        F2* const gv[2] = {&g.a, &g.b};
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+#pragma unroll
+          for (int k = 0; k < K - 1; ++k) { xin[v][k] = xin[v][k + 1]; dus[v][k] = dus[v][k + 1]; }
+          xin[v][K - 1] = xn[v];
+          F2 u = br[v];
+#pragma unroll
+          for (int k = 0; k < K; ++k) u = fma2(wr[v][k], xin[v][k], u);
+          const float2 uv = unpack2(u);
+          const F2 s = pack2(sigmoid_acc(uv.x), sigmoid_acc(uv.y));
+          F2 du = mul2(dn[v], fma2(mul2(u, s), fma2(s, neg, one), s));      // silu'(u) = s + u s (1 - s)
+          if (t >= T) du = 0;                                 // (rows past the end: what lies in the slot is an older row)
+          if (t < t1) {                                       // this run owns the parameter gradients' share of its own rows
+            dbacc[v] = add2(dbacc[v], du);
+#pragma unroll
+            for (int k = 0; k < K; ++k) dwacc[v][k] = fma2(du, xin[v][k], dwacc[v][k]);
+          }
+          dus[v][K - 1] = du;
+          F2 acc = 0;                                         // dxbc[tp] = sum_k w[k] du[tp + (K-1) - k]
+#pragma unroll
+          for (int k = 0; k < K; ++k) acc = fma2(wr[v][k], dus[v][K - 1 - k], acc);
+          *gv[v] = acc;
+        }
+        if (t - (K - 1) >= t0) {
+          if (pair_hi) store_pair4(pair_hi + off, pair_lo ? pair_lo + off : nullptr, g);      // the gradient is only a GEMM operand
+          else store_quad(dxzd + off, g);
+        }
+        off += ldx;
+      }
+    }
+  }
+  float vals[NV];                                             // [channel][tap], [channel]
 #pragma unroll
   for (int v = 0; v < 2; ++v) {
-    dbacc[v] = 0.0f;
 #pragma unroll
-    for (int k = 0; k < K; ++k) dwacc[v][k] = 0.0f;
-  }
-  if (c < X && t0 < T) conv_bwd_thread<K, 2>(xzd, ldx, col0, w, bias, dact, dxzd, X, T, pair_hi, pair_lo, c, b, t0, min(t0 + run, T), dwacc, dbacc, ring);
-  float vals[NV];
-#pragma unroll
-  for (int v = 0; v < 2; ++v) {
-#pragma unroll
-    for (int k = 0; k < K; ++k) vals[v * K + k] = dwacc[v][k];
-    vals[2 * K + v] = dbacc[v];
+    for (int k = 0; k < K; ++k) { const float2 d = unpack2(dwacc[v][k]); vals[2 * v * K + k] = d.x; vals[(2 * v + 1) * K + k] = d.y; }
+    const float2 d = unpack2(dbacc[v]);
+    vals[4 * K + 2 * v] = d.x; vals[4 * K + 2 * v + 1] = d.y;
   }
 #pragma unroll
-  for (int i = 0; i < NV; ++i) vals[i] += __shfl_xor_sync(0xffffffffu, vals[i], 16);      // the two time slices of a warp
-  if ((threadIdx.x & 31) < 16) {
+  for (int i = 0; i < NV; ++i) {                              // the four time slices of a warp
+    vals[i] += __shfl_xor_sync(0xffffffffu, vals[i], 16);
+    vals[i] += __shfl_xor_sync(0xffffffffu, vals[i], 8);
+  }
+  if (lane < 8) {
 #pragma unroll
     for (int i = 0; i < NV; ++i) red[warp][tx][i] = vals[i];
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < 16 * NV; e += CONV_STRIP_THREADS) {
+  for (int e = threadIdx.x; e < 8 * NV; e += CONV_STRIP_THREADS) {
     const int q = e / NV, i = e % NV;
-    const int cc = (blockIdx.x * 16 + q) * 2;
+    const int cc = (blockIdx.x * 8 + q) * 4;
     if (cc < X) {
       float tot = 0.0f;
 #pragma unroll
       for (int wv = 0; wv < NW; ++wv) tot += red[wv][q][i];
-      if (i < 2 * K) partial[(int64_t)blockIdx.y * X * K + (int64_t)cc * K + i] = tot;      // (cc + v) * K + k with i = v * K + k
-      else partial[(int64_t)gridDim.y * X * K + (int64_t)blockIdx.y * X + cc + (i - 2 * K)] = tot;
+      if (i < 4 * K) partial[(int64_t)blockIdx.y * X * K + (int64_t)cc * K + i] = tot;      // (cc + channel) * K + tap
+      else partial[(int64_t)gridDim.y * X * K + (int64_t)blockIdx.y * X + cc + (i - 4 * K)] = tot;
     }
   }
 }
@@ -393,7 +452,7 @@ size_t conv_bwd_ws_bytes(const Dims& d) {
 
 // Rows of `partial` the launch below writes (what column_sum has to add up).
 static int64_t conv_bwd_partial_rows(const Dims& d, bool strip) {
-  return strip ? (int64_t)d.B * cdiv(d.T, CONV_BWD_SLICES * conv_run(d, CONV_BWD_SLICES)) : (int64_t)d.B * cdiv(d.T, conv_run(d));
+  return (int64_t)d.B * cdiv(d.T, (strip ? CONV_SLICES : 1) * conv_run(d));
 }
 static bool conv_bwd_strip_ok(const Dims& d, const float* xzd, const float* dact, const float* dxzd) {
   return (d.X % 4 == 0) && (d.J % 4 == 0) && (d.I % 4 == 0) && d.K <= 4 &&
@@ -407,7 +466,7 @@ static pmb_status launch_conv_bwd_k(cudaStream_t st, const Dims& d, const float*
   bool vec = (d.X % 4 == 0) && (d.J % 4 == 0) && (d.I % 4 == 0) &&
              ((reinterpret_cast<uintptr_t>(xzd) | reinterpret_cast<uintptr_t>(dact) | reinterpret_cast<uintptr_t>(dxzd)) % 16 == 0);
   const unsigned rows = (unsigned)conv_bwd_partial_rows(d, strip);
-  const int run = strip ? conv_run(d, CONV_BWD_SLICES) : conv_run(d);
+  const int run = conv_run(d);
   if (strip) {
     if constexpr (K <= 4)
       PMB_TRY(launch_pdl(st, conv_silu_bwd_strip_kernel<K>, dim3((unsigned)cdiv(d.X, 32), rows), CONV_STRIP_THREADS, 0, xzd, d.J, d.I, w, b, dact, dxzd, partial, d.X, d.T, run, pair_hi, pair_lo));

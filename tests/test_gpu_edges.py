@@ -492,8 +492,8 @@ def test_gemm_pair_tiles_on_pairs(pm, M, N, K):
     assert_close(out, a.double() @ b.double(), tol=3e-5, what=f"{M}x{N}x{K}")
 
 
-# the conv's strips: 16 runs (backward 8) of 8, 16 or 32 steps to a CTA (130 and 240 sequences of 160 channels), four (two) channels per
-# thread, the next four (eight) rows in shared memory (the oracle's fp32 sums in another order: 1e-5 of the largest)
+# the conv's strips: 16 runs of 8, 16 or 32 steps to a CTA (130 and 240 sequences of 160 channels), four channels per
+# thread, the next four rows in shared memory (the oracle's fp32 sums in another order: 1e-5 of the largest)
 @pytest.mark.parametrize("K", [2, 3, 4])
 @pytest.mark.parametrize("B,T", [(1, 1), (2, 7), (1, 8), (1, 63), (2, 65), (3, 300), (40, 260), (130, 260), (240, 260)])
 @pytest.mark.parametrize("H,P,N", [(4, 4, 4), (4, 16, 8), (8, 16, 16)])
