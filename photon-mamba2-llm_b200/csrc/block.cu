@@ -193,8 +193,12 @@ static ChainArgs chain_inputs(const Dims& d, const pmb_block_params& p, const fl
   return a;
 }
 
+// counters of the chain kernel's hand-overs, which the conv kernel in front of it clears
+static uint32_t* chain_flags(const Dims& d, float* seg) { return (int64_t)d.B * d.H > CHAIN_SMS ? ssd_chain_flags(seg, d.P, d.N) : nullptr; }
+
 // bf16-storage blocks on whole chunks: plain bf16 operands, and few long sequences scanned chunk by chunk instead of as chains, which are
-// not cut into segments here (that is built for S and states by steps, not by chunks of two, and would round other sums).  What a chain's steps take, one
+// not cut into segments here (that is built for S and states by steps, not by chunks of two, and would round other sums; more chains than SMs
+// share them in stretches of whole chunks, same sums).  What a chain's steps take, one
 // after the other, beyond a fixed cost, against the chunk-by-chunk kernels' time per step of a head; where a backward follows, the chain also
 // writes what that reads.  Fitted to 130 shapes of 8 to 32 heads, 512 to 8192 tokens: the slower side is taken by at most 1.3 % of a block's
 // forward and 0.6 % of its backward.  us, chains / chunk by chunk: forward 1 x 1024 tokens, 8 heads 53 / 46, 32 heads 70 / 75; 1 x 2048,
@@ -245,6 +249,7 @@ static pmb_status block_fwd_core(cudaStream_t st, const Dims& d, const pmb_block
   if (w.ssd.bc_hi) bc = ConvPairOut{w.ssd.bc_hi, w16 ? nullptr : w.ssd.bc_lo, d.I, 2 * d.G * d.N};
   const bool chain = block_uses_chain_bwd(d, w16 != nullptr);
   if (chain) bc.lo = w.ssd.bc_lo;
+  else if (block_plain16(d, w16 != nullptr)) bc.clear = chain_flags(d, w.seg);
   PMB_TRY(conv_silu_dt_fwd(st, d, w.xzd, p.conv1d_weight, p.conv1d_bias, p.dt_bias, w.act, nullptr, w.ssd.bc_hi ? &bc : nullptr));
   SsdIn sin = ssd_inputs(d, p, w, w16 != nullptr);
   if (chain) {
@@ -254,7 +259,7 @@ static pmb_status block_fwd_core(cudaStream_t st, const Dims& d, const pmb_block
   } else if (block_plain16(d, w16 != nullptr) && bc.hi && ssd_chain_enabled() && !scan_by_chunks(d, true, true)) {
     // the backward reads S, the states, x~, xs and the carried part of y: the chain leaves them on its way
     ChainArgs a = chain_inputs(d, p, w.xzd, w.act, w.ssd.bc_hi, nullptr, w.y);
-    a.blocks = d.Q / SCAN_STEP;
+    a.blocks = d.Q / SCAN_STEP; a.seg = w.seg; a.flags_clear = bc.clear;
     a.S_out = w.ssd.S; a.dt_out = w.dt; a.A_out = w.Aneg; a.hp_hi = w.ssd.hp_hi; a.hprev = w.ssd.hprev; a.xt = w.ssd.xt_hi; a.xs = w.ssd.xs_hi;
     PMB_TRY(ssd_chain_fwd(st, a));
   } else {
@@ -319,12 +324,12 @@ pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, 
       PMB_TRY(gemm_pairs(st, 0, 0, d.M, d.J, d.D, Pair16{f.x_hi, f.x_lo, d.D}, win, f.xzd, d.J, nullptr));
     }
     else PMB_TRY(gemm(st, 0, 0, d.M, d.J, d.D, static_cast<const float*>(x), d.D, p.in_proj_weight, d.J, f.xzd, d.J, nullptr, 0));
-    ConvPairOut bc{f.bc_hi, f.bc_lo, d.I, 2 * d.G * d.N};
+    ConvPairOut bc{f.bc_hi, f.bc_lo, d.I, 2 * d.G * d.N, plain ? chain_flags(d, f.seg) : nullptr};
     PMB_TRY(conv_silu_dt_fwd(st, d, f.xzd, p.conv1d_weight, p.conv1d_bias, p.dt_bias, f.act, nullptr, &bc));
     if (!bc.hi) PMB_TRY(split_pair16_strided(st, f.act + d.I, d.M, 2 * d.G * d.N, d.X, f.bc_hi, f.bc_lo, 2 * d.G * d.N));
     ChainArgs a = chain_inputs(d, p, f.xzd, f.act, f.bc_hi, f.bc_lo, f.y);
     a.blocks = plain ? d.Q / SCAN_STEP : 1;
-    if (!plain) a.seg = f.seg;
+    a.seg = f.seg; a.flags_clear = bc.clear && bc.hi;
     PMB_TRY(ssd_chain_fwd(st, a));
     PMB_TRY(gated_rmsnorm_fwd(st, d.M, d.I, d.eps, f.y, f.xzd, d.J, p.norm_weight, f.normed, f.rstd, f.normed_hi, f.normed_lo));
     w.normed16 = f.normed_hi; w.normed_hi = f.normed_hi; w.normed_lo = f.normed_lo; w.normed = f.normed; w.x_hi = f.x_hi; w.x_lo = f.x_lo;

@@ -129,6 +129,8 @@ __global__ void __launch_bounds__(CONV_STRIP_THREADS) conv_silu_fwd_strip_kernel
   pdl_launch();
   pdl_wait();
   __shared__ __align__(16) float4 rows[CONV_AHEAD][CONV_STRIP_THREADS];
+  if (po.clear && blockIdx.x == 0 && blockIdx.y == 0)
+    for (int i = threadIdx.x; i < CONV_CLEAR_WORDS; i += CONV_STRIP_THREADS) po.clear[i] = 0;
   const int c = (blockIdx.x * 8 + (threadIdx.x & 7)) * 4;
   const int tblocks = (T + CONV_SLICES * run - 1) / (CONV_SLICES * run);
   const int b = blockIdx.y / tblocks, t0 = (blockIdx.y % tblocks) * (CONV_SLICES * run) + (threadIdx.x >> 3) * run;

@@ -18,7 +18,9 @@ pmb_status order_after(cudaStream_t from, cudaEvent_t ev, cudaStream_t to);
 // ---- elementwise.cu
 // optional second output of the conv forward: columns [col0, col0 + width) of `act` (the B | C columns) as a (hi, lo)
 // bf16 pair with row pitch `width`.  Written only by the vector kernel; `hi` is reset to NULL when it was not.
-struct ConvPairOut { uint16_t* hi = nullptr; uint16_t* lo = nullptr; int col0 = 0; int width = 0; };
+// The same kernel sets the CONV_CLEAR_WORDS words at `clear` to zero, for the kernel behind it.
+struct ConvPairOut { uint16_t* hi = nullptr; uint16_t* lo = nullptr; int col0 = 0; int width = 0; uint32_t* clear = nullptr; };
+constexpr int CONV_CLEAR_WORDS = 160;
 pmb_status conv_silu_dt_fwd(cudaStream_t st, const Dims& d, const float* xzd, const float* w, const float* b,
                             const float* dt_bias, float* act, float* dt, ConvPairOut* pair = nullptr);
 size_t conv_bwd_ws_bytes(const Dims& d);

@@ -31,15 +31,17 @@
 //  - the kernel's 63 KB are about what the instruction cache holds for seven roles: an early return and a few selects by block, 72 KB, cost 8 %;
 //  - the segment is the grid's y and not a remainder that stays in a register: on pairs its spills cost 10 % (24.6 -> 22.2 us at 4 x 512).
 // Measured at 24 heads of 64 x 64: 22 us for 4 x 512 tokens on pairs, 25 with what a backward reads (23.9 and 26 before the above); 8 x 2048 on
-// plain operands in chunks of 256, 119 us, and 166 with all that a chunk-by-chunk backward reads (their mean 188); 31 us (two launches over
-// segments) for 1 x 1337 on pairs.  Every mbarrier wait is bounded; on expiry the CTA raises the status
+// plain operands in chunks of 256, 100 us, and 117 with all that a chunk-by-chunk backward reads (118 and 144 where every CTA walks whole chains, see
+// ssd_chain_wrap); 31 us (two launches over segments) for 1 x 1337 on pairs.  Every mbarrier wait is bounded; on expiry the CTA raises the status
 // word, every role stops issuing work, copies in flight are waited for (bounded) and TMEM is freed on the way out.
 #include <cuda_bf16.h>
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 #include "tc_common.cuh"
 #include "kernels.h"
 #include "ssd_fused.h"
+#include "ssd_wrap.cuh"
 
 namespace pmb {
 
@@ -116,11 +118,12 @@ struct Params {
   int late;                                              // needs nothing from the kernel before, which lets this one in after its own wait: waits when it is done
   int state_only;                                        // first of two passes over segments: only seg_h and seg_d are formed
   float *seg_h, *seg_d;                                  // (B*H-whole,nseg-1,N,P), (B*H-whole,nseg-1): state that a segment leaves when it starts from none, decay over it (nobody reads the last one's)
+  uint32_t* flags;                                       // equal stretches of all chains: seg_h (CHAIN_SMS,N,P) and flags are the hand-overs
   unsigned int* status;
 };
 
-template <int NI, int ND, int NK, int NB, bool XIN16>
-__global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid_constant__ Maps maps, const Params p) {
+template <int NI, int ND, int NK, int NB, bool XIN16, bool WRAP>
+__global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ ChainWrap wr, const Params p) {
   using GE = Geo<NI, ND, NK, NB, XIN16>;
   constexpr bool FACT = GE::FACT;
   constexpr int STG = GE::STG, XB = GE::XB, NSB = GE::NSB, OUTW = GE::OUTW, XFW = GE::XFW, XF_THREADS = GE::XF_THREADS, W_XF = W_OUT + OUTW;
@@ -144,13 +147,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   float* sdt = sS + NSB * GE::SLOT;                                 // BIG: dt alone, the last kilobyte is not there
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int bh = p.first + (int)blockIdx.x, seg = (int)blockIdx.y;
+  const int state_only = WRAP ? 0 : p.state_only;
+  int bh = p.first + (int)blockIdx.x, i0 = (int)blockIdx.y * p.per, n = min(p.per, p.nsteps - i0);      // chain, first step and steps of this CTA
+  if (WRAP) {
+    const ChainItem it = chain_item(wr, (int)blockIdx.x, p.nsteps / NB);
+    bh = __shfl_sync(0xffffffffu, it.chain, 0); i0 = __shfl_sync(0xffffffffu, NB * it.from, 0); n = __shfl_sync(0xffffffffu, NB * it.count, 0);      // (uniform to the compiler, as the warp index)
+    if (n <= 0) return;
+  }
+  const int seg = WRAP ? 0 : (int)blockIdx.y;
   const int h = bh % p.H, bb = bh / p.H, g = h / p.hpg;
-  const int i0 = seg * p.per, toff = i0 * L;               // first step and token of this CTA's segment
-  const int n = min(p.per, p.nsteps - i0);
+  const int toff = i0 * L;                                 // first token
   const int64_t tokb = (int64_t)bb * p.T;
   if (threadIdx.x == 0) {
-    const int mmas = p.state_only ? 1 : 2;                  // warps that issue products
+    const int mmas = state_only ? 1 : 2;                  // warps that issue products
     for (int i = 0; i < 2; ++i) {
       mbar_init(bar(FULL + i), 1); mbar_init(bar(EMPTY + i), mmas);
       mbar_init(bar(XIN + i), 1); mbar_init(bar(XRDY + i), XFW); mbar_init(bar(XFREE + i), mmas + (p.store_ops ? 1 : 0));
@@ -171,7 +180,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  if (!p.late) pdl_wait();
+  if (WRAP || !p.late) pdl_wait();
   pdl_launch();
   const uint32_t tG = tmem, tA1 = tmem + 256, tA2 = tmem + 320, tU = tmem + 384;
 
@@ -194,14 +203,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       for (int i = 0; i < n; ++i) {
         const int s = i % STG;
         if (!wait(EMPTY + s, (uint32_t)(i / STG) ^ 1u, 1u)) break;
-        mbar_expect_tx(bar(FULL + s), p.state_only ? GE::BT : GE::STAGE);
+        mbar_expect_tx(bar(FULL + s), state_only ? GE::BT : GE::STAGE);
         const uint32_t dst = ring_s + s * GE::STAGE;
 #pragma unroll
         for (int sp = 0; sp < NI; ++sp)
 #pragma unroll
           for (int kt = 0; kt < NK; ++kt) {
             tma_load_4d(dst + (sp * NK + kt) * T128, &maps.b[sp], 64 * kt, toff + i * L, g, bb, bar(FULL + s));
-            if (!p.state_only) tma_load_4d(dst + GE::BT + (sp * NK + kt) * T128, &maps.c[sp], 64 * kt, toff + i * L, g, bb, bar(FULL + s));
+            if (!state_only) tma_load_4d(dst + GE::BT + (sp * NK + kt) * T128, &maps.c[sp], 64 * kt, toff + i * L, g, bb, bar(FULL + s));
           }
         issued = i + 1;
         if (XIN16) {                                         // bf16 x is the operand tile x~ as it is
@@ -257,7 +266,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       __syncwarp();
       return true;
     };
-    bool ok = !p.state_only && mma_g(0, 0, 0);
+    bool ok = !state_only && mma_g(0, 0, 0);
     int m = 0;                                               // item: (block, column block), the diagonal one last
 #pragma unroll 1
     for (int k = 0; k < n && ok; ++k) {
@@ -333,13 +342,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
           }
           if (rb == NB - 1 || k + 1 == n) umma_commit(bar(UFULL));
           umma_commit(bar(XFREE + xb));
-          if (XB == 1 || p.state_only) umma_commit(bar(EMPTY + s));
+          if (XB == 1 || state_only) umma_commit(bar(EMPTY + s));
         }
         __syncwarp();
         return true;
       };
       // (two buffers of x: xs has been there for a while, and the state's chain does not wait for C h; one: xs is being formed)
-      ok = p.state_only ? update() : XB == 2 ? update() && carried() : carried() && update();
+      ok = state_only ? update() : XB == 2 ? update() && carried() : carried() && update();
     }
   }
   } else if (warp < W_OUT) {
@@ -347,7 +356,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     if (NI == 2) regs_dec<64>();
     const int quarter = warp & 3, grp = (warp - W_MASK) >> 2, r_local = quarter * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-    bool ok = !p.state_only;
+    bool ok = !state_only;
     int k = 0, rb = 0, kc = 0;                              // this item: block k = block rb of its chunk, column block kc
 #pragma unroll 1
     for (int m = 0; k < n && ok; ++m) {
@@ -409,7 +418,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     // fragments of 16 rows x 8 columns (a quad of lanes holds 8 columns of a row: whole 32-byte sectors per store): this thread's
     // output rows are er + {0, 8, 16, 24}
     const int er = quarter * 32 + (lane >> 2), cw = 32 * grp, col = h * p.P + cw + (lane & 3) * 2;
-    bool ok = !p.state_only;
+    bool ok = !state_only;
 #pragma unroll 1
     for (int k = 0; k < n && ok; ++k) {
       const int c = k / NB;
@@ -582,8 +591,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
             if (GE::BIG) sdt[q] = dtv[u]; else sfac[q] = make_float2(dtv[u], __expf(send - v[u]));
             if (q == NB * L - 1) sEnd[c & 3] = send;
             if (t < p.T) {
-              if (p.S_out && !p.state_only) p.S_out[((int64_t)bb * p.H + h) * p.T + t] = v[u];
-              if (p.dt_out && !p.state_only) p.dt_out[(tokb + t) * p.H + h] = dtv[u];
+              if (p.S_out && !state_only) p.S_out[((int64_t)bb * p.H + h) * p.T + t] = v[u];
+              if (p.dt_out && !state_only) p.dt_out[(tokb + t) * p.H + h] = dtv[u];
             }
           }
         }
@@ -651,13 +660,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     const bool tile = quarter * 32 < 64 * NK;               // this warp's rows exist in the operand tile
     const int64_t NP = (int64_t)p.N * p.P;
     float hv[PW];
+    bool ok = true;
+    const float* enters = p.init && !state_only ? p.init + ((int64_t)bb * p.H + h) * NP : nullptr;
+    if (WRAP && i0 > 0) {                                   // the rest of a chain: the state comes from the CTA that walked its beginning
+      const int from = wr.e[blockIdx.x % CHAIN_SMS].sm;
+      ok = chain_take(p.flags + from, abort_flag);
+      if (!ok) give_up(8192u);
+      enters = p.seg_h + (int64_t)from * NP;
+    }
 #pragma unroll
     for (int q = 0; q < PW / 4; ++q) {
       float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      if (p.init && !p.state_only && active && 4 * q < p.P) v = *reinterpret_cast<const float4*>(p.init + ((int64_t)bb * p.H + h) * NP + (int64_t)nr * p.P + 4 * q);
+      if (enters && active && 4 * q < p.P) v = __ldcg(reinterpret_cast<const float4*>(enters + (int64_t)nr * p.P + 4 * q));
       hv[4 * q] = v.x; hv[4 * q + 1] = v.y; hv[4 * q + 2] = v.z; hv[4 * q + 3] = v.w;
     }
-    if (!p.state_only && active)
+    if (!WRAP && !state_only && active)
       for (int j = 0; j < seg; ++j) {                       // what the segments before this one leave
         const int64_t row = (int64_t)(bh - p.first) * (p.nseg - 1) + j;
         const float* F = p.seg_h + row * NP + (int64_t)nr * p.P;
@@ -671,14 +688,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
           if (q % 4 == 3) asm volatile("" ::: "memory");      // (no more than four loads in flight: registers)
         }
       }
-    bool ok = true;
     float stot = 0.0f;
     const int nch = (n + NB - 1) / NB, ncht = (p.nsteps + NB - 1) / NB;
     for (int i = 0; i < nch && ok; ++i) {                   // chunk after chunk
-      if (i > 0 && !p.state_only) ok = __all_sync(0xffffffffu, wait(HFREE, (uint32_t)(i - 1), 256u));
+      if (i > 0 && !state_only) ok = __all_sync(0xffffffffu, wait(HFREE, (uint32_t)(i - 1), 256u));
       if (!ok) break;
       const int64_t so = (((int64_t)bb * ncht + i0 / NB + i) * p.H + h) * NP + (int64_t)nr * p.P;
-      if (tile && !p.state_only) {
+      if (tile && !state_only) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {                       // eight 16-byte chunks of the row
           uint32_t hi[4], lo[4] = {0u, 0u, 0u, 0u};
@@ -693,7 +709,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(HRDY));
       // (what a backward keeps goes out after the operand tile, under the products that read it)
-      if (p.hp_hi && active && !p.state_only) {
+      if (p.hp_hi && active && !state_only) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           if (8 * c >= p.P) continue;
@@ -729,14 +745,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       if (lane == 0) mbar_arrive(bar(UFREE));
     }
     const int64_t row = (int64_t)blockIdx.x * gridDim.y + blockIdx.y;
-    if (ok && p.state_only && nr == 0) p.seg_d[row] = __expf(stot);
-    float* const leave = p.state_only ? p.seg_h + row * NP : p.last && seg + 1 == p.nseg ? p.last + (int64_t)bh * NP : nullptr;
+    if (ok && state_only && nr == 0) p.seg_d[row] = __expf(stot);
+    const bool handed = WRAP && i0 + n < p.nsteps;      // the beginning of a chain whose rest another CTA walks
+    const int to = handed ? wr.e[blockIdx.x % CHAIN_SMS].sm + 1 : 0;
+    float* const leave = state_only ? p.seg_h + row * NP : handed ? p.seg_h + to * NP : p.last && (WRAP || seg + 1 == p.nseg) ? p.last + (int64_t)bh * NP : nullptr;
     if (ok && leave && active) {
       float* dst = leave + (int64_t)nr * p.P;
 #pragma unroll
       for (int q = 0; q < PW / 4; ++q)
         if (4 * q < p.P) *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
     }
+    if (ok && handed) chain_hand_over(p.flags + to);
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -744,7 +763,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
   }
-  if (p.late) pdl_wait();                                  // (a kernel completes after those before it)
+  if (!WRAP && p.late) pdl_wait();                                  // (a kernel completes after those before it)
 }
 
 // ---- host side -------------------------------------------------------------------------------------------
@@ -779,11 +798,21 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
   }
   p.hp_hi = a.hp_hi; p.hp_lo = a.hp_lo; p.last = a.last; p.status = status_ptr();
   const int chains = a.B * a.H;
-  const ChainPlan plan = NB == 1 && a.seg ? ssd_chain_plan(a.B, a.T, a.H) : ChainPlan{chains, 1, p.nsteps};
+  ChainWrap wr{};
+  if constexpr (NI == 1 && !XIN16) {
+    if (a.seg && p.nsteps % NB == 0 && ssd_chain_wrap(chains, p.nsteps / NB, NB, 1.0 / 7.0, &wr)) {
+      p.seg_h = a.seg; p.flags = ssd_chain_flags(a.seg, a.P, a.N); p.store_ops = keep != nullptr;
+      if (!a.flags_clear) PMB_CUDA(cudaMemsetAsync(p.flags, 0, CHAIN_FLAG_BYTES, st));
+      PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16, true>);
+      return launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16, true>, dim3((unsigned)(wr.rounds * CHAIN_SMS)), NTHREADS, GE::SMEM, ms, wr, p);
+    }
+  }
+  // (storage blocks on plain operands keep the sums of one chain, see FACT)
+  const ChainPlan plan = (NI == 2 || XIN16) && a.seg ? ssd_chain_plan(a.B, a.T, a.H) : ChainPlan{chains, 1, p.nsteps};
   const unsigned cut = (unsigned)((chains - plan.whole) * plan.nseg);      // blocks of segments
   if (cut) { p.seg_h = a.seg; p.seg_d = a.seg + (size_t)cut * a.N * a.P; }
-  PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>);
-  auto run = [&](int count, int segments) { return launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16>, dim3((unsigned)count, (unsigned)segments), NTHREADS, GE::SMEM, ms, p); };
+  PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16, false>);
+  auto run = [&](int count, int segments) { return launch_pdl(st, ssd_chain_fwd_kernel<NI, ND, NK, NB, XIN16, false>, dim3((unsigned)count, (unsigned)segments), NTHREADS, GE::SMEM, ms, wr, p); };
   // the segments' states, the segments, and beside both the chains in one piece
   if (cut) {
     p.first = plan.whole; p.nseg = plan.nseg; p.per = plan.per;
@@ -820,7 +849,50 @@ ChainPlan ssd_chain_plan(int B, int T, int H) {
 }
 size_t ssd_chain_seg_floats(int B, int T, int H, int P, int N) {
   const ChainPlan plan = ssd_chain_plan(B, T, H);
-  return plan.nseg > 1 ? ((size_t)B * H - plan.whole) * plan.nseg * ((size_t)N * P + 1) : 0;
+  const size_t cut = plan.nseg > 1 ? ((size_t)B * H - plan.whole) * plan.nseg * ((size_t)N * P + 1) : 0;
+  const size_t wrap = (int64_t)B * H > CHAIN_SMS ? (size_t)CHAIN_SMS * N * P + CHAIN_FLAG_BYTES / sizeof(float) : 0;
+  return cut > wrap ? cut : wrap;
+}
+
+// Chains that fill the SMs a number of times and a bit (192 or 512 of them on 148) leave most SMs idle in the last round.  All their steps laid end to
+// end are cut into 148 equal stretches instead: a chain that lies across a cut begins on one SM and ends on the next, which gets the state in
+// fp32 through memory and so computes the same bits.  An SM walks the beginning of the chain that its stretch ends in FIRST, then its whole
+// chains, then the rest of the chain that its stretch begins in: that one was begun when the launch did, on another SM, and has its state there
+// before this SM comes to it, because a stretch is at least as long as a chain (McNaughton, Management Science 6(1), 1959).  The items are
+// blocks of one launch in the order of their starts, which blocks are placed in; a block waits only for one of the first CHAIN_SMS.
+// An item costs the kernel's filling and draining, two to three steps, which the blocks of a grid that is not cut pay less often.  Same bits, us:
+// the forward of a bf16 block in chunks of 256, 24 heads of 64 x 64, 8 x 1024 tokens 191 -> 184, 8 x 2048 345 -> 320, 7 x 2048 342 -> 304, 32 heads
+// 10 x 1024 296 -> 280, but 8 x 2048 412 -> 421 (an eighth of the steps saved); the scan's backward on bf16 inputs, 32 heads of 128 x 64, 16 x 8192
+// 1927 -> 1750, 5 x 2048 207 -> 194, 8 x 4096 523 -> 485 (an eighth), 30 x 640 of 64 x 64 308 -> 301 (a 17th).  The forward on bf16 inputs, whose
+// steps are shorter, lost as often as it gained (16 x 8192 724 -> 744, 7 x 1024 58 -> 68, 8 x 2048 of 64 x 64 92 -> 92): it stays uncut.
+bool ssd_chain_wrap(int64_t chains, int units, int steps_per_unit, double least_share, ChainWrap* w) {
+  const int64_t total = chains * units, uncut = cdiv(chains, CHAIN_SMS) * units, saved = uncut - cdiv(total, CHAIN_SMS);
+  if (chains <= CHAIN_SMS || chains > 0xffff || units < 2 || units > 0xffff) return false;
+  if (saved * steps_per_unit < 2 || (double)saved < least_share * (double)uncut) return false;
+  auto cut = [&](int j) { return j * total / CHAIN_SMS; };
+  auto wholes = [&](int j) { return (int)(cut(j + 1) / units - cdiv(cut(j), units)); };      // one of two numbers
+  int order[CHAIN_SMS], given[CHAIN_SMS] = {}, place = 0;
+  w->wholes = wholes(0);
+  for (int j = 0; j < CHAIN_SMS; ++j) { order[j] = j; w->wholes = std::min(w->wholes, wholes(j)); }
+  std::stable_sort(order, order + CHAIN_SMS, [&](int a, int b) { return cut(a + 1) % units < cut(b + 1) % units; });
+  // Chains are numbered in the order of their starts, so that those under way at a time are neighbours and find B and C of their sequence in L2
+  // (numbered along the stretches, 16 x 8192 tokens of 32 heads of 128 x 64 took 797 us forward instead of 694 uncut)
+  for (int s = 0; s < CHAIN_SMS; ++s) {
+    ChainWrap::Entry& e = w->e[s];
+    const int j = order[s];
+    e.sm = (uint16_t)j; e.head_units = (uint16_t)(cut(j + 1) % units); e.tail_from = (uint16_t)(cut(j) % units); e.head = e.extra = e.tail = 0;
+    if (e.head_units) given[j + 1] = e.head = (uint16_t)place++;
+  }
+  w->first_whole = place;
+  place += w->wholes * CHAIN_SMS;
+  w->rounds = 0;
+  for (int s = 0; s < CHAIN_SMS; ++s) {
+    ChainWrap::Entry& e = w->e[s];
+    if (wholes(e.sm) > w->wholes) e.extra = (uint16_t)place++;
+    if (e.tail_from) e.tail = (uint16_t)given[e.sm];
+    w->rounds = std::max(w->rounds, 1 + w->wholes + (e.extra > 0) + (e.tail_from > 0));
+  }
+  return true;
 }
 
 pmb_status ssd_chain_fwd(cudaStream_t st, const ChainArgs& a) {
@@ -831,7 +903,7 @@ pmb_status ssd_chain_fwd(cudaStream_t st, const ChainArgs& a) {
   if (!al16(a.x) || !al16(a.x16) || !al16(a.y) || !al16(a.y16) || !al16(a.init) || (a.ldx & (a.x16 ? 7 : 3)) || (a.ldy & 3))
     return fail(PMB_ERR_SHAPE, "ssd_chain: x, y and state rows must be 16-byte aligned");
   if (!pairs && !a.x16 && a.N > 64) return fail(PMB_ERR_UNSUPPORTED, "ssd_chain: fp32 x with plain bf16 B and C takes d_state up to 64");
-  if ((a.hprev || a.xt) && (pairs || a.x16 || a.seg || (a.xt != nullptr) != (a.xs != nullptr))) return fail(PMB_ERR_ARG, "ssd_chain: the chunk outputs go with fp32 x on plain operands");
+  if ((a.hprev || a.xt) && (pairs || a.x16 || (a.xt != nullptr) != (a.xs != nullptr))) return fail(PMB_ERR_ARG, "ssd_chain: the chunk outputs go with fp32 x on plain operands");
   const double tok = (double)a.B * a.T;
   // G and the masked product over the causal half of a step, the state update and the carried-state product
   ProfScope prof(st, "ssd_chain_fwd", tok * a.H * ((double)SCAN_STEP * (a.N + a.P) + 4.0 * a.N * a.P), 0.0);

@@ -27,12 +27,14 @@
 // prefetched into registers (50 us for 4 x 512 tokens, 24 heads of 64 x 64, on pairs) or read again by the output (49).
 // Measured at 24 heads of 64 x 64 on pairs: 45 us for 4 x 512 tokens (the d(states) product, reverse pass, masked product and row
 // kernel it replaces: 118 us), 31 us for 2 x 384, 53 us in segments for 2 x 1000 (1.7 ms of FMA contractions with ssd_heads.cu's share).
+// On bf16 inputs, 16 x 8192 tokens of 32 heads of 128 x 64 take 1073 us where 148 SMs share 512 chains in equal stretches (ssd_chain_wrap), 1240 whole.
 // Every mbarrier wait is bounded, as in the forward.
 #include <cuda_bf16.h>
 #include <type_traits>
 #include "tc_common.cuh"
 #include "kernels.h"
 #include "ssd_fused.h"
+#include "ssd_wrap.cuh"
 
 namespace pmb {
 
@@ -89,6 +91,7 @@ struct Params {
   int rows, fill;                                        // rows of `part` per (b, h); of them a block writes its own, a chain in one piece all (zeros: no more than a warp has lanes)
   int state_only;                                        // first of two passes over segments: only seg_h and seg_d are formed
   float *seg_h, *seg_d;                                  // (B*H-whole,nseg-1,N,P), (B*H-whole,nseg-1): adjoint that a segment hands back when it receives none, decay over it (nobody receives the first one's)
+  uint32_t* flags;                                       // equal stretches of all chains: seg_h (CHAIN_SMS,N,P) and flags are the hand-overs
   unsigned int* status;
 };
 
@@ -111,8 +114,8 @@ __device__ __forceinline__ float warp_column_sums32(float (&v)[8], int lane) {
 }
 __device__ __forceinline__ int column_of(int lane) { return 8 * (lane >> 3) + 2 * (lane & 3) + ((lane >> 2) & 1); }
 
-template <int NI, int ND, int NK, bool IN16>
-__global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid_constant__ Maps maps, const Params p) {
+template <int NI, int ND, int NK, bool IN16, bool WRAP>
+__global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid_constant__ Maps maps, const __grid_constant__ ChainWrap wr, const Params p) {
   using GE = Geo<NI, ND, NK, IN16>;
   constexpr int XB = GE::XB, NSB = GE::NSB;
   extern __shared__ uint8_t smem_raw[];
@@ -135,13 +138,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
   float* sRows = sS + NSB * GE::SLOT;                                     // [2 steps] per-row sums
 
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  const int bh = p.first + (int)blockIdx.x, seg = (int)blockIdx.y + p.state_only;
+  const int state_only = WRAP ? 0 : p.state_only, seg = WRAP ? 0 : (int)blockIdx.y + state_only;
+  int bh = p.first + (int)blockIdx.x, n = min(p.per, p.nsteps - seg * p.per), last = seg * p.per + n - 1;      // chain, steps of this CTA, the last one of them
+  if (WRAP) {
+    const ChainItem it = chain_item(wr, (int)blockIdx.x, p.nsteps);
+    bh = __shfl_sync(0xffffffffu, it.chain, 0); n = __shfl_sync(0xffffffffu, it.count, 0); last = p.nsteps - 1 - __shfl_sync(0xffffffffu, it.from, 0);      // (uniform, as the warp index)
+    if (n <= 0) return;
+  }
   const int h = bh % p.H, bb = bh / p.H, g = h / p.hpg;
-  const int n = min(p.per, p.nsteps - seg * p.per), last = seg * p.per + n - 1;      // steps of this CTA's segment, the last one of them
   const int64_t tokb = (int64_t)bb * p.T;
   if (threadIdx.x == 0) {
-    mbar_init(bar(FULL), 1); mbar_init(bar(EMPTY), p.state_only ? 1 : 6);
-    for (int i = 0; i < 2; ++i) { mbar_init(bar(XIN + i), 1); mbar_init(bar(XRDY + i), 8); mbar_init(bar(XFREE + i), p.state_only ? 1 : IN16 ? 10 : 11); mbar_init(bar(RRDY + i), 12); mbar_init(bar(RFREE + i), 1); }
+    mbar_init(bar(FULL), 1); mbar_init(bar(EMPTY), state_only ? 1 : 6);
+    for (int i = 0; i < 2; ++i) { mbar_init(bar(XIN + i), 1); mbar_init(bar(XRDY + i), 8); mbar_init(bar(XFREE + i), state_only ? 1 : IN16 ? 10 : 11); mbar_init(bar(RRDY + i), 12); mbar_init(bar(RFREE + i), 1); }
     for (int i = 0; i < 4; ++i) mbar_init(bar(SRDY + i), 8);
     mbar_init(bar(GFULL), 1); mbar_init(bar(MRDY), 8); mbar_init(bar(ACCFULL), 2); mbar_init(bar(ACCFREE), 8);
     mbar_init(bar(UFULL), 1); mbar_init(bar(UFREE), 4); mbar_init(bar(HRDY), 4); mbar_init(bar(HFREE), 1);
@@ -157,7 +165,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
-  if (!p.late) pdl_wait();
+  if (WRAP || !p.late) pdl_wait();
   pdl_launch();
   const uint32_t tG = tmem, tM = tmem + 128, tA1 = tmem + 256, tA2 = tmem + 320, tA3 = tmem + 384, tU = tmem + 448;
 
@@ -184,8 +192,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
         auto xload = [&](int k) -> bool {
           const int xb = k % XB;
           if (!wait(XFREE + xb, (uint32_t)(k / XB) ^ 1u, 4096u)) return false;
-          mbar_expect_tx(bar(XIN + xb), (p.state_only ? 1 : 2) * T128);
-          if (!p.state_only) tma_load_4d(xbuf_s + xb * GE::XBUF, &maps.xt[0], 0, (last - k) * L, h, bb, bar(XIN + xb));
+          mbar_expect_tx(bar(XIN + xb), (state_only ? 1 : 2) * T128);
+          if (!state_only) tma_load_4d(xbuf_s + xb * GE::XBUF, &maps.xt[0], 0, (last - k) * L, h, bb, bar(XIN + xb));
           tma_load_4d(xbuf_s + xb * GE::XBUF + GE::XT, &maps.dy[0], 0, (last - k) * L, h, bb, bar(XIN + xb));
           xissued = k + 1;
           return true;
@@ -194,17 +202,17 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
           const int i = last - k;
           if (IN16 && XB == 2 && !xload(k)) break;
           if (!wait(EMPTY, (uint32_t)k ^ 1u, 1u)) break;
-          mbar_expect_tx(bar(FULL), p.state_only ? GE::BT : GE::STAGE);
+          mbar_expect_tx(bar(FULL), state_only ? GE::BT : GE::STAGE);
 #pragma unroll
           for (int kt = 0; kt < NK; ++kt) {
 #pragma unroll
             for (int sp = 0; sp < NI; ++sp) {
               tma_load_4d(c_s + (sp * NK + kt) * T128, &maps.c[sp], 64 * kt, i * L, g, bb, bar(FULL));
-              if (!p.state_only) tma_load_4d(b_s + (sp * NK + kt) * T128, &maps.b[sp], 64 * kt, i * L, g, bb, bar(FULL));
+              if (!state_only) tma_load_4d(b_s + (sp * NK + kt) * T128, &maps.b[sp], 64 * kt, i * L, g, bb, bar(FULL));
             }
 #pragma unroll
             for (int sp = 0; sp < ND; ++sp)
-              if (!p.state_only) tma_load_4d(hin_s + (sp * NK + kt) * T64, &maps.h[sp], 0, 64 * kt, h, bb * p.nsteps + i, bar(FULL));
+              if (!state_only) tma_load_4d(hin_s + (sp * NK + kt) * T64, &maps.h[sp], 0, 64 * kt, h, bb * p.nsteps + i, bar(FULL));
           }
           issued = k + 1;
           if (IN16 && XB == 1 && !xload(k)) break;
@@ -220,7 +228,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       const uint32_t id_v = idesc_bf16(0, 1, L, PW);           // B operand MN-major
       const uint32_t id_u = idesc_bf16(1, 1, L, PW);           // both operands MN-major
       const uint32_t BS = (NK * T128) >> 4, HS = (NK * T64) >> 4, XS = T128 >> 4;      // from a hi tile to its lo tile
-      bool ok = !(warp == 1 && p.state_only);
+      bool ok = !(warp == 1 && state_only);
 #pragma unroll 1
       for (int k = 0; k < n && ok; ++k) {
         const int xb = k % XB;
@@ -298,14 +306,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
 #pragma unroll
               for (int q = 0; q < 8; ++q) mma_split<NI, ND>(tU, cm + ((uint32_t)(q * 2048) >> 4), BS, y0 + ((uint32_t)(q * 2048) >> 4), XS, dhi, id_u, q ? 1u : 0u);
               umma_commit(bar(UFULL)); umma_commit(bar(XFREE + xb));
-              if (XB == 1 || p.state_only) umma_commit(bar(EMPTY));
+              if (XB == 1 || state_only) umma_commit(bar(EMPTY));
             }
             __syncwarp();
             return true;
           };
           // (two buffers: exp(S) dY has been there for a while, and the state's chain does not wait for the draining; one: it is being formed)
-          if (!(ok = p.state_only ? update() : XB == 2 ? update() && carried() : carried() && update())) break;
-          if (!IN16 && !p.state_only && lane == 0) {
+          if (!(ok = state_only ? update() : XB == 2 ? update() && carried() : carried() && update())) break;
+          if (!IN16 && !state_only && lane == 0) {
             // x~ and dY go out as the operands that the sums over heads read
             if (p.store_ops) {
 #pragma unroll
@@ -322,7 +330,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
         }
       }
       if (!IN16 && warp == 3 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-    } else if (p.state_only) {
+    } else if (state_only) {
     } else if (warp == 2) {
       // ---------------- per-token gradients (lane = four consecutive tokens) ----------------
       const bool dtm = p.dt != nullptr;
@@ -497,7 +505,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
     // Fragments of 16 rows x 8 columns: a lane holds rows fr + {0, 8, 16, 24} of the warp's 32 and two adjacent columns of every eight, so
     // a column's sum over the warp takes four additions in the lane and three exchanges of a halving number of columns.
     const int fr = lane >> 2, fc = 2 * (lane & 3);
-    bool ok = !p.state_only;
+    bool ok = !state_only;
 #pragma unroll 1
     for (int k = 0; k < n && ok; ++k) {
       float* R = sRows + (k & 1) * GE::ROWS;
@@ -717,7 +725,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
     float hv[PW];
 #pragma unroll
     for (int q = 0; q < PW; ++q) hv[q] = 0.0f;
-    if (!p.state_only && active)
+    if (!WRAP && !state_only && active)
       for (int j = p.nseg - 1; j > seg; --j) {              // what the segments after this one hand back
         const int64_t row = (int64_t)(bh - p.first) * (p.nseg - 1) + j - 1;
         const float* F = p.seg_h + row * NP + (int64_t)nr * p.P;
@@ -732,10 +740,25 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
         }
       }
     bool ok = true;
+    if (WRAP && last + 1 < p.nsteps) {            // the rest of a chain: dh comes from the CTA that walked its end
+      const int from = wr.e[blockIdx.x % CHAIN_SMS].sm;
+      ok = chain_take(p.flags + from, abort_flag);
+      if (!ok) give_up(8192u);
+      if (ok && active) {
+        const float4* F = reinterpret_cast<const float4*>(p.seg_h + (int64_t)from * NP + (int64_t)nr * p.P);
+#pragma unroll
+        for (int q = 0; q < PW / 4; ++q) {
+          if (4 * q >= p.P) continue;
+          const float4 v = __ldcg(F + q);
+          hv[4 * q] = v.x; hv[4 * q + 1] = v.y; hv[4 * q + 2] = v.z; hv[4 * q + 3] = v.w;
+          if (q % 4 == 3) asm volatile("" ::: "memory");
+        }
+      }
+    }
     float stot = 0.0f;
     for (int k = 0; k < n && ok; ++k) {
       const int i = last - k;
-      if (!p.state_only) {
+      if (!state_only) {
         if (k > 0) ok = all(wait(HFREE, (uint32_t)(k - 1), 256u));
         if (!ok) break;
         const int64_t so = (((int64_t)bb * p.nsteps + i) * p.H + h) * NP + (int64_t)nr * p.P;
@@ -800,20 +823,22 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(UFREE));
     }
-    if (ok && p.state_only) {
-      const int64_t row = (int64_t)blockIdx.x * gridDim.y + blockIdx.y;
-      if (nr == 0) p.seg_d[row] = __expf(stot);
+    const bool handed = WRAP && last + 1 > n;     // the end of a chain whose rest another CTA walks
+    if (ok && (state_only || handed)) {
+      const int64_t row = handed ? wr.e[blockIdx.x % CHAIN_SMS].sm + 1 : (int64_t)blockIdx.x * gridDim.y + blockIdx.y;
+      if (nr == 0 && !handed) p.seg_d[row] = __expf(stot);
       float* dst = p.seg_h + row * NP + (int64_t)nr * p.P;
       if (active) {
 #pragma unroll
         for (int q = 0; q < PW / 4; ++q)
           if (4 * q < p.P) *reinterpret_cast<float4*>(dst + 4 * q) = make_float4(hv[4 * q], hv[4 * q + 1], hv[4 * q + 2], hv[4 * q + 3]);
       }
+      if (handed) chain_hand_over(p.flags + row);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if ((int)threadIdx.x < p.fill && p.part && !p.state_only) {
+  if ((int)threadIdx.x < p.fill && p.part && !state_only) {
     float t = 0.0f;                                         // fixed order
     for (int q = 0; q < 8; ++q) t += dDw[q];
     p.part[p.part_pitch + ((int64_t)bb * p.rows + seg + threadIdx.x) * p.H + h] = threadIdx.x == 0 ? t : 0.0f;
@@ -822,7 +847,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
   }
-  if (p.late) pdl_wait();                                  // (a kernel completes after those before it)
+  if (!WRAP && p.late) pdl_wait();                                  // (a kernel completes after those before it)
 }
 
 // ---- host side -------------------------------------------------------------------------------------------
@@ -859,12 +884,21 @@ static pmb_status launch(cudaStream_t st, const ChainBwdArgs& a) {
   p.dx = a.dx; p.dx16 = a.dx16; p.lddx = a.lddx; p.store_ops = a.xt_hi != nullptr; p.dh_hi = a.dh_hi; p.dh_lo = a.dh_lo; p.da = a.da;
   p.raw_hi = a.raw_hi; p.raw_lo = a.raw_lo; p.ld_raw = a.ld_raw; p.raw_col = a.raw_col; p.part = a.part; p.status = status_ptr();
   const int chains = a.B * a.H;
+  ChainWrap wr{};
+  if constexpr (IN16) {
+    if (a.seg && !a.part && ssd_chain_wrap(chains, n, 1, 0.0, &wr)) {
+      p.seg_h = a.seg; p.flags = ssd_chain_flags(a.seg, a.P, a.N);
+      PMB_CUDA(cudaMemsetAsync(p.flags, 0, CHAIN_FLAG_BYTES, st));
+      PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_bwd_kernel<NI, ND, NK, IN16, true>);
+      return launch_pdl(st, ssd_chain_bwd_kernel<NI, ND, NK, IN16, true>, dim3((unsigned)(wr.rounds * CHAIN_SMS)), NTHREADS, GE::SMEM, ms, wr, p);
+    }
+  }
   const ChainPlan plan = a.seg ? ssd_chain_plan(a.B, a.T, a.H) : ChainPlan{chains, 1, n};
   const unsigned cut = (unsigned)((chains - plan.whole) * plan.nseg);      // blocks of segments
   if (cut) { p.seg_h = a.seg; p.seg_d = a.seg + (size_t)cut * a.N * a.P; }
   p.rows = plan.nseg; p.fill = 1; p.part_pitch = (int64_t)chains * plan.nseg;
-  PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_bwd_kernel<NI, ND, NK, IN16>);
-  auto run = [&](int count, int segments) { return launch_pdl(st, ssd_chain_bwd_kernel<NI, ND, NK, IN16>, dim3((unsigned)count, (unsigned)segments), NTHREADS, GE::SMEM, ms, p); };
+  PMB_SMEM_OPT_IN(GE::SMEM, ssd_chain_bwd_kernel<NI, ND, NK, IN16, false>);
+  auto run = [&](int count, int segments) { return launch_pdl(st, ssd_chain_bwd_kernel<NI, ND, NK, IN16, false>, dim3((unsigned)count, (unsigned)segments), NTHREADS, GE::SMEM, ms, wr, p); };
   // the segments' adjoints, the segments, and beside both the chains in one piece
   if (cut) {
     p.first = plan.whole; p.nseg = plan.nseg; p.per = plan.per;

@@ -45,12 +45,33 @@ struct ChainArgs {
   float* last;                                 // (B,H,N,P)
   float *hprev;                                // plain operands with fp32 x: (B,chunks,H,N,P) state entering each chunk
   uint16_t *xt, *xs;                           // ... and the operands x~ and xs, (B,T,H,P)
-  float* seg = nullptr;                        // ssd_chain_seg_floats() floats: lets few long sequences be walked in segments (blocks == 1)
+  float* seg = nullptr;                        // ssd_chain_seg_floats() floats: lets chains be walked in pieces
+  bool flags_clear = false;                    // ssd_chain_flags() of it are zero already
 };
 // The first `whole` chains (b, h) are walked in one piece, each of the others in `nseg` segments of `per` steps (the last may have fewer).
 struct ChainPlan { int whole, nseg, per; };
 ChainPlan ssd_chain_plan(int B, int T, int H);
 size_t ssd_chain_seg_floats(int B, int T, int H, int P, int N);
+// More chains than SMs on plain operands: every SM takes an equal stretch of all chains' steps laid end to end (ssd_chain.cu says how a chain
+// that two SMs share is handed over).  One entry per SM, sorted by when it comes to its second item: in units of steps, the chains that its
+// stretch begins and ends in and the places there, and the SM's place in the unsorted order, which numbers the hand-overs.
+constexpr int CHAIN_SMS = 148;
+struct ChainWrap {
+  struct Entry {
+    uint16_t head, head_units;                 // the chain that the stretch ends in and how much of it (0: none), walked first
+    uint16_t extra;                            // a last whole chain beyond `wholes` (0: none)
+    uint16_t tail, tail_from;                  // the chain that the stretch begins in and where (0: none), walked last
+    uint16_t sm;                               // place in the order of the stretches, which numbers the hand-overs: sm + 1 is given, sm taken
+  } e[CHAIN_SMS];
+  int wholes, first_whole;                     // whole chains that every SM has, between the other two: first_whole + i CHAIN_SMS + the entry's place
+  int rounds;                                  // blocks: rounds x CHAIN_SMS
+};
+// false: the chains are better walked whole.  `units` of steps to a chain; least_share: of the steps one after the other, what has to be saved
+bool ssd_chain_wrap(int64_t chains, int units, int steps_per_unit, double least_share, ChainWrap* w);
+// counters of the hand-overs, in the buffer `seg` of the two kernels below: zero when a launch begins
+constexpr size_t CHAIN_FLAG_BYTES = (CHAIN_SMS + 12) * sizeof(uint32_t);
+static_assert(CHAIN_FLAG_BYTES == CONV_CLEAR_WORDS * sizeof(uint32_t), "the conv kernel clears them");
+inline uint32_t* ssd_chain_flags(float* seg, int P, int N) { return reinterpret_cast<uint32_t*>(seg + (size_t)CHAIN_SMS * N * P); }
 inline bool ssd_chain_shape(int P, int N) { return P > 0 && P <= 64 && P % 8 == 0 && N > 0 && N <= 128 && N % 8 == 0; }
 bool ssd_chain_enabled();      // false when PMB_SSD_FUSED=0 or PMB_SSD_ENGINE=simt
 // bf16-storage blocks: shapes whose scan reads its operands rounded to bf16 (whole chunks of 128 or 256 tokens at d_state =

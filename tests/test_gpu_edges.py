@@ -715,3 +715,53 @@ def test_block_bf16_backward_of_chunks(pm, B, T, Q, G, decay):
     for k, v in leaves.items():
         assert_close(grads[k], v.grad, tol=2e-2, what=k)
     assert pm.device_status() == 0
+
+
+# more chains than SMs: every SM takes an equal stretch of all chains' steps, and the state of a chain that two SMs share goes through memory.
+# Bit by bit what the same sequences give one batch at a time, where each chain is walked whole; twice, and in a graph.  (db and dc are sums over
+# heads in an order that depends on the number of batches, rounded to bf16: two of them lie one step apart, at most 2^-7 of the value.)
+@pytest.mark.parametrize("B,H,T,P,N,Q", [(2, 80, 512, 64, 64, 128), (2, 80, 700, 64, 128, 128), (3, 100, 640, 64, 128, 128), (2, 75, 513, 8, 8, 64),
+                                         (2, 140, 1024, 64, 64, 256), (7, 96, 512, 32, 64, 512), (4, 76, 1200, 64, 64, 256)])
+def test_scan_of_more_chains_than_sms(pm, B, H, T, P, N, Q):
+    x, b, c, dy = (randn(s, i).bfloat16().cuda() for i, s in enumerate([(B, T, H, P), (B, T, 1, N), (B, T, 1, N), (B, T, H, P)]))
+    a = (-torch.nn.functional.softplus(randn((B, T, H), 5) - 1.0)).cuda()
+    init = randn((B, H, N, P), 6).cuda()
+    scan = pm.SsdScanBf16(x, a, b, c, Q)
+
+    def call(s, dy, init):
+        y, last = s.forward(init, True)
+        return y, last, *s.backward(dy)
+
+    want = [torch.cat(v) for v in zip(*(call(pm.SsdScanBf16(x[i:i + 1], a[i:i + 1], b[i:i + 1], c[i:i + 1], Q), dy[i:i + 1], init[i:i + 1]) for i in range(B)))]
+    side, g = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    got = [call(scan, dy, init) for _ in range(2)]
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.graph(g, stream=side):
+        got.append(call(scan, dy, init))
+    for _ in range(2):
+        g.replay()
+    torch.cuda.synchronize()
+    assert pm.device_status() == 0
+    for run in got:
+        for u, v, what in zip(run, want, ("y", "last", "dx", "da", "db", "dc")):
+            if what in ("db", "dc"):
+                assert_close(u.float(), v.float(), tol=2.0 ** -7, what=what)
+            else:
+                assert torch.equal(u, v), what
+
+
+# the same inside bf16-storage blocks, with what a backward reads (chunks of one and of two steps).  dx: the sums over heads and the recompute of
+# half the batch take other orders there, bf16 storage's own tolerance.
+@pytest.mark.parametrize("B,T,Q", [(8, 1024, 256), (7, 768, 256), (7, 1280, 128)])
+def test_bf16_block_of_more_chains_than_sms(pm, B, T, Q):
+    cfg = pm.Mamba2Config(d_model=256, d_state=64, d_head=64, n_heads=24, n_groups=1, d_conv=4, block_len=Q)
+    p = {k: v.cuda() for k, v in orc.init_block_params(orc.Mamba2Config(256, 64, 64, 24, 1, 4, Q), seed=3).items()}
+    blk = pm.Mamba2Block(cfg, p, compute_dtype=torch.bfloat16)
+    x, dout = randn((B, T, 256), 1).bfloat16().cuda(), randn((B, T, 256), 2).bfloat16().cuda()
+    out = blk.forward(x)
+    dx, _ = blk.backward(x, dout)
+    half = B // 2                              # 72 or 96 chains: each walked whole
+    for lo, hi in ((0, half), (half, B)):
+        assert torch.equal(out[lo:hi], blk.forward(x[lo:hi].contiguous()))
+        assert_close(dx[lo:hi].float(), blk.backward(x[lo:hi].contiguous(), dout[lo:hi].contiguous())[0].float(), tol=2e-2, what="dx")
+    assert pm.device_status() == 0
