@@ -6,16 +6,17 @@
 // Per head the tensor core forms dY x~^T, dY h^T and x~ dh^T from four tiles; the decays are applied where the products are added
 // up in registers, so no copy of dY or x~ scaled by them exists and dG never leaves the SM.  With few tiles the heads of a group
 // are split over CTAs; dC and dB are linear in dG, so every CTA finishes its own heads' share and the shares are added in a fixed
-// order (heads_sum_kernel).  d_state is taken in halves of 64: a second pass over the heads forms the second half.
+// order (heads_sum_kernel).
 //
-// warp 0 = TMA, 1 = MMA issuer, 2 = S of the heads, 4..11 = dG (64 columns per thread), 12..15 = dC, 16..19 = dB (64 columns per
-// thread).  Two or three operand stages, two sets of accumulators: the products of the next head run under the sums of this one.
-// What bounds it: latency.  No pipe or memory level is near its limit at 32 heads of 128 x 64 (issue slots 46 %, DRAM 51 %, exponentials
-// 16 %); warps wait for TMEM loads, each of which is followed at once by its wait, with five warps to a scheduler.
-// Measured at 24 heads of 64 x 64 on pairs, 4 x 512 tokens: 18 us + 3 us for the sum of the shares; the three contractions and their
-// sums that it replaces took 45 us and read copies of dY and x~ scaled by the decays that are not made any more.  bf16, 32 heads of 128 x 64, 16 x 8192 tokens: 836 us with two
-// stages, 820 with three, 680 since the warp index is a shuffle's result (uniform branches and descriptors) and a wait looks at its barrier first
-// (3.2 GB of operands; the contractions it replaces: 1070 us).
+// warp 0 = TMA, 1 = MMA issuer, 2 = S of the heads, then dG (eight warps with 64 columns per thread; d_state above 64: four with 128), four of
+// dC and four of dB (all of d_state).  Two or three operand stages, two accumulators of dG; dC and dB have two up to 64 states, the
+// products of the next head running under the sums of this one, and one above, where the next head's dG product runs ahead instead.
+// What bounds it: the operands' bytes, half of HBM's rate, and the latency of a head's chain (product, TMEM load, sum, hand-over).  Bf16, 8 x 4096
+// tokens, 32 heads of 128 x 64: 197 us when d_state was taken in two passes over the heads (826 MB read) and dG's warps took nine instructions
+// per element one by one; 235 in one pass (558 MB) with half as many dG warps: theirs was the longest chain; 129 now that exponents and sums go
+// in pairs and results below 2^-126 are zeros (53 -> 31 M warp instructions).  16 x 1024 of 64 x 64: 68 and 55 us; 16 x 8192 of 128 x 64:
+// 700 and 450.  (Three stages instead of two, a warp index from a shuffle and a look at the barrier before a wait brought 836 to 680 before.)
+// At 24 heads of 64 x 64 on pairs, 4 x 512 tokens: 18 us + 3 us for the sum of the shares.
 #include <cuda_bf16.h>
 #include "tc_common.cuh"
 #include "kernels.h"
@@ -37,25 +38,29 @@ namespace shd {
 using namespace tcx;
 
 constexpr int L = SCAN_STEP, T128 = L * 128, T64 = 64 * 128;
-constexpr int W_G = 4, W_C = 12, NTHREADS = 32 * 20;
 
-template <int NI, int ND>
+// NK = 64-wide blocks of d_state, all of them in one pass over the heads.
+template <int NI, int ND, int NK>
 struct Geo {
-  static constexpr int XT = NI * T128, HT = ND * T64;
-  static constexpr int STAGE = 2 * XT + 2 * HT;            // [dY | x~ | h | dh]; at the end of a pass [B | C]
+  // warps of dG, then four each of dC and dB; with two blocks their threads have 128 sums each, and there are half as many for dG
+  static constexpr int GW = NK == 2 ? 4 : 8, W_G = 4, W_C = W_G + GW, NTHREADS = 32 * (W_C + 8);
+  static constexpr int GC = L * 4 / GW, CC = 64 * NK;      // columns per thread
+  static constexpr int CB = NK == 2 ? 1 : 2;               // accumulators of dC and dB (TMEM: two of 128 columns for dG, the rest is theirs)
+  static constexpr int XT = NI * T128, HT = ND * NK * T64, BT = NI * NK * T128;
+  static constexpr int STAGE = 2 * XT + 2 * HT;            // [dY | x~ | h | dh]; in the end [B | C]
   static constexpr int DG = ND * 2 * T128;                        // dG as an operand: two 64-column tiles (hi), then lo
-  static constexpr bool OWN_DG = NI == 1;                  // pairs: dG goes over the stage that the last head has left
+  static constexpr bool OWN_DG = NI == 1 && NK == 1;       // otherwise dG goes over the stage that the last head has left
   static constexpr int RING = 4;                           // heads whose S is in shared memory
   static constexpr int STG = NI == 1 && ND == 1 ? 3 : 2;   // (what fits)
   static constexpr int TILES = STG * STAGE + (OWN_DG ? DG : 0);
-  static_assert(OWN_DG || (DG <= STAGE && STG == 2), "dG fits a stage");
+  static_assert((OWN_DG || DG <= STAGE) && 2 * BT <= STAGE, "dG, and B and C, fit a stage");
   static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 256 /*barriers*/ + RING * L * 4;
 };
 
 struct Maps { CUtensorMap dy[2], xt[2], h[2], dh[2], b[2], c[2]; };
 
 struct Params {
-  int T, H, G, hpg, N, n, nsplit, passes;
+  int T, H, G, hpg, N, n, nsplit;
   const float* S;
   float *dc, *db; int64_t ld;                              // token rows, group g at column g * N
   uint16_t *dc16, *db16;                                   // the same as bf16 (instead)
@@ -63,14 +68,10 @@ struct Params {
   unsigned int* status;
 };
 
-__device__ __forceinline__ uint32_t pack2(float a, float b) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-
-template <int NI, int ND>
-__global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_constant__ Maps maps, const Params p) {
-  using GE = Geo<NI, ND>;
+template <int NI, int ND, int NK>
+__global__ void __launch_bounds__(Geo<NI, ND, NK>::NTHREADS, 1) ssd_heads_kernel(const __grid_constant__ Maps maps, const Params p) {
+  using GE = Geo<NI, ND, NK>;
+  constexpr int W_G = GE::W_G, W_C = GE::W_C, CB = GE::CB;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -92,15 +93,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
   const int i = id % p.n, bb = id / p.n;
   const int nh = (p.hpg - split + p.nsplit - 1) / p.nsplit;
   auto head = [&](int j) { return g * p.hpg + split + j * p.nsplit; };
-  const int per_pass = nh + 1, nitems = p.passes * per_pass;     // the heads, then the product with dG
+  const int nitems = nh + 1;                                // the heads, then the product with dG
   if (threadIdx.x == 0) {
     for (int q = 0; q < 2; ++q) {
-      mbar_init(bar(MFULL + q), 1); mbar_init(bar(MFREE + q), 8);
+      mbar_init(bar(MFULL + q), 1); mbar_init(bar(MFREE + q), GE::GW);
       mbar_init(bar(CFULL + q), 1); mbar_init(bar(CFREE + q), 8);
     }
     for (int q = 0; q < GE::STG; ++q) { mbar_init(bar(FULL + q), 1); mbar_init(bar(EMPTY + q), 1); }
-    for (int q = 0; q < 4; ++q) { mbar_init(bar(SRDY + q), 1); mbar_init(bar(SFREE + q), 16); }
-    mbar_init(bar(DGRDY), 8);
+    for (int q = 0; q < 4; ++q) { mbar_init(bar(SRDY + q), 1); mbar_init(bar(SFREE + q), GE::GW + 8); }
+    mbar_init(bar(DGRDY), GE::GW);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -116,8 +117,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
   pdl_launch();
   pdl_wait();
   const uint32_t tM = tmem, tC = tmem + 256, tB = tmem + 384;
-  // the stage that dG goes over: the one the last head of the first pass was in
-  const uint32_t dg_s = GE::OWN_DG ? base + GE::STG * GE::STAGE : base + (uint32_t)((nh - 1) & 1) * GE::STAGE;
+  // the stage that dG goes over: the one the last head was in
+  const uint32_t dg_s = GE::OWN_DG ? base + GE::STG * GE::STAGE : base + (uint32_t)((nh - 1) % GE::STG) * GE::STAGE;
 
   auto give_up = [&](unsigned int code) { atomicOr(p.status, code); *abort_flag = 1; };
   auto wait = [&](int b, uint32_t parity, unsigned int code) -> bool {
@@ -129,11 +130,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
   };
   auto all = [&](bool v) -> bool { return __all_sync(0xffffffffu, v); };
 
+  if (warp < W_G) {
+  if (NK == 2) regs_dec<40>();
   if (warp == 0) {
     if (lane == 0) {
       int issued = 0;
       for (int m = 0; m < nitems; ++m) {
-        const int s = m % GE::STG, ps = m / per_pass, j = m - ps * per_pass;
+        const int s = m % GE::STG, j = m;
         if (!wait(EMPTY + s, (uint32_t)(m / GE::STG) ^ 1u, 1u)) break;
         const uint32_t st = base + s * GE::STAGE;
         if (j < nh) {
@@ -145,17 +148,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
             tma_load_4d(st + GE::XT + sp * T128, &maps.xt[sp], 0, i * L, h, bb, bar(FULL + s));
           }
 #pragma unroll
-          for (int sp = 0; sp < ND; ++sp) {
-            tma_load_4d(st + 2 * GE::XT + sp * T64, &maps.h[sp], 0, 64 * ps, h, bb * p.n + i, bar(FULL + s));
-            tma_load_4d(st + 2 * GE::XT + GE::HT + sp * T64, &maps.dh[sp], 0, 64 * ps, h, bb * p.n + i, bar(FULL + s));
-          }
-        } else {
-          mbar_expect_tx(bar(FULL + s), 2 * GE::XT);
+          for (int sp = 0; sp < ND; ++sp)
 #pragma unroll
-          for (int sp = 0; sp < NI; ++sp) {
-            tma_load_4d(st + sp * T128, &maps.b[sp], 64 * ps, i * L, g, bb, bar(FULL + s));
-            tma_load_4d(st + GE::XT + sp * T128, &maps.c[sp], 64 * ps, i * L, g, bb, bar(FULL + s));
-          }
+            for (int kt = 0; kt < NK; ++kt) {
+              tma_load_4d(st + 2 * GE::XT + (sp * NK + kt) * T64, &maps.h[sp], 0, 64 * kt, h, bb * p.n + i, bar(FULL + s));
+              tma_load_4d(st + 2 * GE::XT + GE::HT + (sp * NK + kt) * T64, &maps.dh[sp], 0, 64 * kt, h, bb * p.n + i, bar(FULL + s));
+            }
+        } else {
+          mbar_expect_tx(bar(FULL + s), 2 * GE::BT);
+#pragma unroll
+          for (int sp = 0; sp < NI; ++sp)
+#pragma unroll
+            for (int kt = 0; kt < NK; ++kt) {
+              tma_load_4d(st + (sp * NK + kt) * T128, &maps.b[sp], 64 * kt, i * L, g, bb, bar(FULL + s));
+              tma_load_4d(st + GE::BT + (sp * NK + kt) * T128, &maps.c[sp], 64 * kt, i * L, g, bb, bar(FULL + s));
+            }
         }
         issued = m + 1;
       }
@@ -164,36 +171,46 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
     }
   } else if (warp == 1) {
     const uint32_t dhi = desc_hi(1024, 2);
-    const uint32_t id_m = idesc_bf16(0, 0, L, L), id_h = idesc_bf16(0, 0, L, 64);      // both operands K-major
-    const uint32_t id_c = idesc_bf16(0, 1, L, 64), id_b = idesc_bf16(1, 1, L, 64);     // dG B and dG^T C
-    const uint32_t XS = T128 >> 4, HS = T64 >> 4, DS = (2 * T128) >> 4;
+    const uint32_t id_m = idesc_bf16(0, 0, L, L), id_h = idesc_bf16(0, 0, L, 64 * NK);      // both operands K-major
+    const uint32_t id_c = idesc_bf16(0, 1, L, 64 * NK), id_b = idesc_bf16(1, 1, L, 64 * NK);     // dG B and dG^T C
+    const uint32_t XS = T128 >> 4, HS = (NK * T64) >> 4, BS = (NK * T128) >> 4, DS = (2 * T128) >> 4;
     bool ok = true;
 #pragma unroll 1
     for (int m = 0; m < nitems && ok; ++m) {
-      const int s = m & 1, sg = m % GE::STG, ps = m / per_pass, j = m - ps * per_pass;
+      const int s = m % CB, sg = m % GE::STG;
       const uint32_t st = base + sg * GE::STAGE;
-      ok = all(wait(FULL + sg, (uint32_t)(m / GE::STG), 2u) && (m < 2 || wait(CFREE + s, (uint32_t)((m >> 1) - 1), 4u)) &&
-               (ps > 0 || j >= nh || j < 2 || wait(MFREE + (j & 1), (uint32_t)((j >> 1) - 1), 8u)) && (j < nh || wait(DGRDY, 0u, 16u)));
+      const uint32_t y0 = desc_lo(st, 16), x0 = desc_lo(st + GE::XT, 16);
+      ok = all(wait(FULL + sg, (uint32_t)(m / GE::STG), 2u) && (m >= nh || m < 2 || wait(MFREE + (m & 1), (uint32_t)((m >> 1) - 1), 8u)));
       if (!ok) break;
+      if (CB == 1 && m < nh) {                               // (the other products wait for dC and dB of the head before to be taken)
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (elect_one()) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) mma_split<NI, NI>(tM + (uint32_t)(128 * (m & 1)), y0 + 2 * q, XS, x0 + 2 * q, XS, dhi, id_m, q ? 1u : 0u);
+          umma_commit(bar(MFULL + (m & 1)));
+        }
+        __syncwarp();
+      }
+      if (!(ok = all((m < CB || wait(CFREE + s, (uint32_t)(m / CB - 1), 4u)) && (m < nh || wait(DGRDY, 0u, 16u))))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (elect_one()) {
         const uint32_t dC = tC + (uint32_t)(64 * s), dB = tB + (uint32_t)(64 * s);
-        if (j < nh) {
-          const uint32_t y0 = desc_lo(st, 16), x0 = desc_lo(st + GE::XT, 16), h0 = desc_lo(st + 2 * GE::XT, 16), d0 = desc_lo(st + 2 * GE::XT + GE::HT, 16);
+        if (m < nh) {
+          const uint32_t h0 = desc_lo(st + 2 * GE::XT, 16), d0 = desc_lo(st + 2 * GE::XT + GE::HT, 16);
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            if (ps == 0) mma_split<NI, NI>(tM + (uint32_t)(128 * (j & 1)), y0 + 2 * q, XS, x0 + 2 * q, XS, dhi, id_m, q ? 1u : 0u);
+            if (CB == 2) mma_split<NI, NI>(tM + (uint32_t)(128 * (m & 1)), y0 + 2 * q, XS, x0 + 2 * q, XS, dhi, id_m, q ? 1u : 0u);
             mma_split<NI, ND>(dC, y0 + 2 * q, XS, h0 + 2 * q, HS, dhi, id_h, q ? 1u : 0u);
             mma_split<NI, ND>(dB, x0 + 2 * q, XS, d0 + 2 * q, HS, dhi, id_h, q ? 1u : 0u);
           }
-          if (ps == 0) umma_commit(bar(MFULL + (j & 1)));
+          if (CB == 2) umma_commit(bar(MFULL + (m & 1)));
         } else {
-          const uint32_t gk = desc_lo(dg_s, 16), gm = desc_lo(dg_s, T128), b0 = desc_lo(st, T128), c0 = desc_lo(st + GE::XT, T128);
+          const uint32_t gk = desc_lo(dg_s, 16), gm = desc_lo(dg_s, T128), b0 = desc_lo(st, T128), c0 = desc_lo(st + GE::BT, T128);
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const uint32_t o = (uint32_t)(q * 2048) >> 4;
-            mma_split<ND, NI>(dC, gk + ((uint32_t)((q >> 2) * T128 + (q & 3) * 32) >> 4), DS, b0 + o, XS, dhi, id_c, q ? 1u : 0u);
-            mma_split<ND, NI>(dB, gm + o, DS, c0 + o, XS, dhi, id_b, q ? 1u : 0u);
+            mma_split<ND, NI>(dC, gk + ((uint32_t)((q >> 2) * T128 + (q & 3) * 32) >> 4), DS, b0 + o, BS, dhi, id_c, q ? 1u : 0u);
+            mma_split<ND, NI>(dB, gm + o, DS, c0 + o, BS, dhi, id_b, q ? 1u : 0u);
           }
         }
         umma_commit(bar(CFULL + s));
@@ -202,11 +219,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
       __syncwarp();
     }
   } else if (warp == 2) {
-    // S of a head's 128 tokens (a = 0 past the end of the sequence); every head once per pass
-    for (int m = 0; m < p.passes * nh; ++m) {
+    // S of a head's 128 tokens (a = 0 past the end of the sequence)
+    for (int m = 0; m < nh; ++m) {
       const int r = m % GE::RING;
       if (m >= GE::RING && !all(wait(SFREE + r, (uint32_t)(m / GE::RING - 1), 32u))) break;
-      const float* Sg = p.S + ((int64_t)bb * p.H + head(m % nh)) * p.T;
+      const float* Sg = p.S + ((int64_t)bb * p.H + head(m)) * p.T;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int t = i * L + lane + 32 * e;
@@ -215,55 +232,63 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(SRDY + r));
     }
-  } else if (warp >= W_G && warp < W_C) {
+  }
+  } else if (warp < W_C) {
     // ---------------- dG ----------------
+    if (NK == 2) regs_inc<152>();
+    constexpr int GC = GE::GC;
     const int quarter = warp & 3, grp = (warp - W_G) >> 2, row = quarter * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-    float acc[64];
+    F2 acc[GC / 2];
 #pragma unroll
-    for (int e = 0; e < 64; ++e) acc[e] = 0.0f;
+    for (int e = 0; e < GC / 2; ++e) acc[e] = 0;
     bool ok = true;
-    const bool above = grp == 1 && quarter < 2;                // every column of this half is past every row of this warp
     for (int j = 0; j < nh && ok; ++j) {
       const float* S = sS + (j % GE::RING) * L;
       ok = all(wait(SRDY + (j % GE::RING), (uint32_t)(j / GE::RING), 64u) && wait(MFULL + (j & 1), (uint32_t)(j >> 1), 64u));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (!above) {
-        const float S_row = S[row];
+      const float S_row = S[row];
+      const F2 Sr2 = pack2(S_row, S_row), neg = pack2(-1.0f, -1.0f), log2e = pack2(1.4426950408889634f, 1.4426950408889634f);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          uint32_t v[16];
-          tmem_ld16(tM + lane_addr + (uint32_t)(128 * (j & 1) + grp * 64 + 16 * q), v);
-          tmem_wait_ld();
+      for (int q = 0; q < GC / 16; ++q) {
+        const int c0 = grp * GC + 16 * q;
+        if (c0 > quarter * 32 + 31) continue;                // every one of these columns is past every row of this warp
+        uint32_t v[16];
+        tmem_ld16(tM + lane_addr + (uint32_t)(128 * (j & 1) + c0), v);
+        F2 w[8];
 #pragma unroll
-          for (int e = 0; e < 16; e += 4) {
-            const int col = grp * 64 + 16 * q + e;
-            const float4 s4 = *reinterpret_cast<const float4*>(S + col);
-            const float sv[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const float w = col + u <= row ? __expf(S_row - sv[u]) : 0.0f;
-              acc[16 * q + e + u] = fmaf(__uint_as_float(v[e + u]), w, acc[16 * q + e + u]);
-            }
-          }
+        for (int e = 0; e < 8; e += 2) {
+          const ulonglong2 s4 = *reinterpret_cast<const ulonglong2*>(S + c0 + 2 * e);
+          const float2 u0 = unpack2(mul2(fma2(s4.x, neg, Sr2), log2e)), u1 = unpack2(mul2(fma2(s4.y, neg, Sr2), log2e));
+          w[e] = pack2(ex2_ftz(u0.x), ex2_ftz(u0.y)); w[e + 1] = pack2(ex2_ftz(u1.x), ex2_ftz(u1.y));
         }
+        if (c0 + 15 > quarter * 32) {                        // (the diagonal may cross)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) { const float2 u = unpack2(w[e]); w[e] = pack2(c0 + 2 * e <= row ? u.x : 0.0f, c0 + 2 * e + 1 <= row ? u.y : 0.0f); }
+        }
+        tmem_wait_ld();
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[8 * q + e] = fma2(pack2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])), w[e], acc[8 * q + e]);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) { mbar_arrive(bar(MFREE + (j & 1))); mbar_arrive(bar(SFREE + (j % GE::RING))); }
     }
+    // (over a stage: when all products of the last head are done)
+    if (ok && !GE::OWN_DG && CB == 1) ok = all(wait(CFULL + (nh - 1) % CB, (uint32_t)((nh - 1) / CB), 64u));
     if (ok) {
-      // (all products of the last head are done: its stage is free for dG)
 #pragma unroll
-      for (int c = 0; c < 8; ++c) {
+      for (int c = 0; c < GC / 8; ++c) {
         uint32_t hi[4], lo[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          hi[e] = pack2(acc[8 * c + 2 * e], acc[8 * c + 2 * e + 1]);
-          lo[e] = pack2(acc[8 * c + 2 * e] - __uint_as_float(hi[e] << 16), acc[8 * c + 2 * e + 1] - __uint_as_float(hi[e] & 0xffff0000u));
+          const float2 u = unpack2(acc[4 * c + e]);
+          hi[e] = bf16_of_two(u.x, u.y);
+          lo[e] = bf16_rest_of_two(u.x, u.y, hi[e]);
         }
-        const uint32_t a = dg_s + (uint32_t)(grp * T128 + row * 128 + ((c ^ (row & 7)) << 4));
+        const int cg = grp * (GC / 8) + c;                     // eight columns of the row
+        const uint32_t a = dg_s + (uint32_t)((cg >> 3) * T128 + row * 128 + (((cg & 7) ^ (row & 7)) << 4));
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]) : "memory");
         if (ND == 2) asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a + 2 * T128), "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]) : "memory");
       }
@@ -271,66 +296,58 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_heads_kernel(const __grid_con
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(DGRDY));
     }
-  } else if (warp >= W_C) {
+  } else {
     // ---------------- dC (first four warps) and dB ----------------
+    if (NK == 2) regs_inc<152>();
+    constexpr int CC = GE::CC;
     const int quarter = warp & 3, which = (warp - W_C) >> 2, row = quarter * 32 + lane;
     const uint32_t src = (which ? tB : tC) + ((uint32_t)(quarter * 32) << 16);
+    F2 acc[CC / 2];
+#pragma unroll
+    for (int e = 0; e < CC / 2; ++e) acc[e] = 0;
     bool ok = true;
-    int m = 0, hs = 0;
-    for (int ps = 0; ps < p.passes && ok; ++ps) {
-      float acc[64];
-#pragma unroll
-      for (int e = 0; e < 64; ++e) acc[e] = 0.0f;
-      for (int j = 0; j <= nh && ok; ++j, ++m) {
-        const int s = m & 1;
-        float f = 1.0f;
-        if (j < nh) {
-          ok = all(wait(SRDY + (hs % GE::RING), (uint32_t)(hs / GE::RING), 128u));
-          if (!ok) break;
-          const float* S = sS + (hs % GE::RING) * L;
-          f = __expf(which ? S[L - 1] - S[row] : S[row]);
-        }
-        ok = all(wait(CFULL + s, (uint32_t)(m >> 1), 128u));
+    for (int j = 0; j <= nh && ok; ++j) {
+      const int s = j % CB;
+      float f = 1.0f;
+      if (j < nh) {
+        ok = all(wait(SRDY + (j % GE::RING), (uint32_t)(j / GE::RING), 128u));
         if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          uint32_t v[16];
-          tmem_ld16(src + (uint32_t)(64 * s + 16 * q), v);
-          tmem_wait_ld();
-#pragma unroll
-          for (int e = 0; e < 16; ++e) acc[16 * q + e] = fmaf(__uint_as_float(v[e]), f, acc[16 * q + e]);
-        }
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(CFREE + s));
-        if (j < nh) {
-          if (lane == 0) {
-            mbar_arrive(bar(SFREE + (hs % GE::RING)));
-            if (ps > 0) mbar_arrive(bar(SFREE + (hs % GE::RING)));      // (the dG warps take part in the first pass only)
-          }
-          ++hs;
-        }
+        const float* S = sS + (j % GE::RING) * L;
+        f = __expf(which ? S[L - 1] - S[row] : S[row]);
       }
+      ok = all(wait(CFULL + s, (uint32_t)(j / CB), 128u));
       if (!ok) break;
-      const int t = i * L + row, w = p.N - 64 * ps;            // columns of this half (a multiple of 8)
-      if (p.nsplit > 1) {
-        float4* dst = reinterpret_cast<float4*>(p.part + ((((int64_t)tile * p.nsplit + split) * 2 + which) * L + row) * p.N + 64 * ps);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const F2 f2 = pack2(f, f);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) if (4 * e < w) dst[e] = make_float4(acc[4 * e], acc[4 * e + 1], acc[4 * e + 2], acc[4 * e + 3]);
-      } else if (t < p.T) {
-        const int64_t o = ((int64_t)bb * p.T + t) * p.ld + (int64_t)g * p.N + 64 * ps;
-        uint16_t* o16 = which ? p.db16 : p.dc16;
-        if (o16) {
+      for (int q = 0; q < CC / 16; ++q) {
+        uint32_t v[16];
+        tmem_ld16(src + (uint32_t)(64 * s + 16 * q), v);
+        tmem_wait_ld();
 #pragma unroll
-          for (int e = 0; e < 8; ++e)
-            if (8 * e < w) *reinterpret_cast<uint4*>(o16 + o + 8 * e) = make_uint4(pack2(acc[8 * e], acc[8 * e + 1]), pack2(acc[8 * e + 2], acc[8 * e + 3]),
-                                                                                    pack2(acc[8 * e + 4], acc[8 * e + 5]), pack2(acc[8 * e + 6], acc[8 * e + 7]));
-        } else {
-          float4* dst = reinterpret_cast<float4*>((which ? p.db : p.dc) + o);
+        for (int e = 0; e < 8; ++e) acc[8 * q + e] = fma2(pack2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])), f2, acc[8 * q + e]);
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) { mbar_arrive(bar(CFREE + s)); if (j < nh) mbar_arrive(bar(SFREE + (j % GE::RING))); }
+    }
+    const int t = i * L + row;
+    if (ok && p.nsplit > 1) {
+      float* dst = p.part + ((((int64_t)tile * p.nsplit + split) * 2 + which) * L + row) * p.N;
 #pragma unroll
-          for (int e = 0; e < 16; ++e) if (4 * e < w) dst[e] = make_float4(acc[4 * e], acc[4 * e + 1], acc[4 * e + 2], acc[4 * e + 3]);
-        }
+      for (int e = 0; e < CC / 4; ++e) if (4 * e < p.N) store_quad(dst + 4 * e, Quad{acc[2 * e], acc[2 * e + 1]});
+    } else if (ok && t < p.T) {
+      const int64_t o = ((int64_t)bb * p.T + t) * p.ld + (int64_t)g * p.N;
+      uint16_t* o16 = which ? p.db16 : p.dc16;
+      if (o16) {
+        auto two = [&](int e) { const float2 u = unpack2(acc[e]); return bf16_of_two(u.x, u.y); };
+#pragma unroll
+        for (int e = 0; e < CC / 8; ++e)
+          if (8 * e < p.N) *reinterpret_cast<uint4*>(o16 + o + 8 * e) = make_uint4(two(4 * e), two(4 * e + 1), two(4 * e + 2), two(4 * e + 3));
+      } else {
+        float* dst = (which ? p.db : p.dc) + o;
+#pragma unroll
+        for (int e = 0; e < CC / 4; ++e) if (4 * e < p.N) store_quad(dst + 4 * e, Quad{acc[2 * e], acc[2 * e + 1]});
       }
     }
   }
@@ -363,7 +380,7 @@ __global__ void __launch_bounds__(256) heads_sum_kernel(const float* __restrict_
   }
   const int64_t o = ((bi / p.n) * p.T + t) * p.ld + (int64_t)g * p.N + 4 * c;
   uint16_t* o16 = which ? p.db16 : p.dc16;
-  if (o16) *reinterpret_cast<uint2*>(o16 + o) = make_uint2(pack2(s.x, s.y), pack2(s.z, s.w));
+  if (o16) *reinterpret_cast<uint2*>(o16 + o) = make_uint2(bf16_of_two(s.x, s.y), bf16_of_two(s.z, s.w));
   else *reinterpret_cast<float4*>((which ? p.db : p.dc) + o) = s;
 }
 
@@ -372,9 +389,9 @@ static unsigned int* status_ptr() {
   return status_address(g_heads_status, known);
 }
 
-template <int NI, int ND>
+template <int NI, int ND, int NK>
 static pmb_status launch(cudaStream_t st, const HeadsArgs& a, int nsplit) {
-  using GE = Geo<NI, ND>;
+  using GE = Geo<NI, ND, NK>;
   static_assert(GE::SMEM <= 227 * 1024, "shared-memory plan");
   const int n = (int)cdiv(a.T, L);
   Maps ms{};
@@ -389,11 +406,11 @@ static pmb_status launch(cudaStream_t st, const HeadsArgs& a, int nsplit) {
     PMB_TRY(sf::bf16_map4(&ms.c[sp], lo ? a.c.lo : a.c.hi, a.N, a.T, a.G, a.B, a.c.pitch, a.N, (int64_t)a.T * a.c.pitch, 64, L));
   }
   Params p{};
-  p.T = a.T; p.H = a.H; p.G = a.G; p.hpg = a.H / a.G; p.N = a.N; p.n = n; p.nsplit = nsplit; p.passes = (int)cdiv(a.N, 64);
+  p.T = a.T; p.H = a.H; p.G = a.G; p.hpg = a.H / a.G; p.N = a.N; p.n = n; p.nsplit = nsplit;
   p.S = a.S; p.dc = a.dc; p.db = a.db; p.ld = a.ld; p.dc16 = a.dc16; p.db16 = a.db16; p.part = a.part; p.status = status_ptr();
   const int64_t tiles = (int64_t)a.B * n * a.G;
-  PMB_SMEM_OPT_IN(GE::SMEM, ssd_heads_kernel<NI, ND>);
-  PMB_TRY(launch_pdl(st, ssd_heads_kernel<NI, ND>, dim3((unsigned)((tiles * nsplit))), NTHREADS, GE::SMEM, ms, p));
+  PMB_SMEM_OPT_IN(GE::SMEM, ssd_heads_kernel<NI, ND, NK>);
+  PMB_TRY(launch_pdl(st, ssd_heads_kernel<NI, ND, NK>, dim3((unsigned)((tiles * nsplit))), GE::NTHREADS, GE::SMEM, ms, p));
   if (nsplit > 1) {
     const int64_t total = tiles * 2 * L * (a.N / 4);
     PMB_TRY(launch_pdl(st, heads_sum_kernel, dim3((unsigned)cdiv(total, 256)), 256, 0, a.part, p, total));
@@ -428,8 +445,9 @@ pmb_status ssd_heads(cudaStream_t st, const HeadsArgs& a) {
   if (!al16(a.dc) || !al16(a.db) || !al16(a.dc16) || !al16(a.db16) || !al16(a.part) || (a.ld & (a.dc16 ? 7 : 3))) return fail(PMB_ERR_SHAPE, "ssd_heads: dB and dC rows must be 16-byte aligned");
   const double tok = (double)a.B * a.T;
   ProfScope prof(st, "ssd_heads", tok * (a.H * ((double)SCAN_STEP * a.P + 4.0 * a.N * a.P) + 2.0 * a.G * SCAN_STEP * a.N), 0.0);
-  if (pairs) return shd::launch<2, 2>(st, a, nsplit);
-  return a.hp_lo ? shd::launch<1, 2>(st, a, nsplit) : shd::launch<1, 1>(st, a, nsplit);
+  if (pairs) return shd::launch<2, 2, 1>(st, a, nsplit);      // (d_state up to 64)
+  if (a.N > 64) return a.hp_lo ? shd::launch<1, 2, 2>(st, a, nsplit) : shd::launch<1, 1, 2>(st, a, nsplit);
+  return a.hp_lo ? shd::launch<1, 2, 1>(st, a, nsplit) : shd::launch<1, 1, 1>(st, a, nsplit);
 }
 
 }  // namespace pmb
