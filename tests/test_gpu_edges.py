@@ -765,3 +765,24 @@ def test_bf16_block_of_more_chains_than_sms(pm, B, T, Q):
         assert torch.equal(out[lo:hi], blk.forward(x[lo:hi].contiguous()))
         assert_close(dx[lo:hi].float(), blk.backward(x[lo:hi].contiguous(), dout[lo:hi].contiguous())[0].float(), tol=2e-2, what="dx")
     assert pm.device_status() == 0
+
+
+# the sums of in_proj's K splits with the conv step: four columns to a thread where the window and the conv weights lie on the 16-byte grid and
+# the taps are four, a column to a thread elsewhere.  Against the oracle's step, as above.
+@pytest.mark.parametrize("K,offset", [(4, 0), (4, 1), (3, 0), (2, 0)])
+@pytest.mark.parametrize("B,N", [(17, 64), (33, 4), (200, 128)])
+def test_decode_finish(pm, B, N, K, offset):
+    cfg = orc.Mamba2Config(64, N, 32, 4, 1, K, 64)
+    p = orc.init_block_params(cfg, seed=5)
+    blk = pm.Mamba2Block(pm.Mamba2Config(d_model=64, d_state=N, d_head=32, n_heads=4, n_groups=1, d_conv=K, block_len=64), {k: v.cuda() for k, v in p.items()})
+    st, st_o = blk.zero_state(B), orc.zero_state(cfg, B)
+    win = torch.empty(st["conv_window"].numel() + offset, device="cuda")[offset:].view_as(st["conv_window"])
+    win.copy_(randn(tuple(win.shape), 2).cuda())
+    st["conv_window"] = win
+    st_o["conv_window"] = win.cpu().clone()
+    for t in range(2):
+        x = randn((B, 1, 64), 10 + t)
+        y, st = blk.step(x.cuda(), st)
+        y_o, st_o = orc.block_step(p, cfg, x, st_o)
+        assert_close(y, y_o, what="y")
+        assert_close(st["conv_window"], st_o["conv_window"], what="window")
