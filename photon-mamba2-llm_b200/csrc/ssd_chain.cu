@@ -32,7 +32,7 @@
 //  - the kernel's 63 KB are about what the instruction cache holds for seven roles: an early return and a few selects by block, 72 KB, cost 8 %;
 //  - the segment is the grid's y and not a remainder that stays in a register: on pairs its spills cost 10 % (24.6 -> 22.2 us at 4 x 512).
 // Measured at 24 heads of 64 x 64: 22 us for 4 x 512 tokens on pairs, 25 with what a backward reads (23.9 and 26 before the above); 8 x 2048 on
-// plain operands in chunks of 256, 100 us, and 117 with all that a chunk-by-chunk backward reads (118 and 144 where every CTA walks whole chains, see
+// plain operands in chunks of 256, 90 us, and 109 with all that a chunk-by-chunk backward reads (118 and 144 where every CTA walks whole chains, see
 // ssd_chain_wrap); 31 us (two launches over segments) for 1 x 1337 on pairs.  Every mbarrier wait is bounded; on expiry the CTA raises the status
 // word, every role stops issuing work, copies in flight are waited for (bounded) and TMEM is freed on the way out.
 #include <cuda_bf16.h>
