@@ -228,9 +228,9 @@ static Pair16 weight_pair(const Weights16* wx, bool in_proj, const float* src, i
   return Pair16{hi, lo, cols};
 }
 
-// x_pair_ready: the (hi, lo) pair of x is already in the workspace (written by the GEMM that produced x)
+// x_pair_ready: the (hi, lo) pair of x is already in the workspace (written by the GEMM that produced x); split_done: the weight's too
 static pmb_status block_fwd_core(cudaStream_t st, const Dims& d, const pmb_block_params& p, const void* x, const BlockWs& w,
-                                 const Weights16* wx, bool x_pair_ready = false) {
+                                 const Weights16* wx, bool x_pair_ready = false, bool split_done = false) {
   const Weights16* w16 = storage_is_bf16(wx) ? wx : nullptr;
   const bool pr = !w16 && block_uses_pairs(d);
   if (w16) PMB_TRY(gemm_bf16(st, 0, 0, d.M, d.J, d.D, x, d.D, w16->in_proj, d.J, w.xzd, d.J, nullptr, 0));
@@ -238,7 +238,7 @@ static pmb_status block_fwd_core(cudaStream_t st, const Dims& d, const pmb_block
     Splits todo;
     if (!x_pair_ready) todo.add(static_cast<const float*>(x), (int64_t)d.M * d.D, w.x_hi, w.x_lo);
     const Pair16 win = weight_pair(wx, true, p.in_proj_weight, d.D, d.J, w.win_hi, w.win_lo, &todo);
-    PMB_TRY(todo.run(st));
+    if (!split_done) PMB_TRY(todo.run(st));
     PMB_TRY(gemm_pairs(st, 0, 0, d.M, d.J, d.D, Pair16{w.x_hi, w.x_lo, d.D}, win, w.xzd, d.J, nullptr));
   }
   else PMB_TRY(gemm(st, 0, 0, d.M, d.J, d.D, static_cast<const float*>(x), d.D, p.in_proj_weight, d.J, w.xzd, d.J, nullptr, 0));
@@ -360,17 +360,17 @@ pmb_status block_fwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, 
 // block_bwd runs both on one stream; stack_bwd runs the recompute of block l-1 on a second stream while the
 // gradient kernels of block l are in flight (two forward slots).
 static pmb_status block_recompute(cudaStream_t st, const Dims& d, const pmb_block_params& p, const void* x, void* ws, size_t ws_bytes,
-                                  const Weights16* wx, int nslots, int slot) {
+                                  const Weights16* wx, int nslots, int slot, bool split_done = false) {
   const bool bf = storage_is_bf16(wx);
   BlockWs w;
   if (block_ws_layout(d, ws, ws_bytes, &w, bf, nslots, slot, wx && wx->pairs) == 0 || !ws)
     return fail(PMB_ERR_WORKSPACE, "block workspace too small (%zu < %zu)", ws_bytes, block_ws_layout(d, nullptr, 0, nullptr, bf, nslots, 0));
-  return block_fwd_core(st, d, p, x, w, wx);
+  return block_fwd_core(st, d, p, x, w, wx, split_done, split_done);
 }
 
 static pmb_status block_grads(cudaStream_t st, const Dims& d, const pmb_block_params& p, const void* x, const void* dout,
                               const void* dx_accum, void* dx, const pmb_block_grads& g, void* ws, size_t ws_bytes, const Weights16* wx,
-                              int nslots, int slot, cudaEvent_t recompute_done, bool dout_pair_ready = false, bool emit_dx_pair = false) {
+                              int nslots, int slot, cudaEvent_t recompute_done, bool dout_pair_ready = false, bool emit_dx_pair = false, SideLane* early = nullptr) {
   const Weights16* w16 = storage_is_bf16(wx) ? wx : nullptr;
   const bool pr = !w16 && block_uses_pairs(d);
   BlockWs w;
@@ -379,8 +379,9 @@ static pmb_status block_grads(cudaStream_t st, const Dims& d, const pmb_block_pa
   // The out_proj gradients do not wait for the recompute (dnormed = dout W_out^T needs neither x nor the recomputed
   // activations) and dW_out is needed only when the block is done: with pair GEMMs both go to a side stream, where
   // their CTAs fill the SMs that the latency-bound recompute and scan kernels leave idle.
-  SideLane* gl = nullptr;
-  if (pr) {
+  // (early: dnormed has been enqueued there, with ev[1] behind it, and the operands have been split)
+  SideLane* gl = early;
+  if (pr && !gl) {
     static const int on = [] { const char* e = getenv("PMB_BLOCK_CONCURRENT"); return (e && e[0] == '0') ? 0 : 1; }();
     if (on) PMB_TRY(get_side_lane(1, &gl));
   }
@@ -390,9 +391,9 @@ static pmb_status block_grads(cudaStream_t st, const Dims& d, const pmb_block_pa
     Splits todo;
     if (!dout_pair_ready) todo.add(static_cast<const float*>(dout), (int64_t)d.M * d.D, w.dout_hi, w.dout_lo);
     wout = weight_pair(wx, false, p.out_proj_weight, d.I, d.D, w.wout_hi, w.wout_lo, &todo);
-    PMB_TRY(todo.run(st));
+    if (!early) PMB_TRY(todo.run(st));
     // dnormed heads the critical chain of this block: it stays on the caller's stream; only dW_out is deferred
-    if (gl) PMB_TRY(gemm_pairs(st, 0, 1, d.M, d.I, d.D, dop, wout, w.dnormed, d.I, nullptr));
+    if (gl && !early) PMB_TRY(gemm_pairs(st, 0, 1, d.M, d.I, d.D, dop, wout, w.dnormed, d.I, nullptr));
   }
   // the recomputed activations (enqueued by the caller, possibly on another stream) are needed from here on
   if (recompute_done) PMB_CUDA(cudaStreamWaitEvent(st, recompute_done, 0));
@@ -418,6 +419,7 @@ static pmb_status block_grads(cudaStream_t st, const Dims& d, const pmb_block_pa
     PMB_TRY(gemm(st, 1, 0, d.I, d.D, d.M, w.normed, d.I, df, d.D, g.out_proj_weight, d.D, nullptr, 0));
     PMB_TRY(gemm(st, 0, 1, d.M, d.I, d.D, df, d.D, p.out_proj_weight, d.D, w.dnormed, d.I, nullptr, 0));
   }
+  if (early) PMB_CUDA(cudaStreamWaitEvent(st, early->ev[1], 0));      // dnormed
   // gate + norm: dy (in place over dnormed), dz -> z columns of dxzd
   // With pair GEMMs the three producers of dxzd (this kernel: dz; the scan's dt path: ddt_raw; the conv backward:
   // dxBC) write the (hi, lo) pair directly and the fp32 dxzd is never formed.  The norm backward also emits
@@ -525,8 +527,30 @@ static pmb_status block_grads(cudaStream_t st, const Dims& d, const pmb_block_pa
 pmb_status block_bwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, const void* x, const void* dout,
                      const void* dx_accum, void* dx, const pmb_block_grads& g, void* ws, size_t ws_bytes, const Weights16* wx,
                      bool dout_pair_ready, bool emit_dx_pair) {
-  PMB_TRY(block_recompute(st, d, p, x, ws, ws_bytes, wx, 1, 0));
-  return block_grads(st, d, p, x, dout, dx_accum, dx, g, ws, ws_bytes, wx, 1, 0, nullptr, dout_pair_ready, emit_dx_pair);
+  // On pairs dnormed = dout W_out^T, which needs nothing of the recompute, runs beside it, and what both multiply is split in one launch, as long as
+  // the recompute's projection leaves room beside it.  Backward in us, after the recompute / beside it, by tiles of in_proj: 3 (2 x 128 tokens, 8
+  // heads of 32 x 16) 115 / 109, 10 (2 x 256, 16 of 64 x 64) 125 / 115, 39 (2 x 384, 24) 188 / 172, 52 200 / 188, 68 237 / 229, 78 238 / 231, but
+  // 104 259 / 275, 136 361 / 360.  (In bf16 storage that product shares a launch with dW_out's, whose tiles it fills up: alone it cost as often as it
+  // gave, 8 x 512 tokens 330 -> 339, 7 x 2048 903 -> 870.)
+  static const int on = [] { const char* e = getenv("PMB_BLOCK_CONCURRENT"); return (e && e[0] == '0') ? 0 : 1; }();
+  SideLane* early = nullptr;
+  if (on && !storage_is_bf16(wx) && block_uses_pairs(d) && tiles256(d.M, d.J) <= 80) PMB_TRY(get_side_lane(1, &early));
+  if (early) {
+    BlockWs w;
+    if (block_ws_layout(d, ws, ws_bytes, &w, false, 1, 0, wx && wx->pairs) == 0 || !ws)
+      return fail(PMB_ERR_WORKSPACE, "block workspace too small (%zu < %zu)", ws_bytes, block_ws_layout(d, nullptr, 0, nullptr, false, 1, 0));
+    Splits todo;
+    todo.add(static_cast<const float*>(x), (int64_t)d.M * d.D, w.x_hi, w.x_lo);
+    weight_pair(wx, true, p.in_proj_weight, d.D, d.J, w.win_hi, w.win_lo, &todo);
+    if (!dout_pair_ready) todo.add(static_cast<const float*>(dout), (int64_t)d.M * d.D, w.dout_hi, w.dout_lo);
+    const Pair16 wout = weight_pair(wx, false, p.out_proj_weight, d.I, d.D, w.wout_hi, w.wout_lo, &todo);
+    PMB_TRY(todo.run(st));
+    PMB_TRY(order_after(st, early->ev[2], early->s));
+    PMB_TRY(gemm_pairs(early->s, 0, 1, d.M, d.I, d.D, Pair16{w.dout_hi, w.dout_lo, d.D}, wout, w.dnormed, d.I, nullptr));
+    PMB_CUDA(cudaEventRecord(early->ev[1], early->s));
+  }
+  PMB_TRY(block_recompute(st, d, p, x, ws, ws_bytes, wx, 1, 0, early != nullptr));
+  return block_grads(st, d, p, x, dout, dx_accum, dx, g, ws, ws_bytes, wx, 1, 0, nullptr, dout_pair_ready, emit_dx_pair, early);
 }
 
 }  // namespace pmb
