@@ -5,7 +5,8 @@
 //   1. G = R K^T on the tensor core into one of two TMEM buffers (R = the CTA's 128 rows of C, K = 64 rows of B in
 //      mode 0; the roles of B and C swap in mode 1), K = d_state;
 //   2. four warps read G from TMEM (thread = row), multiply by exp(S_row - S_col) with the causal test in fp32
-//      registers, and write the masked tile back over G as a bf16 operand (hi and lo halves of the fp32 value in pair mode);
+//      registers (two elements to an operation, selects only where the diagonal crosses, exponentials below 2^-126 zeros: the fp32 scan of 8 x 2048
+//      tokens, 32 heads of 64 x 64, chunks of 256, 386 -> 382 us forward and 791 -> 737 backward, same bits), and write the masked tile back over G as a bf16 operand (hi and lo halves of the fp32 value in pair mode);
 //   3. acc1 += masked tile x V (V = 64 rows of x~ in mode 0, of dY in mode 1; MN-major) on the tensor core;
 // while step 2 of block j runs, the tensor core already computes step 1 of block j+1.  The carried-state term
 // (C h_prev in mode 0, B dh in mode 1) goes to a second accumulator and is scaled per row in the epilogue, which
@@ -27,6 +28,7 @@
 // column blocks), so the mask work of two blocks and the tensor-core work of a third overlap.  Every mbarrier wait is bounded; on
 // expiry the CTA raises the status word, stops issuing work, and leaves through the common exit (TMEM freed).
 #include <cuda_bf16.h>
+#include <type_traits>
 #include <algorithm>
 #include <mutex>
 #include <unordered_map>
@@ -343,6 +345,7 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
       asm volatile("bar.sync 3, %0;" ::"n"(NMASK) : "memory");
     }
     const float S_row = sS[row];
+    const F2 Sr2 = pack2(S_row, S_row), nSr2 = pack2(-S_row, -S_row), neg = pack2(-1.0f, -1.0f), log2e = pack2(1.4426950408889634f, 1.4426950408889634f);
     bool ok = true;
     float c_acc = 0.0f;                                 // mode 1: sum over t > s of W[t,s] for this thread's row s
     // Every iteration reaches the named barrier below whatever happened before it (a warp that gave up skips the
@@ -364,29 +367,40 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
             for (int e = 0; e < 32; ++e) wv[e] = __uint_as_float(d[e]);
           }
           uint32_t mh[16], ml[16];                  // this half's packed hi / lo values
+          // (no column past the diagonal for any row of the warp: no selects)
+          const int b0 = c0 + half * 32, w0r = rb * RB + quarter * 32;
+          const bool inside = MODE == 0 ? b0 + 31 <= w0r : b0 > w0r + 31;
+          auto block = [&](auto all_inside) {
+            constexpr bool IN = decltype(all_inside)::value;
 #pragma unroll
-          for (int q8 = 0; q8 < 4; ++q8) {
+            for (int e4 = 0; e4 < 8; ++e4) {
+              const ulonglong2 s4 = *reinterpret_cast<const ulonglong2*>(sS + b0 + 4 * e4);
 #pragma unroll
-            for (int e2 = 0; e2 < 4; ++e2) {
-              const int e = q8 * 8 + 2 * e2;
-              const int col = c0 + half * 32 + e;
-              const float2 sc = *reinterpret_cast<const float2*>(sS + col);
-              float m0, m1;
-              if (MODE == 0) {       // row = t, col = s: exp(S_t - S_s) for s <= t
-                m0 = col <= row ? __uint_as_float(r[e]) * __expf(S_row - sc.x) : 0.0f;
-                m1 = col + 1 <= row ? __uint_as_float(r[e + 1]) * __expf(S_row - sc.y) : 0.0f;
-              } else {               // row = s, col = t: exp(S_t - S_s) for t >= s
-                m0 = col >= row ? __uint_as_float(r[e]) * __expf(sc.x - S_row) : 0.0f;
-                m1 = col + 1 >= row ? __uint_as_float(r[e + 1]) * __expf(sc.y - S_row) : 0.0f;
-                // W[t,s] for t > s (the diagonal does not depend on S)
-                wv[e] = col > row ? wv[e] * m0 : 0.0f;
-                wv[e + 1] = col + 1 > row ? wv[e + 1] * m1 : 0.0f;
-                c_acc += wv[e] + wv[e + 1];
+              for (int u = 0; u < 2; ++u) {
+                const int e = 4 * e4 + 2 * u, col = b0 + e;
+                const F2 sc = u ? s4.y : s4.x;
+                // MODE 0: row = t, col = s: exp(S_t - S_s) for s <= t;  MODE 1: row = s, col = t: exp(S_t - S_s) for t >= s
+                const float2 x = unpack2(mul2(MODE == 0 ? fma2(sc, neg, Sr2) : add2(sc, nSr2), log2e));
+                const F2 g2 = pack2(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
+                F2 m2 = mul2(g2, pack2(ex2_ftz(x.x), ex2_ftz(x.y)));
+                float2 m = unpack2(m2);
+                if (!IN) {
+                  m.x = (MODE == 0 ? col <= row : col >= row) ? m.x : 0.0f;
+                  m.y = (MODE == 0 ? col + 1 <= row : col + 1 >= row) ? m.y : 0.0f;
+                  m2 = pack2(m.x, m.y);
+                }
+                if (MODE == 1) {       // W[t,s] for t > s (the diagonal does not depend on S)
+                  const float2 w = unpack2(mul2(pack2(wv[e], wv[e + 1]), m2));
+                  wv[e] = IN || col > row ? w.x : 0.0f;
+                  wv[e + 1] = IN || col + 1 > row ? w.y : 0.0f;
+                  c_acc += wv[e] + wv[e + 1];
+                }
+                ml[e >> 1] = 0u;
+                split2(m.x, m.y, mh[e >> 1], ml[e >> 1], NS == 2);
               }
-              ml[q8 * 4 + e2] = 0u;
-              split2(m0, m1, mh[q8 * 4 + e2], ml[q8 * 4 + e2], NS == 2);
             }
-          }
+          };
+          if (inside) block(std::true_type{}); else block(std::false_type{});
           // over the 32 columns of G just read: [hi of these 32 k | lo of these 32 k]
           tmem_st16(tG + lane_addr + (uint32_t)(mb * CW + half * 32), mh);
           if (NS == 2) tmem_st16(tG + lane_addr + (uint32_t)(mb * CW + half * 32 + 16), ml);
