@@ -21,7 +21,7 @@
 // What bounds it: no pipe and no memory level.  A step takes 8000 warp instructions at d_state 128 on plain operands, issued in 41 % of the
 // cycles; every role is a chain of TMEM loads, shared memory and arithmetic with two warps of it on a scheduler.  What shaped the roles are
 // clocks read inside a step of 16 x 8192 tokens, 32 heads of 128 x 64, bf16 (927 us when masking and output were one role and one warp issued
-// all products, 720 now):
+// all products, 622 now):
 //  - the products are issued by two warps: with one, its waits and the issue took 5000 of a step's 5200 clocks.  The warp index comes from a
 //    shuffle, so that the roles' branches and the descriptors are uniform to the compiler (742 -> 711 us, this kernel alone);
 //  - B and C are given back before the masked product waits for the mask, so that the next tiles (2200 clocks) land while it is masked;
@@ -29,6 +29,9 @@
 //  - a and dt are requested two chunks ahead (a head's tokens are a line apart), and below the diagonal the masked tile takes one
 //    exponential per row and block of 32 columns instead of one per element (not where M is rounded for a stream of bf16 values, see FACT);
 //  - the masked tile's exponents and products go in pairs, exponentials below 2^-126 are zeros (16 x 8192 709 -> 688 us, one prompt of 1337 95.5 -> 94.9);
+//  - the states that a backward reads leave by TMA from the operand tile, where they lie: stored by the threads that hold their rows, 32 lines to an
+//    instruction, they took half of the state's 4900 clocks of a step's 5700 (16 x 8192 710 -> 622 us, 9 x 1400 of 64 x 64 118 -> 102,
+//    16 x 512 of 128 x 64 61.5 -> 56.5);
 //  - the kernel's 63 KB are about what the instruction cache holds for seven roles: an early return and a few selects by block, 72 KB, cost 8 %;
 //  - the segment is the grid's y and not a remainder that stays in a register: on pairs its spills cost 10 % (24.6 -> 22.2 us at 4 x 512).
 // Measured at 24 heads of 64 x 64: 22 us for 4 x 512 tokens on pairs, 25 with what a backward reads (23.9 and 26 before the above); 8 x 2048 on
@@ -98,7 +101,7 @@ struct Geo {
   static constexpr int SMEM = TILES + SLACK + BARS + NSB * SLOT * 4 + (BIG ? 4 : 8) * NB * L /*row factors*/ + AHEAD * XF_THREADS * 16;
 };
 
-struct Maps { CUtensorMap b[2], c[2], x, xt, xs; };      // [0] = hi (or the plain bf16 tensor), [1] = lo; x = bf16 x
+struct Maps { CUtensorMap b[2], c[2], x, xt, xs, h[2]; };      // [0] = hi (or the plain bf16 tensor), [1] = lo; x = bf16 x; h = the states kept, 32 rows to a box
 
 struct Params {
   int T, H, hpg, N, P, nsteps;
@@ -109,7 +112,7 @@ struct Params {
   const float* init;                                     // (B,H,N,P) or NULL
   float* y; uint16_t* y16; int64_t ldy;
   float* dt_out; float* A_out; float* S_out;             // optional from here on: what a backward reads
-  uint16_t *hp_hi, *hp_lo;                               // (B,nsteps,H,N,P)
+  int keep_h;                                            // the states entering the chunks go out, (B,chunks,H,N,P)
   float* last;                                           // (B,H,N,P)
   // plain operands, for a backward that works chunk by chunk: state entering each chunk in fp32, and (store_ops) x~ and xs as the
   // kernel formed them.  bf16 x: store_ops leaves a copy of it.
@@ -668,6 +671,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const bool active = nr < p.N;                           // rows past d_state hold zeros
     const bool tile = quarter * 32 < 64 * NK;               // this warp's rows exist in the operand tile
+    const bool kept = p.keep_h && !state_only && quarter * 32 < p.N;      // (N <= 64 NK; rows from N on are outside the map)
     const int64_t NP = (int64_t)p.N * p.P;
     float hv[PW];
     bool ok = true;
@@ -704,6 +708,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       if (i > 0 && !state_only) ok = __all_sync(0xffffffffu, wait(HFREE, (uint32_t)(i - 1), 256u));
       if (!ok) break;
       const int64_t so = (((int64_t)bb * ncht + i0 / NB + i) * p.H + h) * NP + (int64_t)nr * p.P;
+      if (kept && i > 0) {                                  // (the stores of the state before have read its rows)
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        __syncwarp();
+      }
       if (tile && !state_only) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {                       // eight 16-byte chunks of the row
@@ -718,17 +726,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(HRDY));
-      // (what a backward keeps goes out after the operand tile, under the products that read it)
-      if (p.hp_hi && active && !state_only) {
-#pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          if (8 * c >= p.P) continue;
-          uint32_t hi[4], lo[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) split2(hv[8 * c + 2 * e], hv[8 * c + 2 * e + 1], hi[e], lo[e], ND == 2);
-          *reinterpret_cast<uint4*>(p.hp_hi + so + 8 * c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          if (ND == 2) *reinterpret_cast<uint4*>(p.hp_lo + so + 8 * c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-        }
+      // What a backward keeps goes out as it lies in the operand tile, a warp's 32 rows by themselves, under the products that read it (a thread
+      // that stored its own row would touch 32 lines with every instruction)
+      if (kept && lane == 0) {
+        tma_store_4d(&maps.h[0], h_s + (uint32_t)quarter * (32 * 128), 0, quarter * 32, h, bb * ncht + i0 / NB + i);
+        if (ND == 2) tma_store_4d(&maps.h[1], h_s + NK * T64 + (uint32_t)quarter * (32 * 128), 0, quarter * 32, h, bb * ncht + i0 / NB + i);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       }
       if (ND == 1 && p.hprev && active) {
 #pragma unroll
@@ -754,6 +757,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(UFREE));
     }
+    if (kept && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     const int64_t row = (int64_t)blockIdx.x * gridDim.y + blockIdx.y;
     if (ok && state_only && nr == 0) p.seg_d[row] = __expf(stot);
     const bool handed = WRAP && i0 + n < p.nsteps;      // the beginning of a chain whose rest another CTA walks
@@ -806,7 +810,11 @@ static pmb_status launch(cudaStream_t st, const ChainArgs& a) {
     PMB_TRY(sf::bf16_map4(&ms.xt, keep, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
     if (!XIN16) PMB_TRY(sf::bf16_map4(&ms.xs, a.xs, a.P, a.T, a.H, a.B, hp, a.P, a.T * hp, 64, L));
   }
-  p.hp_hi = a.hp_hi; p.hp_lo = a.hp_lo; p.last = a.last; p.status = status_ptr();
+  p.keep_h = a.hp_hi != nullptr; p.last = a.last; p.status = status_ptr();
+  for (int sp = 0; sp < ND && a.hp_hi; ++sp) {
+    const int64_t st_h = (int64_t)a.N * a.P, chunks = cdiv(p.nsteps, NB);
+    PMB_TRY(sf::bf16_map4(&ms.h[sp], sp ? a.hp_lo : a.hp_hi, a.P, a.N, a.H, a.B * chunks, a.P, st_h, a.H * st_h, 64, 32));
+  }
   const int chains = a.B * a.H;
   ChainWrap wr{};
   if constexpr (NI == 1 && !XIN16) {

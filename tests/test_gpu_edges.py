@@ -786,3 +786,21 @@ def test_decode_finish(pm, B, N, K, offset):
         y_o, st_o = orc.block_step(p, cfg, x, st_o)
         assert_close(y, y_o, what="y")
         assert_close(st["conv_window"], st_o["conv_window"], what="window")
+
+
+# the states that a backward reads leave in boxes of 32 rows: d_state at and around the boxes' edges, d_head below the box's width (a box that wrote
+# past its state would change the next head's).  On bf16 (several chunks of 128) and as pairs (a ragged length); bounds as in the tests above.
+@pytest.mark.parametrize("N,P", [(8, 8), (24, 64), (32, 40), (40, 64), (64, 56), (72, 64), (96, 24), (104, 8), (128, 64)])
+@pytest.mark.parametrize("T", [384, 300])
+def test_scan_bf16_kept_states(pm, T, N, P):
+    B, H, G = 2, 6, 1
+    x, b, c, dy = randn((B, T, H, P), 1).bfloat16(), randn((B, T, G, N), 2).bfloat16(), randn((B, T, G, N), 3).bfloat16(), randn((B, T, H, P), 4).bfloat16()
+    a = -torch.nn.functional.softplus(randn((B, T, H), 5) - 2.0)
+    scan = pm.SsdScanBf16(x.cuda(), a.cuda(), b.cuda(), c.cuda(), 128)
+    scan.forward()
+    dx, da, db, dc = scan.backward(dy.cuda())
+    assert pm.device_status() == 0
+    leaves = [t.double().requires_grad_(True) for t in (x, a, b, c)]
+    orc.ssd_scan_chunked(leaves[0], leaves[1], *(t.expand(B, T, H, N) for t in leaves[2:]), 128 if T % 128 == 0 else T).backward(dy.double())
+    for got, ref, tol, what in ((dx.float(), leaves[0].grad, 5e-3, "dx"), (da, leaves[1].grad, 5e-3, "da"), (db.float(), leaves[2].grad, 5e-3, "db"), (dc.float(), leaves[3].grad, 5e-3, "dc")):
+        assert_close(got, ref, tol=tol, what=what)
