@@ -532,6 +532,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     // x: every thread copies the pieces that it will read itself, AHEAD passes before it reads them, into a ring of its own
     // (cp.async; no barrier; rows past the end arrive as zeros)
     constexpr int RING = GE::AHEAD > 0 ? GE::AHEAD : 1;
+    // Pieces that a thread takes, and requests, together: one by one, a piece's wait, shared memory and roundings were a chain of their own, and on plain
+    // operands this role is the busiest (6700 of a step's 6900 clocks).  Block forward of 24 heads, chunks of 256, 8 x 2048 tokens 317 -> 314 us,
+    // 8 x 4096 580 -> 574.  S formed a chunk ahead by warp 3 alone, which takes it out of this role, lost: 16 x 8192 of bf16 x 2342 -> 2448
+    constexpr int UB = RING % 4 == 0 ? 4 : 1;
+    static_assert(RING == 1 || UB == 1 || RING == NIT, "a ring of a step's pieces");
     const uint32_t xring = smem_u32(sfac + NB * L) + (uint32_t)tid * 16u;
     const char* src = reinterpret_cast<const char*>(p.x + (tokb + toff + r0) * p.ldx + h * p.P + (jcol ? EPL * j : 0));
     const int64_t sstep = (int64_t)RPI * p.ldx * 4;
@@ -539,7 +544,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     auto request = [&](uint32_t slot) {
       const bool in = frow < p.T && jcol;
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(xring + slot), "l"(src), "r"(in ? 16 : 0) : "memory");
-      asm volatile("cp.async.commit_group;" ::: "memory");
       frow += RPI;
       if (frow < p.T) src += sstep;                         // (the address stays inside the tensor)
     };
@@ -557,7 +561,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
     if (GE::AHEAD > 0) {
       if (frow >= p.T) src = reinterpret_cast<const char*>(p.x);
 #pragma unroll 1
-      for (int q = 0; q < RING; ++q) request((uint32_t)q * (XF_THREADS * 16));
+      for (int q = 0; q < RING; ++q) {
+        request((uint32_t)q * (XF_THREADS * 16));
+        if (q % UB == UB - 1) asm volatile("cp.async.commit_group;" ::: "memory");
+      }
     }
     fetch_a(0, av);
     fetch_a(1, an);
@@ -619,43 +626,54 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
       else if (ok && i >= XB) ok = __all_sync(0xffffffffu, wait(XFREE + (i % XB), (uint32_t)(i / XB - 1), 128u));
       if (ok) {
         uint32_t dst = xbuf_s + (i % XB) * GE::XBUF + place;
-#pragma unroll (XIN16 ? 4 : 2)
-        for (int it = 0; it < NIT; ++it, dst += RPI * 128) {
-          uint4 xq = make_uint4(0u, 0u, 0u, 0u);
-          if (XIN16) {
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(xq.x), "=r"(xq.y), "=r"(xq.z), "=r"(xq.w) : "r"(dst));
-          } else if (GE::AHEAD > 0) {
-            asm volatile("cp.async.wait_group %0;" ::"n"(RING - 1) : "memory");
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(xq.x), "=r"(xq.y), "=r"(xq.z), "=r"(xq.w) : "r"(xring + slot) : "memory");
-          } else {
-            if (frow < p.T && jcol) xq = *reinterpret_cast<const uint4*>(src);
-            frow += RPI; src += sstep;
-          }
-          const int rc = rb * L + it * RPI + r0;            // row of the chunk
-          const float2 f = GE::BIG ? make_float2(sdt[rc], __expf(sEnd[c & 3] - S[rc])) : sfac[rc];
-          if (XIN16) {
-            const uint32_t in4[4] = {xq.x, xq.y, xq.z, xq.w};
-            uint32_t s4[4], k4[4];
+#pragma unroll (XIN16 ? 4 : UB == 1 ? 2 : 1)
+        for (int it = 0; it < NIT; it += UB, dst += UB * RPI * 128) {
+          uint4 xq[UB];
+          if (GE::AHEAD > 0) asm volatile("cp.async.wait_group %0;" ::"n"(RING / UB - 1) : "memory");
 #pragma unroll
-            for (int e = 0; e < 4; ++e) split2(__uint_as_float(in4[e] << 16) * f.y, __uint_as_float(in4[e] & 0xffff0000u) * f.y, s4[e], k4[e], ND == 2);
-            st_shared_v4(dst + GE::XT, s4[0], s4[1], s4[2], s4[3]);
-            if (ND == 2) st_shared_v4(dst + GE::XT + T128, k4[0], k4[1], k4[2], k4[3]);
-          } else {
-            const float f0 = __uint_as_float(xq.x) * f.x, f1 = __uint_as_float(xq.y) * f.x, f2 = __uint_as_float(xq.z) * f.x, f3 = __uint_as_float(xq.w) * f.x;
-            uint32_t h0, h1, l0 = 0u, l1 = 0u, g0, g1, k0 = 0u, k1 = 0u;
-            split2(f0, f1, h0, l0, ND == 2); split2(f2, f3, h1, l1, ND == 2);
-            if (ND == 2) { split2(f0 * f.y, f1 * f.y, g0, k0, true); split2(f2 * f.y, f3 * f.y, g1, k1, true); }
-            else {                                          // (x (dt exp): rounded as the chunk-by-chunk kernels round it)
-              const float fx = f.x * f.y;
-              split2(__uint_as_float(xq.x) * fx, __uint_as_float(xq.y) * fx, g0, k0, false); split2(__uint_as_float(xq.z) * fx, __uint_as_float(xq.w) * fx, g1, k1, false);
+          for (int u = 0; u < UB; ++u) {
+            xq[u] = make_uint4(0u, 0u, 0u, 0u);
+            if (XIN16) {
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(xq[u].x), "=r"(xq[u].y), "=r"(xq[u].z), "=r"(xq[u].w) : "r"(dst));
+            } else if (GE::AHEAD > 0) {
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(xq[u].x), "=r"(xq[u].y), "=r"(xq[u].z), "=r"(xq[u].w) : "r"(xring + slot + (uint32_t)(u * XF_THREADS * 16)) : "memory");
+            } else {
+              if (frow < p.T && jcol) xq[u] = *reinterpret_cast<const uint4*>(src);
+              frow += RPI; src += sstep;
             }
-            st_shared_v2(dst, h0, h1);
-            st_shared_v2(dst + GE::XT, g0, g1);
-            if (ND == 2) { st_shared_v2(dst + T128, l0, l1); st_shared_v2(dst + GE::XT + T128, k0, k1); }
           }
-          if (GE::AHEAD > 0) {
-            request(slot);                                  // (this pass has consumed the slot)
-            slot = slot + XF_THREADS * 16 == RING * XF_THREADS * 16 ? 0u : slot + XF_THREADS * 16;
+#pragma unroll
+          for (int u = 0; u < UB; ++u) {
+            const uint32_t du = dst + (uint32_t)(u * RPI * 128);
+            const int rc = rb * L + (it + u) * RPI + r0;      // row of the chunk
+            const float2 f = GE::BIG ? make_float2(sdt[rc], __expf(sEnd[c & 3] - S[rc])) : sfac[rc];
+            if (XIN16) {
+              const uint32_t in4[4] = {xq[u].x, xq[u].y, xq[u].z, xq[u].w};
+              uint32_t s4[4], k4[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) split2(__uint_as_float(in4[e] << 16) * f.y, __uint_as_float(in4[e] & 0xffff0000u) * f.y, s4[e], k4[e], ND == 2);
+              st_shared_v4(du + GE::XT, s4[0], s4[1], s4[2], s4[3]);
+              if (ND == 2) st_shared_v4(du + GE::XT + T128, k4[0], k4[1], k4[2], k4[3]);
+            } else {
+              const float x0 = __uint_as_float(xq[u].x), x1 = __uint_as_float(xq[u].y), x2 = __uint_as_float(xq[u].z), x3 = __uint_as_float(xq[u].w);
+              const float f0 = x0 * f.x, f1 = x1 * f.x, f2 = x2 * f.x, f3 = x3 * f.x;
+              uint32_t h0, h1, l0 = 0u, l1 = 0u, g0, g1, k0 = 0u, k1 = 0u;
+              split2(f0, f1, h0, l0, ND == 2); split2(f2, f3, h1, l1, ND == 2);
+              if (ND == 2) { split2(f0 * f.y, f1 * f.y, g0, k0, true); split2(f2 * f.y, f3 * f.y, g1, k1, true); }
+              else {                                          // (x (dt exp): rounded as the chunk-by-chunk kernels round it)
+                const float fx = f.x * f.y;
+                split2(x0 * fx, x1 * fx, g0, k0, false); split2(x2 * fx, x3 * fx, g1, k1, false);
+              }
+              st_shared_v2(du, h0, h1);
+              st_shared_v2(du + GE::XT, g0, g1);
+              if (ND == 2) { st_shared_v2(du + T128, l0, l1); st_shared_v2(du + GE::XT + T128, k0, k1); }
+            }
+          }
+          if (GE::AHEAD > 0) {                              // (this pass has consumed the slots)
+#pragma unroll
+            for (int u = 0; u < UB; ++u) request(slot + (uint32_t)(u * XF_THREADS * 16));
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            slot = slot + UB * XF_THREADS * 16 == RING * XF_THREADS * 16 ? 0u : slot + UB * XF_THREADS * 16;
           }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
