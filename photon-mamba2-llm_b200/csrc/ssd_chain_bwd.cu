@@ -71,7 +71,7 @@ struct Geo {
   static constexpr int SMEM = TILES + 1024 /*alignment slack*/ + 512 /*barriers, small sums*/ + (NSB * SLOT + 2 * ROWS) * 4 + 2 * AHEAD * XF_THREADS * 16;
 };
 
-struct Maps { CUtensorMap b[2], c[2], h[2], xt[2], dy[2]; };      // [0] = hi (or the plain bf16 tensor), [1] = lo; bf16: xt and dy are the inputs
+struct Maps { CUtensorMap b[2], c[2], h[2], dh[2], xt[2], dy[2]; };      // [0] = hi (or the plain bf16 tensor), [1] = lo; bf16: xt and dy are the inputs; dh goes out, 32 rows to a box
 
 struct Params {
   int T, H, hpg, N, P, nsteps;
@@ -82,7 +82,6 @@ struct Params {
   const float* D;
   float* dx; uint16_t* dx16; int64_t lddx;
   int store_ops;                                         // x~ and dY go out as bf16 operands (maps xt, dy)
-  uint16_t *dh_hi, *dh_lo;                               // (B,nsteps,H,N,P)
   float* da;                                             // (B,T,H)
   uint16_t *raw_hi, *raw_lo; int64_t ld_raw; int raw_col;                  // dt mode: gradient before the softplus as a bf16 pair (raw_lo may be NULL)
   float* part; int64_t part_pitch;                       // dt mode: per (b, h) sums for dA, dD and d_dt_bias, `part_pitch` apart
@@ -721,6 +720,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const bool active = nr < p.N;                           // rows past d_state hold zeros
     const bool tile = quarter * 32 < 64 * NK;               // this warp's rows exist in the operand tile
+    const bool kept = !state_only && quarter * 32 < p.N;      // (N <= 64 NK; rows from N on are outside the map)
     const int64_t NP = (int64_t)p.N * p.P;
     float hv[PW];
 #pragma unroll
@@ -761,7 +761,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       if (!state_only) {
         if (k > 0) ok = all(wait(HFREE, (uint32_t)(k - 1), 256u));
         if (!ok) break;
-        const int64_t so = (((int64_t)bb * p.nsteps + i) * p.H + h) * NP + (int64_t)nr * p.P;
+        if (kept && k > 0) {                                  // (the stores of the adjoint before have read its rows)
+          if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          __syncwarp();
+        }
         if (tile) {
 #pragma unroll
           for (int c = 0; c < 8; ++c) {                       // eight 16-byte chunks of the row
@@ -771,15 +774,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
             const uint32_t a = dh_s + (uint32_t)(nr * 128 + ((c ^ (nr & 7)) << 4));
             st_shared_v4(a, hi[0], hi[1], hi[2], hi[3]);
             if (ND == 2) st_shared_v4(a + NK * T64, lo[0], lo[1], lo[2], lo[3]);
-            if (active && 8 * c < p.P) {
-              *reinterpret_cast<uint4*>(p.dh_hi + so + 8 * c) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-              if (ND == 2) *reinterpret_cast<uint4*>(p.dh_lo + so + 8 * c) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-            }
           }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(HRDY));
+        // dh goes out as it lies in the operand tile, a warp's 32 rows by themselves (stored by the threads that hold its rows, an instruction
+        // touched 32 lines; backward of the scan at 9 x 1400 tokens, 32 heads of 64 x 64, kept as pairs, 216 -> 204 us, 16 x 1024 of 128 x 64
+        // 225 -> 220, four layers of 2 x 384 on pairs 935 -> 927 in all)
+        if (kept && lane == 0) {
+          tma_store_4d(&maps.dh[0], dh_s + (uint32_t)quarter * (32 * 128), 0, quarter * 32, h, bb * p.nsteps + i);
+          if (ND == 2) tma_store_4d(&maps.dh[1], dh_s + NK * T64 + (uint32_t)quarter * (32 * 128), 0, quarter * 32, h, bb * p.nsteps + i);
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
         // <dh, h>
         ok = all(wait(FULL, (uint32_t)k, 512u) && (k < 2 || wait(RFREE + (k & 1), (uint32_t)((k >> 1) - 1), 512u)));
         if (!ok) break;
@@ -823,6 +830,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_bwd_kernel(const __grid
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(UFREE));
     }
+    if (kept && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     const bool handed = WRAP && last + 1 > n;     // the end of a chain whose rest another CTA walks
     if (ok && (state_only || handed)) {
       const int64_t row = handed ? wr.e[blockIdx.x % CHAIN_SMS].sm + 1 : (int64_t)blockIdx.x * gridDim.y + blockIdx.y;
@@ -869,6 +877,7 @@ static pmb_status launch(cudaStream_t st, const ChainBwdArgs& a) {
     PMB_TRY(sf::bf16_map4(&ms.b[sp], lo ? a.b.lo : a.b.hi, a.N, a.T, a.G, a.B, a.b.pitch, a.N, (int64_t)a.T * a.b.pitch, 64, L));
     PMB_TRY(sf::bf16_map4(&ms.c[sp], lo ? a.c.lo : a.c.hi, a.N, a.T, a.G, a.B, a.c.pitch, a.N, (int64_t)a.T * a.c.pitch, 64, L));
     PMB_TRY(sf::bf16_map4(&ms.h[sp], lod ? a.hp_lo : a.hp_hi, a.P, a.N, a.H, (int64_t)a.B * n, a.P, st_h, a.H * st_h, 64, 64));
+    PMB_TRY(sf::bf16_map4(&ms.dh[sp], lod ? a.dh_lo : a.dh_hi, a.P, a.N, a.H, (int64_t)a.B * n, a.P, st_h, a.H * st_h, 64, 32));
     if (IN16 && !sp) {
       PMB_TRY(sf::bf16_map4(&ms.xt[0], a.x16, a.P, a.T, a.H, a.B, a.ldx, a.P, a.T * a.ldx, 64, L));
       PMB_TRY(sf::bf16_map4(&ms.dy[0], a.dy16, a.P, a.T, a.H, a.B, a.lddy, a.P, a.T * a.lddy, 64, L));
@@ -881,7 +890,7 @@ static pmb_status launch(cudaStream_t st, const ChainBwdArgs& a) {
   Params p{};
   p.T = a.T; p.H = a.H; p.hpg = a.H / a.G; p.N = a.N; p.P = a.P; p.nsteps = n;
   p.S = a.S; p.x = a.x; p.ldx = a.ldx; p.dy = a.dy; p.lddy = a.lddy; p.dt = a.dt; p.A = a.A; p.D = a.D;
-  p.dx = a.dx; p.dx16 = a.dx16; p.lddx = a.lddx; p.store_ops = a.xt_hi != nullptr; p.dh_hi = a.dh_hi; p.dh_lo = a.dh_lo; p.da = a.da;
+  p.dx = a.dx; p.dx16 = a.dx16; p.lddx = a.lddx; p.store_ops = a.xt_hi != nullptr; p.da = a.da;
   p.raw_hi = a.raw_hi; p.raw_lo = a.raw_lo; p.ld_raw = a.ld_raw; p.raw_col = a.raw_col; p.part = a.part; p.status = status_ptr();
   const int chains = a.B * a.H;
   ChainWrap wr{};
