@@ -195,8 +195,21 @@ __device__ __forceinline__ F2 add2(F2 a, F2 b) { F2 r; asm("add.rn.f32x2 %0, %1,
 __device__ __forceinline__ F2 mul2(F2 a, F2 b) { F2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 __device__ __forceinline__ F2 neg2(F2 v) { return v ^ 0x8000000080000000ull; }
-// 2^x with results below 2^-126 as zero
-__device__ __forceinline__ float ex2_ftz(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+// 2^x of each of the two over the whole range.  Results below 2^-126 as zeros would save three operations per value, but a decay may lie there, and a
+// row whose own x or dY is zero consists of such terms.
+__device__ __forceinline__ F2 ex2_two(F2 x) {
+  float2 v = unpack2(x);
+  asm("ex2.approx.f32 %0, %0;" : "+f"(v.x));
+  asm("ex2.approx.f32 %0, %0;" : "+f"(v.y));
+  return pack2(v.x, v.y);
+}
+// ... of values that are known to give normal numbers
+__device__ __forceinline__ F2 ex2_two_normal(F2 x) {
+  float2 v = unpack2(x);
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(v.x));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(v.y));
+  return pack2(v.x, v.y);
+}
 // softplus in the reference's stable form max(x,0)+log(1+exp(-|x|)) (pm-candle ops_impl.rs:123-133)
 __device__ __forceinline__ float softplus_acc(float x) { return fmaxf(x, 0.0f) + log1pf(expf(-fabsf(x))); }
 

@@ -21,14 +21,15 @@
 // What bounds it: no pipe and no memory level.  A step takes 8000 warp instructions at d_state 128 on plain operands, issued in 41 % of the
 // cycles; every role is a chain of TMEM loads, shared memory and arithmetic with two warps of it on a scheduler.  What shaped the roles are
 // clocks read inside a step of 16 x 8192 tokens, 32 heads of 128 x 64, bf16 (927 us when masking and output were one role and one warp issued
-// all products, 622 now):
+// all products, 602 now):
 //  - the products are issued by two warps: with one, its waits and the issue took 5000 of a step's 5200 clocks.  The warp index comes from a
 //    shuffle, so that the roles' branches and the descriptors are uniform to the compiler (742 -> 711 us, this kernel alone);
 //  - B and C are given back before the masked product waits for the mask, so that the next tiles (2200 clocks) land while it is masked;
 //  - bf16 x is the operand x~ as it is and comes by TMA: copied by the transform warps, their few pieces in flight took 4200 clocks a step;
 //  - a and dt are requested two chunks ahead (a head's tokens are a line apart), and below the diagonal the masked tile takes one
 //    exponential per row and block of 32 columns instead of one per element (not where M is rounded for a stream of bf16 values, see FACT);
-//  - the masked tile's exponents and products go in pairs, exponentials below 2^-126 are zeros (16 x 8192 709 -> 688 us, one prompt of 1337 95.5 -> 94.9);
+//  - the masked tile's exponents and products go in pairs, and a block whose smallest decay is a normal number takes exponentials without the scaling
+//    that smaller ones need (16 x 8192 633 us with the scaling everywhere, 602 with it where needed; a bf16 block of 8 x 2048 tokens 317 and 315);
 //  - the states that a backward reads leave by TMA from the operand tile, where they lie: stored by the threads that hold their rows, 32 lines to an
 //    instruction, they took half of the state's 4900 clocks of a step's 5700 (16 x 8192 710 -> 622 us, 9 x 1400 of 64 x 64 118 -> 102,
 //    16 x 512 of 128 x 64 61.5 -> 56.5);
@@ -41,6 +42,7 @@
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 #include "tc_common.cuh"
 #include "kernels.h"
@@ -397,19 +399,23 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_chain_fwd_kernel(const __grid
               split2(m1.x, m1.y, mh[2 * e4 + 1], ml[2 * e4 + 1], ND == 2);
             }
           } else {
+            auto block = [&](auto normal) {
 #pragma unroll
-            for (int e4 = 0; e4 < 8; ++e4) {
-              const ulonglong2 sv = *reinterpret_cast<const ulonglong2*>(S + 32 * cb + 4 * e4);
+              for (int e4 = 0; e4 < 8; ++e4) {
+                const ulonglong2 sv = *reinterpret_cast<const ulonglong2*>(S + 32 * cb + 4 * e4);
 #pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                const int e2 = 2 * e4 + u;
-                const float2 x = unpack2(mul2(fma2(u ? sv.y : sv.x, neg, Sr2), log2e));
-                float2 m = unpack2(mul2(pack2(__uint_as_float(r[2 * e2]), __uint_as_float(r[2 * e2 + 1])), pack2(ex2_ftz(x.x), ex2_ftz(x.y))));
-                if (FACT || cb == diag) { m.x = 2 * e2 <= lane ? m.x : 0.0f; m.y = 2 * e2 + 1 <= lane ? m.y : 0.0f; }
-                ml[e2] = 0u;
-                split2(m.x, m.y, mh[e2], ml[e2], ND == 2);
+                for (int u = 0; u < 2; ++u) {
+                  const int e2 = 2 * e4 + u;
+                  const F2 x = mul2(fma2(u ? sv.y : sv.x, neg, Sr2), log2e);
+                  float2 m = unpack2(mul2(pack2(__uint_as_float(r[2 * e2]), __uint_as_float(r[2 * e2 + 1])), decltype(normal)::value ? ex2_two_normal(x) : ex2_two(x)));
+                  if (FACT || cb == diag) { m.x = 2 * e2 <= lane ? m.x : 0.0f; m.y = 2 * e2 + 1 <= lane ? m.y : 0.0f; }
+                  ml[e2] = 0u;
+                  split2(m.x, m.y, mh[e2], ml[e2], ND == 2);
+                }
               }
-            }
+            };
+            // exp(S_t - S_s) of a block is a normal number (2^-125.5 and up) where that of the highest S_s is, for all rows
+            if (__any_sync(0xffffffffu, S_row - warp_max(S[32 * cb + lane]) < -87.0f)) block(std::false_type{}); else block(std::true_type{});
           }
         }
         tmem_st16(tg, mh);

@@ -6,8 +6,8 @@
 // Bound by the exponentials: 16 per clock and SM.  A warp may read one quarter of TMEM's lanes only, which is also one scheduler; with the
 // tile's rows in order the quarters of a tile on the diagonal would have one to four blocks of it to compute.  So the rows are dealt to the lanes in
 // groups of eight (lane 32 q + 8 i + r = row 32 i + 8 q + r, a rank-5 tensor map): every quarter has the same 10/16 of a diagonal tile.
-// 16384 tokens of 24 heads, chunks of 256 (192 tiles on 148 SMs): 42 us, 95 as a contraction whose warps loaded each head's S between two barriers;
-// 8192 tokens 21; pairs, 8192 tokens of 16 heads 23 (58).  Half as wide tiles, two CTAs to an SM: 39, 22 and 26.
+// 16384 tokens of 24 heads, chunks of 256 (192 tiles on 148 SMs): 47 us, 95 as a contraction whose warps loaded each head's S between two barriers;
+// 8192 tokens 26; pairs, 8192 tokens of 16 heads 19 (58).
 #include <cuda_bf16.h>
 #include <type_traits>
 #include "tc_common.cuh"
@@ -148,15 +148,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) ssd_dg_kernel(const __grid_consta
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) { mbar_arrive(bar(GFREE + b)); mbar_arrive(bar(EMPTY + s)); }
-      // rows 32 i + 8 q + er: all of them are past the columns (1), the block crosses the diagonal (0), none is (not called)
+      // rows 32 i + 8 q + er: all of them are past the columns (below), or the block crosses the diagonal
       auto fold = [&](int i, auto below) {
 #pragma unroll
         for (int o = 0; o < 4; ++o) {
           const int x = 4 * o + 2 * (i & 1);
-          const float2 u = unpack2(mul2(add2(pack2(nSr[i], nSr[i]), sc[o]), pack2(1.4426950408889634f, 1.4426950408889634f)));
-          float w0 = ex2_ftz(u.x), w1 = ex2_ftz(u.y);
-          if (!decltype(below)::value) { const int d = 8 * (q - o) + er - ec; w0 = d >= 0 ? w0 : 0.0f; w1 = d >= 1 ? w1 : 0.0f; }
-          acc[i][o] = fma2(pack2(__uint_as_float(r[i >> 1][x]), __uint_as_float(r[i >> 1][x + 1])), pack2(w0, w1), acc[i][o]);
+          float2 w = unpack2(ex2_two(mul2(add2(pack2(nSr[i], nSr[i]), sc[o]), pack2(1.4426950408889634f, 1.4426950408889634f))));
+          if (!decltype(below)::value) { const int d = 8 * (q - o) + er - ec; w.x = d >= 0 ? w.x : 0.0f; w.y = d >= 1 ? w.y : 0.0f; }
+          acc[i][o] = fma2(pack2(__uint_as_float(r[i >> 1][x]), __uint_as_float(r[i >> 1][x + 1])), pack2(w.x, w.y), acc[i][o]);
         }
       };
 #pragma unroll

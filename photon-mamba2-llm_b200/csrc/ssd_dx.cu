@@ -11,9 +11,8 @@
 // Bound by the latency of one CTA's chain (load, products, mask, product, epilogue), so the plan is sized for two CTAs per SM: 103 KB of shared
 // memory, 256 columns of TMEM (G 64, dM 64, two accumulators of 64), 96 registers.  Tiles of 32 x 32 above the diagonal are not computed.
 // 16384 tokens of 24 heads, chunks of 256: 206 us with one CTA per SM that wrote dx~ alone and 107 us for a pass over the rows behind it; with two
-// CTAs and the rows' work in the epilogue 158 and 12; 123 us now (400 MB: 61 us at the copy rate), by what clocks inside a CTA showed: a row per
-// thread cost 31 shuffles per 32 x 32 sums of columns (fragments: 7), fp32 operations in pairs and an exponential without the scaling that
-// denormal results need took a block's mask from 3500 to about 2200 clocks, and the epilogue's rows pass through shared memory, so that loads and
+// CTAs and the rows' work in the epilogue 158 and 12; 131 us now (400 MB: 61 us at the copy rate), by what clocks inside a CTA showed: a row per
+// thread cost 31 shuffles per 32 x 32 sums of columns (fragments: 7), fp32 operations in pairs shortened a block's mask of 3500 clocks, and the epilogue's rows pass through shared memory, so that loads and
 // stores are whole lines (a quad of lanes per row took half of the L1's cycles).
 #include <cuda_bf16.h>
 #include <type_traits>
@@ -257,8 +256,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) ssd_dx_kernel(const __grid_consta
 #pragma unroll
           for (int i = 0; i < 4; ++i) {                     // rows er + 8 i
             const int x = 4 * o + 2 * (i & 1), past = 8 * (o - i) + ec - er;      // t - s of the first of the two
-            const float2 u = unpack2(mul2(add2(sc, pack2(-S_row[i], -S_row[i])), pack2(1.4426950408889634f, 1.4426950408889634f)));
-            F2 mv = mul2(pack2(__uint_as_float(r[i >> 1][x]), __uint_as_float(r[i >> 1][x + 1])), pack2(ex2_ftz(u.x), ex2_ftz(u.y)));
+            const F2 w2 = ex2_two(mul2(add2(sc, pack2(-S_row[i], -S_row[i])), pack2(1.4426950408889634f, 1.4426950408889634f)));
+            F2 mv = mul2(pack2(__uint_as_float(r[i >> 1][x]), __uint_as_float(r[i >> 1][x + 1])), w2);
             if (decltype(diag)::value) { const float2 v = unpack2(mv); mv = pack2(past >= 0 ? v.x : 0.0f, past >= -1 ? v.y : 0.0f); }
             F2 w = mul2(pack2(__uint_as_float(d[i >> 1][x]), __uint_as_float(d[i >> 1][x + 1])), mv);
             if (decltype(diag)::value) { const float2 v = unpack2(w); w = pack2(past > 0 ? v.x : 0.0f, past > -1 ? v.y : 0.0f); }

@@ -5,8 +5,9 @@
 //   1. G = R K^T on the tensor core into one of two TMEM buffers (R = the CTA's 128 rows of C, K = 64 rows of B in
 //      mode 0; the roles of B and C swap in mode 1), K = d_state;
 //   2. four warps read G from TMEM (thread = row), multiply by exp(S_row - S_col) with the causal test in fp32
-//      registers (two elements to an operation, selects only where the diagonal crosses, exponentials below 2^-126 zeros: the fp32 scan of 8 x 2048
-//      tokens, 32 heads of 64 x 64, chunks of 256, 386 -> 382 us forward and 791 -> 737 backward, same bits), and write the masked tile back over G as a bf16 operand (hi and lo halves of the fp32 value in pair mode);
+//      registers (two elements to an operation, selects only where the diagonal crosses: the fp32 scan of 8 x 2048 tokens, 32 heads of
+//      64 x 64, chunks of 256, backward 791 -> 755 us, same bits), and write the masked tile back over G as a bf16 operand (hi and lo halves of
+//      the fp32 value in pair mode);
 //   3. acc1 += masked tile x V (V = 64 rows of x~ in mode 0, of dY in mode 1; MN-major) on the tensor core;
 // while step 2 of block j runs, the tensor core already computes step 1 of block j+1.  The carried-state term
 // (C h_prev in mode 0, B dh in mode 1) goes to a second accumulator and is scaled per row in the epilogue, which
@@ -380,9 +381,8 @@ ssd_fused_kernel(const __grid_constant__ Maps maps, const Params p) {
                 const int e = 4 * e4 + 2 * u, col = b0 + e;
                 const F2 sc = u ? s4.y : s4.x;
                 // MODE 0: row = t, col = s: exp(S_t - S_s) for s <= t;  MODE 1: row = s, col = t: exp(S_t - S_s) for t >= s
-                const float2 x = unpack2(mul2(MODE == 0 ? fma2(sc, neg, Sr2) : add2(sc, nSr2), log2e));
-                const F2 g2 = pack2(__uint_as_float(r[e]), __uint_as_float(r[e + 1]));
-                F2 m2 = mul2(g2, pack2(ex2_ftz(x.x), ex2_ftz(x.y)));
+                const F2 w2 = ex2_two(mul2(MODE == 0 ? fma2(sc, neg, Sr2) : add2(sc, nSr2), log2e));
+                F2 m2 = mul2(pack2(__uint_as_float(r[e]), __uint_as_float(r[e + 1])), w2);
                 float2 m = unpack2(m2);
                 if (!IN) {
                   m.x = (MODE == 0 ? col <= row : col >= row) ? m.x : 0.0f;

@@ -13,9 +13,9 @@
 // products of the next head running under the sums of this one, and one above, where the next head's dG product runs ahead instead.
 // What bounds it: the operands' bytes, half of HBM's rate, and the latency of a head's chain (product, TMEM load, sum, hand-over).  Bf16, 8 x 4096
 // tokens, 32 heads of 128 x 64: 197 us when d_state was taken in two passes over the heads (826 MB read) and dG's warps took nine instructions
-// per element one by one; 235 in one pass (558 MB) with half as many dG warps: theirs was the longest chain; 129 now that exponents and sums go
-// in pairs and results below 2^-126 are zeros (53 -> 31 M warp instructions).  16 x 1024 of 64 x 64: 68 and 55 us; 16 x 8192 of 128 x 64:
-// 700 and 450.  (Three stages instead of two, a warp index from a shuffle and a look at the barrier before a wait brought 836 to 680 before.)
+// per element one by one; 235 in one pass (558 MB) with half as many dG warps: theirs was the longest chain; 172 now that exponents and sums go
+// in pairs (146 with decays below 2^-126 as zeros, whose scaling doubles the operations of a pair; a test by 16 columns or by heads that skips it
+// where no decay is that small cost more than it saved).  16 x 1024 of 64 x 64: 61 us; 16 x 8192 of 128 x 64: 570.  (Three stages instead of two, a warp index from a shuffle and a look at the barrier before a wait brought 836 to 680 before.)
 // At 24 heads of 64 x 64 on pairs, 4 x 512 tokens: 18 us + 3 us for the sum of the shares.
 #include <cuda_bf16.h>
 #include "tc_common.cuh"
@@ -260,8 +260,7 @@ __global__ void __launch_bounds__(Geo<NI, ND, NK>::NTHREADS, 1) ssd_heads_kernel
 #pragma unroll
         for (int e = 0; e < 8; e += 2) {
           const ulonglong2 s4 = *reinterpret_cast<const ulonglong2*>(S + c0 + 2 * e);
-          const float2 u0 = unpack2(mul2(fma2(s4.x, neg, Sr2), log2e)), u1 = unpack2(mul2(fma2(s4.y, neg, Sr2), log2e));
-          w[e] = pack2(ex2_ftz(u0.x), ex2_ftz(u0.y)); w[e + 1] = pack2(ex2_ftz(u1.x), ex2_ftz(u1.y));
+          w[e] = ex2_two(mul2(fma2(s4.x, neg, Sr2), log2e)); w[e + 1] = ex2_two(mul2(fma2(s4.y, neg, Sr2), log2e));
         }
         if (c0 + 15 > quarter * 32) {                        // (the diagonal may cross)
 #pragma unroll

@@ -9,7 +9,7 @@ import pytest
 import torch
 
 from oracle import mamba2_oracle as orc
-from util import FP32_TOL, assert_close, block_params, cuda_params, randn, tol_for
+from util import FP32_TOL, assert_close, block_params, cuda_params, rand, randn, tol_for
 
 pytestmark = pytest.mark.gpu
 
@@ -804,3 +804,50 @@ def test_scan_bf16_kept_states(pm, T, N, P):
     orc.ssd_scan_chunked(leaves[0], leaves[1], *(t.expand(B, T, H, N) for t in leaves[2:]), 128 if T % 128 == 0 else T).backward(dy.double())
     for got, ref, tol, what in ((dx.float(), leaves[0].grad, 5e-3, "dx"), (da, leaves[1].grad, 5e-3, "da"), (db.float(), leaves[2].grad, 5e-3, "db"), (dc.float(), leaves[3].grad, 5e-3, "dc")):
         assert_close(got, ref, tol=tol, what=what)
+
+
+# decays between e^-92 and e^-88, below the smallest normal number: every second x and every other dY are zero, so that rows of the results consist of such
+# terms alone.  A masked element is kept in bf16 (pairs), whose steps there are 2^-133: 2^-134 |x| of a result's largest, 3e-37, and a bf16 result's 2^-9.
+@pytest.mark.parametrize("dtype,T,N,Q", [(torch.float32, 256, 64, 128), (torch.float32, 512, 64, 256), (torch.bfloat16, 256, 64, 128), (torch.bfloat16, 512, 128, 256),
+                                         (torch.bfloat16, 200, 64, 128)])
+def test_scan_of_subnormal_decays(pm, dtype, T, N, Q):
+    B, H, P = 2, 4, 64
+    x, b, c, dy = (randn(s, i + 1).to(dtype) for i, s in enumerate([(B, T, H, P), (B, T, 1, N), (B, T, 1, N), (B, T, H, P)]))
+    x[:, 1::2] = 0
+    dy[:, 0::2] = 0
+    a = -88.0 - 4.0 * rand((B, T, H), 5)
+    scan = (pm.SsdScan if dtype == torch.float32 else pm.SsdScanBf16)(x.cuda(), a.cuda(), b.cuda(), c.cuda(), Q if T % Q == 0 else T)
+    y = scan.forward()
+    _, da, db, dc = scan.backward(dy.cuda())
+    assert pm.device_status() == 0
+    leaves = [t.double().requires_grad_(True) for t in (x, a, b, c)]
+    ref = orc.ssd_scan_chunked(leaves[0], leaves[1], *(t.expand(B, T, H, N) for t in leaves[2:]), Q if T % Q == 0 else T)
+    ref.backward(dy.double())
+    for got, want, what in ((y[:, 1::2], ref[:, 1::2], "y"), (da, leaves[1].grad, "da"), (db, leaves[2].grad, "db"), (dc, leaves[3].grad, "dc")):
+        assert_close(got.float(), want, tol=5e-3, what=what)
+
+
+# the same in the backward of whole chunks on plain operands (csrc/ssd_dx.cu): d_a_log is a sum of such terms.  The reference takes the diagonal, which does
+# not depend on the decays, by itself: its row and column sums would leave 1e-16 of it.
+@pytest.mark.parametrize("T,Q", [(128, 128), (256, 256), (512, 256)])
+def test_block_bf16_backward_of_subnormal_decays(pm, monkeypatch, T, Q):
+    def scan(x, a, b, c, block_len):
+        S = torch.cumsum(a, 1).transpose(1, 2)
+        below = torch.ones(T, T, dtype=torch.bool).tril(-1)
+        G = torch.einsum("bthn,bshn->bhts", c, b)
+        M = G * torch.exp((S.unsqueeze(3) - S.unsqueeze(2)).masked_fill(~below, -float("inf"))) + G * torch.eye(T, dtype=G.dtype)
+        return torch.einsum("bhts,bshp->bthp", M, x)
+
+    cfg, p, blk = _block(pm, 256, 8, 64, 64, 1, Q, torch.bfloat16)
+    p["in_proj_weight"][:, -cfg.n_heads:] = 0                       # dt = softplus(0.5413) = 1 everywhere
+    p["dt_bias"].fill_(0.541324854612918)
+    p["a_log"] = torch.log(88.5 + torch.arange(cfg.n_heads) * 0.25)
+    blk = pm.Mamba2Block(blk.config, {k: v.cuda() for k, v in p.items()}, compute_dtype=torch.bfloat16)
+    x, cot = randn((2, T, 256), 32).bfloat16(), (randn((2, T, 256), 33) * 1e4).bfloat16()
+    _, grads = blk.backward(x.cuda(), cot.cuda())
+    monkeypatch.setattr(orc, "ssd_scan_ops_default", scan)
+    leaves = {k: v.double().requires_grad_(True) for k, v in p.items()}
+    orc.block_forward(leaves, cfg, x.double()).backward(cot.double())
+    assert float(leaves["a_log"].grad.abs().max()) < 1e-30
+    assert_close(grads["a_log"], leaves["a_log"].grad, tol=2e-2, what="d_a_log")
+    assert pm.device_status() == 0
