@@ -457,9 +457,18 @@ __global__ void __launch_bounds__(MAXQ) ssd_dx_finish_kernel(const float* __rest
 
 size_t ssd_dx_sum_floats(int B, int T, int H) { return (size_t)sdx::NSUM * B * T * H; }
 
-pmb_status ssd_dx(cudaStream_t st, const DxArgs& a) {
-  if (a.P != 64 || a.N != 64 || (a.Q != 128 && a.Q != 256) || a.T % a.Q || a.H % a.G || (a.ldx | a.lddy | a.lddx) & 1 || (int64_t)a.B * a.T * a.H >= (1LL << 31) / 64)
+pmb_status ssd_dx_check(const DxArgs& a) {
+  if (a.P != 64 || a.N != 64 || (a.Q != 128 && a.Q != 256) || a.T % a.Q || a.H % a.G)
     return fail(PMB_ERR_UNSUPPORTED, "ssd_dx: unsupported shape (P=%d N=%d Q=%d)", a.P, a.N, a.Q);
+  if ((int64_t)a.B * a.T >= (1LL << 31) || (int64_t)a.B * (a.T / a.Q) * a.H * a.N >= (1LL << 31))
+    return fail(PMB_ERR_UNSUPPORTED, "ssd_dx: too many rows for 32-bit tile coordinates");
+  auto off16 = [](const void* q, int64_t ld) { return (reinterpret_cast<uintptr_t>(q) & 15) != 0 || (ld & 3) != 0; };
+  if (off16(a.x, a.ldx) || off16(a.dy, a.lddy) || off16(a.dx, a.lddx)) return fail(PMB_ERR_UNSUPPORTED, "ssd_dx: x, dy and dx rows must be 16-byte aligned");
+  return PMB_OK;
+}
+
+pmb_status ssd_dx(cudaStream_t st, const DxArgs& a) {
+  PMB_TRY(ssd_dx_check(a));
   const int nc = a.T / a.Q, chunks = a.B * nc;
   const int64_t tok = (int64_t)a.B * a.T, HP = (int64_t)a.H * sdx::PW;
   sdx::Maps ms{};

@@ -140,6 +140,7 @@ struct DxArgs {
   SsdGrads::RawDt raw;     // gradient before the softplus (hi alone)
 };
 size_t ssd_dx_sum_floats(int B, int T, int H);
+pmb_status ssd_dx_check(const DxArgs& a);      // what ssd_dx takes; touches no memory
 pmb_status ssd_dx(cudaStream_t st, const DxArgs& a);
 
 unsigned int* ssd_fused_status();

@@ -3,6 +3,7 @@ declares, and its host-only entry points behave (sizes, shape errors).  No kerne
 import ctypes as C
 import pathlib
 import re
+import subprocess
 
 import pytest
 
@@ -78,3 +79,44 @@ def test_rust_ffi_declares_every_symbol():
     ffi = (ROOT / "rust" / "pm-b200" / "src" / "ffi.rs").read_text()
     bound = set(re.findall(r"pub fn (pmb_[a-z0-9_]+)\s*\(", ffi))
     assert bound == declared, sorted(bound ^ declared)
+
+
+DX_CHECK = r"""
+#include <cstdio>
+#include "ssd_fused.h"
+using namespace pmb;
+static float* at(uintptr_t a) { return reinterpret_cast<float*>(a); }
+int main() {
+  auto args = [] {
+    DxArgs a{};
+    a.B = 2; a.T = 512; a.H = 24; a.P = 64; a.N = 64; a.G = 1; a.Q = 256;
+    a.x = at(0x1000); a.dy = at(0x2000); a.dx = at(0x3000); a.ldx = 1668; a.lddy = 1536; a.lddx = 1668;
+    return a;
+  };
+  auto show = [](const DxArgs& a) { printf("%d\n", (int)ssd_dx_check(a)); };
+  DxArgs a = args(); show(a);
+  a = args(); a.B = 1024; a.T = 8192; a.H = 8; show(a);                 // 2^26 (token, head)s: 2^24 rows of states
+  a = args(); a.ldx = 1666; show(a);
+  a = args(); a.lddy = 1538; show(a);
+  a = args(); a.lddx = 1667; show(a);
+  a = args(); a.x = at(0x1004); show(a);
+  a = args(); a.dy = at(0x2008); show(a);
+  a = args(); a.dx = at(0x300c); show(a);
+  a = args(); a.Q = 512; show(a);
+  a = args(); a.T = 500; show(a);
+  a = args(); a.B = 1 << 22; show(a);                                   // 2^31 tokens
+  a = args(); a.B = 1 << 15; a.T = 4096; a.H = 64; show(a);             // 2^31 rows of states
+}
+"""
+
+
+def test_scan_gradient_takes_whole_16_byte_rows_only(tmp_path):
+    """ssd_dx reads and writes rows of x, dy and dx in 16-byte pieces: what is not on that grid is refused before any launch."""
+    import __graft_entry__ as ge
+    ge.build()
+    pkg = ROOT / "photon-mamba2-llm_b200"
+    (tmp_path / "dx.cu").write_text(DX_CHECK)
+    subprocess.run(["nvcc", "-std=c++17", "-arch=sm_100a", "-I", str(pkg / "csrc"), "-o", str(tmp_path / "dx"), str(tmp_path / "dx.cu"),
+                    str(pkg / "pm_b200" / "libpm_b200.so"), "-Xlinker", f"-rpath={pkg / 'pm_b200'}"], check=True, capture_output=True)
+    out = subprocess.run([str(tmp_path / "dx")], check=True, capture_output=True, text=True).stdout.split()
+    assert out[:2] == ["0", "0"] and len(out) == 12 and all(s != "0" for s in out[2:]), out
