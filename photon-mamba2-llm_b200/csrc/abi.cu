@@ -90,6 +90,22 @@ pmb_status order_after(cudaStream_t from, cudaEvent_t ev, cudaStream_t to) {
   return PMB_OK;
 }
 
+static bool same_capture(cudaStream_t a, cudaStream_t b) {
+  cudaStreamCaptureStatus sa, sb;
+  unsigned long long ia = 0, ib = 0;
+  return cudaStreamGetCaptureInfo(a, &sa, &ia) == cudaSuccess && cudaStreamGetCaptureInfo(b, &sb, &ib) == cudaSuccess && sa == sb &&
+         (sa != cudaStreamCaptureStatusActive || ia == ib);
+}
+
+pmb_status lanes_joined(cudaStream_t st, pmb_status s) {
+  int dev = 0;
+  if (s == PMB_OK || cudaGetDevice(&dev) != cudaSuccess) return s;
+  for (auto& [key, l] : t_lanes.lanes)
+    if (key / 7 == dev && l.s && l.s != st && same_capture(st, l.s) && cudaEventRecord(l.ev[5], l.s) == cudaSuccess) cudaStreamWaitEvent(st, l.ev[5], 0);
+  cudaGetLastError();                                        // (what the call failed with is kept)
+  return s;
+}
+
 }  // namespace pmb
 
 using namespace pmb;

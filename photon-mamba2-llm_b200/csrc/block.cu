@@ -524,9 +524,9 @@ static pmb_status block_grads(cudaStream_t st, const Dims& d, const pmb_block_pa
   return PMB_OK;
 }
 
-pmb_status block_bwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, const void* x, const void* dout,
-                     const void* dx_accum, void* dx, const pmb_block_grads& g, void* ws, size_t ws_bytes, const Weights16* wx,
-                     bool dout_pair_ready, bool emit_dx_pair) {
+static pmb_status block_bwd_on_lanes(cudaStream_t st, const Dims& d, const pmb_block_params& p, const void* x, const void* dout,
+                                     const void* dx_accum, void* dx, const pmb_block_grads& g, void* ws, size_t ws_bytes, const Weights16* wx,
+                                     bool dout_pair_ready, bool emit_dx_pair) {
   // On pairs dnormed = dout W_out^T, which needs nothing of the recompute, runs beside it, and what both multiply is split in one launch, as long as
   // the recompute's projection leaves room beside it.  Backward in us, after the recompute / beside it, by tiles of in_proj: 3 (2 x 128 tokens, 8
   // heads of 32 x 16) 115 / 109, 10 (2 x 256, 16 of 64 x 64) 125 / 115, 39 (2 x 384, 24) 188 / 172, 52 200 / 188, 68 237 / 229, 78 238 / 231, but
@@ -551,6 +551,12 @@ pmb_status block_bwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, 
   }
   PMB_TRY(block_recompute(st, d, p, x, ws, ws_bytes, wx, 1, 0, early != nullptr));
   return block_grads(st, d, p, x, dout, dx_accum, dx, g, ws, ws_bytes, wx, 1, 0, nullptr, dout_pair_ready, emit_dx_pair, early);
+}
+
+pmb_status block_bwd(cudaStream_t st, const Dims& d, const pmb_block_params& p, const void* x, const void* dout,
+                     const void* dx_accum, void* dx, const pmb_block_grads& g, void* ws, size_t ws_bytes, const Weights16* wx,
+                     bool dout_pair_ready, bool emit_dx_pair) {
+  return lanes_joined(st, block_bwd_on_lanes(st, d, p, x, dout, dx_accum, dx, g, ws, ws_bytes, wx, dout_pair_ready, emit_dx_pair));
 }
 
 }  // namespace pmb
@@ -605,9 +611,9 @@ pmb_status stack_fwd(cudaStream_t st, const Dims& d, int n_layers, const pmb_blo
 // gradient kernels of block l, into the other forward slot: it needs only the saved block input, and at a few
 // thousand tokens both halves are latency-bound chains that leave most SMs idle, so they overlap well.
 // PMB_RECOMPUTE_AHEAD=0 turns it off.
-pmb_status stack_bwd(cudaStream_t st, const Dims& d, int n_layers, const pmb_block_params* layers, const Weights16* w16,
-                     const pmb_block_grads* grads, const void* saved, void* dhidden, void* ws, size_t ws_bytes,
-                     pmb_layer_callback on_layer_done, void* user) {
+static pmb_status stack_bwd_on_lanes(cudaStream_t st, const Dims& d, int n_layers, const pmb_block_params* layers, const Weights16* w16,
+                                     const pmb_block_grads* grads, const void* saved, void* dhidden, void* ws, size_t ws_bytes,
+                                     pmb_layer_callback on_layer_done, void* user) {
   const bool bf = storage_is_bf16(w16);
   size_t slot = (size_t)d.M * d.D * (bf ? 2 : 4);
   const char* base = static_cast<const char*>(saved);
@@ -667,6 +673,12 @@ pmb_status stack_bwd(cudaStream_t st, const Dims& d, int n_layers, const pmb_blo
   }
   if (cl) PMB_TRY(order_after(st, cl->ev[1], user_st));
   return PMB_OK;
+}
+
+pmb_status stack_bwd(cudaStream_t st, const Dims& d, int n_layers, const pmb_block_params* layers, const Weights16* w16,
+                     const pmb_block_grads* grads, const void* saved, void* dhidden, void* ws, size_t ws_bytes,
+                     pmb_layer_callback on_layer_done, void* user) {
+  return lanes_joined(st, stack_bwd_on_lanes(st, d, n_layers, layers, w16, grads, saved, dhidden, ws, ws_bytes, on_layer_done, user));
 }
 
 }  // namespace pmb

@@ -7,13 +7,16 @@ namespace pmb {
 // ---- abi.cu: side streams for kernels that do not depend on each other.  One stream per (device, lane index) and six events per
 // thread of it, created on first use (so a thread's first call should come before any stream capture).  lane 0: scan
 // backward chains; 1: gradient GEMMs of a block that are off the critical path; 2: scan forward; 3: recompute-ahead;
-// 4: embedding-table gradient (fp32) or gradient of the hidden rows (bf16) of the LM head; 5: unused; 6: the gradient kernels of the stack backward (high priority,
+// 4: embedding-table gradient (fp32) or gradient of the hidden rows (bf16) of the LM head; 5: the dB branch of the scan backward; 6: the gradient kernels of the stack backward (high priority,
 // like lane 0).  *out stays NULL past device 63.
 struct SideLane { cudaStream_t s = nullptr; cudaEvent_t ev[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr}; };
 pmb_status get_side_lane(int idx, SideLane** out);
 void set_lanes_enabled(int on);
 // `to` waits for everything enqueued on `from` so far
 pmb_status order_after(cudaStream_t from, cudaEvent_t ev, cudaStream_t to);
+// Returns s.  A call that fails half-way may have work on lanes that nothing of the caller's waits for: then `st` waits for all that this thread's lanes
+// have been given, so that the caller can free what the call was working on, and a capture has no open fork.
+pmb_status lanes_joined(cudaStream_t st, pmb_status s);
 
 // ---- elementwise.cu
 // optional second output of the conv forward: columns [col0, col0 + width) of `act` (the B | C columns) as a (hi, lo)

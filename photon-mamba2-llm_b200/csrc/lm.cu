@@ -538,8 +538,7 @@ static pmb_status l1_split(pmb_lm* lm, cudaStream_t st, const void* src, int slo
   return PMB_OK;
 }
 
-extern "C" pmb_status pmb_lm_step_device(pmb_lm* lm, void* stream, const int64_t* d_ids, const int64_t* d_targets,
-                                         pmb_layer_callback on_layer_done, void* user) {
+static pmb_status lm_step_on_lanes(pmb_lm* lm, void* stream, const int64_t* d_ids, const int64_t* d_targets, pmb_layer_callback on_layer_done, void* user) {
   if (!lm || !d_ids || !d_targets) return fail(PMB_ERR_ARG, "lm_step: NULL argument");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const Dims& d = lm->d;
@@ -712,6 +711,11 @@ extern "C" pmb_status pmb_lm_step_device(pmb_lm* lm, void* stream, const int64_t
   }
   if (on_layer_done) on_layer_done(-1, user);
   return PMB_OK;
+}
+
+extern "C" pmb_status pmb_lm_step_device(pmb_lm* lm, void* stream, const int64_t* d_ids, const int64_t* d_targets,
+                                         pmb_layer_callback on_layer_done, void* user) {
+  return lanes_joined(static_cast<cudaStream_t>(stream), lm_step_on_lanes(lm, stream, d_ids, d_targets, on_layer_done, user));
 }
 
 // ---- data-parallel step: the same step with each layer's gradient bucket all-reduced (averaged) over the

@@ -1163,8 +1163,8 @@ static FusedArgs fused_args(const SsdIn& in, const SsdWs& ws) {
   return fa;
 }
 
-pmb_status ssd_fwd(cudaStream_t st, const SsdIn& in, const float* init_state, float* y, int64_t ldy, float* final_state,
-                   const SsdWs& ws) {
+static pmb_status ssd_fwd_on_lanes(cudaStream_t st, const SsdIn& in, const float* init_state, float* y, int64_t ldy, float* final_state,
+                                   const SsdWs& ws) {
   SsdP p;
   PMB_TRY(fill_params(in, ws, &p));
   p.yout = y; p.ldyo = ldy; p.yplain = in.y_plain;
@@ -1230,6 +1230,11 @@ pmb_status ssd_fwd(cudaStream_t st, const SsdIn& in, const float* init_state, fl
   return PMB_OK;
 }
 
+pmb_status ssd_fwd(cudaStream_t st, const SsdIn& in, const float* init_state, float* y, int64_t ldy, float* final_state,
+                   const SsdWs& ws) {
+  return lanes_joined(st, ssd_fwd_on_lanes(st, in, init_state, y, ldy, final_state, ws));
+}
+
 // dYs[b,t,h,:] = dY[b,t,h,:] exp(S[b,h,t]) as a bf16 pair (when the producer of dY did not already write it)
 __global__ void __launch_bounds__(256) dys_pair_kernel(const float* __restrict__ dy, int64_t lddy, const float* __restrict__ S,
                                                        uint16_t* __restrict__ hi, uint16_t* __restrict__ lo, int64_t rows, int T, int H, int P) {
@@ -1249,8 +1254,8 @@ bool ssd_bwd_takes_pairs(const SsdIn& in, const float* dy, int64_t lddy, const S
   return tc && fused_enabled() && ssd_fused_supported(in.P, in.N, in.Q) && (g.lddx % 4 == 0) && (reinterpret_cast<uintptr_t>(g.dx) % 16 == 0);
 }
 
-pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy, const float* dy, int64_t lddy,
-                   const SsdGrads& g, const SsdWs& ws) {
+static pmb_status ssd_bwd_on_lanes(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy, const float* dy, int64_t lddy,
+                                   const SsdGrads& g, const SsdWs& ws) {
   SsdP p;
   PMB_TRY(fill_params(in, ws, &p));
   const bool plain = in.y_plain && !in.y_plain_rarely;
@@ -1457,6 +1462,11 @@ pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy
     PMB_TRY(reduce(op.nsplit, p.N, 2, g.db, g.lddbc));
   }
   return PMB_OK;
+}
+
+pmb_status ssd_bwd(cudaStream_t st, const SsdIn& in, const float* y, int64_t ldy, const float* dy, int64_t lddy,
+                   const SsdGrads& g, const SsdWs& ws) {
+  return lanes_joined(st, ssd_bwd_on_lanes(st, in, y, ldy, dy, lddy, g, ws));
 }
 
 // ---------------------------------------------------------------------------------------------

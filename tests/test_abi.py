@@ -120,3 +120,19 @@ def test_scan_gradient_takes_whole_16_byte_rows_only(tmp_path):
                     str(pkg / "pm_b200" / "libpm_b200.so"), "-Xlinker", f"-rpath={pkg / 'pm_b200'}"], check=True, capture_output=True)
     out = subprocess.run([str(tmp_path / "dx")], check=True, capture_output=True, text=True).stdout.split()
     assert out[:2] == ["0", "0"] and len(out) == 12 and all(s != "0" for s in out[2:]), out
+
+
+def test_a_failed_call_leaves_nothing_on_side_streams(tmp_path):
+    """Blocks, stacks, scans and models put kernels on internal streams.  Whichever launch of a call fails, the caller's stream comes after those made before it."""
+    import __graft_entry__ as ge
+    ge.build()
+    pkg = ROOT / "photon-mamba2-llm_b200"
+    objs = [str(pkg / "build" / (f.name + ".o")) for f in sorted((pkg / "csrc").glob("*.cu"))]
+    if not all(pathlib.Path(o).exists() for o in objs):
+        pytest.skip("the library was not built here")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", "/usr/local/cuda/include", "-I", str(ROOT / "include"), "-o", str(tmp_path / "calls"), str(ROOT / "tests" / "fake_cuda.cpp"),
+                    *objs, "-ldl", "-lpthread"], check=True, capture_output=True)
+    out = subprocess.run([str(tmp_path / "calls")], check=True, capture_output=True, text=True).stdout
+    calls = [line.split() for line in out.splitlines()]
+    assert len(calls) == 17 and all(int(n) >= 3 for _, n, _ in calls), out
+    assert all(left == "0" for _, _, left in calls), out
