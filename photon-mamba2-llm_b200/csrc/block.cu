@@ -95,6 +95,8 @@ static bool block_uses_chain_bwd(const Dims& d, bool bf16) {
   return dims && close && ssd_chain_enabled() && ssd_chain_bwd_shape(d.P, d.N, true) && d.I <= 2048;
 }
 
+static bool block_plain16(const Dims& d, bool bf16) { return bf16 && ssd_plain16_shape(d.P, d.N, d.Q); }
+
 // The workspace has a forward part (everything the recompute produces and the gradient kernels read) and a
 // backward part.  With nslots == 2 the forward part exists twice, so that the recompute of the next block can run
 // (on another stream) while the gradient kernels of the current block still read the other copy; `slot` selects
@@ -122,7 +124,7 @@ static size_t block_ws_layout(const Dims& d, void* base, size_t bytes, BlockWs* 
       f.ssd.bc_hi = ar.take<uint16_t>((size_t)d.M * 2 * d.G * d.N); f.ssd.bc_lo = ar.take<uint16_t>((size_t)d.M * 2 * d.G * d.N);
       f.ssd.hp_hi = ar.take<uint16_t>(steps_np); f.ssd.hp_lo = ar.take<uint16_t>(steps_np);
     }
-    else ssd_ws_take(ar, d.B, d.T, d.H, d.P, d.N, d.G, d.Q, &f.ssd, 1);
+    else ssd_ws_take(ar, d.B, d.T, d.H, d.P, d.N, d.G, d.Q, &f.ssd, 1, block_plain16(d, bf16));
     f.seg = ar.take<float>(ssd_chain_shape(d.P, d.N) ? ssd_chain_seg_floats(d.B, d.T, d.H, d.P, d.N) : 0);
     f.normed16 = ar.take<uint16_t>(bf16 ? mi : 0);
     if (pairs) {
@@ -143,7 +145,7 @@ static size_t block_ws_layout(const Dims& d, void* base, size_t bytes, BlockWs* 
     w.seg_bwd = ar.take<float>(ssd_chain_seg_floats(d.B, d.T, d.H, d.P, d.N));
     w.ssd.splitk = ar.take<float>(ssd_heads_part_floats(d.B, d.T, d.H, d.N, d.G));
   }
-  else ssd_ws_take(ar, d.B, d.T, d.H, d.P, d.N, d.G, d.Q, &w.ssd, 2);
+  else ssd_ws_take(ar, d.B, d.T, d.H, d.P, d.N, d.G, d.Q, &w.ssd, 2, block_plain16(d, bf16));
   w.dnormed = pairs ? ar.take<float>(mi) : w.normed;
   // (with pair GEMMs the three producers of dxzd write the pair directly and the fp32 copy is never formed)
   w.dxzd = pairs ? nullptr : ar.take<float>(mj);
@@ -204,7 +206,6 @@ static uint32_t* chain_flags(const Dims& d, float* seg) { return (int64_t)d.B * 
 // forward and 0.6 % of its backward.  us, chains / chunk by chunk: forward 1 x 1024 tokens, 8 heads 53 / 46, 32 heads 70 / 75; 1 x 2048,
 // 24 heads 103 / 99; 2 x 2048, 24 heads 126 / 143; 4 x 2048, 8 heads 106 / 102; backward 1 x 512, 8 heads 115 / 114, 24 heads 156 / 162;
 // 2 x 2048, 24 heads 419 / 409, 32 heads 486 / 497; 4 x 4096, 24 heads 1194 / 1297.
-static bool block_plain16(const Dims& d, bool bf16) { return bf16 && ssd_plain16_shape(d.P, d.N, d.Q); }
 static bool scan_by_chunks(const Dims& d, bool bf16, bool keep) {
   const double steps = (double)cdiv(d.T, SCAN_STEP), chains = (double)d.B * d.H;
   if (!block_plain16(d, bf16)) return false;
@@ -257,7 +258,7 @@ static pmb_status block_fwd_core(cudaStream_t st, const Dims& d, const pmb_block
     a.S_out = w.ssd.S; a.dt_out = w.dt; a.A_out = w.Aneg; a.hp_hi = w.ssd.hp_hi; a.hp_lo = w.ssd.hp_lo; a.seg = w.seg;
     PMB_TRY(ssd_chain_fwd(st, a));
   } else if (block_plain16(d, w16 != nullptr) && bc.hi && ssd_chain_enabled() && !scan_by_chunks(d, true, true)) {
-    // the backward reads S, the states, x~, xs and the carried part of y: the chain leaves them on its way
+    // the backward reads S, the states, x~ and xs: the chain leaves them on its way
     ChainArgs a = chain_inputs(d, p, w.xzd, w.act, w.ssd.bc_hi, nullptr, w.y);
     a.blocks = d.Q / SCAN_STEP; a.seg = w.seg; a.flags_clear = bc.clear;
     a.S_out = w.ssd.S; a.dt_out = w.dt; a.A_out = w.Aneg; a.hp_hi = w.ssd.hp_hi; a.hprev = w.ssd.hprev; a.xt = w.ssd.xt_hi; a.xs = w.ssd.xs_hi;

@@ -102,7 +102,7 @@ size_t ssd_ws_layout(int B, int T, int H, int P, int N, int G, int Q, void* base
 bool ssd_wants_plain_y(int P, int N, int Q);      // shapes whose backward reads y_plain
 // the same buffers taken from a caller's arena in two parts: bit 0 = forward-written / backward-read, bit 1 = backward only
 struct Arena;
-void ssd_ws_take(Arena& ar, int B, int T, int H, int P, int N, int G, int Q, SsdWs* w, int part);
+void ssd_ws_take(Arena& ar, int B, int T, int H, int P, int N, int G, int Q, SsdWs* w, int part, bool plain16 = false);
 // The scan on bf16 inputs as they are (bf16 tensor-core operands, fp32 recurrence; no fp32 staging copies): any length, d_head up to
 // 64 and d_state up to 128 in multiples of 8.
 struct Scan16Ws {

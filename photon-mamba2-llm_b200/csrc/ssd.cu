@@ -991,7 +991,8 @@ static bool fused_enabled();
 
 // Buffers of one scan.  part bit 0: what the forward writes and the backward reads (kept per forward slot by the
 // block workspace); bit 1: what only the backward touches (one copy).  Fields of the other part are left alone.
-void ssd_ws_take(Arena& ar, int B, int T, int H, int P, int N, int G, int Q, SsdWs* wp, int part) {
+// plain16: the products read plain bf16 operands and ssd_dx.cu has the backward (ssd_plain16_shape), which needs neither the carried part of y nor sums of W.
+void ssd_ws_take(Arena& ar, int B, int T, int H, int P, int N, int G, int Q, SsdWs* wp, int part, bool plain16) {
   SsdWs& w = *wp;
   const int nc = T / Q;
   const bool tcshape = Q % 64 == 0 && N % 32 == 0 && P % 64 == 0;
@@ -1008,7 +1009,7 @@ void ssd_ws_take(Arena& ar, int B, int T, int H, int P, int N, int G, int Q, Ssd
     w.xt_hi = fz ? ar.take<uint16_t>(hp) : nullptr; w.xt_lo = fz ? ar.take<uint16_t>(hp) : nullptr;
     w.bc_hi = fz ? ar.take<uint16_t>(gn) : nullptr; w.bc_lo = fz ? ar.take<uint16_t>(gn) : nullptr;
     w.hp_hi = fz ? ar.take<uint16_t>(stn) : nullptr; w.hp_lo = fz ? ar.take<uint16_t>(stn) : nullptr;
-    w.yoff = fz ? ar.take<float>(hp) : nullptr;
+    w.yoff = fz && !plain16 ? ar.take<float>(hp) : nullptr;
   }
   if (part & 2) {
     if (fz) w.CB = ar.take<float>(qq);     // only for a backward that cannot take the fused kernel after a forward that did
@@ -1044,8 +1045,8 @@ void ssd_ws_take(Arena& ar, int B, int T, int H, int P, int N, int G, int Q, Ssd
     w.dy_hi = fz ? ar.take<uint16_t>(hp) : nullptr; w.dy_lo = fz ? ar.take<uint16_t>(hp) : nullptr;
     w.dh_hi = fz ? ar.take<uint16_t>(stn) : nullptr; w.dh_lo = fz ? ar.take<uint16_t>(stn) : nullptr;
     // the sums of W that the fused backward kernel leaves for the row-sum kernel
-    w.csum = fz ? ar.take<float>((size_t)B * T * H) : nullptr;
-    w.esum = fz ? ar.take<float>((size_t)B * T * H) : nullptr;
+    w.csum = fz && !plain16 ? ar.take<float>((size_t)B * T * H) : nullptr;
+    w.esum = fz && !plain16 ? ar.take<float>((size_t)B * T * H) : nullptr;
     w.rpart = fz ? ar.take<float>((size_t)B * T * H * (Q / 128)) : nullptr;
   }
 }
@@ -1315,10 +1316,10 @@ static pmb_status ssd_bwd_on_lanes(cudaStream_t st, const SsdIn& in, const float
   } else if (fz) {
     // dY as a bf16 pair (the B / C / x~ pairs were written by the forward of this scan and are still in the workspace)
     FusedArgs fa = fused_args(in, ws);
-    fa.v = Op16{ws.dy_hi, in.plain16 ? nullptr : ws.dy_lo, (int64_t)p.H * p.P};
-    fa.state = Op16{ws.dh_hi, in.plain16 ? nullptr : ws.dh_lo, p.P};
+    fa.v = Op16{ws.dy_hi, ws.dy_lo, (int64_t)p.H * p.P};
+    fa.state = Op16{ws.dh_hi, ws.dh_lo, p.P};
     fa.out = p.dxt; fa.ldo = (int64_t)p.H * p.P;
-    fa.xt = Op16{ws.xt_hi, in.plain16 ? nullptr : ws.xt_lo, (int64_t)p.H * p.P};
+    fa.xt = Op16{ws.xt_hi, ws.xt_lo, (int64_t)p.H * p.P};
     fa.csum = ws.csum; fa.esum = ws.esum; fa.rpart = ws.rpart;
     PMB_TRY(ssd_fused(st, 1, fa));
   }

@@ -31,6 +31,7 @@ constexpr int T128 = RB * 128, T64 = CW * 128;
 constexpr int STAGES = 3, STAGE = 2 * T64;                  // [C | dY] of a column block, then [dh | h] and the CTA's own rows of C
 constexpr int TILES = 2 * T128 + STAGES * STAGE + T128;     // [B | x~], ring, masked tile
 constexpr int NSUM = 5;                                     // per row: sum of W over t, e, <dx~, x>, <dY, exp(S) C h>, <dY, x>
+static_assert(NSUM <= PW, "the sums take the place of dx~ (B,T,H,P)");
 constexpr int SMEM = TILES + 1024 + 256 + (MAXQ + 4 * MAXQ + RB) * 4;
 constexpr int TMEM_COLS = 256;
 static_assert(2 * (SMEM + 1024) <= 227 * 1024, "two CTAs per SM");
@@ -454,8 +455,6 @@ __global__ void __launch_bounds__(MAXQ) ssd_dx_finish_kernel(const float* __rest
 }
 
 }  // namespace sdx
-
-size_t ssd_dx_sum_floats(int B, int T, int H) { return (size_t)sdx::NSUM * B * T * H; }
 
 pmb_status ssd_dx_check(const DxArgs& a) {
   if (a.P != 64 || a.N != 64 || (a.Q != 128 && a.Q != 256) || a.T % a.Q || a.H % a.G)

@@ -135,11 +135,10 @@ struct DxArgs {
   const float* x; int64_t ldx; const float* dy; int64_t lddy;
   float* dx; int64_t lddx; // dx~ dt + D dY
   const float* dd;         // (B*T/Q,H) <dh, h_prev>
-  float *rpart, *sums;     // scratch: (B*T/Q*H, Q/128, Q) and ssd_dx_sum_floats() floats
+  float *rpart, *sums;     // scratch: (B*T/Q*H, Q/128, Q) and, within the room of dx~ (B,T,H,P), five sums per row
   float* part;             // 3 x (B*T/Q,H): sums for dA, dD, d_dt_bias
   SsdGrads::RawDt raw;     // gradient before the softplus (hi alone)
 };
-size_t ssd_dx_sum_floats(int B, int T, int H);
 pmb_status ssd_dx_check(const DxArgs& a);      // what ssd_dx takes; touches no memory
 pmb_status ssd_dx(cudaStream_t st, const DxArgs& a);
 
