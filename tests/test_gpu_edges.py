@@ -851,3 +851,28 @@ def test_block_bf16_backward_of_subnormal_decays(pm, monkeypatch, T, Q):
     assert float(leaves["a_log"].grad.abs().max()) < 1e-30
     assert_close(grads["a_log"], leaves["a_log"].grad, tol=2e-2, what="d_a_log")
     assert pm.device_status() == 0
+
+
+# more chains than SMs where every head has its own B and C, while another stream's kernels hold SMs that the first blocks would be placed on: the same bits
+# as whole walks of a batch at a time (no sums over heads here)
+@pytest.mark.parametrize("B,H,T,P,N,Q", [(2, 80, 512, 64, 64, 128), (3, 64, 700, 64, 128, 128)])
+def test_scan_of_more_chains_than_sms_beside_another_stream(pm, B, H, T, P, N, Q):
+    x, b, c, dy = (randn(s, i).bfloat16().cuda() for i, s in enumerate([(B, T, H, P), (B, T, H, N), (B, T, H, N), (B, T, H, P)]))
+    a = (-torch.nn.functional.softplus(randn((B, T, H), 5) - 1.0)).cuda()
+
+    def call(i, j):
+        s = pm.SsdScanBf16(x[i:j], a[i:j], b[i:j], c[i:j], Q)
+        return s.forward(), *s.backward(dy[i:j])
+
+    want = [torch.cat(v) for v in zip(*(call(i, i + 1) for i in range(B)))]
+    other, m = torch.cuda.Stream(), torch.randn(4096, 4096, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(other):
+        for _ in range(8):
+            m = torch.tanh(m @ m)
+    got = [call(0, B) for _ in range(4)]
+    torch.cuda.synchronize()
+    assert pm.device_status() == 0
+    for run in got:
+        for u, v, what in zip(run, want, ("y", "dx", "da", "db", "dc")):
+            assert torch.equal(u, v), what
