@@ -88,7 +88,7 @@ static size_t slab_floats(const Dims& d) {
 // <dY, y - D x> - <x~, dx~>, 1e-4 of their norm from fp64 on unit-size inputs of 200 tokens and 2e-4 to 8e-4 at 1000 to 1337 (the chain kernels'
 // sums 1e-5 to 2.5e-5; all other gradients are equally far off; for smaller inputs see outweighed in ssd.cu), nor the faster one (forward and
 // backward of 2 x 1337 tokens, 24 heads of 64 x 64: 2395 us, 514 as chains; a stack of five on 2 x 740: 7.2 ms, 1.9).  That they stay is a choice
-// and no bound: fp32 results are held to 2e-4 between two builds, and those two gradients of a call would move by up to four times that, towards fp64.
+// and no bound: as chains those two gradients of a call would move by up to 8e-4 of their norm, towards fp64.
 static bool block_uses_chain_bwd(const Dims& d, bool bf16) {
   const bool dims = bf16 ? !ssd_plain16_shape(d.P, d.N, d.Q) && d.D % 8 == 0 && d.J % 8 == 0 && d.I % 8 == 0 : block_uses_pairs(d);
   const bool close = bf16 || d.in_model || ssd_fused_supported(d.P, d.N, d.Q) || d.Q <= (d.P >= 64 ? 256 : 64);
@@ -202,10 +202,11 @@ static uint32_t* chain_flags(const Dims& d, float* seg) { return (int64_t)d.B * 
 // not cut into segments here (that is built for S and states by steps, not by chunks of two, and would round other sums; more chains than SMs
 // share them in stretches of whole chunks, same sums).  What a chain's steps take, one
 // after the other, beyond a fixed cost, against the chunk-by-chunk kernels' time per step of a head; where a backward follows, the chain also
-// writes what that reads.  Fitted to 130 shapes of 8 to 32 heads, 512 to 8192 tokens: the slower side is taken by at most 1.3 % of a block's
-// forward and 0.6 % of its backward.  us, chains / chunk by chunk: forward 1 x 1024 tokens, 8 heads 53 / 46, 32 heads 70 / 75; 1 x 2048,
-// 24 heads 103 / 99; 2 x 2048, 24 heads 126 / 143; 4 x 2048, 8 heads 106 / 102; backward 1 x 512, 8 heads 115 / 114, 24 heads 156 / 162;
-// 2 x 2048, 24 heads 419 / 409, 32 heads 486 / 497; 4 x 4096, 24 heads 1194 / 1297.
+// writes what that reads.  Fitted to earlier kernels; of 87 shapes of 8 to 32 heads, 512 to 8192 tokens, the slower side is taken at eight: by 6 % of a
+// block's forward at 1 x 1024 of 24 heads, by 3 % at 3 x 1024 of 8, by less than 1 % elsewhere, and by 2.3 % of its backward at 2 x 512 of 16 heads, 1.7 %
+// at 1 x 512 of 8.  us, chains / chunk by chunk: forward 1 x 1024 tokens, 8 heads 50 / 42, 24 heads 64 / 60, 32 heads 68 / 69; 1 x 2048, 24 heads
+// 101 / 84; 2 x 2048, 24 heads 123 / 122, 32 heads 140 / 160; 4 x 2048, 8 heads 101 / 91; backward 1 x 512, 8 heads 90 / 92, 24 heads 136 / 135;
+// 2 x 2048, 24 heads 342 / 333, 32 heads 411 / 417; 4 x 4096, 24 heads 942 / 1022.
 static bool scan_by_chunks(const Dims& d, bool bf16, bool keep) {
   const double steps = (double)cdiv(d.T, SCAN_STEP), chains = (double)d.B * d.H;
   if (!block_plain16(d, bf16)) return false;

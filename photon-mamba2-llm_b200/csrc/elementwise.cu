@@ -16,12 +16,13 @@ static unsigned column_blocks(int cols) { return (unsigned)cdiv(cols, 32); }
 // row is read (run+K-1)/run times.  Bound by HBM.  A CTA of the vector kernels is 16 runs of 8 channel quads (128-byte strips of
 // its rows): no thread is idle for any channel count that is a multiple of 32.
 // Measured at 8 x 2048 tokens of 1664 channels: forward 68 us with runs of 8 all requested up front, 49 with the next four rows in registers,
-// 41 now: they wait in shared memory (cp.async), which leaves room for more CTAs (eight rows 41, pairs of channels 42); at 8 x 1024 16.4 and 13.9;
+// 43 now: they wait in shared memory (cp.async), which leaves room for more CTAs (eight rows and pairs of channels no better); at 8 x 1024 22;
 // backward (plain bf16 result) 131 us, 110 with four channels per thread and the next four rows in registers (170 of them, three CTAs per SM), 82 with
-// two channels and the next eight rows in shared memory, 57 now: that one was bound by issue (87 warp instructions per element in 79 % of the
+// two channels and the next eight rows in shared memory, 60 now: that one was bound by issue (87 warp instructions per element in 79 % of the
 // issue slots), so four channels go as two pairs of packed fp32 operations, with the next four rows in shared memory (128 registers); its bytes
-// alone take 42.  At 8 x 1024 45 and 34, at 4 x 512 with a (hi, lo) result 24 and 19, at 2 x 128 of 544 channels 5.6 and 5.7.  Sigmoids stay
-// scalar: an exponential of pairs was faster but 12 % further from fp64, and its flipped roundings grew past what two builds agree to.
+// alone take 42.  At 8 x 1024 36, at 4 x 512 with a (hi, lo) result 19 and 15, at 2 x 128 of 544 channels 6 either way.  Sigmoids stay
+// scalar: an exponential of pairs was faster but 12 % further from fp64, and its flipped roundings grew through 24 layers of bf16 storage until a
+// step's gradients had moved by more than 2e-2 of their norm.
 // ---------------------------------------------------------------------------------------------
 constexpr int CONV_AHEAD = 4;
 constexpr int CONV_SLICES = 16;

@@ -94,7 +94,7 @@ struct SsdWs {            // persistent between fwd and bwd of one scan
   uint16_t *dy_hi, *dy_lo;   // (B,T,H,P)  dY
   uint16_t *hp_hi, *hp_lo;   // (B,nc,H,N,P) state entering each chunk
   uint16_t *dh_hi, *dh_lo;   // (B,nc,H,N,P) adjoint of the state leaving each chunk
-  float* yoff;               // (B,T,H,P) exp(S_t) C_t h_prev: the carried-state part of y (forward -> backward)
+  float* yoff;               // (B,T,H,P) exp(S_t) C_t h_prev: the carried-state part of y (forward -> backward); plain operands go without
   float *csum, *esum;        // (B,T,H)   column sums of W and the dh term of dS (fused backward)
   float* rpart;              // (B,nc,H,Q/128,Q) partial row sums of W (fused backward)
 };

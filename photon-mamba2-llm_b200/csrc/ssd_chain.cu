@@ -18,10 +18,10 @@
 // warp 0 = TMA loads (B, C, bf16 x), 1 = products of the masked tile (G one item ahead, M x~), 2 = products of the state (C h, U), 3 = TMA
 // stores, 4..11 = two mask groups of four warps, then twelve warps of output and transform (eight and four; on fp32 pairs, whose
 // transform rounds every element twice, four and eight), 24..27 = state.
-// What bounds it: no pipe and no memory level.  A step takes 8000 warp instructions at d_state 128 on plain operands, issued in 41 % of the
+// What bounds it: no pipe and no memory level.  A step takes 7000 warp instructions at d_state 128 on plain operands, issued in 45 % of the
 // cycles; every role is a chain of TMEM loads, shared memory and arithmetic with two warps of it on a scheduler.  What shaped the roles are
 // clocks read inside a step of 16 x 8192 tokens, 32 heads of 128 x 64, bf16 (927 us when masking and output were one role and one warp issued
-// all products, 602 now):
+// all products, 584 now):
 //  - the products are issued by two warps: with one, its waits and the issue took 5000 of a step's 5200 clocks.  The warp index comes from a
 //    shuffle, so that the roles' branches and the descriptors are uniform to the compiler (742 -> 711 us, this kernel alone);
 //  - B and C are given back before the masked product waits for the mask, so that the next tiles (2200 clocks) land while it is masked;
@@ -35,9 +35,9 @@
 //    16 x 512 of 128 x 64 61.5 -> 56.5);
 //  - the kernel's 63 KB are about what the instruction cache holds for seven roles: an early return and a few selects by block, 72 KB, cost 8 %;
 //  - the segment is the grid's y and not a remainder that stays in a register: on pairs its spills cost 10 % (24.6 -> 22.2 us at 4 x 512).
-// Measured at 24 heads of 64 x 64: 22 us for 4 x 512 tokens on pairs, 25 with what a backward reads (23.9 and 26 before the above); 8 x 2048 on
-// plain operands in chunks of 256, 90 us, and 109 with all that a chunk-by-chunk backward reads (118 and 144 where every CTA walks whole chains, see
-// ssd_chain_wrap); 31 us (two launches over segments) for 1 x 1337 on pairs.  Every mbarrier wait is bounded; on expiry the CTA raises the status
+// Measured at 24 heads of 64 x 64: 23 us for 4 x 512 tokens on pairs, with what a backward reads or without; 8 x 2048 on
+// plain operands in chunks of 256, 96 us, and 109 with all that a chunk-by-chunk backward reads (136 where every CTA walks whole chains, see
+// ssd_chain_wrap); 30 us (two launches over segments) for 1 x 1337 on pairs.  Every mbarrier wait is bounded; on expiry the CTA raises the status
 // word, every role stops issuing work, copies in flight are waited for (bounded) and TMEM is freed on the way out.
 #include <cuda_bf16.h>
 #include <algorithm>
@@ -95,8 +95,8 @@ struct Geo {
   // (BIG: no room for column factors and half of the alignment slack; shared memory starts 1024-byte aligned where nothing static
   // precedes it, and the kernel checks)
   // The masked tile by factors of blocks instead of an exponential per element.  Not for storage blocks on plain operands, whose M is rounded to
-  // bf16 in a stream of bf16 values: a flipped rounding grows through the layers behind it, so that the gradients of two builds would differ
-  // by as much as bf16 storage itself puts them off (2e-2).  That is a choice, for results that repeat.
+  // bf16 in a stream of bf16 values: a flipped rounding grows through the layers behind it, so that the gradients of 24 layers would move
+  // by as much as bf16 storage itself puts them off fp64 (2e-2).  That is a choice, for results that repeat.
   static constexpr bool FACT = NB == 1 && !BIG && (ND == 2 || XIN16);
   static constexpr int BARS = XIN16 ? 320 : 256;         // bytes of barriers and small sums
   static constexpr int SLOT = (BIG ? 1 : 2) * L, SLACK = BIG ? 512 : 1024;    // floats per copy of S: [S | column factors]
@@ -907,6 +907,9 @@ size_t ssd_chain_seg_floats(int B, int T, int H, int P, int N) {
 // 10 x 1024 296 -> 280, but 8 x 2048 412 -> 421 (an eighth of the steps saved); the scan's backward on bf16 inputs, 32 heads of 128 x 64, 16 x 8192
 // 1927 -> 1750, 5 x 2048 207 -> 194, 8 x 4096 523 -> 485 (an eighth), 30 x 640 of 64 x 64 308 -> 301 (a 17th).  The forward on bf16 inputs, whose
 // steps are shorter, lost as often as it gained (16 x 8192 724 -> 744, 7 x 1024 58 -> 68, 8 x 2048 of 64 x 64 92 -> 92): it stays uncut.
+// Chains on pairs keep the segments of ssd_chain_plan, whose sums are others.  The forward of an fp32 block of 24 heads, segments / stretches: 8 x 384
+// tokens 120 / 121, 8 x 512 149 / 157, 9 x 768 231 / 233, 8 x 1024 270 / 266, 7 x 2048 443 / 439, 8 x 2048 502 / 485; 32 heads, 10 x 512 256 / 258,
+// 10 x 1024 487 / 466, 5 x 2048 484 / 462: from some 1000 tokens on stretches would give 1 to 5 %.
 bool ssd_chain_wrap(int64_t chains, int units, int steps_per_unit, double least_share, ChainWrap* w) {
   const int64_t total = chains * units, uncut = cdiv(chains, CHAIN_SMS) * units, saved = uncut - cdiv(total, CHAIN_SMS);
   if (chains <= CHAIN_SMS || chains > 0xffff || units < 2 || units > 0xffff) return false;

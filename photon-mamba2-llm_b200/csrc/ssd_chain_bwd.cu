@@ -25,9 +25,9 @@
 // transform (6500) comes on top.  Warps of their own for the output (28 of 72 registers) were no faster: 1317 us against 1271 for
 // 16 x 8192 tokens, 32 heads of 128 x 64 (1412 with one MMA warp, sums by 16 shuffles per 16 columns and an exponential per element), nor x and dY
 // prefetched into registers (50 us for 4 x 512 tokens, 24 heads of 64 x 64, on pairs) or read again by the output (49).
-// Measured at 24 heads of 64 x 64 on pairs: 45 us for 4 x 512 tokens (the d(states) product, reverse pass, masked product and row
-// kernel it replaces: 118 us), 31 us for 2 x 384, 53 us in segments for 2 x 1000 (1.7 ms of FMA contractions with ssd_heads.cu's share).
-// On bf16 inputs, 16 x 8192 tokens of 32 heads of 128 x 64 take 1073 us where 148 SMs share 512 chains in equal stretches (ssd_chain_wrap), 1240 whole.
+// Measured at 24 heads of 64 x 64 on pairs: 44 us for 4 x 512 tokens (the d(states) product, reverse pass, masked product and row
+// kernel it replaces: 118 us), 30 us for 2 x 384, 50 us in segments for 2 x 1000 (1.7 ms of FMA contractions with ssd_heads.cu's share).
+// On bf16 inputs, 16 x 8192 tokens of 32 heads of 128 x 64 take 1055 us where 148 SMs share 512 chains in equal stretches (ssd_chain_wrap), 1146 whole.
 // Every mbarrier wait is bounded, as in the forward.
 #include <cuda_bf16.h>
 #include <type_traits>

@@ -6,8 +6,8 @@
 // Bound by the exponentials: 16 per clock and SM.  A warp may read one quarter of TMEM's lanes only, which is also one scheduler; with the
 // tile's rows in order the quarters of a tile on the diagonal would have one to four blocks of it to compute.  So the rows are dealt to the lanes in
 // groups of eight (lane 32 q + 8 i + r = row 32 i + 8 q + r, a rank-5 tensor map): every quarter has the same 10/16 of a diagonal tile.
-// 16384 tokens of 24 heads, chunks of 256 (192 tiles on 148 SMs): 47 us, 95 as a contraction whose warps loaded each head's S between two barriers;
-// 8192 tokens 26; pairs, 8192 tokens of 16 heads 19 (58).
+// 16384 tokens of 24 heads, chunks of 256 (192 tiles on 148 SMs): 45 us, 95 as a contraction whose warps loaded each head's S between two barriers;
+// 8192 tokens 25; pairs, 8192 tokens of 16 heads 24 (58).
 #include <cuda_bf16.h>
 #include <type_traits>
 #include "tc_common.cuh"

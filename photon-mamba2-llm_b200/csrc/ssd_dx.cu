@@ -11,7 +11,7 @@
 // Bound by the latency of one CTA's chain (load, products, mask, product, epilogue), so the plan is sized for two CTAs per SM: 103 KB of shared
 // memory, 256 columns of TMEM (G 64, dM 64, two accumulators of 64), 96 registers.  Tiles of 32 x 32 above the diagonal are not computed.
 // 16384 tokens of 24 heads, chunks of 256: 206 us with one CTA per SM that wrote dx~ alone and 107 us for a pass over the rows behind it; with two
-// CTAs and the rows' work in the epilogue 158 and 12; 131 us now (400 MB: 61 us at the copy rate), by what clocks inside a CTA showed: a row per
+// CTAs and the rows' work in the epilogue 158 and 12; 124 us now (400 MB: 61 us at the copy rate), by what clocks inside a CTA showed: a row per
 // thread cost 31 shuffles per 32 x 32 sums of columns (fragments: 7), fp32 operations in pairs shortened a block's mask of 3500 clocks, and the epilogue's rows pass through shared memory, so that loads and
 // stores are whole lines (a quad of lanes per row took half of the L1's cycles).
 #include <cuda_bf16.h>

@@ -13,10 +13,11 @@
 // products of the next head running under the sums of this one, and one above, where the next head's dG product runs ahead instead.
 // What bounds it: the operands' bytes, half of HBM's rate, and the latency of a head's chain (product, TMEM load, sum, hand-over).  Bf16, 8 x 4096
 // tokens, 32 heads of 128 x 64: 197 us when d_state was taken in two passes over the heads (826 MB read) and dG's warps took nine instructions
-// per element one by one; 235 in one pass (558 MB) with half as many dG warps: theirs was the longest chain; 172 now that exponents and sums go
-// in pairs (146 with decays below 2^-126 as zeros, whose scaling doubles the operations of a pair; a test by 16 columns or by heads that skips it
-// where no decay is that small cost more than it saved).  16 x 1024 of 64 x 64: 61 us; 16 x 8192 of 128 x 64: 570.  (Three stages instead of two, a warp index from a shuffle and a look at the barrier before a wait brought 836 to 680 before.)
-// At 24 heads of 64 x 64 on pairs, 4 x 512 tokens: 18 us + 3 us for the sum of the shares.
+// per element one by one; 235 in one pass (558 MB) with half as many dG warps: theirs was the longest chain; 150 now that exponents and sums go
+// in pairs (12 to 15 % less with decays below 2^-126 as zeros, whose scaling doubles the operations of a pair; a test by 16 columns or by heads that skips it
+// where no decay is that small cost more than it saved).  16 x 1024 of 64 x 64: 55 us; 16 x 8192 of 128 x 64: 512.
+// (Three stages instead of two, a warp index from a shuffle and a look at the barrier before a wait brought 836 to 680 before.)
+// At 24 heads of 64 x 64 on pairs, 4 x 512 tokens: 17 us + 4 us for the sum of the shares.
 #include <cuda_bf16.h>
 #include "tc_common.cuh"
 #include "kernels.h"
